@@ -70,35 +70,41 @@ static void sign_bits(const double* v, uint32_t (&out)[4]) {
     if (v[e] < 0) out[e >> 5] |= 1u << (e & 31);
 }
 
-template <typename T>
-static int upload(T** dst, const std::vector<T>& src) {
-  TQ_CUDA(cudaMalloc((void**)dst, src.size() * sizeof(T)));
-  TQ_CUDA(cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return TQ_OK;
-}
+// The device arrays of a quantizer are parts of one allocation, filled by one copy: every allocation and every pageable
+// copy synchronises with the device, and a quantizer that is built inside a program pays for each of them.
+struct DeviceImage {
+  std::vector<uint8_t> bytes;
+  size_t add(const void* src, size_t n) {
+    const size_t at = (bytes.size() + 255) & ~(size_t)255;
+    bytes.resize(at + n);
+    memcpy(bytes.data() + at, src, n);
+    return at;
+  }
+};
 
-static int upload_matrix(const double* m, int d, double** dev, double** dev_t, float** dev32, float** dev32_t) {
-  std::vector<double> a(m, m + (size_t)d * d), t((size_t)d * d);
+struct MatrixParts {
+  size_t m, t, m32, t32;
+};
+static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
+  std::vector<double> t((size_t)d * d);
   std::vector<float> a32((size_t)d * d), t32((size_t)d * d);
   for (int i = 0; i < d; ++i)
     for (int j = 0; j < d; ++j) {
-      t[(size_t)j * d + i] = a[(size_t)i * d + j];
-      a32[(size_t)i * d + j] = (float)a[(size_t)i * d + j];
-      t32[(size_t)j * d + i] = (float)a[(size_t)i * d + j];
+      t[(size_t)j * d + i] = m[(size_t)i * d + j];
+      a32[(size_t)i * d + j] = (float)m[(size_t)i * d + j];
+      t32[(size_t)j * d + i] = (float)m[(size_t)i * d + j];
     }
-  int rc;
-  if ((rc = upload(dev, a)) != TQ_OK) return rc;
-  if ((rc = upload(dev_t, t)) != TQ_OK) return rc;
-  if (dev32 && (rc = upload(dev32, a32)) != TQ_OK) return rc;
-  if (dev32_t && (rc = upload(dev32_t, t32)) != TQ_OK) return rc;
-  return TQ_OK;
+  MatrixParts p;
+  p.m = im.add(m, t.size() * 8);
+  p.t = im.add(t.data(), t.size() * 8);
+  p.m32 = im.add(a32.data(), a32.size() * 4);
+  p.t32 = im.add(t32.data(), t32.size() * 4);
+  return p;
 }
 
 extern "C" int tq_quantizer_destroy(tq_quantizer* q) {
   if (!q) return TQ_OK;
-  void* ptrs[] = {q->rot, q->rot_t, q->s, q->s_t, q->cent64, q->bnd64, q->rot32, q->rot32_t, q->s32, q->s32_t};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
+  if (q->mem) cudaFree(q->mem);
   free(q);
   return TQ_OK;
 }
@@ -165,7 +171,7 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
     for (int i = 0; i < 65536; ++i) {
       const float a = 1.0f + (float)i / 65536.0f;
       double worst = 0.0;
-      for (int k = 0; k < nc; ++k) {
+      for (int k = 0; k < nc && worst < best; ++k) {   // (a factor already beaten needs no further centroids)
         const double want = (double)a * c[k];
         const double got = (double)__half2float(__float2half_rn((float)want));
         const double rel = want != 0.0 ? fabs(got / want - 1.0) : 0.0;
@@ -183,7 +189,9 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
     }
   }
 
-  int rc = TQ_OK;
+  DeviceImage im;
+  MatrixParts mr{}, ms{};
+  const bool dense_rot = desc->rotation == TQ_ROT_DENSE && desc->rot, dense_s = desc->rotation == TQ_ROT_DENSE && desc->qjl;
   if (desc->rotation == TQ_ROT_WHT) {
     sign_bits(desc->signs1, f.s1);
     sign_bits(desc->signs2, f.s2);
@@ -191,16 +199,22 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
       sign_bits(desc->qjl_signs1, f.j1);
       sign_bits(desc->qjl_signs2, f.j2);
     }
-  } else {
-    if (desc->rot) rc = upload_matrix(desc->rot, q->d, &q->rot, &q->rot_t, &q->rot32, &q->rot32_t);
-    if (rc == TQ_OK && desc->qjl) rc = upload_matrix(desc->qjl_s, q->d, &q->s, &q->s_t, &q->s32, &q->s32_t);
   }
-  if (rc == TQ_OK) rc = upload(&q->cent64, c);
-  if (rc == TQ_OK) rc = upload(&q->bnd64, b);
-  if (rc != TQ_OK) {
+  if (dense_rot) mr = add_matrix(im, desc->rot, q->d);
+  if (dense_s) ms = add_matrix(im, desc->qjl_s, q->d);
+  const size_t cent_at = im.add(c.data(), c.size() * 8), bnd_at = im.add(b.data(), b.size() * 8);
+  e = cudaMalloc((void**)&q->mem, im.bytes.size());
+  if (e == cudaSuccess) e = cudaMemcpy(q->mem, im.bytes.data(), im.bytes.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
     tq_quantizer_destroy(q);
-    return rc;
+    return tq_cuda_fail(e, "quantizer constants");
   }
+  auto f64 = [&](size_t at) { return reinterpret_cast<double*>(q->mem + at); };
+  auto f32 = [&](size_t at) { return reinterpret_cast<float*>(q->mem + at); };
+  if (dense_rot) q->rot = f64(mr.m), q->rot_t = f64(mr.t), q->rot32 = f32(mr.m32), q->rot32_t = f32(mr.t32);
+  if (dense_s) q->s = f64(ms.m), q->s_t = f64(ms.t), q->s32 = f32(ms.m32), q->s32_t = f32(ms.t32);
+  q->cent64 = f64(cent_at);
+  q->bnd64 = f64(bnd_at);
   *out = q;
   return TQ_OK;
 }

@@ -31,6 +31,7 @@ struct TqFast {
 struct tq_quantizer {
   int32_t d, bits, rotation, norm_correction, qjl, device;
   TqFast fast;               // valid when rotation == TQ_ROT_WHT
+  uint8_t* mem;              // the one device allocation that the pointers below point into
   // dense mode, device memory (fp64): R row-major, its transpose, S, its transpose
   double *rot, *rot_t, *s, *s_t;
   double* cent64;            // 1 << bits
