@@ -5,8 +5,26 @@ copy out.  Covers asymmetric K/V formats and boundary layers kept at higher prec
 """
 from __future__ import annotations
 
+import contextlib
+import gc
+
 from . import _native as nv
 from .paged import PagedKVCache
+
+
+@contextlib.contextmanager
+def _capture(torch, graph):
+    """torch.cuda.graph without the cyclic collector: what it frees -- another cache's graphs, events of pinned host
+    buffers -- makes CUDA calls that are not allowed while a stream is capturing, and a failure inside a tensor's
+    destructor ends the process."""
+    enabled = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.graph(graph):
+            yield
+    finally:
+        if enabled:
+            gc.enable()
 
 
 def boundary_format_table(num_layers: int, inner=("q8_0", "turbo2"), boundary=("q8_0", "q8_0"), keep: int = 2):
@@ -78,60 +96,54 @@ class LayeredKVCache:
             # pages at l * num_pages in the group's pool
             "slots": torch.zeros((max(len(m) for _, m in self.groups), batch), dtype=torch.int64, device=dev),
         }
-        ws = self.layers[0].workspace(batch, num_q_heads, st["bt"].shape[1])
-
+        st["workspace"] = self.layers[0].workspace(batch, num_q_heads, st["bt"].shape[1])
         # per format group: which layers, and where each layer's pages start inside the group's pool
-        plans = []
-        for whole, members in self.groups:
-            idx = None if members == list(range(L)) else torch.tensor(members, device=dev)
-            plans.append((whole, idx, len(members)))
-
-        def append_part():
-            # slots of the new tokens and the lengths' increment: one launch
-            with torch.cuda.device(dev):
-                nv.call("tq_decode_step_slots", nv.ptr(st["bt"]), st["bt"].shape[1], nv.ptr(st["len"]), self.page_tokens,
-                        batch, st["slots"].shape[0], self.num_pages * self.page_tokens, nv.ptr(st["slots"]),
-                        nv.stream_ptr())
-            # one quantize-on-append launch per format group: the new token of every layer of the group at once
-            for whole, idx, n in plans:
-                k = st["k"] if idx is None else st["k"].index_select(0, idx)
-                v = st["v"] if idx is None else st["v"].index_select(0, idx)
-                whole.append(k.reshape(n * batch, self.num_kv_heads, d), v.reshape(n * batch, self.num_kv_heads, d),
-                             st["slots"][:n].reshape(-1))
-
-        def attend_part(lo, hi):
-            for i in range(lo, hi):
-                layer = self.layers[i]
-                # An attention call that follows another layer's attention call may start early: that kernel writes
-                # nothing this one reads before its dependency wait, and the queries of every layer are in place
-                # before the first launch of the step (they arrive with the step's host-to-device copy).  The first
-                # call follows the append, which writes the cache slot of the new token: it runs in stream order, in
-                # the form of the calls that follow it.
-                layer.attend(st["q"][i], st["bt"], st["len"], out=st["out"][i], workspace=ws,
-                             overlap="q" if i > 0 else False, chain_head=(i == 0))
-
-        def body():
-            append_part()
-            attend_part(0, L)
-
+        st["plans"] = [(whole, None if members == list(range(L)) else torch.tensor(members, device=dev), len(members))
+                       for whole, members in self.groups]
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):      # warm-up outside capture (sets kernel attributes, fills caches)
             saved = st["len"].clone()
-            body()
+            self._append_part(st)
+            self._attend_part(st, 0, L)
             st["len"].copy_(saved)
         torch.cuda.current_stream(dev).wait_stream(side)
         torch.cuda.synchronize(dev)
         graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph):
-            body()
+        with _capture(torch, graph):
+            self._append_part(st)
+            self._attend_part(st, 0, L)
         st["len"].copy_(saved)
         st["graph"] = graph
-        st["body"] = body
-        st["parts"] = (append_part, attend_part)
         st["io_stream"] = side
         self._step = st
         return st
+
+    # (methods that take the step's state, not closures kept in it: a cache that is dropped is then freed at once, with
+    # its graphs and buffers, instead of waiting for the cyclic collector)
+    def _append_part(self, st):
+        """Slots of the new tokens and the lengths' increment, then one quantize-on-append launch per format group: the
+        new token of every layer of the group at once."""
+        torch = nv.require_cuda()
+        _, batch, _, d = st["q"].shape
+        with torch.cuda.device(self.device):
+            nv.call("tq_decode_step_slots", nv.ptr(st["bt"]), st["bt"].shape[1], nv.ptr(st["len"]), self.page_tokens,
+                    batch, st["slots"].shape[0], self.num_pages * self.page_tokens, nv.ptr(st["slots"]), nv.stream_ptr())
+        for whole, idx, n in st["plans"]:
+            k = st["k"] if idx is None else st["k"].index_select(0, idx)
+            v = st["v"] if idx is None else st["v"].index_select(0, idx)
+            whole.append(k.reshape(n * batch, self.num_kv_heads, d), v.reshape(n * batch, self.num_kv_heads, d),
+                         st["slots"][:n].reshape(-1))
+
+    def _attend_part(self, st, lo, hi):
+        for i in range(lo, hi):
+            # An attention call that follows another layer's attention call may start early: that kernel writes
+            # nothing this one reads before its dependency wait, and the queries of every layer are in place
+            # before the first launch of the step (they arrive with the step's host-to-device copy).  The first
+            # call follows the append, which writes the cache slot of the new token: it runs in stream order, in
+            # the form of the calls that follow it.
+            self.layers[i].attend(st["q"][i], st["bt"], st["len"], out=st["out"][i], workspace=st["workspace"],
+                                  overlap="q" if i > 0 else False, chain_head=(i == 0))
 
     def host_buffers(self):
         """Pinned host tensors (q, k, v, out) for decode_step, q/k/v carved from one allocation in the order of the
@@ -170,9 +182,8 @@ class LayeredKVCache:
         if st.get("io_key") == key or all(t.is_pinned() for t in hosts):
             if st.get("io_key") != key:
                 graph = torch.cuda.CUDAGraph()
-                append_part, attend_part = st["parts"]
                 side, half = st["io_stream"], self.num_layers // 2
-                with torch.cuda.graph(graph):
+                with _capture(torch, graph):
                     # The copies are branches of the graph.  In: the new K/V rows first, then the queries on a side
                     # branch under the append, which needs only the rows.  Out: the outputs of the lower half of the
                     # layers leave while the upper half is still computing.
@@ -189,13 +200,13 @@ class LayeredKVCache:
                     side.wait_stream(main)
                     with torch.cuda.stream(side):
                         st["q"].copy_(q_host, non_blocking=True)
-                    append_part()
+                    self._append_part(st)
                     main.wait_stream(side)
-                    attend_part(0, half)
+                    self._attend_part(st, 0, half)
                     side.wait_stream(main)
                     with torch.cuda.stream(side):
                         out_host[:half].copy_(st["out"][:half], non_blocking=True)
-                    attend_part(half, self.num_layers)
+                    self._attend_part(st, half, self.num_layers)
                     out_host[half:].copy_(st["out"][half:], non_blocking=True)
                     main.wait_stream(side)
                 st["io_graph"], st["io_key"], st["io_refs"] = graph, key, hosts   # the graph holds raw host pointers
