@@ -1,4 +1,5 @@
-"""ctypes binding of libtq_b200.so (declared in include/tq_b200.h).
+"""Bindings of libtq_b200.so (declared in include/tq_b200.h): ctypes for every entry point, and the extension module
+_tq_host (csrc_host/), which takes torch tensors straight to the entry points of the hot paths.
 
 There is no CPU fallback: importing this module without the built library, or calling a
 compute entry point without a CUDA device, raises.
@@ -6,12 +7,14 @@ compute entry point without a CUDA device, raises.
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import os
 
 import numpy as np
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libtq_b200.so")
+HOST_PATH = os.path.join(_HERE, "_tq_host.so")
 
 F32, F16, F64, BF16 = 0, 1, 2, 3
 ROT_DENSE, ROT_WHT = 0, 1
@@ -116,6 +119,23 @@ def load():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The extension module _tq_host; raises if it has not been built."""
+    global _host
+    if _host is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise ImportError(f"{HOST_PATH} is missing: run `python -m turboquant_plus_b200.build`")
+        import torch  # noqa: F401  (its libraries resolve the module's symbols)
+        from . import _tq_host
+        _tq_host.set_error(TQError)
+        _host = _tq_host
+    return _host
+
+
 def check(rc: int) -> None:
     if rc >= 0:
         return
@@ -154,6 +174,45 @@ def torch_dtype_code(dt):
     return {torch.float32: F32, torch.float16: F16, torch.float64: F64, torch.bfloat16: BF16}[dt]
 
 
+_stamps = itertools.count()
+
+
+class Constants:
+    """A quantizer's host arrays (rotation, codebook, sketch matrix) as attributes, and whether a caller may have changed
+    them since they were uploaded.
+
+    An array the class alone holds cannot change, so a call only compares a stamp; once an attribute has been read from
+    outside, its holder may write into it at any time, and every call compares the contents with what was uploaded.
+    (Copying and comparing 128 KB per call took 15-20 us of every append and attention call.)"""
+
+    def __init__(self, **arrays):
+        self._arrays, self._lent = dict(arrays), False
+        self.stamp = next(_stamps)      # unique: a replaced object never looks like the one before it
+
+    def set(self, name, value):
+        self._arrays[name] = value
+        self.stamp = next(_stamps)
+
+    def lend(self, name):
+        self._lent = True
+        return self._arrays[name]
+
+    def get(self, name):
+        return self._arrays[name]
+
+    def snapshot(self):
+        """What to compare later calls with: (stamp, contents)."""
+        return self.stamp, {k: v.tobytes() for k, v in self._arrays.items()}
+
+    def same(self, snap) -> bool:
+        stamp, contents = snap
+        if not self._lent:
+            return stamp == self.stamp
+        same_bytes = host().same_bytes
+        return all(same_bytes(v, contents[k]) if v.flags.c_contiguous else v.tobytes() == contents[k]
+                   for k, v in self._arrays.items())
+
+
 def _dbl(a):
     return None if a is None else np.ascontiguousarray(a, dtype=np.float64)
 
@@ -179,6 +238,7 @@ class Quantizer:
         with torch.cuda.device(self.device):
             call("tq_quantizer_create", C.byref(desc), C.byref(h))
         self.handle = h
+        self.address = h.value
         self.d, self.bits, self.rotation = d, bits, rotation
 
     def __del__(self):

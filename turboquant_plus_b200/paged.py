@@ -79,6 +79,9 @@ class PagedKVCache:
             return self._placeholder().handle
         return quantizer._native(self.device).handle
 
+    def _address(self, quantizer):
+        return (self._placeholder() if quantizer is None else quantizer._native(self.device)).address
+
     def _placeholder(self):
         """q8_0 tensors need no codebook; the attention entry point still takes the rotation, which for
         q8_0 is the identity."""
@@ -90,21 +93,18 @@ class PagedKVCache:
     def append(self, k, v, slot_mapping):
         """k, v: (n_tokens, num_kv_heads, head_dim) CUDA tensors (fp16, bf16 or fp32);
         slot_mapping: (n_tokens,) int64, page * page_tokens + offset, negative = skip."""
+        kn = self.k_quantizer._native(self.device) if self.k_quantizer is not None else None
+        vn = self.v_quantizer._native(self.device) if self.v_quantizer is not None else None
+        if (kn is None or kn.rotation == nv.ROT_WHT) and (vn is None or vn.rotation == nv.ROT_WHT):
+            nv.host().append(kn and kn.address, vn and vn.address, C.addressof(self.layout), self.pool, k, v, slot_mapping)
+            return
         torch = nv.require_cuda()
         k, v = k.contiguous(), v.contiguous()
         n = k.shape[0]
         assert k.shape == v.shape == (n, self.num_kv_heads, self.head_dim)
         assert k.dtype == v.dtype
         slots = slot_mapping.to(device=self.device, dtype=torch.int64).contiguous()
-        wht_ok = all(q is None or q._native(self.device).rotation == nv.ROT_WHT
-                     for q in (self.k_quantizer, self.v_quantizer))
         with torch.cuda.device(self.device):
-            if wht_ok:
-                nv.call("tq_cache_append", self._handle(self.k_quantizer) if self.k_quantizer else None,
-                        self._handle(self.v_quantizer) if self.v_quantizer else None, C.byref(self.layout),
-                        nv.ptr(self.pool), nv.ptr(k), nv.ptr(v), nv.torch_dtype_code(k.dtype), n, nv.ptr(slots),
-                        nv.stream_ptr())
-                return
             # dense-rotation quantizers: quantize into rows, then scatter the rows into the pages
             for which, (x, quant, fmt) in enumerate(((k, self.k_quantizer, self.k_format),
                                                      (v, self.v_quantizer, self.v_format))):
@@ -122,12 +122,13 @@ class PagedKVCache:
                         nv.ptr(out["scale"]), nv.ptr(qjl), nv.ptr(rscale), n, nv.ptr(slots), nv.stream_ptr())
 
     def workspace(self, batch: int, num_q_heads: int, max_pages: int):
-        torch = nv.require_cuda()
-        need = nv.load().tq_decode_workspace_bytes(batch, num_q_heads, self.num_kv_heads, max_pages)
-        nv.check(int(need))
+        return self._scratch(nv.host().workspace_bytes(batch, num_q_heads, self.num_kv_heads, max_pages, 0))
+
+    def _scratch(self, need: int):
         if self._ws is None or self._ws.numel() < need:
+            torch = nv.require_cuda()
             # zero-filled: the ticket counters at the end of a workspace must start at zero
-            self._ws = torch.zeros((int(need),), dtype=torch.uint8, device=self.device)
+            self._ws = torch.zeros((need,), dtype=torch.uint8, device=self.device)
         return self._ws
 
     def attend(self, q, block_table, seq_lens, scale=None, out=None, workspace=None, phases=7, overlap=False,
@@ -154,28 +155,10 @@ class PagedKVCache:
             phases = int(phases) | nv.DECODE_CHAIN_HEAD
         if sparse_v:  # skip V work where every weight of a 16-token tile is below 1e-6 (the reference's sparse V)
             phases = int(phases) | nv.DECODE_SPARSE_V
-        torch = nv.require_cuda()
-        q = q.contiguous()
-        bsz, hq, d = q.shape
-        assert d == self.head_dim
-        bt = block_table.to(device=self.device, dtype=torch.int32).contiguous()
-        sl = seq_lens.to(device=self.device, dtype=torch.int32).contiguous()
-        ws = self.workspace(bsz, hq, bt.shape[1]) if workspace is None else workspace
-        if out is None:
-            out = torch.empty_like(q)
-        with torch.cuda.device(self.device):
-            if return_lse:
-                lse = torch.empty((bsz, hq), dtype=torch.float32, device=self.device)
-                nv.call("tq_decode_attn_lse", self._handle(self.k_quantizer), self._handle(self.v_quantizer),
-                        C.byref(self.layout), nv.ptr(self.pool), nv.ptr(bt), bt.shape[1], nv.ptr(sl), nv.ptr(q),
-                        nv.torch_dtype_code(q.dtype), bsz, hq, float(scale) if scale else 0.0, nv.ptr(ws), ws.numel(),
-                        nv.ptr(out), nv.torch_dtype_code(out.dtype), int(phases), nv.ptr(lse), nv.stream_ptr())
-                return out, lse
-            nv.call("tq_decode_attn_phases", self._handle(self.k_quantizer), self._handle(self.v_quantizer),
-                    C.byref(self.layout), nv.ptr(self.pool), nv.ptr(bt), bt.shape[1], nv.ptr(sl), nv.ptr(q),
-                    nv.torch_dtype_code(q.dtype), bsz, hq, float(scale) if scale else 0.0, nv.ptr(ws), ws.numel(),
-                    nv.ptr(out), nv.torch_dtype_code(out.dtype), int(phases), nv.stream_ptr())
-        return out
+        ws = self.workspace(q.shape[0], q.shape[1], block_table.shape[1]) if workspace is None else workspace
+        return nv.host().attend(self._address(self.k_quantizer), self._address(self.v_quantizer), C.addressof(self.layout),
+                                self.pool, q, block_table, seq_lens, float(scale) if scale else 0.0, out, ws, int(phases),
+                                return_lse)
 
     def decay_into(self, dst: "PagedKVCache", src_slots, dst_slots):
         """Temporal decay at cache level (benchmarks/temporal_decay_prototype.py:93-125): the K and V codes of the
@@ -200,13 +183,13 @@ class PagedKVCache:
         tensor of a chunk whose K/V rows are already in the cache; kv_lens: (batch,) cached tokens including
         the chunk.  Query i of a sequence sees cached positions 0 .. kv_len - chunk_tokens + i.  turbo2/3/4 K and V
         take the tcgen05 kernel; PROD or q8_0 tensors run the chunk's queries through the decode kernel."""
-        torch = nv.require_cuda()
-        q = q.contiguous()
         bsz, tq, hq, d = q.shape
         assert d == self.head_dim
-        bt = block_table.to(device=self.device, dtype=torch.int32).contiguous()
-        kl = kv_lens.to(device=self.device, dtype=torch.int32).contiguous()
         if not (self.k_format.startswith("turbo") and self.v_format.startswith("turbo")):
+            torch = nv.require_cuda()
+            q = q.contiguous()
+            bt = block_table.to(device=self.device, dtype=torch.int32).contiguous()
+            kl = kv_lens.to(device=self.device, dtype=torch.int32).contiguous()
             # PROD and q8_0 tensors have no tensor-memory pipeline: every query of the chunk runs as a row of the decode
             # kernel with its own causal length (the cache is read once per query; the pages of a sequence stay in L2)
             lens = (kl[:, None] - tq + 1 + torch.arange(tq, device=self.device, dtype=torch.int32)[None, :]).clamp_(min=0)
@@ -216,22 +199,11 @@ class PagedKVCache:
                 out.copy_(res)
                 return out
             return res
-        if workspace is None:
-            need = int(nv.load().tq_prefill_workspace_bytes(bsz, tq, hq, self.num_kv_heads, bt.shape[1]))
-            nv.check(need)
-            if self._ws is None or self._ws.numel() < need:
-                self._ws = torch.zeros((need,), dtype=torch.uint8, device=self.device)
-            ws = self._ws
-        else:
-            ws = workspace
-        if out is None:
-            out = torch.empty_like(q)
-        with torch.cuda.device(self.device):
-            nv.call("tq_prefill_attn", self._handle(self.k_quantizer), self._handle(self.v_quantizer),
-                    C.byref(self.layout), nv.ptr(self.pool), nv.ptr(bt), bt.shape[1], nv.ptr(kl), nv.ptr(q),
-                    nv.torch_dtype_code(q.dtype), bsz, tq, hq, float(scale) if scale else 0.0, nv.ptr(ws), ws.numel(),
-                    nv.ptr(out), nv.torch_dtype_code(out.dtype), nv.stream_ptr())
-        return out
+        ws = workspace
+        if ws is None:
+            ws = self._scratch(nv.host().workspace_bytes(bsz, hq, self.num_kv_heads, block_table.shape[1], tq))
+        return nv.host().prefill(self._address(self.k_quantizer), self._address(self.v_quantizer), C.addressof(self.layout),
+                                 self.pool, q, block_table, kv_lens, float(scale) if scale else 0.0, out, ws)
 
     # ---- wire / on-disk forms ---------------------------------------------------------------------------
     def block_bytes(self, which: str, block_elems: int = 128) -> int:

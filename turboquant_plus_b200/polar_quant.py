@@ -40,8 +40,8 @@ class PolarQuant:
         rng = np.random.default_rng(seed)
         if rotation == "dense":
             self.signs = None
-            self.rotation = (np.asarray(rotation_matrix, dtype=np.float64) if rotation_matrix is not None
-                             else random_rotation_dense(d, rng))
+            matrix = (np.asarray(rotation_matrix, dtype=np.float64) if rotation_matrix is not None
+                      else random_rotation_dense(d, rng))
         else:
             if signs is None:
                 s1, s2, padded = random_rotation_fast(d, rng)
@@ -49,32 +49,49 @@ class PolarQuant:
                     raise ValueError(f"rotation='wht' needs d to be a power of two (kernels: d == 128), got {d}")
                 signs = (s1, s2)
             self.signs = (np.asarray(signs[0], dtype=np.float64), np.asarray(signs[1], dtype=np.float64))
-            self.rotation = fast_rotation_matrix(*self.signs)
-        self.centroids = (np.asarray(centroids, dtype=np.float64) if centroids is not None
-                          else optimal_centroids(bit_width, d))
+            matrix = fast_rotation_matrix(*self.signs)
+        self._const = nv.Constants(rotation=matrix, centroids=(np.asarray(centroids, dtype=np.float64)
+                                                               if centroids is not None else optimal_centroids(bit_width, d)))
+        if rotation_matrix is not None or centroids is not None:
+            self._const.lend("rotation")        # the caller's own arrays
         self._handles = {}
         self._uploaded = None
 
-    # ---- native handle ------------------------------------------------------------------
-    def _snapshot(self):
-        return (self.rotation.tobytes(), self.centroids.tobytes(), bool(self.norm_correction))
+    @property
+    def rotation(self):
+        return self._const.lend("rotation")
 
+    @rotation.setter
+    def rotation(self, value):
+        self._const.set("rotation", value)
+
+    @property
+    def centroids(self):
+        return self._const.lend("centroids")
+
+    @centroids.setter
+    def centroids(self, value):
+        self._const.set("centroids", value)
+
+    # ---- native handle ------------------------------------------------------------------
     def _native(self, device):
-        """The tq_quantizer for ``device``; rebuilt if rotation / centroids were reassigned."""
-        snap = self._snapshot()
-        if snap != self._uploaded:
+        """The tq_quantizer for ``device``; rebuilt if rotation / centroids were reassigned or written to."""
+        up = self._uploaded
+        if up is None or up[0] != bool(self.norm_correction) or not self._const.same(up[1]):
             self._handles.clear()
-            self._uploaded = snap
-        key = str(device)
-        if key not in self._handles:
+            self._uploaded = (bool(self.norm_correction), self._const.snapshot())
+        q = self._handles.get(device)
+        if q is None:
+            rotation, centroids = self._const.get("rotation"), self._const.get("centroids")
             if self.rotation_kind == "wht" and self.signs is not None and np.array_equal(
-                    self.rotation, fast_rotation_matrix(*self.signs)):
-                self._handles[key] = nv.Quantizer(self.d, self.bit_width, nv.ROT_WHT, self.norm_correction,
-                                                  self.centroids, signs=self.signs, device=device)
+                    rotation, fast_rotation_matrix(*self.signs)):
+                q = nv.Quantizer(self.d, self.bit_width, nv.ROT_WHT, self.norm_correction, centroids,
+                                 signs=self.signs, device=device)
             else:
-                self._handles[key] = nv.Quantizer(self.d, self.bit_width, nv.ROT_DENSE, self.norm_correction,
-                                                  self.centroids, rot=self.rotation, device=device)
-        return self._handles[key]
+                q = nv.Quantizer(self.d, self.bit_width, nv.ROT_DENSE, self.norm_correction, centroids,
+                                 rot=rotation, device=device)
+            self._handles[device] = q
+        return q
 
     @property
     def _is_wht(self):
@@ -84,34 +101,21 @@ class PolarQuant:
     def quantize_device(self, xt, *, packed=False, want_scale=False):
         """xt: (n, d) CUDA tensor.  Returns dict with 'idx' (n, d) uint8 or 'packed'
         (n, d*bits/8) uint8, 'norm' (n,) fp32 and optionally 'scale' (n,) fp32."""
-        torch = nv.require_cuda()
-        n = xt.shape[0]
-        q = self._native(xt.device)
-        out = {"norm": torch.empty((n,), dtype=torch.float32, device=xt.device)}
-        if packed:
-            out["packed"] = torch.empty((n, self.d * self.bit_width // 8), dtype=torch.uint8, device=xt.device)
-        else:
-            out["idx"] = torch.empty((n, self.d), dtype=torch.uint8, device=xt.device)
+        codes, norm, scale, _, _ = nv.host().quantize(self._native(xt.device).address, xt, self.bit_width, packed,
+                                                      want_scale, False)
+        out = {"norm": norm, "packed" if packed else "idx": codes}
         if want_scale:
-            out["scale"] = torch.empty((n,), dtype=torch.float32, device=xt.device)
-        with torch.cuda.device(xt.device):
-            nv.call("tq_quantize", q.handle, nv.ptr(xt), nv.torch_dtype_code(xt.dtype), xt.stride(0), n,
-                    nv.ptr(out.get("packed")), nv.ptr(out.get("idx")), nv.ptr(out["norm"]), nv.ptr(out.get("scale")),
-                    None, None, nv.stream_ptr())
+            out["scale"] = scale
         return out
 
     def dequantize_device(self, norms, *, idx=None, packed=None, out_dtype=None):
         torch = nv.require_cuda()
         src = idx if idx is not None else packed
-        n = src.shape[0]
         q = self._native(src.device)
         if out_dtype is None:
             out_dtype = torch.float32 if q.rotation == nv.ROT_WHT else torch.float64
-        out = torch.empty((n, self.d), dtype=out_dtype, device=src.device)
-        with torch.cuda.device(src.device):
-            nv.call("tq_dequantize", q.handle, nv.ptr(packed), nv.ptr(idx), nv.ptr(norms), None, None, 1.0, n,
-                    nv.ptr(out), nv.torch_dtype_code(out_dtype), nv.stream_ptr())
-        return out
+        return nv.host().dequantize(q.address, src, idx is None, norms, None, None, 1.0, self.d,
+                                    nv.torch_dtype_code(out_dtype))
 
     # ---- reference-shaped API -----------------------------------------------------------------
     def quantize(self, x):

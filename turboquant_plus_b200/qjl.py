@@ -26,35 +26,45 @@ class QJL:
         rng = np.random.default_rng(seed)
         self.signs = None
         if matrix is not None:
-            self.S = np.asarray(matrix, dtype=np.float64)
+            s = np.asarray(matrix, dtype=np.float64)
         elif kind == "dense":
             gauss = rng.standard_normal((d, d))
             q, r = np.linalg.qr(gauss)
-            self.S = q * np.sign(np.diagonal(r))[np.newaxis, :]
+            s = q * np.sign(np.diagonal(r))[np.newaxis, :]
         elif kind == "wht":
             s1, s2, padded = random_rotation_fast(d, rng)
             if padded != d:
                 raise ValueError(f"kind='wht' needs d to be a power of two, got {d}")
             self.signs = (s1, s2)
-            self.S = fast_rotation_matrix(s1, s2)
+            s = fast_rotation_matrix(s1, s2)
         else:
             raise ValueError(f"kind must be 'dense' or 'wht', got {kind!r}")
-        defect = np.linalg.norm(self.S @ self.S.T - np.eye(d), "fro")
+        defect = np.linalg.norm(s @ s.T - np.eye(d), "fro")
         assert defect < self._ORTHO_TOL, (
             f"QJL projection matrix not orthogonal: ||S S^T - I||_F = {defect:.2e} (tolerance {self._ORTHO_TOL:.0e})")
+        self._const = nv.Constants(S=s)
+        if matrix is not None:
+            self._const.lend("S")               # the caller's own array
         self._handles = {}
         self._uploaded = None
 
+    @property
+    def S(self):
+        return self._const.lend("S")
+
+    @S.setter
+    def S(self, value):
+        self._const.set("S", value)
+
     def _native(self, device):
-        snap = self.S.tobytes()
-        if snap != self._uploaded:
+        if self._uploaded is None or not self._const.same(self._uploaded):
             self._handles.clear()
-            self._uploaded = snap
-        key = str(device)
-        if key not in self._handles:
-            self._handles[key] = nv.Quantizer(self.d, 1, nv.ROT_DENSE, True, np.array([-1.0, 1.0]), qjl_s=self.S,
-                                              device=device)
-        return self._handles[key]
+            self._uploaded = self._const.snapshot()
+        q = self._handles.get(device)
+        if q is None:
+            q = self._handles[device] = nv.Quantizer(self.d, 1, nv.ROT_DENSE, True, np.array([-1.0, 1.0]),
+                                                     qjl_s=self._const.get("S"), device=device)
+        return q
 
     def quantize(self, r):
         """(signs int8 in {+1,-1}, ||r||); zeros of the projection count as +1 (turboquant/qjl.py:72-94)."""

@@ -48,60 +48,46 @@ class TurboQuant:
 
     def _native(self, device):
         pq, qj = self.polar_quant, self.qjl
-        snap = (pq.rotation.tobytes(), pq.centroids.tobytes(), bool(pq.norm_correction), qj.S.tobytes())
-        if snap != self._uploaded:
+        up = self._uploaded
+        if (up is None or up[0] != bool(pq.norm_correction) or not pq._const.same(up[1]) or not qj._const.same(up[2])):
             self._handles.clear()
-            self._uploaded = snap
-        key = str(device)
-        if key not in self._handles:
+            self._uploaded = (bool(pq.norm_correction), pq._const.snapshot(), qj._const.snapshot())
+        q = self._handles.get(device)
+        if q is None:
+            rotation, centroids, sketch = pq._const.get("rotation"), pq._const.get("centroids"), qj._const.get("S")
             wht = (self.rotation_kind == "wht" and pq.signs is not None and qj.signs is not None
-                   and np.array_equal(pq.rotation, fast_rotation_matrix(*pq.signs))
-                   and np.array_equal(qj.S, fast_rotation_matrix(*qj.signs)))
+                   and np.array_equal(rotation, fast_rotation_matrix(*pq.signs))
+                   and np.array_equal(sketch, fast_rotation_matrix(*qj.signs)))
             if wht:
-                self._handles[key] = nv.Quantizer(self.d, pq.bit_width, nv.ROT_WHT, pq.norm_correction, pq.centroids,
-                                                  signs=pq.signs, qjl_signs=qj.signs, device=device)
+                q = nv.Quantizer(self.d, pq.bit_width, nv.ROT_WHT, pq.norm_correction, centroids, signs=pq.signs,
+                                 qjl_signs=qj.signs, device=device)
             else:
-                self._handles[key] = nv.Quantizer(self.d, pq.bit_width, nv.ROT_DENSE, pq.norm_correction, pq.centroids,
-                                                  rot=pq.rotation, qjl_s=qj.S, device=device)
-        return self._handles[key]
+                q = nv.Quantizer(self.d, pq.bit_width, nv.ROT_DENSE, pq.norm_correction, centroids, rot=rotation,
+                                 qjl_s=sketch, device=device)
+            self._handles[device] = q
+        return q
 
     # ---- device-level API ---------------------------------------------------------------
     def quantize_device(self, xt, *, packed=False, want_scale=False):
         """(n, d) CUDA tensor -> dict of CUDA tensors: 'idx' or 'packed', 'norm', 'qjl' (n, d/8) packed
         sign bits, 'rnorm', optionally 'scale'."""
-        torch = nv.require_cuda()
-        n = xt.shape[0]
-        q = self._native(xt.device)
-        bits = self.polar_quant.bit_width
-        out = {"norm": torch.empty((n,), dtype=torch.float32, device=xt.device),
-               "rnorm": torch.empty((n,), dtype=torch.float32, device=xt.device),
-               "qjl": torch.empty((n, (self.d + 7) // 8), dtype=torch.uint8, device=xt.device)}
-        if packed:
-            out["packed"] = torch.empty((n, self.d * bits // 8), dtype=torch.uint8, device=xt.device)
-        else:
-            out["idx"] = torch.empty((n, self.d), dtype=torch.uint8, device=xt.device)
+        codes, norm, scale, qjl, rnorm = nv.host().quantize(self._native(xt.device).address, xt, self.polar_quant.bit_width,
+                                                            packed, want_scale, True)
+        out = {"norm": norm, "rnorm": rnorm, "qjl": qjl, "packed" if packed else "idx": codes}
         if want_scale:
-            out["scale"] = torch.empty((n,), dtype=torch.float32, device=xt.device)
-        with torch.cuda.device(xt.device):
-            nv.call("tq_quantize", q.handle, nv.ptr(xt), nv.torch_dtype_code(xt.dtype), xt.stride(0), n,
-                    nv.ptr(out.get("packed")), nv.ptr(out.get("idx")), nv.ptr(out["norm"]), nv.ptr(out.get("scale")),
-                    nv.ptr(out["qjl"]), nv.ptr(out["rnorm"]), nv.stream_ptr())
+            out["scale"] = scale
         return out
 
     # ---- reference-shaped API -----------------------------------------------------------------
     def quantize(self, x) -> CompressedVector:
         """turboquant/turboquant.py:79-100."""
-        torch = nv.require_cuda()
         xt, was_numpy, src_dtype = to_device(x, self.device, allow_f64=self.rotation_kind != "wht")
         single = xt.dim() == 1
         xt = xt.reshape(1, -1) if single else xt.reshape(-1, xt.shape[-1])
         if xt.shape[1] != self.d:
             raise ValueError(f"expected vectors of dimension {self.d}, got {xt.shape[1]}")
         out = self.quantize_device(xt)
-        n = xt.shape[0]
-        signs = torch.empty((n, self.d), dtype=torch.int8, device=xt.device)
-        with torch.cuda.device(xt.device):
-            nv.call("tq_unpack_bits", nv.ptr(out["qjl"]), n, self.d, nv.ptr(signs), nv.stream_ptr())
+        signs = nv.host().sign_bits(out["qjl"], self.d, False)
         idx, nrm, rn = out["idx"], out["norm"], out["rnorm"]
         if was_numpy:
             idx = idx.cpu().numpy().astype(np.int64)
@@ -126,15 +112,10 @@ class TurboQuant:
         as_flat = (lambda a: np.asarray(a).reshape(-1)) if was_numpy else (lambda a: a.reshape(-1))
         nt = floats_to_device(as_flat(compressed.vector_norms), dev)
         rt = floats_to_device(as_flat(compressed.residual_norms), dev)
-        n = it.shape[0]
         q = self._native(dev)
         out_dtype = torch.float32 if q.rotation == nv.ROT_WHT else torch.float64
-        bits = torch.empty((n, (self.d + 7) // 8), dtype=torch.uint8, device=dev)
-        out = torch.empty((n, self.d), dtype=out_dtype, device=dev)
-        with torch.cuda.device(dev):
-            nv.call("tq_pack_bits", nv.ptr(st), n, self.d, nv.ptr(bits), nv.stream_ptr())
-            nv.call("tq_dequantize", q.handle, None, nv.ptr(it), nv.ptr(nt), nv.ptr(bits), nv.ptr(rt),
-                    float(shrinkage), n, nv.ptr(out), nv.torch_dtype_code(out_dtype), nv.stream_ptr())
+        bits = nv.host().sign_bits(st, self.d, True)
+        out = nv.host().dequantize(q.address, it, False, nt, bits, rt, float(shrinkage), self.d, nv.torch_dtype_code(out_dtype))
         if was_numpy:
             out = out.cpu().numpy().astype(np.float64)
         return out[0] if single else out
