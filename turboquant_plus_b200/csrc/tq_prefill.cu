@@ -157,6 +157,7 @@ struct PrefillParams {
   const int32_t* kv_lens;   // cached tokens per sequence, the chunk's own tokens included
   const void* q;            // [B][Tq][Hq][128]
   void* out;                // same shape
+  const float* k_s_t;       // dense sketch matrix transposed (PROD keys of a dense quantizer), or nullptr
   const float* k_rot_t;     // dense K rotation transposed (R x)_j = sum_k rot_t[k][j] x_k, or nullptr
   const float* v_rot;       // dense V rotation row-major (R^T y)_j = sum_k rot[k][j] y_k, or nullptr
   int32_t* status;
@@ -171,8 +172,22 @@ struct PrefillParams {
   tq_cache_layout L;
 };
 
+// KK / VK: 2,3,4 = turbo bits; 8 = q8_0; 18,19,20 = PROD with 1,2,3 PolarQuant bits + sign sketch (keys only).
+template <int KIND> struct PfKind {
+  static constexpr bool Q8 = KIND == 8, PROD = KIND >= 18;
+  static constexpr int BITS = Q8 ? 0 : (PROD ? KIND - 17 : KIND);
+  // K operand tiles of a page.  turbo: centroids (the row scale is applied to the scores in fp32).  q8_0: int8 x block
+  // scale is 19 bits, so its fp16 rounding and the rest, exactly.  PROD: centroids, then +-ratio for the sketch, ratio =
+  // residual scale / row scale (one row scale then serves both parts), as its fp16 rounding and the rest of it.
+  static constexpr int TILES = PROD ? 3 : (Q8 ? 2 : 1);
+  // more than one tile per page: one buffer of them instead of two
+  static constexpr int KBUF = TILES == 1 ? 2 : 1;
+  // PROD queries (rotated and projected, hi and lo) take 256 tensor-memory columns: one score buffer instead of two
+  static constexpr int SBUF = PROD ? 1 : 2;
+};
+
 template <int BITS> struct PfLut {
-  static constexpr int ENTRIES = 1 << (2 * BITS);
+  static constexpr int ENTRIES = BITS ? 1 << (2 * BITS) : 0;
   static constexpr bool REPL = ENTRIES <= 64;
   static constexpr int SHIFT = REPL ? 7 : 2;
   static constexpr int BYTES = ENTRIES << SHIFT;
@@ -217,6 +232,67 @@ __device__ __forceinline__ void pf_dequant_token(const uint8_t* src, uint8_t* ds
 }
 
 
+__device__ __forceinline__ uint32_t pf_s8x2(uint32_t biased, uint32_t sel) {
+  // two int8 values, stored as value ^ 0x80 = value + 128, as exact fp16: (b | 0x6400) is 1024 + b; subtract 1152
+  uint32_t d;
+  asm("sub.f16x2 %0, %1, %2;" : "=r"(d) : "r"(__byte_perm(biased, 0x64646464u, sel)), "r"(0x64806480u));
+  return d;
+}
+
+// One token's 128 int8 values at `src` with its four block scales (sc01, sc23: two fp16 each) -> fp16 products in the
+// operand tile at `dst`, and, SPLIT, what the fp16 rounding left of them (exact: 8 x 11 bits) in the tile at dst + 32 KB.
+// Rows are 128 bytes apart, so a lane starts at a chunk of its own: the lanes of a load then touch every bank.
+template <bool SPLIT>
+__device__ __forceinline__ void pf_q8_token(const uint8_t* src, uint8_t* dst, uint32_t sc01, uint32_t sc23, int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int c = (i + lane) & 7;   // 16 values: dims 16 c .. 16 c + 15, half of block c >> 1
+    const uint4 v = *reinterpret_cast<const uint4*>(src + 16 * c);
+    const uint32_t w[4] = {v.x ^ 0x80808080u, v.y ^ 0x80808080u, v.z ^ 0x80808080u, v.w ^ 0x80808080u};
+    const uint32_t s2 = __byte_perm(c & 4 ? sc23 : sc01, 0, c & 2 ? 0x3232 : 0x1010);
+    uint32_t hi[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t x = pf_s8x2(w[j >> 1], (j & 1) ? 0x4342 : 0x4140);
+      asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(hi[j]) : "r"(x), "r"(s2));
+      if constexpr (SPLIT) asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(lo[j]) : "r"(x), "r"(s2), "r"(hi[j] ^ 0x80008000u));
+    }
+    uint8_t* d = dst + c * 256;
+    *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(d + 128) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+    if constexpr (SPLIT) {
+      *reinterpret_cast<uint4*>(d + 32768) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      *reinterpret_cast<uint4*>(d + 32768 + 128) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+    }
+  }
+}
+
+// One token's 16-byte sign sketch (first dim in the most significant bit, set = +1) -> +-ratio in the tile at `dst`, as
+// the fp16 rounding of the ratio there and the rest of it in the tile behind.
+__device__ __forceinline__ void pf_sketch_token(uint4 z, uint8_t* dst, float ratio) {
+  const __half h = __float2half_rn(ratio);
+  const __half2 h2 = __half2half2(h), e2 = __float2half2_rn(ratio - __half2float(h));
+  const uint32_t hw = *reinterpret_cast<const uint32_t*>(&h2), ew = *reinterpret_cast<const uint32_t*>(&e2);
+  const uint32_t zw[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t n = ~__byte_perm(zw[k], 0, 0x0123);   // set = negative; dim 32 k + i in bit 31 - i
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t m[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {   // dims 2 j, 2 j + 1 of the word: bits 31 - 2 j and 30 - 2 j -> the two sign positions
+        const int j = 4 * c + p;
+        const uint32_t lo = j < 8 ? n >> (16 - 2 * j) : n << (2 * j - 16);
+        m[p] = (lo & 0x8000u) | ((n << (2 * j + 1)) & 0x80000000u);
+      }
+      uint8_t* d = dst + (4 * k + c) * 128;
+      *reinterpret_cast<uint4*>(d) = make_uint4(hw ^ m[0], hw ^ m[1], hw ^ m[2], hw ^ m[3]);
+      *reinterpret_cast<uint4*>(d + 32768) = make_uint4(ew ^ m[0], ew ^ m[1], ew ^ m[2], ew ^ m[3]);
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // k_prefill_attn2: the work split over specialised warps (one CTA per SM, 544 threads):
 //   warps 0-7  rows: two threads per row r = lane r of tensor memory (warps w and w + 4 reach the same 32 lanes), one
@@ -236,7 +312,10 @@ __device__ __forceinline__ void pf_dequant_token(const uint8_t* src, uint8_t* ds
 // fp32 arithmetic, polling loops -- and into the K producers waiting for the product of page i - 2 when the score MMA
 // was all they needed.  Now ~3,300 cycles, against 1,536 of tensor work; the shared-memory pipe is the next limit.)
 // Tensor memory, all 512 columns: Q hi 0-63 | Q lo 64-127 | S0 128-255 | S1 256-383 | O 384-511 (fp32, accumulated
-// by the MMAs across pages).  P overlays the first 64 columns of its S buffer.  Hand-offs are mbarriers (counts in
+// by the MMAs across pages); PROD keys: the projected queries' hi and lo in 128-255 and one score buffer in 256-383.
+// q8_0 and PROD keys have two and three K tiles per page (PfKind), one buffer of them, and sum 3 and 5 products into S:
+// their queries' chunk runs here instead of one decode call per query, which read and dequantized the cache once per
+// query (2 x 128 queries x 32 heads over 8,192 tokens of q8_0 / turbo2: 650 us).  P overlays the first 64 columns of its S buffer.  Hand-offs are mbarriers (counts in
 // brackets): k_ready/v_ready [128 producer arrivals], s_full/o_done [tcgen05.commit], p_ready [128 row arrivals];
 // buffer b of page i completes each of them for the (i >> 1)-th time, which fixes the parity to wait for.  Every
 // wait is bounded; a role that gives up raises the CTA's fail flag, the others see it or run out of time
@@ -245,7 +324,7 @@ __device__ __forceinline__ void pf_dequant_token(const uint8_t* src, uint8_t* ds
 constexpr int PF2_THREADS = 544;
 constexpr float PF2_SLACK = 4.0f;
 
-template <int KB, int VB> struct PfSmem2 {
+template <int KK, int VK> struct PfSmem2 {
   static constexpr int ALIGN = 8192;                    // each table starts on a multiple of its size (at most 8 KB)
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = 8192;
@@ -253,8 +332,8 @@ template <int KB, int VB> struct PfSmem2 {
   static constexpr int OFF_SC = OFF_BAR + 256;          // float K scales[4 slots][128 tokens], then the row halves'
                                                         // exchange area float[2 buffers][2 halves][128 rows], then
                                                         // their parts of the row sum float[2 halves][128 rows]
-  static constexpr int OFF_KT = OFF_SC + 5120;          // K operand tiles, 2 x 32 KB
-  static constexpr int OFF_VT = OFF_KT + 65536;         // V operand tiles
+  static constexpr int OFF_KT = OFF_SC + 5120;          // K operand tiles, 32 KB each
+  static constexpr int OFF_VT = OFF_KT + PfKind<KK>::KBUF * PfKind<KK>::TILES * 32768;   // V operand tiles, two
   static constexpr int OFF_ST = OFF_VT + 65536;         // two page records
   static size_t bytes(int record_bytes) { return (size_t)ALIGN + OFF_ST + 2 * (size_t)record_bytes; }
 };
@@ -282,9 +361,12 @@ __device__ __forceinline__ bool producers_all(bool ok) {
   return r != 0;
 }
 
-template <int KB, int VB>
+template <int KK, int VK>
 __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillParams P, const TqFast fk, const TqFast fv) {
-  using SP = PfSmem2<KB, VB>;
+  using SP = PfSmem2<KK, VK>;
+  using KT = PfKind<KK>;
+  using VT = PfKind<VK>;
+  constexpr int KB = KT::BITS, VB = VT::BITS;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int rb = blockIdx.x / P.num_splits, split = blockIdx.x - rb * P.num_splits, kvh = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -351,7 +433,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
   }
   if (!is_prim) {
     // table fill by the 416 threads that do not rotate a query
-    for (int i = tid - 128; i < PfLut<KB>::BYTES / 16; i += PF2_THREADS - 128) {
+    for (int i = tid - 128; KB && i < PfLut<KB>::BYTES / 16; i += PF2_THREADS - 128) {
       if (PfLut<KB>::REPL) {
         const int e = i >> 3;
         const uint32_t v = (uint32_t)fk.cent16[e >> KB] | ((uint32_t)fk.cent16[e & ((1 << KB) - 1)] << 16);
@@ -366,7 +448,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
         reinterpret_cast<uint4*>(sm + SP::OFF_K)[i] = make_uint4(v[0], v[1], v[2], v[3]);
       }
     }
-    for (int i = tid - 128; i < PfLut<VB>::BYTES / 16; i += PF2_THREADS - 128) {
+    for (int i = tid - 128; VB && i < PfLut<VB>::BYTES / 16; i += PF2_THREADS - 128) {
       if (PfLut<VB>::REPL) {
         const int e = i >> 3;
         const uint32_t v = (uint32_t)fv.cent16[e >> VB] | ((uint32_t)fv.cent16[e & ((1 << VB) - 1)] << 16);
@@ -383,54 +465,46 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
     }
   }
 
-  // ---- prologue (row warps): this row's query, rotated by the K rotation, scaled, fp16 hi + lo into tensor memory;
-  // each of the row's two threads holds one half of its elements ----
+  if constexpr (KT::PROD) {   // both transforms of a row share registers and staging: the first goes to tensor memory first
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  }
+  // ---- prologue (row warps): this row's query, rotated by the K rotation (q8_0 keys: as it is), scaled, fp16 hi + lo
+  // into tensor memory; PROD keys: its projection by the sketch's transform as well.  Each of the row's two threads holds
+  // one half of its elements ----
   float o[PF_HALF];
-  if (is_row) {
-    // The rows come in through shared memory: read directly, a thread's own half row would put the lanes of a load
-    // 256 or 512 bytes apart (one line per lane and instruction); staged, a warp reads whole rows.  Row stride: the
-    // row plus 16 bytes, so that the 16-byte accesses of consecutive rows fall into different banks.
-    {
-      const int esz = P.q_dtype == TQ_F32 ? 4 : 2;
-      const int cpr = TQ_D * esz / 16, stride = TQ_D * esz + 16;   // 16-byte chunks per row
-      uint8_t* stg = ktile;                                        // the operand tiles are not in use yet
-#pragma unroll 8
-      for (int it = 0; it < cpr / 2; ++it) {
-        const int c = it * 256 + tid, r = c / cpr, w = c - r * cpr;
-        const int grow = rb * PF_ROWS + r;
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (grow < nrows) {
-          const int gq = grow / P.group, gh = grow - gq * P.group;
-          const size_t off = ((((size_t)b * P.tq + gq) * P.hq + (size_t)kvh * P.group + gh) * TQ_D) * esz + w * 16;
-          val = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(P.q) + off);
-        }
-        *reinterpret_cast<uint4*>(stg + r * stride + w * 16) = val;
+  const uint32_t TQc = 0, TQLc = 64, TPc = 128, TPLc = 192, TOc = 384;
+  // score buffer of page i; P overlays its first 64 columns
+  auto s_col = [](int bf) { return KT::SBUF == 2 ? 128u + 128u * bf : 256u; };
+  uint8_t* stg = ktile + (KT::PROD ? 65536 : 0);                   // the operand tiles are not in use yet
+  const int q_esz = P.q_dtype == TQ_F32 ? 4 : 2;
+  const int q_stride = TQ_D * q_esz + 16;
+  auto read_row = [&]() {
+    const uint8_t* mine = stg + rtid * q_stride + hf * PF_HALF * q_esz;
+    if (P.q_dtype == TQ_F32) {
+#pragma unroll
+      for (int e = 0; e < PF_HALF; e += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(mine + e * 4);
+        o[e] = v.x; o[e + 1] = v.y; o[e + 2] = v.z; o[e + 3] = v.w;
       }
-      rows_sync();
-      const uint8_t* mine = stg + rtid * stride + hf * PF_HALF * esz;
-      if (P.q_dtype == TQ_F32) {
+    } else {
 #pragma unroll
-        for (int e = 0; e < PF_HALF; e += 4) {
-          const float4 v = *reinterpret_cast<const float4*>(mine + e * 4);
-          o[e] = v.x; o[e + 1] = v.y; o[e + 2] = v.z; o[e + 3] = v.w;
-        }
-      } else {
+      for (int e = 0; e < PF_HALF; e += 8) {
+        const uint4 w4 = *reinterpret_cast<const uint4*>(mine + e * 2);
+        const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-        for (int e = 0; e < PF_HALF; e += 8) {
-          const uint4 w4 = *reinterpret_cast<const uint4*>(mine + e * 2);
-          const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float2 f = P.q_dtype == TQ_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&ww[k]))
-                                                 : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ww[k]));
-            o[e + 2 * k] = f.x; o[e + 2 * k + 1] = f.y;
-          }
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = P.q_dtype == TQ_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&ww[k]))
+                                               : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ww[k]));
+          o[e + 2 * k] = f.x; o[e + 2 * k + 1] = f.y;
         }
       }
-      rows_sync();   // the staged rows are read: the exchange area of the rotation below is the same memory
     }
-    float* xs = reinterpret_cast<float*>(ktile);  // [k][row], 64 KB: the operand tiles are not in use yet
-    if (P.k_rot_t) {
+  };
+  auto rotate = [&](const float* dense_t, const uint32_t (&pre)[4], const uint32_t (&post)[4]) {
+    float* xs = reinterpret_cast<float*>(ktile);  // [k][row], 64 KB
+    if (dense_t) {
       // dense rotation: the rows staged transposed, then this thread's 64 elements of y = R x
 #pragma unroll
       for (int k = 0; k < PF_HALF; ++k) xs[(PF_HALF * hf + k) * PF_ROWS + rtid] = o[k];
@@ -439,7 +513,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
       for (int j = 0; j < PF_HALF; ++j) o[j] = 0.f;
       for (int k = 0; k < TQ_D; ++k) {
         const float xv = xs[k * PF_ROWS + rtid];
-        const float4* rr = reinterpret_cast<const float4*>(P.k_rot_t + (size_t)k * TQ_D + PF_HALF * hf);
+        const float4* rr = reinterpret_cast<const float4*>(dense_t + (size_t)k * TQ_D + PF_HALF * hf);
 #pragma unroll
         for (int j = 0; j < PF_HALF; j += 4) {
           const float4 r4 = __ldg(rr + (j >> 2));
@@ -448,38 +522,67 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
         }
       }
     } else {
-      row_wht128_pair(o, fk.s1, fk.s2, hf, xs, rtid);
+      row_wht128_pair(o, pre, post, hf, xs, rtid);
+    }
+  };
+  auto to_tmem = [&](uint32_t tmem, float sk, uint32_t hi_col, uint32_t lo_col) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint32_t u[16], ul[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float a = o[32 * c + 2 * j] * sk, bq = o[32 * c + 2 * j + 1] * sk;
+        const __half2 h = __floats2half2_rn(a, bq);
+        const float2 hv = __half22float2(h);
+        u[j] = *reinterpret_cast<const uint32_t*>(&h);
+        ul[j] = pf_pack(a - hv.x, bq - hv.y);
+      }
+      tmem_st16(tmem + hi_col + 32 * hf + 16 * c, u);
+      tmem_st16(tmem + lo_col + 32 * hf + 16 * c, ul);
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  };
+  if (is_row) {
+    // The rows come in through shared memory: read directly, a thread's own half row would put the lanes of a load
+    // 256 or 512 bytes apart (one line per lane and instruction); staged, a warp reads whole rows.  Row stride: the
+    // row plus 16 bytes, so that the 16-byte accesses of consecutive rows fall into different banks.
+    const int cpr = TQ_D * q_esz / 16;   // 16-byte chunks per row
+#pragma unroll 8
+    for (int it = 0; it < cpr / 2; ++it) {
+      const int c = it * 256 + tid, r = c / cpr, w = c - r * cpr;
+      const int grow = rb * PF_ROWS + r;
+      uint4 val = make_uint4(0u, 0u, 0u, 0u);
+      if (grow < nrows) {
+        const int gq = grow / P.group, gh = grow - gq * P.group;
+        const size_t off = ((((size_t)b * P.tq + gq) * P.hq + (size_t)kvh * P.group + gh) * TQ_D) * q_esz + w * 16;
+        val = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(P.q) + off);
+      }
+      *reinterpret_cast<uint4*>(stg + r * q_stride + w * 16) = val;
+    }
+    rows_sync();
+    read_row();
+    if constexpr (!KT::PROD) rows_sync();   // the staged rows are read: the rotation's exchange area is the same memory
+    if constexpr (!KT::Q8) rotate(P.k_rot_t, fk.s1, fk.s2);
+    if constexpr (KT::PROD) {
+      const uint32_t tm0 = *tbase + ((uint32_t)((warp & 3) * 32) << 16);
+      to_tmem(tm0, P.qscale / fk.lut_alpha, TQc, TQLc);
+      rows_sync();                          // the exchange area has been read
+      read_row();
+      rotate(P.k_s_t, fk.j1, fk.j2);
+      to_tmem(tm0, P.qscale, TPc, TPLc);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();  // tensor-memory base, tables and barriers visible; the dense staging area is free again
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tb = *tbase;
-  const uint32_t TQc = 0, TQLc = 64, TSc = 128, TOc = 384;   // S buffer b at TSc + 128 b; P overlays its first 64 columns
 
   if (is_row) {
     // =========================== row warps ===========================
     const uint32_t tm = tb + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 lanes
     float* xch = scales + 512;                                     // [buffer][half][row]
-    {
-      const float sk = P.qscale / fk.lut_alpha;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t u[16], ul[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float a = o[32 * c + 2 * j] * sk, bq = o[32 * c + 2 * j + 1] * sk;
-          const __half2 h = __floats2half2_rn(a, bq);
-          const float2 hv = __half22float2(h);
-          u[j] = *reinterpret_cast<const uint32_t*>(&h);
-          ul[j] = pf_pack(a - hv.x, bq - hv.y);
-        }
-        tmem_st16(tm + TQc + 32 * hf + 16 * c, u);
-        tmem_st16(tm + TQLc + 32 * hf + 16 * c, ul);
-      }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    }
+    if constexpr (!KT::PROD) to_tmem(tm, P.qscale / fk.lut_alpha, TQc, TQLc);
     asm volatile("bar.sync 3, 288;" ::: "memory");   // with the MMA warp: the queries are in tensor memory
 
     float m_run = -INFINITY, l_run = 0.f;   // l_run: this half's part of the row sum
@@ -490,7 +593,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
       if (!pf_wait_warp(&s_full[bf], ph)) { *fail = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float4* ksc4 = reinterpret_cast<const float4*>(scales + (i & 3) * PF_ROWS + 64 * hf);
-      const uint32_t ts = tm + TSc + 128 * bf;
+      const uint32_t ts = tm + s_col(bf);
       const int t0 = (page_lo + i) * PT;
       // a page that every row of this warp sees completely needs no causal mask (rows without a query count as
       // seeing everything: nothing of theirs is stored)
@@ -511,9 +614,13 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
           const uint32_t* v = raw + 16 * c;
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
-            const float4 k4 = ksc4[4 * c + (j >> 2)];
-            float2 x01 = pf_mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), make_float2(k4.x, k4.y));
-            float2 x23 = pf_mul2(make_float2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), make_float2(k4.z, k4.w));
+            float2 x01 = make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+            float2 x23 = make_float2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+            if constexpr (!KT::Q8) {   // (q8_0 operands carry their block scales)
+              const float4 k4 = ksc4[4 * c + (j >> 2)];
+              x01 = pf_mul2(x01, make_float2(k4.x, k4.y));
+              x23 = pf_mul2(x23, make_float2(k4.z, k4.w));
+            }
             if (MASKED) {
               const int tt = t0 + 64 * hf + 16 * c + j;
               x01.x = tt <= pos ? x01.x : -INFINITY;
@@ -677,7 +784,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
             o[j + 2] = fmaf(r4.z, yv, o[j + 2]); o[j + 3] = fmaf(r4.w, yv, o[j + 3]);
           }
         }
-      } else {
+      } else if constexpr (!VT::Q8) {
         row_wht128_pair(o, fv.s2, fv.s1, hf, ys, rtid);  // R^T = D1 (H/sqrt d) D2
       }
       // The rows leave through shared memory like they came in: staged, a warp writes whole rows.
@@ -685,8 +792,8 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
       {
         const int esz = P.out_dtype == TQ_F32 ? 4 : 2;
         const int cpr = TQ_D * esz / 16, stride = TQ_D * esz + 16;
-        uint8_t* stg = ktile;
-        uint8_t* mine = stg + rtid * stride + hf * PF_HALF * esz;
+        uint8_t* ost = ktile;
+        uint8_t* mine = ost + rtid * stride + hf * PF_HALF * esz;
         if (P.out_dtype == TQ_F32) {
 #pragma unroll
           for (int j = 0; j < PF_HALF; j += 4)
@@ -717,7 +824,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
             const int gq = grow / P.group, gh = grow - gq * P.group;
             const size_t off = ((((size_t)b * P.tq + gq) * P.hq + (size_t)kvh * P.group + gh) * TQ_D) * esz + w * 16;
             *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(P.out) + off) =
-                *reinterpret_cast<const uint4*>(stg + r * stride + w * 16);
+                *reinterpret_cast<const uint4*>(ost + r * stride + w * 16);
           }
         }
       }
@@ -731,17 +838,33 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
     const uint32_t lv_base = sptr(sm + SP::OFF_V) + (PfLut<VB>::REPL ? lane * 4 : 0);
     const uint32_t tile_row = (uint32_t)(rtid >> 3) * 2048 + (uint32_t)(rtid & 7) * 16;  // token rtid inside an operand tile
     if (hf == 0) {
-      // K producers.  The K tile of buffer bf is free once S of page i - 2 is complete, and so is the scale slot
-      // i & 3 (the rows finished page i - 4 long before): they run one page ahead of the V producers, whose tile is
-      // free only after the product of page i - 2, and S of the next page is ready before the rows ask for it.
+      // K producers.  The K tiles are free once S of the page that used them before is complete (page i - 2 with two
+      // buffers, i - 1 with one), and so is the scale slot i & 3 (the rows finished page i - 4 long before): they run
+      // one page ahead of the V producers, whose tile is free only after the product of page i - 2, and S of the next
+      // page is ready before the rows ask for it.
       for (int i = 0; i < np; ++i) {
         const int bf = i & 1;
         if (*fail) break;
-        if (i >= 2 && !pf_wait(&s_full[bf], (uint32_t)(((i - 2) >> 1) & 1))) { *fail = 1; break; }
+        if constexpr (KT::KBUF == 2) {
+          if (i >= 2 && !pf_wait(&s_full[bf], (uint32_t)(((i - 2) >> 1) & 1))) { *fail = 1; break; }
+        } else {
+          if (i >= 1 && !pf_wait(&s_full[bf ^ 1], (uint32_t)(((i - 1) >> 1) & 1))) { *fail = 1; break; }
+        }
         if (!pf_wait(&rec_full[bf], (uint32_t)((i >> 1) & 1))) { *fail = 1; break; }
         const uint8_t* st = stage0 + (size_t)bf * rec;
-        pf_dequant_token<KB>(st + P.L.k_idx_off + rtid * (16 * KB), ktile + bf * 32768 + tile_row, lk_base);
-        scales[(i & 3) * PF_ROWS + rtid] = reinterpret_cast<const float*>(st + P.L.k_scale_off)[rtid];
+        uint8_t* dst = ktile + (KT::KBUF == 2 ? bf * 32768 : 0) + tile_row;
+        if constexpr (KT::Q8) {
+          const uint2 sc = *reinterpret_cast<const uint2*>(st + P.L.k_scale_off + rtid * 8);
+          pf_q8_token<true>(st + P.L.k_idx_off + rtid * TQ_D, dst, sc.x, sc.y, lane);
+        } else {
+          pf_dequant_token<KB>(st + P.L.k_idx_off + rtid * (16 * KB), dst, lk_base);
+          const float ks = reinterpret_cast<const float*>(st + P.L.k_scale_off)[rtid];
+          scales[(i & 3) * PF_ROWS + rtid] = ks;
+          if constexpr (KT::PROD) {   // (a zero vector has two zero scales)
+            const float rs = reinterpret_cast<const float*>(st + P.L.k_rscale_off)[rtid];
+            pf_sketch_token(*reinterpret_cast<const uint4*>(st + P.L.k_qjl_off + rtid * 16), dst + 32768, ks != 0.f ? rs / ks : 0.f);
+          }
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         pf_arrive(&k_ready[bf]);   // also: this thread has read its part of the record
       }
@@ -762,10 +885,16 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
         // that the P operand is the bare probability, bounded by 2^(2 PF2_SLACK) whatever the norms of the values
         // are; a token past the end of the sequence may hold anything: its row is zeroed (its P is zero too, but
         // 0 x inf would not be).  Scales beyond the fp16 range saturate.
-        const float vsc = (page_lo + i) * PT + rtid < kv_len ? reinterpret_cast<const float*>(st + P.L.v_scale_off)[rtid] : 0.f;
-        const __half2 s2 = __float2half2_rn(fminf(vsc, 65504.0f));
-        pf_dequant_token<VB, true>(st + P.L.v_idx_off + rtid * (16 * VB), vtile + bf * 32768 + tile_row, lv_base,
-                                   *reinterpret_cast<const uint32_t*>(&s2));
+        const bool exists = (page_lo + i) * PT + rtid < kv_len;
+        uint8_t* dst = vtile + bf * 32768 + tile_row;
+        if constexpr (VT::Q8) {
+          const uint2 sc = exists ? *reinterpret_cast<const uint2*>(st + P.L.v_scale_off + rtid * 8) : make_uint2(0u, 0u);
+          pf_q8_token<false>(st + P.L.v_idx_off + rtid * TQ_D, dst, sc.x, sc.y, lane);
+        } else {
+          const float vsc = exists ? reinterpret_cast<const float*>(st + P.L.v_scale_off)[rtid] : 0.f;
+          const __half2 s2 = __float2half2_rn(fminf(vsc, 65504.0f));
+          pf_dequant_token<VB, true>(st + P.L.v_idx_off + rtid * (16 * VB), dst, lv_base, *reinterpret_cast<const uint32_t*>(&s2));
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         pf_arrive(&v_ready[bf]);
         asm volatile("bar.sync 1, 128;" ::: "memory");   // every V producer has read this record
@@ -784,13 +913,22 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (lane == 0 && np > 0) {
       const uint32_t idesc_s = umma_idesc(128, 128, false), idesc_o = umma_idesc(128, 128, true);
-      auto qk = [&](int i) {   // S_i = Q K_i^T (fp16 hi and lo halves of Q), into S buffer i & 1
+      auto qk = [&](int i) {   // S_i = Q K_i^T (fp16 hi and lo halves of Q), into the score buffer of page i
         const int bf = i & 1;
+        const uint32_t kt = sptr(ktile) + (KT::KBUF == 2 ? bf * 32768 : 0), d = tb + s_col(bf);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t kd = umma_desc(sptr(ktile + bf * 32768) + ks * 256, 128, 2048);
-          umma_ts(tb + TSc + 128 * bf, tb + TQc + ks * 8, kd, idesc_s, ks > 0);
-          umma_ts(tb + TSc + 128 * bf, tb + TQLc + ks * 8, kd, idesc_s, 1);
+          const uint64_t kd = umma_desc(kt + ks * 256, 128, 2048);
+          umma_ts(d, tb + TQc + ks * 8, kd, idesc_s, ks > 0);
+          umma_ts(d, tb + TQLc + ks * 8, kd, idesc_s, 1);
+          if constexpr (KT::TILES > 1) {   // q8_0: what the fp16 products left; PROD: the sketch against the projected query
+            const uint64_t k1 = umma_desc(kt + 32768 + ks * 256, 128, 2048);
+            umma_ts(d, tb + (KT::PROD ? TPc : TQc) + ks * 8, k1, idesc_s, 1);
+            if constexpr (KT::PROD) {
+              umma_ts(d, tb + TPLc + ks * 8, k1, idesc_s, 1);
+              umma_ts(d, tb + TPc + ks * 8, umma_desc(kt + 65536 + ks * 256, 128, 2048), idesc_s, 1);
+            }
+          }
         }
         umma_commit(&s_full[bf]);
       };
@@ -803,7 +941,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
         if (*fail) break;
         const int bf = i & 1;
         const uint32_t ph = (uint32_t)((i >> 1) & 1);
-        if (i + 1 < np) {
+        if (KT::SBUF == 2 && i + 1 < np) {
           if (!pf_wait(&k_ready[(i + 1) & 1], (uint32_t)(((i + 1) >> 1) & 1))) { okay = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           qk(i + 1);
@@ -812,9 +950,15 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)   // O += P_i V_i: P from tensor memory, V tile MN-major, N = 128
-          umma_ts(tb + TOc, tb + TSc + 128 * bf + ks * 8, umma_desc(sptr(vtile + bf * 32768) + ks * 4096, 2048, 128),
+          umma_ts(tb + TOc, tb + s_col(bf) + ks * 8, umma_desc(sptr(vtile + bf * 32768) + ks * 4096, 2048, 128),
                   idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
         umma_commit(&o_done[bf]);
+        if (KT::SBUF == 1 && i + 1 < np) {
+          // one score buffer: the next page's scores follow once this page's product, which reads P out of it, is done
+          if (!pf_wait(&o_done[bf], ph) || !pf_wait(&k_ready[(i + 1) & 1], (uint32_t)(((i + 1) >> 1) & 1))) { okay = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          qk(i + 1);
+        }
       }
       if (!okay) *fail = 1;
     }
@@ -826,21 +970,24 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
 
 }  // namespace
 
-template <int KB, int VB>
+template <int KK, int VK>
 static int launch_prefill(const PrefillParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
-  const size_t need = PfSmem2<KB, VB>::bytes(P.L.record_bytes);
-  constexpr size_t LIMIT = 220 * 1024;  // one CTA per SM (it also takes all 512 tensor-memory columns)
+  const size_t need = PfSmem2<KK, VK>::bytes(P.L.record_bytes);
+  constexpr size_t LIMIT = 227 * 1024;  // one CTA per SM (it also takes all 512 tensor-memory columns)
   TQ_REQUIRE(need <= LIMIT, TQ_ERR_TOO_LARGE, "page record of %d bytes does not fit the prefill pipeline",
              P.L.record_bytes);
+  // (the limit is raised to what the call needs and no further: local memory lives in what is left as L1)
   static thread_local int configured_dev = -1;
+  static thread_local size_t configured = 0;
   int dev = 0;
   TQ_CUDA(cudaGetDevice(&dev));
-  if (configured_dev != dev) {
-    TQ_CUDA(cudaFuncSetAttribute(k_prefill_attn2<KB, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIMIT));
+  if (configured_dev != dev || configured < need) {
+    TQ_CUDA(cudaFuncSetAttribute(k_prefill_attn2<KK, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
     configured_dev = dev;
+    configured = need;
   }
   dim3 grid(P.row_blocks * P.num_splits, P.hkv, P.batch);
-  k_prefill_attn2<KB, VB><<<grid, PF2_THREADS, need, st>>>(P, fk, fv);
+  k_prefill_attn2<KK, VK><<<grid, PF2_THREADS, need, st>>>(P, fk, fv);
   return tq_launch_check("k_prefill_attn2");
 }
 
@@ -891,7 +1038,7 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
                                const int32_t* kv_lens_dev, const void* q_dev, int32_t q_dtype, int32_t batch,
                                int32_t chunk_tokens, int32_t num_q_heads, float scale, void* workspace_dev,
                                int64_t workspace_bytes, void* out_dev, int32_t out_dtype, void* stream) {
-  TQ_REQUIRE(kq && vq && L, TQ_ERR_INVALID, "tq_prefill_attn: quantizers or layout missing");
+  TQ_REQUIRE(L, TQ_ERR_INVALID, "tq_prefill_attn: layout missing");
   TQ_REQUIRE(batch >= 0 && chunk_tokens >= 1 && num_q_heads >= 1 && max_pages_per_seq >= 1, TQ_ERR_INVALID, "bad sizes");
   if (batch == 0) return TQ_OK;
   TQ_REQUIRE(pool_dev && block_table_dev && kv_lens_dev && q_dev && out_dev && workspace_dev, TQ_ERR_INVALID,
@@ -900,11 +1047,13 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
              "workspace must be 256-byte aligned and a multiple of 256 bytes");
   TQ_REQUIRE(L->d == TQ_D && L->page_tokens == 128, TQ_ERR_UNSUPPORTED,
              "prefill attention is built for d == 128 and 128-token pages");
-  TQ_REQUIRE(L->k_format >= TQ_FMT_TURBO2 && L->k_format <= TQ_FMT_TURBO4 && L->v_format >= TQ_FMT_TURBO2 &&
-                 L->v_format <= TQ_FMT_TURBO4,
-             TQ_ERR_UNSUPPORTED, "prefill attention is built for turbo2/3/4 K and V, got %d / %d", L->k_format, L->v_format);
-  TQ_REQUIRE(kq->d == TQ_D && vq->d == TQ_D && kq->bits == L->k_format && vq->bits == L->v_format, TQ_ERR_INVALID,
-             "quantizer bit widths do not match the cache formats");
+  const bool k_q8 = L->k_format == TQ_FMT_Q8_0, v_q8 = L->v_format == TQ_FMT_Q8_0, k_prod = L->k_format >= TQ_FMT_PROD2;
+  TQ_REQUIRE(k_q8 || kq, TQ_ERR_INVALID, "tq_prefill_attn: K quantizer missing");
+  TQ_REQUIRE(v_q8 || vq, TQ_ERR_INVALID, "tq_prefill_attn: V quantizer missing");
+  TQ_REQUIRE((k_q8 || (kq->d == TQ_D && kq->bits == (k_prod ? L->k_format - 17 : L->k_format))) &&
+                 (v_q8 || (vq->d == TQ_D && vq->bits == L->v_format)),
+             TQ_ERR_INVALID, "quantizer bit widths do not match the cache formats");
+  TQ_REQUIRE(!k_prod || kq->qjl, TQ_ERR_INVALID, "PROD cache format needs a K quantizer with a QJL stage");
   TQ_REQUIRE(num_q_heads % L->num_kv_heads == 0, TQ_ERR_INVALID, "num_q_heads must be a multiple of num_kv_heads");
   TQ_REQUIRE(q_dtype == TQ_F16 || q_dtype == TQ_BF16 || q_dtype == TQ_F32, TQ_ERR_UNSUPPORTED, "bad query dtype %d", q_dtype);
   TQ_REQUIRE(out_dtype == TQ_F16 || out_dtype == TQ_BF16 || out_dtype == TQ_F32, TQ_ERR_UNSUPPORTED, "bad output dtype %d", out_dtype);
@@ -918,8 +1067,9 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
   P.kv_lens = kv_lens_dev;
   P.q = q_dev;
   P.out = out_dev;
-  P.k_rot_t = kq->rotation == TQ_ROT_DENSE ? kq->rot32_t : nullptr;
-  P.v_rot = vq->rotation == TQ_ROT_DENSE ? vq->rot32 : nullptr;
+  P.k_rot_t = !k_q8 && kq->rotation == TQ_ROT_DENSE ? kq->rot32_t : nullptr;
+  P.k_s_t = k_prod && kq->rotation == TQ_ROT_DENSE ? kq->s32_t : nullptr;
+  P.v_rot = !v_q8 && vq->rotation == TQ_ROT_DENSE ? vq->rot32 : nullptr;
   P.status = reinterpret_cast<int32_t*>((uint8_t*)workspace_dev + workspace_bytes - 256);
   if (scale <= 0.f) scale = TQ_RSQRT_D;
   P.qscale = scale * 1.4426950408889634f;
@@ -945,10 +1095,16 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
   P.row_blocks = plan.row_blocks;
   P.L = *L;
   cudaStream_t st = (cudaStream_t)stream;
+  TqFast none;
+  memset(&none, 0, sizeof(none));
+  none.lut_alpha = 1.0f;
+  const TqFast &fk = k_q8 ? none : kq->fast, &fv = v_q8 ? none : vq->fast;
   int rc = TQ_ERR_UNSUPPORTED;
 #define TQ_PF(K, V) \
-  if (L->k_format == K && L->v_format == V) rc = launch_prefill<K, V>(P, kq->fast, vq->fast, st);
+  if (L->k_format == K && L->v_format == V) rc = launch_prefill<K, V>(P, fk, fv, st);
   TQ_PF(2, 2) TQ_PF(3, 3) TQ_PF(4, 4) TQ_PF(3, 2) TQ_PF(4, 2) TQ_PF(4, 3)
+  TQ_PF(8, 2) TQ_PF(8, 3) TQ_PF(8, 4) TQ_PF(8, 8)
+  TQ_PF(18, 2) TQ_PF(18, 3) TQ_PF(19, 2) TQ_PF(19, 3) TQ_PF(19, 4) TQ_PF(20, 3) TQ_PF(20, 4)
 #undef TQ_PF
   if (rc == TQ_ERR_UNSUPPORTED) tq_set_error("prefill attention: K format %d with V format %d is not instantiated", L->k_format, L->v_format);
   return rc;

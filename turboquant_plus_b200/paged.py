@@ -181,17 +181,17 @@ class PagedKVCache:
     def prefill_attend(self, q, block_table, kv_lens, scale=None, out=None, workspace=None):
         """Chunked prefill on the tcgen05 tensor cores.  q: (batch, chunk_tokens, num_q_heads, head_dim) CUDA
         tensor of a chunk whose K/V rows are already in the cache; kv_lens: (batch,) cached tokens including
-        the chunk.  Query i of a sequence sees cached positions 0 .. kv_len - chunk_tokens + i.  turbo2/3/4 K and V
-        take the tcgen05 kernel; PROD or q8_0 tensors run the chunk's queries through the decode kernel."""
+        the chunk.  Query i of a sequence sees cached positions 0 .. kv_len - chunk_tokens + i.  Every pair of
+        formats on 128-token pages takes the tcgen05 kernel."""
         bsz, tq, hq, d = q.shape
         assert d == self.head_dim
-        if not (self.k_format.startswith("turbo") and self.v_format.startswith("turbo")):
+        if self.page_tokens != 128 and not (self.k_format.startswith("turbo") and self.v_format.startswith("turbo")):
             torch = nv.require_cuda()
             q = q.contiguous()
             bt = block_table.to(device=self.device, dtype=torch.int32).contiguous()
             kl = kv_lens.to(device=self.device, dtype=torch.int32).contiguous()
-            # PROD and q8_0 tensors have no tensor-memory pipeline: every query of the chunk runs as a row of the decode
-            # kernel with its own causal length (the cache is read once per query; the pages of a sequence stay in L2)
+            # PROD and q8_0 tensors in pages of another size: every query of the chunk runs as a row of the decode kernel
+            # with its own causal length (the cache is read once per query; the pages of a sequence stay in L2)
             lens = (kl[:, None] - tq + 1 + torch.arange(tq, device=self.device, dtype=torch.int32)[None, :]).clamp_(min=0)
             res = self.attend(q.reshape(bsz * tq, hq, d), bt.repeat_interleave(tq, dim=0), lens.reshape(-1), scale=scale)
             res = res.reshape(bsz, tq, hq, d)
