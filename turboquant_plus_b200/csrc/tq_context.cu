@@ -83,7 +83,7 @@ struct DeviceImage {
 };
 
 struct MatrixParts {
-  size_t m, t, m32, t32;
+  size_t m, t, m32, t32, mp, tp;   // mp, tp: padded with zeros to dp x dp (m and t themselves when d is a multiple of 8)
 };
 static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
   std::vector<double> t((size_t)d * d);
@@ -97,6 +97,19 @@ static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
   MatrixParts p;
   p.m = im.add(m, t.size() * 8);
   p.t = im.add(t.data(), t.size() * 8);
+  p.mp = p.m;
+  p.tp = p.t;
+  if (d % 8) {
+    const int dp = (d + 7) / 8 * 8;
+    std::vector<double> mp((size_t)dp * dp, 0.0), tp((size_t)dp * dp, 0.0);
+    for (int i = 0; i < d; ++i)
+      for (int j = 0; j < d; ++j) {
+        mp[(size_t)i * dp + j] = m[(size_t)i * d + j];
+        tp[(size_t)j * dp + i] = m[(size_t)i * d + j];
+      }
+    p.mp = im.add(mp.data(), mp.size() * 8);
+    p.tp = im.add(tp.data(), tp.size() * 8);
+  }
   p.m32 = im.add(a32.data(), a32.size() * 4);
   p.t32 = im.add(t32.data(), t32.size() * 4);
   return p;
@@ -211,8 +224,8 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
   }
   auto f64 = [&](size_t at) { return reinterpret_cast<double*>(q->mem + at); };
   auto f32 = [&](size_t at) { return reinterpret_cast<float*>(q->mem + at); };
-  if (dense_rot) q->rot = f64(mr.m), q->rot_t = f64(mr.t), q->rot32 = f32(mr.m32), q->rot32_t = f32(mr.t32);
-  if (dense_s) q->s = f64(ms.m), q->s_t = f64(ms.t), q->s32 = f32(ms.m32), q->s32_t = f32(ms.t32);
+  if (dense_rot) q->rot = f64(mr.m), q->rot_t = f64(mr.t), q->rot32 = f32(mr.m32), q->rot32_t = f32(mr.t32), q->rotp = f64(mr.mp), q->rotp_t = f64(mr.tp);
+  if (dense_s) q->s = f64(ms.m), q->s_t = f64(ms.t), q->s32 = f32(ms.m32), q->s32_t = f32(ms.t32), q->sp = f64(ms.mp), q->sp_t = f64(ms.tp);
   q->cent64 = f64(cent_at);
   q->bnd64 = f64(bnd_at);
   *out = q;

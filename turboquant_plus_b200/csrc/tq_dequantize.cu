@@ -213,6 +213,18 @@ __global__ void __launch_bounds__(128) k_dequantize_dense(const double* __restri
   }
 }
 
+// d <= 256: the fp64 tensor cores (tq_dense.cu); wider vectors stay with k_dequantize_dense
+static bool dequantize_tensor(const tq_quantizer* q, const uint8_t* packed, const uint8_t* idx, const float* norm,
+                              const uint8_t* qjl, const float* rnorm, double shrink, int64_t n, void* out, int32_t dtype,
+                              int64_t ld_out, int32_t accumulate, cudaStream_t st, int* rc) {
+  TqDenseDequant t;
+  t.rot_t = q->rotp_t; t.s_t = q->sp_t; t.cent = q->cent64;
+  t.d = q->d; t.dp = (q->d + 7) / 8 * 8; t.bits = q->bits; t.norm_correction = q->norm_correction;
+  t.packed = packed; t.idx = idx; t.norm = norm; t.qjl = qjl; t.rnorm = rnorm;
+  t.shrink = shrink; t.ld_out = ld_out; t.accumulate = accumulate;
+  return tq_dense_dequantize_try(t, n, out, dtype, st, rc);
+}
+
 extern "C" int tq_dequantize(const tq_quantizer* q, const uint8_t* packed_dev, const uint8_t* idx_dev,
                              const float* norm_dev, const uint8_t* qjl_dev, const float* rnorm_dev, float shrinkage,
                              int64_t n, void* out_dev, int32_t out_dtype, void* stream) {
@@ -256,6 +268,9 @@ extern "C" int tq_dequantize(const tq_quantizer* q, const uint8_t* packed_dev, c
 #undef TQ_DQ
     return tq_launch_check("k_dequantize_wht");
   }
+  int rc = TQ_OK;
+  if (dequantize_tensor(q, packed_dev, idx_dev, norm_dev, qjl_dev, rnorm_dev, (double)shrinkage, n, out_dev, out_dtype, q->d, 0, st, &rc))
+    return rc;
   const size_t smem = (size_t)q->d * DV * 8 * (qjl_dev ? 2 : 1);
   const int grid = (int)((n + DV - 1) / DV);
 #define TQ_DD(T)                                                                                                     \
@@ -288,6 +303,10 @@ extern "C" int tq_dequantize_strided(const tq_quantizer* q, const uint8_t* idx_d
   TQ_REQUIRE(idx_dev && norm_dev && out_dev, TQ_ERR_INVALID, "tq_dequantize_strided: null buffer");
   TQ_REQUIRE(ld_out >= q->d, TQ_ERR_INVALID, "tq_dequantize_strided: row stride %lld smaller than d", (long long)ld_out);
   TQ_REQUIRE(tq_aligned(out_dev, 8), TQ_ERR_ALIGN, "tq_dequantize_strided: output rows must be 8-byte aligned");
+  int rc = TQ_OK;
+  if (dequantize_tensor(q, nullptr, idx_dev, norm_dev, nullptr, nullptr, 1.0, n, out_dev, TQ_F64, ld_out, accumulate ? 1 : 0,
+                        (cudaStream_t)stream, &rc))
+    return rc;
   const size_t smem = (size_t)q->d * DV * 8;
   const int grid = (int)((n + DV - 1) / DV);
   if (smem > 48 * 1024)

@@ -34,6 +34,7 @@ struct tq_quantizer {
   uint8_t* mem;              // the one device allocation that the pointers below point into
   // dense mode, device memory (fp64): R row-major, its transpose, S, its transpose
   double *rot, *rot_t, *s, *s_t;
+  double *rotp, *rotp_t, *sp, *sp_t;   // the same padded with zeros to a multiple of eight
   double* cent64;            // 1 << bits
   double* bnd64;             // (1 << bits) - 1
   float* rot32;              // R row-major in fp32 (query / output rotation of the attention path)
@@ -226,6 +227,32 @@ __device__ __forceinline__ int64_t tq_dst_record(const TqQuantDst& dst, int64_t 
   within64 = within;
   return page * dst.page_stride + head * dst.head_stride;
 }
+
+// dense-mode work on the fp64 tensor cores (tq_dense.cu); matrices padded to dp x dp
+struct TqDenseQuant {
+  const double *rot, *rot_t, *s;   // R, R^T, S, rows contiguous
+  const double *cent, *bnd;
+  int32_t d, dp, bits, norm_correction;
+  uint8_t *out_packed, *out_idx;
+  float *out_norm, *out_scale, *out_rnorm;
+  uint8_t* out_qjl;
+  double* out_res;                 // fp64 rows of stride ld_res; or null
+  int64_t ld_res;
+};
+struct TqDenseDequant {
+  const double *rot_t, *s_t;       // R^T, S^T, rows contiguous
+  const double* cent;
+  int32_t d, dp, bits, norm_correction;
+  const uint8_t *packed, *idx;     // one of the two
+  const float* norm;
+  const uint8_t* qjl;              // with rnorm; or null
+  const float* rnorm;
+  double shrink;
+  int64_t ld_out;
+  int32_t accumulate;
+};
+bool tq_dense_quantize_try(const TqDenseQuant& a, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st, int* rc);
+bool tq_dense_dequantize_try(const TqDenseDequant& a, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
 
 int tq_quantize_wht_launch(const TqFast& f, const void* x, int32_t dtype, int64_t ld, int64_t n,
                            const TqQuantDst& dst, bool want_qjl, cudaStream_t st);

@@ -4,9 +4,10 @@
 //   k_quantize_wht   d = 128, sign * Walsh-Hadamard rotation in registers + warp shuffles, fp32.
 //                    Eight lanes share a vector (16 consecutive elements each); a warp handles
 //                    four vectors per iteration.  Output is the packed stream the cache stores.
-//   k_quantize_dense any d <= 1024, dense d x d rotation in fp64 -- the reference's own
+//   k_quantize_dense 256 < d <= 1024, dense d x d rotation in fp64 -- the reference's own
 //                    arithmetic (turboquant/polar_quant.py:56-85 runs an fp64 GEMM), used where
-//                    index-exact agreement with the reference classes matters more than speed.
+//                    index-exact agreement with the reference classes matters more than speed
+//                    (d <= 256: tq_dense.cu).
 //   k_q8_0_append    int8 + fp16 scale per 32 values.
 #include "tq_internal.cuh"
 
@@ -528,6 +529,17 @@ __global__ void __launch_bounds__(128) k_quantize_dense(const TqDenseArgs a, con
 static int launch_dense(const tq_quantizer* q, const void* x, int32_t dtype, int64_t ld, int64_t n, TqDenseArgs& a,
                         cudaStream_t st) {
   if (n == 0) return TQ_OK;
+  {
+    TqDenseQuant t;
+    t.rot = q->rotp; t.rot_t = q->rotp_t; t.s = q->sp;
+    t.cent = a.cent; t.bnd = a.bnd;
+    t.d = q->d; t.dp = (q->d + 7) / 8 * 8; t.bits = a.bits; t.norm_correction = a.norm_correction;
+    t.out_packed = a.out_packed; t.out_idx = a.out_idx;
+    t.out_norm = a.out_norm; t.out_scale = a.out_scale; t.out_rnorm = a.out_rnorm;
+    t.out_qjl = a.out_qjl; t.out_res = a.out_res; t.ld_res = a.ld_res;
+    int rc = TQ_OK;
+    if (tq_dense_quantize_try(t, x, dtype, ld, n, st, &rc)) return rc;
+  }
   const size_t smem = (size_t)q->d * TV * 8 * 2 + (size_t)q->d * TV + 16;
   const int grid = (int)((n + TV - 1) / TV);
 #define TQ_DENSE(T, W)                                                                                             \
