@@ -6,6 +6,7 @@
 // launch.  Arguments that are already in the form the kernels take (device, type, contiguous) are used as they are;
 // anything else is converted through torch first, as the Python layer did.
 #include <Python.h>
+#include <pybind11/pybind11.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -13,6 +14,7 @@
 #include <ATen/ATen.h>
 
 #include "tq_b200.h"
+#include "tq_host_copy.h"
 
 namespace {
 
@@ -308,6 +310,81 @@ PyObject* sign_bits(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// the elements of a C-contiguous buffer of a type the copies know; PyBuffer released by the caller
+tqhost::HostArray host_array(Py_buffer* b) {
+  char f = b->format ? b->format[0] : 'B';
+  if (f == '<' || f == '=' || f == '@') f = b->format[1];
+  using tqhost::Elem;
+  Elem e = Elem::U8;
+  if (f == 'd') e = Elem::F64;
+  else if (f == 'f') e = Elem::F32;
+  else if (f == 'e') e = Elem::F16;
+  else if ((f == 'l' || f == 'q') && b->itemsize == 8) e = Elem::I64;
+  else if ((f == 'i' || f == 'l') && b->itemsize == 4) e = Elem::I32;
+  else if (f == 'b') e = Elem::I8;
+  else if (f != 'B') raise(PyExc_TypeError, "array type without a host copy");
+  return {b->buf, b->itemsize ? (int64_t)(b->len / b->itemsize) : 0, e};
+}
+
+struct Buffers {
+  std::vector<Py_buffer> all;
+  ~Buffers() {
+    for (auto& b : all) PyBuffer_Release(&b);
+  }
+  tqhost::HostArray get(PyObject* o, int flags) {
+    all.emplace_back();
+    if (PyObject_GetBuffer(o, &all.back(), flags | PyBUF_C_CONTIGUOUS | PyBUF_FORMAT) != 0) {
+      all.pop_back();
+      throw PyRaised{};
+    }
+    return host_array(&all.back());
+  }
+};
+
+// upload(array, device index, dtype code or -2 for bytes, -3 for signed bytes) -> CUDA tensor of the array's shape
+PyObject* upload(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 3, "upload");
+    Buffers bufs;
+    const tqhost::HostArray h = bufs.get(a[0], PyBUF_SIMPLE);
+    const Py_buffer& b = bufs.all.back();
+    std::vector<int64_t> shape(b.shape, b.shape + b.ndim);
+    const int64_t code = integer(a[2]);
+    const at::ScalarType type = code == -2 ? at::kByte : code == -3 ? at::kChar : code == TQ_F64 ? at::kDouble
+                                : code == TQ_F16 ? at::kHalf : at::kFloat;
+    const c10::Device dev(c10::DeviceType::CUDA, (c10::DeviceIndex)integer(a[1]));
+    at::Tensor t;
+    {
+      pybind11::gil_scoped_release nogil;
+      const On on(dev);
+      t = at::empty(shape, at::TensorOptions().device(dev).dtype(type));
+      tqhost::to_device(h, t);
+    }
+    return THPVariable_Wrap(std::move(t));
+  });
+}
+
+// download(tensor, array, tensor, array, ...): fills the arrays, converted to their types
+PyObject* download(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    Buffers bufs;
+    bufs.all.reserve(n);
+    std::vector<std::pair<at::Tensor, tqhost::HostArray>> jobs;
+    for (Py_ssize_t i = 0; i + 1 < n; i += 2) {
+      const at::Tensor& t = tensor(a[i], "source");
+      const tqhost::HostArray h = bufs.get(a[i + 1], PyBUF_WRITABLE);
+      if (!t.is_cuda() || t.numel() != h.count) raise(PyExc_ValueError, "download needs CUDA tensors and arrays of their sizes");
+      jobs.emplace_back(t.is_contiguous() ? t : t.contiguous(), h);
+    }
+    if (!jobs.empty()) {
+      pybind11::gil_scoped_release nogil;
+      const On on(jobs[0].first.device());
+      tqhost::to_host(jobs);
+    }
+    return none();
+  });
+}
+
 #define TQ_FAST(name, f, doc) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, doc}
 PyMethodDef methods[] = {
     {"set_error", set_error, METH_O, "exception type of failed calls"},
@@ -319,6 +396,8 @@ PyMethodDef methods[] = {
     TQ_FAST("quantize", quantize, "tq_quantize on tensors"),
     TQ_FAST("dequantize", dequantize, "tq_dequantize on tensors"),
     TQ_FAST("sign_bits", sign_bits, "tq_pack_bits / tq_unpack_bits on tensors"),
+    TQ_FAST("upload", upload, "host array to a CUDA tensor, converted"),
+    TQ_FAST("download", download, "CUDA tensors into host arrays, converted"),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_tq_host", "tensor front end of libtq_b200.so", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

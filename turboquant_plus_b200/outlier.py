@@ -15,7 +15,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import _native as nv
-from ._io import floats_to_device, ints_to_device, to_device
+from ._io import floats_to_device, ints_to_device, to_device, to_numpy
 from .polar_quant import PolarQuant
 from .qjl import QJL
 
@@ -129,8 +129,7 @@ class OutlierTurboQuant:
                 return np.array([])       # a group without channels, as the reference returns it
             if not was_numpy:
                 return t[0] if single else t
-            a = t.cpu().numpy()
-            a = a.astype({"idx": np.int64, "norm": norm_dtype, "rnorm": np.float64, "signs": np.int8}[kind])
+            a, = to_numpy((t, {"idx": np.int64, "norm": norm_dtype, "rnorm": np.float64, "signs": np.int8}[kind]))
             return a[0] if single else a
 
         return OutlierCompressedVector(
@@ -164,7 +163,7 @@ class OutlierTurboQuant:
             code[name + "_norm"] = floats_to_device(flat(getattr(compressed, name + "_norms")), dev)
         out = self.dequantize_device(code)
         if was_numpy:
-            out = out.cpu().numpy()
+            out, = to_numpy((out, np.float64))
         return out[0] if single else out
 
     def compression_ratio(self, original_bits: int = 16) -> float:

@@ -13,7 +13,7 @@ from __future__ import annotations
 import numpy as np
 
 from . import _native as nv
-from ._io import floats_to_device, ints_to_device, to_device
+from ._io import floats_to_device, ints_to_device, to_device, to_numpy
 from .codebook import optimal_centroids
 from .rotation import fast_rotation_matrix, random_rotation_dense, random_rotation_fast
 
@@ -129,8 +129,7 @@ class PolarQuant:
         out = self.quantize_device(xt)
         idx, nrm = out["idx"], out["norm"]
         if was_numpy:
-            idx = idx.cpu().numpy().astype(np.int64)
-            nrm = nrm.cpu().numpy().astype(src_dtype if src_dtype is not None else np.float64)
+            idx, nrm = to_numpy((idx, np.int64), (nrm, src_dtype if src_dtype is not None else np.float64))
         return (idx[0], nrm[0]) if single else (idx, nrm)
 
     def dequantize(self, indices, norms):
@@ -145,7 +144,7 @@ class PolarQuant:
         nt = floats_to_device(np.asarray(norms).reshape(-1) if was_numpy else norms.reshape(-1), dev)
         out = self.dequantize_device(nt, idx=it)
         if was_numpy:
-            out = out.cpu().numpy().astype(np.float64)
+            out, = to_numpy((out, np.float64))
         return out[0] if single else out
 
     def quantize_and_residual(self, x):
@@ -168,9 +167,8 @@ class PolarQuant:
                 nv.call("tq_quantize_residual", self._native(xt.device).handle, nv.ptr(xt), nv.torch_dtype_code(xt.dtype),
                         xt.stride(0), n, nv.ptr(idx), nv.ptr(nrm), nv.ptr(res), self.d, nv.stream_ptr())
             if was_numpy:
-                idx = idx.cpu().numpy().astype(np.int64)
-                nrm = nrm.cpu().numpy().astype(src_dtype if src_dtype is not None else np.float64)
-                res = res.cpu().numpy()
+                idx, nrm, res = to_numpy((idx, np.int64), (nrm, src_dtype if src_dtype is not None else np.float64),
+                                         (res, np.float64))
             return (idx[0], nrm[0], res[0]) if single else (idx, nrm, res)
         indices, norms = self.quantize(x)
         x_hat = self.dequantize(indices, norms)

@@ -8,7 +8,7 @@ from __future__ import annotations
 import numpy as np
 
 from . import _native as nv
-from ._io import floats_to_device, ints_to_device, to_device
+from ._io import floats_to_device, ints_to_device, to_device, to_numpy
 from .rotation import fast_rotation_matrix, random_rotation_fast
 
 QJL_CONST = np.sqrt(np.pi / 2)
@@ -84,8 +84,7 @@ class QJL:
                     nv.ptr(nrm), nv.stream_ptr())
             nv.call("tq_unpack_bits", nv.ptr(bits), n, self.d, nv.ptr(signs), nv.stream_ptr())
         if was_numpy:
-            signs = signs.cpu().numpy()
-            nrm = nrm.cpu().numpy().astype(src_dtype if src_dtype is not None else np.float64)
+            signs, nrm = to_numpy((signs, np.int8), (nrm, src_dtype if src_dtype is not None else np.float64))
         return (signs[0], nrm[0]) if single else (signs, nrm)
 
     def dequantize(self, signs, norms, shrinkage: float = 1.0):
@@ -108,5 +107,5 @@ class QJL:
             nv.call("tq_qjl_dequantize", q.handle, nv.ptr(bits), nv.ptr(nt), float(shrinkage), n, nv.ptr(out),
                     nv.F64, nv.stream_ptr())
         if was_numpy:
-            out = out.cpu().numpy()
+            out, = to_numpy((out, np.float64))
         return out[0] if single else out

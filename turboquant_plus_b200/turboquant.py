@@ -11,7 +11,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import _native as nv
-from ._io import floats_to_device, ints_to_device, to_device
+from ._io import floats_to_device, ints_to_device, to_device, to_numpy
 from .polar_quant import PolarQuant
 from .qjl import QJL
 from .rotation import fast_rotation_matrix
@@ -90,10 +90,9 @@ class TurboQuant:
         signs = nv.host().sign_bits(out["qjl"], self.d, False)
         idx, nrm, rn = out["idx"], out["norm"], out["rnorm"]
         if was_numpy:
-            idx = idx.cpu().numpy().astype(np.int64)
-            nrm = nrm.cpu().numpy().astype(src_dtype if src_dtype is not None else np.float64)
-            rn = rn.cpu().numpy().astype(np.float64)  # the reference's residual is fp64
-            signs = signs.cpu().numpy()
+            # (the reference's residual is fp64)
+            idx, nrm, rn, signs = to_numpy((idx, np.int64), (nrm, src_dtype if src_dtype is not None else np.float64),
+                                           (rn, np.float64), (signs, np.int8))
         if single:
             idx, nrm, rn, signs = idx[0], nrm[0], rn[0], signs[0]
         return CompressedVector(mse_indices=idx, vector_norms=nrm, qjl_signs=signs, residual_norms=rn,
@@ -117,7 +116,7 @@ class TurboQuant:
         bits = nv.host().sign_bits(st, self.d, True)
         out = nv.host().dequantize(q.address, it, False, nt, bits, rt, float(shrinkage), self.d, nv.torch_dtype_code(out_dtype))
         if was_numpy:
-            out = out.cpu().numpy().astype(np.float64)
+            out, = to_numpy((out, np.float64))
         return out[0] if single else out
 
     def compressed_size_bits(self, n_vectors: int) -> int:
