@@ -85,8 +85,7 @@ def _build_host(verbose: bool) -> None:
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
     inc = [INCLUDE, CSRC_HOST, os.path.join(base, "include"), os.path.join(base, "include/torch/csrc/api/include"),
            sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
-    # -fopenmp: at::parallel_for is a template over torch's OpenMP thread pool
-    _run(["g++", "-O3", "-fopenmp", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w", *[f"-I{p}" for p in inc],
+    _run(["g++", "-O3", "-pthread", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w", *[f"-I{p}" for p in inc],
           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *host_sources(), "-o", HOST_LIB,
           f"-L{os.path.join(base, 'lib')}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python",
           f"-L{PKG}", "-l:libtq_b200.so", "-Wl,-rpath,$ORIGIN"], "g++ for _tq_host.so", verbose)

@@ -1,15 +1,27 @@
 // A copy between pageable memory and the GPU goes through the driver's own staging buffer on one thread (3-10 GB/s), and a
 // change of type around it -- 64-bit indices on the host are bytes on the device -- was a second and third pass on one
 // thread, most of it page faults of the new array.  Here the conversion is the pass between the caller's array and a pinned
-// staging buffer, done by torch's intra-op threads in pieces of a few MB while the neighbouring piece is on the bus: the
-// index array of 65,536 x 128 vectors travels as 8 MB instead of 67, and the threads share the page faults.  The staging
-// buffers come from torch's pinned allocator (two pieces per call), which keeps and reuses them.
+// staging buffer, in pieces that a few threads take from a counter, so that one thread's piece is on the bus while others
+// convert theirs: the index array of 65,536 x 128 vectors travels as 8 MB instead of 67.  A piece is one
+// 2 MB page of a large array (NumPy asks for those), so that the threads clear different pages: with all of them inside one
+// piece the faults of a fresh 67 MB array took 4 ms.  The threads live for one call and block when they wait; the caller
+// works too, and on a busy machine (BLAS threads spin for some 30 ms after a product) does not wait for a helper that has
+// not got to run yet.  The buffers come from torch's pinned allocator in one block of at most 32 MB, which keeps and
+// reuses it.
 #include "tq_host_copy.h"
 
-#include <ATen/Parallel.h>
 #include <c10/core/Event.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <string.h>
+
+#include <algorithm>
+#include <condition_variable>
+#include <exception>
+#include <memory>
+#include <mutex>
+#include <system_error>
+#include <thread>
 
 namespace tqhost {
 
@@ -36,9 +48,9 @@ at::ScalarType scalar_type(Elem e) {
 
 namespace {
 
-constexpr int64_t PIECE = 4 << 20;    // bytes of the host array per piece: short against the whole, long against a launch
-constexpr int64_t SMALL = 256 << 10;  // arrays up to this size travel in one piece, several of them behind one wait
-constexpr int64_t GRAIN = 64 << 10;   // bytes per thread below which more threads do not pay
+constexpr int64_t PAGE = 2 << 20;       // most bytes of the wider side per piece
+constexpr int64_t LEAST = 256 << 10;    // fewest: arrays up to this size travel in one piece, several behind one wait
+constexpr int MOST_THREADS = 8;
 
 Elem elem_of(at::ScalarType t) {
   switch (t) {
@@ -57,13 +69,11 @@ template <typename S, typename D>
 void convert_as(const void* src, void* dst, int64_t n) {
   const S* s = static_cast<const S*>(src);
   D* d = static_cast<D*>(dst);
-  at::parallel_for(0, n, GRAIN / (int64_t)(sizeof(S) > sizeof(D) ? sizeof(S) : sizeof(D)), [=](int64_t lo, int64_t hi) {
-    if constexpr (std::is_same_v<S, D>) {
-      memcpy(d + lo, s + lo, (size_t)(hi - lo) * sizeof(S));
-    } else {
-      for (int64_t i = lo; i < hi; ++i) d[i] = static_cast<D>(s[i]);
-    }
-  });
+  if constexpr (std::is_same_v<S, D>) {
+    memcpy(d, s, (size_t)n * sizeof(S));
+  } else {
+    for (int64_t i = 0; i < n; ++i) d[i] = static_cast<D>(s[i]);
+  }
 }
 
 template <typename S>
@@ -95,78 +105,161 @@ at::Tensor pinned(int64_t count, at::ScalarType type) {
   return at::empty({count}, at::TensorOptions().dtype(type).pinned_memory(true));
 }
 
-// elements per piece of an array whose wider side has `width` bytes per element
-int64_t piece_elems(int64_t count, size_t width) {
-  const int64_t whole = count * (int64_t)width;
-  return whole <= SMALL ? count : PIECE / (int64_t)width;
+size_t wider(Elem a, Elem b) { return elem_size(a) > elem_size(b) ? elem_size(a) : elem_size(b); }
+
+// Elements [begin(p), begin(p + 1)) of an array are piece p; pieces of PAGE bytes end on multiples of PAGE in the host's
+// address space.
+struct Pieces {
+  int64_t count, step, first, n;
+  Pieces(const HostArray& h, Elem dev) : count(h.count) {
+    const int64_t w = (int64_t)wider(h.elem, dev), bytes = count * w;
+    const int64_t piece = std::min(PAGE, std::max(LEAST, bytes / (2 * MOST_THREADS)));
+    step = piece / w;
+    first = step;
+    if (piece == PAGE && (int64_t)elem_size(h.elem) == w) {
+      const int64_t to_page = (int64_t)(PAGE - (reinterpret_cast<uintptr_t>(h.data) & (PAGE - 1))) / w;
+      if (to_page > 0) first = to_page;
+    }
+    first = std::min(first, count);
+    n = 1 + (count - first + step - 1) / step;
+  }
+  int64_t begin(int64_t p) const { return p == 0 ? 0 : std::min(count, first + (p - 1) * step); }
+  int64_t length(int64_t p) const { return begin(p + 1) - begin(p); }
+  int64_t longest() const { return std::min(count, std::max(first, step)); }
+};
+
+// What the threads of one call share.  A helper that starts after the caller has closed it touches nothing else.
+struct Crew {
+  std::mutex lock;
+  std::condition_variable idle;
+  int64_t at = 0, pieces = 0;
+  int active = 0, buffers = 0;
+  bool closed = false;
+  std::exception_ptr failed;
+
+  int64_t next() {
+    const std::lock_guard<std::mutex> hold(lock);
+    return at < pieces && !failed ? at++ : -1;
+  }
+};
+
+// work(buffer, p) for every piece p, on the caller and up to threads - 1 helpers; `buffer` is a thread's own number
+template <typename F>
+void on_threads(int64_t pieces, int threads, const c10::cuda::CUDAStream& stream, const F& work) {
+  auto crew = std::make_shared<Crew>();
+  crew->pieces = pieces;
+  auto take_part = [&work, stream](Crew& c) {
+    int mine;
+    {
+      const std::lock_guard<std::mutex> hold(c.lock);
+      if (c.closed || c.at >= c.pieces) return;
+      mine = c.buffers++;
+      ++c.active;
+    }
+    try {
+      const c10::cuda::CUDAStreamGuard guard(stream);
+      for (int64_t p; (p = c.next()) >= 0;) work(mine, p);
+    } catch (...) {
+      const std::lock_guard<std::mutex> hold(c.lock);
+      if (!c.failed) c.failed = std::current_exception();
+    }
+    const std::lock_guard<std::mutex> hold(c.lock);
+    if (--c.active == 0) c.idle.notify_all();
+  };
+  for (int w = 1; w < threads; ++w) {
+    try {
+      std::thread([crew, take_part] { take_part(*crew); }).detach();
+    } catch (const std::system_error&) {
+      break;   // no more threads to be had: fewer do the work
+    }
+  }
+  take_part(*crew);
+  std::unique_lock<std::mutex> hold(crew->lock);
+  crew->closed = true;
+  crew->idle.wait(hold, [&] { return crew->active == 0; });
+  if (crew->failed) std::rethrow_exception(crew->failed);
 }
 
-size_t wider(Elem a, Elem b) { return elem_size(a) > elem_size(b) ? elem_size(a) : elem_size(b); }
+int thread_count(const Pieces& p, size_t width) {
+  const int64_t cores = std::thread::hardware_concurrency(), mega = p.count * (int64_t)width >> 20;
+  return (int)std::max<int64_t>(1, std::min({(int64_t)MOST_THREADS, p.n, cores / 2, 1 + mega}));
+}
+
+// two buffers per thread: [thread][2] of `room` elements
+struct Staging {
+  int64_t room;
+  at::Tensor all;
+  std::vector<c10::Event> moved;
+  std::vector<int> uses;
+  Staging(const Pieces& p, int threads, at::ScalarType type)
+      : room(p.longest()), all(pinned(2 * threads * room, type)), uses(threads, 0) {
+    for (int i = 0; i < 2 * threads; ++i) moved.emplace_back(c10::DeviceType::CUDA);
+  }
+  // the next of a thread's two buffers, free: what was copied from it before has left it
+  int take(int thread) {
+    const int b = 2 * thread + (uses[thread] & 1);
+    if (uses[thread]++ >= 2) moved[b].synchronize();
+    return b;
+  }
+  at::Tensor buffer(int b, int64_t n) const { return all.narrow(0, b * room, n); }
+};
 
 }  // namespace
 
 void to_device(const HostArray& src, const at::Tensor& dst) {
   if (src.count == 0) return;
   const Elem de = elem_of(dst.scalar_type());
-  const int64_t step = piece_elems(src.count, wider(src.elem, de));
+  const Pieces pieces(src, de);
   const at::Tensor flat = dst.view({-1});
-  at::Tensor stage[2];
-  std::optional<c10::Event> sent[2];
-  const c10::Stream stream = c10::cuda::getCurrentCUDAStream(dst.get_device()).unwrap();
-  int64_t at = 0;
-  for (int i = 0; at < src.count; ++i, at += step) {
-    const int b = i & 1;
-    const int64_t n = std::min(step, src.count - at);
-    if (!stage[b].defined()) {
-      stage[b] = pinned(std::min(step, src.count), dst.scalar_type());
-      sent[b].emplace(c10::DeviceType::CUDA);
-    } else {
-      sent[b]->synchronize();   // the piece before last has left this buffer
-    }
-    convert(static_cast<const uint8_t*>(src.data) + at * (int64_t)elem_size(src.elem), src.elem, stage[b].data_ptr(), de, n);
-    // (the copy tells the pinned allocator that the buffer is in use until it has completed)
-    flat.narrow(0, at, n).copy_(n == stage[b].numel() ? stage[b] : stage[b].narrow(0, 0, n), /*non_blocking=*/true);
-    if (at + step < src.count) sent[b]->record(stream);
-  }
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(dst.get_device());
+  const int threads = thread_count(pieces, wider(src.elem, de));
+  Staging stage(pieces, threads, dst.scalar_type());
+  on_threads(pieces.n, threads, stream, [&](int thread, int64_t p) {
+    const int64_t at = pieces.begin(p), n = pieces.length(p);
+    const int b = stage.take(thread);
+    const at::Tensor buf = stage.buffer(b, n);
+    convert(static_cast<const uint8_t*>(src.data) + at * (int64_t)elem_size(src.elem), src.elem, buf.data_ptr(), de, n);
+    // (the copy tells the pinned allocator that the block is in use until it has completed)
+    flat.narrow(0, at, n).copy_(buf, /*non_blocking=*/true);
+    stage.moved[b].record(stream.unwrap());
+  });
 }
 
 void to_host(const std::vector<std::pair<at::Tensor, HostArray>>& jobs) {
   std::vector<std::pair<at::Tensor, size_t>> small;   // staged, job
-  c10::Device dev(c10::DeviceType::CUDA, 0);
-  bool any = false;
+  c10::DeviceIndex dev = -1;
   for (const auto& [t, h] : jobs)
-    if (h.count) dev = t.device(), any = true;
-  if (!any) return;
-  const c10::Stream stream = c10::cuda::getCurrentCUDAStream(dev.index()).unwrap();
+    if (h.count) dev = (c10::DeviceIndex)t.get_device();
+  if (dev < 0) return;
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(dev);
+  auto is_small = [](const at::Tensor& t, const HostArray& h) {
+    return h.count * (int64_t)wider(elem_of(t.scalar_type()), h.elem) <= LEAST;
+  };
   for (size_t j = 0; j < jobs.size(); ++j) {
     const auto& [t, h] = jobs[j];
-    if (h.count == 0 || h.count * (int64_t)wider(elem_of(t.scalar_type()), h.elem) > SMALL) continue;
+    if (h.count == 0 || !is_small(t, h)) continue;
     small.emplace_back(pinned(h.count, t.scalar_type()), j);
     small.back().first.copy_(t.view({-1}), true);
   }
   c10::Event small_done(c10::DeviceType::CUDA);
-  if (!small.empty()) small_done.record(stream);
-  for (size_t j = 0; j < jobs.size(); ++j) {
-    const auto& [t, h] = jobs[j];
+  if (!small.empty()) small_done.record(stream.unwrap());
+  for (const auto& [t, h] : jobs) {
+    if (h.count == 0 || is_small(t, h)) continue;
     const Elem se = elem_of(t.scalar_type());
-    if (h.count == 0 || h.count * (int64_t)wider(se, h.elem) <= SMALL) continue;
-    const int64_t step = piece_elems(h.count, wider(se, h.elem));
+    const Pieces pieces(h, se);
     const at::Tensor flat = t.view({-1});
-    at::Tensor stage[2] = {pinned(step, t.scalar_type()), pinned(step, t.scalar_type())};
-    c10::Event arrived[2] = {c10::Event(c10::DeviceType::CUDA), c10::Event(c10::DeviceType::CUDA)};
-    const int64_t pieces = (h.count + step - 1) / step;
-    auto fetch = [&](int64_t p) {
-      const int64_t n = std::min(step, h.count - p * step);
-      stage[p & 1].narrow(0, 0, n).copy_(flat.narrow(0, p * step, n), true);
-      arrived[p & 1].record(stream);
-    };
-    fetch(0);
-    for (int64_t p = 0; p < pieces; ++p) {
-      if (p + 1 < pieces) fetch(p + 1);   // (its buffer was emptied by the conversion of piece p - 1)
-      arrived[p & 1].synchronize();
-      convert(stage[p & 1].data_ptr(), se, static_cast<uint8_t*>(h.data) + p * step * (int64_t)elem_size(h.elem), h.elem,
-              std::min(step, h.count - p * step));
-    }
+    const int threads = thread_count(pieces, wider(se, h.elem));
+    Staging stage(pieces, threads, t.scalar_type());
+    const HostArray to = h;
+    on_threads(pieces.n, threads, stream, [&](int thread, int64_t p) {
+      const int64_t at = pieces.begin(p), n = pieces.length(p);
+      const int b = stage.take(thread);
+      const at::Tensor buf = stage.buffer(b, n);
+      buf.copy_(flat.narrow(0, at, n), true);
+      stage.moved[b].record(stream.unwrap());
+      stage.moved[b].synchronize();
+      convert(buf.data_ptr(), se, static_cast<uint8_t*>(to.data) + at * (int64_t)elem_size(to.elem), to.elem, n);
+    });
   }
   if (!small.empty()) {
     small_done.synchronize();
