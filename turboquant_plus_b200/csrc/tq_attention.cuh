@@ -132,8 +132,6 @@ struct AttnParams {
   int32_t tail_late;   // the preceding kernel may write the last cached position of a sequence: its page is fetched
                        // after the dependency wait, every other page before (TQ_DECODE_OVERLAP_APPEND)
   int32_t chain_head;  // attention calls with TQ_DECODE_OVERLAP_Q follow this one (TQ_DECODE_CHAIN_HEAD)
-  int32_t kv_div;      // CTAs (grid.y entries) per KV head of the cache: hkv and group describe the query-head groups
-                       // that a CTA serves, kv_div of which share a KV head (specialised kernel, groups of 5..16 heads)
   tq_cache_layout L;
 };
 
@@ -291,7 +289,8 @@ __device__ __forceinline__ void fold_splits(const AttnParams& P, float v_alpha, 
 // take a ticket; the last CTA of a (sequence, kv head) folds all splits in a fixed order, un-rotates and stores.
 // One thread publishes the CTA's writes (the block barrier orders the other threads' stores before its
 // release), so the rest of the CTA does not execute a device-wide fence.
-template <bool V_Q8, int NT = ATT_THREADS>
+// HEADS: most query heads per KV head of the kernel.
+template <bool V_Q8, int NT = ATT_THREADS, int HEADS = MAX_G>
 __device__ __forceinline__ void finish_splits(const AttnParams& P, const uint32_t (&vs1)[4], const uint32_t (&vs2)[4],
                                               float v_alpha, float* qbuf, uint8_t* stage0, volatile int* s_flags,
                                               size_t row0, int ns, int b, int kvh, int tid = threadIdx.x, int bar_id = 0) {
@@ -313,7 +312,9 @@ __device__ __forceinline__ void finish_splits(const AttnParams& P, const uint32_
   // takes 64 of the 128 dims: lanes 0..15 then read even splits, lanes 16..31 odd ones (16 bytes each), and one
   // lane exchange joins the two at the end; with more heads a warp takes the whole row and every split.
   if (2 * P.group <= NT / 32) fold_splits<2, V_Q8>(P, v_alpha, qbuf, row0, ns, warp);
-  else fold_splits<1, V_Q8>(P, v_alpha, qbuf, row0, ns, warp);
+  else if constexpr (HEADS <= NT / 32) fold_splits<1, V_Q8>(P, v_alpha, qbuf, row0, ns, warp);
+  else
+    for (int w = warp; w < P.group; w += NT / 32) fold_splits<1, V_Q8>(P, v_alpha, qbuf, row0, ns, w);
   group_sync<NT>(bar_id);
   if (P.v_rot) {  // dense rotation: x = R^T y
     for (int e = tid; e < P.group * TQ_D; e += NT) {
@@ -323,13 +324,16 @@ __device__ __forceinline__ void finish_splits(const AttnParams& P, const uint32_
       for (int k = 0; k < TQ_D; ++k) x = fmaf(__ldg(P.v_rot + k * TQ_D + j), qbuf[head * TQ_D + k], x);
       store_out(P.out, P.out_dtype, (row0 + head) * TQ_D + j, x);
     }
-  } else if (warp < P.group) {
-    float x[4];
-    const float4 v = *reinterpret_cast<const float4*>(qbuf + warp * TQ_D + 4 * lane);
-    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-    if (!P.v_ident) warp_wht128(x, vs2, vs1, lane);  // R^T = D1 (H/sqrt d) D2
+  } else {
+    for (int head = warp; head < P.group; head += NT / 32) {
+      float x[4];
+      const float4 v = *reinterpret_cast<const float4*>(qbuf + head * TQ_D + 4 * lane);
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+      if (!P.v_ident) warp_wht128(x, vs2, vs1, lane);  // R^T = D1 (H/sqrt d) D2
 #pragma unroll
-    for (int k = 0; k < 4; ++k) store_out(P.out, P.out_dtype, (row0 + warp) * TQ_D + 4 * lane + k, x[k]);
+      for (int k = 0; k < 4; ++k) store_out(P.out, P.out_dtype, (row0 + head) * TQ_D + 4 * lane + k, x[k]);
+      if constexpr (HEADS <= NT / 32) break;
+    }
   }
 }
 __device__ __forceinline__ void load_q4(const void* q, int dtype, size_t i, float (&x)[4]) {
@@ -355,7 +359,8 @@ struct SplitPlan {
 
 }  // namespace tqatt
 
-// tq_decode_g4.cu: launches the kernel specialised for PolarQuant K and V, <= 4 query heads per KV head, 128-token
-// pages in the layout tq_cache_layout_init produces.  Returns false (nothing launched) when the call is not of that
+// tq_decode_g4.cu, tq_decode_g8.cu: launch the kernel specialised for <= 4 and 5..8 query heads per KV head on 128-token
+// pages in the layout tq_cache_layout_init produces.  Return false (nothing launched) when the call is not of that
 // shape; otherwise *rc is the launch status.
 bool tq_decode_g4_try(const tqatt::AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st, int* rc);
+bool tq_decode_g8_try(const tqatt::AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st, int* rc);
