@@ -6,6 +6,8 @@
 __global__ void k_decode_step_slots(const int32_t* __restrict__ block_table, int32_t max_pages, int32_t* seq_lens,
                                     int32_t page_tokens, int32_t batch, int32_t copies, int64_t copy_stride,
                                     int64_t* __restrict__ slots) {
+  TQ_PDL_ENTER();
+  TQ_PDL_POINTER(block_table);
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= batch) return;
   const int pos = seq_lens[b];
@@ -22,8 +24,8 @@ extern "C" int tq_decode_step_slots(const int32_t* block_table_dev, int32_t max_
   TQ_REQUIRE(batch >= 0 && copies >= 1 && page_tokens >= 1 && max_pages_per_seq >= 1, TQ_ERR_INVALID, "bad sizes");
   if (batch == 0) return TQ_OK;
   TQ_REQUIRE(block_table_dev && seq_lens_dev && slots_dev, TQ_ERR_INVALID, "tq_decode_step_slots: null buffer");
-  k_decode_step_slots<<<(batch + 127) / 128, 128, 0, (cudaStream_t)stream>>>(block_table_dev, max_pages_per_seq, seq_lens_dev,
-                                                                            page_tokens, batch, copies, copy_stride, slots_dev);
+  TQ_CUDA(tq_launch_early(k_decode_step_slots, (batch + 127) / 128, 128, 0, (cudaStream_t)stream, block_table_dev,
+                          max_pages_per_seq, seq_lens_dev, page_tokens, batch, copies, copy_stride, slots_dev));
   return tq_launch_check("k_decode_step_slots");
 }
 
@@ -65,7 +67,7 @@ extern "C" int tq_cache_append(const tq_quantizer* kq, const tq_quantizer* vq, c
     const int sc_off = which == 0 ? L->k_scale_off : L->v_scale_off;
     if (fmt == TQ_FMT_Q8_0) {
       int rc = tq_q8_0_append_launch(x, dtype, n_tokens, H, pool_dev + idx_off, pool_dev + sc_off, slot_dev,
-                                     L->page_tokens, L->page_stride, L->head_stride, st);
+                                     L->page_tokens, L->page_stride, L->head_stride, which == 1, st);
       if (rc != TQ_OK) return rc;
       continue;
     }
@@ -91,6 +93,7 @@ extern "C" int tq_cache_append(const tq_quantizer* kq, const tq_quantizer* vq, c
     dst.head_stride = L->head_stride;
     dst.page_tokens = L->page_tokens;
     dst.heads = H;
+    dst.beside = which;
     int rc = tq_quantize_wht_launch(q->fast, x, dtype, TQ_D, n_tokens * H, dst, prod, st);
     if (rc != TQ_OK) return rc;
   }

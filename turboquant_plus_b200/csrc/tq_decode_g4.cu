@@ -3,22 +3,17 @@
 
 bool tq_decode_g4_try(const tqatt::AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st, int* rc) {
   const int kf = P.L.k_format, vf = P.L.v_format;
-  // The four-warp form pays in a chain of attention calls, where the CTAs of consecutive calls share an SM in
-  // different phases: calls launched with TQ_DECODE_OVERLAP_Q, and the call in front of them when the caller says so
-  // (TQ_DECODE_CHAIN_HEAD).  A call that follows an append overlaps only its start with that short kernel: it takes
-  // the eight-warp form, which is the faster one for a call on its own.
-  // 4-bit tables: only the eight-warp form has room for lane-replicated ones, which is worth more (turbo4 / turbo4, 16
-  // sequences of 8,192 tokens, per call of a chain: 62 us with four warps and one copy of the tables).
-  const bool chain = (P.q_early || P.chain_head) && !P.tail_late && !has_4bit_table(kf) && !has_4bit_table(vf);
+  const bool w4 = four_warps(P);
   // PolarQuant K and V: every pair of widths, with the sparse-V and the measurement variants
 #define TQ_ATT_G4(K, V)                                                                                              \
   if (kf == K && vf == V) {                                                                                          \
     if (!layout_matches<K, V>(P.L)) return false;                                                                    \
     if (P.nodeq && K == 3 && V == 3) *rc = launch_attn_g4<3, 3, false, true>(P, fk, fv, st);                         \
-    else if (P.sparse_v && chain) *rc = launch_attn_g4<K, V, true, false, 4>(P, fk, fv, st);                         \
+    else if (P.sparse_v && w4) *rc = launch_attn_g4<K, V, true, false, 4>(P, fk, fv, st);                         \
     else if (P.sparse_v) *rc = launch_attn_g4<K, V, true, false>(P, fk, fv, st);                                     \
+    else if (P.tail_late && w4) *rc = launch_attn_g4<K, V, false, false, 4, true>(P, fk, fv, st);                   \
     else if (P.tail_late) *rc = launch_attn_g4<K, V, false, false, ATT_WARPS, true>(P, fk, fv, st);                  \
-    else if (chain) *rc = launch_attn_g4<K, V, false, false, 4>(P, fk, fv, st);                                      \
+    else if (w4) *rc = launch_attn_g4<K, V, false, false, 4>(P, fk, fv, st);                                      \
     else *rc = launch_attn_g4<K, V, false, false>(P, fk, fv, st);                                                    \
     return true;                                                                                                     \
   }
@@ -32,8 +27,9 @@ bool tq_decode_g4_try(const tqatt::AttnParams& P, const TqFast& fk, const TqFast
     if (!layout_matches<K, V>(P.L)) return false;                                                          \
     /* the four-warp form where four CTAs with two page records each fit an SM */                         \
     if constexpr (4 * (G4<K, V, 4>::SMEM + 1024) <= 228 * 1024) {                                          \
-      if (chain) {                                                                                         \
-        *rc = launch_attn_g4<K, V, false, false, 4>(P, fk, fv, st);                                        \
+      if (w4) {                                                                                            \
+        if (P.tail_late) *rc = launch_attn_g4<K, V, false, false, 4, true>(P, fk, fv, st);                 \
+        else *rc = launch_attn_g4<K, V, false, false, 4>(P, fk, fv, st);                                   \
         return true;                                                                                       \
       }                                                                                                    \
     }                                                                                                      \

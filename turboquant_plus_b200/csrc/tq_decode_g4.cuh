@@ -579,19 +579,26 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     else touch = warp == 6 ? fv.s1[0] : fv.pad[2];
     asm volatile("" ::"r"(touch));
   }
-  // Programmatic dependent launch: let the next kernel in the stream start as soon as SMs free up.  Everything
-  // this kernel does before its griddepcontrol.wait reads only the cache, the block table and the sequence
-  // lengths -- and, when the caller says that the preceding kernel does not write the queries either (q_early),
-  // the queries.  What comes after the wait runs after the preceding kernel has completed and its writes are
-  // visible: the workspace and the output are only ever touched there.  Without q_early the wait stands in front of
-  // the query load; with it, in front of the first write (after the page loop).  Both instructions do nothing in a
-  // launch without the attribute.
-  if (P.overlap) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t raw = smem_u32(smem_raw);
+  uint8_t* sm = smem_raw + (((raw + C::ALIGN - 1) & ~(uint32_t)(C::ALIGN - 1)) - raw);
+  // Programmatic dependent launch (every launch has the attribute, see TQ_PDL_ENTER).  In stream order the CTA fills the
+  // pair tables, waits for the preceding kernel, lets the next one start and only then reads anything.
+  // With an overlap mode the next kernel may start as soon as SMs free up, and everything before this kernel's
+  // griddepcontrol.wait reads only the cache, the block table and the sequence lengths -- and, when the caller says that
+  // the preceding kernel does not write the queries either (q_early), the queries.  What comes after the wait runs after
+  // the preceding kernel has completed and its writes are visible: the workspace and the output are only ever touched
+  // there.  Without q_early the wait stands in front of the query load; with it, in front of the first write (after the
+  // page loop).
+  if (P.overlap) {
+    TQ_PDL_TRIGGER();
+  } else {
+    if constexpr (KB > 0) g4_lut_fill<typename C::KLut, KB>(sm + C::OFF_K, fk.cent16, tid, NT);
+    if constexpr (VB > 0) g4_lut_fill<typename C::VLut, VB>(sm + C::OFF_V, fv.cent16, tid, NT);
+    TQ_PDL_ENTER();
+  }
   const int page_lo = split * P.chunk_pages;
   const size_t row0 = (size_t)b * P.hq + (size_t)kvh * P.group;
   const int32_t* bt = P.block_table + (size_t)b * P.max_pages;
-  const uint32_t raw = smem_u32(smem_raw);
-  uint8_t* sm = smem_raw + (((raw + C::ALIGN - 1) & ~(uint32_t)(C::ALIGN - 1)) - raw);
   uint8_t* smg = sm + C::OFF_GROUPS;
   float* qbuf = reinterpret_cast<float*>(smg + C::G_Q);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smg + C::G_BAR);
@@ -665,7 +672,8 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     if constexpr (NH <= NW) break;
   }
   __syncwarp();
-  if (NW == 4 || NH == 8) {   // every warp may have rotated a query: all of them fill the tables afterwards
+  if (!P.overlap) {   // filled above
+  } else if (NW == 4 || NH == 8) {   // every warp may have rotated a query: all of them fill the tables afterwards
     if constexpr (KB > 0) g4_lut_fill<typename C::KLut, KB>(sm + C::OFF_K, fk.cent16, tid, NT);
     if constexpr (VB > 0) g4_lut_fill<typename C::VLut, VB>(sm + C::OFF_V, fv.cent16, tid, NT);
   } else if (warp >= P.group) {
@@ -865,18 +873,8 @@ int launch_attn_g4(const AttnParams& P, const TqFast& fk, const TqFast& fv, cuda
   memcpy(ak.s1, fk.s1, 16); memcpy(ak.s2, fk.s2, 16); memcpy(ak.j1, fk.j1, 16); memcpy(ak.j2, fk.j2, 16);
   memcpy(ak.cent16, fk.cent16, 32); ak.alpha = fk.lut_alpha;
   memcpy(av.s1, fv.s1, 16); memcpy(av.s2, fv.s2, 16); memcpy(av.cent16, fv.cent16, 32); av.alpha = fv.lut_alpha;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(P.num_splits, P.hkv, P.batch);
-  cfg.blockDim = dim3(32 * NW);
-  cfg.dynamicSmemBytes = C::SMEM;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = P.overlap ? 1 : 0;
-  TQ_CUDA(cudaLaunchKernelEx(&cfg, k_decode_attn_g4<KK, VK, SPARSE, NODEQ, NW, TAIL, NH>, P, ak, av));
+  TQ_CUDA(tq_launch_early(k_decode_attn_g4<KK, VK, SPARSE, NODEQ, NW, TAIL, NH>, dim3(P.num_splits, P.hkv, P.batch), 32 * NW,
+                          C::SMEM, st, P, ak, av));
   return tq_launch_check("k_decode_attn_g4");
 }
 
@@ -888,6 +886,17 @@ bool layout_matches(const tq_cache_layout& L) {
          L.v_scale_off == C::V_SCALE && L.record_bytes == C::REC && L.k_idx_bytes == C::KIDXB && L.v_idx_bytes == C::VIDXB;
 }
 
-inline bool has_4bit_table(int fmt) { return fmt == TQ_FMT_TURBO4; }   // (prod4: 3 bits and the sketch)
+// The form of a call: four-warp CTAs, four per SM, or eight-warp CTAs, two per SM.
+// Four warps pay where CTAs in different phases share an SM -- one in its latency-bound prologue or merge while the others
+// stream pages: in a chain of attention calls (TQ_DECODE_OVERLAP_Q, and the call in front of them when the caller says so,
+// TQ_DECODE_CHAIN_HEAD), and inside a call of more CTAs than one round at two per SM (256 sequences of 8,192 tokens of
+// turbo3: 529 us with eight warps, 457 with four).  A call of one round on its own takes the eight-warp form (16 sequences:
+// 43 against 47 us).  4-bit tables: only the eight-warp form has room for lane-replicated ones, which is worth more (turbo4 /
+// turbo4, 16 sequences of 8,192 tokens, per call of a chain: 62 us with four warps and one copy of the tables, 40 with eight).
+inline bool four_warps(const AttnParams& P) {
+  if (P.L.k_format == TQ_FMT_TURBO4 || P.L.v_format == TQ_FMT_TURBO4) return false;   // (prod4: 3 bits and the sketch)
+  if ((P.q_early || P.chain_head) && !P.tail_late) return true;
+  return (int64_t)P.num_splits * P.hkv * P.batch > 2 * (int64_t)tq_num_sms();
+}
 
 }  // namespace

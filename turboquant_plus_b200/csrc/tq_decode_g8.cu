@@ -4,12 +4,11 @@
 bool tq_decode_g8_try(const tqatt::AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st, int* rc) {
   const int kf = P.L.k_format, vf = P.L.v_format;
   if (P.group > 8) return false;
-  // four-warp form: see tq_decode_g4_try
-  const bool chain = (P.q_early || P.chain_head) && !P.tail_late && !has_4bit_table(kf) && !has_4bit_table(vf);
+  const bool w4 = four_warps(P);
 #define TQ_ATT_G8S(K, V)                                                                                   \
   if (P.sparse_v && kf == K && vf == V) {                                                                  \
     if (!layout_matches<K, V>(P.L)) return false;                                                          \
-    if (chain) *rc = launch_attn_g4<K, V, true, false, 4, false, 8>(P, fk, fv, st);                        \
+    if (w4) *rc = launch_attn_g4<K, V, true, false, 4, false, 8>(P, fk, fv, st);                           \
     else *rc = launch_attn_g4<K, V, true, false, ATT_WARPS, false, 8>(P, fk, fv, st);                      \
     return true;                                                                                           \
   }
@@ -22,8 +21,9 @@ bool tq_decode_g8_try(const tqatt::AttnParams& P, const TqFast& fk, const TqFast
     if (!layout_matches<K, V>(P.L)) return false;                                                          \
     /* where four CTAs with two page records each fit an SM */                                            \
     if constexpr (4 * (G4<K, V, 4, 8>::SMEM + 1024) <= 228 * 1024) {                                       \
-      if (chain) {                                                                                         \
-        *rc = launch_attn_g4<K, V, false, false, 4, false, 8>(P, fk, fv, st);                              \
+      if (w4) {                                                                                            \
+        if (P.tail_late) *rc = launch_attn_g4<K, V, false, false, 4, true, 8>(P, fk, fv, st);              \
+        else *rc = launch_attn_g4<K, V, false, false, 4, false, 8>(P, fk, fv, st);                         \
         return true;                                                                                       \
       }                                                                                                    \
     }                                                                                                      \

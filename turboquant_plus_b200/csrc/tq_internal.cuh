@@ -66,6 +66,40 @@ static inline bool tq_aligned(const void* p, size_t a) { return (reinterpret_cas
 int tq_launch_check(const char* what);
 int tq_num_sms();
 
+// ---- launches that may overlap the kernel in front of them -----------------------------------------------------------
+// Kernels of a decode loop take a few microseconds, as long as a launch and the prologue of a CTA.  They are therefore
+// launched with programmatic stream serialization: the CTAs of a kernel come up and fill their tables while the kernel in
+// front of it is still running, and wait for its completion (and with it everything before it) in front of their first
+// access to memory that others may write.  A kernel lets the next one start only after its own wait (TQ_PDL_ENTER): what
+// runs beside a kernel's early part is then never more than one kernel.
+#define TQ_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
+#define TQ_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
+#define TQ_PDL_ENTER() \
+  do {                 \
+    TQ_PDL_WAIT();     \
+    TQ_PDL_TRIGGER();  \
+  } while (0)
+
+// A pointer made opaque behind the wait: read-only loads (__ldg, const __restrict__) carry no ordering for the compiler,
+// a dependency on this statement keeps them behind it.
+#define TQ_PDL_POINTER(p) asm volatile("" : "+l"(p)::"memory")
+
+template <typename... P, typename... A>
+inline cudaError_t tq_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- device helpers ---------------------------------------------------------------------
 __device__ __forceinline__ float tq_flip(float v, uint32_t bits16, int k) {
   // multiply v by -1 when bit k of bits16 is set
@@ -168,6 +202,10 @@ struct TqQuantDst {
   int32_t page_tokens;  // 0 => plain arrays
   int32_t heads;        // vectors per token in the input
   int32_t rscale_const; // cache mode: store rnorm * sqrt(pi/2)/sqrt(d) so that attention needs one multiply
+  // The kernel in front is the other half of the same append (the K rows; this one does the V rows): it writes nothing
+  // this one reads or writes and everything before it has completed.  This kernel then runs beside it and waits for it
+  // only at its end, so that its own completion stands for both.
+  int32_t beside;
 };
 
 // address of vector v's record field (elem_bytes per token and head) in plain arrays or in a paged cache;
@@ -262,4 +300,4 @@ bool tq_quantize_mma_try_pair(const TqFast& f0, const void* x0, const TqQuantDst
                               const TqQuantDst& d1, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st, int* rc);
 int tq_q8_0_append_launch(const void* x, int32_t dtype, int64_t n_tokens, int32_t heads, uint8_t* q_base,
                           uint8_t* scale_base, const int64_t* slots, int32_t page_tokens,
-                          int64_t page_stride, int64_t head_stride, cudaStream_t st);
+                          int64_t page_stride, int64_t head_stride, bool beside, cudaStream_t st);

@@ -22,9 +22,8 @@
 template <typename Tin, int BITS, bool SYM, bool QJL>
 __global__ void __launch_bounds__(256) k_quantize_wht(const TqFast f, const Tin* __restrict__ x, int64_t ld, int64_t n,
                                                       const TqQuantDst dst) {
-  // a dependent kernel launched with programmatic stream serialization may start now (it waits for this grid's
-  // completion itself before it touches what this grid writes); without such a dependent this does nothing
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (dst.beside) TQ_PDL_TRIGGER(); else TQ_PDL_ENTER();
+  TQ_PDL_POINTER(x);
   constexpr int NC = 1 << BITS, HALF = NC / 2;
   constexpr int IDXB = 16 * BITS;              // packed bytes per vector
   constexpr int GS = BITS == 4 ? 4 : 8;        // indices per fp32 Horner group (GS * BITS <= 24 bits)
@@ -238,6 +237,7 @@ __global__ void __launch_bounds__(256) k_quantize_wht(const TqFast f, const Tin*
     }
     __syncwarp();
   }
+  if (dst.beside) TQ_PDL_WAIT();
 }
 
 template <typename Tin, int BITS, bool SYM>
@@ -247,9 +247,9 @@ static int launch_wht3(const TqFast& f, const Tin* x, int64_t ld, int64_t n, con
   const int64_t cap = (int64_t)tq_num_sms() * 8;
   const int grid = (int)(tiles < cap ? tiles : cap);
   if (qjl)
-    k_quantize_wht<Tin, BITS, SYM, true><<<grid, 256, 0, st>>>(f, x, ld, n, dst);
+    TQ_CUDA(tq_launch_early(k_quantize_wht<Tin, BITS, SYM, true>, grid, 256, 0, st, f, x, ld, n, dst));
   else
-    k_quantize_wht<Tin, BITS, SYM, false><<<grid, 256, 0, st>>>(f, x, ld, n, dst);
+    TQ_CUDA(tq_launch_early(k_quantize_wht<Tin, BITS, SYM, false>, grid, 256, 0, st, f, x, ld, n, dst));
   return tq_launch_check("k_quantize_wht");
 }
 
@@ -643,8 +643,14 @@ template <typename Tin>
 __global__ void __launch_bounds__(256) k_q8_0_append(const Tin* __restrict__ x, int64_t n_vec, int32_t heads,
                                                      uint8_t* q_base, uint8_t* scale_base,
                                                      const int64_t* __restrict__ slots, int32_t page_tokens,
-                                                     int64_t page_stride, int64_t head_stride) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // see k_quantize_wht
+                                                     int64_t page_stride, int64_t head_stride, int32_t beside) {
+  if (beside) {   // see TqQuantDst
+    TQ_PDL_TRIGGER();
+  } else {
+    TQ_PDL_ENTER();
+  }
+  TQ_PDL_POINTER(x);
+  TQ_PDL_POINTER(slots);
   const int lane = threadIdx.x & 31, sub = lane & 7;
   const int64_t v = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 3;
   const bool ok = v < n_vec;
@@ -667,38 +673,41 @@ __global__ void __launch_bounds__(256) k_q8_0_append(const Tin* __restrict__ x, 
     const int qv = (int)roundf(u[k] * id);
     w[k >> 2] |= ((uint32_t)(qv & 0xff)) << (8 * (k & 3));
   }
-  if (!ok) return;
-  const int64_t tok = v / heads;
-  const int32_t head = (int32_t)(v - tok * heads);
-  const int64_t slot = slots ? slots[tok] : tok;
-  if (slot < 0) return;
-  const int64_t page = slot / page_tokens;
-  const int32_t within = (int32_t)(slot - page * page_tokens);
-  const int64_t rec = page * page_stride + head * head_stride;
-  *reinterpret_cast<uint4*>(q_base + rec + (int64_t)within * TQ_D + sub * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-  if ((sub & 1) == 0)
-    *reinterpret_cast<__half*>(scale_base + rec + (int64_t)within * 8 + (sub >> 1) * 2) = __float2half_rn(dd);
+  if (ok) {
+    const int64_t tok = v / heads;
+    const int32_t head = (int32_t)(v - tok * heads);
+    const int64_t slot = slots ? slots[tok] : tok;
+    if (slot >= 0) {
+      const int64_t page = slot / page_tokens;
+      const int32_t within = (int32_t)(slot - page * page_tokens);
+      const int64_t rec = page * page_stride + head * head_stride;
+      *reinterpret_cast<uint4*>(q_base + rec + (int64_t)within * TQ_D + sub * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+      if ((sub & 1) == 0)
+        *reinterpret_cast<__half*>(scale_base + rec + (int64_t)within * 8 + (sub >> 1) * 2) = __float2half_rn(dd);
+    }
+  }
+  if (beside) TQ_PDL_WAIT();
 }
 
 int tq_q8_0_append_launch(const void* x, int32_t dtype, int64_t n_tokens, int32_t heads, uint8_t* q_base,
                           uint8_t* scale_base, const int64_t* slots, int32_t page_tokens, int64_t page_stride,
-                          int64_t head_stride, cudaStream_t st) {
+                          int64_t head_stride, bool beside, cudaStream_t st) {
   const int64_t n_vec = n_tokens * heads;
   if (n_vec == 0) return TQ_OK;
   TQ_REQUIRE(tq_aligned(x, 16), TQ_ERR_ALIGN, "input must be 16-byte aligned");
   const int grid = (int)((n_vec * 8 + 255) / 256);
   switch (dtype) {
     case TQ_F32:
-      k_q8_0_append<float><<<grid, 256, 0, st>>>((const float*)x, n_vec, heads, q_base, scale_base, slots, page_tokens,
-                                                  page_stride, head_stride);
+      TQ_CUDA(tq_launch_early(k_q8_0_append<float>, grid, 256, 0, st, (const float*)x, n_vec, heads, q_base, scale_base, slots, page_tokens,
+                              page_stride, head_stride, (int32_t)beside));
       break;
     case TQ_F16:
-      k_q8_0_append<__half><<<grid, 256, 0, st>>>((const __half*)x, n_vec, heads, q_base, scale_base, slots,
-                                                   page_tokens, page_stride, head_stride);
+      TQ_CUDA(tq_launch_early(k_q8_0_append<__half>, grid, 256, 0, st, (const __half*)x, n_vec, heads, q_base, scale_base, slots, page_tokens,
+                              page_stride, head_stride, (int32_t)beside));
       break;
     case TQ_BF16:
-      k_q8_0_append<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, n_vec, heads, q_base, scale_base,
-                                                          slots, page_tokens, page_stride, head_stride);
+      TQ_CUDA(tq_launch_early(k_q8_0_append<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)x, n_vec, heads, q_base, scale_base, slots, page_tokens,
+                              page_stride, head_stride, (int32_t)beside));
       break;
     default:
       tq_set_error("q8_0 append accepts fp32, fp16 or bf16 input, got dtype %d", dtype);

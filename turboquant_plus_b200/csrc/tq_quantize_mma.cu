@@ -117,9 +117,7 @@ __device__ __forceinline__ float2 qm_dup(float v) { return make_float2(v, v); }
 template <typename Tin, int BITS, bool NORMC, bool QJLS = false>
 __device__ __forceinline__ void qm_body(const TqFast& f, const Tin* __restrict__ x, int64_t ld, int64_t n,
                                         const TqQuantDst& dst, uint8_t* tile) {
-  // a dependent kernel launched with programmatic stream serialization may start now (it waits for this grid's
-  // completion itself before it touches what this grid writes); without such a dependent this does nothing
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (dst.beside) TQ_PDL_TRIGGER();
   constexpr int QM_ROWB = qm_rowb<Tin>();
   constexpr int BUFB = QM_ROWS * QM_ROWB;                      // bytes of one staged tile
   constexpr int CHUNKS = (int)(TQ_D * sizeof(Tin) / 16);       // 16-byte chunks per row
@@ -177,6 +175,7 @@ __device__ __forceinline__ void qm_body(const TqFast& f, const Tin* __restrict__
 #pragma unroll
       for (int c = 0; c < 4; ++c) j2w = (j2w << 1) | qm_bit(f.j2, 16 * i + 4 * t + c);
   }
+  if (!dst.beside) TQ_PDL_ENTER();   // the tables need the parameters only; rows, slots and pages come after
   __syncthreads();
   const uint4* bfr4 = reinterpret_cast<const uint4*>(bsm) + lane;
   // sign2 mirrors an index (i -> 2^b - 1 - i): an XOR of the packed word.  Word tp of this lane packs, most
@@ -602,6 +601,7 @@ __device__ __forceinline__ void qm_body(const TqFast& f, const Tin* __restrict__
     __syncwarp();  // every lane is done with this buffer before the copies of the tile after next land in it
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (dst.beside) TQ_PDL_WAIT();
 }
 
 // staging memory of one CTA (tiles + B operands): 16-bit rows fit the static limit, fp32 rows (72 KB) are dynamic
@@ -671,11 +671,11 @@ int launch_mma(const TqFast& f, const Tin* x, int64_t ld, int64_t n, const TqQua
     if (f.norm_correction) {
       const int rc = qm_dyn_smem<Tin, k_quantize_mma<Tin, BITS, true, true>, true>(&smem);
       if (rc != TQ_OK) return rc;
-      k_quantize_mma<Tin, BITS, true, true><<<gridq, QM_THREADS, smem, st>>>(f, x, ld, n, dst);
+      TQ_CUDA(tq_launch_early(k_quantize_mma<Tin, BITS, true, true>, gridq, QM_THREADS, smem, st, f, x, ld, n, dst));
     } else {
       const int rc = qm_dyn_smem<Tin, k_quantize_mma<Tin, BITS, false, true>, true>(&smem);
       if (rc != TQ_OK) return rc;
-      k_quantize_mma<Tin, BITS, false, true><<<gridq, QM_THREADS, smem, st>>>(f, x, ld, n, dst);
+      TQ_CUDA(tq_launch_early(k_quantize_mma<Tin, BITS, false, true>, gridq, QM_THREADS, smem, st, f, x, ld, n, dst));
     }
     return tq_launch_check("k_quantize_mma");
   }
@@ -684,11 +684,11 @@ int launch_mma(const TqFast& f, const Tin* x, int64_t ld, int64_t n, const TqQua
   if (f.norm_correction && dst.scale) {
     const int rc = qm_dyn_smem<Tin, k_quantize_mma<Tin, BITS, true>>(&smem);
     if (rc != TQ_OK) return rc;
-    k_quantize_mma<Tin, BITS, true><<<grid, QM_THREADS, smem, st>>>(f, x, ld, n, dst);
+    TQ_CUDA(tq_launch_early(k_quantize_mma<Tin, BITS, true>, grid, QM_THREADS, smem, st, f, x, ld, n, dst));
   } else {
     const int rc = qm_dyn_smem<Tin, k_quantize_mma<Tin, BITS, false>>(&smem);
     if (rc != TQ_OK) return rc;
-    k_quantize_mma<Tin, BITS, false><<<grid, QM_THREADS, smem, st>>>(f, x, ld, n, dst);
+    TQ_CUDA(tq_launch_early(k_quantize_mma<Tin, BITS, false>, grid, QM_THREADS, smem, st, f, x, ld, n, dst));
   }
   return tq_launch_check("k_quantize_mma");
 }
@@ -703,11 +703,11 @@ int launch_mma_pair(const QmJob& j0, const QmJob& j1, int64_t ld, int64_t n, boo
   if (normc) {
     const int rc = qm_dyn_smem<Tin, k_quantize_mma_pair<Tin, BITS, true>>(&smem);
     if (rc != TQ_OK) return rc;
-    k_quantize_mma_pair<Tin, BITS, true><<<grid, QM_THREADS, smem, st>>>(j0, j1, ld, n);
+    TQ_CUDA(tq_launch_early(k_quantize_mma_pair<Tin, BITS, true>, grid, QM_THREADS, smem, st, j0, j1, ld, n));
   } else {
     const int rc = qm_dyn_smem<Tin, k_quantize_mma_pair<Tin, BITS, false>>(&smem);
     if (rc != TQ_OK) return rc;
-    k_quantize_mma_pair<Tin, BITS, false><<<grid, QM_THREADS, smem, st>>>(j0, j1, ld, n);
+    TQ_CUDA(tq_launch_early(k_quantize_mma_pair<Tin, BITS, false>, grid, QM_THREADS, smem, st, j0, j1, ld, n));
   }
   return tq_launch_check("k_quantize_mma_pair");
 }
