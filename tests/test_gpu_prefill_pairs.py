@@ -1,0 +1,47 @@
+"""Chunked prefill by pairs of CTAs: one, two, three and many row blocks (an odd last one), chunks whose two blocks of a pair
+see different numbers of pages, several splits, fp32 / fp16 / bf16 rows, against dequantize-then-attend.
+
+Tolerance: that of the attention tests; one sequence per case may show the oracle's own quantization taking a neighbouring
+index (3e-2, derived in test_gpu_decode_heads)."""
+import numpy as np
+import pytest
+
+from oracle import tq_oracle as o
+from tests.helpers import D, fill_cache, max_rel
+from tests.test_gpu_attention import TOL, oracle_roundtrip
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kf,vf", [("turbo3", "turbo3"), ("turbo4", "turbo4"), ("turbo4", "turbo2"), ("q8_0", "q8_0"), ("prod3", "turbo4")])
+@pytest.mark.parametrize("group,chunk,lens", [(1, 128, [300, 128]), (1, 129, [129, 700]), (2, 128, [128, 257]), (8, 48, [40, 4100]),
+                                              (4, 200, [1000, 200]), (8, 81, [81, 2000])])
+def test_prefill_pairs(kf, vf, group, chunk, lens):
+    import torch
+    import turboquant_plus_b200 as tq
+    rng = np.random.default_rng(chunk)
+    hkv = 2
+    cache = tq.PagedKVCache(D, hkv, num_pages=sum(-(-n // 128) for n in lens) + 1, k_format=kf, v_format=vf, seed=42)
+    ks = [rng.standard_normal((n, hkv, D)).astype(np.float32) for n in lens]
+    vs = [rng.standard_normal((n, hkv, D)).astype(np.float32) for n in lens]
+    bt = fill_cache(cache, ks, vs, lens, rng)
+    q = rng.standard_normal((len(lens), chunk, hkv * group, D)).astype(np.float32)
+    qt, lt = torch.as_tensor(q).cuda(), torch.tensor(lens)
+    out = cache.prefill_attend(qt, bt, lt)
+    assert cache.kernel_status() == 0 and torch.equal(out, cache.prefill_attend(qt, bt, lt))
+    for dt in (torch.float16, torch.bfloat16):                 # rows widened exactly, outputs rounded to nearest
+        assert torch.equal(cache.prefill_attend(qt.to(dt), bt, lt), cache.prefill_attend(qt.to(dt).float(), bt, lt).to(dt))
+    errs = []
+    for b, n in enumerate(lens):
+        kh = np.stack([oracle_roundtrip(cache, ks[b][:, h], "k") for h in range(hkv)])[None]
+        vh = np.stack([oracle_roundtrip(cache, vs[b][:, h], "v") for h in range(hkv)])[None]
+        lo = max(0, chunk - n)
+        some = np.unique(np.concatenate([[lo, chunk - 1], rng.integers(lo, chunk, 24)]))     # the oracle is slow
+        got = out[b].cpu().numpy()
+        assert not got[:lo].any()
+        for i in some:
+            m = n - chunk + i + 1
+            ref = o.attend_gqa(q[b, i][None].astype(np.float64), kh[:, :, :m], vh[:, :, :m], [m])[0]
+            errs.append((max_rel(got[i], ref), b))
+    worst = sorted((max(e for e, bb in errs if bb == b)) for b in range(len(lens)))
+    assert worst[0] < TOL and worst[-1] < 3e-2, f"{kf}/{vf}: {worst}"

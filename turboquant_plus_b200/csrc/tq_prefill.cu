@@ -12,7 +12,7 @@
 
 namespace {
 
-constexpr int PF_ROWS = 128;
+constexpr int PF_ROWS = 128, PF_PAGE = 128;   // rows of a CTA, tokens of a page
 constexpr long long PF_WAIT_CYCLES = 1LL << 30;
 
 __device__ __forceinline__ uint32_t sptr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -44,12 +44,49 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint3
 __device__ __forceinline__ uint32_t umma_idesc(int m, int n, bool b_mn_major) {
   return (1u << 4) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+// CG CTAs on one tile: with two, the accumulator's rows 0-127 are the even CTA's tensor memory and 128-255 the odd one's,
+// A likewise, and each CTA's shared memory holds its half of B's columns (N) at the same offsets.  Executed by a whole warp
+// of the even CTA, one elected thread of which issues it: the warp stays converged, so that addresses and descriptors live
+// in uniform registers, which is where the instruction wants them (issued from a branch of one thread, every MMA spent
+// some 75 cycles moving its operands there).
+template <int CG> __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+  if constexpr (CG == 1)
+    asm volatile("{\n .reg .pred p, q;\n elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+  else
+    asm volatile("{\n .reg .pred p, q;\n elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n @q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sptr(bar)) : "memory");
+// arrival on `bar` of every CTA of the pair once the MMAs issued so far have completed
+template <int CG> __device__ __forceinline__ void umma_commit(uint64_t* bar) {
+  if constexpr (CG == 1)
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(sptr(bar)) : "memory");
+  else
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n @q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n"
+                 ::"r"(sptr(bar)), "h"((uint16_t)3) : "memory");
+}
+// all 512 columns of tensor memory, by one warp of each CTA of the pair
+template <int CG> __device__ __forceinline__ void tmem_alloc_all(uint32_t* where) {
+  if constexpr (CG == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sptr(where)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sptr(where)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+}
+template <int CG> __device__ __forceinline__ void tmem_free_all(uint32_t base) {
+  if constexpr (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512u) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512u) : "memory");
+}
+// every thread of the CTA, or of both CTAs of the pair
+template <int CG> __device__ __forceinline__ void pf_sync_all() {
+  if constexpr (CG == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  }
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
   asm volatile(
@@ -58,14 +95,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
         "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
         "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
         "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(addr) : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(addr) : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -180,39 +209,63 @@ template <int KIND> struct PfKind {
   // scale is 19 bits, so its fp16 rounding and the rest, exactly.  PROD: centroids, then +-ratio for the sketch, ratio =
   // residual scale / row scale (one row scale then serves both parts), as its fp16 rounding and the rest of it.
   static constexpr int TILES = PROD ? 3 : (Q8 ? 2 : 1);
-  // more than one tile per page: one buffer of them instead of two
-  static constexpr int KBUF = TILES == 1 ? 2 : 1;
   // PROD queries (rotated and projected, hi and lo) take 256 tensor-memory columns: one score buffer instead of two
   static constexpr int SBUF = PROD ? 1 : 2;
 };
 
-template <int BITS> struct PfLut {
+// Pair tables, replicated per lane (a lookup then hits the lane's own bank) up to 8 KB; the 256 pairs of a 4-bit codebook
+// only where 32 KB are to be had (REPL4: with one copy a lookup takes 3.4 wavefronts on average).  Tables up to 8 KB start on
+// a multiple of their size, the address of an entry is (field | base); the 32 KB one's start is added.
+template <int BITS, bool REPL4> struct PfLut {
   static constexpr int ENTRIES = BITS ? 1 << (2 * BITS) : 0;
-  static constexpr bool REPL = ENTRIES <= 64;
+  static constexpr bool BIG = BITS == 4 && REPL4;
+  static constexpr bool REPL = BIG || ENTRIES <= 64;
   static constexpr int SHIFT = REPL ? 7 : 2;
   static constexpr int BYTES = ENTRIES << SHIFT;
+  static __device__ __forceinline__ uint32_t load(uint32_t field, uint32_t base, uint32_t start) {
+    return pf_lds(BIG ? (field | base) + start : field | base);
+  }
+  static __device__ __forceinline__ uint32_t base(uint32_t start, int lane) { return (BIG ? 0u : start) + (REPL ? lane * 4 : 0); }
+  static __device__ __forceinline__ void fill(uint8_t* lut, const uint16_t* c16, int tid, int threads) {
+    if constexpr (BITS > 0)
+      for (int i = tid; i < BYTES / 16; i += threads) {
+        uint32_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int e = REPL ? i >> 3 : 4 * i + k;
+          v[k] = (uint32_t)c16[e >> BITS] | ((uint32_t)c16[e & ((1 << BITS) - 1)] << 16);
+        }
+        reinterpret_cast<uint4*>(lut)[i] = make_uint4(v[0], v[1], v[2], v[3]);
+      }
+  }
 };
 
-// One token's packed indices (16*BITS bytes at `src`) -> 128 fp16 values written as sixteen 16-byte rows of the
-// operand tile: chunk c (dims 8c..8c+7) goes to tile + c*128 (+ the token's row offset, already in `dst`).
-// SCALED: every pair is multiplied by `scale2` (one fp16 factor in both halves) on its way to the tile.
-template <int BITS, bool SCALED = false>
-__device__ __forceinline__ void pf_dequant_token(const uint8_t* src, uint8_t* dst, uint32_t lut_base, uint32_t scale2 = 0) {
-  constexpr int SH = PfLut<BITS>::SHIFT;
+// DIMS of one token's packed indices (DIMS * BITS / 8 bytes at `src`) -> fp16 values written as 16-byte rows of the operand
+// tile: chunk c (8 dims) goes to dst + c*128.  SCALED: every pair is multiplied by `scale2` (one fp16 factor in both halves).
+template <int BITS, class LUT, int DIMS, bool SCALED = false>
+__device__ __forceinline__ void pf_dequant_token(const uint8_t* src, uint8_t* dst, uint32_t lut_base, uint32_t lut_start,
+                                                 uint32_t scale2 = 0) {
+  constexpr int SH = LUT::SHIFT;
   constexpr uint32_t MASK = ((1u << (2 * BITS)) - 1) << SH;
-  constexpr int NW = 4 * BITS;  // 32-bit words per token
-  const uint4* s4 = reinterpret_cast<const uint4*>(src);
+  constexpr int NW = DIMS * BITS / 32;  // 32-bit words
   uint32_t w[NW];
+  if constexpr (DIMS == 128) {
 #pragma unroll
-  for (int i = 0; i < BITS; ++i) {
-    const uint4 v = s4[i];
-    w[4 * i] = __byte_perm(v.x, 0, 0x0123);
-    w[4 * i + 1] = __byte_perm(v.y, 0, 0x0123);
-    w[4 * i + 2] = __byte_perm(v.z, 0, 0x0123);
-    w[4 * i + 3] = __byte_perm(v.w, 0, 0x0123);
+    for (int i = 0; i < BITS; ++i) {
+      const uint4 v = reinterpret_cast<const uint4*>(src)[i];
+      w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < BITS; ++i) {
+      const uint2 v = reinterpret_cast<const uint2*>(src)[i];
+      w[2 * i] = v.x; w[2 * i + 1] = v.y;
+    }
   }
 #pragma unroll
-  for (int c = 0; c < 16; ++c) {
+  for (int i = 0; i < NW; ++i) w[i] = __byte_perm(w[i], 0, 0x0123);
+#pragma unroll
+  for (int c = 0; c < DIMS / 8; ++c) {
     uint32_t o4[4];
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
@@ -224,13 +277,12 @@ __device__ __forceinline__ void pf_dequant_token(const uint8_t* src, uint8_t* ds
       } else {
         f = __funnelshift_l(w[k + 1 < NW ? k + 1 : k], w[k], o) >> (32 - 2 * BITS - SH);
       }
-      o4[p] = pf_lds((f & MASK) | lut_base);   // the table starts on a multiple of its size: one logic instruction
+      o4[p] = LUT::load(f & MASK, lut_base, lut_start);
       if constexpr (SCALED) asm("mul.f16x2 %0, %0, %1;" : "+r"(o4[p]) : "r"(scale2));
     }
     *reinterpret_cast<uint4*>(dst + c * 128) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
   }
 }
-
 
 __device__ __forceinline__ uint32_t pf_s8x2(uint32_t biased, uint32_t sel) {
   // two int8 values, stored as value ^ 0x80 = value + 128, as exact fp16: (b | 0x6400) is 1024 + b; subtract 1152
@@ -239,14 +291,14 @@ __device__ __forceinline__ uint32_t pf_s8x2(uint32_t biased, uint32_t sel) {
   return d;
 }
 
-// One token's 128 int8 values at `src` with its four block scales (sc01, sc23: two fp16 each) -> fp16 products in the
-// operand tile at `dst`, and, SPLIT, what the fp16 rounding left of them (exact: 8 x 11 bits) in the tile at dst + 32 KB.
+// One token's DIMS int8 values at `src` with their block scales (sc01, sc23: two fp16 each) -> fp16 products in the
+// operand tile at `dst`, and, SPLIT, what the fp16 rounding left of them (exact: 8 x 11 bits) in the tile at dst + TILE.
 // Rows are 128 bytes apart, so a lane starts at a chunk of its own: the lanes of a load then touch every bank.
-template <bool SPLIT>
+template <bool SPLIT, int DIMS, int TILE>
 __device__ __forceinline__ void pf_q8_token(const uint8_t* src, uint8_t* dst, uint32_t sc01, uint32_t sc23, int lane) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int c = (i + lane) & 7;   // 16 values: dims 16 c .. 16 c + 15, half of block c >> 1
+  for (int i = 0; i < DIMS / 16; ++i) {
+    const int c = (i + lane) & (DIMS / 16 - 1);   // 16 values: dims 16 c .. 16 c + 15, half of block c >> 1
     const uint4 v = *reinterpret_cast<const uint4*>(src + 16 * c);
     const uint32_t w[4] = {v.x ^ 0x80808080u, v.y ^ 0x80808080u, v.z ^ 0x80808080u, v.w ^ 0x80808080u};
     const uint32_t s2 = __byte_perm(c & 4 ? sc23 : sc01, 0, c & 2 ? 0x3232 : 0x1010);
@@ -261,21 +313,28 @@ __device__ __forceinline__ void pf_q8_token(const uint8_t* src, uint8_t* dst, ui
     *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(d + 128) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
     if constexpr (SPLIT) {
-      *reinterpret_cast<uint4*>(d + 32768) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-      *reinterpret_cast<uint4*>(d + 32768 + 128) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+      *reinterpret_cast<uint4*>(d + TILE) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      *reinterpret_cast<uint4*>(d + TILE + 128) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
     }
   }
 }
 
-// One token's 16-byte sign sketch (first dim in the most significant bit, set = +1) -> +-ratio in the tile at `dst`, as
+// One token's sign sketch, DIMS bits (first dim in the most significant bit, set = +1) -> +-ratio in the tile at `dst`, as
 // the fp16 rounding of the ratio there and the rest of it in the tile behind.
-__device__ __forceinline__ void pf_sketch_token(uint4 z, uint8_t* dst, float ratio) {
+template <int DIMS, int TILE>
+__device__ __forceinline__ void pf_sketch_token(const uint8_t* src, uint8_t* dst, float ratio) {
   const __half h = __float2half_rn(ratio);
   const __half2 h2 = __half2half2(h), e2 = __float2half2_rn(ratio - __half2float(h));
   const uint32_t hw = *reinterpret_cast<const uint32_t*>(&h2), ew = *reinterpret_cast<const uint32_t*>(&e2);
-  const uint32_t zw[4] = {z.x, z.y, z.z, z.w};
+  uint32_t zw[DIMS / 32];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < DIMS / 64; ++k) {
+    const uint2 v = reinterpret_cast<const uint2*>(src)[k];
+    zw[2 * k] = v.x;
+    zw[2 * k + 1] = v.y;
+  }
+#pragma unroll
+  for (int k = 0; k < DIMS / 32; ++k) {
     const uint32_t n = ~__byte_perm(zw[k], 0, 0x0123);   // set = negative; dim 32 k + i in bit 31 - i
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -288,58 +347,88 @@ __device__ __forceinline__ void pf_sketch_token(uint4 z, uint8_t* dst, float rat
       }
       uint8_t* d = dst + (4 * k + c) * 128;
       *reinterpret_cast<uint4*>(d) = make_uint4(hw ^ m[0], hw ^ m[1], hw ^ m[2], hw ^ m[3]);
-      *reinterpret_cast<uint4*>(d + 32768) = make_uint4(ew ^ m[0], ew ^ m[1], ew ^ m[2], ew ^ m[3]);
+      *reinterpret_cast<uint4*>(d + TILE) = make_uint4(ew ^ m[0], ew ^ m[1], ew ^ m[2], ew ^ m[3]);
     }
   }
 }
 
 // ------------------------------------------------------------------------------------------
-// k_prefill_attn2: the work split over specialised warps (one CTA per SM, 544 threads):
+// k_prefill_attn2: the work split over specialised warps, one CTA per SM.
+//
+// Two CTAs of a cluster take two neighbouring row blocks over one range of pages (CG = 2): tcgen05.mma.cta_group::2 multiplies
+// both blocks with one operand tile of which each CTA holds half, so that each dequantizes half of every page.  Alone (CG =
+// 1: a single row block, PROD keys) a CTA dequantizes the whole page, and the shared-memory pipe -- tiles written, read by
+// the tensor core, table lookups -- is busy 92 % of a page's ~3,000 cycles.  In a pair it is half as busy, and a page takes
+// ~2,500 cycles: the row warps' softmax (2,250: 16 KB of scores read, maxima exchanged, 64 exponentials per thread) and the
+// MMAs (1,536 at the tensor core's rate, ~2,100 as issued) are the two limits.  Measured per page and CTA: turbo3 / turbo3
+// 1.64 -> 1.37 us, turbo4 / turbo3 2.1 -> 1.4 (with lane-replicated 4-bit tables, for which a pair has room), turbo4 /
+// turbo4 2.5 -> 1.4, q8_0 / turbo2 2.1 -> 1.7.
 //   warps 0-7  rows: two threads per row r = lane r of tensor memory (warps w and w + 4 reach the same 32 lanes), one
 //              per half of a page's 128 score columns: reads S, online softmax (the halves exchange their maxima
 //              through shared memory), writes P, rescales its half of O (lazily: only when the row maximum grows by
 //              more than 2^4); both threads share the query rotation, the split partial, the merge and the output
 //              (64 elements each; query and output rows pass through shared memory and the partials are laid out
 //              by warp, so that every global access of a warp covers whole lines);
-//   warps 8-11 K producers: thread t dequantizes the K row of token t of the page into a double-buffered operand tile
-//              and copies its scale; they wait for the score MMA of page i - 2 only, one page ahead of
-//   warps 12-15 V producers: the V row of token t times its V scale; their tile is free after the product of page
-//              i - 2; one of them issues the bulk copies of the page records;
-//   warp 16    one lane issues every tcgen05.mma: S_{i+1} = Q K_{i+1}^T is queued before O += P_i V_i, so the
-//              tensor core works on the next page while the row warps are in the softmax of this one.
-// (With one warp per row quarter and one per token quarter -- nine warps -- a page took 4,350 cycles.  Seventeen warps
-// alone changed nothing: the time went into executed instructions -- a causal mask evaluated on every page, scalar
-// fp32 arithmetic, polling loops -- and into the K producers waiting for the product of page i - 2 when the score MMA
-// was all they needed.  Now ~3,300 cycles, against 1,536 of tensor work; the shared-memory pipe is the next limit.)
+//   PW warps   K producers: a thread dequantizes the K row of one token of the page into a double-buffered operand tile;
+//              they wait for the score MMA of page i - 2 only, one page ahead of
+//   PW warps   V producers: V rows times the V scale; their tile is free after the product of page i - 2;
+//   one warp   issues every tcgen05.mma (the even CTA's, for both): S_{i+1} = Q K_{i+1}^T is queued before O += P_i V_i, so
+//              that the tensor core works on the next page while the row warps are in the softmax of this one;
+//   one warp   issues the bulk copies of the page records.
 // Tensor memory, all 512 columns: Q hi 0-63 | Q lo 64-127 | S0 128-255 | S1 256-383 | O 384-511 (fp32, accumulated
 // by the MMAs across pages); PROD keys: the projected queries' hi and lo in 128-255 and one score buffer in 256-383.
-// q8_0 and PROD keys have two and three K tiles per page (PfKind), one buffer of them, and sum 3 and 5 products into S:
-// their queries' chunk runs here instead of one decode call per query, which read and dequantized the cache once per
-// query (2 x 128 queries x 32 heads over 8,192 tokens of q8_0 / turbo2: 650 us).  P overlays the first 64 columns of its S buffer.  Hand-offs are mbarriers (counts in
-// brackets): k_ready/v_ready [128 producer arrivals], s_full/o_done [tcgen05.commit], p_ready [128 row arrivals];
-// buffer b of page i completes each of them for the (i >> 1)-th time, which fixes the parity to wait for.  Every
-// wait is bounded; a role that gives up raises the CTA's fail flag, the others see it or run out of time
-// themselves, and the tensor memory is released on every path.
+// P overlays the first 64 columns of its S buffer.
+// q8_0 and PROD keys have two and three K tiles per page (PfKind) and sum 3 and 5 products into S: their queries' chunk runs
+// here instead of one decode call per query, which read and dequantized the cache once per query (2 x 128 queries x 32
+// heads over 8,192 tokens of q8_0 / turbo2: 650 us).
+// Hand-offs are mbarriers (counts in brackets, times the CTAs of a pair where they count for both): k_ready/v_ready [PW
+// producer warps], s_full/o_done [tcgen05.commit, to both CTAs], p_ready [8 row warps], rec_free [2 PW producer warps];
+// buffer b of page i completes each of the first five for the (i >> 1)-th time, which fixes the parity to wait for.  No
+// generic-proxy data crosses the CTAs (scales, maxima and records are each CTA's own), so arrivals at the other CTA carry
+// no cluster-wide fence: with acquire and release at cluster scope a page took 0.4 us longer.  Every wait is bounded; a
+// role that gives up raises the CTA's fail flag, the others see it or run out of time themselves, and the tensor memory
+// is released on every path.
+// Tried without gain: probabilities formed ahead of the exchanged maximum; a part of the exponentials as polynomials on the
+// fp32 pipe (one pair in two to one in six).
 // ------------------------------------------------------------------------------------------
-constexpr int PF2_THREADS = 544;
 constexpr float PF2_SLACK = 4.0f;
 
-template <int KK, int VK> struct PfSmem2 {
-  static constexpr int ALIGN = 8192;                    // each table starts on a multiple of its size (at most 8 KB)
+// CG: CTAs per operand tile (1, or a pair of 2)
+template <int KK, int VK, int CG> struct PfSmem2 {
+  using KT = PfKind<KK>;
+  using VT = PfKind<VK>;
+  // Producer warps of K and of V.  A pair's CTA dequantizes half as much and gets by with two each: 14 warps then, at most
+  // four per scheduler, which leaves the row warps 128 registers (96 with 17 to 20 warps).
+  static constexpr int PW = CG == 2 ? 2 : 4;
+  static constexpr int K_AT = 256, V_AT = K_AT + 32 * PW, MMA_AT = V_AT + 32 * PW, COPIER = MMA_AT + 32, THREADS = COPIER + 32;
+  static constexpr bool REPL4 = CG == 2;
+  using KLut = PfLut<KT::BITS, REPL4>;
+  using VLut = PfLut<VT::BITS, REPL4>;
+  static constexpr int TILE = 32768 / CG;               // one operand tile: this CTA's half of it in a pair
+  static constexpr int KBUF = CG == 2 || KT::TILES == 1 ? 2 : 1;   // buffers of K tiles
+  static constexpr int REC = 128 * ((KT::Q8 ? 136 : 16 * KT::BITS + 4) + (KT::PROD ? 20 : 0) + (VT::Q8 ? 136 : 16 * VT::BITS + 4));
+  static constexpr int ALIGN = 8192;                    // each table starts on a multiple of its size (or of 8 KB)
   static constexpr int OFF_K = 0;
-  static constexpr int OFF_V = 8192;
-  static constexpr int OFF_BAR = 16384;              // 12 mbarriers, tensor-memory base, fail flag, 4 exchange mbarriers
+  static constexpr int OFF_V = KLut::BYTES > 8192 ? KLut::BYTES : 8192;
+  static constexpr int OFF_BAR = OFF_V + (VLut::BYTES > 8192 ? VLut::BYTES : 8192);   // mbarriers, tensor-memory base, fail flag
   static constexpr int OFF_SC = OFF_BAR + 256;          // float K scales[4 slots][128 tokens], then the row halves'
                                                         // exchange area float[2 buffers][2 halves][128 rows], then
                                                         // their parts of the row sum float[2 halves][128 rows]
-  static constexpr int OFF_KT = OFF_SC + 5120;          // K operand tiles, 32 KB each
-  static constexpr int OFF_VT = OFF_KT + PfKind<KK>::KBUF * PfKind<KK>::TILES * 32768;   // V operand tiles, two
-  static constexpr int OFF_ST = OFF_VT + 65536;         // two page records
-  static size_t bytes(int record_bytes) { return (size_t)ALIGN + OFF_ST + 2 * (size_t)record_bytes; }
+  static constexpr int OFF_KT = OFF_SC + 5120;          // K operand tiles (the first 64 KB from here also stage the rows)
+  static constexpr int OFF_VT = OFF_KT + KBUF * KT::TILES * TILE;   // V operand tiles, two
+  static constexpr int OFF_ST = OFF_VT + 2 * TILE;      // page records in flight: as many as fit, at most four
+  static constexpr int LIMIT = 227 * 1024;
+  static constexpr int NST_FIT = (LIMIT - ALIGN - OFF_ST) / REC;
+  static constexpr int NST = CG == 1 ? 2 : NST_FIT > 4 ? 4 : NST_FIT;
+  static constexpr int BYTES = ALIGN + OFF_ST + NST * REC;
+  static_assert(NST >= 2 && BYTES <= LIMIT && OFF_ST - OFF_KT >= 65536, "shared memory of the prefill kernel");
 };
 
-__device__ __forceinline__ void pf_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sptr(bar)) : "memory");
+// One arrival for a whole warp: its lanes' earlier accesses are ordered in front of it by the warp barrier.  (An arrival
+// per thread is an operation of the shared-memory pipe per thread, 768 per page.)
+__device__ __forceinline__ void pf_arrive_warp(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sptr(bar)) : "memory");
 }
 __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]) {
   asm volatile(
@@ -349,121 +438,105 @@ __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]
         "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
         "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
 }
+// ... on the barrier of the CTA that issues the MMAs: the even one of a pair
+template <int CG> __device__ __forceinline__ void pf_arrive_leader(uint64_t* bar, int lane) {
+  if constexpr (CG == 1) {
+    pf_arrive_warp(bar, lane);
+  } else {
+    __syncwarp();
+    if (lane == 0) {
+      uint32_t addr;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(addr) : "r"(sptr(bar)));
+      asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+    }
+  }
+}
 // bounded wait whose verdict is the same in every lane of the warp (warp-collective tcgen05 instructions follow)
 __device__ __forceinline__ bool pf_wait_warp(uint64_t* bar, uint32_t parity) {
   return __all_sync(0xffffffffu, pf_wait(bar, parity));
 }
-// AND of a predicate over the 128 V producer threads (named barrier 1)
-__device__ __forceinline__ bool producers_all(bool ok) {
-  uint32_t r;
-  asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n bar.red.and.pred q, 1, 128, p;\n selp.u32 %0, 1, 0, q;\n}\n"
-               : "=r"(r) : "r"((uint32_t)ok) : "memory");
-  return r != 0;
-}
-
-template <int KK, int VK>
-__global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillParams P, const TqFast fk, const TqFast fv) {
-  using SP = PfSmem2<KK, VK>;
+template <int KK, int VK, int CG>
+__global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_attn2(const __grid_constant__ PrefillParams P,
+                                                                  const __grid_constant__ TqFast fk, const __grid_constant__ TqFast fv) {
+  using SP = PfSmem2<KK, VK, CG>;
   using KT = PfKind<KK>;
   using VT = PfKind<VK>;
-  constexpr int KB = KT::BITS, VB = VT::BITS;
+  constexpr int KB = KT::BITS, VB = VT::BITS, NST = SP::NST;
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  const int rb = blockIdx.x / P.num_splits, split = blockIdx.x - rb * P.num_splits, kvh = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int PT = P.L.page_tokens;  // 128 (checked on the host)
-  const int kv_len = P.kv_lens[b];
-  const int nrows = P.tq * P.group;
-  const int rtid = tid & 127;                        // row (warps 0-7) or token (warps 8-15) this thread serves
-  const int row = rb * PF_ROWS + rtid;
-  const bool is_row = tid < 256, is_prod = tid >= 256 && tid < 512;
-  const bool is_prim = tid < 128;                    // the row thread that stages the query and writes the output
-  const int hf = (tid >> 7) & 1;                     // row threads: half of a page's columns; producers: 0 = K, 1 = V
-  const bool row_ok = is_row && row < nrows;
-  const int qi = row_ok ? row / P.group : 0, hl = row_ok ? row - qi * P.group : 0;
-  const int pos = row_ok ? kv_len - P.tq + qi : -1;
-  const int last_row = min(nrows, (rb + 1) * PF_ROWS) - 1;
-  const int pos_max = kv_len - P.tq + last_row / P.group;
-  const int np_all = min(P.max_pages, pos_max >= 0 ? pos_max / PT + 1 : 0);
-  const int ns = np_all > 0 ? (np_all + P.chunk_pages - 1) / P.chunk_pages : 1;
-  if (split >= ns) return;                           // nothing to do, and no tensor memory taken yet
-  const int page_lo = split * P.chunk_pages;
-  const int np = max(0, min(np_all, page_lo + P.chunk_pages) - page_lo);
-
   const uint32_t raw = sptr(smem_raw);
   uint8_t* sm = smem_raw + (((raw + SP::ALIGN - 1) & ~(uint32_t)(SP::ALIGN - 1)) - raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + SP::OFF_BAR);
-  uint64_t *rec_full = bars, *k_ready = bars + 2, *v_ready = bars + 4, *s_full = bars + 6, *p_ready = bars + 8,
-           *o_done = bars + 10;
-  uint64_t* xbar = bars + 16;   // one per row quarter: both halves' maxima of a page are in shared memory [64 arrivals]
-  uint32_t* tbase = reinterpret_cast<uint32_t*>(sm + SP::OFF_BAR + 96);
-  volatile int* fail = reinterpret_cast<volatile int*>(sm + SP::OFF_BAR + 104);
+  // (k_ready, v_ready, p_ready and q_ready count in the even CTA of a pair)
+  uint64_t *rec_full = bars, *rec_free = bars + 4, *k_ready = bars + 8, *v_ready = bars + 10, *s_full = bars + 12,
+           *p_ready = bars + 14, *o_done = bars + 16, *q_ready = bars + 18;
+  uint64_t* xbar = bars + 19;   // one per row quarter: both halves' maxima of a page are in shared memory [2 warps]
+  uint32_t* tbase = reinterpret_cast<uint32_t*>(sm + SP::OFF_BAR + 224);
+  volatile int* fail = reinterpret_cast<volatile int*>(sm + SP::OFF_BAR + 232);
+  if (tid == SP::COPIER) {   // lane 0 of the last warp issues the record copies
+    auto init = [](uint64_t* bar, int count) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sptr(bar)), "r"(count) : "memory");
+    };
+    for (int i = 0; i < NST; ++i) {
+      init(&rec_full[i], 1);
+      init(&rec_free[i], 2 * SP::PW);
+    }
+    for (int i = 0; i < 2; ++i) {
+      init(&k_ready[i], SP::PW * CG);
+      init(&v_ready[i], SP::PW * CG);
+      init(&p_ready[i], 8 * CG);
+      init(&s_full[i], 1);
+      init(&o_done[i], 1);
+    }
+    for (int i = 0; i < 4; ++i) init(&xbar[i], 2);
+    init(q_ready, 8 * CG);
+    *fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  SP::KLut::fill(sm + SP::OFF_K, fk.cent16, tid, SP::THREADS);
+  SP::VLut::fill(sm + SP::OFF_V, fv.cent16, tid, SP::THREADS);
+  TQ_PDL_ENTER();   // so far only the parameters have been read
+
+  // Row blocks from the last to the first: the later ones of a causal chunk see more pages, and what is left when the SMs
+  // run dry should be short.  A pair's CTAs take two neighbouring blocks over one range of pages.
+  const int unit = blockIdx.x / CG, per = P.batch * P.hkv * P.num_splits, crank = CG == 2 ? (int)(blockIdx.x & 1) : 0;
+  const int rbp = (P.row_blocks + CG - 1) / CG - 1 - unit / per, item = unit % per;
+  const int split = item % P.num_splits, kvh = item / P.num_splits % P.hkv, b = item / (P.num_splits * P.hkv);
+  const int rb = rbp * CG + crank;
+  const int PT = P.L.page_tokens;  // 128 (checked on the host)
+  const int kv_len = P.kv_lens[b];
+  const int nrows = P.tq * P.group;
+  const int rtid = tid & 127;                        // row of a row thread
+  const int row = rb * PF_ROWS + rtid;
+  const bool is_row = tid < SP::K_AT;
+  const bool is_prim = tid < 128;
+  const int hf = (tid >> 7) & 1;                     // row threads: half of a page's columns
+  const bool row_ok = is_row && row < nrows;
+  const int qi = row_ok ? row / P.group : 0;
+  const int pos = row_ok ? kv_len - P.tq + qi : -1;
+  const int last_row = min(nrows, (rbp + 1) * CG * PF_ROWS) - 1;
+  const int pos_max = kv_len - P.tq + last_row / P.group;
+  const int np_all = min(P.max_pages, pos_max >= 0 ? pos_max / PT + 1 : 0);
+  const int ns = np_all > 0 ? (np_all + P.chunk_pages - 1) / P.chunk_pages : 1;
+  if (split >= ns) return;                           // nothing to do (for both CTAs of a pair), and no tensor memory taken yet
+  const int page_lo = split * P.chunk_pages;
+  const int np = max(0, min(np_all, page_lo + P.chunk_pages) - page_lo);
   float* scales = reinterpret_cast<float*>(sm + SP::OFF_SC);
   uint8_t* ktile = sm + SP::OFF_KT;
   uint8_t* vtile = sm + SP::OFF_VT;
   uint8_t* stage0 = sm + SP::OFF_ST;
-  const uint32_t rec = (uint32_t)P.L.record_bytes;
-  const int32_t* bt = P.block_table + (size_t)b * P.max_pages;
+  if (warp == 0) tmem_alloc_all<CG>(tbase);          // all 512 columns of the SM (one CTA per SM)
 
   auto issue = [&](int i) {
-    const int64_t page = bt[page_lo + i];
+    const int64_t page = P.block_table[(size_t)b * P.max_pages + page_lo + i];
     const uint8_t* src = P.pool + page * P.L.page_stride + (int64_t)kvh * P.L.head_stride;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(&rec_full[i & 1])), "r"(rec) : "memory");
+    const int st = i % NST;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(&rec_full[st])), "r"(SP::REC) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     sptr(stage0 + (size_t)(i & 1) * rec)), "l"(src), "r"(rec), "r"(sptr(&rec_full[i & 1])) : "memory");
+                     sptr(stage0 + st * SP::REC)), "l"(src), "r"(SP::REC), "r"(sptr(&rec_full[st])) : "memory");
   };
-  if (tid == 256) {
-    for (int i = 0; i < 2; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sptr(&rec_full[i])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(sptr(&k_ready[i])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(sptr(&v_ready[i])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sptr(&s_full[i])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(sptr(&p_ready[i])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sptr(&o_done[i])) : "memory");
-    }
-    for (int i = 0; i < 4; ++i)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 64;" ::"r"(sptr(&xbar[i])) : "memory");
-    *fail = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (np > 0) issue(0);
-    if (np > 1) issue(1);
-  }
-  if (warp == 0) {  // tensor memory: all 512 columns of the SM (one CTA per SM)
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sptr(tbase)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (!is_prim) {
-    // table fill by the 416 threads that do not rotate a query
-    for (int i = tid - 128; KB && i < PfLut<KB>::BYTES / 16; i += PF2_THREADS - 128) {
-      if (PfLut<KB>::REPL) {
-        const int e = i >> 3;
-        const uint32_t v = (uint32_t)fk.cent16[e >> KB] | ((uint32_t)fk.cent16[e & ((1 << KB) - 1)] << 16);
-        reinterpret_cast<uint4*>(sm + SP::OFF_K)[i] = make_uint4(v, v, v, v);
-      } else {
-        uint32_t v[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int e = 4 * i + k;
-          v[k] = (uint32_t)fk.cent16[e >> KB] | ((uint32_t)fk.cent16[e & ((1 << KB) - 1)] << 16);
-        }
-        reinterpret_cast<uint4*>(sm + SP::OFF_K)[i] = make_uint4(v[0], v[1], v[2], v[3]);
-      }
-    }
-    for (int i = tid - 128; VB && i < PfLut<VB>::BYTES / 16; i += PF2_THREADS - 128) {
-      if (PfLut<VB>::REPL) {
-        const int e = i >> 3;
-        const uint32_t v = (uint32_t)fv.cent16[e >> VB] | ((uint32_t)fv.cent16[e & ((1 << VB) - 1)] << 16);
-        reinterpret_cast<uint4*>(sm + SP::OFF_V)[i] = make_uint4(v, v, v, v);
-      } else {
-        uint32_t v[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int e = 4 * i + k;
-          v[k] = (uint32_t)fv.cent16[e >> VB] | ((uint32_t)fv.cent16[e & ((1 << VB) - 1)] << 16);
-        }
-        reinterpret_cast<uint4*>(sm + SP::OFF_V)[i] = make_uint4(v[0], v[1], v[2], v[3]);
-      }
-    }
-  }
+  if (tid == SP::COPIER)
+    for (int i = 0; i < NST && i < np; ++i) issue(i);
 
   if constexpr (KT::PROD) {   // both transforms of a row share registers and staging: the first goes to tensor memory first
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -477,21 +550,38 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
   const uint32_t TQc = 0, TQLc = 64, TPc = 128, TPLc = 192, TOc = 384;
   // score buffer of page i; P overlays its first 64 columns
   auto s_col = [](int bf) { return KT::SBUF == 2 ? 128u + 128u * bf : 256u; };
-  uint8_t* stg = ktile + (KT::PROD ? 65536 : 0);                   // the operand tiles are not in use yet
+  uint8_t* stg = ktile;                                            // the operand tiles are not in use yet
   const int q_esz = P.q_dtype == TQ_F32 ? 4 : 2;
-  const int q_stride = TQ_D * q_esz + 16;
+  // Rows pass through shared memory: accessed directly, a thread's own half row would put the lanes of a load 256 or 512
+  // bytes apart (one line per lane and instruction); staged, a warp moves whole rows.  16-byte chunk w of row r sits at
+  // chunk w ^ (r & 7) of its row, so that the accesses of consecutive rows fall into different banks.
+  auto chunk_at = [&](int r, int w, int esz) { return stg + r * (TQ_D * esz) + ((w ^ (r & 7)) << 4); };
+  auto stage_rows = [&]() {
+    const int cpr = TQ_D * q_esz / 16;   // chunks per row
+#pragma unroll 8
+    for (int it = 0; it < cpr / 2; ++it) {
+      const int c = it * 256 + tid, r = c / cpr, w = c - r * cpr;
+      const int grow = rb * PF_ROWS + r;
+      uint4 val = make_uint4(0u, 0u, 0u, 0u);
+      if (grow < nrows) {
+        const int gq = grow / P.group, gh = grow - gq * P.group;
+        const size_t off = ((((size_t)b * P.tq + gq) * P.hq + (size_t)kvh * P.group + gh) * TQ_D) * q_esz + w * 16;
+        val = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(P.q) + off);
+      }
+      *reinterpret_cast<uint4*>(chunk_at(r, w, q_esz)) = val;
+    }
+  };
   auto read_row = [&]() {
-    const uint8_t* mine = stg + rtid * q_stride + hf * PF_HALF * q_esz;
     if (P.q_dtype == TQ_F32) {
 #pragma unroll
       for (int e = 0; e < PF_HALF; e += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(mine + e * 4);
+        const float4 v = *reinterpret_cast<const float4*>(chunk_at(rtid, (PF_HALF * hf + e) / 4, 4));
         o[e] = v.x; o[e + 1] = v.y; o[e + 2] = v.z; o[e + 3] = v.w;
       }
     } else {
 #pragma unroll
       for (int e = 0; e < PF_HALF; e += 8) {
-        const uint4 w4 = *reinterpret_cast<const uint4*>(mine + e * 2);
+        const uint4 w4 = *reinterpret_cast<const uint4*>(chunk_at(rtid, (PF_HALF * hf + e) / 8, 2));
         const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -544,37 +634,25 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   };
   if (is_row) {
-    // The rows come in through shared memory: read directly, a thread's own half row would put the lanes of a load
-    // 256 or 512 bytes apart (one line per lane and instruction); staged, a warp reads whole rows.  Row stride: the
-    // row plus 16 bytes, so that the 16-byte accesses of consecutive rows fall into different banks.
-    const int cpr = TQ_D * q_esz / 16;   // 16-byte chunks per row
-#pragma unroll 8
-    for (int it = 0; it < cpr / 2; ++it) {
-      const int c = it * 256 + tid, r = c / cpr, w = c - r * cpr;
-      const int grow = rb * PF_ROWS + r;
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (grow < nrows) {
-        const int gq = grow / P.group, gh = grow - gq * P.group;
-        const size_t off = ((((size_t)b * P.tq + gq) * P.hq + (size_t)kvh * P.group + gh) * TQ_D) * q_esz + w * 16;
-        val = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(P.q) + off);
-      }
-      *reinterpret_cast<uint4*>(stg + r * q_stride + w * 16) = val;
-    }
+    stage_rows();
     rows_sync();
     read_row();
-    if constexpr (!KT::PROD) rows_sync();   // the staged rows are read: the rotation's exchange area is the same memory
+    rows_sync();                            // the staged rows are read: the rotation's exchange area is the same memory
     if constexpr (!KT::Q8) rotate(P.k_rot_t, fk.s1, fk.s2);
     if constexpr (KT::PROD) {
       const uint32_t tm0 = *tbase + ((uint32_t)((warp & 3) * 32) << 16);
       to_tmem(tm0, P.qscale / fk.lut_alpha, TQc, TQLc);
       rows_sync();                          // the exchange area has been read
+      stage_rows();
+      rows_sync();
       read_row();
+      rows_sync();
       rotate(P.k_s_t, fk.j1, fk.j2);
       to_tmem(tm0, P.qscale, TPc, TPLc);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();  // tensor-memory base, tables and barriers visible; the dense staging area is free again
+  pf_sync_all<CG>();  // tensor-memory base, tables and barriers visible; the staging area is free again
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tb = *tbase;
 
@@ -583,11 +661,11 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
     const uint32_t tm = tb + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 lanes
     float* xch = scales + 512;                                     // [buffer][half][row]
     if constexpr (!KT::PROD) to_tmem(tm, P.qscale / fk.lut_alpha, TQc, TQLc);
-    asm volatile("bar.sync 3, 288;" ::: "memory");   // with the MMA warp: the queries are in tensor memory
+    pf_arrive_leader<CG>(q_ready, lane);             // the queries are in tensor memory
 
     float m_run = -INFINITY, l_run = 0.f;   // l_run: this half's part of the row sum
     for (int i = 0; i < np; ++i) {
-      if (*fail) break;
+      if (__any_sync(0xffffffffu, *fail != 0)) break;
       const int bf = i & 1;
       const uint32_t ph = (uint32_t)((i >> 1) & 1);
       if (!pf_wait_warp(&s_full[bf], ph)) { *fail = 1; break; }
@@ -639,7 +717,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
       // the other half's maximum: both threads of a row then take the same decisions below.  (The arrival also tells
       // the other half that this one has read its scores: the P columns that half writes overlay them.)
       xch[(bf * 2 + hf) * PF_ROWS + rtid] = mx;
-      pf_arrive(&xbar[warp & 3]);
+      pf_arrive_warp(&xbar[warp & 3], lane);
       if (!pf_wait_warp(&xbar[warp & 3], (uint32_t)(i & 1))) { *fail = 1; break; }
       mx = fmaxf(mx, xch[(bf * 2 + (hf ^ 1)) * PF_ROWS + rtid]);
       // The row maximum moves only when it grows by more than 2^PF2_SLACK (probabilities stay below 2^PF2_SLACK).
@@ -689,7 +767,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
       l_run += ls2.x + ls2.y;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      pf_arrive(&p_ready[bf]);
+      pf_arrive_leader<CG>(&p_ready[bf], lane);
     }
     // this thread's half of the accumulated row of O, once the last product has completed
     scales[(8 + hf) * PF_ROWS + rtid] = l_run;   // the halves' parts of the row sum
@@ -710,8 +788,9 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();  // every role is done with tensor memory
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(512u) : "memory");
+    pf_sync_all<CG>();  // every role, of both CTAs, is done with tensor memory and the operand tiles
+    if (warp == 0) tmem_free_all<CG>(tb);
+    if (CG == 2 && rb >= P.row_blocks) return;   // the pair's second block of an odd number
     l_run = scales[8 * PF_ROWS + rtid] + scales[9 * PF_ROWS + rtid];
     // A CTA that gave up a wait reports it, writes no partial and merges nothing, but still takes its ticket below:
     // the counter of its (sequence, KV head, row block) then returns to zero like after a clean call, and a later
@@ -791,17 +870,15 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
       rows_sync();   // the exchange area of the rotation is read: the staging below is the same memory
       {
         const int esz = P.out_dtype == TQ_F32 ? 4 : 2;
-        const int cpr = TQ_D * esz / 16, stride = TQ_D * esz + 16;
-        uint8_t* ost = ktile;
-        uint8_t* mine = ost + rtid * stride + hf * PF_HALF * esz;
+        const int cpr = TQ_D * esz / 16;
         if (P.out_dtype == TQ_F32) {
 #pragma unroll
           for (int j = 0; j < PF_HALF; j += 4)
-            *reinterpret_cast<float4*>(mine + j * 4) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+            *reinterpret_cast<float4*>(chunk_at(rtid, (PF_HALF * hf + j) / 4, 4)) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
         } else if (P.out_dtype == TQ_F16) {
 #pragma unroll
           for (int j = 0; j < PF_HALF; j += 8)
-            *reinterpret_cast<uint4*>(mine + j * 2) = make_uint4(pf_pack(o[j], o[j + 1]), pf_pack(o[j + 2], o[j + 3]),
+            *reinterpret_cast<uint4*>(chunk_at(rtid, (PF_HALF * hf + j) / 8, 2)) = make_uint4(pf_pack(o[j], o[j + 1]), pf_pack(o[j + 2], o[j + 3]),
                                                                  pf_pack(o[j + 4], o[j + 5]), pf_pack(o[j + 6], o[j + 7]));
         } else {
 #pragma unroll
@@ -812,7 +889,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
               const __nv_bfloat162 h = __floats2bfloat162_rn(o[j + 2 * k], o[j + 2 * k + 1]);
               w[k] = *reinterpret_cast<const uint32_t*>(&h);
             }
-            *reinterpret_cast<uint4*>(mine + j * 2) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4*>(chunk_at(rtid, (PF_HALF * hf + j) / 8, 2)) = make_uint4(w[0], w[1], w[2], w[3]);
           }
         }
         rows_sync();
@@ -824,7 +901,7 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
             const int gq = grow / P.group, gh = grow - gq * P.group;
             const size_t off = ((((size_t)b * P.tq + gq) * P.hq + (size_t)kvh * P.group + gh) * TQ_D) * esz + w * 16;
             *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(P.out) + off) =
-                *reinterpret_cast<const uint4*>(ost + r * stride + w * 16);
+                *reinterpret_cast<const uint4*>(chunk_at(r, w, esz));
           }
         }
       }
@@ -832,163 +909,195 @@ __global__ void __launch_bounds__(PF2_THREADS, 1) k_prefill_attn2(const PrefillP
     return;
   }
 
-  if (is_prod) {
+  if (tid < SP::MMA_AT) {
     // =========================== producer warps ===========================
-    const uint32_t lk_base = sptr(sm + SP::OFF_K) + (PfLut<KB>::REPL ? lane * 4 : 0);
-    const uint32_t lv_base = sptr(sm + SP::OFF_V) + (PfLut<VB>::REPL ? lane * 4 : 0);
-    const uint32_t tile_row = (uint32_t)(rtid >> 3) * 2048 + (uint32_t)(rtid & 7) * 16;  // token rtid inside an operand tile
-    if (hf == 0) {
-      // K producers.  The K tiles are free once S of the page that used them before is complete (page i - 2 with two
-      // buffers, i - 1 with one), and so is the scale slot i & 3 (the rows finished page i - 4 long before): they run
-      // one page ahead of the V producers, whose tile is free only after the product of page i - 2, and S of the next
-      // page is ready before the rows ask for it.
+    // In a pair a CTA dequantizes K of its 64 tokens (its half of the columns of S) and, of all 128 tokens, its 64 dims of V
+    // (its half of the columns of O).
+    constexpr int TILE = SP::TILE;
+    const uint32_t lk_start = sptr(sm + SP::OFF_K), lv_start = sptr(sm + SP::OFF_V);
+    const uint32_t lk_base = SP::KLut::base(lk_start, lane), lv_base = SP::VLut::base(lv_start, lane);
+    if (tid < SP::V_AT) {
+      // K producers, a token per thread.  The K tiles are free once S of the page that used them before is complete (page
+      // i - 2 with two buffers, i - 1 with one), and so is the scale slot i & 3 (the rows finished page i - 4 long before):
+      // they run one page ahead of the V producers, whose tile is free only after the product of page i - 2, and S of the
+      // next page is ready before the rows ask for it.
+      const int tl = tid - SP::K_AT, tok = 64 * crank + tl;
+      uint8_t* drow = ktile + (tl >> 3) * 2048 + (tl & 7) * 16;
       for (int i = 0; i < np; ++i) {
-        const int bf = i & 1;
-        if (*fail) break;
-        if constexpr (KT::KBUF == 2) {
-          if (i >= 2 && !pf_wait(&s_full[bf], (uint32_t)(((i - 2) >> 1) & 1))) { *fail = 1; break; }
+        const int bf = i & 1, st_i = i % NST;
+        bool ok = !*fail;
+        if constexpr (SP::KBUF == 2) {
+          if (ok && i >= 2) ok = pf_wait(&s_full[bf], (uint32_t)(((i - 2) >> 1) & 1));
         } else {
-          if (i >= 1 && !pf_wait(&s_full[bf ^ 1], (uint32_t)(((i - 1) >> 1) & 1))) { *fail = 1; break; }
+          if (ok && i >= 1) ok = pf_wait(&s_full[bf ^ 1], (uint32_t)(((i - 1) >> 1) & 1));
         }
-        if (!pf_wait(&rec_full[bf], (uint32_t)((i >> 1) & 1))) { *fail = 1; break; }
-        const uint8_t* st = stage0 + (size_t)bf * rec;
-        uint8_t* dst = ktile + (KT::KBUF == 2 ? bf * 32768 : 0) + tile_row;
+        if (ok) ok = pf_wait(&rec_full[st_i], (uint32_t)((i / NST) & 1));
+        if (!__all_sync(0xffffffffu, ok)) { *fail = 1; break; }   // a warp goes on or gives up as a whole
+        const uint8_t* st = stage0 + st_i * SP::REC;
+        uint8_t* dst = drow + (SP::KBUF == 2 ? bf * KT::TILES * TILE : 0);
         if constexpr (KT::Q8) {
-          const uint2 sc = *reinterpret_cast<const uint2*>(st + P.L.k_scale_off + rtid * 8);
-          pf_q8_token<true>(st + P.L.k_idx_off + rtid * TQ_D, dst, sc.x, sc.y, lane);
+          const uint2 sc = *reinterpret_cast<const uint2*>(st + P.L.k_scale_off + tok * 8);
+          pf_q8_token<true, TQ_D, TILE>(st + P.L.k_idx_off + tok * TQ_D, dst, sc.x, sc.y, lane);
         } else {
-          pf_dequant_token<KB>(st + P.L.k_idx_off + rtid * (16 * KB), dst, lk_base);
-          const float ks = reinterpret_cast<const float*>(st + P.L.k_scale_off)[rtid];
-          scales[(i & 3) * PF_ROWS + rtid] = ks;
+          pf_dequant_token<KB, typename SP::KLut, TQ_D>(st + P.L.k_idx_off + tok * (16 * KB), dst, lk_base, lk_start);
+          for (int t = tl; t < PF_PAGE; t += 32 * SP::PW)   // the scales of all columns of S
+            scales[(i & 3) * PF_ROWS + t] = reinterpret_cast<const float*>(st + P.L.k_scale_off)[t];
           if constexpr (KT::PROD) {   // (a zero vector has two zero scales)
-            const float rs = reinterpret_cast<const float*>(st + P.L.k_rscale_off)[rtid];
-            pf_sketch_token(*reinterpret_cast<const uint4*>(st + P.L.k_qjl_off + rtid * 16), dst + 32768, ks != 0.f ? rs / ks : 0.f);
+            const float ks = reinterpret_cast<const float*>(st + P.L.k_scale_off)[tok];
+            const float rs = reinterpret_cast<const float*>(st + P.L.k_rscale_off)[tok];
+            pf_sketch_token<TQ_D, TILE>(st + P.L.k_qjl_off + tok * 16, dst + TILE, ks != 0.f ? rs / ks : 0.f);
           }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        pf_arrive(&k_ready[bf]);   // also: this thread has read its part of the record
+        pf_arrive_leader<CG>(&k_ready[bf], lane);
+        pf_arrive_warp(&rec_free[st_i], lane);
       }
     } else {
-      // V producers; one of them refills a record's stage once both groups have read it
+      // V producers
+      constexpr int DIMS = TQ_D / CG;
       for (int i = 0; i < np; ++i) {
-        const int bf = i & 1;
-        const uint32_t ph = (uint32_t)((i >> 1) & 1);
+        const int bf = i & 1, st_i = i % NST;
         bool ok = !*fail;
         if (ok && i >= 2) ok = pf_wait(&o_done[bf], (uint32_t)(((i - 2) >> 1) & 1));
-        if (ok) ok = pf_wait(&rec_full[bf], ph);
-        if (!producers_all(ok)) {  // the 128 V producers go on or give up together (they share a named barrier below)
-          *fail = 1;
-          break;
-        }
-        const uint8_t* st = stage0 + (size_t)bf * rec;
+        if (ok) ok = pf_wait(&rec_full[st_i], (uint32_t)((i / NST) & 1));
+        if (!__all_sync(0xffffffffu, ok)) { *fail = 1; break; }
+        const uint8_t* st = stage0 + st_i * SP::REC;
         // The token's V scale goes into its row of the operand tile (fp16 product, rounding 2^-11 per element), so
         // that the P operand is the bare probability, bounded by 2^(2 PF2_SLACK) whatever the norms of the values
         // are; a token past the end of the sequence may hold anything: its row is zeroed (its P is zero too, but
         // 0 x inf would not be).  Scales beyond the fp16 range saturate.
-        const bool exists = (page_lo + i) * PT + rtid < kv_len;
-        uint8_t* dst = vtile + bf * 32768 + tile_row;
-        if constexpr (VT::Q8) {
-          const uint2 sc = exists ? *reinterpret_cast<const uint2*>(st + P.L.v_scale_off + rtid * 8) : make_uint2(0u, 0u);
-          pf_q8_token<false>(st + P.L.v_idx_off + rtid * TQ_D, dst, sc.x, sc.y, lane);
-        } else {
-          const float vsc = exists ? reinterpret_cast<const float*>(st + P.L.v_scale_off)[rtid] : 0.f;
-          const __half2 s2 = __float2half2_rn(fminf(vsc, 65504.0f));
-          pf_dequant_token<VB, true>(st + P.L.v_idx_off + rtid * (16 * VB), dst, lv_base, *reinterpret_cast<const uint32_t*>(&s2));
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        pf_arrive(&v_ready[bf]);
-        asm volatile("bar.sync 1, 128;" ::: "memory");   // every V producer has read this record
-        if (tid == 384 && i + 2 < np) {
-          if (!pf_wait(&k_ready[bf], ph)) { *fail = 1; } else { issue(i + 2); }   // ... and every K producer
-        }
-      }
-    }
-    asm volatile("bar.sync 5, 256;" ::: "memory");   // both groups have left their loops: no copy will be issued any more
-    if (*fail && tid == 256) {  // copies in flight get the same bounded time before the CTA leaves
-      for (int st_i = 0; st_i < 2; ++st_i) pf_wait(&rec_full[st_i], 0), pf_wait(&rec_full[st_i], 1);
-    }
-  } else {
-    // =========================== MMA warp ===========================
-    asm volatile("bar.sync 3, 288;" ::: "memory");
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (lane == 0 && np > 0) {
-      const uint32_t idesc_s = umma_idesc(128, 128, false), idesc_o = umma_idesc(128, 128, true);
-      auto qk = [&](int i) {   // S_i = Q K_i^T (fp16 hi and lo halves of Q), into the score buffer of page i
-        const int bf = i & 1;
-        const uint32_t kt = sptr(ktile) + (KT::KBUF == 2 ? bf * 32768 : 0), d = tb + s_col(bf);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t kd = umma_desc(kt + ks * 256, 128, 2048);
-          umma_ts(d, tb + TQc + ks * 8, kd, idesc_s, ks > 0);
-          umma_ts(d, tb + TQLc + ks * 8, kd, idesc_s, 1);
-          if constexpr (KT::TILES > 1) {   // q8_0: what the fp16 products left; PROD: the sketch against the projected query
-            const uint64_t k1 = umma_desc(kt + 32768 + ks * 256, 128, 2048);
-            umma_ts(d, tb + (KT::PROD ? TPc : TQc) + ks * 8, k1, idesc_s, 1);
-            if constexpr (KT::PROD) {
-              umma_ts(d, tb + TPLc + ks * 8, k1, idesc_s, 1);
-              umma_ts(d, tb + TPc + ks * 8, umma_desc(kt + 65536 + ks * 256, 128, 2048), idesc_s, 1);
-            }
+        for (int k = 0; k < PF_PAGE / (32 * SP::PW); ++k) {
+          const int tok = tid - SP::V_AT + k * 32 * SP::PW;
+          const bool exists = (page_lo + i) * PT + tok < kv_len;
+          uint8_t* dst = vtile + bf * TILE + (tok >> 3) * (2048 / CG) + (tok & 7) * 16;
+          if constexpr (VT::Q8) {
+            const uint2 sc = exists ? *reinterpret_cast<const uint2*>(st + P.L.v_scale_off + tok * 8) : make_uint2(0u, 0u);
+            pf_q8_token<false, DIMS, TILE>(st + P.L.v_idx_off + tok * TQ_D + crank * DIMS, dst, crank ? sc.y : sc.x, sc.y, lane);
+          } else {
+            const float vsc = exists ? reinterpret_cast<const float*>(st + P.L.v_scale_off)[tok] : 0.f;
+            const __half2 s2 = __float2half2_rn(fminf(vsc, 65504.0f));
+            pf_dequant_token<VB, typename SP::VLut, DIMS, true>(st + P.L.v_idx_off + tok * (16 * VB) + crank * (DIMS * VB / 8), dst,
+                                                                lv_base, lv_start, *reinterpret_cast<const uint32_t*>(&s2));
           }
         }
-        umma_commit(&s_full[bf]);
-      };
-      bool okay = pf_wait(&k_ready[0], 0);
-      if (okay) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        qk(0);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        pf_arrive_leader<CG>(&v_ready[bf], lane);
+        pf_arrive_warp(&rec_free[st_i], lane);
       }
-      for (int i = 0; okay && i < np; ++i) {
-        if (*fail) break;
-        const int bf = i & 1;
-        const uint32_t ph = (uint32_t)((i >> 1) & 1);
-        if (KT::SBUF == 2 && i + 1 < np) {
-          if (!pf_wait(&k_ready[(i + 1) & 1], (uint32_t)(((i + 1) >> 1) & 1))) { okay = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          qk(i + 1);
-        }
-        if (!pf_wait(&p_ready[bf], ph) || !pf_wait(&v_ready[bf], ph)) { okay = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)   // O += P_i V_i: P from tensor memory, V tile MN-major, N = 128
-          umma_ts(tb + TOc, tb + s_col(bf) + ks * 8, umma_desc(sptr(vtile + bf * 32768) + ks * 4096, 2048, 128),
-                  idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&o_done[bf]);
-        if (KT::SBUF == 1 && i + 1 < np) {
-          // one score buffer: the next page's scores follow once this page's product, which reads P out of it, is done
-          if (!pf_wait(&o_done[bf], ph) || !pf_wait(&k_ready[(i + 1) & 1], (uint32_t)(((i + 1) >> 1) & 1))) { okay = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          qk(i + 1);
-        }
-      }
-      if (!okay) *fail = 1;
     }
-    __syncwarp();
+  } else if (tid == SP::COPIER) {
+    // =========================== record copies ===========================
+    int issued = min(np, NST);
+    while (issued < np && !*fail) {   // the stage of page issued - NST, once all producer warps have read it
+      if (!pf_wait(&rec_free[issued % NST], (uint32_t)((issued / NST - 1) & 1))) { *fail = 1; break; }
+      issue(issued++);
+    }
+    for (int i = max(0, issued - NST); i < issued; ++i) pf_wait(&rec_full[i % NST], (uint32_t)((i / NST) & 1));   // none in flight at the end
+  } else if (warp == SP::MMA_AT / 32 && crank == 0 && np > 0) {
+    // =========================== MMA warp ===========================
+    // (all 512 columns are this CTA's: its tensor memory starts at address 0)
+    bool okay = pf_wait_warp(q_ready, 0) && __all_sync(0xffffffffu, tb == 0);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t idesc_s = umma_idesc(128 * CG, 128, false), idesc_o = umma_idesc(128 * CG, 128, true);
+    auto qk = [&](int i) {   // S_i = Q K_i^T (fp16 hi and lo halves of Q), into the score buffer of page i
+      const int bf = i & 1;
+      const uint32_t kt = sptr(ktile) + (SP::KBUF == 2 ? bf * KT::TILES * SP::TILE : 0), d = s_col(bf);
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        const uint64_t kd = umma_desc(kt + ks * 256, 128, 2048);
+        umma_ts<CG>(d, TQc + ks * 8, kd, idesc_s, ks > 0);
+        umma_ts<CG>(d, TQLc + ks * 8, kd, idesc_s, 1);
+        if constexpr (KT::TILES > 1) {   // q8_0: what the fp16 products left; PROD: the sketch against the projected query
+          const uint64_t k1 = umma_desc(kt + SP::TILE + ks * 256, 128, 2048);
+          umma_ts<CG>(d, (KT::PROD ? TPc : TQc) + ks * 8, k1, idesc_s, 1);
+          if constexpr (KT::PROD) {
+            umma_ts<CG>(d, TPLc + ks * 8, k1, idesc_s, 1);
+            umma_ts<CG>(d, TPc + ks * 8, umma_desc(kt + 2 * SP::TILE + ks * 256, 128, 2048), idesc_s, 1);
+          }
+        }
+      }
+      umma_commit<CG>(&s_full[bf]);
+    };
+    if (okay) okay = pf_wait_warp(&k_ready[0], 0);
+    if (okay) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      qk(0);
+    }
+    for (int i = 0; okay && i < np; ++i) {
+      if (__any_sync(0xffffffffu, *fail != 0)) break;
+      const int bf = i & 1;
+      const uint32_t ph = (uint32_t)((i >> 1) & 1);
+      if (KT::SBUF == 2 && i + 1 < np) {
+        if (!pf_wait_warp(&k_ready[(i + 1) & 1], (uint32_t)(((i + 1) >> 1) & 1))) { okay = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        qk(i + 1);
+      }
+      if (!pf_wait_warp(&p_ready[bf], ph) || !pf_wait_warp(&v_ready[bf], ph)) { okay = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks)   // O += P_i V_i: P from tensor memory, V tile MN-major, N = 128
+        umma_ts<CG>(TOc, s_col(bf) + ks * 8,
+                    umma_desc(sptr(vtile + bf * SP::TILE) + ks * (4096 / CG), 2048 / CG, 128), idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
+      umma_commit<CG>(&o_done[bf]);
+      if (KT::SBUF == 1 && i + 1 < np) {
+        // one score buffer: the next page's scores follow once this page's product, which reads P out of it, is done
+        if (!pf_wait_warp(&o_done[bf], ph) || !pf_wait_warp(&k_ready[(i + 1) & 1], (uint32_t)(((i + 1) >> 1) & 1))) { okay = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        qk(i + 1);
+      }
+    }
+    if (!okay) *fail = 1;
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();  // matches the row warps' barrier before the tensor memory is released
+  pf_sync_all<CG>();  // matches the row warps' barrier before the tensor memory is released
 }
 
 }  // namespace
 
-template <int KK, int VK>
-static int launch_prefill(const PrefillParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
-  const size_t need = PfSmem2<KK, VK>::bytes(P.L.record_bytes);
-  constexpr size_t LIMIT = 227 * 1024;  // one CTA per SM (it also takes all 512 tensor-memory columns)
-  TQ_REQUIRE(need <= LIMIT, TQ_ERR_TOO_LARGE, "page record of %d bytes does not fit the prefill pipeline",
-             P.L.record_bytes);
-  // (the limit is raised to what the call needs and no further: local memory lives in what is left as L1)
+template <int KK, int VK, int CG>
+static int launch_prefill_cg(const PrefillParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
+  using SP = PfSmem2<KK, VK, CG>;
+  TQ_REQUIRE(P.L.record_bytes == SP::REC, TQ_ERR_UNSUPPORTED, "prefill attention: page record of %d bytes, expected %d",
+             P.L.record_bytes, SP::REC);
   static thread_local int configured_dev = -1;
-  static thread_local size_t configured = 0;
   int dev = 0;
   TQ_CUDA(cudaGetDevice(&dev));
-  if (configured_dev != dev || configured < need) {
-    TQ_CUDA(cudaFuncSetAttribute(k_prefill_attn2<KK, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+  if (configured_dev != dev) {
+    TQ_CUDA(cudaFuncSetAttribute(k_prefill_attn2<KK, VK, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SP::BYTES));
     configured_dev = dev;
-    configured = need;
   }
-  dim3 grid(P.row_blocks * P.num_splits, P.hkv, P.batch);
-  k_prefill_attn2<KK, VK><<<grid, PF2_THREADS, need, st>>>(P, fk, fv);
+  const int64_t grid = (int64_t)CG * ((P.row_blocks + CG - 1) / CG) * P.batch * P.hkv * P.num_splits;
+  TQ_REQUIRE(grid < (1LL << 31), TQ_ERR_TOO_LARGE, "prefill attention: %lld CTAs", (long long)grid);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(SP::THREADS);
+  cfg.dynamicSmemBytes = SP::BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CG;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CG == 1 ? 1 : 2;
+  TQ_CUDA(cudaLaunchKernelEx(&cfg, k_prefill_attn2<KK, VK, CG>, P, fk, fv));
   return tq_launch_check("k_prefill_attn2");
+}
+
+// CTAs per operand tile: a pair as soon as there are two row blocks to pair.  Not with PROD keys: their one score buffer puts
+// scores, softmax and product of a page one after the other, 3.6 us a page in either form.
+static bool pf_prod(int k_format) { return k_format >= TQ_FMT_PROD2; }
+static int pf_cta_group(int row_blocks, bool prod) { return row_blocks > 1 && !prod ? 2 : 1; }
+
+template <int KK, int VK>
+static int launch_prefill(const PrefillParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
+  if constexpr (!PfKind<KK>::PROD)
+    if (pf_cta_group(P.row_blocks, false) == 2) return launch_prefill_cg<KK, VK, 2>(P, fk, fv, st);
+  return launch_prefill_cg<KK, VK, 1>(P, fk, fv, st);
 }
 
 struct PfPlan {
@@ -996,13 +1105,14 @@ struct PfPlan {
   size_t part_o, part_ml, total;
 };
 static const size_t PF_TAIL = 65536 * 4 + 256;  // tickets + status word, at the end of the workspace
-static const long PF_CTA_COST_PAGES = 16;  // prologue, partial and merge of a CTA, in units of one page of the main loop
+static const long PF_CTA_COST_PAGES = 12;  // prologue, partial and merge of a CTA, in units of one page of the main loop
 
-static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_pages) {
+static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_pages, bool prod) {
   PfPlan p;
   p.row_blocks = (chunk_tokens * (hq / hkv) + PF_ROWS - 1) / PF_ROWS;
-  const long base = (long)p.row_blocks * hkv * batch;
-  const int slots = tq_num_sms();  // one CTA per SM
+  const int cg = pf_cta_group(p.row_blocks, prod);
+  const long base = (long)((p.row_blocks + cg - 1) / cg) * hkv * batch;
+  const int slots = tq_num_sms() / cg;  // one CTA per SM
   const int cap = max_pages / 8 > 1 ? max_pages / 8 : 1;  // at least eight pages per split
   // splits per row block: the count that minimises (waves of CTAs) x (pages per split + fixed cost of a CTA)
   int s = 1;
@@ -1017,7 +1127,7 @@ static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_page
   }
   p.chunk_pages = (max_pages + s - 1) / s;
   p.num_splits = (max_pages + p.chunk_pages - 1) / p.chunk_pages;
-  const size_t slots_total = (size_t)base * p.num_splits;
+  const size_t slots_total = (size_t)p.row_blocks * hkv * batch * p.num_splits;
   p.part_o = 0;
   p.part_ml = slots_total * PF_ROWS * TQ_D * 4;
   p.total = p.part_ml + slots_total * PF_ROWS * 2 * 4 + PF_TAIL;
@@ -1030,7 +1140,9 @@ extern "C" int64_t tq_prefill_workspace_bytes(int32_t batch, int32_t chunk_token
   if (batch < 1 || chunk_tokens < 1 || num_q_heads < 1 || num_kv_heads < 1 || max_pages_per_seq < 1 ||
       num_q_heads % num_kv_heads)
     return TQ_ERR_INVALID;
-  return (int64_t)pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq).total;
+  const size_t a = pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq, false).total;
+  const size_t b = pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq, true).total;
+  return (int64_t)(a > b ? a : b);   // enough for every pair of formats
 }
 
 extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, const tq_cache_layout* L,
@@ -1081,7 +1193,7 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
   P.hq = num_q_heads;
   P.hkv = L->num_kv_heads;
   P.group = num_q_heads / L->num_kv_heads;
-  const PfPlan plan = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq);
+  const PfPlan plan = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, pf_prod(L->k_format));
   TQ_REQUIRE((int64_t)plan.total <= workspace_bytes, TQ_ERR_TOO_LARGE,
              "prefill workspace of %lld bytes is smaller than the %lld needed (tq_prefill_workspace_bytes)",
              (long long)workspace_bytes, (long long)plan.total);
