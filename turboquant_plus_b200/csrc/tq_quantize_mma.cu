@@ -605,11 +605,15 @@ __device__ __forceinline__ void qm_body(const TqFast& f, const Tin* __restrict__
 }
 
 // staging memory of one CTA (tiles + B operands): 16-bit rows fit the static limit, fp32 rows (72 KB) are dynamic
-// (the QJL stage adds 4 KB of sign factors and keeps more values live: one CTA less per SM)
+// (the QJL stage adds 4 KB of sign factors)
 template <typename Tin, bool QJLS = false> constexpr int qm_tile_bytes() {
   return QM_WARPS * 2 * QM_ROWS * qm_rowb<Tin>() + 8 * 32 * 16 + (QJLS ? 8 * 32 * 16 : 0);
 }
-template <typename Tin, bool QJLS = false> constexpr int qm_ctas_per_sm() { return (sizeof(Tin) == 4 ? 3 : 5) - (QJLS ? 1 : 0); }
+// CTAs per SM, i.e. registers per thread.  The QJL stage keeps the residuals of both vectors live beside its own values: at 128
+// registers (four CTAs) it spilled, at 168 (three) 524,288 bf16 keys take 113 us instead of 123 with a 2-bit PolarQuant stage and
+// 146 instead of 215 with a 3-bit one.  The other forms are bound by their pipes (issue slots 62 %, integer 54 %): four CTAs
+// (111 us for two tensors of 3-bit indices) or six (124, spills) are slower than five (110).
+template <typename Tin, bool QJLS = false> constexpr int qm_ctas_per_sm() { return sizeof(Tin) == 4 ? (QJLS ? 2 : 3) : (QJLS ? 3 : 5); }
 template <typename Tin, bool QJLS = false> __device__ __forceinline__ uint8_t* qm_tile() {
   if constexpr (sizeof(Tin) == 4) {
     extern __shared__ __align__(16) uint8_t qm_dyn[];
