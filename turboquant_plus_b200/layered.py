@@ -97,53 +97,88 @@ class LayeredKVCache:
             "slots": torch.zeros((max(len(m) for _, m in self.groups), batch), dtype=torch.int64, device=dev),
         }
         st["workspace"] = self.layers[0].workspace(batch, num_q_heads, st["bt"].shape[1])
-        # per format group: which layers, and where each layer's pages start inside the group's pool
-        st["plans"] = [(whole, None if members == list(range(L)) else torch.tensor(members, device=dev), len(members))
-                       for whole, members in self.groups]
+        st["jobs"] = self._append_jobs(0, L)
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):      # warm-up outside capture (sets kernel attributes, fills caches)
             saved = st["len"].clone()
-            self._append_part(st)
+            self._slots_part(st)
+            self._append_part(st, st["jobs"])
             self._attend_part(st, 0, L)
             st["len"].copy_(saved)
         torch.cuda.current_stream(dev).wait_stream(side)
         torch.cuda.synchronize(dev)
         graph = torch.cuda.CUDAGraph()
         with _capture(torch, graph):
-            self._append_part(st)
+            self._slots_part(st)
+            self._append_part(st, st["jobs"])
             self._attend_part(st, 0, L)
         st["len"].copy_(saved)
         st["graph"] = graph
-        st["io_stream"] = side
+        st["io_streams"] = side, torch.cuda.Stream(device=dev)
         self._step = st
         return st
 
     # (methods that take the step's state, not closures kept in it: a cache that is dropped is then freed at once, with
     # its graphs and buffers, instead of waiting for the cyclic collector)
-    def _append_part(self, st):
-        """Slots of the new tokens and the lengths' increment, then one quantize-on-append launch per format group: the
-        new token of every layer of the group at once."""
+    def _append_jobs(self, lo, hi):
+        """The append launches of layers [lo, hi), as (cache of the group, the layers' places in it, their rows): per format
+        group one for each run of neighbouring layers, or a single one with its rows gathered where the group's layers are
+        scattered (a launch costs less than gathering K and V)."""
         torch = nv.require_cuda()
-        _, batch, _, d = st["q"].shape
+        jobs = []
+        for whole, members in self.groups:
+            runs = []
+            for j in (j for j, i in enumerate(members) if lo <= i < hi):      # places in the group: consecutive
+                if runs and members[j] == members[j - 1] + 1:
+                    runs[-1].append(j)
+                else:
+                    runs.append([j])
+            if len(runs) <= 2:
+                jobs += [(whole, slice(run[0], run[-1] + 1), slice(members[run[0]], members[run[-1]] + 1)) for run in runs]
+            else:
+                at = slice(runs[0][0], runs[-1][-1] + 1)
+                jobs.append((whole, at, torch.tensor(members[at], device=self.device)))
+        return jobs
+
+    def _slots_part(self, st):
+        """Slots of the step's new tokens, and the lengths' increment."""
+        torch = nv.require_cuda()
         with torch.cuda.device(self.device):
             nv.call("tq_decode_step_slots", nv.ptr(st["bt"]), st["bt"].shape[1], nv.ptr(st["len"]), self.page_tokens,
-                    batch, st["slots"].shape[0], self.num_pages * self.page_tokens, nv.ptr(st["slots"]), nv.stream_ptr())
-        for whole, idx, n in st["plans"]:
-            k = st["k"] if idx is None else st["k"].index_select(0, idx)
-            v = st["v"] if idx is None else st["v"].index_select(0, idx)
-            whole.append(k.reshape(n * batch, self.num_kv_heads, d), v.reshape(n * batch, self.num_kv_heads, d),
-                         st["slots"][:n].reshape(-1))
+                    st["q"].shape[1], st["slots"].shape[0], self.num_pages * self.page_tokens, nv.ptr(st["slots"]), nv.stream_ptr())
+
+    def _append_part(self, st, jobs):
+        """Quantize-on-append of the new token of the layers of ``jobs``."""
+        _, batch, _, d = st["q"].shape
+        for whole, at, rows in jobs:
+            k, v = (t[rows] if isinstance(rows, slice) else t.index_select(0, rows) for t in (st["k"], st["v"]))
+            n = (at.stop - at.start) * batch
+            whole.append(k.reshape(n, self.num_kv_heads, d), v.reshape(n, self.num_kv_heads, d), st["slots"][at].reshape(-1))
 
     def _attend_part(self, st, lo, hi):
         for i in range(lo, hi):
             # An attention call that follows another layer's attention call may start early: that kernel writes
-            # nothing this one reads before its dependency wait, and the queries of every layer are in place
-            # before the first launch of the step (they arrive with the step's host-to-device copy).  The first
-            # call follows the append, which writes the cache slot of the new token: it runs in stream order, in
-            # the form of the calls that follow it.
+            # nothing this one reads before its dependency wait, and the queries and the new rows of its layer are in
+            # place before the first launch of its part.  The first call of a step follows the append, which writes
+            # the cache slot of the new token: it runs in stream order, in the form of the calls that follow it.
             self.layers[i].attend(st["q"][i], st["bt"], st["len"], out=st["out"][i], workspace=st["workspace"],
                                   overlap="q" if i > 0 else False, chain_head=(i == 0))
+
+    # Parts of a step: the bytes that the first copy in and the last copy out carry, about 5 and 2.5 us of the bus --
+    # what is left of the copies outside the kernels -- and the growth from one part to the next.  A layer's cache is
+    # read far slower than its rows cross the bus, so that a part four times as large arrives under the one in front
+    # of it; each part costs its own append launches, which is why a step below four first copies stays in one part.
+    _PART_IN, _PART_OUT, _PART_GROWTH = 256 << 10, 128 << 10, 4
+
+    @staticmethod
+    def _cuts(layers, layer_bytes, first, growth):
+        """Bounds of parts of ``layers`` layers, the first of at least ``first`` bytes, each ``growth`` times the last."""
+        cuts, n = [0], max(1, -(-first // layer_bytes))
+        while layers - cuts[-1] > n:
+            cuts.append(cuts[-1] + n)
+            n *= growth
+        return cuts + [layers]
 
     def host_buffers(self):
         """Pinned host tensors (q, k, v, out) for decode_step, q/k/v carved from one allocation in the order of the
@@ -182,34 +217,62 @@ class LayeredKVCache:
         if st.get("io_key") == key or all(t.is_pinned() for t in hosts):
             if st.get("io_key") != key:
                 graph = torch.cuda.CUDAGraph()
-                side, half = st["io_stream"], self.num_layers // 2
+                (side, back), L = st["io_streams"], self.num_layers
+                esz = st["qkv"].element_size()
+                rows = (st["q"][0].numel() + 2 * st["k"][0].numel()) * esz
+                ins = [0, L]
+                if L * rows >= 4 * self._PART_IN:
+                    ins = self._cuts(L, rows, self._PART_IN, self._PART_GROWTH)
+                outs = [L - c for c in reversed(self._cuts(L, st["out"][0].numel() * esz, self._PART_OUT, 2))]
+                if len(outs) == 2:
+                    outs = sorted({0, L // 2, L})
+                jobs = [self._append_jobs(lo, hi) for lo, hi in zip(ins, ins[1:])]
                 with _capture(torch, graph):
-                    # The copies are branches of the graph.  In: the new K/V rows first, then the queries on a side
-                    # branch under the append, which needs only the rows.  Out: the outputs of the lower half of the
-                    # layers leave while the upper half is still computing.
+                    # The copies are branches of the graph.  In: the new K/V rows of a part of the layers, their
+                    # append, and their queries -- the first part's queries under its append, which needs only the rows,
+                    # every further part's under the attention of the part in front.  Out: the outputs of a part
+                    # leave while the next is computing.
                     main = torch.cuda.current_stream(self.device)
                     nq, nk = st["q"].numel(), st["k"].numel()
-                    if (k_host.is_contiguous() and v_host.is_contiguous() and k_host.dtype == st["qkv"].dtype
-                            and k_host.numel() == nk and v_host.numel() == nk
-                            and v_host.data_ptr() == k_host.data_ptr() + nk * k_host.element_size()):
-                        # rows of K and V adjacent on the host (host_buffers()): one copy
-                        st["qkv"][nq:].copy_(k_host.reshape(-1).as_strided((2 * nk,), (1,)), non_blocking=True)
-                    else:
-                        st["k"].copy_(k_host, non_blocking=True)
-                        st["v"].copy_(v_host, non_blocking=True)
+                    adjacent = (len(ins) == 2 and k_host.is_contiguous() and v_host.is_contiguous()
+                                and k_host.dtype == st["qkv"].dtype and k_host.numel() == nk and v_host.numel() == nk
+                                and v_host.data_ptr() == k_host.data_ptr() + nk * k_host.element_size())
                     side.wait_stream(main)
-                    with torch.cuda.stream(side):
-                        st["q"].copy_(q_host, non_blocking=True)
-                    self._append_part(st)
+                    self._slots_part(st)
+                    slots = main.record_event()
+                    here = []                       # per part: what its first attention call waits for
+                    for part, (lo, hi) in enumerate(zip(ins, ins[1:])):
+                        with torch.cuda.stream(side):
+                            if adjacent:            # rows of K and V side by side on the host (host_buffers()): one copy
+                                st["qkv"][nq:].copy_(k_host.reshape(-1).as_strided((2 * nk,), (1,)), non_blocking=True)
+                            else:
+                                st["k"][lo:hi].copy_(k_host[lo:hi], non_blocking=True)
+                                st["v"][lo:hi].copy_(v_host[lo:hi], non_blocking=True)
+                            if part:
+                                side.wait_event(slots)
+                                self._append_part(st, jobs[part])
+                        if part == 0:
+                            main.wait_stream(side)
+                            self._append_part(st, jobs[part])
+                        with torch.cuda.stream(side):
+                            # (after the append of a further part: the edge from a copy to a kernel is a full one, so
+                            # that no call of the part starts before the append has completed)
+                            st["q"][lo:hi].copy_(q_host[lo:hi], non_blocking=True)
+                            here.append(side.record_event())
+                    done = 0
+                    bounds = sorted({*ins, *outs})
+                    for lo, hi in zip(bounds, bounds[1:]):
+                        if lo in ins:
+                            main.wait_event(here[ins.index(lo)])
+                        self._attend_part(st, lo, hi)
+                        if hi in outs:
+                            back.wait_stream(main)
+                            with torch.cuda.stream(back):
+                                out_host[done:hi].copy_(st["out"][done:hi], non_blocking=True)
+                            done = hi
                     main.wait_stream(side)
-                    self._attend_part(st, 0, half)
-                    side.wait_stream(main)
-                    with torch.cuda.stream(side):
-                        out_host[:half].copy_(st["out"][:half], non_blocking=True)
-                    self._attend_part(st, half, self.num_layers)
-                    out_host[half:].copy_(st["out"][half:], non_blocking=True)
-                    main.wait_stream(side)
-                st["io_graph"], st["io_key"], st["io_refs"] = graph, key, hosts   # the graph holds raw host pointers
+                    main.wait_stream(back)
+                st["io_graph"], st["io_key"], st["io_refs"] = graph, key, (hosts, jobs)   # the graph holds raw pointers
             st["io_graph"].replay()
         else:
             self._copy_in(q_host, k_host, v_host)
