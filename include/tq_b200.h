@@ -311,7 +311,7 @@ int tq_decode_attn(const tq_quantizer* kq, const tq_quantizer* vq, const tq_cach
  * benchmark step, the calls over the old and the recent part of a sequence that tq_attn_merge joins).  The
  * kernel then reads its queries and streams its pages while the preceding kernel is still finishing, and waits for
  * it only before its first write (split partials, tickets, output).  Honoured by the kernel for PolarQuant K and V
- * with <= 4 query heads per KV head and a sign-WHT K rotation; elsewhere it means TQ_DECODE_OVERLAP. */
+ * with <= 8 query heads per KV head and a sign-WHT K rotation; elsewhere it means TQ_DECODE_OVERLAP. */
 #define TQ_DECODE_OVERLAP_Q (8 | 64)
 /* TQ_DECODE_OVERLAP_APPEND (bits 3, 6 and 7): for the attention call that follows the append of the step's new token.
  * The caller states that, of everything this call reads, the preceding kernel writes at most the last cached position
