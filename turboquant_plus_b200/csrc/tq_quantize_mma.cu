@@ -114,7 +114,8 @@ __device__ __forceinline__ float2 qm_dup(float v) { return make_float2(v, v); }
 
 // `tile`: the CTA's staging memory, QM_WARPS x 2 buffers of QM_ROWS rows of qm_rowb<Tin>() bytes, then 4 KB for the
 // B operands of the MMAs
-template <typename Tin, int BITS, bool NORMC, bool QJLS = false>
+// PAIR: the two-tensor kernel, behind which no launch of the same append follows.
+template <typename Tin, int BITS, bool NORMC, bool QJLS = false, bool PAIR = false>
 __device__ __forceinline__ void qm_body(const TqFast& f, const Tin* __restrict__ x, int64_t ld, int64_t n,
                                         const TqQuantDst& dst, uint8_t* tile) {
   if (dst.beside) TQ_PDL_TRIGGER();
@@ -175,7 +176,17 @@ __device__ __forceinline__ void qm_body(const TqFast& f, const Tin* __restrict__
 #pragma unroll
       for (int c = 0; c < 4; ++c) j2w = (j2w << 1) | qm_bit(f.j2, 16 * i + 4 * t + c);
   }
-  if (!dst.beside) TQ_PDL_ENTER();   // the tables need the parameters only; rows, slots and pages come after
+  // The tables need the parameters only; rows, slots and pages come after the wait.  The kernel behind comes up at once, except
+  // beside a two-tensor grid of more than two CTAs per SM: its waiting CTAs would settle unevenly there -- on the SMs with
+  // room, several to one -- and run so when their turn comes.  It then comes up as the tiles run out.  (fp16 rows, appends one
+  // after the other, 8 heads: 8,192 tokens of turbo3 18.6 -> 17.4 us, 2,048 of turbo4 9.5 -> 8.1; with 1,024 tokens of
+  // turbo4, 256 CTAs, the early form is ahead, 6.1 against 6.6 us, and the attention call behind a decode step's append streams
+  // pages meanwhile.)
+  const bool early = !PAIR || gridDim.x * gridDim.y <= 296;
+  if (!dst.beside) {
+    TQ_PDL_WAIT();
+    if (early) TQ_PDL_TRIGGER();
+  }
   __syncthreads();
   const uint4* bfr4 = reinterpret_cast<const uint4*>(bsm) + lane;
   // sign2 mirrors an index (i -> 2^b - 1 - i): an XOR of the packed word.  Word tp of this lane packs, most
@@ -601,6 +612,7 @@ __device__ __forceinline__ void qm_body(const TqFast& f, const Tin* __restrict__
     __syncwarp();  // every lane is done with this buffer before the copies of the tile after next land in it
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (!early) TQ_PDL_TRIGGER();
   if (dst.beside) TQ_PDL_WAIT();
 }
 
@@ -641,8 +653,8 @@ __global__ void __launch_bounds__(QM_THREADS, qm_ctas_per_sm<Tin>()) k_quantize_
                                                                                         const __grid_constant__ QmJob j1, int64_t ld,
                                                                                         int64_t n) {
   uint8_t* tile = qm_tile<Tin>();
-  if (blockIdx.y == 0) qm_body<Tin, BITS, NORMC>(j0.f, reinterpret_cast<const Tin*>(j0.x), ld, n, j0.dst, tile);
-  else qm_body<Tin, BITS, NORMC>(j1.f, reinterpret_cast<const Tin*>(j1.x), ld, n, j1.dst, tile);
+  if (blockIdx.y == 0) qm_body<Tin, BITS, NORMC, false, true>(j0.f, reinterpret_cast<const Tin*>(j0.x), ld, n, j0.dst, tile);
+  else qm_body<Tin, BITS, NORMC, false, true>(j1.f, reinterpret_cast<const Tin*>(j1.x), ld, n, j1.dst, tile);
 }
 
 // dynamic shared memory of a launch (0 for 16-bit rows); raises the kernel's limit once per device
