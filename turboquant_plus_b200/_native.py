@@ -182,7 +182,8 @@ class Constants:
     them since they were uploaded.
 
     An array the class alone holds cannot change, so a call only compares a stamp; once an attribute has been read from
-    outside, its holder may write into it at any time, and every call compares the contents with what was uploaded.
+    or assigned from outside, its holder may write into it at any time, and every call compares the contents with what was
+    uploaded.
     (Copying and comparing 128 KB per call took 15-20 us of every append and attention call.)"""
 
     def __init__(self, **arrays):
@@ -190,7 +191,7 @@ class Constants:
         self.stamp = next(_stamps)      # unique: a replaced object never looks like the one before it
 
     def set(self, name, value):
-        self._arrays[name] = value
+        self._arrays[name], self._lent = value, True      # the array stays in the caller's hands
         self.stamp = next(_stamps)
 
     def lend(self, name):
