@@ -206,7 +206,9 @@ template <int KIND> struct PfKind {
   static constexpr bool Q8 = KIND == 8, PROD = KIND >= 18;
   static constexpr int BITS = Q8 ? 0 : (PROD ? KIND - 17 : KIND);
   // K operand tiles of a page.  turbo: centroids (the row scale is applied to the scores in fp32).  q8_0: int8 x block
-  // scale is 19 bits, so its fp16 rounding and the rest, exactly.  PROD: centroids, then +-ratio for the sketch, ratio =
+  // scale is 19 bits, so its fp16 rounding and the rest, exactly; of a token with a block scale above PF_Q8_BIG, whose
+  // products may exceed the fp16 range, divided by 128, which the scores get back in fp32 (what falls below fp16's
+  // smallest number then is under 2^-32 of the token's largest element).  PROD: centroids, then +-ratio for the sketch, ratio =
   // residual scale / row scale (one row scale then serves both parts), as its fp16 rounding and the rest of it.
   static constexpr int TILES = PROD ? 3 : (Q8 ? 2 : 1);
   // PROD queries (rotated and projected, hi and lo) take 256 tensor-memory columns: one score buffer instead of two
@@ -282,6 +284,18 @@ __device__ __forceinline__ void pf_dequant_token(const uint8_t* src, uint8_t* ds
     }
     *reinterpret_cast<uint4*>(dst + c * 128) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
   }
+}
+
+// q8_0 keys: block scales (fp16 bits; scales are not negative, so that their bits compare like their values) up to this
+// one keep every product int8 x scale within 127 x 512 = 65,024; above it 127 x 65,504 / 128 = 64,992 does
+constexpr uint32_t PF_Q8_BIG = 0x6000;   // 512
+__device__ __forceinline__ bool pf_q8_big(uint2 sc) {
+  return max(max(sc.x & 0xffffu, sc.x >> 16), max(sc.y & 0xffffu, sc.y >> 16)) > PF_Q8_BIG;
+}
+__device__ __forceinline__ uint32_t pf_div128(uint32_t h2) {
+  uint32_t d;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(h2), "r"(0x20002000u));
+  return d;
 }
 
 __device__ __forceinline__ uint32_t pf_s8x2(uint32_t biased, uint32_t sel) {
@@ -473,6 +487,7 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   uint64_t* xbar = bars + 19;   // one per row quarter: both halves' maxima of a page are in shared memory [2 warps]
   uint32_t* tbase = reinterpret_cast<uint32_t*>(sm + SP::OFF_BAR + 224);
   volatile int* fail = reinterpret_cast<volatile int*>(sm + SP::OFF_BAR + 232);
+  uint32_t* q8_big = reinterpret_cast<uint32_t*>(sm + SP::OFF_BAR + 236);   // [4 slots], a byte per K producer warp: see PfKind
   if (tid == SP::COPIER) {   // lane 0 of the last warp issues the record copies
     auto init = [](uint64_t* bar, int count) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sptr(bar)), "r"(count) : "memory");
@@ -491,6 +506,7 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
     for (int i = 0; i < 4; ++i) init(&xbar[i], 2);
     init(q_ready, 8 * CG);
     *fail = 0;
+    for (int i = 0; i < 4; ++i) q8_big[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   SP::KLut::fill(sm + SP::OFF_K, fk.cent16, tid, SP::THREADS);
@@ -685,6 +701,18 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       tmem_ld16_nowait<32>(ts + 64 * hf + 32, raw);
       tmem_ld16_nowait<48>(ts + 64 * hf + 48, raw);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if constexpr (KT::Q8) {   // scores of tokens whose operands are divided by 128: none on most pages
+        if (*reinterpret_cast<volatile uint32_t*>(q8_big + (i & 3))) {
+#pragma unroll
+          for (int j = 0; j < 64; j += 4) {
+            const float4 k4 = ksc4[j >> 2];
+            raw[j] = __float_as_uint(__uint_as_float(raw[j]) * k4.x);
+            raw[j + 1] = __float_as_uint(__uint_as_float(raw[j + 1]) * k4.y);
+            raw[j + 2] = __float_as_uint(__uint_as_float(raw[j + 2]) * k4.z);
+            raw[j + 3] = __float_as_uint(__uint_as_float(raw[j + 3]) * k4.w);
+          }
+        }
+      }
       auto pass1 = [&](auto masked_c) {   // two copies behind a warp-uniform branch: only the diagonal pages pay for the mask
         constexpr bool MASKED = decltype(masked_c)::value;
 #pragma unroll
@@ -936,8 +964,17 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
         const uint8_t* st = stage0 + st_i * SP::REC;
         uint8_t* dst = drow + (SP::KBUF == 2 ? bf * KT::TILES * TILE : 0);
         if constexpr (KT::Q8) {
-          const uint2 sc = *reinterpret_cast<const uint2*>(st + P.L.k_scale_off + tok * 8);
+          uint2 sc = *reinterpret_cast<const uint2*>(st + P.L.k_scale_off + tok * 8);
+          if (pf_q8_big(sc)) sc = make_uint2(pf_div128(sc.x), pf_div128(sc.y));
           pf_q8_token<true, TQ_D, TILE>(st + P.L.k_idx_off + tok * TQ_D, dst, sc.x, sc.y, lane);
+          bool any = false;
+          for (int t = tl; t < PF_PAGE; t += 32 * SP::PW) {   // the factors of all columns of S
+            const bool big = pf_q8_big(*reinterpret_cast<const uint2*>(st + P.L.k_scale_off + t * 8));
+            scales[(i & 3) * PF_ROWS + t] = big ? 128.f : 1.f;
+            any = any || big;
+          }
+          any = __any_sync(0xffffffffu, any);
+          if (lane == 0) *(reinterpret_cast<volatile uint8_t*>(q8_big + (i & 3)) + (tl >> 5)) = any ? 1 : 0;
         } else {
           pf_dequant_token<KB, typename SP::KLut, TQ_D>(st + P.L.k_idx_off + tok * (16 * KB), dst, lk_base, lk_start);
           for (int t = tl; t < PF_PAGE; t += 32 * SP::PW)   // the scales of all columns of S
