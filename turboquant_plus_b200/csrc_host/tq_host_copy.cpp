@@ -7,12 +7,16 @@
 // piece the faults of a fresh 67 MB array took 4 ms.  The threads live for one call and block when they wait; the caller
 // works too, and on a busy machine (BLAS threads spin for some 30 ms after a product) does not wait for a helper that has
 // not got to run yet.  The buffers come from torch's pinned allocator in one block of at most 32 MB, which keeps and
-// reuses it.
+// reuses it.  Pieces move by plain CUDA copies: a helper thread does not have the caller's torch state (inference mode,
+// dispatch modes), and a torch operation on a tensor made under it may be refused there.
 #include "tq_host_copy.h"
 
+#include <ATen/core/CachingHostAllocator.h>
 #include <c10/core/Event.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <string.h>
 
 #include <algorithm>
@@ -185,15 +189,32 @@ int thread_count(const Pieces& p, size_t width) {
   return (int)std::max<int64_t>(1, std::min({(int64_t)MOST_THREADS, p.n, cores / 2, 1 + mega}));
 }
 
+void move(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, const c10::cuda::CUDAStream& stream) {
+  C10_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, kind, stream.stream()));
+}
+
+// tells the pinned allocator that a block is in use until what the stream holds so far has completed
+void in_use(const at::Tensor& t, const c10::cuda::CUDAStream& stream) {
+  at::getHostAllocator(at::kCUDA)->record_event(t.data_ptr(), t.storage().data_ptr().get_context(), stream.unwrap());
+}
+
 // two buffers per thread: [thread][2] of `room` elements
 struct Staging {
   int64_t room;
+  size_t size;                     // bytes of an element
+  c10::cuda::CUDAStream stream;
   at::Tensor all;
   std::vector<c10::Event> moved;
   std::vector<int> uses;
-  Staging(const Pieces& p, int threads, at::ScalarType type)
-      : room(p.longest()), all(pinned(2 * threads * room, type)), uses(threads, 0) {
+  Staging(const Pieces& p, int threads, at::ScalarType type, const c10::cuda::CUDAStream& st)
+      : room(p.longest()), size(at::elementSize(type)), stream(st), all(pinned(2 * threads * room, type)), uses(threads, 0) {
     for (int i = 0; i < 2 * threads; ++i) moved.emplace_back(c10::DeviceType::CUDA);
+  }
+  ~Staging() {
+    try {
+      in_use(all, stream);
+    } catch (...) {   // an earlier error of the device, reported where it was met
+    }
   }
   // the next of a thread's two buffers, free: what was copied from it before has left it
   int take(int thread) {
@@ -201,7 +222,7 @@ struct Staging {
     if (uses[thread]++ >= 2) moved[b].synchronize();
     return b;
   }
-  at::Tensor buffer(int b, int64_t n) const { return all.narrow(0, b * room, n); }
+  uint8_t* buffer(int b) const { return static_cast<uint8_t*>(all.data_ptr()) + (size_t)(b * room) * size; }
 };
 
 }  // namespace
@@ -210,17 +231,16 @@ void to_device(const HostArray& src, const at::Tensor& dst) {
   if (src.count == 0) return;
   const Elem de = elem_of(dst.scalar_type());
   const Pieces pieces(src, de);
-  const at::Tensor flat = dst.view({-1});
+  auto* const to = static_cast<uint8_t*>(dst.data_ptr());
   const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(dst.get_device());
   const int threads = thread_count(pieces, wider(src.elem, de));
-  Staging stage(pieces, threads, dst.scalar_type());
+  Staging stage(pieces, threads, dst.scalar_type(), stream);
   on_threads(pieces.n, threads, stream, [&](int thread, int64_t p) {
     const int64_t at = pieces.begin(p), n = pieces.length(p);
     const int b = stage.take(thread);
-    const at::Tensor buf = stage.buffer(b, n);
-    convert(static_cast<const uint8_t*>(src.data) + at * (int64_t)elem_size(src.elem), src.elem, buf.data_ptr(), de, n);
-    // (the copy tells the pinned allocator that the block is in use until it has completed)
-    flat.narrow(0, at, n).copy_(buf, /*non_blocking=*/true);
+    uint8_t* const buf = stage.buffer(b);
+    convert(static_cast<const uint8_t*>(src.data) + at * (int64_t)elem_size(src.elem), src.elem, buf, de, n);
+    move(to + (size_t)at * stage.size, buf, (size_t)n * stage.size, cudaMemcpyHostToDevice, stream);
     stage.moved[b].record(stream.unwrap());
   });
 }
@@ -239,7 +259,8 @@ void to_host(const std::vector<std::pair<at::Tensor, HostArray>>& jobs) {
     const auto& [t, h] = jobs[j];
     if (h.count == 0 || !is_small(t, h)) continue;
     small.emplace_back(pinned(h.count, t.scalar_type()), j);
-    small.back().first.copy_(t.view({-1}), true);
+    move(small.back().first.data_ptr(), t.const_data_ptr(), t.nbytes(), cudaMemcpyDeviceToHost, stream);
+    in_use(small.back().first, stream);
   }
   c10::Event small_done(c10::DeviceType::CUDA);
   if (!small.empty()) small_done.record(stream.unwrap());
@@ -247,18 +268,18 @@ void to_host(const std::vector<std::pair<at::Tensor, HostArray>>& jobs) {
     if (h.count == 0 || is_small(t, h)) continue;
     const Elem se = elem_of(t.scalar_type());
     const Pieces pieces(h, se);
-    const at::Tensor flat = t.view({-1});
+    const auto* const from = static_cast<const uint8_t*>(t.const_data_ptr());
     const int threads = thread_count(pieces, wider(se, h.elem));
-    Staging stage(pieces, threads, t.scalar_type());
+    Staging stage(pieces, threads, t.scalar_type(), stream);
     const HostArray to = h;
     on_threads(pieces.n, threads, stream, [&](int thread, int64_t p) {
       const int64_t at = pieces.begin(p), n = pieces.length(p);
       const int b = stage.take(thread);
-      const at::Tensor buf = stage.buffer(b, n);
-      buf.copy_(flat.narrow(0, at, n), true);
+      uint8_t* const buf = stage.buffer(b);
+      move(buf, from + (size_t)at * stage.size, (size_t)n * stage.size, cudaMemcpyDeviceToHost, stream);
       stage.moved[b].record(stream.unwrap());
       stage.moved[b].synchronize();
-      convert(buf.data_ptr(), se, static_cast<uint8_t*>(to.data) + at * (int64_t)elem_size(to.elem), to.elem, n);
+      convert(buf, se, static_cast<uint8_t*>(to.data) + at * (int64_t)elem_size(to.elem), to.elem, n);
     });
   }
   if (!small.empty()) {
