@@ -26,6 +26,7 @@ template <> __device__ __forceinline__ double dn_d<__half>(__half v) { return (d
 // A CTA's eight warps: WM along the vectors, WN along the outputs; a warp holds 16 MF vectors x 8 NF outputs.
 template <int MF_, int NF_, int WM_> struct DnTile {
   static constexpr int MF = MF_, NF = NF_, WM = WM_, WN = DN_WARPS / WM, MT = 16 * MF * WM;
+  static constexpr int DP = 8 * NF * WN;   // largest padded d
 };
 
 template <int MF, int NF> __device__ __forceinline__ void dn_zero(double (&c)[MF][NF][4]) {
@@ -414,15 +415,15 @@ __global__ void __launch_bounds__(DN_THREADS, 2) k_dense_dequantize(const TqDens
       }
 }
 
-template <auto kernel> int dn_configure(size_t smem) {
+// Raises the kernel's limit to `most`, what it takes at its largest d whatever this call's d is: the limit belongs to the
+// process, and a thread that set it to the size of its own call would lower it under the others'.
+template <auto kernel> int dn_configure(size_t most) {
   static thread_local int configured_dev = -1;   // one per kernel: the kernel is a template argument
-  static thread_local size_t configured = 0;
   int dev = 0;
   TQ_CUDA(cudaGetDevice(&dev));
-  if (configured_dev != dev || configured < smem) {
-    TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (configured_dev != dev) {
+    TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     configured_dev = dev;
-    configured = smem;
   }
   return TQ_OK;
 }
@@ -441,8 +442,9 @@ template <typename Tin, typename E>
 int dn_launch_quantize(const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, cudaStream_t st) {
   return dn_pick(a.dp, n, [&](auto tile) {
     using TL = decltype(tile);
-    const size_t smem = dn_stage_bytes<E, TL::MT>(a.dp) + (size_t)TL::MT * dn_istride(a.d);
-    const int rc = dn_configure<k_dense_quantize<Tin, E, TL>>(smem);
+    auto bytes = [](int d, int dp) { return dn_stage_bytes<E, TL::MT>(dp) + (size_t)TL::MT * dn_istride(d); };
+    const size_t smem = bytes(a.d, a.dp);
+    const int rc = dn_configure<k_dense_quantize<Tin, E, TL>>(bytes(TL::DP, TL::DP));
     if (rc != TQ_OK) return rc;
     k_dense_quantize<Tin, E, TL><<<(unsigned)((n + TL::MT - 1) / TL::MT), DN_THREADS, smem, st>>>(a, (const Tin*)x, ld, n);
     return tq_launch_check("k_dense_quantize");
@@ -454,7 +456,7 @@ int dn_launch_dequantize(const TqDenseDequant& a, int64_t n, void* out, cudaStre
   return dn_pick(a.dp, n, [&](auto tile) {
     using TL = decltype(tile);
     const size_t smem = (size_t)TL::MT * (dn_istride(a.d) + (a.qjl ? (a.d + 7) / 8 : 0));
-    const int rc = dn_configure<k_dense_dequantize<Tout, TL>>(smem);
+    const int rc = dn_configure<k_dense_dequantize<Tout, TL>>((size_t)TL::MT * (dn_istride(TL::DP) + TL::DP / 8));
     if (rc != TQ_OK) return rc;
     k_dense_dequantize<Tout, TL><<<(unsigned)((n + TL::MT - 1) / TL::MT), DN_THREADS, smem, st>>>(a, n, (Tout*)out);
     return tq_launch_check("k_dense_dequantize");
