@@ -241,16 +241,17 @@ PyObject* workspace_bytes(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// quantize(quantizer, x (n, d), bits, packed, want_scale, want_qjl) -> (codes, norms, scales or None, sketch or None,
-// residual norms or None), all on x's device
+// quantize(quantizer, x (n, d or more columns, of which the first d count), d, bits, packed, want_scale, want_qjl) -> (codes,
+// norms, scales or None, sketch or None, residual norms or None), all on x's device
 PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    need(n, 6, "quantize");
+    need(n, 7, "quantize");
     const at::Tensor& x = tensor(a[1], "x");
     const c10::Device dev = x.device();
-    if (!dev.is_cuda() || x.dim() != 2) raise(PyExc_ValueError, "x must be a CUDA tensor of shape (n, d)");
-    const int64_t nv = x.size(0), d = x.size(1), bits = integer(a[2]);
-    const bool packed = PyObject_IsTrue(a[3]) == 1, scale = PyObject_IsTrue(a[4]) == 1, qjl = PyObject_IsTrue(a[5]) == 1;
+    const int64_t d = integer(a[2]), bits = integer(a[3]);
+    if (!dev.is_cuda() || x.dim() != 2 || x.size(1) < d) raise(PyExc_ValueError, "x must be a CUDA tensor of shape (n, d)");
+    const int64_t nv = x.size(0);
+    const bool packed = PyObject_IsTrue(a[4]) == 1, scale = PyObject_IsTrue(a[5]) == 1, qjl = PyObject_IsTrue(a[6]) == 1;
     const auto u8 = x.options().dtype(at::kByte), f32 = x.options().dtype(at::kFloat);
     at::Tensor codes = at::empty({nv, packed ? d * bits / 8 : d}, u8), norms = at::empty({nv}, f32), scales, sketch, rnorms;
     if (scale) scales = at::empty({nv}, f32);

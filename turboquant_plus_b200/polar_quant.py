@@ -101,7 +101,7 @@ class PolarQuant:
     def quantize_device(self, xt, *, packed=False, want_scale=False):
         """xt: (n, d) CUDA tensor.  Returns dict with 'idx' (n, d) uint8 or 'packed'
         (n, d*bits/8) uint8, 'norm' (n,) fp32 and optionally 'scale' (n,) fp32."""
-        codes, norm, scale, _, _ = nv.host().quantize(self._native(xt.device).address, xt, self.bit_width, packed,
+        codes, norm, scale, _, _ = nv.host().quantize(self._native(xt.device).address, xt, self.d, self.bit_width, packed,
                                                       want_scale, False)
         out = {"norm": norm, "packed" if packed else "idx": codes}
         if want_scale:

@@ -71,7 +71,7 @@ class TurboQuant:
     def quantize_device(self, xt, *, packed=False, want_scale=False):
         """(n, d) CUDA tensor -> dict of CUDA tensors: 'idx' or 'packed', 'norm', 'qjl' (n, d/8) packed
         sign bits, 'rnorm', optionally 'scale'."""
-        codes, norm, scale, qjl, rnorm = nv.host().quantize(self._native(xt.device).address, xt, self.polar_quant.bit_width,
+        codes, norm, scale, qjl, rnorm = nv.host().quantize(self._native(xt.device).address, xt, self.d, self.polar_quant.bit_width,
                                                             packed, want_scale, True)
         out = {"norm": norm, "rnorm": rnorm, "qjl": qjl, "packed" if packed else "idx": codes}
         if want_scale:
