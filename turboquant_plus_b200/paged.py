@@ -178,6 +178,13 @@ class PagedKVCache:
                 nv.call("tq_cache_requantize", self._handle(a), dst._handle(b), C.byref(self.layout), nv.ptr(self.pool),
                         nv.ptr(ss), C.byref(dst.layout), nv.ptr(dst.pool), nv.ptr(ds), which, ss.numel(), nv.stream_ptr())
 
+    @staticmethod
+    def _rows_like(out, q):
+        """Whether a kernel can store its rows for ``q`` in ``out`` directly."""
+        torch = nv.require_cuda()
+        return (out.shape == q.shape and out.is_contiguous() and out.device == q.device and out.data_ptr() % 16 == 0
+                and out.dtype in (torch.float16, torch.bfloat16, torch.float32))
+
     def prefill_attend(self, q, block_table, kv_lens, scale=None, out=None, workspace=None):
         """Chunked prefill on the tcgen05 tensor cores.  q: (batch, chunk_tokens, num_q_heads, head_dim) CUDA
         tensor of a chunk whose K/V rows are already in the cache; kv_lens: (batch,) cached tokens including
@@ -185,7 +192,8 @@ class PagedKVCache:
         formats on 128-token pages takes the tcgen05 kernel."""
         bsz, tq, hq, d = q.shape
         assert d == self.head_dim
-        if self.page_tokens != 128 and not (self.k_format.startswith("turbo") and self.v_format.startswith("turbo")):
+        turbo = self.k_format.startswith("turbo") and self.v_format.startswith("turbo")
+        if self.page_tokens != 128 and not turbo:
             torch = nv.require_cuda()
             q = q.contiguous()
             bt = block_table.to(device=self.device, dtype=torch.int32).contiguous()
@@ -199,9 +207,17 @@ class PagedKVCache:
                 out.copy_(res)
                 return out
             return res
+        need = nv.host().workspace_bytes(bsz, hq, self.num_kv_heads, block_table.shape[1], tq)
         ws = workspace
+        if not turbo:
+            # (PROD and q8_0 tensors took the decode kernel's own scratch and a copy into ``out``: what was passed then still is)
+            if out is not None and not self._rows_like(out, q):
+                out.copy_(self.prefill_attend(q, block_table, kv_lens, scale, None, workspace))
+                return out
+            if ws is not None and (ws.numel() < need or ws.numel() % 256 or ws.data_ptr() % 256):
+                ws = None
         if ws is None:
-            ws = self._scratch(nv.host().workspace_bytes(bsz, hq, self.num_kv_heads, block_table.shape[1], tq))
+            ws = self._scratch(need)
         return nv.host().prefill(self._address(self.k_quantizer), self._address(self.v_quantizer), C.addressof(self.layout),
                                  self.pool, q, block_table, kv_lens, float(scale) if scale else 0.0, out, ws)
 
