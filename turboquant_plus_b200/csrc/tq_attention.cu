@@ -488,6 +488,17 @@ SplitPlan plan_splits(int batch, int hkv, int max_pages) {
   return p;
 }
 
+// The coarsest plan that gives every CTA place an item: the fewest partials of a call that fills the GPU.
+SplitPlan plan_splits_coarse(int batch, int hkv, int max_pages) {
+  const long slots = 2 * tq_num_sms(), items = (long)batch * hkv;
+  if (items >= slots) return plan_splits(batch, hkv, max_pages);
+  const int s = (int)((slots + items - 1) / items);
+  SplitPlan p;
+  p.chunk_pages = (max_pages + s - 1) / s;
+  p.num_splits = (max_pages + p.chunk_pages - 1) / p.chunk_pages;
+  return p;
+}
+
 struct WsLayout {
   size_t qrot, qproj, part_o, part_ml, total;
 };
@@ -592,7 +603,7 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
                        const uint8_t* pool_dev, const int32_t* block_table_dev, int32_t max_pages_per_seq,
                        const int32_t* seq_lens_dev, const void* q_dev, int32_t q_dtype, int32_t batch,
                        int32_t num_q_heads, float scale, void* workspace_dev, int64_t workspace_bytes, void* out_dev,
-                       int32_t out_dtype, int32_t phases, float* lse_dev, void* stream) {
+                       int32_t out_dtype, int32_t phases, float* lse_dev, void* stream, bool coarse = false) {
   TQ_REQUIRE(L, TQ_ERR_INVALID, "tq_decode_attn: layout missing");
   TQ_REQUIRE(batch >= 0 && num_q_heads >= 1 && max_pages_per_seq >= 1, TQ_ERR_INVALID, "bad sizes");
   if (batch == 0) return TQ_OK;
@@ -624,7 +635,7 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
   }
   if (!v_q8) TQ_REQUIRE(vq->d == TQ_D && vq->bits == L->v_format, TQ_ERR_INVALID,
                         "V quantizer bit width does not match the cache format");
-  const SplitPlan plan = plan_splits(batch, L->num_kv_heads, max_pages_per_seq);
+  const SplitPlan plan = (coarse ? plan_splits_coarse : plan_splits)(batch, L->num_kv_heads, max_pages_per_seq);
   const WsLayout w = ws_layout(batch, num_q_heads, plan.num_splits);
   TQ_REQUIRE((int64_t)w.total <= workspace_bytes, TQ_ERR_TOO_LARGE, "workspace of %lld bytes is smaller than the %lld needed",
              (long long)workspace_bytes, (long long)w.total);
@@ -830,8 +841,11 @@ extern "C" int tq_decode_attn_static(const tq_quantizer* kq, const tq_quantizer*
   TQ_REQUIRE(L, TQ_ERR_INVALID, "tq_decode_attn_static: layout missing");
   TQ_REQUIRE(batch >= 0 && num_q_heads >= 1 && max_pages_per_seq >= 1, TQ_ERR_INVALID, "bad sizes");
   if (batch == 0) return TQ_OK;
-  const int64_t need = tq_decode_workspace_bytes(batch, num_q_heads, L->num_kv_heads, max_pages_per_seq);
+  int64_t need = tq_decode_workspace_bytes(batch, num_q_heads, L->num_kv_heads, max_pages_per_seq);
   TQ_REQUIRE(need > 0, TQ_ERR_INVALID, "bad sizes");
+  const bool coarse = need > TQ_STATIC_SCRATCH_BYTES;   // a plan of several rounds has several times the partials
+  if (coarse)
+    need = (int64_t)ws_layout(batch, num_q_heads, plan_splits_coarse(batch, L->num_kv_heads, max_pages_per_seq).num_splits).total;
   TQ_REQUIRE(need <= TQ_STATIC_SCRATCH_BYTES, TQ_ERR_TOO_LARGE,
              "tq_decode_attn_static: this shape needs %lld bytes of scratch, the built-in array holds %d "
              "(batch %d x %d query heads x %d pages); use tq_decode_attn with a caller-owned workspace",
@@ -847,9 +861,8 @@ extern "C" int tq_decode_attn_static(const tq_quantizer* kq, const tq_quantizer*
   uint8_t* tail = (uint8_t*)scratch + TQ_STATIC_SCRATCH_BYTES - TAIL_BYTES;
   const size_t counters = (size_t)batch * L->num_kv_heads;
   TQ_CUDA(cudaMemsetAsync(tail, 0, (counters < (size_t)MAX_TICKETS ? counters : (size_t)MAX_TICKETS) * 4, (cudaStream_t)stream));
-  return tq_decode_attn_phases(kq, vq, L, pool_dev, block_table_dev, max_pages_per_seq, seq_lens_dev, q_dev, q_dtype,
-                               batch, num_q_heads, scale, scratch, TQ_STATIC_SCRATCH_BYTES, out_dev, out_dtype, 3,
-                               stream);
+  return decode_impl(kq, vq, L, pool_dev, block_table_dev, max_pages_per_seq, seq_lens_dev, q_dev, q_dtype, batch,
+                     num_q_heads, scale, scratch, TQ_STATIC_SCRATCH_BYTES, out_dev, out_dtype, 3, nullptr, stream, coarse);
 }
 
 extern "C" int tq_decode_static_status_sync(int32_t* status_out) {
