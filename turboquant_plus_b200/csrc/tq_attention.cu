@@ -57,14 +57,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) k_decode_attn(const AttnParams
   using SP = SmemPlan<KK, VK>;
   constexpr int KB = KT::BITS, VB = VT::BITS;
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  int split, kvh, b;
+  split_index(P, split, kvh, b);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int PT = P.L.page_tokens;
   // a length beyond the block-table row (or a negative one) is clamped: page numbers are only ever read from the
   // row's max_pages entries, and the split count stays inside the plan the workspace was sized for
   const int seq_len = min(max(P.seq_lens[b], 0), P.max_pages * PT);
   const int n_pages = (seq_len + PT - 1) / PT;
-  const int page_lo = split * P.chunk_pages;
+  const int chunk = split_chunk(P, PT, lane), page_lo = split * chunk;
   const size_t row0 = (size_t)b * P.hq + (size_t)kvh * P.group;  // first query / output row of this CTA
   if (n_pages == 0 && split == 0) {  // empty sequence: zeros
     for (int e = tid; e < P.group * TQ_D; e += ATT_THREADS) store_out(P.out, P.out_dtype, row0 * TQ_D + e, 0.f);
@@ -72,9 +73,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) k_decode_attn(const AttnParams
     return;
   }
   if (page_lo >= n_pages) return;
-  const int page_hi = min(n_pages, page_lo + P.chunk_pages);
+  const int page_hi = min(n_pages, page_lo + chunk);
   const int np = page_hi - page_lo;
-  const int ns = (n_pages + P.chunk_pages - 1) / P.chunk_pages;  // splits of this sequence that run
+  const int ns = (n_pages + chunk - 1) / chunk;  // splits of this sequence that run
 
   // align the carve-up to the largest table
   const uint32_t raw = smem_u32(smem_raw);
@@ -465,19 +466,82 @@ __global__ void __launch_bounds__(128) k_prepare_queries(const Tq* __restrict__ 
 // cost of a CTA, about six pages: prologue, partial, tail) + the fold of the partials (a page per 32 splits).  Rounds
 // count whole: 16 items x 19 splits are 304 CTAs on 296 places, and the eight of the second round took as long as all
 // others together (2 x 131,072 tokens of turbo4, 64/8 heads: 133 us).
+//
+// That is the plan of a batch whose sequences are all as long as the block table is wide.  Its long chunks are one CTA's
+// serial stream each: of a ragged batch the longest sequence alone sets the time, while places whose items were short stay
+// empty (16 sequences spread evenly over [1,024, 32,768] tokens, 8 KV heads, turbo3: 2 x 128 pages per item 150 us, as
+// long as 16 full ones; 3 x 86 105).  The lengths are on the device, so a batch of several sequences gets a second, finer
+// chunk (SplitPlan::Spread) and every CTA chooses by the sum of the lengths.  In pages: with all CTAs resident a call takes
+// its longest chunk, 1.15 (c + 6) with two CTAs per SM and 2 (c + 6) with four; otherwise the whole work (pages + 7 per
+// CTA) over the places, 13 % less with four per SM, and about half of a chunk's time for the tail; a page per 16 splits goes
+// into the fold.  The second chunk is the best by this estimate for lengths spread evenly up to the table's width, and the
+// line where the two plans meet is the bound; a batch of at least nine tenths of the table always takes the first, and a
+// bound that such a ragged batch would not reach is not worth the sum (0.3 us of a call).  A plan finer than the coarsest
+// that fills the GPU has to promise 7 %: closer ones were behind (12 sequences up to 8,192 tokens: 4 x 16 pages 27.1 us,
+// 6 x 11 28.9).  Turbo3, 32/8 heads, spread evenly over [1/32, 1] of 32,768 tokens, one plan -> two: 8 sequences 79 -> 55 us,
+// 16 150 -> 94, 32 274 -> 160; full ones as before (147 and 283 us for 16 and 32).
+struct SplitCost {
+  double fixed, per_page;   // time of a call as a function of its pages
+  double at(double pages) const { return fixed + per_page * pages; }
+};
+SplitCost split_cost(long chunk, long splits, int batch, int hkv, int four) {
+  const double places = 2.0 * tq_num_sms(), unit = (double)chunk + 6, fold = (double)splits / 16;
+  if ((double)batch * hkv * splits <= places * (1 + four)) return {(four ? 2.0 : 1.15) * unit + fold, 0.0};
+  const double k = (four ? 0.87 : 1.0) * hkv / places;
+  return {k * 3.5 * batch + (four ? 0.6 : 0.5) * unit + fold, k * (1 + 7.0 / (double)chunk)};
+}
+SplitPlan::Spread plan_spread(const SplitPlan& p, int batch, int hkv, int max_pages, int four) {
+  const long places = 2L * tq_num_sms() * (1 + four), items = (long)batch * hkv;
+  SplitPlan::Spread best{};
+  const SplitCost even = split_cost(p.chunk_pages, p.num_splits, batch, hkv, four);
+  const double table = (double)batch * max_pages;
+  double least = 0;
+  long best_rounds = 0;
+  SplitCost cost{};
+  for (long rounds = 0; rounds <= 8; ++rounds) {   // (0: the coarsest plan that fills the GPU)
+    long s = rounds ? rounds * places / items : (2L * tq_num_sms() + items - 1) / items;
+    if (s < 1) continue;
+    if (s > max_pages) s = max_pages;
+    if (s > 2L * tq_num_sms()) s = 2L * tq_num_sms();
+    const long chunk = (max_pages + s - 1) / s;
+    if (chunk >= p.chunk_pages) continue;
+    s = (max_pages + chunk - 1) / chunk;
+    const SplitCost c = split_cost(chunk, s, batch, hkv, four);
+    double t = c.at(0.515 * table + 0.5 * batch);
+    if (four && t < 2.0 * (chunk + 6)) t = 2.0 * (chunk + 6);
+    if (best.chunk_pages && t >= (best_rounds ? 1.0 : 0.93) * least) continue;
+    best_rounds = rounds;
+    least = t;
+    cost = c;
+    best.chunk_pages = (int)chunk;
+    best.num_splits = (int)s;
+  }
+  if (!best.chunk_pages || even.fixed <= cost.fixed) return {};
+  double below = 0.9 * table;
+  if (cost.per_page > even.per_page) {
+    const double meet = (even.fixed - cost.fixed) / (cost.per_page - even.per_page);
+    if (meet < below) below = meet;
+  }
+  if (below <= 0.52 * table) return {};
+  best.below = (int)below;
+  return best;
+}
 SplitPlan plan_splits(int batch, int hkv, int max_pages) {
   const long slots = 2 * tq_num_sms(), items = (long)batch * hkv;
-  SplitPlan p;
+  SplitPlan p{};
   if (max_pages < 1) max_pages = 1;
   if (items >= slots) {   // enough items: chunks of 32 pages balance ragged sequences
     p.chunk_pages = max_pages < 32 ? max_pages : 32;
   } else {
+    // candidates: the largest count of each number of rounds, and the one where a page less per split costs as much fold
     const long most = slots < max_pages ? slots : max_pages;
     long best = -1;
     p.chunk_pages = max_pages;
-    for (long s = 1; s <= most; ++s) {
-      const long pages = (max_pages + s - 1) / s, rounds = (items * ((max_pages + pages - 1) / pages) + slots - 1) / slots;
-      const long cost = 32 * rounds * (pages + 6) + s;
+    for (long r = 0; r <= 16 && r <= items; ++r) {
+      long s = r ? r * slots / items : (long)sqrt(32.0 * max_pages);
+      s = s < 1 ? 1 : s > most ? most : s;
+      const long pages = (max_pages + s - 1) / s, splits = (max_pages + pages - 1) / pages;
+      const long cost = 32 * ((items * splits + slots - 1) / slots) * (pages + 6) + splits;
       if (best < 0 || cost < best) {
         best = cost;
         p.chunk_pages = (int)pages;
@@ -485,6 +549,8 @@ SplitPlan plan_splits(int batch, int hkv, int max_pages) {
     }
   }
   p.num_splits = (max_pages + p.chunk_pages - 1) / p.chunk_pages;
+  if (items < slots && batch > 1)
+    for (int four = 0; four < 2; ++four) p.spread[four] = plan_spread(p, batch, hkv, max_pages, four);
   return p;
 }
 
@@ -493,7 +559,7 @@ SplitPlan plan_splits_coarse(int batch, int hkv, int max_pages) {
   const long slots = 2 * tq_num_sms(), items = (long)batch * hkv;
   if (items >= slots) return plan_splits(batch, hkv, max_pages);
   const int s = (int)((slots + items - 1) / items);
-  SplitPlan p;
+  SplitPlan p{};
   p.chunk_pages = (max_pages + s - 1) / s;
   p.num_splits = (max_pages + p.chunk_pages - 1) / p.chunk_pages;
   return p;
@@ -521,7 +587,8 @@ WsLayout ws_layout(int batch, int hq, int num_splits) {
 }
 
 template <int KK, int VK>
-int launch_attn(const AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
+int launch_attn(const AttnParams& P_in, const SplitPlan& plan, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
+  const AttnParams P = with_splits(P_in, plan, false);
   const size_t need = SmemPlan<KK, VK>::bytes(P.L.record_bytes, P.stages);
   TQ_REQUIRE(need <= 113 * 1024, TQ_ERR_TOO_LARGE, "page record of %d bytes does not fit the shared-memory pipeline",
              P.L.record_bytes);
@@ -532,8 +599,7 @@ int launch_attn(const AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStr
     TQ_CUDA(cudaFuncSetAttribute(k_decode_attn<KK, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024));
     configured_dev = dev;
   }
-  dim3 grid(P.num_splits, P.hkv, P.batch);
-  k_decode_attn<KK, VK><<<grid, ATT_THREADS, need, st>>>(P, fk, fv);
+  k_decode_attn<KK, VK><<<split_grid(P), ATT_THREADS, need, st>>>(P, fk, fv);
   return tq_launch_check("k_decode_attn");
 }
 
@@ -549,7 +615,7 @@ extern "C" int64_t tq_decode_workspace_bytes(int32_t batch, int32_t num_q_heads,
                                              int32_t max_pages_per_seq) {
   if (batch < 1 || num_q_heads < 1 || num_kv_heads < 1 || max_pages_per_seq < 1) return TQ_ERR_INVALID;
   const SplitPlan p = plan_splits(batch, num_kv_heads, max_pages_per_seq);
-  return (int64_t)ws_layout(batch, num_q_heads, p.num_splits).total;
+  return (int64_t)ws_layout(batch, num_q_heads, p.most()).total;
 }
 
 extern "C" int tq_decode_workspace_init(void* workspace_dev, int64_t workspace_bytes, void* stream) {
@@ -636,7 +702,7 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
   if (!v_q8) TQ_REQUIRE(vq->d == TQ_D && vq->bits == L->v_format, TQ_ERR_INVALID,
                         "V quantizer bit width does not match the cache format");
   const SplitPlan plan = (coarse ? plan_splits_coarse : plan_splits)(batch, L->num_kv_heads, max_pages_per_seq);
-  const WsLayout w = ws_layout(batch, num_q_heads, plan.num_splits);
+  const WsLayout w = ws_layout(batch, num_q_heads, plan.most());
   TQ_REQUIRE((int64_t)w.total <= workspace_bytes, TQ_ERR_TOO_LARGE, "workspace of %lld bytes is smaller than the %lld needed",
              (long long)workspace_bytes, (long long)w.total);
   cudaStream_t st = (cudaStream_t)stream;
@@ -688,8 +754,6 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
   P.hq = num_q_heads;
   P.hkv = L->num_kv_heads;
   P.group = group;
-  P.chunk_pages = plan.chunk_pages;
-  P.num_splits = plan.num_splits;
   P.stages = L->record_bytes > 24 * 1024 ? 2 : 3;
   P.overlap = (phases & TQ_DECODE_OVERLAP) ? 1 : 0;
   P.sparse_v = (phases & TQ_DECODE_SPARSE_V) ? 1 : 0;
@@ -711,11 +775,11 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
   rc = TQ_ERR_UNSUPPORTED;
   tq_set_error("decode attention: K format %d with V format %d is not instantiated", L->k_format, L->v_format);
   // 128-token pages take the kernel specialised for that shape and the number of heads (tq_decode_g4.cuh)
-  if (group <= 4 ? tq_decode_g4_try(P, fk, fv, st, &rc) : tq_decode_g8_try(P, fk, fv, st, &rc)) return rc;
+  if (group <= 4 ? tq_decode_g4_try(P, plan, fk, fv, st, &rc) : tq_decode_g8_try(P, plan, fk, fv, st, &rc)) return rc;
   if (after_append) P.overlap = P.q_early = P.tail_late = 0;   // the general kernel: stream order
   rc = TQ_ERR_UNSUPPORTED;
 #define TQ_ATT(K, V) \
-  if (L->k_format == K && L->v_format == V) rc = launch_attn<K, V>(P, fk, fv, st);
+  if (L->k_format == K && L->v_format == V) rc = launch_attn<K, V>(P, plan, fk, fv, st);
   TQ_ATT(2, 2) TQ_ATT(2, 3) TQ_ATT(2, 4) TQ_ATT(3, 2) TQ_ATT(3, 3) TQ_ATT(3, 4) TQ_ATT(4, 2) TQ_ATT(4, 3) TQ_ATT(4, 4)
   TQ_ATT(8, 2) TQ_ATT(8, 3) TQ_ATT(8, 4) TQ_ATT(8, 8)
   TQ_ATT(18, 2) TQ_ATT(18, 3) TQ_ATT(19, 2) TQ_ATT(19, 3) TQ_ATT(19, 4) TQ_ATT(20, 3) TQ_ATT(20, 4)

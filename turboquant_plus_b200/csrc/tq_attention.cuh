@@ -132,6 +132,8 @@ struct AttnParams {
   int32_t tail_late;   // the preceding kernel may write the last cached position of a sequence: its page is fetched
                        // after the dependency wait, every other page before (TQ_DECODE_OVERLAP_APPEND)
   int32_t chain_head;  // attention calls with TQ_DECODE_OVERLAP_Q follow this one (TQ_DECODE_CHAIN_HEAD)
+  int32_t chunk_spread, spread_below;  // second chunk of SplitPlan, and the cached pages of the batch below which it is
+                                       // taken; 0: none.  The grid then has the splits as its slowest dimension.
   tq_cache_layout L;
 };
 
@@ -352,15 +354,60 @@ __device__ __forceinline__ void load_q4(const void* q, int dtype, size_t i, floa
   }
 }
 
-// Split plan shared by the launchers and the workspace sizing.
+// Split plan shared by the launchers and the workspace sizing: pages per CTA (chunk_pages) and CTAs per (sequence, KV
+// head) for a batch whose sequences fill the block table, and, per form of the kernel ([0]: two CTAs per SM, [1]: four),
+// those of a batch whose sequences together have fewer than `below` pages (chunk_pages 0: the same).
 struct SplitPlan {
   int chunk_pages, num_splits;
+  struct Spread {
+    int chunk_pages, num_splits, below;
+  } spread[2];
+  int most() const {   // partials per row that a workspace holds
+    int m = num_splits;
+    for (const Spread& s : spread)
+      if (s.chunk_pages && s.num_splits > m) m = s.num_splits;
+    return m;
+  }
 };
+
+// `P` with the splits of a launch of a form.  Calls in a chain overlap each other's tails, which is what the second chunk
+// is for: they keep the first.
+inline AttnParams with_splits(const AttnParams& P, const SplitPlan& plan, bool four) {
+  AttnParams Q = P;
+  const SplitPlan::Spread& s = plan.spread[four ? 1 : 0];
+  Q.chunk_pages = plan.chunk_pages;
+  Q.num_splits = plan.num_splits;
+  Q.chunk_spread = Q.spread_below = 0;
+  if (s.chunk_pages && (!(P.q_early || P.chain_head) || P.tail_late)) {
+    Q.chunk_spread = s.chunk_pages;
+    Q.spread_below = s.below;
+    if (s.num_splits > Q.num_splits) Q.num_splits = s.num_splits;
+  }
+  return Q;
+}
+inline dim3 split_grid(const AttnParams& P) {
+  return P.chunk_spread ? dim3(P.hkv, P.batch, P.num_splits) : dim3(P.num_splits, P.hkv, P.batch);
+}
+// this CTA's split, KV head and sequence
+__device__ __forceinline__ void split_index(const AttnParams& P, int& split, int& kvh, int& b) {
+  const bool last = P.chunk_spread != 0;
+  split = last ? blockIdx.z : blockIdx.x;
+  kvh = last ? blockIdx.x : blockIdx.y;
+  b = last ? blockIdx.y : blockIdx.z;
+}
+// pages per CTA of this call, the same in every CTA; called by whole warps
+__device__ __forceinline__ int split_chunk(const AttnParams& P, int page_tokens, int lane) {
+  if (P.chunk_spread == 0) return P.chunk_pages;
+  int pages = 0;
+  for (int i = lane; i < P.batch; i += 32)
+    pages += (min(max(P.seq_lens[i], 0), P.max_pages * page_tokens) + page_tokens - 1) / page_tokens;
+  return __reduce_add_sync(0xffffffffu, pages) < P.spread_below ? P.chunk_spread : P.chunk_pages;
+}
 
 }  // namespace tqatt
 
 // tq_decode_g4.cu, tq_decode_g8.cu: launch the kernel specialised for <= 4 and 5..8 query heads per KV head on 128-token
 // pages in the layout tq_cache_layout_init produces.  Return false (nothing launched) when the call is not of that
 // shape; otherwise *rc is the launch status.
-bool tq_decode_g4_try(const tqatt::AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st, int* rc);
-bool tq_decode_g8_try(const tqatt::AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st, int* rc);
+bool tq_decode_g4_try(const tqatt::AttnParams& P, const tqatt::SplitPlan& plan, const TqFast& fk, const TqFast& fv, cudaStream_t st, int* rc);
+bool tq_decode_g8_try(const tqatt::AttnParams& P, const tqatt::SplitPlan& plan, const TqFast& fk, const TqFast& fv, cudaStream_t st, int* rc);

@@ -568,7 +568,8 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
   using VT = Kind<VK>;
   constexpr int KB = KT::BITS, VB = VT::BITS;
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  int split, kvh, b;
+  split_index(P, split, kvh, b);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   constexpr int bar_id = 0;
   {  // one parameter line per warp, all misses in flight together
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     if constexpr (VB > 0) g4_lut_fill<typename C::VLut, VB>(sm + C::OFF_V, fv.cent16, tid, NT);
     TQ_PDL_ENTER();
   }
-  const int page_lo = split * P.chunk_pages;
+  const int chunk = split_chunk(P, G4_PT, lane), page_lo = split * chunk;
   const size_t row0 = (size_t)b * P.hq + (size_t)kvh * P.group;
   const int32_t* bt = P.block_table + (size_t)b * P.max_pages;
   uint8_t* smg = sm + C::OFF_GROUPS;
@@ -620,7 +621,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
   // row's max_pages entries and the split count stays inside the plan the workspace was sized for.
   const int seq_len = min(max(P.seq_lens[b], 0), P.max_pages * G4_PT);
   const int n_pages = (seq_len + G4_PT - 1) / G4_PT;
-  const int np = min(n_pages, page_lo + P.chunk_pages) - page_lo;   // pages of this CTA (<= 0: none)
+  const int np = min(n_pages, page_lo + chunk) - page_lo;   // pages of this CTA (<= 0: none)
   int pg_ahead = 0;  // producer: block-table entry of the page issued in the next iteration
   if (tid == PRODUCER) {   // (where every warp rotates a query, this one does so afterwards)
     int pg_next[G4_NS];
@@ -687,7 +688,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     for (int e = tid; e < P.group * TQ_D; e += NT) store_out(P.out, P.out_dtype, row0 * TQ_D + e, 0.f);
     if (P.lse && tid < P.group) P.lse[row0 + tid] = -INFINITY;
   }
-  const int ns = (n_pages + P.chunk_pages - 1) / P.chunk_pages;
+  const int ns = (n_pages + chunk - 1) / chunk;
   __syncthreads();               // tables, query buffer and mbarriers are ready
   if (np <= 0) return;           // this CTA has no pages (its split lies beyond the sequence)
 
@@ -857,7 +858,8 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
 }
 
 template <int KK, int VK, bool SPARSE, bool NODEQ, int NW = ATT_WARPS, bool TAIL = false, int NH = 4>
-int launch_attn_g4(const AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
+int launch_attn_g4(const AttnParams& P_in, const SplitPlan& plan, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
+  const AttnParams P = with_splits(P_in, plan, NW == 4);
   using C = G4<KK, VK, NW, NH>;
   static_assert((16 / NW) * (C::SMEM + 1024) <= 228 * 1024, "CTAs of the specialised decode kernel per SM");
   static thread_local int configured_dev = -1;  // per instantiation
@@ -873,7 +875,7 @@ int launch_attn_g4(const AttnParams& P, const TqFast& fk, const TqFast& fv, cuda
   memcpy(ak.s1, fk.s1, 16); memcpy(ak.s2, fk.s2, 16); memcpy(ak.j1, fk.j1, 16); memcpy(ak.j2, fk.j2, 16);
   memcpy(ak.cent16, fk.cent16, 32); ak.alpha = fk.lut_alpha;
   memcpy(av.s1, fv.s1, 16); memcpy(av.s2, fv.s2, 16); memcpy(av.cent16, fv.cent16, 32); av.alpha = fv.lut_alpha;
-  TQ_CUDA(tq_launch_early(k_decode_attn_g4<KK, VK, SPARSE, NODEQ, NW, TAIL, NH>, dim3(P.num_splits, P.hkv, P.batch), 32 * NW,
+  TQ_CUDA(tq_launch_early(k_decode_attn_g4<KK, VK, SPARSE, NODEQ, NW, TAIL, NH>, split_grid(P), 32 * NW,
                           C::SMEM, st, P, ak, av));
   return tq_launch_check("k_decode_attn_g4");
 }
@@ -893,10 +895,10 @@ bool layout_matches(const tq_cache_layout& L) {
 // turbo3: 529 us with eight warps, 457 with four).  A call of one round on its own takes the eight-warp form (16 sequences:
 // 43 against 47 us).  4-bit tables: only the eight-warp form has room for lane-replicated ones, which is worth more (turbo4 /
 // turbo4, 16 sequences of 8,192 tokens, per call of a chain: 62 us with four warps and one copy of the tables, 40 with eight).
-inline bool four_warps(const AttnParams& P) {
+inline bool four_warps(const AttnParams& P, const SplitPlan& plan) {
   if (P.L.k_format == TQ_FMT_TURBO4 || P.L.v_format == TQ_FMT_TURBO4) return false;   // (prod4: 3 bits and the sketch)
   if ((P.q_early || P.chain_head) && !P.tail_late) return true;
-  return (int64_t)P.num_splits * P.hkv * P.batch > 2 * (int64_t)tq_num_sms();
+  return (int64_t)plan.num_splits * P.hkv * P.batch > 2 * (int64_t)tq_num_sms();
 }
 
 }  // namespace
