@@ -668,8 +668,15 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     const int tq = lane >> 3, jq = lane & 7;
     *reinterpret_cast<float4*>(qbuf + hd * TQ_D + 4 * (8 * tq + (jq ^ (tq + 4 * (hd & 1))))) =
         make_float4(x[0], x[1], x[2], x[3]);
-    if constexpr (KT::PROD)   // projected queries: plain rows behind the rotated ones
-      *reinterpret_cast<float4*>(qbuf + (NH + hd) * TQ_D + 4 * lane) = make_float4(y[0], y[1], y[2], y[3]);
+    if constexpr (KT::PROD) {
+      // projected queries behind the rotated ones, dim 32 t + c of head h at (c NH + h) 4 + t: the fragment reads below (one
+      // c, all t and h) then are 32 neighbouring floats.  As plain rows they all fell into one bank, 32 reads of 32
+      // wavefronts in every warp: with eight heads this cost more than the general kernel's whole lead (prod3 / turbo3, one
+      // sequence of 4,096 tokens, 64/8 heads: general kernel 16.6 us, 19.0 -> 11.4; 32/8 heads 12.7 -> 9.0)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        qbuf[NH * TQ_D + ((4 * (lane & 7) + k) * NH + hd) * 4 + (lane >> 3)] = y[k];
+    }
     if constexpr (NH <= NW) break;
   }
   __syncwarp();
@@ -721,9 +728,9 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
       if constexpr (KT::PROD) {
         // sign-sketch operands pair dims i and i + 16 of the thread's 32 (i = 2j for the first register of the
         // k-step, 2j + 1 for the second), dim i + 16 in the low half
-        const float* ph = qh + NH * TQ_D + 32 * t;
-        const float a0 = hv ? ph[16 + 2 * j] : 0.f, a1 = hv ? ph[2 * j] : 0.f;
-        const float b0 = hv ? ph[16 + 2 * j + 1] : 0.f, b1 = hv ? ph[2 * j + 1] : 0.f;
+        const float* ph = qbuf + NH * TQ_D + (hv ? head : 0) * 4 + t;
+        auto proj = [&](int c) { return hv ? ph[c * (4 * NH)] : 0.f; };
+        const float a0 = proj(16 + 2 * j), a1 = proj(2 * j), b0 = proj(16 + 2 * j + 1), b1 = proj(2 * j + 1);
         const __half2 e0 = __floats2half2_rn(a0, a1), e1 = __floats2half2_rn(b0, b1);
         const float2 r0 = __half22float2(e0), r1 = __half22float2(e1);
         const uint32_t m0 = pack_h2(a0 - r0.x, a1 - r0.y), m1 = pack_h2(b0 - r1.x, b1 - r1.y);
