@@ -900,12 +900,19 @@ bool layout_matches(const tq_cache_layout& L) {
 // stream pages: in a chain of attention calls (TQ_DECODE_OVERLAP_Q, and the call in front of them when the caller says so,
 // TQ_DECODE_CHAIN_HEAD), and inside a call of more CTAs than one round at two per SM (256 sequences of 8,192 tokens of
 // turbo3: 529 us with eight warps, 457 with four).  A call of one round on its own takes the eight-warp form (16 sequences:
-// 43 against 47 us).  4-bit tables: only the eight-warp form has room for lane-replicated ones, which is worth more (turbo4 /
-// turbo4, 16 sequences of 8,192 tokens, per call of a chain: 62 us with four warps and one copy of the tables, 40 with eight).
+// 43 against 47 us).
+// 4-bit tables: only the eight-warp form has room for lane-replicated ones (32 KB each), which is worth more where a CTA
+// streams pages (turbo4 / turbo4, 16 sequences of 8,192 tokens, per call of a chain: 62 us with four warps and one copy of the
+// tables, 37 with eight), but they are filled anew by every CTA: a chain of calls with one or two pages per CTA is ahead with
+// four warps (32/8 heads, 32 sequences of 100 tokens 7.5 -> 5.5 us, 16 of 256 6.9 -> 5.6, 8 of 1,024 7.4 -> 7.1; 16 of 1,024,
+// four pages: 9.9 against 11.0), unless many splits leave a long fold to the four (32 splits of a page: 5.8 against 6.1).
 inline bool four_warps(const AttnParams& P, const SplitPlan& plan) {
-  if (P.L.k_format == TQ_FMT_TURBO4 || P.L.v_format == TQ_FMT_TURBO4) return false;   // (prod4: 3 bits and the sketch)
-  if ((P.q_early || P.chain_head) && !P.tail_late) return true;
-  return (int64_t)plan.num_splits * P.hkv * P.batch > 2 * (int64_t)tq_num_sms();
+  const bool wide = P.L.k_format == TQ_FMT_TURBO4 || P.L.v_format == TQ_FMT_TURBO4;   // (prod4: 3 bits and the sketch)
+  if ((P.q_early || P.chain_head) && !P.tail_late) {
+    if (P.group > 4) return !wide;
+    return !wide || (plan.chunk_pages <= 2 && plan.num_splits <= 16);
+  }
+  return !wide && (int64_t)plan.num_splits * P.hkv * P.batch > 2 * (int64_t)tq_num_sms();
 }
 
 }  // namespace
