@@ -906,10 +906,14 @@ bool layout_matches(const tq_cache_layout& L) {
 // tables, 37 with eight), but they are filled anew by every CTA: a chain of calls with one or two pages per CTA is ahead with
 // four warps (32/8 heads, 32 sequences of 100 tokens 7.5 -> 5.5 us, 16 of 256 6.9 -> 5.6, 8 of 1,024 7.4 -> 7.1; 16 of 1,024,
 // four pages: 9.9 against 11.0), unless many splits leave a long fold to the four (32 splits of a page: 5.8 against 6.1).
+// Five to eight heads: four warps rotate and fold two heads each, 0.6 us and, with several splits, 0.8 us and 0.045 us per
+// split of a chained call, against 0.55 us saved per page of a CTA (64/8 heads of turbo3, eight warps / four: one sequence
+// of 4,096 tokens, 32 x 1 pages 6.7 / 9.8 us, of 65,536, 37 x 14, 23.7 / 21.2; 4 of 4,096, 8 x 4, 9.6 / 9.1; 16/2 heads, one
+// of 65,536, 128 x 4, 11.8 / 17.3).
 inline bool four_warps(const AttnParams& P, const SplitPlan& plan) {
   const bool wide = P.L.k_format == TQ_FMT_TURBO4 || P.L.v_format == TQ_FMT_TURBO4;   // (prod4: 3 bits and the sketch)
   if ((P.q_early || P.chain_head) && !P.tail_late) {
-    if (P.group > 4) return !wide;
+    if (P.group > 4) return !wide && 12 * plan.chunk_pages > (plan.num_splits > 1 ? 31 : 13) + plan.num_splits;
     return !wide || (plan.chunk_pages <= 2 && plan.num_splits <= 16);
   }
   return !wide && (int64_t)plan.num_splits * P.hkv * P.batch > 2 * (int64_t)tq_num_sms();
