@@ -45,13 +45,16 @@ __device__ __forceinline__ uint32_t umma_idesc(int m, int n, bool b_mn_major) {
   return (1u << 4) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 // CG CTAs on one tile: with two, the accumulator's rows 0-127 are the even CTA's tensor memory and 128-255 the odd one's,
-// A likewise, and each CTA's shared memory holds its half of B's columns (N) at the same offsets.  Executed by a whole warp
-// of the even CTA, one elected thread of which issues it: the warp stays converged, so that addresses and descriptors live
-// in uniform registers, which is where the instruction wants them (issued from a branch of one thread, every MMA spent
-// some 75 cycles moving its operands there).
+// A likewise, and each CTA's shared memory holds its half of B's columns (N) at the same offsets.
+// A pair's are executed by a whole warp of the even CTA, one elected thread of which issues them: the warp stays converged, so
+// that addresses and descriptors live in uniform registers, which is where the instruction wants them (issued from a branch
+// of one thread, every MMA spent some 75 cycles moving its operands there).  A CTA on its own issues them from a branch of
+// one thread all the same: it is bound by its shared-memory pipe, and the 18th warp's elections cost more than they save
+// (nine row blocks of 32 query tokens, 8 KV heads, 1,024 pages of turbo3: 838 us with one thread in an earlier form of
+// the kernel, 895 with elections, 851 with one thread now).
 template <int CG> __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
   if constexpr (CG == 1)
-    asm volatile("{\n .reg .pred p, q;\n elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
                  ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
   else
     asm volatile("{\n .reg .pred p, q;\n elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n @q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
@@ -60,7 +63,7 @@ template <int CG> __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint3
 // arrival on `bar` of every CTA of the pair once the MMAs issued so far have completed
 template <int CG> __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   if constexpr (CG == 1)
-    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(sptr(bar)) : "memory");
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sptr(bar)) : "memory");
   else
     asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n @q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n"
                  ::"r"(sptr(bar)), "h"((uint16_t)3) : "memory");
@@ -1037,7 +1040,9 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
     bool okay = pf_wait_warp(q_ready, 0) && __all_sync(0xffffffffu, tb == 0);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t idesc_s = umma_idesc(128 * CG, 128, false), idesc_o = umma_idesc(128 * CG, 128, true);
+    const bool issues = CG == 2 || lane == 0;
     auto qk = [&](int i) {   // S_i = Q K_i^T (fp16 hi and lo halves of Q), into the score buffer of page i
+      if (!issues) return;
       const int bf = i & 1;
       const uint32_t kt = sptr(ktile) + (SP::KBUF == 2 ? bf * KT::TILES * SP::TILE : 0), d = s_col(bf);
 #pragma unroll
@@ -1072,11 +1077,14 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       }
       if (!pf_wait_warp(&p_ready[bf], ph) || !pf_wait_warp(&v_ready[bf], ph)) { okay = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (issues) {
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks)   // O += P_i V_i: P from tensor memory, V tile MN-major, N = 128
-        umma_ts<CG>(TOc, s_col(bf) + ks * 8,
-                    umma_desc(sptr(vtile + bf * SP::TILE) + ks * (4096 / CG), 2048 / CG, 128), idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
-      umma_commit<CG>(&o_done[bf]);
+        for (int ks = 0; ks < 8; ++ks)   // O += P_i V_i: P from tensor memory, V tile MN-major, N = 128
+          umma_ts<CG>(TOc, s_col(bf) + ks * 8,
+                      umma_desc(sptr(vtile + bf * SP::TILE) + ks * (4096 / CG), 2048 / CG, 128), idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
+        umma_commit<CG>(&o_done[bf]);
+      }
+      __syncwarp();
       if (KT::SBUF == 1 && i + 1 < np) {
         // one score buffer: the next page's scores follow once this page's product, which reads P out of it, is done
         if (!pf_wait_warp(&o_done[bf], ph) || !pf_wait_warp(&k_ready[(i + 1) & 1], (uint32_t)(((i + 1) >> 1) & 1))) { okay = false; break; }
