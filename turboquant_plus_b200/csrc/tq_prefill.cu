@@ -209,7 +209,7 @@ template <int KIND> struct PfKind {
   static constexpr bool Q8 = KIND == 8, PROD = KIND >= 18;
   static constexpr int BITS = Q8 ? 0 : (PROD ? KIND - 17 : KIND);
   // K operand tiles of a page.  turbo: centroids (the row scale is applied to the scores in fp32).  q8_0: int8 x block
-  // scale is 19 bits, so its fp16 rounding and the rest, exactly; of a token with a block scale above PF_Q8_BIG, whose
+  // scale is 19 bits, so its fp16 rounding and the rest, exactly; of a token with a block scale of 512 or more, whose
   // products may exceed the fp16 range, divided by 128, which the scores get back in fp32 (what falls below fp16's
   // smallest number then is under 2^-32 of the token's largest element).  PROD: centroids, then +-ratio for the sketch, ratio =
   // residual scale / row scale (one row scale then serves both parts), as its fp16 rounding and the rest of it.
@@ -289,11 +289,10 @@ __device__ __forceinline__ void pf_dequant_token(const uint8_t* src, uint8_t* ds
   }
 }
 
-// q8_0 keys: block scales (fp16 bits; scales are not negative, so that their bits compare like their values) up to this
-// one keep every product int8 x scale within 127 x 512 = 65,024; above it 127 x 65,504 / 128 = 64,992 does
-constexpr uint32_t PF_Q8_BIG = 0x6000;   // 512
+// q8_0 keys: whether one of a token's four block scales (fp16, not negative) is 512 or more, i.e. has its two upper exponent
+// bits set.  Below, every product int8 x scale is at most 127 x 511.75 = 64,992, above, 127 x 65,504 / 128 = 64,992.
 __device__ __forceinline__ bool pf_q8_big(uint2 sc) {
-  return max(max(sc.x & 0xffffu, sc.x >> 16), max(sc.y & 0xffffu, sc.y >> 16)) > PF_Q8_BIG;
+  return (((sc.x & (sc.x << 1)) | (sc.y & (sc.y << 1))) & 0x40004000u) != 0;
 }
 __device__ __forceinline__ uint32_t pf_div128(uint32_t h2) {
   uint32_t d;
@@ -490,7 +489,8 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   uint64_t* xbar = bars + 19;   // one per row quarter: both halves' maxima of a page are in shared memory [2 warps]
   uint32_t* tbase = reinterpret_cast<uint32_t*>(sm + SP::OFF_BAR + 224);
   volatile int* fail = reinterpret_cast<volatile int*>(sm + SP::OFF_BAR + 232);
-  uint32_t* q8_big = reinterpret_cast<uint32_t*>(sm + SP::OFF_BAR + 236);   // [4 slots], a byte per K producer warp: see PfKind
+  uint32_t* q8_big = reinterpret_cast<uint32_t*>(sm + SP::OFF_BAR + 236);   // [4 slots], a byte per K producer warp: its tokens
+                                                                            // have factors (see PfKind) in `scales`
   if (tid == SP::COPIER) {   // lane 0 of the last warp issues the record copies
     auto init = [](uint64_t* bar, int count) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sptr(bar)), "r"(count) : "memory");
@@ -694,7 +694,10 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       const int t0 = (page_lo + i) * PT;
       // a page that every row of this warp sees completely needs no causal mask (rows without a query count as
       // seeing everything: nothing of theirs is stored)
-      const bool masked = !__all_sync(0xffffffffu, !row_ok || t0 + PT - 1 <= pos);
+      // (q8_0: neither does one without factors, which nearly all are: both are the business of the other copy of pass 1)
+      uint32_t big = 0;
+      if constexpr (KT::Q8) big = *reinterpret_cast<volatile uint32_t*>(q8_big + (i & 3));
+      const bool masked = !__all_sync(0xffffffffu, !row_ok || t0 + PT - 1 <= pos) || big != 0;
       // pass 1: this half's scaled scores into registers, row maximum
       float sv[64];
       float mx = -INFINITY;
@@ -704,18 +707,6 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       tmem_ld16_nowait<32>(ts + 64 * hf + 32, raw);
       tmem_ld16_nowait<48>(ts + 64 * hf + 48, raw);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if constexpr (KT::Q8) {   // scores of tokens whose operands are divided by 128: none on most pages
-        if (*reinterpret_cast<volatile uint32_t*>(q8_big + (i & 3))) {
-#pragma unroll
-          for (int j = 0; j < 64; j += 4) {
-            const float4 k4 = ksc4[j >> 2];
-            raw[j] = __float_as_uint(__uint_as_float(raw[j]) * k4.x);
-            raw[j + 1] = __float_as_uint(__uint_as_float(raw[j + 1]) * k4.y);
-            raw[j + 2] = __float_as_uint(__uint_as_float(raw[j + 2]) * k4.z);
-            raw[j + 3] = __float_as_uint(__uint_as_float(raw[j + 3]) * k4.w);
-          }
-        }
-      }
       auto pass1 = [&](auto masked_c) {   // two copies behind a warp-uniform branch: only the diagonal pages pay for the mask
         constexpr bool MASKED = decltype(masked_c)::value;
 #pragma unroll
@@ -729,6 +720,12 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
               const float4 k4 = ksc4[4 * c + (j >> 2)];
               x01 = pf_mul2(x01, make_float2(k4.x, k4.y));
               x23 = pf_mul2(x23, make_float2(k4.z, k4.w));
+            } else if (MASKED) {   // (columns 32 c .. + 31 are producer warp c's, of a pair's two warps c & 1)
+              if ((big >> (8 * ((2 * hf + (c >> 1)) & (SP::PW - 1)))) & 1u) {
+                const float4 k4 = ksc4[4 * c + (j >> 2)];
+                x01 = pf_mul2(x01, make_float2(k4.x, k4.y));
+                x23 = pf_mul2(x23, make_float2(k4.z, k4.w));
+              }
             }
             if (MASKED) {
               const int tt = t0 + 64 * hf + 16 * c + j;
@@ -954,6 +951,7 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       // next page is ready before the rows ask for it.
       const int tl = tid - SP::K_AT, tok = 64 * crank + tl;
       uint8_t* drow = ktile + (tl >> 3) * 2048 + (tl & 7) * 16;
+      uint32_t marked = 0;   // q8_0: slots whose q8_big byte of this warp is set
       for (int i = 0; i < np; ++i) {
         const int bf = i & 1, st_i = i % NST;
         bool ok = !*fail;
@@ -968,16 +966,22 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
         uint8_t* dst = drow + (SP::KBUF == 2 ? bf * KT::TILES * TILE : 0);
         if constexpr (KT::Q8) {
           uint2 sc = *reinterpret_cast<const uint2*>(st + P.L.k_scale_off + tok * 8);
-          if (pf_q8_big(sc)) sc = make_uint2(pf_div128(sc.x), pf_div128(sc.y));
-          pf_q8_token<true, TQ_D, TILE>(st + P.L.k_idx_off + tok * TQ_D, dst, sc.x, sc.y, lane);
-          bool any = false;
-          for (int t = tl; t < PF_PAGE; t += 32 * SP::PW) {   // the factors of all columns of S
-            const bool big = pf_q8_big(*reinterpret_cast<const uint2*>(st + P.L.k_scale_off + t * 8));
-            scales[(i & 3) * PF_ROWS + t] = big ? 128.f : 1.f;
-            any = any || big;
+          // (a pair's CTA has the columns of both: this thread's other token is the other CTA's)
+          const bool own = pf_q8_big(sc);
+          bool other = false;
+          if constexpr (CG == 2) other = pf_q8_big(*reinterpret_cast<const uint2*>(st + P.L.k_scale_off + (tok ^ 64) * 8));
+          const uint32_t slot = 1u << (i & 3);
+          if (__any_sync(0xffffffffu, own || other)) {   // not on most pages: nothing is written for them
+            scales[(i & 3) * PF_ROWS + tok] = own ? 128.f : 1.f;
+            if constexpr (CG == 2) scales[(i & 3) * PF_ROWS + (tok ^ 64)] = other ? 128.f : 1.f;
+            if (own) sc = make_uint2(pf_div128(sc.x), pf_div128(sc.y));
+            if (lane == 0) *(reinterpret_cast<volatile uint8_t*>(q8_big + (i & 3)) + (tl >> 5)) = 1;
+            marked |= slot;
+          } else if (marked & slot) {
+            if (lane == 0) *(reinterpret_cast<volatile uint8_t*>(q8_big + (i & 3)) + (tl >> 5)) = 0;
+            marked &= ~slot;
           }
-          any = __any_sync(0xffffffffu, any);
-          if (lane == 0) *(reinterpret_cast<volatile uint8_t*>(q8_big + (i & 3)) + (tl >> 5)) = any ? 1 : 0;
+          pf_q8_token<true, TQ_D, TILE>(st + P.L.k_idx_off + tok * TQ_D, dst, sc.x, sc.y, lane);
         } else {
           pf_dequant_token<KB, typename SP::KLut, TQ_D>(st + P.L.k_idx_off + tok * (16 * KB), dst, lk_base, lk_start);
           for (int t = tl; t < PF_PAGE; t += 32 * SP::PW)   // the scales of all columns of S
