@@ -1137,29 +1137,25 @@ static int launch_prefill_cg(const PrefillParams& P, const TqFast& fk, const TqF
   return tq_launch_check("k_prefill_attn2");
 }
 
-// CTAs per operand tile: a pair as soon as there are two row blocks to pair.  Not with PROD keys: their one score buffer puts
-// scores, softmax and product of a page one after the other, 3.6 us a page in either form.
-static bool pf_prod(int k_format) { return k_format >= TQ_FMT_PROD2; }
-static int pf_cta_group(int row_blocks, bool prod) { return row_blocks > 1 && !prod ? 2 : 1; }
-
 template <int KK, int VK>
-static int launch_prefill(const PrefillParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
+static int launch_prefill(const PrefillParams& P, int cg, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
   if constexpr (!PfKind<KK>::PROD)
-    if (pf_cta_group(P.row_blocks, false) == 2) return launch_prefill_cg<KK, VK, 2>(P, fk, fv, st);
+    if (cg == 2) return launch_prefill_cg<KK, VK, 2>(P, fk, fv, st);
   return launch_prefill_cg<KK, VK, 1>(P, fk, fv, st);
 }
 
 struct PfPlan {
   int row_blocks, chunk_pages, num_splits;
+  long waves;   // of CTAs
   size_t part_o, part_ml, total;
 };
 static const size_t PF_TAIL = 65536 * 4 + 256;  // tickets + status word, at the end of the workspace
 static const long PF_CTA_COST_PAGES = 12;  // prologue, partial and merge of a CTA, in units of one page of the main loop
 
-static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_pages, bool prod) {
+// the plan of a form: cg CTAs per operand tile
+static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_pages, int cg) {
   PfPlan p;
   p.row_blocks = (chunk_tokens * (hq / hkv) + PF_ROWS - 1) / PF_ROWS;
-  const int cg = pf_cta_group(p.row_blocks, prod);
   const long base = (long)((p.row_blocks + cg - 1) / cg) * hkv * batch;
   const int slots = tq_num_sms() / cg;  // one CTA per SM
   const int cap = max_pages / 8 > 1 ? max_pages / 8 : 1;  // at least eight pages per split
@@ -1176,6 +1172,7 @@ static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_page
   }
   p.chunk_pages = (max_pages + s - 1) / s;
   p.num_splits = (max_pages + p.chunk_pages - 1) / p.chunk_pages;
+  p.waves = (base * p.num_splits + slots - 1) / slots;
   const size_t slots_total = (size_t)p.row_blocks * hkv * batch * p.num_splits;
   p.part_o = 0;
   p.part_ml = slots_total * PF_ROWS * TQ_D * 4;
@@ -1184,13 +1181,28 @@ static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_page
   return p;
 }
 
+// Time of a plan, by which the form of a call is chosen.  A pair's page takes less (its CTAs dequantize half of it each), but
+// an odd last row block occupies a whole pair, and the plan rounds on 74 places instead of 148: three row blocks x 8 KV heads
+// x 256 pages of turbo3 are 144 CTAs of 43 pages alone and 64 of 64 as pairs, 99 us against 113; nine x 16 x 32 one wave alone
+// and three as pairs, 71 against 113; at 2, 5, 7 and 11 row blocks pairs are ahead (5 x 8 x 1,024: 495 against 540).  Page
+// times are what long chunks measure; a CTA costs 18 us beside its pages, a split its partial and its part of the merge.  PROD keys have no pairs: their
+// one score buffer puts scores, softmax and product of a page one after the other, 4 us a page in either form.
+static long pf_time_ns(const PfPlan& p, int k_format, int v_format, int cg) {
+  const int wide = (k_format == TQ_FMT_TURBO4) + (v_format == TQ_FMT_TURBO4);   // tables of 256 pairs
+  long page;
+  if (k_format == TQ_FMT_Q8_0) page = cg == 1 ? 2280 : v_format == TQ_FMT_Q8_0 ? 1940 : 1790;
+  else if (cg == 2) page = 1430 + 20 * wide;
+  else page = wide == 0 ? 1620 : wide == 1 ? 1830 : 2200;
+  return p.waves * (p.chunk_pages * page + 18000) + p.num_splits * (cg == 2 ? 700 : 1300);
+}
+
 extern "C" int64_t tq_prefill_workspace_bytes(int32_t batch, int32_t chunk_tokens, int32_t num_q_heads,
                                               int32_t num_kv_heads, int32_t max_pages_per_seq) {
   if (batch < 1 || chunk_tokens < 1 || num_q_heads < 1 || num_kv_heads < 1 || max_pages_per_seq < 1 ||
       num_q_heads % num_kv_heads)
     return TQ_ERR_INVALID;
-  const size_t a = pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq, false).total;
-  const size_t b = pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq, true).total;
+  const size_t a = pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq, 1).total;
+  const size_t b = pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq, 2).total;
   return (int64_t)(a > b ? a : b);   // enough for every pair of formats
 }
 
@@ -1242,7 +1254,12 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
   P.hq = num_q_heads;
   P.hkv = L->num_kv_heads;
   P.group = num_q_heads / L->num_kv_heads;
-  const PfPlan plan = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, pf_prod(L->k_format));
+  PfPlan plan = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, 1);
+  int cg = 1;
+  if (plan.row_blocks > 1 && !k_prod) {
+    const PfPlan pair = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, 2);
+    if (pf_time_ns(pair, L->k_format, L->v_format, 2) < pf_time_ns(plan, L->k_format, L->v_format, 1)) plan = pair, cg = 2;
+  }
   TQ_REQUIRE((int64_t)plan.total <= workspace_bytes, TQ_ERR_TOO_LARGE,
              "prefill workspace of %lld bytes is smaller than the %lld needed (tq_prefill_workspace_bytes)",
              (long long)workspace_bytes, (long long)plan.total);
@@ -1262,7 +1279,7 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
   const TqFast &fk = k_q8 ? none : kq->fast, &fv = v_q8 ? none : vq->fast;
   int rc = TQ_ERR_UNSUPPORTED;
 #define TQ_PF(K, V) \
-  if (L->k_format == K && L->v_format == V) rc = launch_prefill<K, V>(P, fk, fv, st);
+  if (L->k_format == K && L->v_format == V) rc = launch_prefill<K, V>(P, cg, fk, fv, st);
   TQ_PF(2, 2) TQ_PF(3, 3) TQ_PF(4, 4) TQ_PF(3, 2) TQ_PF(4, 2) TQ_PF(4, 3)
   TQ_PF(8, 2) TQ_PF(8, 3) TQ_PF(8, 4) TQ_PF(8, 8)
   TQ_PF(18, 2) TQ_PF(18, 3) TQ_PF(19, 2) TQ_PF(19, 3) TQ_PF(19, 4) TQ_PF(20, 3) TQ_PF(20, 4)
