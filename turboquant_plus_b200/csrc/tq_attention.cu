@@ -61,9 +61,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) k_decode_attn(const AttnParams
   split_index(P, split, kvh, b);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int PT = P.L.page_tokens;
-  // a length beyond the block-table row (or a negative one) is clamped: page numbers are only ever read from the
-  // row's max_pages entries, and the split count stays inside the plan the workspace was sized for
-  const int seq_len = min(max(P.seq_lens[b], 0), P.max_pages * PT);
+  int seq;
+  const int seq_len = row_length(P, b, PT, seq);
   const int n_pages = (seq_len + PT - 1) / PT;
   const int chunk = split_chunk(P, PT, lane), page_lo = split * chunk;
   const size_t row0 = (size_t)b * P.hq + (size_t)kvh * P.group;  // first query / output row of this CTA
@@ -87,7 +86,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) k_decode_attn(const AttnParams
   const uint32_t rec = (uint32_t)P.L.record_bytes;
   const int NS = P.stages;
 
-  const int32_t* bt = P.block_table + (size_t)b * P.max_pages;
+  const int32_t* bt = P.block_table + (size_t)seq * P.max_pages;
   auto issue = [&](int i) {
     const int64_t page = bt[page_lo + i];
     const uint8_t* src = P.pool + page * P.L.page_stride + (int64_t)kvh * P.L.head_stride;
@@ -669,7 +668,7 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
                        const uint8_t* pool_dev, const int32_t* block_table_dev, int32_t max_pages_per_seq,
                        const int32_t* seq_lens_dev, const void* q_dev, int32_t q_dtype, int32_t batch,
                        int32_t num_q_heads, float scale, void* workspace_dev, int64_t workspace_bytes, void* out_dev,
-                       int32_t out_dtype, int32_t phases, float* lse_dev, void* stream, bool coarse = false) {
+                       int32_t out_dtype, int32_t phases, float* lse_dev, void* stream, bool coarse = false, int32_t queries = 1) {
   TQ_REQUIRE(L, TQ_ERR_INVALID, "tq_decode_attn: layout missing");
   TQ_REQUIRE(batch >= 0 && num_q_heads >= 1 && max_pages_per_seq >= 1, TQ_ERR_INVALID, "bad sizes");
   if (batch == 0) return TQ_OK;
@@ -701,7 +700,8 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
   }
   if (!v_q8) TQ_REQUIRE(vq->d == TQ_D && vq->bits == L->v_format, TQ_ERR_INVALID,
                         "V quantizer bit width does not match the cache format");
-  const SplitPlan plan = (coarse ? plan_splits_coarse : plan_splits)(batch, L->num_kv_heads, max_pages_per_seq);
+  SplitPlan plan = (coarse ? plan_splits_coarse : plan_splits)(batch, L->num_kv_heads, max_pages_per_seq);
+  if (queries > 1) plan.spread[0] = plan.spread[1] = {};   // (the rows of a chunk are alike)
   const WsLayout w = ws_layout(batch, num_q_heads, plan.most());
   TQ_REQUIRE((int64_t)w.total <= workspace_bytes, TQ_ERR_TOO_LARGE, "workspace of %lld bytes is smaller than the %lld needed",
              (long long)workspace_bytes, (long long)w.total);
@@ -751,6 +751,7 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
   P.v_ident = v_q8 ? 1 : 0;
   P.max_pages = max_pages_per_seq;
   P.batch = batch;
+  P.queries = queries;
   P.hq = num_q_heads;
   P.hkv = L->num_kv_heads;
   P.group = group;
@@ -785,6 +786,14 @@ static int decode_impl(const tq_quantizer* kq, const tq_quantizer* vq, const tq_
   TQ_ATT(18, 2) TQ_ATT(18, 3) TQ_ATT(19, 2) TQ_ATT(19, 3) TQ_ATT(19, 4) TQ_ATT(20, 3) TQ_ATT(20, 4)
 #undef TQ_ATT
   return rc;
+}
+
+int tq_decode_chunk(const tq_quantizer* kq, const tq_quantizer* vq, const tq_cache_layout* L, const uint8_t* pool_dev,
+                    const int32_t* block_table_dev, int32_t max_pages_per_seq, const int32_t* kv_lens_dev, const void* q_dev,
+                    int32_t q_dtype, int32_t batch, int32_t queries, int32_t num_q_heads, float scale, void* workspace_dev,
+                    int64_t workspace_bytes, void* out_dev, int32_t out_dtype, void* stream) {
+  return decode_impl(kq, vq, L, pool_dev, block_table_dev, max_pages_per_seq, kv_lens_dev, q_dev, q_dtype, batch * queries,
+                     num_q_heads, scale, workspace_dev, workspace_bytes, out_dev, out_dtype, 3, nullptr, stream, false, queries);
 }
 
 extern "C" int tq_decode_attn_phases(const tq_quantizer* kq, const tq_quantizer* vq, const tq_cache_layout* L,

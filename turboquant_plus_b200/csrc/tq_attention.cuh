@@ -132,6 +132,8 @@ struct AttnParams {
   int32_t tail_late;   // the preceding kernel may write the last cached position of a sequence: its page is fetched
                        // after the dependency wait, every other page before (TQ_DECODE_OVERLAP_APPEND)
   int32_t chain_head;  // attention calls with TQ_DECODE_OVERLAP_Q follow this one (TQ_DECODE_CHAIN_HEAD)
+  int32_t queries;     // rows of the batch per sequence of the block table and of seq_lens: 1, or the queries of a chunk, of
+                       // which row i sees all cached positions but the last queries - 1 - i
   int32_t chunk_spread, spread_below;  // second chunk of SplitPlan, and the cached pages of the batch below which it is
                                        // taken; 0: none.  The grid then has the splits as its slowest dimension.
   tq_cache_layout L;
@@ -387,6 +389,20 @@ inline AttnParams with_splits(const AttnParams& P, const SplitPlan& plan, bool f
 }
 inline dim3 split_grid(const AttnParams& P) {
   return P.chunk_spread ? dim3(P.hkv, P.batch, P.num_splits) : dim3(P.num_splits, P.hkv, P.batch);
+}
+// the sequence that row b of the batch belongs to, and the cached positions that the row sees.  A length beyond the
+// block-table row (or a negative one) is clamped: page numbers are only ever read from the row's max_pages entries and the
+// split count stays inside the plan the workspace was sized for.
+__device__ __forceinline__ int row_length(const AttnParams& P, int b, int page_tokens, int& seq) {
+  seq = b;
+  int len;
+  if (P.queries == 1) {
+    len = P.seq_lens[b];
+  } else {
+    seq = b / P.queries;
+    len = P.seq_lens[seq] - (P.queries - 1 - (b - seq * P.queries));
+  }
+  return min(max(len, 0), P.max_pages * page_tokens);
 }
 // this CTA's split, KV head and sequence
 __device__ __forceinline__ void split_index(const AttnParams& P, int& split, int& kvh, int& b) {

@@ -599,7 +599,9 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
   }
   const int chunk = split_chunk(P, G4_PT, lane), page_lo = split * chunk;
   const size_t row0 = (size_t)b * P.hq + (size_t)kvh * P.group;
-  const int32_t* bt = P.block_table + (size_t)b * P.max_pages;
+  int seq;
+  const int seq_len = row_length(P, b, G4_PT, seq);
+  const int32_t* bt = P.block_table + (size_t)seq * P.max_pages;
   uint8_t* smg = sm + C::OFF_GROUPS;
   float* qbuf = reinterpret_cast<float*>(smg + C::G_Q);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smg + C::G_BAR);
@@ -617,9 +619,6 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
   // The warps take different roles so that their global-load latencies (and their instruction fetches, which are
   // cold in every launch) overlap: the producer sends the first pages on their way as early as it can, the first
   // `group` warps rotate one query head each, the others fill the pair tables.
-  // A length beyond the block-table row (or a negative one) is clamped: page numbers are only ever read from the
-  // row's max_pages entries and the split count stays inside the plan the workspace was sized for.
-  const int seq_len = min(max(P.seq_lens[b], 0), P.max_pages * G4_PT);
   const int n_pages = (seq_len + G4_PT - 1) / G4_PT;
   const int np = min(n_pages, page_lo + chunk) - page_lo;   // pages of this CTA (<= 0: none)
   int pg_ahead = 0;  // producer: block-table entry of the page issued in the next iteration

@@ -292,6 +292,12 @@ struct TqDenseDequant {
 bool tq_dense_quantize_try(const TqDenseQuant& a, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st, int* rc);
 bool tq_dense_dequantize_try(const TqDenseDequant& a, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
 
+// A chunk of queries per sequence as rows of the decode kernel, each with its causal length.  The workspace is one of
+// tq_decode_workspace_bytes(batch * queries, ...).
+int tq_decode_chunk(const tq_quantizer* kq, const tq_quantizer* vq, const tq_cache_layout* L, const uint8_t* pool_dev,
+                    const int32_t* block_table_dev, int32_t max_pages_per_seq, const int32_t* kv_lens_dev, const void* q_dev,
+                    int32_t q_dtype, int32_t batch, int32_t queries, int32_t num_q_heads, float scale, void* workspace_dev,
+                    int64_t workspace_bytes, void* out_dev, int32_t out_dtype, void* stream);
 int tq_quantize_wht_launch(const TqFast& f, const void* x, int32_t dtype, int64_t ld, int64_t n,
                            const TqQuantDst& dst, bool want_qjl, cudaStream_t st);
 bool tq_quantize_mma_try(const TqFast& f, const void* x, int32_t dtype, int64_t ld, int64_t n, const TqQuantDst& dst,

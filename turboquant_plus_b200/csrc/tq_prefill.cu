@@ -1196,6 +1196,25 @@ static long pf_time_ns(const PfPlan& p, int k_format, int v_format, int cg) {
   return p.waves * (p.chunk_pages * page + 18000) + p.num_splits * (cg == 2 ? 700 : 1300);
 }
 
+// A short chunk over q8_0 or PROD tensors: every query as a row of the decode kernel, which reads a page per row and KV head
+// where the kernel here multiplies 128 rows whatever the chunk has, converts every key to two or three operand tiles, and
+// splits no finer than eight pages.  Rows x KV heads x pages, and 12 ns a row and KV head, bound the one; pages of a wave, the
+// splits' merge and a start the other (q8_0 / turbo2, 32/8 heads, rows | tiles: 1 query over 256 pages 17 | 77 us, 4 47 | 78,
+// 8 over 32 pages 18 | 35, over 256 some 90 | 78; 48 over 2 pages 12 | 16; prod3 / turbo3, 4 over 256 53 | 109).  (turbo2/3/4
+// K and V always take the kernel here.)
+static const int64_t PF_MOST_ROW_PAGES = 49152;   // above: tiles, for any pair of formats
+static int64_t pf_row_pages(int32_t batch, int32_t chunk_tokens, int32_t hq, int32_t hkv, int32_t max_pages) {
+  const int64_t rows = (int64_t)batch * chunk_tokens;
+  if (hq / hkv > 8 || rows > 65535 || rows * hkv > 65536) return PF_MOST_ROW_PAGES + 1;   // the decode kernel's limits
+  return rows * hkv * max_pages;
+}
+static bool pf_takes_rows(const PfPlan& single, int64_t row_pages, int64_t row_heads, bool prod, int group) {
+  if (row_pages > PF_MOST_ROW_PAGES) return false;
+  const int64_t rows_ns = 8000 + row_pages * (prod ? (group > 4 ? 9500 : 7000) : (group > 4 ? 8000 : 6500)) / 1000 + 12 * row_heads;
+  const int64_t tiles_ns = single.waves * (single.chunk_pages * (prod ? 4100L : 2200L) + (prod ? 19000 : 8000)) + 1900L * single.num_splits;
+  return rows_ns < tiles_ns;
+}
+
 extern "C" int64_t tq_prefill_workspace_bytes(int32_t batch, int32_t chunk_tokens, int32_t num_q_heads,
                                               int32_t num_kv_heads, int32_t max_pages_per_seq) {
   if (batch < 1 || chunk_tokens < 1 || num_q_heads < 1 || num_kv_heads < 1 || max_pages_per_seq < 1 ||
@@ -1203,7 +1222,12 @@ extern "C" int64_t tq_prefill_workspace_bytes(int32_t batch, int32_t chunk_token
     return TQ_ERR_INVALID;
   const size_t a = pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq, 1).total;
   const size_t b = pf_plan(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq, 2).total;
-  return (int64_t)(a > b ? a : b);   // enough for every pair of formats
+  int64_t most = (int64_t)(a > b ? a : b);   // enough for every pair of formats
+  if (pf_row_pages(batch, chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq) <= PF_MOST_ROW_PAGES) {
+    const int64_t c = tq_decode_workspace_bytes(batch * chunk_tokens, num_q_heads, num_kv_heads, max_pages_per_seq);
+    if (c > most) most = c;
+  }
+  return most;
 }
 
 extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, const tq_cache_layout* L,
@@ -1255,6 +1279,12 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
   P.hkv = L->num_kv_heads;
   P.group = num_q_heads / L->num_kv_heads;
   PfPlan plan = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, 1);
+  if ((k_q8 || k_prod || v_q8) &&
+      pf_takes_rows(plan, pf_row_pages(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq),
+                    (int64_t)batch * chunk_tokens * L->num_kv_heads, k_prod, P.group) &&
+      tq_decode_workspace_bytes(batch * chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq) <= workspace_bytes)
+    return tq_decode_chunk(kq, vq, L, pool_dev, block_table_dev, max_pages_per_seq, kv_lens_dev, q_dev, q_dtype, batch, chunk_tokens,
+                           num_q_heads, scale, workspace_dev, workspace_bytes, out_dev, out_dtype, stream);
   int cg = 1;
   if (plan.row_blocks > 1 && !k_prod) {
     const PfPlan pair = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, 2);

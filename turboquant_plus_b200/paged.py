@@ -188,8 +188,9 @@ class PagedKVCache:
     def prefill_attend(self, q, block_table, kv_lens, scale=None, out=None, workspace=None):
         """Chunked prefill on the tcgen05 tensor cores.  q: (batch, chunk_tokens, num_q_heads, head_dim) CUDA
         tensor of a chunk whose K/V rows are already in the cache; kv_lens: (batch,) cached tokens including
-        the chunk.  Query i of a sequence sees cached positions 0 .. kv_len - chunk_tokens + i.  Every pair of
-        formats on 128-token pages takes the tcgen05 kernel."""
+        the chunk.  Query i of a sequence sees cached positions 0 .. kv_len - chunk_tokens + i.  Pairs of formats: those
+        of attend() but turbo2 K with turbo3 or turbo4 V and turbo3 K with turbo4 V.  (A short chunk over q8_0 or PROD
+        tensors runs as rows of the decode kernel, one per query.)"""
         bsz, tq, hq, d = q.shape
         assert d == self.head_dim
         turbo = self.k_format.startswith("turbo") and self.v_format.startswith("turbo")
