@@ -206,6 +206,7 @@ struct TqQuantDst {
   // this one reads or writes and everything before it has completed.  This kernel then runs beside it and waits for it
   // only at its end, so that its own completion stands for both.
   int32_t beside;
+  int32_t late;         // two-tensor launch: the kernel behind comes up as the tiles run out (qm_body)
 };
 
 // address of vector v's record field (elem_bytes per token and head) in plain arrays or in a paged cache;

@@ -182,7 +182,7 @@ __device__ __forceinline__ void qm_body(const TqFast& f, const Tin* __restrict__
   // after the other, 8 heads: 8,192 tokens of turbo3 18.6 -> 17.4 us, 2,048 of turbo4 9.5 -> 8.1; with 1,024 tokens of
   // turbo4, 256 CTAs, the early form is ahead, 6.1 against 6.6 us, and the attention call behind a decode step's append streams
   // pages meanwhile.)
-  const bool early = !PAIR || gridDim.x * gridDim.y <= 296;
+  const bool early = !PAIR || !dst.late;
   if (!dst.beside) {
     TQ_PDL_WAIT();
     if (early) TQ_PDL_TRIGGER();
@@ -710,11 +710,12 @@ int launch_mma(const TqFast& f, const Tin* x, int64_t ld, int64_t n, const TqQua
 }
 
 template <typename Tin, int BITS>
-int launch_mma_pair(const QmJob& j0, const QmJob& j1, int64_t ld, int64_t n, bool normc, cudaStream_t st) {
+int launch_mma_pair(QmJob& j0, QmJob& j1, int64_t ld, int64_t n, bool normc, cudaStream_t st) {
   const int64_t tiles = (n + QM_ROWS - 1) / QM_ROWS;
   const int64_t ctas = (tiles + QM_WARPS - 1) / QM_WARPS;
   const int64_t cap = (int64_t)tq_num_sms() * qm_ctas_per_sm<Tin>() / 2;  // two jobs share the SMs
   dim3 grid((unsigned)(ctas < cap ? ctas : cap), 2);
+  j0.dst.late = j1.dst.late = grid.x > (unsigned)tq_num_sms() ? 1 : 0;   // more than two CTAs per SM
   size_t smem = 0;
   if (normc) {
     const int rc = qm_dyn_smem<Tin, k_quantize_mma_pair<Tin, BITS, true>>(&smem);
