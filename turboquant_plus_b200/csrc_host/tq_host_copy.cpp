@@ -17,6 +17,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
+#include <sched.h>
 #include <string.h>
 
 #include <algorithm>
@@ -184,8 +185,16 @@ void on_threads(int64_t pieces, int threads, const c10::cuda::CUDAStream& stream
   if (crew->failed) std::rethrow_exception(crew->failed);
 }
 
+// cores that this process may run on (hardware_concurrency counts those of the machine)
+int64_t usable_cores() {
+  cpu_set_t set;
+  CPU_ZERO(&set);
+  if (sched_getaffinity(0, sizeof(set), &set) == 0) return CPU_COUNT(&set);
+  return std::thread::hardware_concurrency();
+}
+
 int thread_count(const Pieces& p, size_t width) {
-  const int64_t cores = std::thread::hardware_concurrency(), mega = p.count * (int64_t)width >> 20;
+  const int64_t cores = usable_cores(), mega = p.count * (int64_t)width >> 20;
   return (int)std::max<int64_t>(1, std::min({(int64_t)MOST_THREADS, p.n, cores / 2, 1 + mega}));
 }
 
