@@ -365,8 +365,9 @@ int tq_attn_merge(const void* out_a_dev, const float* lse_a_dev, const void* out
  * sees the cached tokens 0 .. that position.  Per (sequence, query, head) this is again the
  * reference tests' dequantize-then-attend (tests/test_kv_cache.py:73-89) restricted to the visible
  * prefix; the reference has no chunked or masked variant of its own.
- *   q_dev, out_dev [batch][chunk_tokens][num_q_heads][d]; turbo2/3/4, q8_0 and PROD K, turbo2/3/4 and q8_0 V (the pairs of
- *   tq_decode_attn); 128-token pages; the quantizer of a q8_0 tensor is ignored and may be NULL.
+ *   q_dev, out_dev [batch][chunk_tokens][num_q_heads][d]; the pairs of formats of tq_decode_attn but turbo2 K with turbo3 or
+ *   turbo4 V and turbo3 K with turbo4 V; 128-token pages; the quantizer of a q8_0 tensor is ignored and may be NULL.
+ *   Short chunks over q8_0 or PROD tensors run as rows of the decode kernel, one per query with its causal length.
  *   The page range of a row block is split over several CTAs when the grid would otherwise not fill
  *   the GPU; the last split to finish folds the partials (ticket, as in tq_decode_attn).
  *   workspace_dev: tq_prefill_workspace_bytes(...) bytes, 256-byte aligned, initialised once with

@@ -56,3 +56,31 @@ def fill_cache(cache, k, v, seq_lens, rng, page_tokens=128):
         cache.append(torch.as_tensor(k[b]).to(cache.device), torch.as_tensor(v[b]).to(cache.device),
                      torch.as_tensor(slots))
     return torch.as_tensor(bt)
+
+
+def stored_rows(cache, which, pages, n):
+    """(n, heads, D) fp64 rows that a cache holds for a sequence, decoded from its records in plain NumPy: what attention has
+    to see, whichever neighbouring index a coordinate on a decision boundary took when it was quantized."""
+    lay, pt = cache.layout, cache.page_tokens
+    fmt = cache.k_format if which == "k" else cache.v_format
+    pool = cache.pool[np.asarray(pages, dtype=np.int64)].cpu().numpy()           # (pages, heads, record)
+
+    def field(off, per_token, dtype):
+        a = np.ascontiguousarray(pool[:, :, off:off + pt * per_token]).view(dtype)
+        return a.reshape(pool.shape[0], pool.shape[1], pt, -1).transpose(0, 2, 1, 3).reshape(-1, pool.shape[1], a.shape[2] // pt)[:n]
+
+    idx = field(getattr(lay, which + "_idx_off"), getattr(lay, which + "_idx_bytes"), np.uint8)
+    if fmt == "q8_0":
+        scale = field(getattr(lay, which + "_scale_off"), 8, np.float16).astype(np.float64)
+        return idx.view(np.int8).astype(np.float64) * np.repeat(scale, 32, axis=2)
+    quant = cache.k_quantizer if which == "k" else cache.v_quantizer
+    prod = fmt.startswith("prod")
+    pq = quant.polar_quant if prod else quant
+    bits = np.unpackbits(idx, axis=2).reshape(*idx.shape[:2], D, pq.bit_width)
+    codes = (bits * (1 << np.arange(pq.bit_width - 1, -1, -1))).sum(axis=3)
+    scale = field(getattr(lay, which + "_scale_off"), 4, np.float32).astype(np.float64)
+    rows = (pq.centroids[codes] @ pq.rotation) * scale
+    if prod:
+        signs = 2.0 * np.unpackbits(field(lay.k_qjl_off, D // 8, np.uint8), axis=2) - 1.0
+        rows = rows + (signs @ quant.qjl.S) * field(lay.k_rscale_off, 4, np.float32).astype(np.float64)
+    return rows

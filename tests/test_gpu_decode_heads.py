@@ -1,16 +1,14 @@
 """Decode attention for every group size of the two specialised forms (1..4 and 5..8 query heads per KV head) and every
 format pair, in stream order, in a chain and after an append, against dequantize-then-attend.
 
-Tolerance: 2e-3 max-relative, that of the attention tests, for the arithmetic of the kernels.  The oracle quantizes the
-inputs itself: a coordinate within rounding of a decision boundary may take the neighbouring index there (1 in some 10^5).
-In a value that moves one rotated coordinate by a level step, at most 0.81 ||v|| / sqrt(d) = 0.81 (3 bits, outermost;
-||v|| ~ sqrt(d)), i.e. every output coordinate by 0.81 / sqrt(d) = 0.072 times the token's weight, against a row maximum of
-about 2.5: up to 3e-2 where one of few tokens has all the weight.  One sequence per case may show that."""
+Tolerance: 2e-3 max-relative, that of the attention tests, against the rows that the cache holds (an oracle that quantizes
+the inputs itself takes a neighbouring index at one coordinate in some 10^5, up to 3e-2 of an output row)."""
 import numpy as np
 import pytest
 
-from tests.helpers import D, fill_cache, max_rel
-from tests.test_gpu_attention import TOL, oracle_attention
+from oracle import tq_oracle as o
+from tests.helpers import D, fill_cache, max_rel, stored_rows
+from tests.test_gpu_attention import TOL
 
 pytestmark = pytest.mark.gpu
 
@@ -33,10 +31,14 @@ def test_decode_heads(kf, vf, group):
     sl = torch.tensor(lens, dtype=torch.int32, device="cuda")
     q = rng.standard_normal((len(lens), hkv * group, D)).astype(np.float32)
     qt = torch.as_tensor(q).cuda()
-    want = oracle_attention(cache, ks, vs, q, lens)
+    want = []
+    for b, n in enumerate(lens):
+        pages = bt[b, :-(-n // 128)].cpu().numpy()
+        kh, vh = (stored_rows(cache, w, pages, n).transpose(1, 0, 2)[None] for w in "kv")
+        want.append(o.attend_gqa(q[b:b + 1].astype(np.float64), kh, vh, [n])[0])
     for mode in (False, True, "q", "append"):
         out, lse = cache.attend(qt, bt, sl, overlap=mode, return_lse=True)
         again = cache.attend(qt, bt, sl, overlap=mode)
         assert cache.kernel_status() == 0 and torch.equal(out, again) and torch.isfinite(lse).all()
-        err = sorted(max_rel(out[b].cpu().numpy().reshape(-1, D), want[b].reshape(-1, D)) for b in range(len(lens)))
-        assert err[-2] < TOL and err[-1] < 3e-2, f"{kf}/{vf} {group} heads, overlap={mode}: {err}"
+        err = max(max_rel(out[b].cpu().numpy().reshape(-1, D), want[b].reshape(-1, D)) for b in range(len(lens)))
+        assert err < TOL, f"{kf}/{vf} {group} heads, overlap={mode}: {err}"

@@ -1,14 +1,13 @@
 """Chunked prefill by pairs of CTAs: one, two, three and many row blocks (an odd last one), chunks whose two blocks of a pair
 see different numbers of pages, several splits, fp32 / fp16 / bf16 rows, against dequantize-then-attend.
 
-Tolerance: that of the attention tests; one sequence per case may show the oracle's own quantization taking a neighbouring
-index (3e-2, derived in test_gpu_decode_heads)."""
+Tolerance: that of the attention tests, against the rows that the cache holds."""
 import numpy as np
 import pytest
 
 from oracle import tq_oracle as o
-from tests.helpers import D, fill_cache, max_rel
-from tests.test_gpu_attention import TOL, oracle_roundtrip
+from tests.helpers import D, fill_cache, max_rel, stored_rows
+from tests.test_gpu_attention import TOL
 
 pytestmark = pytest.mark.gpu
 
@@ -33,8 +32,8 @@ def test_prefill_pairs(kf, vf, group, chunk, lens):
         assert torch.equal(cache.prefill_attend(qt.to(dt), bt, lt), cache.prefill_attend(qt.to(dt).float(), bt, lt).to(dt))
     errs = []
     for b, n in enumerate(lens):
-        kh = np.stack([oracle_roundtrip(cache, ks[b][:, h], "k") for h in range(hkv)])[None]
-        vh = np.stack([oracle_roundtrip(cache, vs[b][:, h], "v") for h in range(hkv)])[None]
+        pages = bt[b, :-(-n // 128)].numpy()
+        kh, vh = (stored_rows(cache, w, pages, n).transpose(1, 0, 2)[None] for w in "kv")
         lo = max(0, chunk - n)
         some = np.unique(np.concatenate([[lo, chunk - 1], rng.integers(lo, chunk, 24)]))     # the oracle is slow
         got = out[b].cpu().numpy()
@@ -42,6 +41,5 @@ def test_prefill_pairs(kf, vf, group, chunk, lens):
         for i in some:
             m = n - chunk + i + 1
             ref = o.attend_gqa(q[b, i][None].astype(np.float64), kh[:, :, :m], vh[:, :, :m], [m])[0]
-            errs.append((max_rel(got[i], ref), b))
-    worst = sorted((max(e for e, bb in errs if bb == b)) for b in range(len(lens)))
-    assert worst[0] < TOL and worst[-1] < 3e-2, f"{kf}/{vf}: {worst}"
+            errs.append(max_rel(got[i], ref))
+    assert max(errs) < TOL, f"{kf}/{vf}: {max(errs)}"
