@@ -8,42 +8,11 @@
 // products.  The kernel, its roles, its tensor-memory map and its hand-offs are described above k_prefill_attn2.
 // Every wait is bounded in time; a CTA that gives up sets the status word and still frees its tensor memory.
 #include <type_traits>
-#include "tq_internal.cuh"
+#include "tq_tcgen05.cuh"
 
 namespace {
 
 constexpr int PF_ROWS = 128, PF_PAGE = 128;   // rows of a CTA, tokens of a page
-constexpr long long PF_WAIT_CYCLES = 1LL << 30;
-
-__device__ __forceinline__ uint32_t sptr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ bool pf_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  // the hint lets the hardware keep the thread suspended for up to that many nanoseconds before the instruction returns
-  // false: a waiting role then spends few issue slots on polling
-  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
-               : "=r"(ok) : "r"(sptr(bar)), "r"(parity), "r"(20000u) : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool pf_wait(uint64_t* bar, uint32_t parity) {
-  if (pf_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (clock64() - t0 < PF_WAIT_CYCLES)
-    if (pf_try_wait(bar, parity)) return true;
-  return false;
-}
-
-// shared-memory matrix descriptor, no swizzle: start address, leading-dimension and stride byte offsets (16-byte
-// units), descriptor version 1.  K-major operand: LBO = distance between 8-element K chunks, SBO = distance
-// between 8-row groups.  MN-major operand: LBO = distance between 8-row K groups, SBO = between 8-element N chunks.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)((lbo >> 4) & 0x3fff) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3fff) << 32) | ((uint64_t)1 << 46);
-}
-// instruction descriptor, kind::f16: fp32 accumulator, fp16 A and B, A K-major, B major as given, N, M
-__device__ __forceinline__ uint32_t umma_idesc(int m, int n, bool b_mn_major) {
-  return (1u << 4) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
 // CG CTAs on one tile: with two, the accumulator's rows 0-127 are the even CTA's tensor memory and 128-255 the odd one's,
 // A likewise, and each CTA's shared memory holds its half of B's columns (N) at the same offsets.
 // A pair's are executed by a whole warp of the even CTA, one elected thread of which issues them: the warp stays converged, so
@@ -90,32 +59,6 @@ template <int CG> __device__ __forceinline__ void pf_sync_all() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   }
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(addr) : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// sixteen columns into v[OFF .. OFF + 15], no wait: the caller waits once for all of its loads
-template <int OFF, int N>
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t addr, uint32_t (&v)[N]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[OFF]), "=r"(v[OFF + 1]), "=r"(v[OFF + 2]), "=r"(v[OFF + 3]), "=r"(v[OFF + 4]), "=r"(v[OFF + 5]),
-        "=r"(v[OFF + 6]), "=r"(v[OFF + 7]), "=r"(v[OFF + 8]), "=r"(v[OFF + 9]), "=r"(v[OFF + 10]), "=r"(v[OFF + 11]),
-        "=r"(v[OFF + 12]), "=r"(v[OFF + 13]), "=r"(v[OFF + 14]), "=r"(v[OFF + 15])
-      : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
 __device__ __forceinline__ float pf_exp2(float x) {
   float y;
@@ -446,14 +389,6 @@ __device__ __forceinline__ void pf_arrive_warp(uint64_t* bar, int lane) {
   __syncwarp();
   if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sptr(bar)) : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
-}
 // ... on the barrier of the CTA that issues the MMAs: the even one of a pair
 template <int CG> __device__ __forceinline__ void pf_arrive_leader(uint64_t* bar, int lane) {
   if constexpr (CG == 1) {
@@ -469,7 +404,7 @@ template <int CG> __device__ __forceinline__ void pf_arrive_leader(uint64_t* bar
 }
 // bounded wait whose verdict is the same in every lane of the warp (warp-collective tcgen05 instructions follow)
 __device__ __forceinline__ bool pf_wait_warp(uint64_t* bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, pf_wait(bar, parity));
+  return __all_sync(0xffffffffu, tc_wait(bar, parity));
 }
 template <int KK, int VK, int CG>
 __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_attn2(const __grid_constant__ PrefillParams P,
@@ -956,11 +891,11 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
         const int bf = i & 1, st_i = i % NST;
         bool ok = !*fail;
         if constexpr (SP::KBUF == 2) {
-          if (ok && i >= 2) ok = pf_wait(&s_full[bf], (uint32_t)(((i - 2) >> 1) & 1));
+          if (ok && i >= 2) ok = tc_wait(&s_full[bf], (uint32_t)(((i - 2) >> 1) & 1));
         } else {
-          if (ok && i >= 1) ok = pf_wait(&s_full[bf ^ 1], (uint32_t)(((i - 1) >> 1) & 1));
+          if (ok && i >= 1) ok = tc_wait(&s_full[bf ^ 1], (uint32_t)(((i - 1) >> 1) & 1));
         }
-        if (ok) ok = pf_wait(&rec_full[st_i], (uint32_t)((i / NST) & 1));
+        if (ok) ok = tc_wait(&rec_full[st_i], (uint32_t)((i / NST) & 1));
         if (!__all_sync(0xffffffffu, ok)) { *fail = 1; break; }   // a warp goes on or gives up as a whole
         const uint8_t* st = stage0 + st_i * SP::REC;
         uint8_t* dst = drow + (SP::KBUF == 2 ? bf * KT::TILES * TILE : 0);
@@ -1002,8 +937,8 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       for (int i = 0; i < np; ++i) {
         const int bf = i & 1, st_i = i % NST;
         bool ok = !*fail;
-        if (ok && i >= 2) ok = pf_wait(&o_done[bf], (uint32_t)(((i - 2) >> 1) & 1));
-        if (ok) ok = pf_wait(&rec_full[st_i], (uint32_t)((i / NST) & 1));
+        if (ok && i >= 2) ok = tc_wait(&o_done[bf], (uint32_t)(((i - 2) >> 1) & 1));
+        if (ok) ok = tc_wait(&rec_full[st_i], (uint32_t)((i / NST) & 1));
         if (!__all_sync(0xffffffffu, ok)) { *fail = 1; break; }
         const uint8_t* st = stage0 + st_i * SP::REC;
         // The token's V scale goes into its row of the operand tile (fp16 product, rounding 2^-11 per element), so
@@ -1034,10 +969,10 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
     // =========================== record copies ===========================
     int issued = min(np, NST);
     while (issued < np && !*fail) {   // the stage of page issued - NST, once all producer warps have read it
-      if (!pf_wait(&rec_free[issued % NST], (uint32_t)((issued / NST - 1) & 1))) { *fail = 1; break; }
+      if (!tc_wait(&rec_free[issued % NST], (uint32_t)((issued / NST - 1) & 1))) { *fail = 1; break; }
       issue(issued++);
     }
-    for (int i = max(0, issued - NST); i < issued; ++i) pf_wait(&rec_full[i % NST], (uint32_t)((i / NST) & 1));   // none in flight at the end
+    for (int i = max(0, issued - NST); i < issued; ++i) tc_wait(&rec_full[i % NST], (uint32_t)((i / NST) & 1));   // none in flight at the end
   } else if (warp == SP::MMA_AT / 32 && crank == 0 && np > 0) {
     // =========================== MMA warp ===========================
     // (all 512 columns are this CTA's: its tensor memory starts at address 0)

@@ -26,7 +26,7 @@
 //     register layout (element 16 i + 4 t + c of lane t: the bits of i and c are butterflies in registers, the two
 //     bits of t two lane exchanges), with the sign flips in between from a lane-indexed table in shared memory.
 // Everything else (1-bit PolarQuant stages, asymmetric codebooks, unpacked output) stays with k_quantize_wht.
-#include "tq_internal.cuh"
+#include "tq_quantize_math.cuh"
 
 namespace {
 
@@ -74,43 +74,6 @@ __device__ __forceinline__ void qm_split3(float x0, float x1, uint32_t& hi, uint
   const float s0 = r0 - __uint_as_float(v0 & 0xffff0000u), s1 = r1 - __uint_as_float(v1 & 0xffff0000u);
   lo = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);
 }
-
-__device__ __forceinline__ uint32_t qm_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint32_t qm_bit(const uint32_t (&m)[4], int e) { return (m[e >> 5] >> (e & 31)) & 1u; }
-// 1.0f when a > b, else 0.0f, in one instruction
-__device__ __forceinline__ float qm_gt(float a, float b) {
-  float d;
-  asm("set.gt.f32.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
-  return d;
-}
-
-// packed fp32 arithmetic (two operations per instruction); operands are register pairs as the MMA leaves them
-__device__ __forceinline__ float2 qm_add2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n add.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}\n"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 qm_sub2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n sub.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}\n"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 qm_mul2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n mul.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}\n"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 qm_fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n .reg .b64 ra, rb, rc, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n mov.b64 rc, {%6, %7};\n"
-      " fma.rn.f32x2 rd, ra, rb, rc;\n mov.b64 {%0, %1}, rd;\n}\n"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-__device__ __forceinline__ float2 qm_dup(float v) { return make_float2(v, v); }
 
 // `tile`: the CTA's staging memory, QM_WARPS x 2 buffers of QM_ROWS rows of qm_rowb<Tin>() bytes, then 4 KB for the
 // B operands of the MMAs
@@ -751,6 +714,7 @@ bool tq_quantize_mma_try_pair(const TqFast& f0, const void* x0, const TqQuantDst
   j0.f = f0; j0.x = x0; j0.dst = d0;
   j1.f = f1; j1.x = x1; j1.dst = d1;
   const bool normc = f0.norm_correction && d0.scale;
+  if (tq_quantize_tc_try(f0, x0, d0, &f1, x1, &d1, dtype, ld, n, normc, false, st, rc)) return true;
 #define TQ_CASE(B)                                                                              \
   case B:                                                                                       \
     *rc = dtype == TQ_F16    ? launch_mma_pair<__half, B>(j0, j1, ld, n, normc, st)             \
@@ -770,6 +734,9 @@ bool tq_quantize_mma_try_pair(const TqFast& f0, const void* x0, const TqQuantDst
 bool tq_quantize_mma_try(const TqFast& f, const void* x, int32_t dtype, int64_t ld, int64_t n, const TqQuantDst& dst,
                          bool want_qjl, cudaStream_t st, int* rc) {
   if (!qm_serves(f, dtype, ld, dst, want_qjl)) return false;
+  // (the residual needs the norm correction whether or not the scale is stored)
+  if (tq_quantize_tc_try(f, x, dst, nullptr, nullptr, nullptr, dtype, ld, n, f.norm_correction && (dst.scale || want_qjl), want_qjl, st, rc))
+    return true;
 #define TQ_CASE(B)                                                                                           \
   case B:                                                                                                    \
     *rc = dtype == TQ_F16    ? launch_mma<__half, B>(f, (const __half*)x, ld, n, dst, want_qjl, st)               \
