@@ -1,0 +1,82 @@
+"""Dense-mode calls of many vectors (integer products of base-256 digits) against the same vectors in small calls (fp64 products):
+edges of the 128-vector tiles, both row types, all widths, rows that are zero, tiny, huge or not finite, matrices that are not
+rotations.  Both paths are within 7e-16 of exact sums, so indices and signs are equal except within 1e-14 of a boundary, which
+these inputs do not meet; reconstructions agree to 256 roundings of 2^-53 of the largest one of their row (sums of 256 terms)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+D = 128
+PIECE = 4096          # small calls
+
+
+def _pieces(fn, x):
+    import torch
+    parts = [fn(x[lo:lo + PIECE]) for lo in range(0, len(x), PIECE)]
+    return [torch.cat(p) for p in zip(*parts)]
+
+
+def _same(a, b):
+    import torch
+    return bool(((a == b) | (torch.isnan(a) & torch.isnan(b))).all()) if a.is_floating_point() else torch.equal(a, b)
+
+
+def _rows(n, dtype, special):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, D, device="cuda", generator=gen) * torch.exp(0.5 * torch.randn(n, 1, device="cuda", generator=gen))
+    x[:, 5] *= 10
+    x[n // 2] = 0
+    if special:
+        big, small = (1e30, 1e-30) if dtype == "float32" else (6e4, 1e-7)
+        x[3] = 0
+        x[3, 7] = small
+        x[4] = big
+        x[9] *= small
+        x[10, 3], x[11, 3], x[n - 1, 0] = float("nan"), float("inf"), float("-inf")
+        x[129, 100], x[130, 100] = float("inf"), float("-inf")
+    return x.to(getattr(torch, dtype))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+@pytest.mark.parametrize("n,bits,special", [(9473, 2, False), (9600, 3, True), (9601, 4, False), (18944, 3, False), (19073, 2, True), (40000, 4, True)])
+@pytest.mark.parametrize("matrix", ["rotation", "arbitrary"])
+def test_many_vectors_equal_few(n, bits, special, dtype, matrix):
+    import torch
+    import turboquant_plus_b200 as tq
+    x = _rows(n, dtype, special)
+    q = tq.TurboQuant(D, bits, seed=5)          # bits - 1 for the indices, one for the sketch
+    m = tq.TurboQuantMSE(D, bits, seed=6)
+    if matrix == "arbitrary":                   # residuals of many times the vector's length
+        rng = np.random.default_rng(n)
+        q.polar_quant.rotation = rng.standard_normal((D, D)) * np.exp(rng.standard_normal((D, D)))
+        m.polar_quant.rotation = np.diag(np.exp2(rng.integers(-20, 20, D).astype(float)))
+
+    def quantize(v):
+        c = q.quantize(v)
+        return c.mse_indices, c.vector_norms, c.qjl_signs, c.residual_norms
+
+    whole, parts = quantize(x), _pieces(quantize, x)
+    assert _same(whole[0], parts[0]) and _same(whole[1], parts[1])
+    finite = torch.isfinite(parts[3])
+    assert torch.equal(torch.isfinite(whole[3]), finite)
+    assert bool(((whole[3] - parts[3]).abs() <= 1.2e-7 * parts[3])[finite].all())          # fp32 results of sums that agree
+    if matrix == "rotation":                    # (arbitrary: projections of any size beside others, signs within rounding of zero)
+        assert torch.equal(whole[2], parts[2])
+    else:
+        assert float((whole[2] != parts[2]).float().mean()) < 1e-6
+    idx, norms = m.quantize(x)
+    few = _pieces(m.quantize, x)
+    assert _same(idx, few[0]) and _same(norms, few[1])
+
+    def close(a, b):
+        scale = b.abs().amax(dim=1, keepdim=True).nan_to_num(posinf=1.0)
+        ok = ((a - b).abs() <= 256 * 2.0 ** -53 * scale) | (a == b) | (~torch.isfinite(a) & ~torch.isfinite(b))
+        return bool(ok.all())
+
+    code = q.quantize(x)
+    back = q.dequantize(code)
+    parts = torch.cat([q.dequantize(type(code)(**{f: (getattr(code, f)[lo:lo + PIECE] if torch.is_tensor(getattr(code, f)) else getattr(code, f))
+                                                  for f in code.__dataclass_fields__})) for lo in range(0, n, PIECE)])
+    assert close(back, parts)
+    assert close(m.dequantize(idx, norms), torch.cat([m.dequantize(idx[lo:lo + PIECE], norms[lo:lo + PIECE]) for lo in range(0, n, PIECE)]))

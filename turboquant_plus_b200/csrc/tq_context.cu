@@ -84,6 +84,7 @@ struct DeviceImage {
 
 struct MatrixParts {
   size_t m, t, m32, t32, mp, tp;   // mp, tp: padded with zeros to dp x dp (m and t themselves when d is a multiple of 8)
+  double scale;                    // d = 128: what the digits of tq_dense_i8.cu are relative to (0: it has none)
 };
 static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
   std::vector<double> t((size_t)d * d);
@@ -94,7 +95,7 @@ static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
       a32[(size_t)i * d + j] = (float)m[(size_t)i * d + j];
       t32[(size_t)j * d + i] = (float)m[(size_t)i * d + j];
     }
-  MatrixParts p;
+  MatrixParts p{};
   p.m = im.add(m, t.size() * 8);
   p.t = im.add(t.data(), t.size() * 8);
   p.mp = p.m;
@@ -110,6 +111,7 @@ static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
     p.mp = im.add(mp.data(), mp.size() * 8);
     p.tp = im.add(tp.data(), tp.size() * 8);
   }
+  p.scale = d == TQ_D ? tq_dense_digits_scale(m) : 0.0;
   p.m32 = im.add(a32.data(), a32.size() * 4);
   p.t32 = im.add(t32.data(), t32.size() * 4);
   return p;
@@ -216,7 +218,9 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
   if (dense_rot) mr = add_matrix(im, desc->rot, q->d);
   if (dense_s) ms = add_matrix(im, desc->qjl_s, q->d);
   const size_t cent_at = im.add(c.data(), c.size() * 8), bnd_at = im.add(b.data(), b.size() * 8);
-  e = cudaMalloc((void**)&q->mem, im.bytes.size());
+  const size_t digits_at = (im.bytes.size() + 255) & ~(size_t)255;   // digits of R, R^T, S, S^T, made on the device
+  const size_t total = mr.scale != 0.0 || ms.scale != 0.0 ? digits_at + 4 * TQ_DENSE_DIGITS_BYTES : im.bytes.size();
+  e = cudaMalloc((void**)&q->mem, total);
   if (e == cudaSuccess) e = cudaMemcpy(q->mem, im.bytes.data(), im.bytes.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     tq_quantizer_destroy(q);
@@ -226,6 +230,26 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
   auto f32 = [&](size_t at) { return reinterpret_cast<float*>(q->mem + at); };
   if (dense_rot) q->rot = f64(mr.m), q->rot_t = f64(mr.t), q->rot32 = f32(mr.m32), q->rot32_t = f32(mr.t32), q->rotp = f64(mr.mp), q->rotp_t = f64(mr.tp);
   if (dense_s) q->s = f64(ms.m), q->s_t = f64(ms.t), q->s32 = f32(ms.m32), q->s32_t = f32(ms.t32), q->sp = f64(ms.mp), q->sp_t = f64(ms.tp);
+  uint8_t* digits = q->mem + digits_at;
+  auto add_digits = [&](const double* m, double scale) -> const uint8_t* {
+    uint8_t* at = digits;
+    digits += TQ_DENSE_DIGITS_BYTES;
+    if (e == cudaSuccess) e = tq_dense_digits(m, scale, at);
+    return at;
+  };
+  if (mr.scale != 0.0) q->dig.r = add_digits(q->rot, mr.scale), q->dig.rt = add_digits(q->rot_t, mr.scale), q->dig.r_scale = mr.scale;
+  if (ms.scale != 0.0) q->dig.s = add_digits(q->s, ms.scale), q->dig.st = add_digits(q->s_t, ms.scale), q->dig.s_scale = ms.scale;
+  if (e == cudaSuccess && total > im.bytes.size()) e = cudaStreamSynchronize(cudaStreamLegacy);   // other streams may use them at once
+  if (e != cudaSuccess) {
+    tq_quantizer_destroy(q);
+    return tq_cuda_fail(e, "digits of the dense matrices");
+  }
+  {
+    const double most = fabs(c.front()) > fabs(c.back()) ? fabs(c.front()) : fabs(c.back());   // (strictly increasing)
+    int exponent = 0;
+    if (most > 1e-100 && most < 1e100) frexp(most, &exponent), q->dig.cent_scale = ldexp(1.0, exponent);
+    for (size_t i = 0; i < b.size(); ++i) q->dig.bnd[i] = b[i];
+  }
   q->cent64 = f64(cent_at);
   q->bnd64 = f64(bnd_at);
   *out = q;

@@ -222,7 +222,7 @@ static bool dequantize_tensor(const tq_quantizer* q, const uint8_t* packed, cons
   t.d = q->d; t.dp = (q->d + 7) / 8 * 8; t.bits = q->bits; t.norm_correction = q->norm_correction;
   t.packed = packed; t.idx = idx; t.norm = norm; t.qjl = qjl; t.rnorm = rnorm;
   t.shrink = shrink; t.ld_out = ld_out; t.accumulate = accumulate;
-  return tq_dense_dequantize_try(t, n, out, dtype, st, rc);
+  return tq_dense_i8_dequantize_try(t, q->dig, n, out, dtype, st, rc) || tq_dense_dequantize_try(t, n, out, dtype, st, rc);
 }
 
 extern "C" int tq_dequantize(const tq_quantizer* q, const uint8_t* packed_dev, const uint8_t* idx_dev,

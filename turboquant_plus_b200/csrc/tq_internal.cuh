@@ -28,6 +28,17 @@ struct TqFast {
   int32_t has_qjl;
 };
 
+// The dense matrices of d = 128 as base-256 digits (tq_dense_i8.cu); a scale of 0: none
+struct TqDenseDigits {
+  const uint8_t *r, *rt, *s, *st;   // of R, R^T, S, S^T
+  double r_scale, s_scale;          // powers of two that the digits are relative to
+  double cent_scale;                // a power of two above every centroid's magnitude
+  double bnd[15];                   // boundaries
+};
+#define TQ_DENSE_DIGITS_BYTES (7 * TQ_D * TQ_D)
+double tq_dense_digits_scale(const double* m);
+cudaError_t tq_dense_digits(const double* m_dev, double scale, uint8_t* out_dev);   // on the legacy stream
+
 struct tq_quantizer {
   int32_t d, bits, rotation, norm_correction, qjl, device;
   TqFast fast;               // valid when rotation == TQ_ROT_WHT
@@ -42,6 +53,7 @@ struct tq_quantizer {
   float* s32;                // S row-major fp32
   float* s32_t;
   double host_cent[16];
+  TqDenseDigits dig;
 };
 
 void tq_set_error(const char* fmt, ...);
@@ -292,6 +304,10 @@ struct TqDenseDequant {
 };
 bool tq_dense_quantize_try(const TqDenseQuant& a, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st, int* rc);
 bool tq_dense_dequantize_try(const TqDenseDequant& a, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
+
+bool tq_dense_i8_quantize_try(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
+                              int* rc);
+bool tq_dense_i8_dequantize_try(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
 
 // A chunk of queries per sequence as rows of the decode kernel, each with its causal length.  The workspace is one of
 // tq_decode_workspace_bytes(batch * queries, ...).

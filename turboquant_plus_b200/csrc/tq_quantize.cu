@@ -538,6 +538,7 @@ static int launch_dense(const tq_quantizer* q, const void* x, int32_t dtype, int
     t.out_norm = a.out_norm; t.out_scale = a.out_scale; t.out_rnorm = a.out_rnorm;
     t.out_qjl = a.out_qjl; t.out_res = a.out_res; t.ld_res = a.ld_res;
     int rc = TQ_OK;
+    if (tq_dense_i8_quantize_try(t, q->dig, x, dtype, ld, n, st, &rc)) return rc;
     if (tq_dense_quantize_try(t, x, dtype, ld, n, st, &rc)) return rc;
   }
   const size_t smem = (size_t)q->d * TV * 8 * 2 + (size_t)q->d * TV + 16;
