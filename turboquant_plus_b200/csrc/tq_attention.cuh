@@ -190,6 +190,21 @@ __device__ __forceinline__ uint32_t field_off(const uint32_t (&w)[NW], int p) {
   return __funnelshift_r(w[k + 1 < NW ? k + 1 : k], w[k], sr) & MASK;
 }
 
+// fields p and p + 1 (p even).  Where p takes a right shift, p + 1 is the same value shifted left: left shifts go to the
+// multiply-add pipe, right shifts to the integer pipe, which the page loop loads most.  (The statement in between keeps the
+// compiler from making two right shifts of the two again.)
+template <int FB, int SH, int NW>
+__device__ __forceinline__ uint2 field_pair(const uint32_t (&w)[NW], int p) {
+  constexpr uint32_t MASK = ((1u << FB) - 1) << SH;
+  const int start = p * FB, k = start >> 5, o = start & 31, sr = 32 - FB - o;
+  if (FB <= SH && sr > SH && sr - FB > SH && o + 2 * FB <= 32) {
+    uint32_t v = w[k] >> (sr - SH);
+    asm("" : "+r"(v));
+    return make_uint2(v & MASK, (v << FB) & MASK);
+  }
+  return make_uint2(field_off<FB, SH, NW>(w, p), field_off<FB, SH, NW>(w, p + 1));
+}
+
 __device__ __forceinline__ float load_q(const void* q, int dtype, size_t i) {
   if (dtype == TQ_F16) return __half2float(reinterpret_cast<const __half*>(q)[i]);
   if (dtype == TQ_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(q)[i]);

@@ -305,10 +305,11 @@ __device__ __forceinline__ void g4_scores(float (&s)[4], uint32_t st, const G4Th
       if constexpr (NODEQ) {
         a0 = w0[j % KB]; a1 = w1[j % KB]; a2 = w0[(j + 1) % KB]; a3 = w1[(j + 1) % KB];
       } else {
-        a0 = Lut::load(field_off<2 * KB, SH, KB>(w0, 2 * j), Q.lk_base, Q.lk_start);
-        a1 = Lut::load(field_off<2 * KB, SH, KB>(w1, 2 * j), Q.lk_base, Q.lk_start);
-        a2 = Lut::load(field_off<2 * KB, SH, KB>(w0, 2 * j + 1), Q.lk_base, Q.lk_start);
-        a3 = Lut::load(field_off<2 * KB, SH, KB>(w1, 2 * j + 1), Q.lk_base, Q.lk_start);
+        const uint2 f0 = field_pair<2 * KB, SH, KB>(w0, 2 * j), f1 = field_pair<2 * KB, SH, KB>(w1, 2 * j);
+        a0 = Lut::load(f0.x, Q.lk_base, Q.lk_start);
+        a1 = Lut::load(f1.x, Q.lk_base, Q.lk_start);
+        a2 = Lut::load(f0.y, Q.lk_base, Q.lk_start);
+        a3 = Lut::load(f1.y, Q.lk_base, Q.lk_start);
       }
       mma16816(s, a0, a1, a2, a3, Q.qf[j][0], Q.qf[j][1]);
       lo_half(sl, j, a0, a1, a2, a3, false);
@@ -399,7 +400,11 @@ __device__ __forceinline__ void g4_tile(G4State<NH>& S, uint32_t st, const G4Thr
         } else if constexpr (NODEQ) {
           h[q2][jj] = vw[2 * u + q2][jj & 1] ^ (uint32_t)jj;
         } else {
-          h[q2][jj] = VLut::load(field_off<2 * VB, SHV, 2>(vw[2 * u + q2], jj), Q.lv_base, Q.lv_start);
+          if ((jj & 1) == 0) {
+            const uint2 f = field_pair<2 * VB, SHV, 2>(vw[2 * u + q2], jj);
+            h[q2][jj] = VLut::load(f.x, Q.lv_base, Q.lv_start);
+            h[q2][jj + 1] = VLut::load(f.y, Q.lv_base, Q.lv_start);
+          }
         }
       }
     }
