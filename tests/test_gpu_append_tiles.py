@@ -1,8 +1,7 @@
 """Long appends, which take 128 vectors a tensor-core tile, against the same rows appended in short pieces, which the warp-level
 kernel takes: vectors around a tile's edge, head counts that leave a ragged last tile, zero rows, tokens without a slot.
 Both form every sum behind an index in the same order: indices are equal.  Scales come from sums of counts in another order:
-six roundings of 2^-24 in all; the residual of the sketch, rounded to 2^-24 of the vector's length, carries that to its norm (a
-third of the vector's length), and projections within 1e-6 of zero may change sign: 0.8e-6 of the bits."""
+six roundings of 2^-24 in all.  PROD keys take the warp-level kernel at every length: all of their record is equal."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -21,8 +20,7 @@ def _fields(cache):
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 @pytest.mark.parametrize("k,v,vectors", [("turbo2", "turbo2", 24568), ("turbo3", "turbo3", 24567), ("turbo3", "turbo3", 24568),
                                          ("turbo4", "turbo4", 24569), ("turbo3", "turbo3", 24703), ("turbo3", "turbo3", 75777),
-                                         ("turbo4", "turbo4", 131072), ("prod3", "q8_0", 63936), ("prod4", "turbo4", 85377),
-                                         ("prod3", "turbo3", 130049), ("q8_0", "turbo2", 262849), ("prod3", "turbo3", 284673)])
+                                         ("turbo4", "turbo4", 131072), ("q8_0", "turbo2", 262849), ("prod3", "turbo3", 284673)])
 def test_long_append_equals_short_ones(k, v, vectors, dtype):
     import torch
     import turboquant_plus_b200 as tq
@@ -50,15 +48,12 @@ def test_long_append_equals_short_ones(k, v, vectors, dtype):
     a, b = (_fields(c) for c in got)
     for t, fmt in (("k", k), ("v", v)):
         assert torch.equal(a[t], b[t])
-        if fmt == "q8_0":
-            assert torch.equal(a[t + "_scale"], b[t + "_scale"])
+        if fmt == "q8_0" or fmt.startswith("prod"):
+            for name in a:
+                assert not name.startswith(t) or torch.equal(a[name], b[name])
             continue
         written = torch.zeros(n_pages * 128, heads, device="cuda", dtype=torch.bool)
         written[slots[slots >= 0]] = True
         written = written.view(n_pages, 128, heads).transpose(1, 2)
         sa, sb = a[t + "_scale"][..., 0][written], b[t + "_scale"][..., 0][written]
         assert bool(((sa - sb).abs() <= 6 * 2.0 ** -24 * sb.abs()).all())
-        if fmt.startswith("prod"):
-            assert (a[t + "_sketch"] != b[t + "_sketch"]).any(-1).sum() <= 2 + 0.8e-6 * vectors * D
-            ra, rb = a[t + "_rscale"][..., 0][written], b[t + "_rscale"][..., 0][written]
-            assert bool(((ra - rb).abs() <= 2e-6 * rb.abs()).all())

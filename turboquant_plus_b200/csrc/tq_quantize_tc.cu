@@ -1,33 +1,28 @@
 // d = 128 sign-WHT quantizer for long appends: 128 vectors a tcgen05 tile, a thread a vector.
 //
-//   k_quantize_tc<Tin, BITS, NORMC, QJLS>   Tin = __half or __nv_bfloat16, symmetric codebook, packed output.
+//   k_quantize_tc<Tin, BITS, NORMC>   Tin = __half or __nv_bfloat16, symmetric codebook, packed output.
 //
 // The 16-point stage of the rotation, H128 = H8 (x) H16, is eight 128 x 16 x 16 products whose second operand is +-1: exact
 // products, fp32 sums.  With the sums in tensor memory a thread owns one vector (lane = vector): the 8-point stage, norms,
-// level counts and residual norms are sums in its own registers and the packed indices are its own 16 b bytes: no
-// exchanges between lanes, no staging.  The warp-level kernel (tq_quantize_mma.cu) deals a vector to four lanes: quad
-// reductions, a 4 x 4 word transpose, and with the sketch two more transforms through lane exchanges, 72
-// warp-instructions per turbo3 vector and 134 per PROD key.  Every sum that decides an index is formed in that kernel's order
-// (the whole 128-point rotation as one product rounds otherwise, and a handful of indices in a million vectors then differ).
+// and level counts are sums in its own registers and the packed indices are its own 16 b bytes: no exchanges between lanes,
+// no staging.  The warp-level kernel (tq_quantize_mma.cu) deals a vector to four lanes: quad reductions and a 4 x 4 word
+// transpose, 72 warp-instructions per turbo3 vector.  Every sum that decides an index is formed in that kernel's order (the whole
+// 128-point rotation as one product rounds otherwise, and a handful of indices in a million vectors then differ).
 //
 //   * One CTA per SM: a warp issues the tiled copies of the rows (a ring of operand tiles), a warp the MMAs (a ring of
 //     accumulators in tensor memory), and four groups of four warps take the accumulators in turn: 96 registers a thread, one
-//     piece of 32 columns at a time.  Three groups with 128, which the form with the sketch needs (and whose tensor memory
-//     holds three accumulators and the projections), are a sixth slower without it; loads and MMAs issued by the groups themselves
-//     a half.
+//     piece of 32 columns at a time.  Three groups with 128 are a sixth slower; loads and MMAs issued by the groups themselves a half.
 //   * the operand holds minus the transform: the sign bit of a sum alone decides the centre boundary (a zero is not above it).
 //   * thresholds are scaled by the vector's norm; a magnitude level is found bit by bit, the threshold of the next bit picked
 //     arithmetically; eight indices are an exact fp32 Horner sum; sign2 mirrors an index, an XOR of the packed words; level
 //     counts, exact small integers, give the norm correction.
-//   * QJLS (PROD keys with a 2- or 3-bit PolarQuant stage): sign(S r) for S = J2 H J1 in the coordinates before sign2 is one
-//     more product, J2 H J1 D1 H E, whose matrix holds even integers up to 128: M[n][k] = j2[n] T[n ^ k] with T the
-//     transform of j1 d1.  The residual, in units of the vector's length, goes to tensor memory as fp16 hi + lo (2^-24
-//     relative, as its own fp32 rounding) and is the A operand from there.
+//   * PROD keys stay with the warp-level kernel: the two transforms of their sign sketch are one product with an integer matrix
+//     here (1,048,576 keys 228 -> 129 us), but its sums round in another order, and of 33.6 M sketch bits some four then
+//     differ, which a key that a softmax rests on shows.
 //   * loops over the columns stay loops: unrolled, a tile's code misses the instruction caches.
 //
-// 1,048,576 fp16 vectors: turbo3 106 -> 87 us (3.7 TB/s; HBM would take 49), prod3 keys 228 -> 129; the arithmetic on the
-// coordinates bounds it, most of it on the half-rate compare and packed fp32 pipes.  Against 64 bits (33.6 M coordinates): the
-// warp-level kernel's indices, 0 to 4 sketch bits off (there 0 to 7), scales within 4e-7.
+// 1,048,576 fp16 vectors of turbo3: 106 -> 87 us (3.7 TB/s; HBM would take 49); the arithmetic on the coordinates bounds it, most of it
+// on the half-rate compare and packed fp32 pipes.  Scales are within 4e-7 of 64 bits, as the warp-level kernel's.
 #include <cuda.h>
 #include <type_traits>
 #include "tq_quantize_math.cuh"
@@ -42,9 +37,8 @@ namespace {
 //     turbo4 24,576 12.5 / 13.1, 65,536 23.4 / 25.1; turbo2 24,576 7.7 / 8.1, 65,536 13.6 / 14.2
 //   one tensor beside another kernel: q8_0 / turbo3 131,072 27.2 / 27.7, 262,144 51.2 / 51.4, 1,048,576 171 / 190; q8_0 / turbo2
 //     131,072 25.7 / 24.7, 262,144 45.8 / 45.7, 1,048,576 147 / 168
-//   with the sketch: prod3 / turbo3 32,768 18.0 / 13.7, 65,536 24.5 / 25.7, 1,048,576 216 / 334; prod4 / turbo4 32.5 / 33, 345 / 449
 // In vectors per SM (148), so that a device with fewer SMs takes the step earlier.
-inline int64_t qt_min_vectors(bool pair, bool qjl) { return (int64_t)tq_num_sms() * (pair ? 166 : qjl ? 432 : 1776); }
+inline int64_t qt_min_vectors(bool pair) { return (int64_t)tq_num_sms() * (pair ? 166 : 1776); }
 
 struct QtJob {
   CUtensorMap map;   // of the rows: 64 elements x 128 rows a box, 128-byte swizzle
@@ -52,18 +46,12 @@ struct QtJob {
   TqQuantDst dst;
 };
 
-template <int BITS, bool QJLS> struct QtShape {
-  static constexpr int GROUPS = QJLS ? 3 : 4, TMA_WARP = 4 * GROUPS, MMA_WARP = TMA_WARP + 1;
-  // four groups: a fifth, whole warpgroup, most of whose registers go to the groups (640 x 96 = 512 x 112 + 128 x 32)
-  static constexpr int THREADS = 32 * (MMA_WARP + 1);
-  static constexpr int SLOTS = QJLS ? 3 : 4;                // 128-column accumulators; QJLS: the fourth holds projections
-  static constexpr int STAGES = QJLS ? 5 : 6;            // row tiles in flight
-  static constexpr int TILE = TQ_D * TQ_D * 2;           // bytes of a 128 x 128 operand tile
-  static constexpr int OFF_A = 0;
-  static constexpr int OFF_B = OFF_A + STAGES * TILE;
-  static constexpr int OFF_M = OFF_B + 8 * 512;          // the eight 16 x 16 matrices first
-  static constexpr int BYTES = OFF_M + (QJLS ? TILE : 0) + 1024;   // + alignment (128-byte swizzle: 1,024)
-};
+constexpr int QT_GROUPS = 4, QT_TMA_WARP = 4 * QT_GROUPS, QT_MMA_WARP = QT_TMA_WARP + 1, QT_THREADS = 32 * (QT_MMA_WARP + 1);
+constexpr int QT_SLOTS = 4;                            // 128-column accumulators
+constexpr int QT_STAGES = 6;                           // row tiles in flight
+constexpr int QT_TILE = TQ_D * TQ_D * 2;               // bytes of a row tile
+constexpr int QT_OFF_B = QT_STAGES * QT_TILE;          // the eight 16 x 16 matrices
+constexpr int QT_BYTES = QT_OFF_B + 8 * 512 + 1024;    // + alignment (128-byte swizzle: 1,024)
 
 template <typename T> struct QtIn;
 template <> struct QtIn<__half> { static constexpr uint32_t ONES = 0x3C003C00u, FMT = 0; };
@@ -72,14 +60,10 @@ template <> struct QtIn<__nv_bfloat16> { static constexpr uint32_t ONES = 0x3F80
 // row a of the 8-point Hadamard matrix as bits: bit j = parity(a & j)
 __device__ __forceinline__ uint32_t qt_had8(uint32_t a) { return (uint32_t)(0x963C5AF066CCAA00ull >> (8 * a)) & 0xffu; }
 
-// D = A B^T (128 x 128 x 16, one CTA), A from shared or tensor memory
+// D = A B^T (128 x 16 x 16, one CTA)
 __device__ __forceinline__ void qt_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
                ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
-}
-__device__ __forceinline__ void qt_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void qt_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sptr(bar)) : "memory");
@@ -196,15 +180,6 @@ __device__ __forceinline__ void qt_pack32(const uint32_t (&nu)[32], const QtLeve
   }
 }
 
-// the residual of two coordinates in units of the vector's length (times a power of two), as fp16 hi and lo pairs
-__device__ __forceinline__ void qt_split2(float2 e, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(e.x, e.y);
-  const float2 r = qm_sub2(e, __half22float2(h));
-  const __half2 l = __floats2half2_rn(r.x, r.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
 // K-major operand in 128-byte swizzle atoms of 8 rows x 64 elements (what the tiled copies write)
 __device__ __forceinline__ uint64_t qt_desc_sw128(uint32_t addr) {
   return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
@@ -227,36 +202,18 @@ __device__ __forceinline__ void qt_ld_wait(uint32_t (&v)[32]) {
         "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]) :: "memory");
 }
 // 128 columns as two turns of two pieces of 32: use(half, turn, values) twice, then done(turn).  A loop, not unrolled: the code of
-// a tile then fits the instruction caches (prod3 keys of 131,072 tokens x 8 heads: 168 us unrolled, 125 so).  AHEAD: the next piece
-// is on its way while use() works on one, for which 96 registers have no room.
-template <bool AHEAD, typename U, typename D> __device__ __forceinline__ void qt_columns(uint32_t addr, U&& use, D&& done) {
-  using First = std::integral_constant<int, 0>;
-  using Second = std::integral_constant<int, 1>;
-  if constexpr (AHEAD) {
-    uint32_t ua[32], ub[32];
-    qt_ld32(addr, ua);
+// a tile then fits the instruction caches.
+template <typename U, typename D> __device__ __forceinline__ void qt_columns(uint32_t addr, U&& use, D&& done) {
+  uint32_t u[32];
 #pragma unroll 1
-    for (int turn = 0; turn < 2; ++turn) {
-      qt_ld_wait(ua);
-      qt_ld32(addr + 64 * turn + 32, ub);
-      use(First{}, turn, ua);
-      qt_ld_wait(ub);
-      if (turn == 0) qt_ld32(addr + 64, ua);
-      use(Second{}, turn, ub);
-      done(turn);
-    }
-  } else {
-    uint32_t u[32];
-#pragma unroll 1
-    for (int turn = 0; turn < 2; ++turn) {
-      qt_ld32(addr + 64 * turn, u);
-      qt_ld_wait(u);
-      use(First{}, turn, u);
-      qt_ld32(addr + 64 * turn + 32, u);
-      qt_ld_wait(u);
-      use(Second{}, turn, u);
-      done(turn);
-    }
+  for (int turn = 0; turn < 2; ++turn) {
+    qt_ld32(addr + 64 * turn, u);
+    qt_ld_wait(u);
+    use(std::integral_constant<int, 0>{}, turn, u);
+    qt_ld32(addr + 64 * turn + 32, u);
+    qt_ld_wait(u);
+    use(std::integral_constant<int, 1>{}, turn, u);
+    done(turn);
   }
 }
 // eight columns
@@ -278,19 +235,15 @@ __device__ __forceinline__ void qt_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sptr(bar)) : "memory");
 }
 
-template <typename Tin, int BITS, bool NORMC, bool QJLS>
-__global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc(const __grid_constant__ QtJob j0, const __grid_constant__ QtJob j1,
+template <typename Tin, int BITS, bool NORMC>
+__global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_constant__ QtJob j0, const __grid_constant__ QtJob j1,
                                                                          int64_t n) {
-  using SH = QtShape<BITS, QJLS>;
-  constexpr int IDXB = 16 * BITS, NC = 1 << BITS, HALF = NC / 2, SLOTS = SH::SLOTS, STAGES = SH::STAGES;
-  // residuals are carried times 2^6: below 600 for a unit vector, and the lo halves stay above fp16's subnormals
-  constexpr float ESCALE = 64.0f;
+  constexpr int IDXB = 16 * BITS, NC = 1 << BITS, HALF = NC / 2, SLOTS = QT_SLOTS, STAGES = QT_STAGES;
   extern __shared__ __align__(128) uint8_t qt_raw[];
-  __shared__ uint64_t a_full[STAGES], a_free[STAGES], d_full[SLOTS], d_free[SLOTS], e_full[SH::GROUPS], p_full[SH::GROUPS], p_free[SH::GROUPS];
+  __shared__ uint64_t a_full[STAGES], a_free[STAGES], d_full[SLOTS], d_free[SLOTS];
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_failed;   // a wait gave up: every role stops at its next tile
   __shared__ __align__(16) uint32_t s_flip[4 * BITS];
-  __shared__ __half s_T[QJLS ? TQ_D : 1];
   const QtJob& job = blockIdx.y == 0 ? j0 : j1;
   const TqFast& f = job.f;
   const TqQuantDst& dst = job.dst;
@@ -305,7 +258,6 @@ __global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc
     };
     for (int i = 0; i < STAGES; ++i) init(&a_full[i], 1), init(&a_free[i], 1);
     for (int i = 0; i < SLOTS; ++i) init(&d_full[i], 1), init(&d_free[i], 4);
-    for (int i = 0; i < SH::GROUPS; ++i) init(&e_full[i], 4), init(&p_full[i], 1), init(&p_free[i], 4);
     s_failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -319,38 +271,12 @@ __global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc
 #pragma unroll
       for (int p = 0; p < 4; ++p)
         w[p] = QtIn<Tin>::ONES ^ (((m >> (2 * p)) & 1u) << 15) ^ (((m >> (2 * p + 1)) & 1u) << 31);
-      *reinterpret_cast<uint4*>(sm + SH::OFF_B + tid * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(sm + QT_OFF_B + tid * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     } else if (tid < 256 + 4 * BITS) {   // sign2 mirrors an index (i -> 2^b - 1 - i): all bits of its field in the packed stream
       uint32_t w = 0;
 #pragma unroll
       for (int k = 0; k < 32; ++k) w |= qm_bit(f.s2, (32 * (tid - 256) + k) / BITS) << (8 * (k >> 3) + 7 - (k & 7));
       s_flip[tid - 256] = w;
-    }
-    if constexpr (QJLS) {
-      if (tid < TQ_D) {   // T = transform of the signs j1 d1: 128 - 2 x (positions where a Hadamard row differs from them)
-        const uint32_t row8 = qt_had8(tid & 7);
-        int differ = 0;
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          uint32_t row = 0;
-#pragma unroll
-          for (int b = 0; b < 4; ++b) row |= (row8 ^ ((__popc((tid >> 3) & (4 * w + b)) & 1) ? 0xffu : 0u)) << (8 * b);
-          differ += __popc(row ^ f.s1[w] ^ f.j1[w]);
-        }
-        s_T[tid] = __int2half_rn(TQ_D - 2 * differ);
-      }
-      __syncthreads();
-      for (int i = tid; i < TQ_D * 16; i += SH::THREADS) {
-        const int out = (i >> 7) * 8 + (i & 7), c = (i >> 3) & 15;
-        const uint32_t neg = qm_bit(f.j2, out) * 0x80008000u;
-        uint32_t w[4];
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          const uint32_t lo = __half_as_ushort(s_T[out ^ (8 * c + 2 * p)]), hi = __half_as_ushort(s_T[out ^ (8 * c + 2 * p + 1)]);
-          w[p] = (lo | (hi << 16)) ^ neg;
-        }
-        *reinterpret_cast<uint4*>(sm + SH::OFF_M + i * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -367,25 +293,25 @@ __global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc
   const int64_t tiles = (n + TQ_D - 1) / TQ_D, step = gridDim.x;
   const int mine = (int)((tiles - blockIdx.x + step - 1) / step);   // tiles of this CTA: blockIdx.x + i step
 
-  if (warp == SH::TMA_WARP) {
+  if (warp == QT_TMA_WARP) {
     if (lane == 0) {
       int i = 0;
       for (; i < mine && !s_failed; ++i) {
         const int st = i % STAGES;
         if (i >= STAGES && !tc_wait(&a_free[st], (uint32_t)((i / STAGES - 1) & 1))) { s_failed = 1; break; }
-        const uint32_t dsts = sptr(sm) + SH::OFF_A + st * SH::TILE;
+        const uint32_t dsts = sptr(sm) + st * QT_TILE;
         const int row = (int)((blockIdx.x + i * step) * TQ_D);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(&a_full[st])), "r"(SH::TILE) : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(&a_full[st])), "r"(QT_TILE) : "memory");
 #pragma unroll
         for (int h = 0; h < 2; ++h)   // (rows past n come as zeros)
           asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                           dsts + h * (SH::TILE / 2)), "l"(&job.map), "r"(64 * h), "r"(row), "r"(sptr(&a_full[st])) : "memory");
+                           dsts + h * (QT_TILE / 2)), "l"(&job.map), "r"(64 * h), "r"(row), "r"(sptr(&a_full[st])) : "memory");
       }
       for (int k = i < STAGES ? 0 : i - STAGES; k < i; ++k) tc_wait(&a_full[k % STAGES], (uint32_t)((k / STAGES) & 1));   // none in flight at the end
     }
-  } else if (warp == SH::MMA_WARP) {
+  } else if (warp == QT_MMA_WARP) {
     if (lane == 0) {
-      const uint32_t idesc = umma_idesc(128, 16, false) | QtIn<Tin>::FMT, b = sptr(sm) + SH::OFF_B;
+      const uint32_t idesc = umma_idesc(128, 16, false) | QtIn<Tin>::FMT, b = sptr(sm) + QT_OFF_B;
       for (int i = 0; i < mine && !s_failed; ++i) {
         const int st = i % STAGES, sl = i % SLOTS;
         if (!tc_wait(&a_full[st], (uint32_t)((i / STAGES) & 1)) || (i >= SLOTS && !tc_wait(&d_free[sl], (uint32_t)((i / SLOTS - 1) & 1)))) {
@@ -393,19 +319,19 @@ __global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a = sptr(sm) + SH::OFF_A + st * SH::TILE;
+        const uint32_t a = sptr(sm) + st * QT_TILE;
 #pragma unroll
         for (int i16 = 0; i16 < 8; ++i16)
-          qt_mma_ss(tb + 128 * sl + 16 * i16, qt_desc_sw128(a + (i16 >> 2) * (SH::TILE / 2) + (i16 & 3) * 32),
+          qt_mma_ss(tb + 128 * sl + 16 * i16, qt_desc_sw128(a + (i16 >> 2) * (QT_TILE / 2) + (i16 & 3) * 32),
                     umma_desc(b + i16 * 512, 128, 256), idesc, 0);
         qt_commit(&a_free[st]);
         qt_commit(&d_full[sl]);
       }
     }
-  } else if (warp < SH::TMA_WARP) {
+  } else if (warp < QT_TMA_WARP) {
   const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;   // this warp's 32 lanes
   const uint32_t zero_idx = 0.f > f.bnd[HALF - 1] ? HALF : HALF - 1;   // index of the value 0
-  for (int i = group; i < mine; i += SH::GROUPS) {
+  for (int i = group; i < mine; i += QT_GROUPS) {
     const int sl = i % SLOTS;
     const uint32_t tm = tb + 128 * sl + lanes;
     const int64_t v = (blockIdx.x + i * step) * TQ_D + gtid;
@@ -418,7 +344,6 @@ __global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc
     // ---- the 8-point stage over the blocks, in place, eight columns of every block a turn, and ||x||: ||H x||^2 = 128 ||x||^2.
     // Sums in the warp-level kernel's order (four columns of all blocks, then those four sums in pairs): both kernels then
     // find the same indices ----
-    constexpr bool AHEAD = SH::GROUPS == 3;
     float ss = 0.f;
 #pragma unroll 1
     for (int turn = 0; turn < 2; ++turn) {
@@ -471,9 +396,8 @@ __global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc
     const uint32_t zero24 = zero_idx * 0x249249u;
     const uint32_t zero0 = BITS == 2 ? zero_idx * 0x55555555u : BITS == 4 ? zero_idx * 0x11111111u : __byte_perm(zero24, zero24, 0x6012);
     const uint32_t zero1 = BITS == 3 ? __byte_perm(zero24, zero24, 0x5601) : zero0, zero2 = BITS == 3 ? __byte_perm(zero24, zero24, 0x4560) : zero0;
-    auto nothing = [](int) {};
     uint32_t w[2 * BITS];
-    qt_columns<AHEAD>(tm, [&](auto half, int turn, const uint32_t (&u)[32]) {
+    qt_columns(tm, [&](auto half, int turn, const uint32_t (&u)[32]) {
       uint32_t o[BITS];
       qt_pack32<BITS, NORMC>(u, lv, cnt, o);
 #pragma unroll
@@ -487,11 +411,9 @@ __global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc
         else if (k % 4 == 0) reinterpret_cast<uint4*>(p)[k / 4] = make_uint4(w[k], w[k + 1], w[k + 2], w[k + 3]);
       }
     });
-    if constexpr (!QJLS) {   // the accumulator is free
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) qt_arrive(&d_free[sl]);
-    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");   // the accumulator is free
+    __syncwarp();
+    if (lane == 0) qt_arrive(&d_free[sl]);
     float invn = 1.0f;
     if constexpr (NORMC) {
       float cn = sqrtf(fmaf((float)TQ_D, f.cent[HALF] * f.cent[HALF], cnt.squares(f.cent)));
@@ -503,75 +425,6 @@ __global__ void __launch_bounds__(QtShape<BITS, QJLS>::THREADS, 1) k_quantize_tc
       *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.scale) + rec + within * 4) = nrm * invn;
     }
     if (v < n && dst.norm) dst.norm[v] = nrm;
-    if constexpr (QJLS) {
-      // ---- residual y - c / ||c||, in place of the sums: hi and lo halves of 32 coordinates over the columns they come from ----
-      const float rts = -ESCALE / ts, cs = ESCALE * invn;
-      float c0, c1, c2 = 0.f, c21 = 0.f;                // magnitude of the chosen centroid: c0 + p1 c1 + p2 (c2 + p1 c21)
-      c0 = f.cent[HALF] * cs;
-      c1 = (f.cent[HALF + 1] - f.cent[HALF]) * cs;
-      if constexpr (BITS == 3) {
-        c2 = (f.cent[HALF + 2] - f.cent[HALF]) * cs;
-        c21 = ((f.cent[HALF + 3] - f.cent[HALF + 2]) - (f.cent[HALF + 1] - f.cent[HALF])) * cs;
-      }
-      float2 eea = make_float2(0.f, 0.f), eeb = eea;
-      qt_columns<AHEAD>(tm, [&](auto half, int turn, const uint32_t (&u)[32]) {
-        uint32_t hl[32];
-#pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-          float2 p4, p2, p1, cm;
-          const float2 nu = make_float2(__uint_as_float(u[k]), __uint_as_float(u[k + 1]));
-          lv.test(make_float2(fabsf(nu.x), fabsf(nu.y)), p4, p2, p1);
-          if constexpr (BITS == 2) cm = qm_fma2(p1, qm_dup(c1), qm_dup(c0));
-          else cm = qm_fma2(p1, qm_fma2(p2, qm_dup(c21), qm_dup(c1)), qm_fma2(p2, qm_dup(c2), qm_dup(c0)));
-          // minus the centroid, which carries the value's sign: nu's sign is clear where the value is not above zero
-          cm.x = __uint_as_float(__float_as_uint(cm.x) | (u[k] & 0x80000000u));
-          cm.y = __uint_as_float(__float_as_uint(cm.y) | (u[k + 1] & 0x80000000u));
-          const float2 e = qm_fma2(nu, qm_dup(rts), cm);
-          if (k & 2) eeb = qm_fma2(e, e, eeb); else eea = qm_fma2(e, e, eea);
-          qt_split2(e, hl[k >> 1], hl[16 + (k >> 1)]);
-        }
-        tmem_st32(tm + 64 * turn + 32 * decltype(half)::value, hl);
-      }, nothing);
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) qt_arrive(&e_full[group]);
-      if (gtid == 0) {   // the projections' columns serve the tiles in turn: the group of the tile before has read its own
-        if (!tc_wait(&e_full[group], (uint32_t)((i / SH::GROUPS) & 1)) || (i > 0 && !tc_wait(&p_free[(i - 1) % SH::GROUPS], (uint32_t)(((i - 1) / SH::GROUPS) & 1)))) s_failed = 1;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t b = sptr(sm) + SH::OFF_M, e = tb + 128 * sl;
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t bd = umma_desc(b + ks * 256, 128, 2048);
-          const uint32_t hi = e + 32 * (ks >> 1) + 8 * (ks & 1);
-          qt_mma_ts(tb + 384, hi, bd, umma_idesc(128, 128, false), ks > 0);
-          qt_mma_ts(tb + 384, hi + 16, bd, umma_idesc(128, 128, false), 1);
-        }
-        qt_commit(&p_full[group]);
-      }
-      const float2 ee2 = qm_add2(eea, eeb);
-      const float rn = nrm > 0.f ? sqrtf(ee2.x + ee2.y) * (safe / ESCALE) : 0.f;   // ||r|| = ||x|| * ||y - yhat'||
-      if (!__all_sync(0xffffffffu, tc_wait(&p_full[group], (uint32_t)((i / SH::GROUPS) & 1)))) s_failed = 1, failed = true;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (lane == 0) qt_arrive(&d_free[sl]);   // the residual has been read
-      uint32_t sk[2];
-      qt_columns<AHEAD>(tb + 384 + lanes, [&](auto half, int, const uint32_t (&u)[32]) {
-        uint32_t m = 0;
-#pragma unroll
-        for (int k = 0; k < 32; ++k) m = __funnelshift_l(u[k], m, 1);
-        // bit = 1 where the projection is >= 0 (turboquant/qjl.py:89-90), the first one in the most significant place;
-        // zero input -> zero residual -> all +1
-        sk[decltype(half)::value] = nrm > 0.f ? __byte_perm(~m, 0, 0x0123) : 0xffffffffu;
-      }, [&](int turn) {
-        if (good && dst.qjl) *reinterpret_cast<uint2*>(dst.qjl + rec + within * 16 + 8 * turn) = make_uint2(sk[0], sk[1]);
-      });
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) qt_arrive(&p_free[group]);
-      if (v < n && good && dst.rnorm)   // sqrt(pi/2)/sqrt(d): turboquant/qjl.py:32,131
-        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.rnorm) + rec + within * 4) =
-            failed ? __int_as_float(0x7fffffff) : dst.rscale_const ? rn * (1.2533141373155001f * TQ_RSQRT_D) : rn;
-    }
     if (failed) break;
   }
   }
@@ -604,29 +457,27 @@ bool qt_map(CUtensorMap* map, const void* x, int32_t dtype, int64_t ld, int64_t 
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename Tin, int BITS, bool NORMC, bool QJLS>
+template <typename Tin, int BITS, bool NORMC>
 int launch_tc(const QtJob& j0, const QtJob& j1, int jobs, int64_t n, cudaStream_t st) {
-  using SH = QtShape<BITS, QJLS>;
-  auto kernel = k_quantize_tc<Tin, BITS, NORMC, QJLS>;
+  auto kernel = k_quantize_tc<Tin, BITS, NORMC>;
   static thread_local int configured_dev = -1;   // one per kernel
   int dev = 0;
   TQ_CUDA(cudaGetDevice(&dev));
   if (configured_dev != dev) {
-    TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::BYTES));
+    TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, QT_BYTES));
     configured_dev = dev;
   }
   const int64_t tiles = (n + TQ_D - 1) / TQ_D, places = tq_num_sms() / jobs > 0 ? tq_num_sms() / jobs : 1;
   const dim3 grid((unsigned)(tiles < places ? tiles : places), jobs);   // one CTA per SM; few tiles: one group of each
-  TQ_CUDA(tq_launch_early(kernel, grid, SH::THREADS, SH::BYTES, st, j0, j1, n));
+  TQ_CUDA(tq_launch_early(kernel, grid, QT_THREADS, QT_BYTES, st, j0, j1, n));
   return tq_launch_check("k_quantize_tc");
 }
 
 template <typename Tin>
-int launch_tc_bits(const QtJob& j0, const QtJob& j1, int jobs, bool normc, bool qjl, int64_t n, cudaStream_t st) {
-#define TQ_TC(B, Q)                                                                                       \
-  if (j0.f.bits == B && qjl == Q)                                                                         \
-    return normc ? launch_tc<Tin, B, true, Q>(j0, j1, jobs, n, st) : launch_tc<Tin, B, false, Q>(j0, j1, jobs, n, st);
-  TQ_TC(2, false) TQ_TC(3, false) TQ_TC(4, false) TQ_TC(2, true) TQ_TC(3, true)
+int launch_tc_bits(const QtJob& j0, const QtJob& j1, int jobs, bool normc, int64_t n, cudaStream_t st) {
+#define TQ_TC(B) \
+  if (j0.f.bits == B) return normc ? launch_tc<Tin, B, true>(j0, j1, jobs, n, st) : launch_tc<Tin, B, false>(j0, j1, jobs, n, st);
+  TQ_TC(2) TQ_TC(3) TQ_TC(4)
 #undef TQ_TC
   return TQ_ERR_UNSUPPORTED;
 }
@@ -634,14 +485,14 @@ int launch_tc_bits(const QtJob& j0, const QtJob& j1, int jobs, bool normc, bool 
 }  // namespace
 
 // One tensor, or two of the same shape and format (x1 != nullptr), whose requests the warp-level kernel serves: false where that
-// kernel is to take them.  want_qjl: with the sign sketch (one tensor).
+// kernel is to take them.
 bool tq_quantize_tc_try(const TqFast& f0, const void* x0, const TqQuantDst& d0, const TqFast* f1, const void* x1, const TqQuantDst* d1,
-                        int32_t dtype, int64_t ld, int64_t n, bool normc, bool want_qjl, cudaStream_t st, int* rc) {
+                        int32_t dtype, int64_t ld, int64_t n, bool normc, cudaStream_t st, int* rc) {
   if (dtype != TQ_F16 && dtype != TQ_BF16) return false;
-  if (n < qt_min_vectors(x1 != nullptr, want_qjl)) return false;
-  // a thread stores its vector's indices and sketch up to 16 bytes at a time
+  if (n < qt_min_vectors(x1 != nullptr)) return false;
+  // a thread stores its vector's indices up to 16 bytes at a time
   auto aligned = [](const TqQuantDst& d) {
-    return tq_aligned(d.idx, 16) && tq_aligned(d.qjl, 16) && d.page_stride % 16 == 0 && d.head_stride % 16 == 0;
+    return tq_aligned(d.idx, 16) && d.page_stride % 16 == 0 && d.head_stride % 16 == 0;
   };
   if (!tq_aligned(x0, 16) || !aligned(d0) || (x1 && (!tq_aligned(x1, 16) || !aligned(*d1)))) return false;
   QtJob j0, j1;
@@ -654,7 +505,7 @@ bool tq_quantize_tc_try(const TqFast& f0, const void* x0, const TqQuantDst& d0, 
     j1 = j0;
   }
   const int jobs = x1 ? 2 : 1;
-  *rc = dtype == TQ_F16 ? launch_tc_bits<__half>(j0, j1, jobs, normc, want_qjl, n, st)
-                        : launch_tc_bits<__nv_bfloat16>(j0, j1, jobs, normc, want_qjl, n, st);
+  *rc = dtype == TQ_F16 ? launch_tc_bits<__half>(j0, j1, jobs, normc, n, st)
+                        : launch_tc_bits<__nv_bfloat16>(j0, j1, jobs, normc, n, st);
   return true;
 }
