@@ -16,8 +16,8 @@
 //     immediate offsets; only the last page of a sequence runs the variant that masks tokens past the end.
 //   * q8_0 operands are int8 -> fp16 by byte permute + one subtract (exact), the per-block scales applied to the
 //     partial scores of each 32-dim block in fp32 (keys) or to the operand pairs (values); the sign sketch of PROD
-//     keys becomes +-1 operands by one shift and one logic op per pair (dims d and d + 16 of a 32-bit word pair up,
-//     so that their bits land on the two fp16 sign positions together), against the S-projected query.
+//     keys becomes operands by one logic op per pair: dims d and d + 16 of a 32-bit word pair up, and the masked word is a
+//     pair of fp16 numbers of one set bit each (or zero), against the S-projected query divided by them.
 //   * eight heads: the columns of S are the heads, hi and lo halves are two MMAs into two accumulators and no exchange is
 //     needed (thread (g, t) owns tokens g and g + 8, heads 2t and 2t + 1); O^T takes two MMAs per operand, heads 0..3 and
 //     4..7, for the same dequantized words.  Dequantization is the cost, and eight heads share it: dealt to two CTAs of
@@ -224,12 +224,19 @@ __device__ __forceinline__ uint32_t s8x2_to_h2(uint32_t biased, uint32_t sel) {
   return hsub2_u32(__byte_perm(biased, 0x64646464u, sel), 0x64806480u);
 }
 
+// Sign sketch: where a half of a pair word has the bit of dim i (of 0..15), and what fp16 number that is, inverted
+__device__ __forceinline__ constexpr int g4_sketch_bit(int i) { return 13 - (i & 7); }
+__device__ __forceinline__ constexpr float g4_sketch_scale(int i) {
+  const int b = g4_sketch_bit(i);   // 13, 12, 11, 10: exponents 8, 4, 2, 1; below: subnormal
+  return (float)(1 << (b == 13 ? 7 : b == 12 ? 11 : b == 11 ? 13 : b == 10 ? 14 : 24 - b));
+}
 // The queries as B operands, and what goes with the tables
 template <int KK, int NH> struct G4Q {
   static constexpr bool PROD = Kind<KK>::PROD;
   uint32_t qf[8][2];                                  // NH 4: columns 0-3 the hi halves, 4-7 the lo halves; NH 8: hi
   uint32_t ql[NH == 8 && !PROD ? 8 : 1][2];           // NH 8: lo
-  uint32_t qp[PROD ? 8 : 1][2];                       // PROD: the projected query, as qf
+  uint32_t qp[PROD ? 8 : 1][2];                       // PROD: the projected query, as qf, over the sketch operands' values
+  float zs0, zs1, zc0, zc1;                           // PROD: <S q, z> of columns 2t, 2t + 1 = sums x zs - zc
   uint32_t lo;                                        // PROD, NH 8: shared-memory address of this lane's lo fragments
   uint32_t lk_base, lk_start, lv_base, lv_start;
 };
@@ -316,22 +323,25 @@ __device__ __forceinline__ void g4_scores(float (&s)[4], uint32_t st, const G4Th
     }
     if constexpr (NH == 8) { s[0] += sl[0]; s[1] += sl[1]; s[2] += sl[2]; s[3] += sl[3]; }
     if constexpr (KT::PROD) {
-      // + sqrt(pi/2)/sqrt(d) * ||r|| * <S q, z>: the sign sketch as +-1 operands.  Word t of a row holds its 32 dims
-      // 32t .. 32t+31, first dim in the most significant bit; dims i and i + 16 form a pair, so that after a shift by
-      // i their bits sit on the sign positions of the two fp16 halves (bit set = +1).
+      // + sqrt(pi/2)/sqrt(d) * ||r|| * <S q, z>, as 2 sum over the set bits minus the sum over all.  Word t of a row holds its 32 dims
+      // 32t .. 32t+31, first dim in the most significant bit; dims i and i + 16 form a pair, whose bits sit at the same place of
+      // the word's two halves.  A half with one of the bits 6..13 set is the fp16 number 2^-18 .. 2^-7 (g4_sketch_scale), by which the
+      // projected query is divided beforehand: after two shifts a pair is one logic operation (a shift and one for +-1
+      // operands made PROD keys wait for the integer pipe).
       const uint32_t z0 = __byte_perm(lds_u32<TOK0 * 16>(st + T.z_thr), 0, 0x0123);
       const uint32_t z1 = __byte_perm(lds_u32<(TOK0 + 8) * 16>(st + T.z_thr), 0, 0x0123);
       float s2[4] = {0.f, 0.f, 0.f, 0.f}, sl2[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const uint32_t a0 = (~(z0 << (2 * j)) & 0x80008000u) | 0x3C003C00u;
-        const uint32_t a1 = (~(z1 << (2 * j)) & 0x80008000u) | 0x3C003C00u;
-        const uint32_t a2 = (~(z0 << (2 * j + 1)) & 0x80008000u) | 0x3C003C00u;
-        const uint32_t a3 = (~(z1 << (2 * j + 1)) & 0x80008000u) | 0x3C003C00u;
+        const uint32_t m0 = 0x00010001u << g4_sketch_bit(2 * j), m1 = 0x00010001u << g4_sketch_bit(2 * j + 1);
+        const uint32_t x0 = j < 4 ? z0 >> 2 : z0 << 6, x1 = j < 4 ? z1 >> 2 : z1 << 6;
+        const uint32_t a0 = x0 & m0, a1 = x1 & m0, a2 = x0 & m1, a3 = x1 & m1;
         mma16816(s2, a0, a1, a2, a3, Q.qp[j][0], Q.qp[j][1]);
         lo_half(sl2, j, a0, a1, a2, a3, true);
       }
       if constexpr (NH == 8) { s2[0] += sl2[0]; s2[1] += sl2[1]; s2[2] += sl2[2]; s2[3] += sl2[3]; }
+      s2[0] = fmaf(s2[0], Q.zs0, -Q.zc0); s2[1] = fmaf(s2[1], Q.zs1, -Q.zc1);
+      s2[2] = fmaf(s2[2], Q.zs0, -Q.zc0); s2[3] = fmaf(s2[3], Q.zs1, -Q.zc1);
       const float k0 = lds_f32<TOK0 * 4>(st + T.ks_thr), k1 = lds_f32<TOK0 * 4 + 32>(st + T.ks_thr);
       const float r0 = lds_f32<TOK0 * 4>(st + T.rs_thr), r1 = lds_f32<TOK0 * 4 + 32>(st + T.rs_thr);
       s[0] = fmaf(s2[0], r0, s[0] * k0); s[1] = fmaf(s2[1], r0, s[1] * k0);
@@ -711,6 +721,30 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     const float* qh = qbuf + (hv ? head : 0) * TQ_D;
     uint2* lo_frag = reinterpret_cast<uint2*>(smg + C::G_LO) + lane;   // (LO_SMEM: the same in every warp, written by the first)
     Q.lo = smem_u32(lo_frag);
+    // PROD: the projected query's largest element is brought to 2^-4 .. 2^-3, so that 2^18 times it is an fp16 number
+    float zscale = 1.f;
+    if constexpr (KT::PROD) {
+      const float* ph = qbuf + NH * TQ_D + (hv ? head : 0) * 4 + t;
+      float most = 0.f, total = 0.f;
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        const float y = hv ? ph[c * (4 * NH)] : 0.f;
+        most = fmaxf(most, fabsf(y));
+        total += y;
+      }
+#pragma unroll
+      for (int m = 1; m <= 2; m <<= 1) {   // the quad's four parts of the row
+        most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, m));
+        total += __shfl_xor_sync(0xffffffffu, total, m);
+      }
+      const int e = (int)((__float_as_uint(most) >> 23) & 255u);            // most < 2^(e - 126)
+      zscale = e > 0 && e < 240 ? __uint_as_float((uint32_t)(250 - e) << 23) : 1.f;   // 2^(123 - e): most x zscale < 2^-3
+      const float back = 2.f / zscale, take = lo ? 0.f : total;             // (the lo halves are part of the same sum)
+      Q.zs0 = __shfl_sync(0xffffffffu, back, 8 * t);                        // column 2t is that of the lanes g = 2t
+      Q.zs1 = __shfl_sync(0xffffffffu, back, 8 * t + 4);
+      Q.zc0 = __shfl_sync(0xffffffffu, take, 8 * t);
+      Q.zc1 = __shfl_sync(0xffffffffu, take, 8 * t + 4);
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       // dims this thread supplies in k-step j: 32t + 4j .. +3 (packed formats), or, for q8_0 keys, its 8 dims of
@@ -734,7 +768,8 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
         // k-step, 2j + 1 for the second), dim i + 16 in the low half
         const float* ph = qbuf + NH * TQ_D + (hv ? head : 0) * 4 + t;
         auto proj = [&](int c) { return hv ? ph[c * (4 * NH)] : 0.f; };
-        const float a0 = proj(16 + 2 * j), a1 = proj(2 * j), b0 = proj(16 + 2 * j + 1), b1 = proj(2 * j + 1);
+        const float za = zscale * g4_sketch_scale(2 * j), zb = zscale * g4_sketch_scale(2 * j + 1);
+        const float a0 = proj(16 + 2 * j) * za, a1 = proj(2 * j) * za, b0 = proj(16 + 2 * j + 1) * zb, b1 = proj(2 * j + 1) * zb;
         const __half2 e0 = __floats2half2_rn(a0, a1), e1 = __floats2half2_rn(b0, b1);
         const float2 r0 = __half22float2(e0), r1 = __half22float2(e1);
         const uint32_t m0 = pack_h2(a0 - r0.x, a1 - r0.y), m1 = pack_h2(b0 - r1.x, b1 - r1.y);
