@@ -57,3 +57,59 @@ def test_long_append_equals_short_ones(k, v, vectors, dtype):
         written = written.view(n_pages, 128, heads).transpose(1, 2)
         sa, sb = a[t + "_scale"][..., 0][written], b[t + "_scale"][..., 0][written]
         assert bool(((sa - sb).abs() <= 6 * 2.0 ** -24 * sb.abs()).all())
+
+
+def _odd_rows(tokens, heads, dtype, gen):
+    """Rows whose coordinates are exact zeros in number (few nonzeros of one magnitude, small integers, signed zeros), rows with
+    outlier channels, and rows at the ends of the type's range or beyond it: row i is of kind i % 12."""
+    import torch
+    x = torch.randn(tokens * heads, D, device="cuda", generator=gen)
+    i = torch.arange(tokens * heads, device="cuda")
+    for kind, nonzeros in ((0, 1), (1, 2), (2, 4), (3, 8)):
+        r = i[i % 12 == kind]
+        at = torch.rand(len(r), D, device="cuda", generator=gen).argsort(1)[:, :nonzeros]
+        sign = torch.randint(0, 2, at.shape, device="cuda", generator=gen) * 2.0 - 1.0
+        x[r] = torch.zeros(len(r), D, device="cuda").scatter_(1, at, sign)
+    r = i[i % 12 == 4]                                        # two equal neighbours
+    at = torch.randint(0, D - 1, (len(r), 1), device="cuda", generator=gen)
+    x[r] = torch.zeros(len(r), D, device="cuda").scatter_(1, torch.cat([at, at + 1], 1), 3.0)
+    r = i[i % 12 == 5]
+    x[r] = torch.randint(-7, 8, (len(r), D), device="cuda", generator=gen).float()
+    r = i[i % 12 == 6]                                        # zeros of both signs
+    x[r] = torch.where(torch.rand(len(r), D, device="cuda", generator=gen) < 0.9, torch.zeros_like(x[r]).copysign(x[r]), x[r].sign())
+    x[i[i % 12 == 7], 3:7] *= 1000
+    r = i[i % 12 == 8]                                        # channels of very different sizes
+    x[r] *= torch.exp2(torch.randint(-8, 9, (len(r), D), device="cuda", generator=gen).float())
+    big, small = (6e4, 6e-8) if dtype == "float16" else (3e38, 1e-38)
+    r = i[i % 12 == 9]
+    x[r] = torch.where((r % 2 == 0)[:, None], x[r].sign() * big, x[r] * small)
+    r = i[i % 12 == 10]
+    x[r, r % D] = torch.tensor([float("nan"), float("inf"), float("-inf")], device="cuda")[r % 36 // 12]
+    return x.view(tokens, heads, D).to(getattr(torch, dtype))
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("norm_correction", [True, False])
+@pytest.mark.parametrize("heads", [1, 3, 8])
+@pytest.mark.parametrize("fmt", ["turbo2", "turbo3", "turbo4"])
+def test_odd_rows_of_long_appends(fmt, heads, norm_correction, dtype):
+    import torch
+    import turboquant_plus_b200 as tq
+    vectors = 166 * torch.cuda.get_device_properties(0).multi_processor_count       # the shortest append of the tile kernel
+    tokens = -(-vectors // heads) + 5
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    rows = [_odd_rows(tokens, heads, dtype, gen) for _ in range(2)]
+    n_pages = -(-tokens // 128)
+    slots = torch.arange(tokens, device="cuda")
+    got = []
+    for piece in (tokens, 1000):
+        cache = tq.PagedKVCache(D, heads, n_pages, 128, fmt, fmt, seed=42, norm_correction=norm_correction)
+        cache.pool.zero_()
+        for lo in range(0, tokens, piece):
+            cache.append(rows[0][lo:lo + piece], rows[1][lo:lo + piece], slots[lo:lo + piece])
+        got.append(_fields(cache))
+    a, b = got
+    for t in ("k", "v"):
+        assert torch.equal(a[t], b[t])
+        sa, sb = a[t + "_scale"], b[t + "_scale"]
+        assert bool((((sa - sb).abs() <= 6 * 2.0 ** -24 * sb.abs()) | (sa == sb) | (sa.isnan() & sb.isnan())).all())

@@ -12,7 +12,9 @@
 //   * One CTA per SM: a warp issues the tiled copies of the rows (a ring of operand tiles), a warp the MMAs (a ring of
 //     accumulators in tensor memory), and four groups of four warps take the accumulators in turn: 96 registers a thread, one
 //     piece of 32 columns at a time.  Three groups with 128 are a sixth slower; loads and MMAs issued by the groups themselves a half.
-//   * the operand holds minus the transform: the sign bit of a sum alone decides the centre boundary (a zero is not above it).
+//   * the last stage of the 8-point transform gives minus the value, (-a) - b and b - a, as in the warp-level kernel: the sign bit
+//     of a sum alone decides the centre boundary.  A zero by cancellation is not above it; one from two zeros comes out as -0 and
+//     takes the upper central index -- in both kernels, so that a record does not depend on its append's length.
 //   * thresholds are scaled by the vector's norm; a magnitude level is found bit by bit, the threshold of the next bit picked
 //     arithmetically; eight indices are an exact fp32 Horner sum; sign2 mirrors an index, an XOR of the packed words; level
 //     counts, exact small integers, give the norm correction.
@@ -262,10 +264,10 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   {
-    // minus H16 D1 of block i as +-1, 16-byte chunk c of it: outputs 8 (c >> 4) + (c & 7), inputs 8 ((c >> 3) & 1) ..
+    // H16 D1 of block i as +-1, 16-byte chunk c of it: outputs 8 (c >> 4) + (c & 7), inputs 8 ((c >> 3) & 1) ..
     if (tid < 256) {
       const int i = tid >> 5, c = tid & 31, out = 8 * (c >> 4) + (c & 7), k8 = (c >> 3) & 1, e = 16 * i + 8 * k8;
-      uint32_t m = 0xffu ^ qt_had8(out & 7) ^ ((f.s1[e >> 5] >> (e & 31)) & 0xffu);
+      uint32_t m = qt_had8(out & 7) ^ ((f.s1[e >> 5] >> (e & 31)) & 0xffu);
       if ((out >> 3) & k8) m ^= 0xffu;
       uint32_t w[4];
 #pragma unroll
@@ -360,7 +362,9 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
             for (int c = 0; c < 8; c += 2) {
               const float2 a = make_float2(__uint_as_float(u[i16][c]), __uint_as_float(u[i16][c + 1]));
               const float2 b = make_float2(__uint_as_float(u[i16 + h][c]), __uint_as_float(u[i16 + h][c + 1]));
-              const float2 sum = qm_add2(a, b), dif = qm_sub2(a, b);
+              // (the last stage costs no more: the negation is part of the subtraction)
+              const float2 sum = h < 4 ? qm_add2(a, b) : qm_sub2(make_float2(-a.x, -a.y), b);
+              const float2 dif = h < 4 ? qm_sub2(a, b) : qm_sub2(b, a);
               u[i16][c] = __float_as_uint(sum.x);
               u[i16][c + 1] = __float_as_uint(sum.y);
               u[i16 + h][c] = __float_as_uint(dif.x);
