@@ -1,6 +1,6 @@
 """Dense-mode calls of many vectors (integer products of base-256 digits) against the same vectors in small calls (fp64 products):
 edges of the 128-vector tiles, both row types, all widths, rows that are zero, tiny, huge or not finite, matrices that are not
-rotations.  Both paths are within 7e-16 of exact sums, so indices and signs are equal except within 1e-14 of a boundary, which
+rotations (uneven ones stay with the fp64 products).  Both paths are within 7e-16 of exact sums, so indices and signs are equal except within 1e-14 of a boundary, which
 these inputs do not meet; reconstructions agree to 256 roundings of 2^-53 of the largest one of their row (sums of 256 terms)."""
 import numpy as np
 import pytest
@@ -40,7 +40,7 @@ def _rows(n, dtype, special):
 
 @pytest.mark.parametrize("dtype", ["float32", "float16"])
 @pytest.mark.parametrize("n,bits,special", [(9473, 2, False), (9600, 3, True), (9601, 4, False), (18944, 3, False), (19073, 2, True), (40000, 4, True)])
-@pytest.mark.parametrize("matrix", ["rotation", "arbitrary"])
+@pytest.mark.parametrize("matrix", ["rotation", "arbitrary", "long"])
 def test_many_vectors_equal_few(n, bits, special, dtype, matrix):
     import torch
     import turboquant_plus_b200 as tq
@@ -51,6 +51,9 @@ def test_many_vectors_equal_few(n, bits, special, dtype, matrix):
         rng = np.random.default_rng(n)
         q.polar_quant.rotation = rng.standard_normal((D, D)) * np.exp(rng.standard_normal((D, D)))
         m.polar_quant.rotation = np.diag(np.exp2(rng.integers(-20, 20, D).astype(float)))
+    if matrix == "long":                        # the same from matrices whose entries are of one size, which have digits
+        rng = np.random.default_rng(n)
+        q.polar_quant.rotation, m.polar_quant.rotation = 3 * rng.standard_normal((D, D)), rng.standard_normal((D, D))
 
     def quantize(v):
         c = q.quantize(v)
@@ -61,7 +64,7 @@ def test_many_vectors_equal_few(n, bits, special, dtype, matrix):
     finite = torch.isfinite(parts[3])
     assert torch.equal(torch.isfinite(whole[3]), finite)
     assert bool(((whole[3] - parts[3]).abs() <= 1.2e-7 * parts[3])[finite].all())          # fp32 results of sums that agree
-    if matrix == "rotation":                    # (arbitrary: projections of any size beside others, signs within rounding of zero)
+    if matrix == "rotation":                    # (otherwise: projections of any size beside others, signs within rounding of zero)
         assert torch.equal(whole[2], parts[2])
     else:
         assert float((whole[2] != parts[2]).float().mean()) < 1e-6
@@ -80,3 +83,58 @@ def test_many_vectors_equal_few(n, bits, special, dtype, matrix):
                                                   for f in code.__dataclass_fields__})) for lo in range(0, n, PIECE)])
     assert close(back, parts)
     assert close(m.dequantize(idx, norms), torch.cat([m.dequantize(idx[lo:lo + PIECE], norms[lo:lo + PIECE]) for lo in range(0, n, PIECE)]))
+
+
+def _uneven(kind, rng):
+    """(rotation or None, S or None, centroids or None) that fixed-point digits of one scale do not carry to 53 bits."""
+    r = np.linalg.qr(rng.standard_normal((D, D)))[0]
+    s = rng.standard_normal((D, D))
+    sizes = np.exp(rng.uniform(-40, 0, D))
+    if kind == "rotation rows":
+        return r * sizes[:, None], None, None
+    if kind == "rotation columns":
+        return r * sizes, None, None
+    if kind == "sketch rows":
+        return None, s * sizes[:, None], None
+    if kind == "blocks":                        # outputs that see some of the elements only
+        b = np.zeros((D, D))
+        for lo in range(0, D, 16):
+            b[lo:lo + 16, lo:lo + 16] = np.linalg.qr(rng.standard_normal((16, 16)))[0]
+        return b, None, None
+    return None, None, np.array([-1.0, -3e-9, 1e-9, 1.0])       # centroids
+
+
+@pytest.mark.parametrize("kind", ["rotation rows", "rotation columns", "sketch rows", "blocks", "centroids"])
+def test_uneven_constants(kind):
+    """Matrices and codebooks whose entries differ much in size: many vectors as few, error held for every column, or row, by
+    its own size (sums of 256 terms, as above)."""
+    import torch
+    import turboquant_plus_b200 as tq
+    n = 9601
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, D, device="cuda", generator=gen)
+    if kind == "blocks":
+        x[:, 16:] *= 1e-20
+    q = tq.TurboQuant(D, 3, seed=5)
+    rot, s, cent = _uneven(kind, np.random.default_rng(n))
+    if rot is not None:
+        q.polar_quant.rotation = rot
+    if s is not None:
+        q.qjl.S = s
+    if cent is not None:
+        q.polar_quant.centroids = cent
+
+    def quantize(v):
+        c = q.quantize(v)
+        return c.mse_indices, c.vector_norms, c.qjl_signs, c.residual_norms
+
+    whole, parts = quantize(x), _pieces(quantize, x)
+    assert torch.equal(whole[0], parts[0]) and torch.equal(whole[1], parts[1]) and torch.equal(whole[2], parts[2])
+    pq = q.polar_quant
+    idx, norms = whole[0], whole[1]
+    if kind == "centroids":
+        idx = 1 + (idx & 1)                     # the small ones only
+    back = pq.dequantize(idx, norms)
+    few = torch.cat([pq.dequantize(idx[lo:lo + PIECE], norms[lo:lo + PIECE]) for lo in range(0, n, PIECE)])
+    size = few.abs().amax(dim=1 if kind == "centroids" else 0, keepdim=True)
+    assert bool(((back - few).abs() <= 256 * 2.0 ** -53 * size).all())

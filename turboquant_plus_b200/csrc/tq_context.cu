@@ -244,12 +244,8 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
     tq_quantizer_destroy(q);
     return tq_cuda_fail(e, "digits of the dense matrices");
   }
-  {
-    const double most = fabs(c.front()) > fabs(c.back()) ? fabs(c.front()) : fabs(c.back());   // (strictly increasing)
-    int exponent = 0;
-    if (most > 1e-100 && most < 1e100) frexp(most, &exponent), q->dig.cent_scale = ldexp(1.0, exponent);
-    for (size_t i = 0; i < b.size(); ++i) q->dig.bnd[i] = b[i];
-  }
+  q->dig.cent_scale = tq_dense_digits_centroids(c.data(), nc);
+  for (size_t i = 0; i < b.size(); ++i) q->dig.bnd[i] = b[i];
   q->cent64 = f64(cent_at);
   q->bnd64 = f64(bnd_at);
   *out = q;

@@ -760,18 +760,40 @@ template <typename Tout> int di_dequantize(const DiDequant& A, int64_t n, void* 
 
 }  // namespace
 
-// The power of two that a matrix's digits are relative to, or 0 for a matrix that has no such form (a value that is not finite, all
-// zeros, far out of the ordinary range)
+// The power of two that a matrix's digits are relative to, or 0 for a matrix that stays with the fp64 kernels.
+// The digits are fixed-point numbers of 2^-54 of the largest entry, where fp64 keeps every entry's own exponent.  No product may lose
+// by that, so: every row and column is at least sqrt(2) times as long as the largest entry (the rounding of a row's digits is then
+// 2^-55 of that row's length, below that of fp64 sums), and no entry is below 2^-30 of it (a row of x enters with 2^-54 of its length;
+// an entry of zero would hide its large elements, and what an output then sees may be smaller than that).  Random rotations
+// and Gaussian matrices are of this kind (their rows are three times and twice as long); uneven, diagonal or block matrices and what
+// is not finite are not.
 double tq_dense_digits_scale(const double* m) {
-  double most = 0.0;
-  for (int i = 0; i < TQ_D * TQ_D; ++i) {
-    const double a = fabs(m[i]);
-    if (!(a < 1e200)) return 0.0;
-    most = a > most ? a : most;
-  }
-  if (!(most > 1e-200)) return 0.0;
+  double most = 0.0, least = 1e300, row[TQ_D] = {}, col[TQ_D] = {};
+  for (int i = 0; i < TQ_D; ++i)
+    for (int j = 0; j < TQ_D; ++j) {
+      const double a = fabs(m[i * TQ_D + j]);
+      most = a > most ? a : most;
+      least = a < least ? a : least;
+      row[i] += a * a;
+      col[j] += a * a;
+    }
+  if (!(most > 1e-100 && most < 1e100 && least >= most * 0x1p-30)) return 0.0;
+  for (int i = 0; i < TQ_D; ++i)
+    if (!(row[i] >= 2.0 * most * most && col[i] >= 2.0 * most * most)) return 0.0;   // (also what is not a number)
   int e = 0;
   frexp(most, &e);   // most < 2^e
+  return ldexp(1.0, e);
+}
+// A power of two above every centroid's magnitude, or 0 for a codebook whose centroids differ much in size: those of a row
+// may all be small ones, whose digits would be short.  (Codebooks of one to four bits span a factor of 21 at most.)
+double tq_dense_digits_centroids(const double* c, int n) {
+  double most = 0.0;
+  for (int i = 0; i < n; ++i) most = fabs(c[i]) > most ? fabs(c[i]) : most;
+  if (!(most > 1e-100 && most < 1e100)) return 0.0;
+  for (int i = 0; i < n; ++i)
+    if (c[i] != 0.0 && !(fabs(c[i]) >= most / 64.0)) return 0.0;
+  int e = 0;
+  frexp(most, &e);
   return ldexp(1.0, e);
 }
 cudaError_t tq_dense_digits(const double* m_dev, double scale, uint8_t* out_dev) {

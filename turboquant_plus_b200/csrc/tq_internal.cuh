@@ -37,6 +37,7 @@ struct TqDenseDigits {
 };
 #define TQ_DENSE_DIGITS_BYTES (7 * TQ_D * TQ_D)
 double tq_dense_digits_scale(const double* m);
+double tq_dense_digits_centroids(const double* c, int n);
 cudaError_t tq_dense_digits(const double* m_dev, double scale, uint8_t* out_dev);   // on the legacy stream
 
 struct tq_quantizer {
