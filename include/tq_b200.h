@@ -103,6 +103,20 @@ int tq_quantizer_destroy(tq_quantizer* q);
 int tq_quantize(const tq_quantizer* q, const void* x_dev, int32_t x_dtype, int64_t ld, int64_t n,
                 uint8_t* out_packed_dev, uint8_t* out_idx_dev, float* out_norm_dev,
                 float* out_scale_dev, uint8_t* out_qjl_dev, float* out_rnorm_dev, void* stream);
+/* After a synchronisation: 0 if every tq_quantize / tq_dequantize / tq_cache_append of the current device since the previous
+ * read finished cleanly, 1 if a bounded wait inside one of their kernels gave up (new surface; the reference has no device
+ * code).  What such a call did not compute says so itself: norms, factors (in a cache, the records' scales) and
+ * reconstructions are not numbers.  Synchronous (a few bytes are copied); reading clears it. */
+int tq_quantize_status_sync(int32_t* status_out);
+/* Self-tests of that: a quantize or dequantize call whose kernel never reports one product of its first CTA's second tile as
+ * done, with waits of 2^20 SM clocks (half a millisecond) instead of 2^30.  The kernels end normally, the context stays
+ * usable.  Quantize: fp16 rows of a 3-bit WHT-mode quantizer with norm correction, or fp32 rows of a dense-mode
+ * one of d = 128, 2 bits and a sketch; outputs as tq_quantize's (codes packed, or one a byte).  Dequantize: the latter's. */
+int tq_selftest_quantize_gives_up(const tq_quantizer* q, const void* x_dev, int64_t ld, int64_t n, uint8_t* out_codes_dev,
+                                  float* out_norm_dev, float* out_scale_dev, uint8_t* out_qjl_dev, float* out_rnorm_dev, void* stream);
+int tq_selftest_dequantize_gives_up(const tq_quantizer* q, const uint8_t* idx_dev, const float* norm_dev, const uint8_t* qjl_dev,
+                                    const float* rnorm_dev, int64_t n, double* out_dev, void* stream);
+
 
 /* ------------------------------------------------------------------------------------------
  * tq_dequantize: PolarQuant.dequantize (turboquant/polar_quant.py:87-119) plus, when qjl_dev is

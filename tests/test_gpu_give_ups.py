@@ -1,0 +1,90 @@
+"""Bounded waits of the tensor-core quantize and dequantize kernels that run out: a call whose first CTA never reports one product of
+its second tile as done.  What it did compute is right, the rest is marked as not a number, the status word says so once, and
+the same calls then run as before."""
+import ctypes
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+D, TILE = 128, 128
+
+
+def _status(nv):
+    import torch
+    torch.cuda.synchronize()
+    word = ctypes.c_int32()
+    nv.call("tq_quantize_status_sync", ctypes.byref(word))
+    return word.value
+
+
+def _first_cta(n, sms):
+    """Tile of every vector, counted within its CTA, where that is the first one; else -1."""
+    import torch
+    tile = torch.arange(n, device="cuda") // TILE
+    return torch.where(tile % sms == 0, tile // sms, -1)
+
+
+def _check(seen, right, at):
+    """Rows of the outputs in `seen`, the first of which marks what was given up: tile 0 and other CTAs are right, tile 1 is not there."""
+    import torch
+    lost = seen[0].reshape(len(at), -1).isnan().any(1)
+    assert bool(lost[at == 1].all()) and not bool(lost[at <= 0].any())
+    for a, b in zip(seen, right):
+        a, b = a.reshape(len(at), -1), b.reshape(len(at), -1)
+        assert torch.equal(a[~lost], b[~lost])
+        assert not a.is_floating_point() or bool(a[lost].isnan().all())
+
+
+def test_long_append_gives_up():
+    import torch
+    import turboquant_plus_b200 as tq
+    from turboquant_plus_b200 import _native as nv
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = TILE * 15 * sms + 37                                  # 15 or 16 tiles a CTA: more than the rings hold
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, D, device="cuda", generator=gen).half()
+    q = tq.PolarQuant(D, 3, seed=1, rotation="wht")
+    right = q.quantize_device(x, packed=True, want_scale=True)
+    right = right["norm"], right["scale"], right["packed"]
+    assert _status(nv) == 0
+    seen = torch.zeros_like(right[0]), torch.zeros_like(right[1]), torch.zeros_like(right[2])
+    nv.call("tq_selftest_quantize_gives_up", q._native(x.device).handle, nv.ptr(x), D, n, nv.ptr(seen[2]), nv.ptr(seen[0]),
+            nv.ptr(seen[1]), None, None, nv.stream_ptr())
+    assert _status(nv) == 1 and _status(nv) == 0
+    _check(seen, right, _first_cta(n, sms))
+    again = q.quantize_device(x, packed=True, want_scale=True)
+    assert torch.equal(again["packed"], right[2]) and torch.equal(again["scale"], right[1]) and _status(nv) == 0
+
+
+def test_dense_calls_give_up():
+    import torch
+    import turboquant_plus_b200 as tq
+    from turboquant_plus_b200 import _native as nv
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = TILE * 3 * sms + 37
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, D, device="cuda", generator=gen)
+    q = tq.TurboQuant(D, 3, seed=1)
+    out = q.quantize_device(x)
+    right = out["norm"], out["rnorm"], out["idx"], out["qjl"]
+    seen = tuple(torch.zeros_like(t) for t in right)
+    handle, at = q._native(x.device).handle, _first_cta(n, sms)
+    nv.call("tq_selftest_quantize_gives_up", handle, nv.ptr(x), D, n, nv.ptr(seen[2]), nv.ptr(seen[0]), None, nv.ptr(seen[3]),
+            nv.ptr(seen[1]), nv.stream_ptr())
+    assert _status(nv) == 1 and _status(nv) == 0
+    _check(seen, right, at)
+
+    def back():
+        y = torch.empty(n, D, device="cuda", dtype=torch.float64)
+        nv.call("tq_dequantize", handle, None, nv.ptr(right[2]), nv.ptr(right[0]), nv.ptr(right[3]), nv.ptr(right[1]), 1.0, n, nv.ptr(y),
+                nv.F64, nv.stream_ptr())
+        return y
+
+    y, lost = back(), torch.zeros(n, D, device="cuda", dtype=torch.float64)
+    nv.call("tq_selftest_dequantize_gives_up", handle, nv.ptr(right[2]), nv.ptr(right[0]), nv.ptr(right[3]), nv.ptr(right[1]), n,
+            nv.ptr(lost), nv.stream_ptr())
+    assert _status(nv) == 1 and _status(nv) == 0
+    _check((lost,), (y,), at)
+    assert bool(lost[at >= 1].isnan().all())
+    again = q.quantize_device(x)
+    assert torch.equal(again["idx"], right[2]) and torch.equal(again["qjl"], right[3]) and torch.equal(back(), y) and _status(nv) == 0

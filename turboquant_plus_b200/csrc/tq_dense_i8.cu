@@ -23,11 +23,16 @@
 // MMAs, 120 without) and their fp64 additions, eight of each of 128 x 128 sums, run between the MMAs rather than under them.
 // 65,536 fp32 vectors, before (fp64 tensor cores) / now: quantize 134 / 77 us, with the sketch 302 / 182, dequantize 90 / 63 and 164 / 93.
 //
+// A wait that gives up ends the waits of all roles; the results of its tile and of those behind it are then not numbers, and a
+// status word is set (tq_quantize_status_sync).
+//
 // A row that this arithmetic does not carry -- values that are not finite or too small for a norm, residuals far beyond the
 // vector's length, which an arbitrary matrix can produce -- is computed by one warp in plain fp64.
 #include "tq_tcgen05.cuh"
 
 namespace {
+
+__device__ int32_t di_status;   // 1: a wait gave up
 
 constexpr int DI_DIGITS = 7, DI_SUMS = 8;
 constexpr int DI_ROWS = 128, DI_ROW_THREADS = 512, DI_COPIER = 16, DI_MMA = 17, DI_THREADS = 576;
@@ -119,17 +124,13 @@ __device__ __forceinline__ double di_double(uint32_t v) { return __hiloint2doubl
 
 // Barriers and the way of the roles through them; the row warps and the MMA warp count alike.
 struct DiShared {
-  uint64_t b_full[DI_DIGITS], b_free[DI_DIGITS], d_full[2], d_free[2], a_ready;
+  uint64_t b_full[DI_DIGITS], b_free[DI_DIGITS], d_full[2], d_free[2], a_ready, drained;
   uint32_t tmem;
   volatile int failed;   // a wait gave up: nobody waits any more
 };
-__device__ __forceinline__ void di_wait(DiShared& s, uint64_t* bar, uint32_t parity) {
-  if (tc_try_wait(bar, parity)) return;
-  const long long t0 = clock64();
-  while (!s.failed) {
-    if (tc_try_wait(bar, parity)) return;
-    if (clock64() - t0 > TC_WAIT_CYCLES) s.failed = 1;
-  }
+// SELFTEST: waits are short, and one accumulator of the first CTA's second tile is never reported as full (di_issue)
+template <bool SELFTEST> __device__ __forceinline__ void di_wait(DiShared& s, uint64_t* bar, uint32_t parity) {
+  tc_wait(bar, parity, &s.failed, SELFTEST ? TC_SELFTEST_CYCLES : TC_WAIT_CYCLES);
 }
 __device__ __forceinline__ void di_init(DiShared& s) {
   auto init = [](uint64_t* bar, int count) {
@@ -138,6 +139,7 @@ __device__ __forceinline__ void di_init(DiShared& s) {
   for (int i = 0; i < DI_DIGITS; ++i) init(&s.b_full[i], 1), init(&s.b_free[i], 1);
   for (int i = 0; i < 2; ++i) init(&s.d_full[i], 1), init(&s.d_free[i], DI_ROW_THREADS / 32);
   init(&s.a_ready, DI_ROW_THREADS / 32);
+  init(&s.drained, 1);
   s.failed = 0;
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -153,34 +155,36 @@ __device__ __forceinline__ bool di_rows_any(bool p) {
 }
 
 // The copier's way: the digits of the matrices that `matrix(i)` gives, each into the place of the matrix before
-template <typename M> __device__ __forceinline__ void di_copier(DiShared& s, uint8_t* tiles, int count, M&& matrix) {
-  int i = 0;
-  for (; i < count && !s.failed; ++i) {
+template <bool SELFTEST, typename M> __device__ __forceinline__ void di_copier(DiShared& s, uint8_t* tiles, int count, M&& matrix) {
+  int copies = 0;
+  for (int i = 0; i < count && !s.failed; ++i) {
     const uint8_t* src = matrix(i);
-    for (int p = DI_DIGITS - 1; p >= 0; --p) {
-      if (i > 0) di_wait(s, &s.b_free[p], (uint32_t)((i - 1) & 1));
+    for (int p = DI_DIGITS - 1; p >= 0; --p, ++copies) {
+      if (i > 0) di_wait<SELFTEST>(s, &s.b_free[p], (uint32_t)((i - 1) & 1));
       if (s.failed) break;
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(&s.b_full[p])), "r"(DI_TILE) : "memory");
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sptr(tiles + p * DI_TILE)),
                    "l"(src + p * DI_TILE), "r"(DI_TILE), "r"(sptr(&s.b_full[p])) : "memory");
     }
   }
-  if (i > 0)   // none in flight at the end
-    for (int p = 0; p < DI_DIGITS; ++p) di_wait(s, &s.b_full[p], (uint32_t)((i - 1) & 1));
+  for (int p = 0; p < DI_DIGITS; ++p) {   // none in flight at the end, also after a wait that gave up
+    const int mine = (copies + p) / DI_DIGITS;
+    if (mine > 0) tc_wait(&s.b_full[p], (uint32_t)((mine - 1) & 1));
+  }
 }
 
 // The MMA warp: the operand at `area`, of DIGITS digits, against the `matrix`-th matrix; s from the last to the first
-template <int DIGITS>
+template <int DIGITS, bool SELFTEST>
 __device__ __forceinline__ void di_issue(DiShared& s, int& item, const uint8_t* tiles, int matrix, uint32_t area, uint32_t acc_base) {
   constexpr int TOP = DI_DIGITS - 1, LAST = DIGITS == 1 ? TOP : DI_SUMS - 1;
   const uint32_t b = sptr(tiles), idesc = di_idesc();
 #pragma unroll
   for (int sum = LAST; sum >= 0; --sum, ++item) {
     const int sl = item & 1;
-    if (item >= 2) di_wait(s, &s.d_free[sl], (uint32_t)((item / 2 - 1) & 1));
+    if (item >= 2) di_wait<SELFTEST>(s, &s.d_free[sl], (uint32_t)((item / 2 - 1) & 1));
 #pragma unroll
     for (int q = 0; q < DI_DIGITS; ++q)   // digits used for the first time
-      if (DIGITS == 1 ? q == sum : sum == LAST ? q > 0 : sum == LAST - 1 && q == 0) di_wait(s, &s.b_full[q], (uint32_t)(matrix & 1));
+      if (DIGITS == 1 ? q == sum : sum == LAST ? q > 0 : sum == LAST - 1 && q == 0) di_wait<SELFTEST>(s, &s.b_full[q], (uint32_t)(matrix & 1));
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -192,13 +196,21 @@ __device__ __forceinline__ void di_issue(DiShared& s, int& item, const uint8_t* 
         di_mma(acc_base + 128 * sl, area + 32 * p + 8 * ks, umma_desc(b + q * DI_TILE + ks * 256, 128, 1024), idesc,
                p == (sum > TOP ? sum - TOP : 0) && ks == 0 ? 0u : 1u);
     }
-    di_commit(&s.d_full[sl]);
+    if (!(SELFTEST && blockIdx.x == 0 && item == 26)) di_commit(&s.d_full[sl]);   // (a tile with a sketch: 24 items, 15 to dequantize)
     if (sum < DI_DIGITS) di_commit(&s.b_free[sum]);
   }
 }
 
+// ... and nothing of its in flight at the end, also after a wait that gave up (else the rows have waited for every product)
+__device__ __forceinline__ void di_drain(DiShared& s) {
+  if (!__any_sync(0xffffffffu, s.failed)) return;
+  __syncwarp();
+  di_commit(&s.drained);
+  tc_wait(&s.drained, 0);
+}
+
 // A row warp: acc += base x (the product's sums, 256^-s each), 32 columns of a thread
-template <int DIGITS>
+template <int DIGITS, bool SELFTEST>
 __device__ __forceinline__ void di_take(DiShared& s, int& item, uint32_t acc_base, int lane, double base, double (&acc)[DI_COLS]) {
   constexpr int LAST = DIGITS == 1 ? DI_DIGITS - 1 : DI_SUMS - 1;
   double factor = base;
@@ -207,7 +219,7 @@ __device__ __forceinline__ void di_take(DiShared& s, int& item, uint32_t acc_bas
 #pragma unroll 1
   for (int sum = LAST; sum >= 0; --sum, ++item, factor *= 256.0) {
     const int sl = item & 1;
-    di_wait(s, &s.d_full[sl], (uint32_t)((item / 2) & 1));
+    di_wait<SELFTEST>(s, &s.d_full[sl], (uint32_t)((item / 2) & 1));
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t v[2][8];
@@ -321,11 +333,33 @@ __device__ void di_row_plain(const TqDenseQuant& a, const uint8_t* xrow, float n
   if ((lane & 1) == 0) a.out_qjl[v * 16 + (lane >> 1)] = (uint8_t)((nib << 4) | up);
 }
 
+template <typename T> __device__ __forceinline__ T di_from(double v) { return (T)v; }
+template <> __device__ __forceinline__ __half di_from<__half>(double v) { return __float2half_rn((float)v); }
+// A wait gave up: the results of this CTA's tiles from `t` on are not to come.  (Functions of their own: inlined, they cost the kernels registers.)
+__device__ __noinline__ void di_give_up(const TqDenseQuant& a, int t, int mine, int row, int64_t n) {
+  const float nan = __int_as_float(0x7fffffff);
+  for (; t < mine; ++t) {
+    const int64_t v = (blockIdx.x + (int64_t)t * gridDim.x) * DI_ROWS + row;
+    if (row < 0 || v >= n) continue;
+    if (a.out_norm) a.out_norm[v] = nan;
+    if (a.out_scale) a.out_scale[v] = nan;
+    if (a.out_rnorm) a.out_rnorm[v] = nan;
+  }
+  di_status = 1;
+}
+template <typename Tout> __device__ __noinline__ void di_give_up(const TqDenseDequant& a, int t, int mine, int row, int col, int64_t n, Tout* out) {
+  for (; t < mine; ++t) {
+    const int64_t v = (blockIdx.x + (int64_t)t * gridDim.x) * DI_ROWS + row;
+    for (int k = 0; k < DI_COLS && v < n; ++k) out[v * a.ld_out + col + k] = di_from<Tout>(__longlong_as_double(0x7ff8000000000000ll));
+  }
+  di_status = 1;
+}
+
 template <typename Tin> constexpr int di_row_bytes() { return TQ_D * (int)sizeof(Tin) + 16; }   // (rows 4 banks apart: no conflicts)
 template <typename Tin> constexpr int di_quant_smem() { return DI_DIGITS * DI_TILE + DI_ROWS * di_row_bytes<Tin>() + 128; }
 
 // PROD: residual, its norm and the sketch as well
-template <typename Tin, int BITS, bool PROD>
+template <typename Tin, int BITS, bool PROD, bool SELFTEST = false>
 __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __grid_constant__ DiQuant A, const Tin* __restrict__ x, int64_t ld,
                                                                      int64_t n) {
   constexpr int ROWB = di_row_bytes<Tin>();
@@ -358,13 +392,14 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
   constexpr int PHASES = PROD ? 3 : 1;
 
   if (warp == DI_COPIER) {
-    if (lane == 0) di_copier(sh, tiles_b, mine * PHASES, [&](int i) { return !PROD || i % 3 == 0 ? A.r : i % 3 == 1 ? A.rt : A.s; });
+    if (lane == 0) di_copier<SELFTEST>(sh, tiles_b, mine * PHASES, [&](int i) { return !PROD || i % 3 == 0 ? A.r : i % 3 == 1 ? A.rt : A.s; });
   } else if (warp == DI_MMA) {
     int item = 0;
     for (int i = 0; i < mine * PHASES && !__any_sync(0xffffffffu, sh.failed); ++i) {
-      di_wait(sh, &sh.a_ready, (uint32_t)(i & 1));
-      di_issue<DI_DIGITS>(sh, item, tiles_b, i, tb, tb + DI_ACC);
+      di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(i & 1));
+      di_issue<DI_DIGITS, SELFTEST>(sh, item, tiles_b, i, tb, tb + DI_ACC);
     }
+    di_drain(sh);
   } else {
     const int row = 32 * (warp & 3) + lane, h = warp >> 2;       // this thread's vector, and its columns 32 h .. + 31
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
@@ -388,12 +423,12 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int item = 0;
+    int item = 0, t = 0;
     if (mine > 0) load_tile(blockIdx.x);
-    for (int t = 0; t < mine; ++t) {
+    for (; t < mine; ++t) {
       const int64_t v0 = (blockIdx.x + t * step) * DI_ROWS, v = v0 + row;
       asm volatile("cp.async.wait_group 0;" ::: "memory");
-      if (di_rows_any(sh.failed)) break;
+      if (di_rows_any(sh.failed)) break;   // (in the tile before)
       // norms in the rows' own precision and NumPy's order (first term + pairwise sum of the rest), eight lanes a vector, two
       // vectors of a lane at once
       {
@@ -464,7 +499,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       // ---- y = R w: indices, ||c[idx]||^2, the centroids as the next operand ----
       double acc[DI_COLS], cc[4] = {0.0, 0.0, 0.0, 0.0};
       di_zero(acc);
-      di_take<DI_DIGITS>(sh, item, myacc, lane, A.r_scale, acc);
+      di_take<DI_DIGITS, SELFTEST>(sh, item, myacc, lane, A.r_scale, acc);
       uint32_t packed[DI_COLS / 4];
 #pragma unroll
       for (int g = 0; g < DI_COLS / 4; ++g) {
@@ -498,7 +533,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       double cn = sqrt((s_part[0][row] + s_part[1][row]) + (s_part[2][row] + s_part[3][row]));
       cn = cn > 1e-10 ? cn : 1.0;                                                 // turboquant/polar_quant.py:110-111
       if (h == 0 && live) {
-        if (a.out_norm) a.out_norm[v] = sh.failed ? __int_as_float(0x7fffffff) : nrm;
+        if (a.out_norm) a.out_norm[v] = nrm;
         if (a.out_scale) a.out_scale[v] = (float)(a.norm_correction ? (double)nrm / cn : (double)nrm);
       }
       if constexpr (PROD) {
@@ -507,7 +542,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
         const double unit = nrm > 0.f && nrm < 1e38f ? ldexp(1.0, -(ilogbf(nrm) + 2)) : 1.0;   // |residual| x unit < 1 for a rotation
         double rr[4] = {0.0, 0.0, 0.0, 0.0};
         di_zero(acc);
-        di_take<DI_DIGITS>(sh, item, myacc, lane, back, acc);
+        di_take<DI_DIGITS, SELFTEST>(sh, item, myacc, lane, back, acc);
         const uint8_t* xr = xs + row * ROWB + DI_COLS * h * sizeof(Tin);
 #pragma unroll
         for (int c = 0; c < DI_COLS / 8; ++c) {
@@ -534,7 +569,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
         if (t + 1 < mine) load_tile(blockIdx.x + (t + 1) * step);
         // ---- sketch: sign(S r), zero counts as +1 (turboquant/qjl.py:89-90), first column in the most significant bit ----
         di_zero(acc);
-        di_take<DI_DIGITS>(sh, item, myacc, lane, 1.0, acc);
+        di_take<DI_DIGITS, SELFTEST>(sh, item, myacc, lane, 1.0, acc);
         uint32_t m = 0;
 #pragma unroll
         for (int k = 0; k < DI_COLS; ++k) m = (m << 1) | (acc[k] < 0.0 ? 0u : 1u);
@@ -547,6 +582,9 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (di_rows_any(sh.failed)) {   // the last tile begun and those behind it
+      di_give_up(a, t > 0 ? t - 1 : 0, mine, h == 0 ? row : -1, n);
+    }
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -555,12 +593,10 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
 }
 
 constexpr int DI_IDX_ROW = TQ_D + 16, DI_OUT_ROW = 16 * 8 + 16;   // bytes between staged rows: 16 bytes on, no bank conflicts
-
-template <typename T> __device__ __forceinline__ T di_from(double v) { return (T)v; }
-template <> __device__ __forceinline__ __half di_from<__half>(double v) { return __float2half_rn((float)v); }
+constexpr int DI_DEQUANT_SMEM = DI_DIGITS * DI_TILE + DI_ROWS * DI_IDX_ROW + DI_ROW_THREADS * DI_OUT_ROW + 128;
 
 // x_hat = (norm / ||c[idx]||) R^T c[idx] + shrink sqrt(pi/2)/sqrt(d) rnorm S^T z.  The signs z are one digit, +-1: seven products.
-template <typename Tout, bool PROD>
+template <typename Tout, bool PROD, bool SELFTEST = false>
 __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __grid_constant__ DiDequant A, int64_t n, Tout* __restrict__ out) {
   extern __shared__ __align__(128) uint8_t di_raw[];
   __shared__ DiShared sh;
@@ -592,14 +628,15 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
   constexpr int PHASES = PROD ? 2 : 1;   // (the signs' product first)
 
   if (warp == DI_COPIER) {
-    if (lane == 0) di_copier(sh, tiles_b, mine * PHASES, [&](int i) { return PROD && (i & 1) == 0 ? A.st : A.rt; });
+    if (lane == 0) di_copier<SELFTEST>(sh, tiles_b, mine * PHASES, [&](int i) { return PROD && (i & 1) == 0 ? A.st : A.rt; });
   } else if (warp == DI_MMA) {
     int item = 0;
     for (int i = 0; i < mine && !__any_sync(0xffffffffu, sh.failed); ++i) {
-      di_wait(sh, &sh.a_ready, (uint32_t)(i & 1));
-      if constexpr (PROD) di_issue<1>(sh, item, tiles_b, 2 * i, tb + DI_SIGNS, tb + DI_ACC);
-      di_issue<DI_DIGITS>(sh, item, tiles_b, PROD ? 2 * i + 1 : i, tb, tb + DI_ACC);
+      di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(i & 1));
+      if constexpr (PROD) di_issue<1, SELFTEST>(sh, item, tiles_b, 2 * i, tb + DI_SIGNS, tb + DI_ACC);
+      di_issue<DI_DIGITS, SELFTEST>(sh, item, tiles_b, PROD ? 2 * i + 1 : i, tb, tb + DI_ACC);
     }
+    di_drain(sh);
   } else {
     const int row = 32 * (warp & 3) + lane, h = warp >> 2;
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
@@ -618,14 +655,14 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int item = 0;
+    int item = 0, t = 0;
     if (mine > 0) load_tile(blockIdx.x);
-    for (int t = 0; t < mine; ++t) {
+    for (; t < mine; ++t) {
       const int64_t v0 = (blockIdx.x + t * step) * DI_ROWS, v = v0 + row;
       const bool live = v < n;
       const float norm = live ? a.norm[v] : 0.f, rnorm = PROD && live ? a.rnorm[v] : 0.f;
       asm volatile("cp.async.wait_group 0;" ::: "memory");
-      if (di_rows_any(sh.failed)) break;
+      if (di_rows_any(sh.failed)) break;   // (in the tile before)
       // ---- digits of the centroids, ||c||^2, signs ----
       double cc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
@@ -668,9 +705,8 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
       }
       double acc[DI_COLS];
       di_zero(acc);
-      if constexpr (PROD) di_take<1>(sh, item, myacc, lane, g, acc);
-      di_take<DI_DIGITS>(sh, item, myacc, lane, f, acc);
-      if (sh.failed) acc[0] = __longlong_as_double(0x7ff8000000000000ll);   // a wait gave up: the result says so
+      if constexpr (PROD) di_take<1, SELFTEST>(sh, item, myacc, lane, g, acc);
+      di_take<DI_DIGITS, SELFTEST>(sh, item, myacc, lane, f, acc);
       Tout* o = out + v * a.ld_out + DI_COLS * h;
       if (a.accumulate && live) {
 #pragma unroll
@@ -708,6 +744,9 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (di_rows_any(sh.failed)) {   // the last tile begun and those behind it
+      di_give_up<Tout>(a, t > 0 ? t - 1 : 0, mine, row, DI_COLS * h, n, out);
+    }
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -753,9 +792,8 @@ template <typename Tin> int di_quantize(const DiQuant& A, const void* x, int64_t
 }
 template <typename Tout> int di_dequantize(const DiDequant& A, int64_t n, void* out, cudaStream_t st) {
   Tout* o = reinterpret_cast<Tout*>(out);
-  constexpr int smem = DI_DIGITS * DI_TILE + DI_ROWS * DI_IDX_ROW + DI_ROW_THREADS * DI_OUT_ROW + 128;
-  if (A.q.qjl) return di_launch<k_dense_dequantize_i8<Tout, true>>(smem, n, st, "k_dense_dequantize_i8", A, n, o);
-  return di_launch<k_dense_dequantize_i8<Tout, false>>(smem, n, st, "k_dense_dequantize_i8", A, n, o);
+  if (A.q.qjl) return di_launch<k_dense_dequantize_i8<Tout, true>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, o);
+  return di_launch<k_dense_dequantize_i8<Tout, false>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, o);
 }
 
 }  // namespace
@@ -807,36 +845,65 @@ cudaError_t tq_dense_digits(const double* m_dev, double scale, uint8_t* out_dev)
 // 6,000 29 / 31, 65,536 93 / 164.
 static bool di_enough(int64_t n, bool sketched_dequantize) { return n > (sketched_dequantize ? 32 : 64) * (int64_t)tq_num_sms(); }
 
-// false: not of these kernels' kind, nothing launched
-bool tq_dense_i8_quantize_try(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
-                              int* rc) {
+// The kernels' arguments; false: not of these kernels' kind
+static bool di_quant_args(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int32_t dtype, int64_t ld, DiQuant& A) {
   const bool prod = a.out_qjl || a.out_rnorm;
   if (a.d != TQ_D || g.r_scale == 0.0 || g.cent_scale == 0.0 || a.out_packed || a.out_res || (prod && g.s_scale == 0.0)) return false;
-  if ((dtype != TQ_F32 && dtype != TQ_F16) || !di_enough(n, false)) return false;
+  if (dtype != TQ_F32 && dtype != TQ_F16) return false;
   if (!tq_aligned(x, 16) || ld * (dtype == TQ_F32 ? 4 : 2) % 16 || !tq_aligned(a.out_idx, 16)) return false;
-  DiQuant A;
   A.r = g.r; A.rt = g.rt; A.s = g.s;
   A.r_scale = g.r_scale / 4096.0;
   A.cent_scale = g.cent_scale;
   for (int i = 0; i < 15; ++i) A.bnd[i] = g.bnd[i];
   A.q = a;
-  *rc = dtype == TQ_F32 ? di_quantize<float>(A, x, ld, n, st) : di_quantize<__half>(A, x, ld, n, st);
   return true;
 }
-
-bool tq_dense_i8_dequantize_try(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc) {
+static bool di_dequant_args(const TqDenseDequant& a, const TqDenseDigits& g, DiDequant& A) {
   if (a.d != TQ_D || g.r_scale == 0.0 || g.cent_scale == 0.0 || !a.idx || (a.qjl && g.s_scale == 0.0)) return false;
-  if (!tq_aligned(a.idx, 16) || !di_enough(n, a.qjl != nullptr)) return false;
-  DiDequant A;
+  if (!tq_aligned(a.idx, 16)) return false;
   A.rt = g.rt; A.st = g.st;
   A.r_scale = g.r_scale / 4096.0;
   A.s_scale = g.s_scale / 64.0;
   A.cent_scale = g.cent_scale;
   A.q = a;
+  return true;
+}
+
+// false: not of these kernels' kind, nothing launched
+bool tq_dense_i8_quantize_try(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
+                              int* rc) {
+  DiQuant A;
+  if (!di_enough(n, false) || !di_quant_args(a, g, x, dtype, ld, A)) return false;
+  *rc = dtype == TQ_F32 ? di_quantize<float>(A, x, ld, n, st) : di_quantize<__half>(A, x, ld, n, st);
+  return true;
+}
+
+bool tq_dense_i8_dequantize_try(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc) {
+  DiDequant A;
+  if (!di_enough(n, a.qjl != nullptr) || !di_dequant_args(a, g, A)) return false;
   switch (dtype) {
     case TQ_F64: *rc = di_dequantize<double>(A, n, out, st); return true;
     case TQ_F32: *rc = di_dequantize<float>(A, n, out, st); return true;
     case TQ_F16: *rc = di_dequantize<__half>(A, n, out, st); return true;
     default: return false;
   }
+}
+
+// The self-tests' forms: fp32 rows of 2 bits and a sketch; fp64 results with a sketch
+int tq_dense_i8_quantize_selftest(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int64_t ld, int64_t n, cudaStream_t st) {
+  DiQuant A;
+  TQ_REQUIRE(a.bits == 2 && a.out_qjl && di_quant_args(a, g, x, TQ_F32, ld, A), TQ_ERR_UNSUPPORTED,
+             "self-test of the dense quantizer: fp32 rows of 128 elements, 2 bits and a sketch");
+  return di_launch<k_dense_quantize_i8<float, 2, true, true>>(di_quant_smem<float>(), n, st, "k_dense_quantize_i8", A,
+                                                              reinterpret_cast<const float*>(x), ld, n);
+}
+int tq_dense_i8_dequantize_selftest(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, double* out, cudaStream_t st) {
+  DiDequant A;
+  TQ_REQUIRE(a.qjl && di_dequant_args(a, g, A), TQ_ERR_UNSUPPORTED, "self-test of the dense dequantizer: 128 elements and a sketch");
+  return di_launch<k_dense_dequantize_i8<double, true, true>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, out);
+}
+cudaError_t tq_dense_i8_status_sync(int32_t* out) {
+  void* word = nullptr;
+  const cudaError_t e = cudaGetSymbolAddress(&word, di_status);
+  return e == cudaSuccess ? tc_status_sync((int32_t*)word, out) : e;
 }

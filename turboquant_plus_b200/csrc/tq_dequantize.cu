@@ -214,15 +214,28 @@ __global__ void __launch_bounds__(128) k_dequantize_dense(const double* __restri
 }
 
 // d <= 256: the fp64 tensor cores (tq_dense.cu); wider vectors stay with k_dequantize_dense
-static bool dequantize_tensor(const tq_quantizer* q, const uint8_t* packed, const uint8_t* idx, const float* norm,
-                              const uint8_t* qjl, const float* rnorm, double shrink, int64_t n, void* out, int32_t dtype,
-                              int64_t ld_out, int32_t accumulate, cudaStream_t st, int* rc) {
+static TqDenseDequant dense_tensor_args(const tq_quantizer* q, const uint8_t* packed, const uint8_t* idx, const float* norm,
+                                        const uint8_t* qjl, const float* rnorm, double shrink, int64_t ld_out, int32_t accumulate) {
   TqDenseDequant t;
   t.rot_t = q->rotp_t; t.s_t = q->sp_t; t.cent = q->cent64;
   t.d = q->d; t.dp = (q->d + 7) / 8 * 8; t.bits = q->bits; t.norm_correction = q->norm_correction;
   t.packed = packed; t.idx = idx; t.norm = norm; t.qjl = qjl; t.rnorm = rnorm;
   t.shrink = shrink; t.ld_out = ld_out; t.accumulate = accumulate;
+  return t;
+}
+static bool dequantize_tensor(const tq_quantizer* q, const uint8_t* packed, const uint8_t* idx, const float* norm,
+                              const uint8_t* qjl, const float* rnorm, double shrink, int64_t n, void* out, int32_t dtype,
+                              int64_t ld_out, int32_t accumulate, cudaStream_t st, int* rc) {
+  const TqDenseDequant t = dense_tensor_args(q, packed, idx, norm, qjl, rnorm, shrink, ld_out, accumulate);
   return tq_dense_i8_dequantize_try(t, q->dig, n, out, dtype, st, rc) || tq_dense_dequantize_try(t, n, out, dtype, st, rc);
+}
+
+extern "C" int tq_selftest_dequantize_gives_up(const tq_quantizer* q, const uint8_t* idx_dev, const float* norm_dev, const uint8_t* qjl_dev,
+                                               const float* rnorm_dev, int64_t n, double* out_dev, void* stream) {
+  TQ_REQUIRE(q && q->rotation == TQ_ROT_DENSE && q->qjl && idx_dev && norm_dev && qjl_dev && rnorm_dev && out_dev && n > 0, TQ_ERR_INVALID,
+             "tq_selftest_dequantize_gives_up: bad arguments");
+  return tq_dense_i8_dequantize_selftest(dense_tensor_args(q, nullptr, idx_dev, norm_dev, qjl_dev, rnorm_dev, 1.0, q->d, 0), q->dig, n,
+                                         out_dev, (cudaStream_t)stream);
 }
 
 extern "C" int tq_dequantize(const tq_quantizer* q, const uint8_t* packed_dev, const uint8_t* idx_dev,

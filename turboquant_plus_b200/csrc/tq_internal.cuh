@@ -309,6 +309,12 @@ bool tq_dense_dequantize_try(const TqDenseDequant& a, int64_t n, void* out, int3
 bool tq_dense_i8_quantize_try(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
                               int* rc);
 bool tq_dense_i8_dequantize_try(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
+// Runs in which one wait runs out, and the words that say so (tq_selftest_quantize_gives_up, tq_quantize_status_sync)
+int tq_dense_i8_quantize_selftest(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int64_t ld, int64_t n, cudaStream_t st);
+int tq_dense_i8_dequantize_selftest(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, double* out, cudaStream_t st);
+int tq_quantize_tc_selftest(const TqFast& f, const void* x, const TqQuantDst& d, int64_t ld, int64_t n, cudaStream_t st);
+cudaError_t tq_dense_i8_status_sync(int32_t* out);
+cudaError_t tq_quantize_tc_status_sync(int32_t* out);
 
 // A chunk of queries per sequence as rows of the decode kernel, each with its causal length.  The workspace is one of
 // tq_decode_workspace_bytes(batch * queries, ...).

@@ -526,14 +526,20 @@ __global__ void __launch_bounds__(128) k_quantize_dense(const TqDenseArgs a, con
   }
 }
 
+static TqDenseQuant dense_tensor_args(const tq_quantizer* q) {
+  TqDenseQuant t;
+  memset(&t, 0, sizeof(t));
+  t.rot = q->rotp; t.rot_t = q->rotp_t; t.s = q->sp;
+  t.cent = q->cent64; t.bnd = q->bnd64;
+  t.d = q->d; t.dp = (q->d + 7) / 8 * 8; t.bits = q->bits; t.norm_correction = q->norm_correction;
+  return t;
+}
+
 static int launch_dense(const tq_quantizer* q, const void* x, int32_t dtype, int64_t ld, int64_t n, TqDenseArgs& a,
                         cudaStream_t st) {
   if (n == 0) return TQ_OK;
   {
-    TqDenseQuant t;
-    t.rot = q->rotp; t.rot_t = q->rotp_t; t.s = q->sp;
-    t.cent = a.cent; t.bnd = a.bnd;
-    t.d = q->d; t.dp = (q->d + 7) / 8 * 8; t.bits = a.bits; t.norm_correction = a.norm_correction;
+    TqDenseQuant t = dense_tensor_args(q);
     t.out_packed = a.out_packed; t.out_idx = a.out_idx;
     t.out_norm = a.out_norm; t.out_scale = a.out_scale; t.out_rnorm = a.out_rnorm;
     t.out_qjl = a.out_qjl; t.out_res = a.out_res; t.ld_res = a.ld_res;
@@ -607,6 +613,36 @@ extern "C" int tq_quantize(const tq_quantizer* q, const void* x_dev, int32_t x_d
   a.out_qjl = out_qjl_dev;
   a.out_rnorm = out_rnorm_dev;
   return launch_dense(q, x_dev, x_dtype, ld, n, a, st);
+}
+
+extern "C" int tq_selftest_quantize_gives_up(const tq_quantizer* q, const void* x_dev, int64_t ld, int64_t n, uint8_t* out_codes_dev,
+                                             float* out_norm_dev, float* out_scale_dev, uint8_t* out_qjl_dev, float* out_rnorm_dev,
+                                             void* stream) {
+  TQ_REQUIRE(q && x_dev && out_codes_dev && n > 0 && ld >= q->d, TQ_ERR_INVALID, "tq_selftest_quantize_gives_up: bad arguments");
+  if (q->rotation == TQ_ROT_WHT) {
+    TQ_REQUIRE(!out_qjl_dev && !out_rnorm_dev && tq_aligned(out_codes_dev, 16), TQ_ERR_INVALID, "tq_selftest_quantize_gives_up: bad outputs");
+    TqQuantDst dst;
+    memset(&dst, 0, sizeof(dst));
+    dst.idx = out_codes_dev;
+    dst.norm = out_norm_dev;
+    dst.scale = out_scale_dev;
+    dst.heads = 1;
+    return tq_quantize_tc_selftest(q->fast, x_dev, dst, ld, n, (cudaStream_t)stream);
+  }
+  TqDenseQuant t = dense_tensor_args(q);
+  t.out_idx = out_codes_dev;
+  t.out_norm = out_norm_dev; t.out_scale = out_scale_dev; t.out_rnorm = out_rnorm_dev;
+  t.out_qjl = out_qjl_dev;
+  return tq_dense_i8_quantize_selftest(t, q->dig, x_dev, ld, n, (cudaStream_t)stream);
+}
+
+extern "C" int tq_quantize_status_sync(int32_t* status_out) {
+  TQ_REQUIRE(status_out, TQ_ERR_INVALID, "tq_quantize_status_sync: status_out is null");
+  int32_t tiles = 0, dense = 0;
+  TQ_CUDA(tq_quantize_tc_status_sync(&tiles));
+  TQ_CUDA(tq_dense_i8_status_sync(&dense));
+  *status_out = tiles | dense;
+  return TQ_OK;
 }
 
 extern "C" int tq_quantize_residual(const tq_quantizer* q, const void* x_dev, int32_t x_dtype, int64_t ld, int64_t n,

@@ -21,6 +21,8 @@
 //   * PROD keys stay with the warp-level kernel: the two transforms of their sign sketch are one product with an integer matrix
 //     here (1,048,576 keys 228 -> 129 us), but its sums round in another order, and of 33.6 M sketch bits some four then
 //     differ, which a key that a softmax rests on shows.
+//   * a wait that gives up ends the other roles' waits too; the vectors whose indices were not found then have norms and factors that
+//     are not a number, and a status word is set (tq_quantize_status_sync).
 //   * loops over the columns stay loops: unrolled, a tile's code misses the instruction caches.
 //
 // 1,048,576 fp16 vectors of turbo3: 106 -> 87 us (3.7 TB/s; HBM would take 49); the arithmetic on the coordinates bounds it, most of it
@@ -41,6 +43,8 @@ namespace {
 //     131,072 25.7 / 24.7, 262,144 45.8 / 45.7, 1,048,576 147 / 168
 // In vectors per SM (148), so that a device with fewer SMs takes the step earlier.
 inline int64_t qt_min_vectors(bool pair) { return (int64_t)tq_num_sms() * (pair ? 166 : 1776); }
+
+__device__ int32_t qt_status;   // 1: a wait gave up
 
 struct QtJob {
   CUtensorMap map;   // of the rows: 64 elements x 128 rows a box, 128-byte swizzle
@@ -237,14 +241,16 @@ __device__ __forceinline__ void qt_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sptr(bar)) : "memory");
 }
 
-template <typename Tin, int BITS, bool NORMC>
+// SELFTEST: the first CTA's second tile is never reported as multiplied, and waits are short
+template <typename Tin, int BITS, bool NORMC, bool SELFTEST = false>
 __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_constant__ QtJob j0, const __grid_constant__ QtJob j1,
                                                                          int64_t n) {
+  constexpr long long LIMIT = SELFTEST ? TC_SELFTEST_CYCLES : TC_WAIT_CYCLES;
   constexpr int IDXB = 16 * BITS, NC = 1 << BITS, HALF = NC / 2, SLOTS = QT_SLOTS, STAGES = QT_STAGES;
   extern __shared__ __align__(128) uint8_t qt_raw[];
   __shared__ uint64_t a_full[STAGES], a_free[STAGES], d_full[SLOTS], d_free[SLOTS];
   __shared__ uint32_t s_tmem;
-  __shared__ volatile int s_failed;   // a wait gave up: every role stops at its next tile
+  __shared__ volatile int s_failed;   // a wait gave up: nobody waits any more
   __shared__ __align__(16) uint32_t s_flip[4 * BITS];
   const QtJob& job = blockIdx.y == 0 ? j0 : j1;
   const TqFast& f = job.f;
@@ -300,7 +306,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
       int i = 0;
       for (; i < mine && !s_failed; ++i) {
         const int st = i % STAGES;
-        if (i >= STAGES && !tc_wait(&a_free[st], (uint32_t)((i / STAGES - 1) & 1))) { s_failed = 1; break; }
+        if (i >= STAGES && !tc_wait(&a_free[st], (uint32_t)((i / STAGES - 1) & 1), &s_failed, LIMIT)) break;
         const uint32_t dsts = sptr(sm) + st * QT_TILE;
         const int row = (int)((blockIdx.x + i * step) * TQ_D);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(&a_full[st])), "r"(QT_TILE) : "memory");
@@ -314,12 +320,12 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
   } else if (warp == QT_MMA_WARP) {
     if (lane == 0) {
       const uint32_t idesc = umma_idesc(128, 16, false) | QtIn<Tin>::FMT, b = sptr(sm) + QT_OFF_B;
-      for (int i = 0; i < mine && !s_failed; ++i) {
+      int i = 0;
+      for (; i < mine && !s_failed; ++i) {
         const int st = i % STAGES, sl = i % SLOTS;
-        if (!tc_wait(&a_full[st], (uint32_t)((i / STAGES) & 1)) || (i >= SLOTS && !tc_wait(&d_free[sl], (uint32_t)((i / SLOTS - 1) & 1)))) {
-          s_failed = 1;
+        if (!tc_wait(&a_full[st], (uint32_t)((i / STAGES) & 1), &s_failed, LIMIT) ||
+            (i >= SLOTS && !tc_wait(&d_free[sl], (uint32_t)((i / SLOTS - 1) & 1), &s_failed, LIMIT)))
           break;
-        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a = sptr(sm) + st * QT_TILE;
 #pragma unroll
@@ -327,21 +333,22 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
           qt_mma_ss(tb + 128 * sl + 16 * i16, qt_desc_sw128(a + (i16 >> 2) * (QT_TILE / 2) + (i16 & 3) * 32),
                     umma_desc(b + i16 * 512, 128, 256), idesc, 0);
         qt_commit(&a_free[st]);
-        qt_commit(&d_full[sl]);
+        if (!(SELFTEST && blockIdx.x == 0 && i == 1)) qt_commit(&d_full[sl]);
       }
+      if (s_failed && i > 0) tc_wait(&a_free[(i - 1) % STAGES], (uint32_t)(((i - 1) / STAGES) & 1));   // none in flight at the end
     }
   } else if (warp < QT_TMA_WARP) {
   const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;   // this warp's 32 lanes
   const uint32_t zero_idx = 0.f > f.bnd[HALF - 1] ? HALF : HALF - 1;   // index of the value 0
-  for (int i = group; i < mine; i += QT_GROUPS) {
+  int i = group;
+  for (; i < mine; i += QT_GROUPS) {
     const int sl = i % SLOTS;
     const uint32_t tm = tb + 128 * sl + lanes;
     const int64_t v = (blockIdx.x + i * step) * TQ_D + gtid;
     bool good = v < n;
     int64_t within = 0;
     const int64_t rec = good ? tq_dst_record(dst, v, within, good) : 0;   // (the slot's load flies under the MMAs)
-    bool failed = !__all_sync(0xffffffffu, tc_wait(&d_full[sl], (uint32_t)((i / SLOTS) & 1)));
-    if (failed) s_failed = 1;
+    if (!__all_sync(0xffffffffu, tc_wait(&d_full[sl], (uint32_t)((i / SLOTS) & 1), &s_failed, LIMIT))) break;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // ---- the 8-point stage over the blocks, in place, eight columns of every block a turn, and ||x||: ||H x||^2 = 128 ||x||^2.
     // Sums in the warp-level kernel's order (four columns of all blocks, then those four sums in pairs): both kernels then
@@ -424,12 +431,19 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
       cn = cn > 1e-10f ? cn : 1.0f;                      // turboquant/polar_quant.py:110-111
       invn = 1.0f / cn;
     }
-    if (failed) invn = __int_as_float(0x7fffffff);      // a wait gave up: the scales say so
     if (good && dst.scale) {
       *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.scale) + rec + within * 4) = nrm * invn;
     }
     if (v < n && dst.norm) dst.norm[v] = nrm;
-    if (failed) break;
+  }
+  for (; i < mine; i += QT_GROUPS) {   // a wait gave up: this tile and the group's others are not to come
+    const int64_t v = (blockIdx.x + i * step) * TQ_D + gtid;
+    bool good = v < n;
+    int64_t within = 0;
+    const int64_t rec = good ? tq_dst_record(dst, v, within, good) : 0;
+    if (good && dst.scale) *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.scale) + rec + within * 4) = __int_as_float(0x7fffffff);
+    if (v < n && dst.norm) dst.norm[v] = __int_as_float(0x7fffffff);
+    qt_status = 1;
   }
   }
   __syncwarp();
@@ -461,9 +475,9 @@ bool qt_map(CUtensorMap* map, const void* x, int32_t dtype, int64_t ld, int64_t 
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename Tin, int BITS, bool NORMC>
+template <typename Tin, int BITS, bool NORMC, bool SELFTEST = false>
 int launch_tc(const QtJob& j0, const QtJob& j1, int jobs, int64_t n, cudaStream_t st) {
-  auto kernel = k_quantize_tc<Tin, BITS, NORMC>;
+  auto kernel = k_quantize_tc<Tin, BITS, NORMC, SELFTEST>;
   static thread_local int configured_dev = -1;   // one per kernel
   int dev = 0;
   TQ_CUDA(cudaGetDevice(&dev));
@@ -512,4 +526,18 @@ bool tq_quantize_tc_try(const TqFast& f0, const void* x0, const TqQuantDst& d0, 
   *rc = dtype == TQ_F16 ? launch_tc_bits<__half>(j0, j1, jobs, normc, n, st)
                         : launch_tc_bits<__nv_bfloat16>(j0, j1, jobs, normc, n, st);
   return true;
+}
+
+// fp16 rows of a 3-bit quantizer with norm correction, plain arrays
+int tq_quantize_tc_selftest(const TqFast& f, const void* x, const TqQuantDst& d, int64_t ld, int64_t n, cudaStream_t st) {
+  QtJob j;
+  j.f = f; j.dst = d;
+  TQ_REQUIRE(f.bits == 3 && f.norm_correction && tq_aligned(x, 16) && ld % 8 == 0 && qt_map(&j.map, x, TQ_F16, ld, n), TQ_ERR_UNSUPPORTED,
+             "self-test of the long append: fp16 rows of a 3-bit quantizer with norm correction");
+  return launch_tc<__half, 3, true, true>(j, j, 1, n, st);
+}
+cudaError_t tq_quantize_tc_status_sync(int32_t* out) {
+  void* word = nullptr;
+  const cudaError_t e = cudaGetSymbolAddress(&word, qt_status);
+  return e == cudaSuccess ? tc_status_sync((int32_t*)word, out) : e;
 }

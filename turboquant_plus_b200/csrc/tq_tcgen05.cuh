@@ -24,6 +24,25 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// The wait of a role of a kernel whose roles wait for one another: `failed`, in shared memory, is set by the first one that gives up
+// and ends the waits of all.  The limit is an argument for the self-tests' sake, which make a wait run out.
+constexpr long long TC_SELFTEST_CYCLES = 1LL << 20;
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* failed, long long limit) {
+  if (tc_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!*failed) {
+    if (tc_try_wait(bar, parity)) return true;
+    if (clock64() - t0 > limit) *failed = 1;
+  }
+  return false;
+}
+// Reads and clears a kernel's status word
+inline cudaError_t tc_status_sync(int32_t* word_dev, int32_t* out) {
+  cudaError_t e = cudaMemcpy(out, word_dev, 4, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess && *out != 0) e = cudaMemset(word_dev, 0, 4);
+  return e;
+}
+
 // shared-memory matrix descriptor, no swizzle: start address, leading-dimension and stride byte offsets (16-byte
 // units), descriptor version 1.  K-major operand: LBO = distance between 8-element K chunks, SBO = distance
 // between 8-row groups.  MN-major operand: LBO = distance between 8-row K groups, SBO = between 8-element N chunks.
