@@ -138,3 +138,54 @@ def test_uneven_constants(kind):
     few = torch.cat([pq.dequantize(idx[lo:lo + PIECE], norms[lo:lo + PIECE]) for lo in range(0, n, PIECE)])
     size = few.abs().amax(dim=1 if kind == "centroids" else 0, keepdim=True)
     assert bool(((back - few).abs() <= 256 * 2.0 ** -53 * size).all())
+
+
+def test_first_large_calls():
+    """The first call of many vectors makes the digits: from several threads' streams at once, in a graph being captured (which
+    takes the fp64 products), and in the direction of ``dequantize``."""
+    import threading
+
+    import torch
+    import turboquant_plus_b200 as tq
+    n, threads = 20011, 6
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, D, device="cuda", generator=gen)
+
+    def fresh():
+        q = tq.TurboQuant(D, 4, seed=9)
+        q.quantize_device(x[:100])              # the constants are on the device, the digits are not
+        return q
+
+    def same(a, b):
+        return all(torch.equal(a[name], b[name]) for name in b)
+
+    right = fresh().quantize_device(x)
+    for _ in range(3):
+        q, got, start = fresh(), [None] * threads, threading.Barrier(threads)
+        torch.cuda.synchronize()
+
+        def work(i):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait()
+                got[i] = q.quantize_device(x)
+                torch.cuda.current_stream().synchronize()
+
+        pool = [threading.Thread(target=work, args=(i,)) for i in range(threads)]
+        [t.start() for t in pool]
+        [t.join() for t in pool]
+        assert all(same(g, right) for g in got)
+
+    q, graph, other = fresh(), torch.cuda.CUDAGraph(), fresh()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        captured = q.quantize_device(x)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert same(captured, right) and same(q.quantize_device(x), right)
+    graph.reset()
+
+    code = other.quantize(x)
+    back = fresh().dequantize(code)
+    few = torch.cat([other.dequantize(type(code)(**{f: (getattr(code, f)[lo:lo + PIECE] if torch.is_tensor(getattr(code, f)) else getattr(code, f))
+                                                     for f in code.__dataclass_fields__})) for lo in range(0, n, PIECE)])
+    assert bool(((back - few).abs() <= 256 * 2.0 ** -53 * few.abs().amax(dim=1, keepdim=True)).all())

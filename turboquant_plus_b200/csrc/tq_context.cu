@@ -120,6 +120,7 @@ static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
 extern "C" int tq_quantizer_destroy(tq_quantizer* q) {
   if (!q) return TQ_OK;
   if (q->mem) cudaFree(q->mem);
+  if (q->digits_event) cudaEventDestroy(q->digits_event);
   free(q);
   return TQ_OK;
 }
@@ -218,8 +219,9 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
   if (dense_rot) mr = add_matrix(im, desc->rot, q->d);
   if (dense_s) ms = add_matrix(im, desc->qjl_s, q->d);
   const size_t cent_at = im.add(c.data(), c.size() * 8), bnd_at = im.add(b.data(), b.size() * 8);
-  const size_t digits_at = (im.bytes.size() + 255) & ~(size_t)255;   // digits of R, R^T, S, S^T, made on the device
-  const size_t total = mr.scale != 0.0 || ms.scale != 0.0 ? digits_at + 4 * TQ_DENSE_DIGITS_BYTES : im.bytes.size();
+  // room for the digits of R, R^T, S, S^T, which the first call of many vectors makes (tq_dense_i8.cu)
+  const size_t digits_at = (im.bytes.size() + 255) & ~(size_t)255;
+  const size_t total = digits_at + ((mr.scale != 0.0 ? 2 : 0) + (ms.scale != 0.0 ? 2 : 0)) * (size_t)TQ_DENSE_DIGITS_BYTES;
   e = cudaMalloc((void**)&q->mem, total);
   if (e == cudaSuccess) e = cudaMemcpy(q->mem, im.bytes.data(), im.bytes.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
@@ -231,19 +233,13 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
   if (dense_rot) q->rot = f64(mr.m), q->rot_t = f64(mr.t), q->rot32 = f32(mr.m32), q->rot32_t = f32(mr.t32), q->rotp = f64(mr.mp), q->rotp_t = f64(mr.tp);
   if (dense_s) q->s = f64(ms.m), q->s_t = f64(ms.t), q->s32 = f32(ms.m32), q->s32_t = f32(ms.t32), q->sp = f64(ms.mp), q->sp_t = f64(ms.tp);
   uint8_t* digits = q->mem + digits_at;
-  auto add_digits = [&](const double* m, double scale) -> const uint8_t* {
+  auto digits_place = [&]() {
     uint8_t* at = digits;
     digits += TQ_DENSE_DIGITS_BYTES;
-    if (e == cudaSuccess) e = tq_dense_digits(m, scale, at);
     return at;
   };
-  if (mr.scale != 0.0) q->dig.r = add_digits(q->rot, mr.scale), q->dig.rt = add_digits(q->rot_t, mr.scale), q->dig.r_scale = mr.scale;
-  if (ms.scale != 0.0) q->dig.s = add_digits(q->s, ms.scale), q->dig.st = add_digits(q->s_t, ms.scale), q->dig.s_scale = ms.scale;
-  if (e == cudaSuccess && total > im.bytes.size()) e = cudaStreamSynchronize(cudaStreamLegacy);   // other streams may use them at once
-  if (e != cudaSuccess) {
-    tq_quantizer_destroy(q);
-    return tq_cuda_fail(e, "digits of the dense matrices");
-  }
+  if (mr.scale != 0.0) q->dig.r = digits_place(), q->dig.rt = digits_place(), q->dig.r_scale = mr.scale;
+  if (ms.scale != 0.0) q->dig.s = digits_place(), q->dig.st = digits_place(), q->dig.s_scale = ms.scale;
   q->dig.cent_scale = tq_dense_digits_centroids(c.data(), nc);
   for (size_t i = 0; i < b.size(); ++i) q->dig.bnd[i] = b[i];
   q->cent64 = f64(cent_at);

@@ -28,6 +28,7 @@
 //
 // A row that this arithmetic does not carry -- values that are not finite or too small for a norm, residuals far beyond the
 // vector's length, which an arbitrary matrix can produce -- is computed by one warp in plain fp64.
+#include <mutex>
 #include "tq_tcgen05.cuh"
 
 namespace {
@@ -754,14 +755,65 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(512u) : "memory");
 }
 
-// Digits of a 128 x 128 matrix (rows are outputs) as the B operand: [digit][8-output group][16-element chunk][output][element]
+// Digits of 128 x 128 matrices (rows are outputs) as B operands: [digit][8-output group][16-element chunk][output][element]
 // bytes, TQ_DENSE_DIGITS_BYTES in all; `scale` times a value is below 2^54.  A thread takes one element.
-__global__ void __launch_bounds__(128) k_dense_digits(const double* __restrict__ m, double scale, uint8_t* __restrict__ out) {
-  const int n = blockIdx.x, k = threadIdx.x;
-  const uint64_t u = di_digits(__double2ll_rn(m[n * TQ_D + k] * scale));
-  uint8_t* at = out + (n >> 3) * 1024 + (k >> 4) * 128 + (n & 7) * 16 + (k & 15);
+struct DiMatrices {
+  const double* m[4];
+  double scale[4];
+  uint8_t* out[4];
+};
+__global__ void __launch_bounds__(128) k_dense_digits(const __grid_constant__ DiMatrices a) {
+  const int n = blockIdx.x, k = threadIdx.x, i = blockIdx.y;
+  const uint64_t u = di_digits(__double2ll_rn(a.m[i][n * TQ_D + k] * a.scale[i]));
+  uint8_t* at = a.out[i] + (n >> 3) * 1024 + (k >> 4) * 128 + (n & 7) * 16 + (k & 15);
 #pragma unroll
   for (int p = 0; p < DI_DIGITS; ++p) at[p * DI_TILE] = (uint8_t)(u >> (48 - 8 * p));
+}
+
+// The digits of a quantizer's matrices, behind which `st` may go on; false where they are not to be had now: the call then takes the
+// fp64 kernels.  The first call makes them, on its own stream, so that quantizers which never see one do not pay for it
+// (made with the quantizer they cost 30 to 90 us of its 1,100); later ones on any stream wait for its event until it
+// has been seen.  A call that is being captured neither makes them nor waits: its graph could run before, or alone.
+constexpr int32_t DI_MADE = 1, DI_SEEN = 2;
+bool di_digits_ready(const tq_quantizer* q, cudaStream_t st) {
+  if (__atomic_load_n(&q->digits_state, __ATOMIC_ACQUIRE) == DI_SEEN) return true;
+  static std::mutex lock;
+  const std::lock_guard<std::mutex> hold(lock);
+  // (other threads may be capturing: nothing here touches their streams)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return false;
+  auto prepare = [&]() -> cudaError_t {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &capture);
+    if (e != cudaSuccess) return e;
+    if (q->digits_state >= DI_MADE) {
+      e = cudaEventQuery(q->digits_event);
+      if (e == cudaSuccess) __atomic_store_n(&q->digits_state, DI_SEEN, __ATOMIC_RELEASE);
+      if (e != cudaErrorNotReady) return e;
+      (void)cudaGetLastError();
+      return capture == cudaStreamCaptureStatusNone ? cudaStreamWaitEvent(st, q->digits_event, 0) : cudaErrorNotReady;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return cudaErrorNotReady;
+    if (!q->digits_event && (e = cudaEventCreateWithFlags(&q->digits_event, cudaEventDisableTiming)) != cudaSuccess) return e;
+    DiMatrices a;
+    int count = 0;
+    auto add = [&](const double* m, double scale, const uint8_t* out) {
+      a.m[count] = m;
+      a.scale[count] = 18014398509481984.0 / scale;
+      a.out[count++] = const_cast<uint8_t*>(out);
+    };
+    const TqDenseDigits& g = q->dig;
+    if (g.r_scale != 0.0) add(q->rot, g.r_scale, g.r), add(q->rot_t, g.r_scale, g.rt);
+    if (g.s_scale != 0.0) add(q->s, g.s_scale, g.s), add(q->s_t, g.s_scale, g.st);
+    k_dense_digits<<<dim3(TQ_D, count), TQ_D, 0, st>>>(a);
+    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaEventRecord(q->digits_event, st)) != cudaSuccess) return e;
+    __atomic_store_n(&q->digits_state, DI_MADE, __ATOMIC_RELEASE);
+    return cudaSuccess;
+  };
+  const cudaError_t e = prepare();
+  (void)cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e == cudaSuccess;
 }
 
 template <auto kernel, typename... Args> int di_launch(int smem, int64_t n, cudaStream_t st, const char* what, const Args&... args) {
@@ -834,10 +886,6 @@ double tq_dense_digits_centroids(const double* c, int n) {
   frexp(most, &e);
   return ldexp(1.0, e);
 }
-cudaError_t tq_dense_digits(const double* m_dev, double scale, uint8_t* out_dev) {
-  k_dense_digits<<<TQ_D, TQ_D>>>(m_dev, 18014398509481984.0 / scale, out_dev);
-  return cudaGetLastError();
-}
 
 // Calls that come here, us here / in the fp64 kernels (which take tiles of 16, 32 or 64 vectors, two CTAs an SM, and step up at 32
 // and 64 vectors per SM): quantize 8,192 vectors 23.2 / 23.2, 12,000 23.2 / 39.6, 65,536 77 / 134; with the sketch 4,096 50 / 34, 8,192
@@ -870,36 +918,36 @@ static bool di_dequant_args(const TqDenseDequant& a, const TqDenseDigits& g, DiD
 }
 
 // false: not of these kernels' kind, nothing launched
-bool tq_dense_i8_quantize_try(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
+bool tq_dense_i8_quantize_try(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
                               int* rc) {
   DiQuant A;
-  if (!di_enough(n, false) || !di_quant_args(a, g, x, dtype, ld, A)) return false;
+  if (!di_enough(n, false) || !di_quant_args(a, q->dig, x, dtype, ld, A) || !di_digits_ready(q, st)) return false;
   *rc = dtype == TQ_F32 ? di_quantize<float>(A, x, ld, n, st) : di_quantize<__half>(A, x, ld, n, st);
   return true;
 }
 
-bool tq_dense_i8_dequantize_try(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc) {
+bool tq_dense_i8_dequantize_try(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc) {
   DiDequant A;
-  if (!di_enough(n, a.qjl != nullptr) || !di_dequant_args(a, g, A)) return false;
+  if (dtype != TQ_F64 && dtype != TQ_F32 && dtype != TQ_F16) return false;
+  if (!di_enough(n, a.qjl != nullptr) || !di_dequant_args(a, q->dig, A) || !di_digits_ready(q, st)) return false;
   switch (dtype) {
     case TQ_F64: *rc = di_dequantize<double>(A, n, out, st); return true;
     case TQ_F32: *rc = di_dequantize<float>(A, n, out, st); return true;
-    case TQ_F16: *rc = di_dequantize<__half>(A, n, out, st); return true;
-    default: return false;
+    default: *rc = di_dequantize<__half>(A, n, out, st); return true;
   }
 }
 
 // The self-tests' forms: fp32 rows of 2 bits and a sketch; fp64 results with a sketch
-int tq_dense_i8_quantize_selftest(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int64_t ld, int64_t n, cudaStream_t st) {
+int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, cudaStream_t st) {
   DiQuant A;
-  TQ_REQUIRE(a.bits == 2 && a.out_qjl && di_quant_args(a, g, x, TQ_F32, ld, A), TQ_ERR_UNSUPPORTED,
+  TQ_REQUIRE(a.bits == 2 && a.out_qjl && di_quant_args(a, q->dig, x, TQ_F32, ld, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED,
              "self-test of the dense quantizer: fp32 rows of 128 elements, 2 bits and a sketch");
   return di_launch<k_dense_quantize_i8<float, 2, true, true>>(di_quant_smem<float>(), n, st, "k_dense_quantize_i8", A,
                                                               reinterpret_cast<const float*>(x), ld, n);
 }
-int tq_dense_i8_dequantize_selftest(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, double* out, cudaStream_t st) {
+int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st) {
   DiDequant A;
-  TQ_REQUIRE(a.qjl && di_dequant_args(a, g, A), TQ_ERR_UNSUPPORTED, "self-test of the dense dequantizer: 128 elements and a sketch");
+  TQ_REQUIRE(a.qjl && di_dequant_args(a, q->dig, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED, "self-test of the dense dequantizer: 128 elements and a sketch");
   return di_launch<k_dense_dequantize_i8<double, true, true>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, out);
 }
 cudaError_t tq_dense_i8_status_sync(int32_t* out) {

@@ -227,14 +227,14 @@ static bool dequantize_tensor(const tq_quantizer* q, const uint8_t* packed, cons
                               const uint8_t* qjl, const float* rnorm, double shrink, int64_t n, void* out, int32_t dtype,
                               int64_t ld_out, int32_t accumulate, cudaStream_t st, int* rc) {
   const TqDenseDequant t = dense_tensor_args(q, packed, idx, norm, qjl, rnorm, shrink, ld_out, accumulate);
-  return tq_dense_i8_dequantize_try(t, q->dig, n, out, dtype, st, rc) || tq_dense_dequantize_try(t, n, out, dtype, st, rc);
+  return tq_dense_i8_dequantize_try(q, t, n, out, dtype, st, rc) || tq_dense_dequantize_try(t, n, out, dtype, st, rc);
 }
 
 extern "C" int tq_selftest_dequantize_gives_up(const tq_quantizer* q, const uint8_t* idx_dev, const float* norm_dev, const uint8_t* qjl_dev,
                                                const float* rnorm_dev, int64_t n, double* out_dev, void* stream) {
   TQ_REQUIRE(q && q->rotation == TQ_ROT_DENSE && q->qjl && idx_dev && norm_dev && qjl_dev && rnorm_dev && out_dev && n > 0, TQ_ERR_INVALID,
              "tq_selftest_dequantize_gives_up: bad arguments");
-  return tq_dense_i8_dequantize_selftest(dense_tensor_args(q, nullptr, idx_dev, norm_dev, qjl_dev, rnorm_dev, 1.0, q->d, 0), q->dig, n,
+  return tq_dense_i8_dequantize_selftest(q, dense_tensor_args(q, nullptr, idx_dev, norm_dev, qjl_dev, rnorm_dev, 1.0, q->d, 0), n,
                                          out_dev, (cudaStream_t)stream);
 }
 

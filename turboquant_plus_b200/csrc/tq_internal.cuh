@@ -38,7 +38,6 @@ struct TqDenseDigits {
 #define TQ_DENSE_DIGITS_BYTES (7 * TQ_D * TQ_D)
 double tq_dense_digits_scale(const double* m);
 double tq_dense_digits_centroids(const double* c, int n);
-cudaError_t tq_dense_digits(const double* m_dev, double scale, uint8_t* out_dev);   // on the legacy stream
 
 struct tq_quantizer {
   int32_t d, bits, rotation, norm_correction, qjl, device;
@@ -55,6 +54,9 @@ struct tq_quantizer {
   float* s32_t;
   double host_cent[16];
   TqDenseDigits dig;
+  // whether dig's matrices have been made, and the event behind that (tq_dense_i8.cu; created with calloc, zero: not yet)
+  mutable cudaEvent_t digits_event;
+  mutable int32_t digits_state;
 };
 
 void tq_set_error(const char* fmt, ...);
@@ -306,12 +308,12 @@ struct TqDenseDequant {
 bool tq_dense_quantize_try(const TqDenseQuant& a, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st, int* rc);
 bool tq_dense_dequantize_try(const TqDenseDequant& a, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
 
-bool tq_dense_i8_quantize_try(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
+bool tq_dense_i8_quantize_try(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
                               int* rc);
-bool tq_dense_i8_dequantize_try(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
+bool tq_dense_i8_dequantize_try(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
 // Runs in which one wait runs out, and the words that say so (tq_selftest_quantize_gives_up, tq_quantize_status_sync)
-int tq_dense_i8_quantize_selftest(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int64_t ld, int64_t n, cudaStream_t st);
-int tq_dense_i8_dequantize_selftest(const TqDenseDequant& a, const TqDenseDigits& g, int64_t n, double* out, cudaStream_t st);
+int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, cudaStream_t st);
+int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st);
 int tq_quantize_tc_selftest(const TqFast& f, const void* x, const TqQuantDst& d, int64_t ld, int64_t n, cudaStream_t st);
 cudaError_t tq_dense_i8_status_sync(int32_t* out);
 cudaError_t tq_quantize_tc_status_sync(int32_t* out);

@@ -544,7 +544,7 @@ static int launch_dense(const tq_quantizer* q, const void* x, int32_t dtype, int
     t.out_norm = a.out_norm; t.out_scale = a.out_scale; t.out_rnorm = a.out_rnorm;
     t.out_qjl = a.out_qjl; t.out_res = a.out_res; t.ld_res = a.ld_res;
     int rc = TQ_OK;
-    if (tq_dense_i8_quantize_try(t, q->dig, x, dtype, ld, n, st, &rc)) return rc;
+    if (tq_dense_i8_quantize_try(q, t, x, dtype, ld, n, st, &rc)) return rc;
     if (tq_dense_quantize_try(t, x, dtype, ld, n, st, &rc)) return rc;
   }
   const size_t smem = (size_t)q->d * TV * 8 * 2 + (size_t)q->d * TV + 16;
@@ -633,7 +633,7 @@ extern "C" int tq_selftest_quantize_gives_up(const tq_quantizer* q, const void* 
   t.out_idx = out_codes_dev;
   t.out_norm = out_norm_dev; t.out_scale = out_scale_dev; t.out_rnorm = out_rnorm_dev;
   t.out_qjl = out_qjl_dev;
-  return tq_dense_i8_quantize_selftest(t, q->dig, x_dev, ld, n, (cudaStream_t)stream);
+  return tq_dense_i8_quantize_selftest(q, t, x_dev, ld, n, (cudaStream_t)stream);
 }
 
 extern "C" int tq_quantize_status_sync(int32_t* status_out) {
