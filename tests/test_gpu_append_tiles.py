@@ -1,5 +1,6 @@
 """Long appends, which take 128 vectors a tensor-core tile, against the same rows appended in short pieces, which the warp-level
-kernel takes: vectors around a tile's edge, head counts that leave a ragged last tile, zero rows, tokens without a slot.
+kernel takes: vectors around a tile's edge, head counts that leave a ragged last tile, zero rows, tokens without a slot, rows of
+exact zeros, of both ends of their type's range and beyond it, plain packed arrays.
 Both form every sum behind an index in the same order: indices are equal.  Scales come from sums of counts in another order:
 six roundings of 2^-24 in all.  PROD keys take the warp-level kernel at every length: all of their record is equal."""
 import pytest
@@ -17,14 +18,19 @@ def _fields(cache):
     return out
 
 
+# vectors per SM from which two tensors of one format, and one beside another kernel, take the tile kernel
+PAIR, ALONE = 166, 1776
+
+
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
-@pytest.mark.parametrize("k,v,vectors", [("turbo2", "turbo2", 24568), ("turbo3", "turbo3", 24567), ("turbo3", "turbo3", 24568),
-                                         ("turbo4", "turbo4", 24569), ("turbo3", "turbo3", 24703), ("turbo3", "turbo3", 75777),
-                                         ("turbo4", "turbo4", 131072), ("q8_0", "turbo2", 262849), ("prod3", "turbo3", 284673)])
-def test_long_append_equals_short_ones(k, v, vectors, dtype):
+@pytest.mark.parametrize("k,v,heads,per_sm,more", [("turbo2", "turbo2", 1, PAIR, 0), ("turbo3", "turbo3", 1, PAIR, -1), ("turbo3", "turbo3", 3, PAIR, 2),
+                                                   ("turbo4", "turbo4", 8, PAIR, 8), ("turbo3", "turbo3", 1, PAIR, 135), ("turbo3", "turbo3", 3, 512, 1),
+                                                   ("turbo2", "turbo2", 8, 880, 8), ("turbo4", "turbo4", 3, 880, 2), ("q8_0", "turbo2", 8, ALONE, 8),
+                                                   ("q8_0", "turbo4", 3, ALONE, 2), ("turbo3", "turbo3", 8, ALONE, 136), ("prod3", "turbo3", 3, 1923, 0)])
+def test_long_append_equals_short_ones(k, v, heads, per_sm, more, dtype):
     import torch
     import turboquant_plus_b200 as tq
-    heads = 3 if vectors % 3 == 0 else 1
+    vectors = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + more
     tokens = vectors // heads
     gen = torch.Generator(device="cuda").manual_seed(vectors)
     rows = []
@@ -95,7 +101,7 @@ def _odd_rows(tokens, heads, dtype, gen):
 def test_odd_rows_of_long_appends(fmt, heads, norm_correction, dtype):
     import torch
     import turboquant_plus_b200 as tq
-    vectors = 166 * torch.cuda.get_device_properties(0).multi_processor_count       # the shortest append of the tile kernel
+    vectors = PAIR * torch.cuda.get_device_properties(0).multi_processor_count
     tokens = -(-vectors // heads) + 5
     gen = torch.Generator(device="cuda").manual_seed(heads)
     rows = [_odd_rows(tokens, heads, dtype, gen) for _ in range(2)]
@@ -113,3 +119,22 @@ def test_odd_rows_of_long_appends(fmt, heads, norm_correction, dtype):
         assert torch.equal(a[t], b[t])
         sa, sb = a[t + "_scale"], b[t + "_scale"]
         assert bool((((sa - sb).abs() <= 6 * 2.0 ** -24 * sb.abs()) | (sa == sb) | (sa.isnan() & sb.isnan())).all())
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("bits,norm_correction,width", [(2, True, 128), (3, True, 136), (3, False, 128), (4, True, 256), (4, False, 136)])
+def test_long_packed_arrays(bits, norm_correction, width, dtype):
+    """Packed indices, norms and factors as plain arrays, rows with elements between them."""
+    import torch
+    import turboquant_plus_b200 as tq
+    n = ALONE * torch.cuda.get_device_properties(0).multi_processor_count + 77
+    gen = torch.Generator(device="cuda").manual_seed(n + bits)
+    rows = torch.full((n, width), float("nan"), device="cuda", dtype=getattr(torch, dtype))
+    rows[:, :D] = _odd_rows(n, 1, dtype, gen)[:, 0]
+    q = tq.PolarQuant(D, bits, seed=3, norm_correction=norm_correction, rotation="wht")
+    whole = q.quantize_device(rows, packed=True, want_scale=True)
+    few = [q.quantize_device(rows[lo:lo + 50000], packed=True, want_scale=True) for lo in range(0, n, 50000)]
+    assert torch.equal(whole["packed"], torch.cat([f["packed"] for f in few]))
+    for name, roundings in (("norm", 0), ("scale", 6)):
+        a, b = whole[name], torch.cat([f[name] for f in few])
+        assert bool((((a - b).abs() <= roundings * 2.0 ** -24 * b.abs()) | (a == b) | (a.isnan() & b.isnan())).all())
