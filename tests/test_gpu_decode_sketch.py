@@ -72,3 +72,21 @@ def test_sketch_share(fmt, group, factor):
     bound = 2.0 ** -19 * mass + 2.0 ** -21 * np.abs(lse).reshape(2, n, hq).max(0)
     err = np.abs((lse[:n] - lse[n:]) / 2 - share)
     assert (err <= bound).all(), (err / np.maximum(bound, 1e-300)).max()
+
+
+@pytest.mark.parametrize("group", [1, 4, 7])
+def test_tiny_queries(group):
+    """Queries down to the smallest numbers of their type: scores of next to nothing, the outputs are those of zero queries."""
+    import torch
+    import turboquant_plus_b200 as tq
+    n, hq = 300, HKV * group
+    gen = torch.Generator(device="cuda").manual_seed(group)
+    cache = tq.PagedKVCache(D, HKV, 3, 128, "prod3", "turbo3", seed=42)
+    k, v = (torch.randn(n, HKV, D, device="cuda", generator=gen).half() for _ in range(2))
+    cache.append(k, v, torch.arange(n, device="cuda"))
+    powers = torch.arange(20, 46, device="cuda")
+    q = torch.randn(len(powers), hq, D, device="cuda", generator=gen) * (10.0 ** -powers.double())[:, None, None].float()
+    table = torch.arange(3, device="cuda", dtype=torch.int32).repeat(len(powers), 1)
+    lens = torch.full((len(powers),), n, device="cuda", dtype=torch.int32)
+    out, zero = cache.attend(q, table, lens), cache.attend(torch.zeros_like(q), table, lens)
+    assert torch.equal(out, zero) and bool(out.isfinite().all())

@@ -737,8 +737,8 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
         most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, m));
         total += __shfl_xor_sync(0xffffffffu, total, m);
       }
-      const int e = (int)((__float_as_uint(most) >> 23) & 255u);            // most < 2^(e - 126)
-      zscale = e > 0 && e < 240 ? __uint_as_float((uint32_t)(250 - e) << 23) : 1.f;   // 2^(123 - e): most x zscale < 2^-3
+      const int e = max((int)((__float_as_uint(most) >> 23) & 255u), 14);   // most < 2^(e - 126); from 14: 2^18 zscale is a finite number
+      zscale = e < 240 ? __uint_as_float((uint32_t)(250 - e) << 23) : 1.f;  // 2^(123 - e): most x zscale < 2^-3
       const float back = 2.f / zscale, take = lo ? 0.f : total;             // (the lo halves are part of the same sum)
       Q.zs0 = __shfl_sync(0xffffffffu, back, 8 * t);                        // column 2t is that of the lanes g = 2t
       Q.zs1 = __shfl_sync(0xffffffffu, back, 8 * t + 4);
