@@ -117,6 +117,33 @@ static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
   return p;
 }
 
+// (tq_quantize_status_word; this file has no kernels)
+static __device__ int32_t quantize_status;
+
+int32_t* tq_quantize_status_word() {
+  static thread_local int word_dev = -1;
+  static thread_local int32_t* word = nullptr;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  if (word_dev != dev) {
+    if (cudaGetSymbolAddress((void**)&word, quantize_status) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    word_dev = dev;
+  }
+  return word;
+}
+
+extern "C" int tq_quantize_status_sync(int32_t* status_out) {
+  TQ_REQUIRE(status_out, TQ_ERR_INVALID, "tq_quantize_status_sync: status_out is null");
+  int32_t* word = tq_quantize_status_word();
+  TQ_REQUIRE(word, TQ_ERR_CUDA, "tq_quantize_status_sync: no status word on this device");
+  TQ_CUDA(cudaMemcpy(status_out, word, 4, cudaMemcpyDeviceToHost));
+  if (*status_out != 0) TQ_CUDA(cudaMemset(word, 0, 4));
+  return TQ_OK;
+}
+
 extern "C" int tq_quantizer_destroy(tq_quantizer* q) {
   if (!q) return TQ_OK;
   if (q->mem) cudaFree(q->mem);
@@ -156,6 +183,7 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
   q->rotation = desc->rotation;
   q->norm_correction = desc->norm_correction ? 1 : 0;
   q->qjl = desc->qjl ? 1 : 0;
+  (void)tq_quantize_status_word();   // its module is loaded here, not by a call that may be captured
   cudaError_t e = cudaGetDevice(&q->device);
   if (e != cudaSuccess) {
     free(q);

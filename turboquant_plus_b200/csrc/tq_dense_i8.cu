@@ -33,8 +33,6 @@
 
 namespace {
 
-__device__ int32_t di_status;   // 1: a wait gave up
-
 constexpr int DI_DIGITS = 7, DI_SUMS = 8;
 constexpr int DI_ROWS = 128, DI_ROW_THREADS = 512, DI_COPIER = 16, DI_MMA = 17, DI_THREADS = 576;
 constexpr int DI_COLS = 32;                         // columns of a row thread: four threads a row
@@ -266,11 +264,13 @@ struct DiQuant {
   double r_scale;                     // R w = sums x this
   double cent_scale;                  // power of two above every centroid's magnitude
   double bnd[15];                     // boundaries (parameters: operands of the comparisons as they are)
+  int32_t* status;                    // raised when a wait gives up
   TqDenseQuant q;
 };
 struct DiDequant {
   const uint8_t *rt, *st;
   double r_scale, s_scale, cent_scale;
+  int32_t* status;
   TqDenseDequant q;
 };
 
@@ -337,7 +337,7 @@ __device__ void di_row_plain(const TqDenseQuant& a, const uint8_t* xrow, float n
 template <typename T> __device__ __forceinline__ T di_from(double v) { return (T)v; }
 template <> __device__ __forceinline__ __half di_from<__half>(double v) { return __float2half_rn((float)v); }
 // A wait gave up: the results of this CTA's tiles from `t` on are not to come.  (Functions of their own: inlined, they cost the kernels registers.)
-__device__ __noinline__ void di_give_up(const TqDenseQuant& a, int t, int mine, int row, int64_t n) {
+__device__ __noinline__ void di_give_up(const TqDenseQuant& a, int t, int mine, int row, int64_t n, int32_t* status) {
   const float nan = __int_as_float(0x7fffffff);
   for (; t < mine; ++t) {
     const int64_t v = (blockIdx.x + (int64_t)t * gridDim.x) * DI_ROWS + row;
@@ -346,14 +346,14 @@ __device__ __noinline__ void di_give_up(const TqDenseQuant& a, int t, int mine, 
     if (a.out_scale) a.out_scale[v] = nan;
     if (a.out_rnorm) a.out_rnorm[v] = nan;
   }
-  di_status = 1;
+  if (status) *status = 1;
 }
-template <typename Tout> __device__ __noinline__ void di_give_up(const TqDenseDequant& a, int t, int mine, int row, int col, int64_t n, Tout* out) {
+template <typename Tout> __device__ __noinline__ void di_give_up(const TqDenseDequant& a, int t, int mine, int row, int col, int64_t n, Tout* out, int32_t* status) {
   for (; t < mine; ++t) {
     const int64_t v = (blockIdx.x + (int64_t)t * gridDim.x) * DI_ROWS + row;
     for (int k = 0; k < DI_COLS && v < n; ++k) out[v * a.ld_out + col + k] = di_from<Tout>(__longlong_as_double(0x7ff8000000000000ll));
   }
-  di_status = 1;
+  if (status) *status = 1;
 }
 
 template <typename Tin> constexpr int di_row_bytes() { return TQ_D * (int)sizeof(Tin) + 16; }   // (rows 4 banks apart: no conflicts)
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (di_rows_any(sh.failed)) {   // the last tile begun and those behind it
-      di_give_up(a, t > 0 ? t - 1 : 0, mine, h == 0 ? row : -1, n);
+      di_give_up(a, t > 0 ? t - 1 : 0, mine, h == 0 ? row : -1, n, A.status);
     }
   }
   __syncwarp();
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (di_rows_any(sh.failed)) {   // the last tile begun and those behind it
-      di_give_up<Tout>(a, t > 0 ? t - 1 : 0, mine, row, DI_COLS * h, n, out);
+      di_give_up<Tout>(a, t > 0 ? t - 1 : 0, mine, row, DI_COLS * h, n, out, A.status);
     }
   }
   __syncwarp();
@@ -902,6 +902,7 @@ static bool di_quant_args(const TqDenseQuant& a, const TqDenseDigits& g, const v
   A.r = g.r; A.rt = g.rt; A.s = g.s;
   A.r_scale = g.r_scale / 4096.0;
   A.cent_scale = g.cent_scale;
+  A.status = tq_quantize_status_word();
   for (int i = 0; i < 15; ++i) A.bnd[i] = g.bnd[i];
   A.q = a;
   return true;
@@ -913,6 +914,7 @@ static bool di_dequant_args(const TqDenseDequant& a, const TqDenseDigits& g, DiD
   A.r_scale = g.r_scale / 4096.0;
   A.s_scale = g.s_scale / 64.0;
   A.cent_scale = g.cent_scale;
+  A.status = tq_quantize_status_word();
   A.q = a;
   return true;
 }
@@ -949,9 +951,4 @@ int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant&
   DiDequant A;
   TQ_REQUIRE(a.qjl && di_dequant_args(a, q->dig, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED, "self-test of the dense dequantizer: 128 elements and a sketch");
   return di_launch<k_dense_dequantize_i8<double, true, true>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, out);
-}
-cudaError_t tq_dense_i8_status_sync(int32_t* out) {
-  void* word = nullptr;
-  const cudaError_t e = cudaGetSymbolAddress(&word, di_status);
-  return e == cudaSuccess ? tc_status_sync((int32_t*)word, out) : e;
 }

@@ -311,12 +311,14 @@ bool tq_dense_dequantize_try(const TqDenseDequant& a, int64_t n, void* out, int3
 bool tq_dense_i8_quantize_try(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
                               int* rc);
 bool tq_dense_i8_dequantize_try(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc);
-// Runs in which one wait runs out, and the words that say so (tq_selftest_quantize_gives_up, tq_quantize_status_sync)
+// The current device's word that a quantize or dequantize kernel raises when a wait gives up; null where there is none.  A kernel
+// takes its address as a parameter: a device variable in a kernel's own module costs every launch outside a graph 0.6 to
+// 0.9 us (append of 8,192 tokens of turbo3: 14.1 us, 14.8 with a variable that only a branch not taken writes).
+int32_t* tq_quantize_status_word();
+// Runs in which one wait runs out (tq_selftest_quantize_gives_up)
 int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, cudaStream_t st);
 int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st);
 int tq_quantize_tc_selftest(const TqFast& f, const void* x, const TqQuantDst& d, int64_t ld, int64_t n, cudaStream_t st);
-cudaError_t tq_dense_i8_status_sync(int32_t* out);
-cudaError_t tq_quantize_tc_status_sync(int32_t* out);
 
 // A chunk of queries per sequence as rows of the decode kernel, each with its causal length.  The workspace is one of
 // tq_decode_workspace_bytes(batch * queries, ...).

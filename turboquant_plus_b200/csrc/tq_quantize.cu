@@ -636,15 +636,6 @@ extern "C" int tq_selftest_quantize_gives_up(const tq_quantizer* q, const void* 
   return tq_dense_i8_quantize_selftest(q, t, x_dev, ld, n, (cudaStream_t)stream);
 }
 
-extern "C" int tq_quantize_status_sync(int32_t* status_out) {
-  TQ_REQUIRE(status_out, TQ_ERR_INVALID, "tq_quantize_status_sync: status_out is null");
-  int32_t tiles = 0, dense = 0;
-  TQ_CUDA(tq_quantize_tc_status_sync(&tiles));
-  TQ_CUDA(tq_dense_i8_status_sync(&dense));
-  *status_out = tiles | dense;
-  return TQ_OK;
-}
-
 extern "C" int tq_quantize_residual(const tq_quantizer* q, const void* x_dev, int32_t x_dtype, int64_t ld, int64_t n,
                                     uint8_t* out_idx_dev, float* out_norm_dev, double* out_residual_dev,
                                     int64_t ld_res, void* stream) {

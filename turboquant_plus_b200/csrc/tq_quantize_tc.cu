@@ -44,8 +44,6 @@ namespace {
 // In vectors per SM (148), so that a device with fewer SMs takes the step earlier.
 inline int64_t qt_min_vectors(bool pair) { return (int64_t)tq_num_sms() * (pair ? 166 : 1776); }
 
-__device__ int32_t qt_status;   // 1: a wait gave up
-
 struct QtJob {
   CUtensorMap map;   // of the rows: 64 elements x 128 rows a box, 128-byte swizzle
   TqFast f;
@@ -241,10 +239,25 @@ __device__ __forceinline__ void qt_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sptr(bar)) : "memory");
 }
 
+// A wait gave up: a group's tiles from the i-th of this CTA's on are not to come.  (A function of its own: inlined, it costs the kernel registers.)
+__device__ __noinline__ void qt_give_up(const TqQuantDst& dst, int i, int mine, int gtid, int64_t n, int32_t* status) {
+  const float nan = __int_as_float(0x7fffffff);
+  for (; i < mine; i += QT_GROUPS) {
+    const int64_t v = (blockIdx.x + (int64_t)i * gridDim.x) * TQ_D + gtid;
+    if (v >= n) continue;
+    bool good = true;
+    int64_t within = 0;
+    const int64_t rec = tq_dst_record(dst, v, within, good);
+    if (good && dst.scale) *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.scale) + rec + within * 4) = nan;
+    if (dst.norm) dst.norm[v] = nan;
+  }
+  if (status) *status = 1;
+}
+
 // SELFTEST: the first CTA's second tile is never reported as multiplied, and waits are short
 template <typename Tin, int BITS, bool NORMC, bool SELFTEST = false>
 __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_constant__ QtJob j0, const __grid_constant__ QtJob j1,
-                                                                         int64_t n) {
+                                                                         int64_t n, int32_t* status) {
   constexpr long long LIMIT = SELFTEST ? TC_SELFTEST_CYCLES : TC_WAIT_CYCLES;
   constexpr int IDXB = 16 * BITS, NC = 1 << BITS, HALF = NC / 2, SLOTS = QT_SLOTS, STAGES = QT_STAGES;
   extern __shared__ __align__(128) uint8_t qt_raw[];
@@ -436,15 +449,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
     }
     if (v < n && dst.norm) dst.norm[v] = nrm;
   }
-  for (; i < mine; i += QT_GROUPS) {   // a wait gave up: this tile and the group's others are not to come
-    const int64_t v = (blockIdx.x + i * step) * TQ_D + gtid;
-    bool good = v < n;
-    int64_t within = 0;
-    const int64_t rec = good ? tq_dst_record(dst, v, within, good) : 0;
-    if (good && dst.scale) *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.scale) + rec + within * 4) = __int_as_float(0x7fffffff);
-    if (v < n && dst.norm) dst.norm[v] = __int_as_float(0x7fffffff);
-    qt_status = 1;
-  }
+  if (i < mine) qt_give_up(dst, i, mine, gtid, n, status);
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -487,7 +492,7 @@ int launch_tc(const QtJob& j0, const QtJob& j1, int jobs, int64_t n, cudaStream_
   }
   const int64_t tiles = (n + TQ_D - 1) / TQ_D, places = tq_num_sms() / jobs > 0 ? tq_num_sms() / jobs : 1;
   const dim3 grid((unsigned)(tiles < places ? tiles : places), jobs);   // one CTA per SM; few tiles: one group of each
-  TQ_CUDA(tq_launch_early(kernel, grid, QT_THREADS, QT_BYTES, st, j0, j1, n));
+  TQ_CUDA(tq_launch_early(kernel, grid, QT_THREADS, QT_BYTES, st, j0, j1, n, tq_quantize_status_word()));
   return tq_launch_check("k_quantize_tc");
 }
 
@@ -535,9 +540,4 @@ int tq_quantize_tc_selftest(const TqFast& f, const void* x, const TqQuantDst& d,
   TQ_REQUIRE(f.bits == 3 && f.norm_correction && tq_aligned(x, 16) && ld % 8 == 0 && qt_map(&j.map, x, TQ_F16, ld, n), TQ_ERR_UNSUPPORTED,
              "self-test of the long append: fp16 rows of a 3-bit quantizer with norm correction");
   return launch_tc<__half, 3, true, true>(j, j, 1, n, st);
-}
-cudaError_t tq_quantize_tc_status_sync(int32_t* out) {
-  void* word = nullptr;
-  const cudaError_t e = cudaGetSymbolAddress(&word, qt_status);
-  return e == cudaSuccess ? tc_status_sync((int32_t*)word, out) : e;
 }

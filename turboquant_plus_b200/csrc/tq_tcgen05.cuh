@@ -36,12 +36,6 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
   }
   return false;
 }
-// Reads and clears a kernel's status word
-inline cudaError_t tc_status_sync(int32_t* word_dev, int32_t* out) {
-  cudaError_t e = cudaMemcpy(out, word_dev, 4, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && *out != 0) e = cudaMemset(word_dev, 0, 4);
-  return e;
-}
 
 // shared-memory matrix descriptor, no swizzle: start address, leading-dimension and stride byte offsets (16-byte
 // units), descriptor version 1.  K-major operand: LBO = distance between 8-element K chunks, SBO = distance
