@@ -79,7 +79,7 @@ typedef struct tq_quantizer_desc {
   const double* qjl_signs2;
 } tq_quantizer_desc;
 
-/* Allocates a few hundred KB of device memory on the current device and uploads the constants. */
+/* Allocates device memory on the current device (dense mode, d = 128 with a sketch: 1.3 MB) and uploads the constants. */
 int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer** out);
 int tq_quantizer_destroy(tq_quantizer* q);
 
