@@ -138,3 +138,40 @@ def test_long_packed_arrays(bits, norm_correction, width, dtype):
     for name, roundings in (("norm", 0), ("scale", 6)):
         a, b = whole[name], torch.cat([f[name] for f in few])
         assert bool((((a - b).abs() <= roundings * 2.0 ** -24 * b.abs()) | (a == b) | (a.isnan() & b.isnan())).all())
+
+
+def test_captured_by_a_new_thread():
+    """A long append whose first call in a thread is captured there."""
+    import threading
+
+    import torch
+    import turboquant_plus_b200 as tq
+    heads = 8
+    tokens = PAIR * torch.cuda.get_device_properties(0).multi_processor_count // heads + 1
+    n_pages = -(-tokens // 128)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    k, v = (torch.randn(tokens, heads, D, device="cuda", generator=gen).half() for _ in range(2))
+    slots = torch.arange(tokens, device="cuda")
+    caches = [tq.PagedKVCache(D, heads, n_pages, 128, "turbo3", "turbo3", seed=42) for _ in range(2)]
+    for cache in caches:
+        cache.pool.zero_()
+        cache.append(k[:1], v[:1], slots[:1])                       # (constants on the device)
+    torch.cuda.synchronize()
+    graph, failed = torch.cuda.CUDAGraph(), []
+
+    def work():
+        try:
+            with torch.cuda.graph(graph):
+                caches[0].append(k, v, slots)
+        except Exception as e:                                      # noqa: BLE001
+            failed.append(e)
+
+    thread = threading.Thread(target=work)
+    thread.start()
+    thread.join()
+    assert not failed, failed
+    graph.replay()
+    caches[1].append(k, v, slots)
+    torch.cuda.synchronize()
+    assert torch.equal(caches[0].pool, caches[1].pool)
+    graph.reset()
