@@ -488,7 +488,7 @@ def run_ours(args):
                                 "max_rel_deviation_from_dense": sparse_dev,
                                 "note": "TQ_DECODE_SPARSE_V: V work of a 16-token tile skipped when all its weights "
                                         "are below 1e-6 of the running maximum; an option, not the headline"},
-            "roofline_quantize": {"bound": "hbm", "kernel": "k_quantize_mma<half,3>, 2 launches of 2^22 vectors into pages",
+            "roofline_quantize": {"bound": "hbm", "kernel": "k_quantize_tc<half,3>, 2 launches of 2^22 vectors into pages",
                                   "append_one_layer_ms": append_layer_ms,
                                   "achieved": append_bytes / (append_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                                   "frac": append_bytes / (append_ms * 1e-3) / 1e9 / peak,
@@ -501,7 +501,7 @@ def run_ours(args):
             "decode_loop_us_per_layer": {"stream_order": loop.get("stream_order"), "overlap_append": loop.get("overlap_append"),
                                          "note": "per layer: quantize-on-append of one token, then decode attention over "
                                                  "ctx + 1 tokens; 40 layers, one graph, no host copies"},
-            "roofline_quantize_prod": {"bound": "hbm", "kernel": "k_quantize_mma<half,2,QJL stage> for the K rows + k_quantize_mma<half,3> for the V rows, 2^21 vectors each",
+            "roofline_quantize_prod": {"bound": "hbm", "kernel": "k_quantize_mma<half,2,QJL stage> for the K rows + k_quantize_tc<half,3> for the V rows, 2^21 vectors each",
                                        "vectors_per_s": 2 * nq32 / (appendp_ms * 1e-3),
                                        "achieved": appendp_bytes / (appendp_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                                        "frac": appendp_bytes / (appendp_ms * 1e-3) / 1e9 / peak,
@@ -786,7 +786,7 @@ def measure_config3(steps, warmup):
             "parallelism": f"KV heads sharded x{world}",
             "roofline": {"bound": "hbm", "achieved": vectors * 308 / (append_ms * 1e-3) / 1e9 / world, "peak": hbm,
                          "unit": "GB/s", "frac": vectors * 308 / (append_ms * 1e-3) / 1e9 / world / hbm,
-                         "peak_source": src, "kernel": "k_quantize_mma<half,3>", "bytes_per_vector": 308},
+                         "peak_source": src, "kernel": "k_quantize_tc<half,3>", "bytes_per_vector": 308},
             "prefill": {"ms": prefill_ms, "tflops": flops / (prefill_ms * 1e-3) / 1e12,
                         "frac_of_tensor_peak": flops / (prefill_ms * 1e-3) / 1e12 / world / tpeak, "peak": tpeak,
                         "peak_source": tsrc, "kernel": "k_prefill_attn2<3,3> (tcgen05)"},
