@@ -189,3 +189,51 @@ def test_first_large_calls():
     few = torch.cat([other.dequantize(type(code)(**{f: (getattr(code, f)[lo:lo + PIECE] if torch.is_tensor(getattr(code, f)) else getattr(code, f))
                                                      for f in code.__dataclass_fields__})) for lo in range(0, n, PIECE)])
     assert bool(((back - few).abs() <= 256 * 2.0 ** -53 * few.abs().amax(dim=1, keepdim=True)).all())
+
+
+def _next_to_boundaries(quantizer, n, seed):
+    """fp32 rows, some of whose rotated coordinates lie a relative 1e-9 to 1e-5 beside a decision boundary: one, a few or most of a row."""
+    import torch
+    rng = np.random.default_rng(seed)
+    rot, cent = quantizer.rotation, quantizer.centroids
+    bnd = (cent[1:] + cent[:-1]) / 2
+    bnd = bnd[np.abs(bnd) > 1e-6]               # (beside the centre, what fp32 rows can hold)
+    y = rng.standard_normal((n, D)) / np.sqrt(D)
+    if len(bnd):
+        near = rng.random((n, D)) < np.array([1 / D, 5 / D, 0.5])[np.arange(n) // 128 % 3][:, None]
+        at = rng.choice(bnd, (n, D)) * (1 + rng.choice([-1, 1], (n, D)) * 10.0 ** rng.uniform(-9, -5, (n, D)))
+        rest = 1 - (at ** 2 * near).sum(1)
+        near[rest < 0.1] = False
+        rest = np.where(rest < 0.1, 1, rest)
+        y *= ~near
+        y *= np.sqrt(rest / (y ** 2).sum(1))[:, None]
+        y += at * near
+    else:
+        y[:, ::7] *= 1e-8
+    x = (y @ rot) * np.exp(rng.standard_normal((n, 1)))
+    x[5] = 0
+    return torch.from_numpy(x.astype(np.float32)).cuda()
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [4737, 9601, 40000])
+def test_outputs_next_to_boundaries(n, bits):
+    """What the leading products cannot decide: by the checker, by whole rows once its list is full, and with the sketch."""
+    import torch
+    import turboquant_plus_b200 as tq
+    m, q = tq.TurboQuantMSE(D, bits, seed=6), tq.TurboQuant(D, bits + 1, seed=6)
+    x = _next_to_boundaries(m.polar_quant, n, 10 * n + bits)
+    idx, norms = m.quantize(x)
+    few = _pieces(m.quantize, x)
+    assert torch.equal(idx, few[0]) and torch.equal(norms, few[1])
+    scaled = m.polar_quant.quantize_device(x, want_scale=True)
+    parts = torch.cat([m.polar_quant.quantize_device(x[lo:lo + PIECE], want_scale=True)["scale"] for lo in range(0, n, PIECE)])
+    assert torch.equal(scaled["idx"], few[0]) and bool(((scaled["scale"] - parts).abs() <= 1.2e-7 * parts).all())
+
+    def quantize(v):
+        c = q.quantize(v)
+        return c.mse_indices, c.vector_norms, c.qjl_signs, c.residual_norms
+
+    whole, parts = quantize(x), _pieces(quantize, x)
+    assert torch.equal(whole[0], parts[0]) and torch.equal(whole[1], parts[1]) and torch.equal(whole[2], parts[2])
+    assert bool(((whole[3] - parts[3]).abs() <= 1.2e-7 * parts[3]).all())

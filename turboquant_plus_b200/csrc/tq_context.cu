@@ -85,6 +85,7 @@ struct DeviceImage {
 struct MatrixParts {
   size_t m, t, m32, t32, mp, tp;   // mp, tp: padded with zeros to dp x dp (m and t themselves when d is a multiple of 8)
   double scale;                    // d = 128: what the digits of tq_dense_i8.cu are relative to (0: it has none)
+  double rows, length;             // the largest sum of magnitudes of a row, and the longest row's length, over that
 };
 static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
   std::vector<double> t((size_t)d * d);
@@ -111,7 +112,7 @@ static MatrixParts add_matrix(DeviceImage& im, const double* m, int d) {
     p.mp = im.add(mp.data(), mp.size() * 8);
     p.tp = im.add(tp.data(), tp.size() * 8);
   }
-  p.scale = d == TQ_D ? tq_dense_digits_scale(m) : 0.0;
+  p.scale = d == TQ_D ? tq_dense_digits_scale(m, &p.rows, &p.length) : 0.0;
   p.m32 = im.add(a32.data(), a32.size() * 4);
   p.t32 = im.add(t32.data(), t32.size() * 4);
   return p;
@@ -266,9 +267,10 @@ extern "C" int tq_quantizer_create(const tq_quantizer_desc* desc, tq_quantizer**
     digits += TQ_DENSE_DIGITS_BYTES;
     return at;
   };
-  if (mr.scale != 0.0) q->dig.r = digits_place(), q->dig.rt = digits_place(), q->dig.r_scale = mr.scale;
+  if (mr.scale != 0.0) q->dig.r = digits_place(), q->dig.rt = digits_place(), q->dig.r_scale = mr.scale, q->dig.r_rows = mr.rows, q->dig.r_length = mr.length;
   if (ms.scale != 0.0) q->dig.s = digits_place(), q->dig.st = digits_place(), q->dig.s_scale = ms.scale;
   q->dig.cent_scale = tq_dense_digits_centroids(c.data(), nc);
+  if (q->dig.cent_scale != 0.0) tq_dense_digits_words(c.data(), nc, q->dig.cent_scale, q->dig.words);
   for (size_t i = 0; i < b.size(); ++i) q->dig.bnd[i] = b[i];
   q->cent64 = f64(cent_at);
   q->bnd64 = f64(bnd_at);

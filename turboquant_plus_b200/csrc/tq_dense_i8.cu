@@ -8,27 +8,36 @@
 // the largest value and the products left out (s >= 8) together are off by 1.0e-16 of the result's norm (random rotation, rows
 // with outlier channels), fp64 sums of 128 terms by 4.9e-16.
 //
+// What only decides something -- an index, a sign of the sketch -- needs fewer: the leading ten (indices) to 21 products (the sketch) leave a known
+// bound out, and what lies within it of a boundary is decided in fp64 (di_index, di_checker, di_rows_plain).  A residual is taken from 21
+// products.  Reconstructions are results themselves and take all 34.
+//
 // One persistent CTA per SM, 128 vectors a tile:
 //   warps 0-15 rows: warps w, w + 4, w + 8 and w + 12 share the 32 vectors that are lanes 32 (w & 3) .. of tensor memory, a thread
 //              32 columns of a vector (64 in eight warps: their loads of sums waited behind the MMAs' own traffic).  They norm
-//              the rows (in NumPy's order), write the digits of the first operand into tensor memory (7 x 32 columns, four
-//              digits a word) and add up the sums of its product with R: indices, whose centroids' digits are the next
+//              the rows (in NumPy's order), write the digits of the first operand into tensor memory (32 columns a digit, four
+//              elements a word) and add up the sums of its product with R: indices, whose centroids' digits are the next
 //              operand; then, with the sketch, the residual's digits, and the signs.
-//   warp 16    bulk copies of the matrices' digits, 16 KB each (laid out by k_dense_digits).  The sums run from s = 7 to 0, so that
-//              digit s of a matrix has been read for the last time after sum s, and the next matrix follows it.
+//   warp 16    bulk copies of the matrices' digits, 16 KB each (laid out by k_dense_digits).  The sums run from the last to 0, so that
+//              digit s of a matrix has been read for the last time after sum s, and the next matrix follows it.  A single matrix stays; the
+//              warp then looks after the outputs that are too close to a boundary.
 //   warp 17    every MMA: one s of all 128 outputs is an accumulator of 128 columns, of which two take turns.
 // Shapes by measurement: an MMA of 128 x N x 32 takes 44 clocks (its issue) for N = 32 and 64, 65 for N = 128.
 //
-// What bounds it: a product takes 18,600 clocks where its 136 MMAs take 8,800.  The rows' loads of sums (700 clocks each under
-// MMAs, 120 without) and their fp64 additions, eight of each of 128 x 128 sums, run between the MMAs rather than under them.
-// 65,536 fp32 vectors, before (fp64 tensor cores) / now: quantize 134 / 77 us, with the sketch 302 / 182, dequantize 90 / 63 and 164 / 93.
+// What bounds quantize: its rows' arithmetic, 12,000 clocks a tile without the sketch (norms 1,300, digits 2,100, sums 4,000, indices 2,600, the rest
+// barriers and stores) and 40,000 with it (sums 20,000, of which the MMAs take 13,000; residuals 7,000).  65,536 fp32 vectors, fp64
+// tensor cores / all 34 products each / here: 134 / 78 / 33 us, with the sketch 302 / 163 / 90 (105 where a row on a CTA's way is for
+// di_rows_plain, 14 us; about every second call).
+// What bounds dequantize: its rows.  A tile's 136 MMAs take 8,800 clocks, the rows' loads of sums (700 clocks each under MMAs, 120 without) and
+// their fp64 additions run between the MMAs rather than under them.  65,536 vectors, fp64 tensor cores / here: 90 / 62 us, with the sketch 164 / 93.
 //
 // A wait that gives up ends the waits of all roles; the results of its tile and of those behind it are then not numbers, and a
 // status word is set (tq_quantize_status_sync).
 //
 // A row that this arithmetic does not carry -- values that are not finite or too small for a norm, residuals far beyond the
-// vector's length, which an arbitrary matrix can produce -- is computed by one warp in plain fp64.
+// vector's length, which an arbitrary matrix can produce -- is computed by all row threads in plain fp64.
 #include <mutex>
+#include <type_traits>
 #include "tq_tcgen05.cuh"
 
 namespace {
@@ -79,15 +88,6 @@ __device__ __forceinline__ void di_st2(uint32_t addr, uint32_t a, uint32_t b) {
 // value x 2^54 as balanced base-256 digits: byte 6 the leading one (signed), bytes 5..0 the others
 __device__ __forceinline__ uint64_t di_digits(long long w) { return (uint64_t)(w + 0x808080808080ll) ^ 0x808080808080ull; }
 __device__ __forceinline__ uint2 di_split(uint64_t u) { return make_uint2((uint32_t)u, (uint32_t)(u >> 32)); }
-// the digits of an fp32 value below 2 in magnitude, from its bits: significand x 2^(exponent - 96); what a value below 2^-31 has
-// beyond 2^-54 is cut off
-__device__ __forceinline__ uint2 di_digits_f32(float v) {
-  const uint32_t u = __float_as_uint(v), e = (u >> 23) & 255u, m = (u & 0x7fffffu) | (e ? 0x800000u : 0u);
-  const uint32_t lo = e >= 96u ? m << ((e - 96u) & 31u) : e > 64u ? m >> (96u - e) : 0u, hi = e >= 96u ? __funnelshift_l(m, 0u, e - 96u) : 0u;
-  const uint32_t neg = (uint32_t)((int)u >> 31);
-  const uint64_t w = (((uint64_t)(hi ^ neg) << 32) | (lo ^ neg)) + (0x808080808080ull + (neg & 1u));   // -x = ~x + 1
-  return make_uint2((uint32_t)w ^ 0x80808080u, (uint32_t)(w >> 32) ^ 0x8080u);
-}
 // of an fp64 value below 2 in magnitude: to a whole number of 2^-54 in two steps of a large constant's rounding
 __device__ __forceinline__ uint2 di_digits_f64(double v) {
   constexpr double BIG = 6755399441055744.0;                            // 1.5 x 2^52: a sum's low bits are the whole number
@@ -97,25 +97,33 @@ __device__ __forceinline__ uint2 di_digits_f64(double v) {
   const long long w = (__double_as_longlong(lo) - __double_as_longlong(BIG)) + ((long long)__double2loint(hi) << 32);
   return di_split(di_digits(w));
 }
-// digits of eight consecutive elements -> the seven operand words of each four of them, stored at column `col` of every digit
-__device__ __forceinline__ void di_store8(uint32_t area, int col, const uint2 (&u)[8]) {
-  uint32_t w[DI_DIGITS][2];
+// byte k of four words -> operand word k of the four elements
+__device__ __forceinline__ void di_transpose(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&w)[4]) {
+  const uint32_t ab = __byte_perm(a, b, 0x5140), cd = __byte_perm(c, d, 0x5140);
+  const uint32_t ab2 = __byte_perm(a, b, 0x7362), cd2 = __byte_perm(c, d, 0x7362);
+  w[0] = __byte_perm(ab, cd, 0x5410);
+  w[1] = __byte_perm(ab, cd, 0x7632);
+  w[2] = __byte_perm(ab2, cd2, 0x5410);
+  w[3] = __byte_perm(ab2, cd2, 0x7632);
+}
+// digits of eight consecutive elements -> the operand words of each four of them, the leading COUNT digits, stored at column `col`
+// of every digit.  LOW: the byte of the last digit (its low bytes are those of x, the next of y)
+template <int COUNT, int LOW> __device__ __forceinline__ void di_store8(uint32_t area, int col, const uint2 (&u)[8]) {
+  uint32_t w[COUNT][2];
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
     const uint2 a = u[4 * g], b = u[4 * g + 1], c = u[4 * g + 2], d = u[4 * g + 3];
-    const uint32_t ab = __byte_perm(a.x, b.x, 0x5140), cd = __byte_perm(c.x, d.x, 0x5140);
-    const uint32_t ab2 = __byte_perm(a.x, b.x, 0x7362), cd2 = __byte_perm(c.x, d.x, 0x7362);
-    const uint32_t hab = __byte_perm(a.y, b.y, 0x5140), hcd = __byte_perm(c.y, d.y, 0x5140);
-    w[6][g] = __byte_perm(ab, cd, 0x5410);
-    w[5][g] = __byte_perm(ab, cd, 0x7632);
-    w[4][g] = __byte_perm(ab2, cd2, 0x5410);
-    w[3][g] = __byte_perm(ab2, cd2, 0x7632);
-    w[2][g] = __byte_perm(hab, hcd, 0x5410);
-    w[1][g] = __byte_perm(hab, hcd, 0x7632);
-    w[0][g] = __byte_perm(__byte_perm(a.y, b.y, 0x0062), __byte_perm(c.y, d.y, 0x0062), 0x5410);
+    uint32_t lo[4], hi[4];
+    di_transpose(a.x, b.x, c.x, d.x, lo);
+    di_transpose(a.y, b.y, c.y, d.y, hi);
+#pragma unroll
+    for (int p = 0; p < COUNT; ++p) {
+      const int byte = LOW + COUNT - 1 - p;
+      w[p][g] = byte < 4 ? lo[byte & 3] : hi[byte & 3];
+    }
   }
 #pragma unroll
-  for (int p = 0; p < DI_DIGITS; ++p) di_st2(area + 32 * p + col, w[p][0], w[p][1]);
+  for (int p = 0; p < COUNT; ++p) di_st2(area + 32 * p + col, w[p][0], w[p][1]);
 }
 
 // int32 -> double: 2^52 + 2^31 + v has v ^ 0x80000000 in its low word
@@ -127,8 +135,8 @@ struct DiShared {
   uint32_t tmem;
   volatile int failed;   // a wait gave up: nobody waits any more
 };
-// SELFTEST: waits are short, and one accumulator of the first CTA's second tile is never reported as full (di_issue)
-template <bool SELFTEST> __device__ __forceinline__ void di_wait(DiShared& s, uint64_t* bar, uint32_t parity) {
+// SELFTEST: 0, or the product sum of the first CTA that is never reported (di_issue), one of its second tile; waits are short then
+template <int SELFTEST> __device__ __forceinline__ void di_wait(DiShared& s, uint64_t* bar, uint32_t parity) {
   tc_wait(bar, parity, &s.failed, SELFTEST ? TC_SELFTEST_CYCLES : TC_WAIT_CYCLES);
 }
 __device__ __forceinline__ void di_init(DiShared& s) {
@@ -153,50 +161,51 @@ __device__ __forceinline__ bool di_rows_any(bool p) {
   return any != 0;
 }
 
-// The copier's way: the digits of the matrices that `matrix(i)` gives, each into the place of the matrix before
-template <bool SELFTEST, typename M> __device__ __forceinline__ void di_copier(DiShared& s, uint8_t* tiles, int count, M&& matrix) {
-  int copies = 0;
-  for (int i = 0; i < count && !s.failed; ++i) {
+// The copier's way: the digits of the matrices that `matrix(i)` gives, the leading count(i) of each, from the last to the first, each
+// into the place of the matrix before.  uses(i, p): how many of the matrices before i had a digit p
+template <int SELFTEST, typename M, typename C, typename U>
+__device__ __forceinline__ void di_copier(DiShared& s, uint8_t* tiles, int matrices, M&& matrix, C&& count, U&& uses) {
+  int i = 0, p = 0;
+  for (; i < matrices && !s.failed; ++i) {
     const uint8_t* src = matrix(i);
-    for (int p = DI_DIGITS - 1; p >= 0; --p, ++copies) {
-      if (i > 0) di_wait<SELFTEST>(s, &s.b_free[p], (uint32_t)((i - 1) & 1));
+    for (p = count(i) - 1; p >= 0; --p) {
+      const int before = uses(i, p);
+      if (before > 0) di_wait<SELFTEST>(s, &s.b_free[p], (uint32_t)((before - 1) & 1));
       if (s.failed) break;
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sptr(&s.b_full[p])), "r"(DI_TILE) : "memory");
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sptr(tiles + p * DI_TILE)),
                    "l"(src + p * DI_TILE), "r"(DI_TILE), "r"(sptr(&s.b_full[p])) : "memory");
     }
+    if (p >= 0) break;   // (a wait gave up in front of digit p)
   }
-  for (int p = 0; p < DI_DIGITS; ++p) {   // none in flight at the end, also after a wait that gave up
-    const int mine = (copies + p) / DI_DIGITS;
-    if (mine > 0) tc_wait(&s.b_full[p], (uint32_t)((mine - 1) & 1));
+  for (int q = 0; q < DI_DIGITS; ++q) {   // none in flight at the end, also after a wait that gave up
+    const int mine = uses(i, q) + (i < matrices && p >= 0 && q > p && q < count(i) ? 1 : 0);
+    if (mine > 0) tc_wait(&s.b_full[q], (uint32_t)((mine - 1) & 1));
   }
 }
 
-// The MMA warp: the operand at `area`, of DIGITS digits, against the `matrix`-th matrix; s from the last to the first
-template <int DIGITS, bool SELFTEST>
-__device__ __forceinline__ void di_issue(DiShared& s, int& item, const uint8_t* tiles, int matrix, uint32_t area, uint32_t acc_base) {
-  constexpr int TOP = DI_DIGITS - 1, LAST = DIGITS == 1 ? TOP : DI_SUMS - 1;
+// The MMA warp: the operand at `area`, of PA digits, against the leading QB digits of a matrix, sums s = LAST to 0 of the products of
+// digits p + q = s.  uses(q): the matrices before that had a digit q
+template <int PA, int QB, int LAST, int SELFTEST, typename U>
+__device__ __forceinline__ void di_issue(DiShared& s, int& item, const uint8_t* tiles, U&& uses, uint32_t area, uint32_t acc_base) {
   const uint32_t b = sptr(tiles), idesc = di_idesc();
-#pragma unroll
+#pragma unroll 1
   for (int sum = LAST; sum >= 0; --sum, ++item) {
     const int sl = item & 1;
+    if (sum == LAST)
+      for (int q = 0; q < QB; ++q) di_wait<SELFTEST>(s, &s.b_full[q], (uint32_t)(uses(q) & 1));
     if (item >= 2) di_wait<SELFTEST>(s, &s.d_free[sl], (uint32_t)((item / 2 - 1) & 1));
-#pragma unroll
-    for (int q = 0; q < DI_DIGITS; ++q)   // digits used for the first time
-      if (DIGITS == 1 ? q == sum : sum == LAST ? q > 0 : sum == LAST - 1 && q == 0) di_wait<SELFTEST>(s, &s.b_full[q], (uint32_t)(matrix & 1));
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int from = sum < QB ? 0 : sum - QB + 1, to = sum < PA ? sum : PA - 1;
+#pragma unroll 1
+    for (int p = from; p <= to; ++p) {
+      const uint64_t desc = umma_desc(b + (sum - p) * DI_TILE, 128, 1024);
 #pragma unroll
-    for (int p = 0; p < DIGITS; ++p) {
-      const int q = sum - p;
-      if (q < 0 || q > TOP) continue;
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        di_mma(acc_base + 128 * sl, area + 32 * p + 8 * ks, umma_desc(b + q * DI_TILE + ks * 256, 128, 1024), idesc,
-               p == (sum > TOP ? sum - TOP : 0) && ks == 0 ? 0u : 1u);
+      for (int ks = 0; ks < 4; ++ks) di_mma(acc_base + 128 * sl, area + 32 * p + 8 * ks, desc + 16 * ks, idesc, p > from || ks > 0 ? 1u : 0u);
     }
-    if (!(SELFTEST && blockIdx.x == 0 && item == 26)) di_commit(&s.d_full[sl]);   // (a tile with a sketch: 24 items, 15 to dequantize)
-    if (sum < DI_DIGITS) di_commit(&s.b_free[sum]);
+    if (!(SELFTEST && blockIdx.x == 0 && item == SELFTEST)) di_commit(&s.d_full[sl]);
+    if (sum < QB) di_commit(&s.b_free[sum]);
   }
 }
 
@@ -208,35 +217,83 @@ __device__ __forceinline__ void di_drain(DiShared& s) {
   tc_wait(&s.drained, 0);
 }
 
-// A row warp: acc += base x (the product's sums, 256^-s each), 32 columns of a thread
-template <int DIGITS, bool SELFTEST>
+// A row warp waits for a sum, use(column, value) for its 32 columns; frees the accumulator once all are loaded
+template <int SELFTEST, typename U>
+__device__ __forceinline__ void di_columns(DiShared& s, int item, uint32_t acc_base, int lane, U&& use) {
+  const int sl = item & 1;
+  di_wait<SELFTEST>(s, &s.d_full[sl], (uint32_t)((item / 2) & 1));
+  __syncwarp();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  uint32_t v[2][8];
+  di_ld8(acc_base + 128 * sl, v[0]);
+#pragma unroll
+  for (int c = 0; c < DI_COLS / 8; ++c) {
+    di_ld8_wait(v[c & 1]);
+    if (c + 1 < DI_COLS / 8) {
+      di_ld8(acc_base + 128 * sl + 8 * (c + 1), v[(c + 1) & 1]);
+    } else {   // all read
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) di_arrive(&s.d_free[sl]);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) use(8 * c + k, v[c & 1][k]);
+  }
+}
+// The same with all columns at once
+template <int SELFTEST>
+__device__ __forceinline__ void di_sum(DiShared& s, int& item, uint32_t acc_base, int lane, uint32_t (&v)[32]) {
+  const int sl = item & 1;
+  di_wait<SELFTEST>(s, &s.d_full[sl], (uint32_t)((item / 2) & 1));
+  __syncwarp();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  tmem_ld32(acc_base + 128 * sl, v);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) di_arrive(&s.d_free[sl]);
+  ++item;
+}
+// The product's sums s = LAST to 0 (s counts 2^(-12 - 8 s)) as a number of 2^(shift - 44), shift = 15 or 17; what is below is cut off each
+// time.  Sums wrap, the result is in range
+template <int LAST, int SELFTEST>
+__device__ __forceinline__ void di_take32(DiShared& s, int& item, uint32_t acc_base, int lane, int shift, int32_t (&y)[DI_COLS]) {
+#pragma unroll
+  for (int sum = LAST; sum >= 0; --sum) {
+    uint32_t v[32];
+    di_sum<SELFTEST>(s, item, acc_base, lane, v);
+    const int right = sum == 2 ? shift - 14 : shift - 32 + 8 * sum;
+    const uint32_t left = 1u << (32 - 8 * sum - shift & 31);
+#pragma unroll
+    for (int k = 0; k < DI_COLS; ++k) {
+      if (sum >= 2) y[k] = (sum == LAST ? 0 : y[k]) + ((sum == 2 ? (int32_t)(v[k] << 2) : (int32_t)v[k]) >> right);
+      else y[k] = (int32_t)((uint32_t)y[k] + v[k] * left);
+    }
+  }
+}
+// The product's sums s = 5 to 0 as a number of 2^-44; of s = 5 what is nearest.  (A loop: unrolled, registers spill)
+template <int SELFTEST>
+__device__ __forceinline__ void di_take64(DiShared& s, int& item, uint32_t acc_base, int lane, long long (&y)[DI_COLS]) {
+  di_columns<SELFTEST>(s, item++, acc_base, lane, [&](int k, uint32_t v) { y[k] = ((int32_t)v + 128) >> 8; });
+  int32_t weight = 1;
+#pragma unroll 1
+  for (int sum = 4; sum > 0; --sum, weight <<= 8)
+    di_columns<SELFTEST>(s, item++, acc_base, lane, [&](int k, uint32_t v) { y[k] += (long long)(int32_t)v * weight; });
+  di_columns<SELFTEST>(s, item++, acc_base, lane, [&](int k, uint32_t v) { y[k] += (long long)((unsigned long long)v << 32); });
+}
+// A whole number below 2^51 in magnitude as fp64
+__device__ __forceinline__ double di_double(long long v) {
+  return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
+}
+
+// acc += base x (the product's sums, 256^-s each)
+template <int LAST, int SELFTEST>
 __device__ __forceinline__ void di_take(DiShared& s, int& item, uint32_t acc_base, int lane, double base, double (&acc)[DI_COLS]) {
-  constexpr int LAST = DIGITS == 1 ? DI_DIGITS - 1 : DI_SUMS - 1;
   double factor = base;
 #pragma unroll
   for (int i = 0; i < LAST; ++i) factor *= 0.00390625;
 #pragma unroll 1
-  for (int sum = LAST; sum >= 0; --sum, ++item, factor *= 256.0) {
-    const int sl = item & 1;
-    di_wait<SELFTEST>(s, &s.d_full[sl], (uint32_t)((item / 2) & 1));
-    __syncwarp();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    uint32_t v[2][8];
-    di_ld8(acc_base + 128 * sl, v[0]);
-#pragma unroll
-    for (int c = 0; c < DI_COLS / 8; ++c) {
-      di_ld8_wait(v[c & 1]);
-      if (c + 1 < DI_COLS / 8) {
-        di_ld8(acc_base + 128 * sl + 8 * (c + 1), v[(c + 1) & 1]);
-      } else {   // all read
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) di_arrive(&s.d_free[sl]);
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc[8 * c + k] = fma(di_double(v[c & 1][k]), factor, acc[8 * c + k]);
-    }
-  }
+  for (int sum = LAST; sum >= 0; --sum, ++item, factor *= 256.0)
+    di_columns<SELFTEST>(s, item, acc_base, lane, [&](int k, uint32_t v) { acc[k] = fma(di_double(v), factor, acc[k]); });
 }
 __device__ __forceinline__ void di_zero(double (&acc)[DI_COLS]) {
 #pragma unroll
@@ -261,9 +318,15 @@ template <typename T> __device__ __forceinline__ void di_load8(const uint8_t* p,
 
 struct DiQuant {
   const uint8_t *r, *rt, *s;          // digits of R, R^T and S (k_dense_digits)
-  double r_scale;                     // R w = sums x this
+  double r_scale;                     // sums x this: R w
   double cent_scale;                  // power of two above every centroid's magnitude
-  double bnd[15];                     // boundaries (parameters: operands of the comparisons as they are)
+  uint2 words[DI_DIGITS];             // digits of the first eight centroids (di_store_codes)
+  int32_t thr[15];                    // boundaries over r_scale, as numbers of 2^-27 or 2^-29
+  uint32_t near;                      // an output that is closer to one is decided in fp64
+  float step, offset[15];             // the same without the sketch (di_index_float)
+  int32_t zero_idx;                   // index of the value 0
+  int32_t shift;                      // sums of 2^-44 to numbers of the boundaries
+  double slack;                       // of a projection, per unit of the reconstruction's factor (di_quant_args)
   int32_t* status;                    // raised when a wait gives up
   TqDenseQuant q;
 };
@@ -274,66 +337,89 @@ struct DiDequant {
   TqDenseDequant q;
 };
 
-// A whole row in fp64, by one warp (four outputs a lane)
-template <typename Tin>
-__device__ void di_row_plain(const TqDenseQuant& a, const uint8_t* xrow, float nrm, int64_t v, int lane) {
-  const Tin* x = reinterpret_cast<const Tin*>(xrow);
-  const float safe = nrm > 0.f ? nrm : 1.0f;
-  const int nb = (1 << a.bits) - 1;
-  double y[4] = {0, 0, 0, 0};
-  for (int k = 0; k < TQ_D; ++k) {
-    const double w = (double)(di_f<Tin>(x[k]) / safe);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) y[j] = fma(a.rot[(size_t)(4 * lane + j) * TQ_D + k], w, y[j]);
-  }
-  int m[4];
-  double cc = 0.0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    m[j] = 0;
-    for (int b = 0; b < nb; ++b) m[j] += a.bnd[b] < y[j] ? 1 : 0;
-    cc += a.cent[m[j]] * a.cent[m[j]];
-    if (a.out_idx) a.out_idx[v * TQ_D + 4 * lane + j] = (uint8_t)m[j];
-  }
-#pragma unroll
-  for (int h = 16; h > 0; h >>= 1) cc += __shfl_xor_sync(0xffffffffu, cc, h);
-  double cn = sqrt(cc);
-  cn = cn > 1e-10 ? cn : 1.0;
-  if (lane == 0) {
-    if (a.out_norm) a.out_norm[v] = nrm;
-    if (a.out_scale) a.out_scale[v] = (float)(a.norm_correction ? (double)nrm / cn : (double)nrm);
-  }
-  if (!a.out_qjl && !a.out_rnorm) return;
-  const double inv = a.norm_correction ? 1.0 / cn : 1.0;
-  double e[4] = {0, 0, 0, 0}, rr = 0.0;
-  for (int k = 0; k < TQ_D; ++k) {
-    const int mk = __shfl_sync(0xffffffffu, (k & 2) ? ((k & 1) ? m[3] : m[2]) : ((k & 1) ? m[1] : m[0]), k >> 2);
-    const double c = a.cent[mk] * inv;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) e[j] = fma(a.rot_t[(size_t)(4 * lane + j) * TQ_D + k], c, e[j]);
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    e[j] = (double)di_f<Tin>(x[4 * lane + j]) - e[j] * (double)nrm;
-    rr += e[j] * e[j];
-  }
-#pragma unroll
-  for (int h = 16; h > 0; h >>= 1) rr += __shfl_xor_sync(0xffffffffu, rr, h);
-  if (lane == 0 && a.out_rnorm) a.out_rnorm[v] = (float)sqrt(rr);
-  if (!a.out_qjl) return;
-  double p[4] = {0, 0, 0, 0};
-  for (int k = 0; k < TQ_D; ++k) {
-    const double ek = __shfl_sync(0xffffffffu, (k & 2) ? ((k & 1) ? e[3] : e[2]) : ((k & 1) ? e[1] : e[0]), k >> 2);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = fma(a.s[(size_t)(4 * lane + j) * TQ_D + k], ek, p[j]);
-  }
-  uint32_t nib = 0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) nib = (nib << 1) | (p[j] < 0.0 ? 0u : 1u);
-  const uint32_t up = __shfl_down_sync(0xffffffffu, nib, 1);
-  if ((lane & 1) == 0) a.out_qjl[v * 16 + (lane >> 1)] = (uint8_t)((nib << 4) | up);
+// Centroids and boundaries in shared memory
+struct DiCodes {
+  double cent[16], bnd[16], square[64];   // square: of the centroids of two indices, the sum (3 bits at most), else of one
+};
+__device__ __forceinline__ int di_search(const DiCodes& c, int bits, double y) {   // boundaries below y (searchsorted, side = 'left')
+  int m = 0;
+#pragma unroll 1
+  for (int b = 0; b < (1 << bits) - 1; ++b) m += c.bnd[b] < y ? 1 : 0;
+  return m;
 }
-
+// Whole rows in fp64, one after the other, by all row threads: a warp multiplies eight elements of a vector with their rows of a matrix, all
+// loads in flight, and thread j < 128 adds up output j.  (A warp per row waited for one load after the other: 75 us a row.)
+struct DiPlain {
+  double part[DI_ROW_THREADS / 32][TQ_D], v[TQ_D], sum[4];
+};
+__device__ __forceinline__ double di_plain_product(DiPlain& s, const double* __restrict__ m, int tid) {   // of s.v; thread j < 128: output j
+  const int lane = tid & 31, warp = tid >> 5;
+  di_rows_sync();
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  double2 r[8][2];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const double2* at = reinterpret_cast<const double2*>(m + (size_t)(8 * warp + k) * TQ_D + 4 * lane);
+    r[k][0] = __ldg(at);
+    r[k][1] = __ldg(at + 1);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const double vk = s.v[8 * warp + k];
+    acc[0] = fma(r[k][0].x, vk, acc[0]);
+    acc[1] = fma(r[k][0].y, vk, acc[1]);
+    acc[2] = fma(r[k][1].x, vk, acc[2]);
+    acc[3] = fma(r[k][1].y, vk, acc[3]);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s.part[warp][4 * lane + j] = acc[j];
+  di_rows_sync();
+  double y = 0.0;
+  if (tid < TQ_D)
+#pragma unroll 4
+    for (int w = 0; w < DI_ROW_THREADS / 32; ++w) y += s.part[w][tid];
+  return y;
+}
+__device__ __forceinline__ double di_plain_sum(DiPlain& s, double x, int tid) {   // over the first 128 threads
+#pragma unroll
+  for (int h = 16; h > 0; h >>= 1) x += __shfl_xor_sync(0xffffffffu, x, h);
+  if (tid < TQ_D && (tid & 31) == 0) s.sum[tid >> 5] = x;
+  di_rows_sync();
+  return (s.sum[0] + s.sum[1]) + (s.sum[2] + s.sum[3]);
+}
+template <typename Tin>
+__device__ __noinline__ void di_rows_plain(DiPlain& s, const TqDenseQuant& a, const DiCodes& c, const uint8_t* plain, const float* norms, const Tin* x,
+                                           int64_t ld, int64_t v0, int64_t n, int tid) {
+#pragma unroll 1
+  for (int row = 0; row < DI_ROWS; ++row) {
+    const int64_t v = v0 + row;
+    if (!plain[row] || v >= n) continue;
+    const float nrm = norms[row], safe = nrm > 0.f ? nrm : 1.0f;
+    const double f = tid < TQ_D ? (double)di_f<Tin>(x[v * ld + tid]) : 0.0;
+    if (tid < TQ_D) s.v[tid] = (double)((float)f / safe);
+    const double y = di_plain_product(s, a.rot_t, tid);
+    const int m = di_search(c, a.bits, y);
+    if (tid < TQ_D && a.out_idx) a.out_idx[v * TQ_D + tid] = (uint8_t)m;
+    double cn = sqrt(di_plain_sum(s, tid < TQ_D ? c.cent[m] * c.cent[m] : 0.0, tid));
+    cn = cn > 1e-10 ? cn : 1.0;
+    if (tid == 0) {
+      if (a.out_norm) a.out_norm[v] = nrm;
+      if (a.out_scale) a.out_scale[v] = (float)(a.norm_correction ? (double)nrm / cn : (double)nrm);
+    }
+    if (a.out_qjl || a.out_rnorm) {
+      if (tid < TQ_D) s.v[tid] = a.norm_correction ? c.cent[m] * (1.0 / cn) : c.cent[m];
+      const double e = f - di_plain_product(s, a.rot, tid) * (double)nrm;
+      const double rr = di_plain_sum(s, tid < TQ_D ? e * e : 0.0, tid);
+      if (tid == 0 && a.out_rnorm) a.out_rnorm[v] = (float)sqrt(rr);
+      if (a.out_qjl) {
+        if (tid < TQ_D) s.v[tid] = e;
+        const uint32_t z = __brev(__ballot_sync(0xffffffffu, !(di_plain_product(s, a.s_t, tid) < 0.0)));   // (first output in the most significant bit)
+        if (tid < TQ_D && (tid & 7) == 0) a.out_qjl[v * 16 + (tid >> 3)] = (uint8_t)(z >> (24 - (tid & 24)));
+      }
+    }
+    di_rows_sync();
+  }
+}
 template <typename T> __device__ __forceinline__ T di_from(double v) { return (T)v; }
 template <> __device__ __forceinline__ __half di_from<__half>(double v) { return __float2half_rn((float)v); }
 // A wait gave up: the results of this CTA's tiles from `t` on are not to come.  (Functions of their own: inlined, they cost the kernels registers.)
@@ -357,28 +443,154 @@ template <typename Tout> __device__ __noinline__ void di_give_up(const TqDenseDe
 }
 
 template <typename Tin> constexpr int di_row_bytes() { return TQ_D * (int)sizeof(Tin) + 16; }   // (rows 4 banks apart: no conflicts)
-template <typename Tin> constexpr int di_quant_smem() { return DI_DIGITS * DI_TILE + DI_ROWS * di_row_bytes<Tin>() + 128; }
+// digits of a matrix in shared memory: of R in place for all tiles, or of R, R^T and S in turn
+template <bool PROD> constexpr int di_quant_digits() { return PROD ? 6 : 4; }
+template <typename Tin, bool PROD> constexpr int di_quant_smem() {
+  return di_quant_digits<PROD>() * DI_TILE + DI_ROWS * di_row_bytes<Tin>() + 128 + (int)sizeof(DiPlain);
+}
 
-// PROD: residual, its norm and the sketch as well
-template <typename Tin, int BITS, bool PROD, bool SELFTEST = false>
+// Operand words of four indices below 8 (one a byte): a byte permute of eight digits picks a digit of all four.  words[p]: the digit p of
+// centroids 0-3, 4-7
+template <int COUNT> __device__ __forceinline__ void di_store_codes(uint32_t area, int col, const uint2 (&words)[DI_DIGITS], uint32_t q0, uint32_t q1) {
+  const uint32_t s0 = __byte_perm(q0 | (q0 >> 4), 0, 0x4420), s1 = __byte_perm(q1 | (q1 >> 4), 0, 0x4420);
+#pragma unroll
+  for (int p = 0; p < COUNT; ++p) di_st2(area + 32 * p + col, __byte_perm(words[p].x, words[p].y, s0), __byte_perm(words[p].x, words[p].y, s1));
+}
+
+// R, R^T and S with 5, 6 and 6 digits, in turn: those among the first i matrices that have a digit p
+__device__ __forceinline__ int di_uses(int i, int p) { return p < 5 ? i : p == 5 ? i - (i + 2) / 3 : 0; }
+
+// Index of y: the boundaries below it, found bit by bit; near: the least distance of y + reach above one of those compared (the two
+// next to y are among them), as an unsigned number: at most 2 `reach` if y is within `reach` of one
+template <int BITS> __device__ __forceinline__ uint32_t di_index(const int32_t (&thr)[15], uint32_t reach, int32_t y, uint32_t& near) {
+  const uint32_t yn = (uint32_t)y + reach;
+  auto above = [&](int32_t t) {
+    near = min(near, yn - (uint32_t)t);
+    return y > t;
+  };
+  if constexpr (BITS == 1) {
+    return above(thr[0]) ? 1u : 0u;
+  } else if constexpr (BITS == 2) {
+    const bool b1 = above(thr[1]), b0 = above(b1 ? thr[2] : thr[0]);
+    return (b1 ? 2u : 0u) + (b0 ? 1u : 0u);
+  } else if constexpr (BITS == 3) {
+    const bool b2 = above(thr[3]), b1 = above(b2 ? thr[5] : thr[1]), b0 = above(b2 ? (b1 ? thr[6] : thr[4]) : (b1 ? thr[2] : thr[0]));
+    return (b2 ? 4u : 0u) + (b1 ? 2u : 0u) + (b0 ? 1u : 0u);
+  } else {
+    const bool b3 = above(thr[7]), b2 = above(b3 ? thr[11] : thr[3]);
+    const bool b1 = above(b3 ? (b2 ? thr[13] : thr[9]) : (b2 ? thr[5] : thr[1]));
+    const bool b0 = above(b3 ? (b2 ? (b1 ? thr[14] : thr[12]) : (b1 ? thr[10] : thr[8])) : (b2 ? (b1 ? thr[6] : thr[4]) : (b1 ? thr[2] : thr[0])));
+    return (b3 ? 8u : 0u) + (b2 ? 4u : 0u) + (b1 ? 2u : 0u) + (b0 ? 1u : 0u);
+  }
+}
+
+// The same on the fp32 pipe: a boundary is a ramp from 0 to 1 over the values too close to it, the index the ramps' sum, in the low byte
+// of the result; frac, at most 1/2: how far from a whole number.  Integer compares and selects, at half the rate, took 4,600 clocks of a
+// tile's 14,300 with eight centroids.
+template <int BITS> __device__ __forceinline__ uint32_t di_index_float(const DiQuant& A, int32_t y, float& frac) {
+  const float z = (float)y;
+  float m = 0.f;
+#pragma unroll
+  for (int b = 0; b < (1 << BITS) - 1; ++b) {
+    const float ramp = __saturatef(fmaf(z, A.step, A.offset[b]));
+    m = b == 0 ? ramp : m + ramp;
+  }
+  const float whole = m + 12582912.f;                          // 1.5 x 2^23
+  frac = fmaxf(frac, fabsf(m - (whole - 12582912.f)));
+  return __float_as_uint(whole);
+}
+
+// Outputs that are too close to a boundary, eight neighbouring columns an entry: the row warps add them once the indices are stored, the
+// copier's warp, which has nothing else to do by then, decides them in fp64.  (By the row warps themselves, whose code for it is not in the
+// instruction caches, a check cost 3 to 4 us, and some CTA of a large call had several.)
+struct DiList {
+  static constexpr int ROOM = 256;
+  static constexpr uint32_t NONE = 0xffffffffu;
+  volatile uint32_t entry[ROOM];   // row, column / 8 from bit 7, tile of the CTA from bit 11 on; written last
+  float norm[ROOM];
+  int count;                       // entries, and those that found no room: their rows are for di_rows_plain
+  volatile int closed;             // no more to come
+};
+// Indices of eight outputs of a row in fp64, by one warp: four lanes a column, 32 elements each, every load in flight
+template <typename Tin>
+__device__ __forceinline__ int di_check8(const TqDenseQuant& a, const DiCodes& c, const Tin* x, float nrm, int column, int lane) {
+  const double2* r = reinterpret_cast<const double2*>(a.rot + (size_t)(column + (lane >> 2)) * TQ_D + 32 * (lane & 3));
+  const uint8_t* xr = reinterpret_cast<const uint8_t*>(x + 32 * (lane & 3));
+  const float inv = 1.0f / nrm;
+  double2 rk[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) rk[k] = __ldg(r + k);
+  double y = 0.0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float f[8];
+    di_load8<Tin>(xr + 8 * k * sizeof(Tin), f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float w = f[j] * inv;
+      w = fmaf(fmaf(-w, nrm, f[j]), inv, w);
+      y = fma(j & 1 ? rk[4 * k + j / 2].y : rk[4 * k + j / 2].x, (double)w, y);
+    }
+  }
+  y += __shfl_xor_sync(0xffffffffu, y, 1);
+  y += __shfl_xor_sync(0xffffffffu, y, 2);
+  return di_search(c, a.bits, y);
+}
+template <typename Tin>
+__device__ __forceinline__ void di_checker(DiList& list, const TqDenseQuant& a, const DiCodes& c, const Tin* x, int64_t ld, int lane) {
+  int done = 0;
+  long long since = clock64();
+#pragma unroll 1
+  while (done < DiList::ROOM) {
+    const bool last = list.closed != 0;
+    const uint32_t e = list.entry[done];
+    if (__any_sync(0xffffffffu, e == DiList::NONE)) {
+      if (__any_sync(0xffffffffu, last || clock64() - since > TC_WAIT_CYCLES)) break;   // (the limit: rows that never come to an end)
+      __nanosleep(100);
+      continue;
+    }
+    since = clock64();
+    __threadfence_block();
+    const int64_t v = (blockIdx.x + (int64_t)(e >> 11) * gridDim.x) * DI_ROWS + (e & 127);
+    const int column = 8 * ((e >> 7) & 15) + (lane >> 2);
+    const float nrm = list.norm[done++];
+    const int m = di_check8<Tin>(a, c, x + v * ld, nrm, 8 * ((e >> 7) & 15), lane);
+    if ((lane & 3) == 0) a.out_idx[v * TQ_D + column] = (uint8_t)m;
+  }
+}
+
+// PROD: residual, its norm and the sketch as well.  SELFTEST: see di_wait
+template <typename Tin, int BITS, bool PROD, int SELFTEST = 0>
 __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __grid_constant__ DiQuant A, const Tin* __restrict__ x, int64_t ld,
                                                                      int64_t n) {
   constexpr int ROWB = di_row_bytes<Tin>();
   extern __shared__ __align__(128) uint8_t di_raw[];
   __shared__ DiShared sh;
   __shared__ uint2 s_cdig[16];                  // digits of the centroids
-  __shared__ double s_sq[16], s_part[4][DI_ROWS];
-  __shared__ float s_norm[DI_ROWS];
-  __shared__ uint8_t s_plain[DI_ROWS];          // rows for di_row_plain
+  __shared__ DiCodes s_codes;
+  __shared__ std::conditional_t<PROD, int, DiList> s_list;
+  DiPlain& s_rows = *reinterpret_cast<DiPlain*>(di_raw + di_quant_smem<Tin, PROD>() - sizeof(DiPlain));
+  __shared__ double s_part[4][DI_ROWS];
+  __shared__ float s_norms[2][DI_ROWS];         // of two tiles in turn
+  __shared__ uint8_t s_plains[2][DI_ROWS];      // rows for di_rows_plain
   const TqDenseQuant& a = A.q;
   uint8_t* tiles_b = di_raw + (((sptr(di_raw) + 127u) & ~127u) - sptr(di_raw));
-  uint8_t* xs = tiles_b + DI_DIGITS * DI_TILE;
+  uint8_t* xs = tiles_b + di_quant_digits<PROD>() * DI_TILE;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) di_init(sh);
   if (tid < 16) {
     const double c = tid < (1 << BITS) ? a.cent[tid] : 0.0;
-    s_sq[tid] = c * c;
+    s_codes.cent[tid] = c;
+    s_codes.bnd[tid] = tid < (1 << BITS) - 1 ? a.bnd[tid] : 0.0;
     s_cdig[tid] = di_digits_f64(c / A.cent_scale);
+  } else if (tid >= 32 && tid < 96) {
+    const int i = tid - 32, lo = BITS < 4 ? i & 7 : i & 15, hi = BITS < 4 ? i >> 3 : 16;
+    const double c0 = lo < (1 << BITS) ? a.cent[lo] : 0.0, c1 = hi < (1 << BITS) ? a.cent[hi] : 0.0;
+    s_codes.square[i] = c0 * c0 + c1 * c1;
+  }
+  if constexpr (!PROD) {
+    if (tid < DiList::ROOM) s_list.entry[tid] = DiList::NONE;
+    if (tid == 0) s_list.count = 0, s_list.closed = 0;
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sptr(&sh.tmem)), "r"(512u) : "memory");
@@ -390,15 +602,33 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
   const uint32_t tb = sh.tmem;
   const int64_t tiles = (n + DI_ROWS - 1) / DI_ROWS, step = gridDim.x;
   const int mine = (int)((tiles - blockIdx.x + step - 1) / step);
-  constexpr int PHASES = PROD ? 3 : 1;
 
   if (warp == DI_COPIER) {
-    if (lane == 0) di_copier<SELFTEST>(sh, tiles_b, mine * PHASES, [&](int i) { return !PROD || i % 3 == 0 ? A.r : i % 3 == 1 ? A.rt : A.s; });
+    if (lane == 0) {
+      if constexpr (PROD)
+        di_copier<SELFTEST>(sh, tiles_b, 3 * mine, [&](int i) { return i % 3 == 0 ? A.r : i % 3 == 1 ? A.rt : A.s; },
+                            [](int i) { return i % 3 == 0 ? 5 : 6; },
+                            [](int i, int p) { return di_uses(i, p); });
+      else
+        di_copier<SELFTEST>(sh, tiles_b, mine > 0 ? 1 : 0, [&](int) { return A.r; }, [](int) { return 4; }, [](int i, int p) { return p < 4 ? i : 0; });
+    }
+    if constexpr (!PROD) {
+      __syncwarp();
+      di_checker<Tin>(s_list, a, s_codes, x, ld, lane);
+    }
   } else if (warp == DI_MMA) {
-    int item = 0;
-    for (int i = 0; i < mine * PHASES && !__any_sync(0xffffffffu, sh.failed); ++i) {
-      di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(i & 1));
-      di_issue<DI_DIGITS, SELFTEST>(sh, item, tiles_b, i, tb, tb + DI_ACC);
+    int item = 0, operands = 0;
+    for (int i = 0; i < mine && !__any_sync(0xffffffffu, sh.failed); ++i) {
+      di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
+      if constexpr (!PROD) {
+        di_issue<4, 4, 3, SELFTEST>(sh, item, tiles_b, [](int) { return 0; }, tb + 128 * (i & 1), tb + DI_ACC);
+      } else {
+        di_issue<4, 5, 4, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i, q); }, tb, tb + DI_ACC);
+        di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
+        di_issue<6, 6, 5, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i + 1, q); }, tb, tb + DI_ACC);
+        di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
+        di_issue<6, 6, 5, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i + 2, q); }, tb, tb + DI_ACC);
+      }
     }
     di_drain(sh);
   } else {
@@ -424,22 +654,22 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int item = 0, t = 0;
-    if (mine > 0) load_tile(blockIdx.x);
-    for (; t < mine; ++t) {
-      const int64_t v0 = (blockIdx.x + t * step) * DI_ROWS, v = v0 + row;
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      if (di_rows_any(sh.failed)) break;   // (in the tile before)
+    // Norms and the digits of w of a tile.  Without the sketch a tile ahead of the indices, into the other half of the operand: its
+    // products are then done when the rows ask for them
+    float nrm = 0.f, next_nrm = 0.f;
+    bool plain = false, next_plain = false;
+    auto prepare = [&](int t) {
+      float* s_norm = s_norms[t & 1];
       // norms in the rows' own precision and NumPy's order (first term + pairwise sum of the rest), eight lanes a vector, two
-      // vectors of a lane at once
+      // vectors of a lane at once; the four vectors of a warp's load are two rows apart: no bank conflicts
       {
-        const int j = tid & 7;
+        const int j = tid & 7, i8 = tid >> 3, r0 = (i8 & ~7) | ((i8 & 3) << 1) | ((i8 >> 2) & 1);
         const Tin* xr[2] = {};
         float s[2];
         auto sq = [&](int q, int k) { const float f = di_f<Tin>(xr[q][k]); return __fmul_rn(f, f); };
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          xr[q] = reinterpret_cast<const Tin*>(xs + ((tid >> 3) + 64 * q) * ROWB);
+          xr[q] = reinterpret_cast<const Tin*>(xs + (r0 + 64 * q) * ROWB);
           s[q] = sq(q, 1 + j);
         }
 #pragma unroll
@@ -456,94 +686,170 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
           for (int q = 0; q < 2; ++q) s[q] = __fadd_rn(s[q], sq(q, i));
 #pragma unroll
         for (int q = 0; q < 2; ++q)
-          if (j == 0) s_norm[(tid >> 3) + 64 * q] = sqrtf(__fadd_rn(sq(q, 0), s[q]));
+          if (j == 0) s_norm[r0 + 64 * q] = sqrtf(__fadd_rn(sq(q, 0), s[q]));
       }
-      if (tid < DI_ROWS) s_plain[tid] = 0;
+      if (tid < DI_ROWS) s_plains[t & 1][tid] = 0;
       di_rows_sync();
-      const float nrm = s_norm[row], safe = nrm > 0.f ? nrm : 1.0f;                // turboquant/polar_quant.py:74
-      bool plain = false;
-      {
-        // w = x / ||x|| in the rows' precision (:75).  As x times the fp64 reciprocal, rounded once to fp32: the quotient of two 24-bit
-        // significands is never within 2^-49 of a rounding boundary, and the fp64 product is off by 2^-52 at most, so this is the
-        // correctly rounded quotient, without the branch of a division.
-        const double inv = 1.0 / (double)safe;
-        const uint8_t* xr = xs + row * ROWB + DI_COLS * h * sizeof(Tin);
-#pragma unroll 1
-        for (int c = 0; c < DI_COLS / 8; ++c) {
-          float f[8];
-          di_load8<Tin>(xr + 8 * c * sizeof(Tin), f);
-          uint2 u[8];
+      next_nrm = s_norm[row];
+      const float safe = next_nrm > 0.f ? next_nrm : 1.0f;                // turboquant/polar_quant.py:74
+      // w = x / ||x|| in the rows' precision (:75), times 2^30: the product with the reciprocal, corrected by its own exact remainder,
+      // is the correctly rounded quotient (P. W. Markstein, IBM J. Res. Dev. 34 (1990), for a correctly rounded reciprocal of a divisor
+      // that is not all ones).  Its digits: the nearest whole number, of which w may be off by half of one.
+      const float inv = 1.0f / safe * 0x1p30f, back = safe * -0x1p-30f;
+      const uint8_t* xr = xs + row * ROWB + DI_COLS * h * sizeof(Tin);
+      float most = 0.f;
+#pragma unroll 2
+      for (int c = 0; c < DI_COLS / 8; ++c) {
+        float f[8];
+        di_load8<Tin>(xr + 8 * c * sizeof(Tin), f);
+        uint2 u[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float w = (float)((double)f[k] * inv);
-            plain |= !(fabsf(w) < DI_LARGEST) || (nrm == 0.f && f[k] != 0.f);   // (squares below the fp32 range: w = x)
-            u[k] = di_digits_f32(w);
-          }
-          di_store8(area, 8 * h + 2 * c, u);
+        for (int k = 0; k < 8; ++k) {
+          float w = f[k] * inv;
+          w = fmaf(fmaf(w, back, f[k]), inv, w);
+          most = fmaxf(most, fabsf(w));
+          u[k] = make_uint2(((uint32_t)__float2int_rn(w) + 0x00808080u) ^ 0x00808080u, 0u);
         }
+        di_store8<4, 0>(area + (PROD ? 0 : 128 * (t & 1)), 8 * h + 2 * c, u);
       }
-      if (plain) s_plain[row] = 1;
+      // Norms that squares below or beyond the fp32 range have gone into (and w = x where all are below it), infinities and NaN; divisors
+      // of all ones
+      next_plain = next_nrm > 0.f ? !(next_nrm > 0x1p-60f && next_nrm < 0x1p63f && most < DI_LARGEST * 0x1p30f) || (__float_as_uint(next_nrm) & 0x7fffffu) == 0x7fffffu
+                                  : next_nrm != 0.f || most != 0.f;
       operand_ready();
-      // rows for the plain arithmetic: whole ones, while the rows are in shared memory; their results otherwise are dropped
-      auto plain_rows = [&]() {
-        if (!di_rows_any(plain)) return;
-        for (int r = warp; r < DI_ROWS; r += DI_ROW_THREADS / 32)
-          if (s_plain[r] && v0 + r < n) di_row_plain<Tin>(a, xs + r * ROWB, s_norm[r], v0 + r, lane);
-        plain = s_plain[row] != 0;
-        di_rows_sync();
-      };
       if constexpr (!PROD) {
-        plain_rows();
+        di_rows_sync();                                            // (the rows have been read)
         if (t + 1 < mine) load_tile(blockIdx.x + (t + 1) * step);
       }
-      bool live = v < n && !plain;
-      // ---- y = R w: indices, ||c[idx]||^2, the centroids as the next operand ----
-      double acc[DI_COLS], cc[4] = {0.0, 0.0, 0.0, 0.0};
-      di_zero(acc);
-      di_take<DI_DIGITS, SELFTEST>(sh, item, myacc, lane, A.r_scale, acc);
+    };
+    int item = 0, t = PROD ? 0 : -1;
+    if (mine > 0) load_tile(blockIdx.x);
+    for (; t < mine; ++t) {
+      if (const int ahead = PROD ? t : t + 1; ahead < mine) {
+        nrm = next_nrm;
+        plain = next_plain;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (di_rows_any(sh.failed)) break;   // (in a tile before)
+        prepare(ahead);
+        if (!PROD && t < 0) continue;
+      }
+      if (PROD || t + 1 >= mine) {
+        nrm = next_nrm;
+        plain = next_plain;
+      }
+      const int64_t v0 = (blockIdx.x + t * step) * DI_ROWS, v = v0 + row;
+      const bool live = v < n;
+      const float* s_norm = s_norms[t & 1];
+      uint8_t* s_plain = s_plains[t & 1];
+      // ---- y = R w: indices, ||c[idx]||^2, the centroids as the next operand.  Without the sketch of the 34 products of all digits ten,
+      // which leave less than 2^-21 of r_scale out: one output in 90,000 of a rotation's with eight centroids is too close to a boundary
+      // and is left to the checker.  With the sketch, where other outputs hang on it, 14 products: one in six million; its row is for
+      // di_rows_plain.  Rows of zeros are on no boundary.
       uint32_t packed[DI_COLS / 4];
+      uint32_t unsure = 0;   // groups of eight columns
+      {
+        int32_t y[DI_COLS];
+        di_take32<PROD ? 4 : 3, SELFTEST>(sh, item, myacc, lane, PROD ? A.shift : 17, y);
+        if constexpr (PROD) {
+          uint32_t near = 0xffffffffu;
 #pragma unroll
-      for (int g = 0; g < DI_COLS / 4; ++g) {
-        packed[g] = 0;
+          for (int g = 0; g < DI_COLS / 4; ++g) {
+            packed[g] = 0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          uint32_t m = 0;                                  // boundaries below y (searchsorted, side = 'left')
+            for (int k = 0; k < 4; ++k) packed[g] |= di_index<BITS>(A.thr, A.near, y[4 * g + k], near) << (8 * k);
+          }
+          plain |= near <= 2 * A.near && nrm != 0.f;
+        } else {
 #pragma unroll
-          for (int b = 0; b < (1 << BITS) - 1; ++b) m += A.bnd[b] < acc[4 * g + k] ? 1u : 0u;
-          packed[g] |= m << (8 * k);
-          cc[k] += s_sq[m];
+          for (int c = 0; c < DI_COLS / 8; ++c) {
+            float frac = 0.f;
+#pragma unroll
+            for (int g = 2 * c; g < 2 * c + 2; ++g) {
+              uint32_t m[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) m[k] = di_index_float<BITS>(A, y[4 * g + k], frac);
+              packed[g] = __byte_perm(__byte_perm(m[0], m[1], 0x0040), __byte_perm(m[2], m[3], 0x0040), 0x5410);
+            }
+            unsure |= frac > 0.f ? 1u << c : 0u;
+          }
+          if (nrm == 0.f || !live) unsure = 0;
+          if (a.out_scale && unsure) plain = true;
         }
+#pragma unroll
+        for (int g = 0; g < DI_COLS / 4; ++g)
+          if (nrm == 0.f) packed[g] = 0x01010101u * (uint32_t)A.zero_idx;
+      }
+      if (PROD || a.out_scale) {
+        double cc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int g = 0; g < DI_COLS / 4; ++g) {
+          if constexpr (BITS < 4) {
+            const uint32_t two = packed[g] | (packed[g] >> 5);
+            cc[0] += s_codes.square[two & 63];
+            cc[1] += s_codes.square[(two >> 16) & 63];
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) cc[k] += s_codes.square[(packed[g] >> (8 * k)) & 15];
+          }
+        }
+        s_part[h][row] = (cc[0] + cc[1]) + (cc[2] + cc[3]);
       }
       if (live && a.out_idx) {
 #pragma unroll
         for (int g = 0; g < DI_COLS / 4; g += 4)
           *reinterpret_cast<uint4*>(a.out_idx + v * TQ_D + DI_COLS * h + 4 * g) = make_uint4(packed[g], packed[g + 1], packed[g + 2], packed[g + 3]);
       }
-      s_part[h][row] = (cc[0] + cc[1]) + (cc[2] + cc[3]);
       if constexpr (PROD) {
 #pragma unroll
         for (int c = 0; c < DI_COLS / 8; ++c) {
-          uint2 u[8];
+          if constexpr (BITS < 4) {
+            di_store_codes<6>(area, 8 * h + 2 * c, A.words, packed[2 * c], packed[2 * c + 1]);
+          } else {
+            uint2 u[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) u[k] = s_cdig[(packed[2 * c + (k >> 2)] >> (8 * (k & 3))) & 15];
-          di_store8(area, 8 * h + 2 * c, u);
+            for (int k = 0; k < 8; ++k) u[k] = s_cdig[(packed[2 * c + (k >> 2)] >> (8 * (k & 3))) & 15];
+            di_store8<6, 1>(area, 8 * h + 2 * c, u);
+          }
         }
         operand_ready();
       }
-      di_rows_sync();
-      double cn = sqrt((s_part[0][row] + s_part[1][row]) + (s_part[2][row] + s_part[3][row]));
-      cn = cn > 1e-10 ? cn : 1.0;                                                 // turboquant/polar_quant.py:110-111
+      if constexpr (!PROD) {
+        if (unsure && !plain && a.out_idx) {
+          __threadfence_block();   // (the indices have been stored)
+          for (; unsure; unsure &= unsure - 1) {
+            const int at = atomicAdd(&s_list.count, 1);
+            if (at >= DiList::ROOM) {
+              plain = true;
+              continue;
+            }
+            s_list.norm[at] = nrm;
+            __threadfence_block();
+            s_list.entry[at] = (uint32_t)row | (uint32_t)(4 * h + __ffs(unsure) - 1) << 7 | (uint32_t)t << 11;
+          }
+        }
+      }
+      double cn = 1.0;
+      if (PROD || a.out_scale) {
+        di_rows_sync();
+        cn = sqrt((s_part[0][row] + s_part[1][row]) + (s_part[2][row] + s_part[3][row]));
+        cn = cn > 1e-10 ? cn : 1.0;                                               // turboquant/polar_quant.py:110-111
+      }
       if (h == 0 && live) {
         if (a.out_norm) a.out_norm[v] = nrm;
         if (a.out_scale) a.out_scale[v] = (float)(a.norm_correction ? (double)nrm / cn : (double)nrm);
       }
       if constexpr (PROD) {
-        // ---- x_hat = norm R^T c / ||c||, residual x - x_hat, with the norm that is returned and stored (fp32) ----
-        const double back = A.r_scale * A.cent_scale * (a.norm_correction ? 1.0 / cn : 1.0) * (double)nrm;
+        // ---- x_hat = norm R^T c / ||c||, residual x - x_hat, with the norm that is returned and stored (fp32).  Six digits each:
+        // what the 13 products left out would add is below 2^-36.4 of r_scale cent_scale, in practice 2^-44 of the residual's length, whose
+        // fp32 rounding is 2^-25 (with five digits 2^-36, and one residual norm in 4,000 came out a neighbour) ----
+        const double inv = a.norm_correction ? 1.0 / cn : 1.0;
+        const double back = -0x1p-32 * A.r_scale * A.cent_scale * inv * (double)nrm;
         const double unit = nrm > 0.f && nrm < 1e38f ? ldexp(1.0, -(ilogbf(nrm) + 2)) : 1.0;   // |residual| x unit < 1 for a rotation
+        const double unit46 = unit * 0x1p46;
+        uint32_t over = 0;
         double rr[4] = {0.0, 0.0, 0.0, 0.0};
-        di_zero(acc);
-        di_take<DI_DIGITS, SELFTEST>(sh, item, myacc, lane, back, acc);
+        long long acc[DI_COLS];
+        di_take64<SELFTEST>(sh, item, myacc, lane, acc);
         const uint8_t* xr = xs + row * ROWB + DI_COLS * h * sizeof(Tin);
 #pragma unroll
         for (int c = 0; c < DI_COLS / 8; ++c) {
@@ -552,28 +858,36 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
           uint2 u[8];
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            const double e = (double)f[k] - acc[8 * c + k], es = e * unit;
+            const double e = fma(di_double(acc[8 * c + k]), back, (double)f[k]);
             rr[k & 3] = fma(e, e, rr[k & 3]);
-            plain |= !(fabs(es) < (double)DI_LARGEST);
-            u[k] = di_digits_f64(es);
+            // to a whole number of 2^-46, in balanced digits; the upper half tells what is too large
+            const unsigned long long w = (unsigned long long)__double_as_longlong(fma(e, unit46, 6755399441055744.0));
+            over = max(over, (uint32_t)(w >> 32) - 0x43380000u + 31000u);
+            u[k] = di_split((w + 0x8080808080ull) ^ 0x8080808080ull);
           }
-          di_store8(area, 8 * h + 2 * c, u);
+          di_store8<6, 0>(area, 8 * h + 2 * c, u);
         }
-        di_rows_sync();   // (the sums of the squared centroids have been read)
-        s_part[h][row] = (rr[0] + rr[1]) + (rr[2] + rr[3]);
-        if (plain) s_plain[row] = 1;
+        plain |= over > 62000u;
         operand_ready();
-        plain_rows();
-        live = v < n && !plain;
+        di_rows_sync();   // (the sums of the squared centroids have been read, and the rows)
+        s_part[h][row] = (rr[0] + rr[1]) + (rr[2] + rr[3]);
+        if (t + 1 < mine) load_tile(blockIdx.x + (t + 1) * step);
+        di_rows_sync();
         if (h == 0 && live && a.out_rnorm)
           a.out_rnorm[v] = (float)sqrt((s_part[0][row] + s_part[1][row]) + (s_part[2][row] + s_part[3][row]));
-        if (t + 1 < mine) load_tile(blockIdx.x + (t + 1) * step);
-        // ---- sketch: sign(S r), zero counts as +1 (turboquant/qjl.py:89-90), first column in the most significant bit ----
-        di_zero(acc);
-        di_take<DI_DIGITS, SELFTEST>(sh, item, myacc, lane, 1.0, acc);
+        // ---- sketch: sign(S r), zero counts as +1 (turboquant/qjl.py:89-90), first column in the most significant bit.  A projection
+        // that what has been left out here (2^-36.3 s_scale) and of the residual may turn: di_rows_plain (with five digits each, three rows
+        // of 64,000, each 20 us of a CTA) ----
+        di_take64<SELFTEST>(sh, item, myacc, lane, acc);
+        const long long band = (long long)fmin(256.0 + A.slack * (double)nrm * unit * inv, 0x1p60);
         uint32_t m = 0;
+        bool close = false;
 #pragma unroll
-        for (int k = 0; k < DI_COLS; ++k) m = (m << 1) | (acc[k] < 0.0 ? 0u : 1u);
+        for (int k = 0; k < DI_COLS; ++k) {
+          m = (m << 1) | (acc[k] < 0 ? 0u : 1u);
+          close |= (unsigned long long)(acc[k] + band) <= 2 * (unsigned long long)band;
+        }
+        plain |= close && nrm != 0.f;
         m = __byte_perm(m, 0, 0x0123);
         if (live && a.out_qjl) {
           uint8_t* z = a.out_qjl + v * 16 + 4 * h;
@@ -581,9 +895,17 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
           else z[0] = (uint8_t)m, z[1] = (uint8_t)(m >> 8), z[2] = (uint8_t)(m >> 16), z[3] = (uint8_t)(m >> 24);
         }
       }
+      if (plain) s_plain[row] = 1;
+      if (di_rows_any(plain)) {   // whole rows in plain arithmetic, over what has been stored
+        di_rows_plain<Tin>(s_rows, a, s_codes, s_plain, s_norm, x, ld, v0, n, tid);
+        di_rows_sync();
+      }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (di_rows_any(sh.failed)) {   // the last tile begun and those behind it
+    const bool failed = di_rows_any(sh.failed);
+    if constexpr (!PROD)
+      if (tid == 0) s_list.closed = 1;
+    if (failed) {   // the last tile begun and those behind it
       di_give_up(a, t > 0 ? t - 1 : 0, mine, h == 0 ? row : -1, n, A.status);
     }
   }
@@ -597,7 +919,7 @@ constexpr int DI_IDX_ROW = TQ_D + 16, DI_OUT_ROW = 16 * 8 + 16;   // bytes betwe
 constexpr int DI_DEQUANT_SMEM = DI_DIGITS * DI_TILE + DI_ROWS * DI_IDX_ROW + DI_ROW_THREADS * DI_OUT_ROW + 128;
 
 // x_hat = (norm / ||c[idx]||) R^T c[idx] + shrink sqrt(pi/2)/sqrt(d) rnorm S^T z.  The signs z are one digit, +-1: seven products.
-template <typename Tout, bool PROD, bool SELFTEST = false>
+template <typename Tout, bool PROD, int SELFTEST = 0>
 __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __grid_constant__ DiDequant A, int64_t n, Tout* __restrict__ out) {
   extern __shared__ __align__(128) uint8_t di_raw[];
   __shared__ DiShared sh;
@@ -629,13 +951,15 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
   constexpr int PHASES = PROD ? 2 : 1;   // (the signs' product first)
 
   if (warp == DI_COPIER) {
-    if (lane == 0) di_copier<SELFTEST>(sh, tiles_b, mine * PHASES, [&](int i) { return PROD && (i & 1) == 0 ? A.st : A.rt; });
+    if (lane == 0)
+      di_copier<SELFTEST>(sh, tiles_b, mine * PHASES, [&](int i) { return PROD && (i & 1) == 0 ? A.st : A.rt; }, [](int) { return DI_DIGITS; },
+                          [](int i, int) { return i; });
   } else if (warp == DI_MMA) {
     int item = 0;
     for (int i = 0; i < mine && !__any_sync(0xffffffffu, sh.failed); ++i) {
       di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(i & 1));
-      if constexpr (PROD) di_issue<1, SELFTEST>(sh, item, tiles_b, 2 * i, tb + DI_SIGNS, tb + DI_ACC);
-      di_issue<DI_DIGITS, SELFTEST>(sh, item, tiles_b, PROD ? 2 * i + 1 : i, tb, tb + DI_ACC);
+      if constexpr (PROD) di_issue<1, DI_DIGITS, DI_DIGITS - 1, SELFTEST>(sh, item, tiles_b, [&](int) { return 2 * i; }, tb + DI_SIGNS, tb + DI_ACC);
+      di_issue<DI_DIGITS, DI_DIGITS, DI_SUMS - 1, SELFTEST>(sh, item, tiles_b, [&](int) { return PROD ? 2 * i + 1 : i; }, tb, tb + DI_ACC);
     }
     di_drain(sh);
   } else {
@@ -676,7 +1000,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
           u[k] = s_cdig[m];
           cc[k & 3] += s_sq[m];
         }
-        di_store8(area, 8 * h + 2 * c, u);
+        di_store8<DI_DIGITS, 0>(area, 8 * h + 2 * c, u);
         if constexpr (PROD) {   // eight sketch bits, the first in the most significant place
           const uint32_t z = live ? a.qjl[v * 16 + 4 * h + c] : 0u;
           di_st2(area + DI_SIGNS + 8 * h + 2 * c, s_sign[z >> 4], s_sign[z & 15]);
@@ -706,8 +1030,8 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
       }
       double acc[DI_COLS];
       di_zero(acc);
-      if constexpr (PROD) di_take<1, SELFTEST>(sh, item, myacc, lane, g, acc);
-      di_take<DI_DIGITS, SELFTEST>(sh, item, myacc, lane, f, acc);
+      if constexpr (PROD) di_take<DI_DIGITS - 1, SELFTEST>(sh, item, myacc, lane, g, acc);
+      di_take<DI_SUMS - 1, SELFTEST>(sh, item, myacc, lane, f, acc);
       Tout* o = out + v * a.ld_out + DI_COLS * h;
       if (a.accumulate && live) {
 #pragma unroll
@@ -830,8 +1154,8 @@ template <auto kernel, typename... Args> int di_launch(int smem, int64_t n, cuda
 }
 template <typename Tin, int BITS> int di_quantize_bits(const DiQuant& A, const Tin* x, int64_t ld, int64_t n, cudaStream_t st) {
   if (A.q.out_qjl || A.q.out_rnorm)
-    return di_launch<k_dense_quantize_i8<Tin, BITS, true>>(di_quant_smem<Tin>(), n, st, "k_dense_quantize_i8", A, x, ld, n);
-  return di_launch<k_dense_quantize_i8<Tin, BITS, false>>(di_quant_smem<Tin>(), n, st, "k_dense_quantize_i8", A, x, ld, n);
+    return di_launch<k_dense_quantize_i8<Tin, BITS, true>>(di_quant_smem<Tin, true>(), n, st, "k_dense_quantize_i8", A, x, ld, n);
+  return di_launch<k_dense_quantize_i8<Tin, BITS, false>>(di_quant_smem<Tin, false>(), n, st, "k_dense_quantize_i8", A, x, ld, n);
 }
 template <typename Tin> int di_quantize(const DiQuant& A, const void* x, int64_t ld, int64_t n, cudaStream_t st) {
   const Tin* xt = reinterpret_cast<const Tin*>(x);
@@ -850,15 +1174,16 @@ template <typename Tout> int di_dequantize(const DiDequant& A, int64_t n, void* 
 
 }  // namespace
 
-// The power of two that a matrix's digits are relative to, or 0 for a matrix that stays with the fp64 kernels.
+// The power of two that a matrix's digits are relative to, or 0 for a matrix that stays with the fp64 kernels; rows, length: the largest
+// sum of a row's magnitudes and the length of the longest row over it.
 // The digits are fixed-point numbers of 2^-54 of the largest entry, where fp64 keeps every entry's own exponent.  No product may lose
 // by that, so: every row and column is at least sqrt(2) times as long as the largest entry (the rounding of a row's digits is then
 // 2^-55 of that row's length, below that of fp64 sums), and no entry is below 2^-30 of it (a row of x enters with 2^-54 of its length;
 // an entry of zero would hide its large elements, and what an output then sees may be smaller than that).  Random rotations
 // and Gaussian matrices are of this kind (their rows are three times and twice as long); uneven, diagonal or block matrices and what
 // is not finite are not.
-double tq_dense_digits_scale(const double* m) {
-  double most = 0.0, least = 1e300, row[TQ_D] = {}, col[TQ_D] = {};
+double tq_dense_digits_scale(const double* m, double* rows, double* length) {
+  double most = 0.0, least = 1e300, row[TQ_D] = {}, col[TQ_D] = {}, sum[TQ_D] = {};
   for (int i = 0; i < TQ_D; ++i)
     for (int j = 0; j < TQ_D; ++j) {
       const double a = fabs(m[i * TQ_D + j]);
@@ -866,12 +1191,15 @@ double tq_dense_digits_scale(const double* m) {
       least = a < least ? a : least;
       row[i] += a * a;
       col[j] += a * a;
+      sum[i] += a;
     }
   if (!(most > 1e-100 && most < 1e100 && least >= most * 0x1p-30)) return 0.0;
   for (int i = 0; i < TQ_D; ++i)
     if (!(row[i] >= 2.0 * most * most && col[i] >= 2.0 * most * most)) return 0.0;   // (also what is not a number)
   int e = 0;
   frexp(most, &e);   // most < 2^e
+  *rows = *length = 0.0;
+  for (int i = 0; i < TQ_D; ++i) *rows = fmax(*rows, ldexp(sum[i], -e)), *length = fmax(*length, ldexp(sqrt(row[i]), -e));
   return ldexp(1.0, e);
 }
 // A power of two above every centroid's magnitude, or 0 for a codebook whose centroids differ much in size: those of a row
@@ -887,11 +1215,20 @@ double tq_dense_digits_centroids(const double* c, int n) {
   return ldexp(1.0, e);
 }
 
+// The digits of the first eight centroids, whole numbers of 2^-54 of the scale, as the kernels' operands are made from
+void tq_dense_digits_words(const double* c, int n, double scale, uint32_t (&words)[7][2]) {
+  memset(words, 0, sizeof(words));
+  for (int i = 0; i < (n < 8 ? n : 8); ++i) {
+    const uint64_t u = ((uint64_t)llrint(c[i] / scale * 18014398509481984.0) + 0x808080808080ull) ^ 0x808080808080ull;
+    for (int p = 0; p < 7; ++p) words[p][i >> 2] |= (uint32_t)(uint8_t)(u >> (48 - 8 * p)) << (8 * (i & 3));
+  }
+}
+
 // Calls that come here, us here / in the fp64 kernels (which take tiles of 16, 32 or 64 vectors, two CTAs an SM, and step up at 32
-// and 64 vectors per SM): quantize 8,192 vectors 23.2 / 23.2, 12,000 23.2 / 39.6, 65,536 77 / 134; with the sketch 4,096 50 / 34, 8,192
-// 52 / 52, 12,000 56 / 94, 65,536 182 / 302; dequantize 8,192 19 / 17, 12,000 19 / 29, 65,536 63 / 90; with the sketch 4,096 28 / 23,
-// 6,000 29 / 31, 65,536 93 / 164.
-static bool di_enough(int64_t n, bool sketched_dequantize) { return n > (sketched_dequantize ? 32 : 64) * (int64_t)tq_num_sms(); }
+// and 64 vectors per SM): quantize 4,096 vectors 14.6 / 14.6, 4,800 14.5 / 22.8, 9,472 14.6 / 22.8, 65,536 33 / 134; with the sketch 4,096
+// 27 / 27, 4,800 27 / 43, 12,000 27 / 94, 65,536 90 / 302; dequantize 8,192 19 / 17, 12,000 19 / 29, 65,536 62 / 90; with the sketch 4,096
+// 27 / 23, 6,000 27 / 31, 65,536 93 / 164.
+static bool di_enough(int64_t n, bool dequantize, bool sketch) { return n > (dequantize && !sketch ? 64 : 32) * (int64_t)tq_num_sms(); }
 
 // The kernels' arguments; false: not of these kernels' kind
 static bool di_quant_args(const TqDenseQuant& a, const TqDenseDigits& g, const void* x, int32_t dtype, int64_t ld, DiQuant& A) {
@@ -902,8 +1239,29 @@ static bool di_quant_args(const TqDenseQuant& a, const TqDenseDigits& g, const v
   A.r = g.r; A.rt = g.rt; A.s = g.s;
   A.r_scale = g.r_scale / 4096.0;
   A.cent_scale = g.cent_scale;
+  A.slack = 32768.0 * g.r_scale * g.cent_scale;
   A.status = tq_quantize_status_word();
-  for (int i = 0; i < 15; ++i) A.bnd[i] = g.bnd[i];
+  for (int p = 0; p < DI_DIGITS; ++p) A.words[p] = make_uint2(g.words[p][0], g.words[p][1]);
+  // Boundaries as numbers of 2^-27 of r_scale (no y is beyond 16 of them: entries of R are below r_scale, rows of w shorter than 1 + 2^-20),
+  // and what a y may be off by: the products left out (1.004 x 2^-21), half of 2^-30 of every element of w, two fields cut off, the
+  // boundary's rounding; in fp32 also a rounding of y and one of the ramp's constant.  With the sketch numbers of 2^-29 where rows of R
+  // are that short, products left out 2^-29, two or three fields.
+  const double unit = !prod || g.r_length > 3.9 ? 0x1p27 : 0x1p29;
+  A.shift = unit == 0x1p27 ? 17 : 15;
+  double most = 0.0;
+  for (int i = 0; i < 15; ++i) {
+    const double t = fmin(fmax(rint(g.bnd[i] / g.r_scale * unit), -2147483000.0), 2147483000.0);
+    A.thr[i] = (int32_t)t;
+    if (i < (1 << a.bits) - 1) most = fmax(most, fabs(t));
+  }
+  A.near = (uint32_t)(A.shift == 15 ? ceil(g.r_rows * 0.25 + 3.6) : ceil(g.r_rows * 0.0625 + (prod ? 3.8 : 67.5)));
+  const double reach = A.near + most * 0x1p-22;
+  for (int i = 1; i < (1 << a.bits) - 1 && !prod; ++i)   // (ramps that overlap may add up to a whole number)
+    if ((double)A.thr[i] - A.thr[i - 1] < 2.0 * reach + 8.0) return false;
+  A.step = (float)(0.5 / reach);
+  for (int i = 0; i < 15; ++i) A.offset[i] = (float)(0.5 - A.thr[i] * (double)A.step);
+  A.zero_idx = 0;
+  for (int i = 0; i < (1 << a.bits) - 1; ++i) A.zero_idx += g.bnd[i] < 0.0 ? 1 : 0;
   A.q = a;
   return true;
 }
@@ -923,7 +1281,7 @@ static bool di_dequant_args(const TqDenseDequant& a, const TqDenseDigits& g, DiD
 bool tq_dense_i8_quantize_try(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int32_t dtype, int64_t ld, int64_t n, cudaStream_t st,
                               int* rc) {
   DiQuant A;
-  if (!di_enough(n, false) || !di_quant_args(a, q->dig, x, dtype, ld, A) || !di_digits_ready(q, st)) return false;
+  if (!di_enough(n, false, a.out_qjl || a.out_rnorm) || !di_quant_args(a, q->dig, x, dtype, ld, A) || !di_digits_ready(q, st)) return false;
   *rc = dtype == TQ_F32 ? di_quantize<float>(A, x, ld, n, st) : di_quantize<__half>(A, x, ld, n, st);
   return true;
 }
@@ -931,7 +1289,7 @@ bool tq_dense_i8_quantize_try(const tq_quantizer* q, const TqDenseQuant& a, cons
 bool tq_dense_i8_dequantize_try(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, void* out, int32_t dtype, cudaStream_t st, int* rc) {
   DiDequant A;
   if (dtype != TQ_F64 && dtype != TQ_F32 && dtype != TQ_F16) return false;
-  if (!di_enough(n, a.qjl != nullptr) || !di_dequant_args(a, q->dig, A) || !di_digits_ready(q, st)) return false;
+  if (!di_enough(n, true, a.qjl != nullptr) || !di_dequant_args(a, q->dig, A) || !di_digits_ready(q, st)) return false;
   switch (dtype) {
     case TQ_F64: *rc = di_dequantize<double>(A, n, out, st); return true;
     case TQ_F32: *rc = di_dequantize<float>(A, n, out, st); return true;
@@ -944,11 +1302,11 @@ int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, 
   DiQuant A;
   TQ_REQUIRE(a.bits == 2 && a.out_qjl && di_quant_args(a, q->dig, x, TQ_F32, ld, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED,
              "self-test of the dense quantizer: fp32 rows of 128 elements, 2 bits and a sketch");
-  return di_launch<k_dense_quantize_i8<float, 2, true, true>>(di_quant_smem<float>(), n, st, "k_dense_quantize_i8", A,
+  return di_launch<k_dense_quantize_i8<float, 2, true, 18>>(di_quant_smem<float, true>(), n, st, "k_dense_quantize_i8", A,
                                                               reinterpret_cast<const float*>(x), ld, n);
 }
 int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st) {
   DiDequant A;
   TQ_REQUIRE(a.qjl && di_dequant_args(a, q->dig, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED, "self-test of the dense dequantizer: 128 elements and a sketch");
-  return di_launch<k_dense_dequantize_i8<double, true, true>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, out);
+  return di_launch<k_dense_dequantize_i8<double, true, 26>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, out);
 }

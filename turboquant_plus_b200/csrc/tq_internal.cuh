@@ -32,12 +32,15 @@ struct TqFast {
 struct TqDenseDigits {
   const uint8_t *r, *rt, *s, *st;   // of R, R^T, S, S^T
   double r_scale, s_scale;          // powers of two that the digits are relative to
+  double r_rows, r_length;          // the largest sum of magnitudes of a row of R, and the longest row's length, over r_scale
   double cent_scale;                // a power of two above every centroid's magnitude
   double bnd[15];                   // boundaries
+  uint32_t words[7][2];             // digit p of centroids 0-3 and 4-7, a byte each
 };
 #define TQ_DENSE_DIGITS_BYTES (7 * TQ_D * TQ_D)
-double tq_dense_digits_scale(const double* m);
+double tq_dense_digits_scale(const double* m, double* rows, double* length);
 double tq_dense_digits_centroids(const double* c, int n);
+void tq_dense_digits_words(const double* c, int n, double scale, uint32_t (&words)[7][2]);
 
 struct tq_quantizer {
   int32_t d, bits, rotation, norm_correction, qjl, device;
@@ -284,7 +287,7 @@ __device__ __forceinline__ int64_t tq_dst_record(const TqQuantDst& dst, int64_t 
 
 // dense-mode work on the fp64 tensor cores (tq_dense.cu); matrices padded to dp x dp
 struct TqDenseQuant {
-  const double *rot, *rot_t, *s;   // R, R^T, S, rows contiguous
+  const double *rot, *rot_t, *s, *s_t;   // R, R^T, S, S^T, rows contiguous
   const double *cent, *bnd;
   int32_t d, dp, bits, norm_correction;
   uint8_t *out_packed, *out_idx;
