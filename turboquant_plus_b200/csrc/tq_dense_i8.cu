@@ -28,8 +28,9 @@
 // barriers and stores) and 40,000 with it (sums 20,000, of which the MMAs take 13,000; residuals 7,000).  65,536 fp32 vectors, fp64
 // tensor cores / all 34 products each / here: 134 / 78 / 33 us, with the sketch 302 / 163 / 90 (105 where a row on a CTA's way is for
 // di_rows_plain, 14 us; about every second call).
-// What bounds dequantize: its rows.  A tile's 136 MMAs take 8,800 clocks, the rows' loads of sums (700 clocks each under MMAs, 120 without) and
-// their fp64 additions run between the MMAs rather than under them.  65,536 vectors, fp64 tensor cores / here: 90 / 62 us, with the sketch 164 / 93.
+// What bounds dequantize: its rows, 20,000 clocks a tile where the MMAs (88 clocks each under the rows' loads of sums) take 12,000: sums 900 clocks
+// each, half of it fp64 additions, the next operand 500 a digit, results 3,700, norms and factors 3,000.  65,536 vectors, fp64 tensor
+// cores / all of it behind the last sum / here: 90 / 62 / 56 us, with the sketch 164 / 93 / 85.
 //
 // A wait that gives up ends the waits of all roles; the results of its tile and of those behind it are then not numbers, and a
 // status word is set (tq_quantize_status_sync).
@@ -57,6 +58,9 @@ template <> __device__ __forceinline__ double di_d<__half>(__half v) { return (d
 
 __device__ __forceinline__ void di_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sptr(bar)) : "memory");
+}
+__device__ __forceinline__ void di_arrive_warp(uint64_t* bar, int lane) {
+  if (lane == 0) di_arrive(bar);
 }
 // MMAs and commits are executed by a converged warp, one elected thread of which issues them: addresses and descriptors then live
 // in uniform registers (from a branch of one thread an MMA took 115 clocks to issue, not the 65 that it takes to execute)
@@ -96,6 +100,12 @@ __device__ __forceinline__ uint2 di_digits_f64(double v) {
   const double lo = fma(rest, 18014398509481984.0, BIG);                // the rest x 2^54, at most 2^31
   const long long w = (__double_as_longlong(lo) - __double_as_longlong(BIG)) + ((long long)__double2loint(hi) << 32);
   return di_split(di_digits(w));
+}
+// byte permute by a selector as it is: where the fourth bit of a nibble is set the byte's sign bit is repeated eight times (the intrinsic masks it)
+__device__ __forceinline__ uint32_t di_prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
 }
 // byte k of four words -> operand word k of the four elements
 __device__ __forceinline__ void di_transpose(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&w)[4]) {
@@ -185,15 +195,17 @@ __device__ __forceinline__ void di_copier(DiShared& s, uint8_t* tiles, int matri
 }
 
 // The MMA warp: the operand at `area`, of PA digits, against the leading QB digits of a matrix, sums s = LAST to 0 of the products of
-// digits p + q = s.  uses(q): the matrices before that had a digit q
-template <int PA, int QB, int LAST, int SELFTEST, typename U>
-__device__ __forceinline__ void di_issue(DiShared& s, int& item, const uint8_t* tiles, U&& uses, uint32_t area, uint32_t acc_base) {
+// digits p + q = s.  uses(q): the matrices before that had a digit q;
+// operand(s): waits for the operand's digits that the sum is the first to take
+template <int PA, int QB, int LAST, int SELFTEST, typename U, typename W>
+__device__ __forceinline__ void di_issue(DiShared& s, int& item, const uint8_t* tiles, U&& uses, W&& operand, uint32_t area, uint32_t acc_base) {
   const uint32_t b = sptr(tiles), idesc = di_idesc();
 #pragma unroll 1
   for (int sum = LAST; sum >= 0; --sum, ++item) {
     const int sl = item & 1;
-    if (sum == LAST)
-      for (int q = 0; q < QB; ++q) di_wait<SELFTEST>(s, &s.b_full[q], (uint32_t)(uses(q) & 1));
+    for (int q = sum - PA + 1 > 0 ? sum - PA + 1 : 0; q < QB && (sum == LAST || q + PA - 1 == sum); ++q)   // digits used for the first time
+      di_wait<SELFTEST>(s, &s.b_full[q], (uint32_t)(uses(q) & 1));
+    operand(sum);
     if (item >= 2) di_wait<SELFTEST>(s, &s.d_free[sl], (uint32_t)((item / 2 - 1) & 1));
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -285,19 +297,29 @@ __device__ __forceinline__ double di_double(long long v) {
   return __longlong_as_double(v + 0x4338000000000000ll) - 6755399441055744.0;
 }
 
-// acc += base x (the product's sums, 256^-s each)
-template <int LAST, int SELFTEST>
-__device__ __forceinline__ void di_take(DiShared& s, int& item, uint32_t acc_base, int lane, double base, double (&acc)[DI_COLS]) {
-  double factor = base;
+// ... for two sums, s and s - 1: of both accumulators 256 times the second plus the first
+template <int SELFTEST, typename U>
+__device__ __forceinline__ void di_columns2(DiShared& s, int item, uint32_t acc_base, int lane, U&& use) {
+  di_wait<SELFTEST>(s, &s.d_full[item & 1], (uint32_t)((item / 2) & 1));
+  di_wait<SELFTEST>(s, &s.d_full[(item + 1) & 1], (uint32_t)(((item + 1) / 2) & 1));
+  __syncwarp();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t lo = acc_base + 128 * (item & 1), hi = acc_base + 128 * ((item + 1) & 1);
 #pragma unroll
-  for (int i = 0; i < LAST; ++i) factor *= 0.00390625;
-#pragma unroll 1
-  for (int sum = LAST; sum >= 0; --sum, ++item, factor *= 256.0)
-    di_columns<SELFTEST>(s, item, acc_base, lane, [&](int k, uint32_t v) { acc[k] = fma(di_double(v), factor, acc[k]); });
-}
-__device__ __forceinline__ void di_zero(double (&acc)[DI_COLS]) {
+  for (int c = 0; c < DI_COLS / 8; ++c) {
+    uint32_t v[8], w[8];
+    di_ld8(lo + 8 * c, v);
+    di_ld8(hi + 8 * c, w);
+    di_ld8_wait(v);
+    di_ld8_wait(w);
+    if (c + 1 == DI_COLS / 8) {   // all read
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) di_arrive(&s.d_free[item & 1]), di_arrive(&s.d_free[(item + 1) & 1]);
+    }
 #pragma unroll
-  for (int k = 0; k < DI_COLS; ++k) acc[k] = 0.0;
+    for (int k = 0; k < 8; ++k) use(8 * c + k, w[k] * 256u + v[k]);
+  }
 }
 
 // eight consecutive elements of a staged row (16-byte aligned) as fp32
@@ -332,7 +354,9 @@ struct DiQuant {
 };
 struct DiDequant {
   const uint8_t *rt, *st;
+  uint4 words[DI_DIGITS];             // digits of the sixteen centroids, a byte each
   double r_scale, s_scale, cent_scale;
+  int32_t tiled;                      // fp64 results go out by tiled copies
   int32_t* status;
   TqDenseDequant q;
 };
@@ -454,7 +478,7 @@ template <typename Tin, bool PROD> constexpr int di_quant_smem() {
 template <int COUNT> __device__ __forceinline__ void di_store_codes(uint32_t area, int col, const uint2 (&words)[DI_DIGITS], uint32_t q0, uint32_t q1) {
   const uint32_t s0 = __byte_perm(q0 | (q0 >> 4), 0, 0x4420), s1 = __byte_perm(q1 | (q1 >> 4), 0, 0x4420);
 #pragma unroll
-  for (int p = 0; p < COUNT; ++p) di_st2(area + 32 * p + col, __byte_perm(words[p].x, words[p].y, s0), __byte_perm(words[p].x, words[p].y, s1));
+  for (int p = 0; p < COUNT; ++p) di_st2(area + 32 * p + col, di_prmt(words[p].x, words[p].y, s0), di_prmt(words[p].x, words[p].y, s1));
 }
 
 // R, R^T and S with 5, 6 and 6 digits, in turn: those among the first i matrices that have a digit p
@@ -621,13 +645,13 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
     for (int i = 0; i < mine && !__any_sync(0xffffffffu, sh.failed); ++i) {
       di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
       if constexpr (!PROD) {
-        di_issue<4, 4, 3, SELFTEST>(sh, item, tiles_b, [](int) { return 0; }, tb + 128 * (i & 1), tb + DI_ACC);
+        di_issue<4, 4, 3, SELFTEST>(sh, item, tiles_b, [](int) { return 0; }, [](int) {}, tb + 128 * (i & 1), tb + DI_ACC);
       } else {
-        di_issue<4, 5, 4, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i, q); }, tb, tb + DI_ACC);
+        di_issue<4, 5, 4, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i, q); }, [](int) {}, tb, tb + DI_ACC);
         di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
-        di_issue<6, 6, 5, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i + 1, q); }, tb, tb + DI_ACC);
+        di_issue<6, 6, 5, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i + 1, q); }, [](int) {}, tb, tb + DI_ACC);
         di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
-        di_issue<6, 6, 5, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i + 2, q); }, tb, tb + DI_ACC);
+        di_issue<6, 6, 5, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i + 2, q); }, [](int) {}, tb, tb + DI_ACC);
       }
     }
     di_drain(sh);
@@ -915,25 +939,31 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(512u) : "memory");
 }
 
-constexpr int DI_IDX_ROW = TQ_D + 16, DI_OUT_ROW = 16 * 8 + 16;   // bytes between staged rows: 16 bytes on, no bank conflicts
-constexpr int DI_DEQUANT_SMEM = DI_DIGITS * DI_TILE + DI_ROWS * DI_IDX_ROW + DI_ROW_THREADS * DI_OUT_ROW + 128;
+constexpr int DI_IDX_ROW = TQ_D + 16;   // bytes between staged rows: 16 bytes on, no bank conflicts
+constexpr int DI_DEQUANT_SMEM = DI_DIGITS * DI_TILE + DI_ROW_THREADS * 128 + DI_ROWS * DI_IDX_ROW + 1024;
 
 // x_hat = (norm / ||c[idx]||) R^T c[idx] + shrink sqrt(pi/2)/sqrt(d) rnorm S^T z.  The signs z are one digit, +-1: seven products.
+// Once the sum s of a tile has been read, digit s of its operand is of no more use, and the rows write that digit of the next tile's: the MMAs
+// go on from tile to tile, while the rows add up the last sums and store.
 template <typename Tout, bool PROD, int SELFTEST = 0>
-__global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __grid_constant__ DiDequant A, int64_t n, Tout* __restrict__ out) {
+__global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __grid_constant__ DiDequant A, const __grid_constant__ CUtensorMap map,
+                                                                       int64_t n, Tout* __restrict__ out) {
   extern __shared__ __align__(128) uint8_t di_raw[];
   __shared__ DiShared sh;
-  __shared__ uint2 s_cdig[16];
+  __shared__ uint64_t s_digit[DI_DIGITS];       // digits of the operand, in place of a_ready, which is the signs'
   __shared__ uint32_t s_sign[16];               // four sketch bits, the first in bit 3, as +-1 digits
-  __shared__ double s_sq[16], s_part[4][DI_ROWS];
+  __shared__ double s_sq[16], s_part[2][4][DI_ROWS];
   const TqDenseDequant& a = A.q;
-  uint8_t* tiles_b = di_raw + (((sptr(di_raw) + 127u) & ~127u) - sptr(di_raw));
+  uint8_t* tiles_b = di_raw + (((sptr(di_raw) + 1023u) & ~1023u) - sptr(di_raw));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) di_init(sh);
+  if (tid == 0) {
+    for (int p = 0; p < DI_DIGITS; ++p)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sptr(&s_digit[p])), "r"(DI_ROW_THREADS / 32) : "memory");
+    di_init(sh);
+  }
   if (tid < 16) {
     const double c = tid < (1 << a.bits) ? a.cent[tid] : 0.0;
     s_sq[tid] = c * c;
-    s_cdig[tid] = di_digits_f64(c / A.cent_scale);
     uint32_t w = 0;
     for (int k = 0; k < 4; ++k) w |= ((tid >> (3 - k)) & 1 ? 0x01u : 0xffu) << (8 * k);
     s_sign[tid] = w;
@@ -948,18 +978,26 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
   const uint32_t tb = sh.tmem;
   const int64_t tiles = (n + DI_ROWS - 1) / DI_ROWS, step = gridDim.x;
   const int mine = (int)((tiles - blockIdx.x + step - 1) / step);
-  constexpr int PHASES = PROD ? 2 : 1;   // (the signs' product first)
+  constexpr int PHASES = PROD ? 2 : 1;   // (the signs' product last)
 
   if (warp == DI_COPIER) {
+    // (without a sketch R^T stays in place)
     if (lane == 0)
-      di_copier<SELFTEST>(sh, tiles_b, mine * PHASES, [&](int i) { return PROD && (i & 1) == 0 ? A.st : A.rt; }, [](int) { return DI_DIGITS; },
-                          [](int i, int) { return i; });
+      di_copier<SELFTEST>(sh, tiles_b, PROD ? mine * PHASES : mine > 0 ? 1 : 0, [&](int i) { return PROD && (i & 1) ? A.st : A.rt; },
+                          [](int) { return DI_DIGITS; }, [](int i, int) { return i; });
   } else if (warp == DI_MMA) {
     int item = 0;
     for (int i = 0; i < mine && !__any_sync(0xffffffffu, sh.failed); ++i) {
-      di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(i & 1));
-      if constexpr (PROD) di_issue<1, DI_DIGITS, DI_DIGITS - 1, SELFTEST>(sh, item, tiles_b, [&](int) { return 2 * i; }, tb + DI_SIGNS, tb + DI_ACC);
-      di_issue<DI_DIGITS, DI_DIGITS, DI_SUMS - 1, SELFTEST>(sh, item, tiles_b, [&](int) { return PROD ? 2 * i + 1 : i; }, tb, tb + DI_ACC);
+      // (sum 7 takes digits 1 to 6, sum 6 the leading one as well)
+      di_issue<DI_DIGITS, DI_DIGITS, DI_SUMS - 1, SELFTEST>(sh, item, tiles_b, [&](int) { return PROD ? 2 * i : 0; }, [&](int sum) {
+        if (sum == DI_SUMS - 1)
+          for (int p = 1; p < DI_DIGITS; ++p) di_wait<SELFTEST>(sh, &s_digit[p], (uint32_t)(i & 1));
+        if (sum == DI_SUMS - 2) di_wait<SELFTEST>(sh, &s_digit[0], (uint32_t)(i & 1));
+      }, tb, tb + DI_ACC);
+      if constexpr (PROD) {
+        di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(i & 1));
+        di_issue<1, DI_DIGITS, DI_DIGITS - 1, SELFTEST>(sh, item, tiles_b, [&](int) { return 2 * i + 1; }, [](int) {}, tb + DI_SIGNS, tb + DI_ACC);
+      }
     }
     di_drain(sh);
   } else {
@@ -967,8 +1005,8 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t area = tb + lanes, myacc = tb + DI_ACC + lanes + DI_COLS * h;
     const bool wide = (a.ld_out * sizeof(Tout)) % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-    uint8_t* xi = tiles_b + DI_DIGITS * DI_TILE;                           // indices of a tile
-    uint8_t* stage = xi + DI_ROWS * DI_IDX_ROW + warp * 32 * DI_OUT_ROW;   // 32 rows x 16 columns of this warp on their way out
+    uint8_t* stage = tiles_b + DI_DIGITS * DI_TILE + warp * 4096;          // 32 rows x 128 bytes of this warp on their way out
+    uint8_t* xi = tiles_b + DI_DIGITS * DI_TILE + DI_ROW_THREADS * 128;    // indices of a tile
     auto load_tile = [&](int64_t tile) {
       for (int i = tid; i < DI_ROWS * 8; i += DI_ROW_THREADS) {
         const int r = i >> 3, c = i & 7;
@@ -980,78 +1018,166 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int item = 0, t = 0;
-    if (mine > 0) load_tile(blockIdx.x);
-    for (; t < mine; ++t) {
-      const int64_t v0 = (blockIdx.x + t * step) * DI_ROWS, v = v0 + row;
-      const bool live = v < n;
-      const float norm = live ? a.norm[v] : 0.f, rnorm = PROD && live ? a.rnorm[v] : 0.f;
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      if (di_rows_any(sh.failed)) break;   // (in the tile before)
-      // ---- digits of the centroids, ||c||^2, signs ----
-      double cc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 1
-      for (int c = 0; c < DI_COLS / 8; ++c) {
-        const uint2 q = *reinterpret_cast<const uint2*>(xi + row * DI_IDX_ROW + DI_COLS * h + 8 * c);
-        uint2 u[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int m = ((k < 4 ? q.x : q.y) >> (8 * (k & 3))) & 15;
-          u[k] = s_cdig[m];
-          cc[k & 3] += s_sq[m];
-        }
-        di_store8<DI_DIGITS, 0>(area, 8 * h + 2 * c, u);
-        if constexpr (PROD) {   // eight sketch bits, the first in the most significant place
-          const uint32_t z = live ? a.qjl[v * 16 + 4 * h + c] : 0u;
-          di_st2(area + DI_SIGNS + 8 * h + 2 * c, s_sign[z >> 4], s_sign[z & 15]);
-        }
-      }
-      s_part[h][row] = (cc[0] + cc[1]) + (cc[2] + cc[3]);
+    auto ready = [&](uint64_t* bar) {   // what has been stored to tensor memory is there
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) di_arrive(&sh.a_ready);
-      di_rows_sync();
-      if (t + 1 < mine) load_tile(blockIdx.x + (t + 1) * step);
-      double f = 0.0, g = 0.0;
-      if (live) {
-        double cn = 1.0;
-        if (a.norm_correction) {
-          cn = sqrt((s_part[0][row] + s_part[1][row]) + (s_part[2][row] + s_part[3][row]));
-          cn = cn > 1e-10 ? cn : 1.0;
-        }
-        f = (double)norm / cn;
-        if constexpr (PROD) g = a.shrink * 1.2533141373155001 / sqrt((double)TQ_D) * (double)rnorm;   // turboquant/qjl.py:131-132
-        // a factor that is not finite: sums of terms of both signs, not a number
-        if (!(fabs(f) < 1e300)) f = __longlong_as_double(0x7ff8000000000000ll);
-        if (!(fabs(g) < 1e300)) g = __longlong_as_double(0x7ff8000000000000ll);
-        f *= A.r_scale * A.cent_scale;
-        g *= A.s_scale;
+      if (lane == 0) di_arrive(bar);
+    };
+    // of the next tile: indices, a nibble each, norms and the sketch bits of this thread's columns
+    uint32_t codes[4] = {}, signs = 0;
+    bool high = false;                                                     // indices above 7
+    float next_norm = 0.f, next_rnorm = 0.f;
+    auto prepare = [&](int t) {
+      const int64_t v = (blockIdx.x + t * step) * DI_ROWS + row;
+      next_norm = v < n ? a.norm[v] : 0.f;
+      if constexpr (PROD) {
+        next_rnorm = v < n ? a.rnorm[v] : 0.f;
+        signs = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) signs = (signs << 8) | (v < n ? a.qjl[v * 16 + 4 * h + k] : 0u);
       }
+      double cc[4] = {0.0, 0.0, 0.0, 0.0};
+      uint32_t any = 0;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const uint4 q = *reinterpret_cast<const uint4*>(xi + row * DI_IDX_ROW + DI_COLS * h + 16 * c);
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const uint32_t m = w[g] & 0x0f0f0f0fu, nibbles = __byte_perm(m | (m >> 4), 0, 0x4420);
+          any |= m;
+          if (g & 1) codes[2 * c + (g >> 1)] |= nibbles << 16; else codes[2 * c + (g >> 1)] = nibbles;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) cc[k] += s_sq[(m >> (8 * k)) & 15];
+        }
+      }
+      high = __any_sync(0xffffffffu, (any & 0x08080808u) != 0);
+      s_part[t & 1][h][row] = (cc[0] + cc[1]) + (cc[2] + cc[3]);
+    };
+    // digit p of the 32 centroids of this thread; a byte permute picks four (where a selector's fourth bit is set it repeats a sign bit instead)
+    auto write_digit = [&](int p) {
+      uint32_t w[8];
+      const uint32_t lo0 = A.words[p].x, lo1 = A.words[p].y, hi0 = A.words[p].z, hi1 = A.words[p].w;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t sel = i & 1 ? codes[i >> 1] >> 16 : codes[i >> 1];
+        w[i] = di_prmt(lo0, lo1, sel);
+        if (high) {
+          const uint32_t above = (di_prmt(0x80808080u, 0x80808080u, sel) & 0x01010101u) * 255u;
+          w[i] = (w[i] & ~above) | (di_prmt(hi0, hi1, sel & 0x7777u) & above);
+        }
+      }
+      asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                   ::"r"(area + 32 * p + 8 * h), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+    };
+    auto write_signs = [&]() {   // eight sketch bits a step, the first in the most significant place
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t z = (signs >> (24 - 8 * k)) & 255u;
+        di_st2(area + DI_SIGNS + 8 * h + 2 * k, s_sign[z >> 4], s_sign[z & 15]);
+      }
+      ready(&sh.a_ready);
+    };
+    int item = 0, t = 0;
+    if (mine > 0) {
+      load_tile(blockIdx.x);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      di_rows_sync();
+      prepare(0);
+      if constexpr (PROD) write_signs();
+#pragma unroll 1
+      for (int p = DI_DIGITS - 1; p >= 0; --p) write_digit(p);
+      for (int p = DI_DIGITS - 1; p >= 0; --p) ready(&s_digit[p]);
+      di_rows_sync();
+      if (mine > 1) load_tile(blockIdx.x + step);
+    }
+    for (; t < mine; ++t) {
+      const int64_t v0 = (blockIdx.x + t * step) * DI_ROWS, v = v0 + row;
+      const bool live = v < n, more = t + 1 < mine;
+      const float norm = next_norm, rnorm = next_rnorm;
       double acc[DI_COLS];
-      di_zero(acc);
-      if constexpr (PROD) di_take<DI_DIGITS - 1, SELFTEST>(sh, item, myacc, lane, g, acc);
-      di_take<DI_SUMS - 1, SELFTEST>(sh, item, myacc, lane, f, acc);
+      double f = 0.0, g = 0.0;
+      {
+        // sums 7 to 4, whole numbers of 2^-68 below 2^48.  The next tile's indices and this one's factors while the MMAs, which have the most to do
+        // here, are ahead; a digit is published after the sum behind the one that freed it: by then its store has come to an end
+        long long y[DI_COLS];
+        di_columns<SELFTEST>(sh, item++, myacc, lane, [&](int k, uint32_t x) { y[k] = (int32_t)x; });
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (di_rows_any(sh.failed)) break;
+        if (live) {
+          double cn = 1.0;
+          if (a.norm_correction) {
+            cn = sqrt((s_part[t & 1][0][row] + s_part[t & 1][1][row]) + (s_part[t & 1][2][row] + s_part[t & 1][3][row]));
+            cn = cn > 1e-10 ? cn : 1.0;
+          }
+          f = (double)norm / cn;
+          if constexpr (PROD) g = a.shrink * 1.2533141373155001 / sqrt((double)TQ_D) * (double)rnorm;   // turboquant/qjl.py:131-132
+          // a factor that is not finite: sums of terms of both signs, not a number
+          if (!(fabs(f) < 1e300)) f = __longlong_as_double(0x7ff8000000000000ll);
+          if (!(fabs(g) < 1e300)) g = __longlong_as_double(0x7ff8000000000000ll);
+          f *= A.r_scale * A.cent_scale;
+          g *= A.s_scale;
+        }
+        if (more) prepare(t + 1);
+        int32_t weight = 256;
+#pragma unroll 1
+        for (int sum = 6; sum > 3; --sum, weight <<= 8) {
+          di_columns<SELFTEST>(sh, item++, myacc, lane, [&](int k, uint32_t x) { y[k] += (long long)(int32_t)x * weight; });
+          if (more) {
+            if (sum < 6) ready(&s_digit[sum + 1]);
+            write_digit(sum);
+          }
+        }
+        const double unit = f * 0x1p-56;
+#pragma unroll
+        for (int k = 0; k < DI_COLS; ++k) acc[k] = di_double(y[k]) * unit;
+      }
+      double unit = f * 0x1p-24;
+#pragma unroll 1
+      for (int sum = 3; sum > 0; sum -= 2, item += 2, unit *= 65536.0) {   // (256 times the sum s - 1 <= 2 plus the sum s is below 2^31)
+        di_columns2<SELFTEST>(sh, item, myacc, lane, [&](int k, uint32_t x) { acc[k] = fma(di_double(x), unit, acc[k]); });
+        if (more) {
+          if (sum == 3) ready(&s_digit[4]);
+          else ready(&s_digit[3]), di_arrive_warp(&s_digit[2], lane);
+          write_digit(sum);
+          write_digit(sum - 1);
+        }
+      }
+      if (more) ready(&s_digit[1]), di_arrive_warp(&s_digit[0], lane);
+      di_rows_sync();                      // (the indices have been read)
+      if (t + 2 < mine) load_tile(blockIdx.x + (t + 2) * step);
+      if constexpr (PROD) {   // seven sums, below 2^14
+        unit = g * 0x1p-48;
+        di_columns<SELFTEST>(sh, item++, myacc, lane, [&](int k, uint32_t x) { acc[k] = fma(di_double(x), unit, acc[k]); });
+        unit *= 256.0;
+#pragma unroll 1
+        for (int sum = 5; sum > 0; sum -= 2, item += 2, unit *= 65536.0)
+          di_columns2<SELFTEST>(sh, item, myacc, lane, [&](int k, uint32_t x) { acc[k] = fma(di_double(x), unit, acc[k]); });
+        if (more) write_signs();
+      }
       Tout* o = out + v * a.ld_out + DI_COLS * h;
       if (a.accumulate && live) {
 #pragma unroll
         for (int k = 0; k < DI_COLS; ++k) acc[k] += di_d<Tout>(o[k]);
       }
-      if (sizeof(Tout) == 8 && wide) {
-        // Sixteen columns at a time through shared memory: a warp then stores whole lines, four rows an instruction (straight from
-        // the registers every store touched 32 lines: 4,400 clocks a tile)
+      if (sizeof(Tout) == 8 && A.tiled) {
+        // Sixteen columns at a time through shared memory, 16-byte chunks swizzled as the map has it, and out by a tiled copy that clips rows
+        // past n (plain stores of whole lines took 5,800 clocks of a tile's 24,000)
+        const int first = 32 * (warp & 3);
 #pragma unroll
         for (int c = 0; c < DI_COLS / 16; ++c) {
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();
 #pragma unroll
-          for (int k = 0; k < 16; k += 2) *reinterpret_cast<double2*>(stage + lane * DI_OUT_ROW + 8 * k) = make_double2(acc[16 * c + k], acc[16 * c + k + 1]);
+          for (int k = 0; k < 8; ++k)
+            *reinterpret_cast<double2*>(stage + 128 * lane + 16 * (k ^ (lane & 7))) = make_double2(acc[16 * c + 2 * k], acc[16 * c + 2 * k + 1]);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int r = 4 * i + (lane >> 3);
-            const double2 p = *reinterpret_cast<const double2*>(stage + r * DI_OUT_ROW + 16 * (lane & 7));
-            const int64_t vr = v0 + 32 * (warp & 3) + r;
-            if (vr < n) *reinterpret_cast<double2*>(out + vr * a.ld_out + DI_COLS * h + 16 * c + 2 * (lane & 7)) = p;
+          if (lane == 0 && v0 + first < n) {
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&map), "r"(DI_COLS * h + 16 * c),
+                         "r"((int)(v0 + first)), "r"(sptr(stage)) : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
       } else if (live && wide) {
@@ -1069,6 +1195,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (di_rows_any(sh.failed)) {   // the last tile begun and those behind it
       di_give_up<Tout>(a, t > 0 ? t - 1 : 0, mine, row, DI_COLS * h, n, out, A.status);
     }
@@ -1166,10 +1293,16 @@ template <typename Tin> int di_quantize(const DiQuant& A, const void* x, int64_t
     default: return di_quantize_bits<Tin, 4>(A, xt, ld, n, st);
   }
 }
-template <typename Tout> int di_dequantize(const DiDequant& A, int64_t n, void* out, cudaStream_t st) {
+template <typename Tout, bool PROD, int SELFTEST = 0> int di_dequantize_launch(DiDequant& A, int64_t n, Tout* out, cudaStream_t st) {
+  CUtensorMap map;
+  memset(&map, 0, sizeof(map));
+  A.tiled = sizeof(Tout) == 8 && tq_aligned(out, 16) && A.q.ld_out % 2 == 0 &&
+            tc_map(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, out, TQ_D, n, A.q.ld_out * 8, 16, 32);
+  return di_launch<k_dense_dequantize_i8<Tout, PROD, SELFTEST>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, map, n, out);
+}
+template <typename Tout> int di_dequantize(DiDequant& A, int64_t n, void* out, cudaStream_t st) {
   Tout* o = reinterpret_cast<Tout*>(out);
-  if (A.q.qjl) return di_launch<k_dense_dequantize_i8<Tout, true>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, o);
-  return di_launch<k_dense_dequantize_i8<Tout, false>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, o);
+  return A.q.qjl ? di_dequantize_launch<Tout, true>(A, n, o, st) : di_dequantize_launch<Tout, false>(A, n, o, st);
 }
 
 }  // namespace
@@ -1215,10 +1348,10 @@ double tq_dense_digits_centroids(const double* c, int n) {
   return ldexp(1.0, e);
 }
 
-// The digits of the first eight centroids, whole numbers of 2^-54 of the scale, as the kernels' operands are made from
-void tq_dense_digits_words(const double* c, int n, double scale, uint32_t (&words)[7][2]) {
+// The digits of the centroids, whole numbers of 2^-54 of the scale, as the kernels' operands are made from
+void tq_dense_digits_words(const double* c, int n, double scale, uint32_t (&words)[7][4]) {
   memset(words, 0, sizeof(words));
-  for (int i = 0; i < (n < 8 ? n : 8); ++i) {
+  for (int i = 0; i < n; ++i) {
     const uint64_t u = ((uint64_t)llrint(c[i] / scale * 18014398509481984.0) + 0x808080808080ull) ^ 0x808080808080ull;
     for (int p = 0; p < 7; ++p) words[p][i >> 2] |= (uint32_t)(uint8_t)(u >> (48 - 8 * p)) << (8 * (i & 3));
   }
@@ -1226,8 +1359,8 @@ void tq_dense_digits_words(const double* c, int n, double scale, uint32_t (&word
 
 // Calls that come here, us here / in the fp64 kernels (which take tiles of 16, 32 or 64 vectors, two CTAs an SM, and step up at 32
 // and 64 vectors per SM): quantize 4,096 vectors 14.6 / 14.6, 4,800 14.5 / 22.8, 9,472 14.6 / 22.8, 65,536 33 / 134; with the sketch 4,096
-// 27 / 27, 4,800 27 / 43, 12,000 27 / 94, 65,536 90 / 302; dequantize 8,192 19 / 17, 12,000 19 / 29, 65,536 62 / 90; with the sketch 4,096
-// 27 / 23, 6,000 27 / 31, 65,536 93 / 164.
+// 27 / 27, 4,800 27 / 43, 12,000 27 / 94, 65,536 90 / 302; dequantize 8,192 19 / 17, 12,000 19 / 29, 65,536 56 / 90; with the sketch 4,096
+// 27 / 23, 6,000 27 / 31, 65,536 85 / 164.
 static bool di_enough(int64_t n, bool dequantize, bool sketch) { return n > (dequantize && !sketch ? 64 : 32) * (int64_t)tq_num_sms(); }
 
 // The kernels' arguments; false: not of these kernels' kind
@@ -1269,6 +1402,7 @@ static bool di_dequant_args(const TqDenseDequant& a, const TqDenseDigits& g, DiD
   if (a.d != TQ_D || g.r_scale == 0.0 || g.cent_scale == 0.0 || !a.idx || (a.qjl && g.s_scale == 0.0)) return false;
   if (!tq_aligned(a.idx, 16)) return false;
   A.rt = g.rt; A.st = g.st;
+  for (int p = 0; p < DI_DIGITS; ++p) A.words[p] = make_uint4(g.words[p][0], g.words[p][1], g.words[p][2], g.words[p][3]);
   A.r_scale = g.r_scale / 4096.0;
   A.s_scale = g.s_scale / 64.0;
   A.cent_scale = g.cent_scale;
@@ -1308,5 +1442,5 @@ int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, 
 int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st) {
   DiDequant A;
   TQ_REQUIRE(a.qjl && di_dequant_args(a, q->dig, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED, "self-test of the dense dequantizer: 128 elements and a sketch");
-  return di_launch<k_dense_dequantize_i8<double, true, 26>>(DI_DEQUANT_SMEM, n, st, "k_dense_dequantize_i8", A, n, out);
+  return di_dequantize_launch<double, true, 26>(A, n, out, st);
 }

@@ -35,12 +35,12 @@ struct TqDenseDigits {
   double r_rows, r_length;          // the largest sum of magnitudes of a row of R, and the longest row's length, over r_scale
   double cent_scale;                // a power of two above every centroid's magnitude
   double bnd[15];                   // boundaries
-  uint32_t words[7][2];             // digit p of centroids 0-3 and 4-7, a byte each
+  uint32_t words[7][4];             // digit p of the centroids, a byte each
 };
 #define TQ_DENSE_DIGITS_BYTES (7 * TQ_D * TQ_D)
 double tq_dense_digits_scale(const double* m, double* rows, double* length);
 double tq_dense_digits_centroids(const double* c, int n);
-void tq_dense_digits_words(const double* c, int n, double scale, uint32_t (&words)[7][2]);
+void tq_dense_digits_words(const double* c, int n, double scale, uint32_t (&words)[7][4]);
 
 struct tq_quantizer {
   int32_t d, bits, rotation, norm_correction, qjl, device;

@@ -27,7 +27,6 @@
 //
 // 1,048,576 fp16 vectors of turbo3: 106 -> 87 us (3.7 TB/s; HBM would take 49); the arithmetic on the coordinates bounds it, most of it
 // on the half-rate compare and packed fp32 pipes.  Scales are within 4e-7 of 64 bits, as the warp-level kernel's.
-#include <cuda.h>
 #include <type_traits>
 #include "tq_quantize_math.cuh"
 #include "tq_tcgen05.cuh"
@@ -460,24 +459,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
 
 // the rows as a tensor of n x 128 16-bit elements, copied in boxes of 128 x 64; false where no such map can be made
 bool qt_map(CUtensorMap* map, const void* x, int32_t dtype, int64_t ld, int64_t n) {
-  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static const Encode encode = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult found;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
-        found != cudaDriverEntryPointSuccess) {
-      (void)cudaGetLastError();
-      p = nullptr;
-    }
-    return reinterpret_cast<Encode>(p);
-  }();
-  if (!encode || n > 0x7fffff00LL) return false;   // (box coordinates are 32-bit)
-  const cuuint64_t dims[2] = {TQ_D, (cuuint64_t)n}, strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {64, TQ_D}, ones[2] = {1, 1};
-  return encode(map, dtype == TQ_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides,
-                box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return tc_map(map, dtype == TQ_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, TQ_D, n, ld * 2, 64, TQ_D);
 }
 
 template <typename Tin, int BITS, bool NORMC, bool SELFTEST = false>

@@ -1,8 +1,31 @@
 // Fifth-generation tensor cores (tcgen05): descriptors, tensor-memory loads and stores, bounded mbarrier waits.
 #pragma once
+#include <cuda.h>
 #include "tq_internal.cuh"
 
 namespace {
+
+// cuTensorMapEncodeTiled for a matrix of `rows` rows of `columns` elements, `pitch` bytes apart, in boxes of box_columns (128 bytes) x box_rows,
+// 128-byte swizzle; false where no such map can be made
+inline bool tc_map(CUtensorMap* map, CUtensorMapDataType type, const void* x, int64_t columns, int64_t rows, int64_t pitch, int box_columns, int box_rows) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      (void)cudaGetLastError();
+      p = nullptr;
+    }
+    return reinterpret_cast<Encode>(p);
+  }();
+  if (!encode || rows > 0x7fffff00LL) return false;   // (box coordinates are 32-bit)
+  const cuuint64_t dims[2] = {(cuuint64_t)columns, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch};
+  const cuuint32_t box[2] = {(cuuint32_t)box_columns, (cuuint32_t)box_rows}, ones[2] = {1, 1};
+  return encode(map, type, 2, const_cast<void*>(x), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 constexpr long long TC_WAIT_CYCLES = 1LL << 30;
 
