@@ -421,3 +421,20 @@ def test_input_dtypes_and_errors(tq):
     for n in (1, 2, 3, 5, 33):
         r = q.quantize_device(torch.as_tensor(x[:n]).cuda(), packed=True)
         assert torch.equal(r["packed"], a["packed"][:n]) and torch.equal(r["norm"], a["norm"][:n])
+
+
+@pytest.mark.parametrize("rows,d", [(1, 16), (3, 48), (17, 128), (1, 128), (2049, 128), (5, 8), (7, 21), (9, 24)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_sign_bits_by_pieces(rows, d, shift):
+    """Rows of a multiple of sixteen signs move by aligned pieces, others and unaligned ones byte by byte; any int8: above zero is a set bit."""
+    import torch
+    from turboquant_plus_b200 import _native as nv
+    rng = np.random.default_rng(rows * d)
+    signs = rng.integers(-128, 128, (rows, d)).astype(np.int8)
+    signs[rng.random((rows, d)) < 0.2] = 0
+    packed = np.packbits(signs > 0, axis=1)
+    flat = torch.empty(rows * d + shift, dtype=torch.int8, device="cuda")[shift:]
+    s = flat.view(rows, d).copy_(torch.from_numpy(signs))
+    assert np.array_equal(nv.host().sign_bits(s, d, True).cpu().numpy(), packed)
+    bits = torch.empty(packed.size + shift, dtype=torch.uint8, device="cuda")[shift:].view(packed.shape).copy_(torch.from_numpy(packed))
+    assert np.array_equal(nv.host().sign_bits(bits, d, False).cpu().numpy(), np.where(signs > 0, 1, -1))

