@@ -1,6 +1,7 @@
 """Host-side logic that needs no GPU: constants, size formulae, error behaviour, no CPU fallback."""
 import numpy as np
 import pytest
+import torch
 
 import turboquant_plus_b200 as tq
 from turboquant_plus_b200 import codebook, rotation, utils
@@ -67,3 +68,40 @@ def test_no_cpu_fallback():
         utils.pack_bits(np.ones(8, np.int8))
     with pytest.raises(RuntimeError, match="no CPU fallback"):
         tq.PagedKVCache(128, 8, 4)
+
+
+@pytest.mark.parametrize("layers,heads,rows,width", [(1, 1, 5, 128), (4, 8, 25, 128), (3, 2, 7, 3), (2, 3, 0, 128), (5, 1, 1, 0)])
+def test_runs_of_rows(layers, heads, rows, width):
+    """cut gives views, join makes one view of runs that lie one after the other and a copy of others."""
+    from turboquant_plus_b200 import _native as nv
+    host = nv.host()
+    t = torch.arange(layers * heads * rows * max(width, 1), dtype=torch.float32).reshape(-1, *([width] if width else []))
+    if t.dim() == 1:
+        t = t[:layers * heads * rows]
+    runs = host.cut(t, layers, heads)
+    flat = [r for layer in runs for r in layer]
+    assert len(runs) == layers and all(len(layer) == heads for layer in runs)
+    assert all(torch.equal(r, t[i * rows:(i + 1) * rows]) for i, r in enumerate(flat))
+    assert not rows or flat[-1].data_ptr() == t[(len(flat) - 1) * rows:].data_ptr()
+    whole = host.join(flat)
+    assert torch.equal(whole, t) and whole.is_contiguous() and (not rows or whole.data_ptr() == t.data_ptr())
+    for other in (flat[::-1], [r.clone() for r in flat], flat + flat, [r.flip(0) for r in flat], [torch.cat([r, r])[::2] for r in flat]):
+        assert torch.equal(host.join(other), torch.cat(other))
+    odd = torch.zeros(1 + t.numel())[1:].reshape(t.shape).copy_(t)       # runs that no kernel's aligned loads could take
+    pieces = [r for layer in host.cut(odd, layers, heads) for r in layer]
+    assert torch.equal(host.join(pieces), t) and (len(pieces) < 2 or not rows or host.join(pieces).data_ptr() != odd.data_ptr())
+
+
+def test_runs_of_rows_refuses():
+    from turboquant_plus_b200 import _native as nv
+    host, t = nv.host(), torch.zeros(6, 4)
+    for bad in ((t, 4, 1), (t, 0, 2), (torch.tensor(1.0), 1, 1)):
+        with pytest.raises(ValueError):
+            host.cut(*bad)
+    for bad in ([], (t, t)):
+        with pytest.raises(ValueError):
+            host.join(bad)
+    with pytest.raises(TypeError):
+        host.join([t, 3])
+    with pytest.raises(RuntimeError):
+        host.join([t, torch.zeros(6, 5)])

