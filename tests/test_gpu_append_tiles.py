@@ -2,7 +2,7 @@
 kernel takes: vectors around a tile's edge, head counts that leave a ragged last tile, zero rows, tokens without a slot, rows of
 exact zeros, of both ends of their type's range and beyond it, plain packed arrays.
 Both form every sum behind an index in the same order: indices are equal.  Scales come from sums of counts in another order:
-six roundings of 2^-24 in all.  PROD keys take the warp-level kernel at every length: all of their record is equal."""
+six roundings of 2^-24 in all.  PROD keys form all of their sums in the same order: all of their record is equal."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -18,15 +18,18 @@ def _fields(cache):
     return out
 
 
-# vectors per SM from which two tensors of one format, and one beside another kernel, take the tile kernel
+# vectors per SM from which two tensors of one format, one beside another kernel, and PROD keys, take the tile kernel
 PAIR, ALONE = 166, 1776
+SKETCH = 332
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 @pytest.mark.parametrize("k,v,heads,per_sm,more", [("turbo2", "turbo2", 1, PAIR, 0), ("turbo3", "turbo3", 1, PAIR, -1), ("turbo3", "turbo3", 3, PAIR, 2),
                                                    ("turbo4", "turbo4", 8, PAIR, 8), ("turbo3", "turbo3", 1, PAIR, 135), ("turbo3", "turbo3", 3, 512, 1),
                                                    ("turbo2", "turbo2", 8, 880, 8), ("turbo4", "turbo4", 3, 880, 2), ("q8_0", "turbo2", 8, ALONE, 8),
-                                                   ("q8_0", "turbo4", 3, ALONE, 2), ("turbo3", "turbo3", 8, ALONE, 136), ("prod3", "turbo3", 3, 1923, 0)])
+                                                   ("q8_0", "turbo4", 3, ALONE, 2), ("turbo3", "turbo3", 8, ALONE, 136), ("prod3", "turbo3", 3, 1923, 0),
+                                                   ("prod3", "turbo3", 1, SKETCH, 0), ("prod3", "turbo2", 3, SKETCH, -1), ("prod4", "turbo4", 8, SKETCH, 136),
+                                                   ("prod4", "turbo3", 3, 512, 1), ("prod3", "turbo3", 8, 1333, 8)])
 def test_long_append_equals_short_ones(k, v, heads, per_sm, more, dtype):
     import torch
     import turboquant_plus_b200 as tq
@@ -119,6 +122,34 @@ def test_odd_rows_of_long_appends(fmt, heads, norm_correction, dtype):
         assert torch.equal(a[t], b[t])
         sa, sb = a[t + "_scale"], b[t + "_scale"]
         assert bool((((sa - sb).abs() <= 6 * 2.0 ** -24 * sb.abs()) | (sa == sb) | (sa.isnan() & sb.isnan())).all())
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("norm_correction", [True, False])
+@pytest.mark.parametrize("fmt,heads", [("prod3", 1), ("prod3", 8), ("prod4", 3)])
+def test_odd_rows_of_long_appends_of_keys_with_a_sketch(fmt, heads, norm_correction, dtype):
+    """Zero residuals and projections among them; rows beyond the type's range and not finite ones have the same indices."""
+    import torch
+    import turboquant_plus_b200 as tq
+    tokens = -(-SKETCH * torch.cuda.get_device_properties(0).multi_processor_count // heads) + 5
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    rows = _odd_rows(tokens, heads, dtype, gen)
+    n_pages = -(-tokens // 128)
+    slots = torch.arange(tokens, device="cuda")
+    got = []
+    for piece in (tokens, 1000):
+        cache = tq.PagedKVCache(D, heads, n_pages, 128, fmt, "turbo2", seed=42, norm_correction=norm_correction)
+        cache.pool.zero_()
+        for lo in range(0, tokens, piece):
+            cache.append(rows[lo:lo + piece], rows[lo:lo + piece], slots[lo:lo + piece])
+        got.append(_fields(cache))
+    a, b = got
+    assert torch.equal(a["k"], b["k"])
+    i = torch.arange(n_pages * 128 * heads, device="cuda") % 12
+    plain = ((i != 9) & (i != 10)).view(n_pages, 128, heads).transpose(1, 2)
+    for name in a:
+        if name.startswith("k"):
+            assert torch.equal(a[name][plain], b[name][plain]), name
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])

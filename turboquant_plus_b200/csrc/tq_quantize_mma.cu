@@ -714,7 +714,7 @@ bool tq_quantize_mma_try_pair(const TqFast& f0, const void* x0, const TqQuantDst
   j0.f = f0; j0.x = x0; j0.dst = d0;
   j1.f = f1; j1.x = x1; j1.dst = d1;
   const bool normc = f0.norm_correction && d0.scale;
-  if (tq_quantize_tc_try(f0, x0, d0, &f1, x1, &d1, dtype, ld, n, normc, st, rc)) return true;
+  if (tq_quantize_tc_try(f0, x0, d0, &f1, x1, &d1, dtype, ld, n, normc, false, st, rc)) return true;
 #define TQ_CASE(B)                                                                              \
   case B:                                                                                       \
     *rc = dtype == TQ_F16    ? launch_mma_pair<__half, B>(j0, j1, ld, n, normc, st)             \
@@ -734,7 +734,7 @@ bool tq_quantize_mma_try_pair(const TqFast& f0, const void* x0, const TqQuantDst
 bool tq_quantize_mma_try(const TqFast& f, const void* x, int32_t dtype, int64_t ld, int64_t n, const TqQuantDst& dst,
                          bool want_qjl, cudaStream_t st, int* rc) {
   if (!qm_serves(f, dtype, ld, dst, want_qjl)) return false;
-  if (!want_qjl && tq_quantize_tc_try(f, x, dst, nullptr, nullptr, nullptr, dtype, ld, n, f.norm_correction && dst.scale, st, rc)) return true;
+  if (tq_quantize_tc_try(f, x, dst, nullptr, nullptr, nullptr, dtype, ld, n, f.norm_correction && dst.scale, want_qjl, st, rc)) return true;
 #define TQ_CASE(B)                                                                                           \
   case B:                                                                                                    \
     *rc = dtype == TQ_F16    ? launch_mma<__half, B>(f, (const __half*)x, ld, n, dst, want_qjl, st)               \

@@ -18,9 +18,11 @@
 //   * thresholds are scaled by the vector's norm; a magnitude level is found bit by bit, the threshold of the next bit picked
 //     arithmetically; eight indices are an exact fp32 Horner sum; sign2 mirrors an index, an XOR of the packed words; level
 //     counts, exact small integers, give the norm correction.
-//   * PROD keys stay with the warp-level kernel: the two transforms of their sign sketch are one product with an integer matrix
-//     here (1,048,576 keys 228 -> 129 us), but its sums round in another order, and of 33.6 M sketch bits some four then
-//     differ, which a key that a softmax rests on shows.
+//   * PROD keys (2 or 3 index bits): the residual and the two 128-point transforms of the sign sketch are butterflies in a thread's registers,
+//     64 values at a time and back to tensor memory in between (qt_sketch), every sum in the warp-level kernel's order, so that a
+//     key's record is the same at every length.  (The two transforms as one product with an integer matrix are a third faster, but round
+//     otherwise: of 33.6 M sketch bits some four then differ, which a key that a softmax rests on shows.)  The warp-level kernel does the
+//     same butterflies with 128 lane exchanges a vector and 134 warp-instructions: 1,048,576 keys with 2 index bits 228 -> 165 us.
 //   * a wait that gives up ends the other roles' waits too; the vectors whose indices were not found then have norms and factors that
 //     are not a number, and a status word is set (tq_quantize_status_sync).
 //   * loops over the columns stay loops: unrolled, a tile's code misses the instruction caches.
@@ -40,8 +42,10 @@ namespace {
 //     turbo4 24,576 12.5 / 13.1, 65,536 23.4 / 25.1; turbo2 24,576 7.7 / 8.1, 65,536 13.6 / 14.2
 //   one tensor beside another kernel: q8_0 / turbo3 131,072 27.2 / 27.7, 262,144 51.2 / 51.4, 1,048,576 171 / 190; q8_0 / turbo2
 //     131,072 25.7 / 24.7, 262,144 45.8 / 45.7, 1,048,576 147 / 168
+//   PROD keys and the V rows beside them: prod3 / turbo3 32,768 15.1 / 13.8, 49,152 19.3 / 19.7, 65,536 23.6 / 25.5, 1,048,576 250 / 302;
+//     prod4 / turbo4 32,768 19.5 / 17.4, 49,152 25.0 / 25.1, 65,536 31.0 / 32.6, 1,048,576 382 / 451
 // In vectors per SM (148), so that a device with fewer SMs takes the step earlier.
-inline int64_t qt_min_vectors(bool pair) { return (int64_t)tq_num_sms() * (pair ? 166 : 1776); }
+inline int64_t qt_min_vectors(bool pair, bool sketch) { return (int64_t)tq_num_sms() * (pair ? 166 : sketch ? 332 : 1776); }
 
 struct QtJob {
   CUtensorMap map;   // of the rows: 64 elements x 128 rows a box, 128-byte swizzle
@@ -105,7 +109,7 @@ template <int BITS> struct QtLevels {
 template <int BITS> struct QtCounts {
   float2 s1, s2, s21, s4, s42, s41, s421;
   __device__ __forceinline__ void zero() { s1 = s2 = s21 = s4 = s42 = s41 = s421 = make_float2(0.f, 0.f); }
-  __device__ __forceinline__ void add(float2 p4, float2 p2, float2 p1) {
+  __device__ __forceinline__ void add(int, float2 p4, float2 p2, float2 p1) {
     s1 = qm_add2(s1, p1);
     if constexpr (BITS >= 3) {
       s2 = qm_add2(s2, p2);
@@ -144,9 +148,38 @@ template <int BITS> struct QtCounts {
   }
 };
 
+// The same for keys with a sketch (2 or 3 bits), where the factor goes into the residual and with it into signs: a sum for each of the four
+// lanes that share a vector in the warp-level kernel (every fourth group of four columns), joined as there.  The three counts of three
+// bits, at most 32 each, are digits of one exact fp32 number.
+template <int BITS> struct QtLaneCounts {
+  float2 s[4];
+  __device__ __forceinline__ void zero() { s[0] = s[1] = s[2] = s[3] = make_float2(0.f, 0.f); }
+  __device__ __forceinline__ void add(int e, float2, float2 p2, float2 p1) {
+    float2& t = s[(e & 15) >> 2];
+    t = qm_add2(t, p1);
+    if constexpr (BITS == 3) t = qm_fma2(p2, qm_fma2(p1, qm_dup(4096.f), qm_dup(64.f)), t);
+  }
+  __device__ __forceinline__ float squares(const float (&cent)[16]) const {
+    constexpr int H = 1 << (BITS - 1);
+    auto step = [&](int j) { return cent[H + j] * cent[H + j] - cent[H + j - 1] * cent[H + j - 1]; };
+    float part[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float v = s[t].x + s[t].y;
+      if constexpr (BITS == 2) {
+        part[t] = __fmul_rn(v, step(1));   // (not part of the sums below)
+      } else {
+        const uint32_t n = __float2uint_rn(v), a1 = n & 63u, a2 = (n >> 6) & 63u, a21 = n >> 12;
+        part[t] = fmaf((float)a2, step(2), fmaf((float)a21, step(3), (float)(a1 + a2 - a21) * step(1)));
+      }
+    }
+    return (part[0] + part[1]) + (part[2] + part[3]);
+  }
+};
+
 // 32 coordinates (minus the rotated values) -> BITS words of the packed stream, most significant bit first
-template <int BITS, bool COUNT>
-__device__ __forceinline__ void qt_pack32(const uint32_t (&nu)[32], const QtLevels<BITS>& lv, QtCounts<BITS>& cnt, uint32_t (&out)[BITS]) {
+template <int BITS, bool COUNT, class CNT>
+__device__ __forceinline__ void qt_pack32(const uint32_t (&nu)[32], const QtLevels<BITS>& lv, CNT& cnt, uint32_t (&out)[BITS]) {
   constexpr int NC = 1 << BITS, HG = BITS == 4 ? 4 : 8;   // digits per exact fp32 Horner sum (at most 24 bits)
   constexpr float RADIX = (float)NC, HALF = (float)(NC / 2);
   constexpr float OFF = (HALF - 0.5f) * (float)(((1u << (HG * BITS)) - 1) / (NC - 1));
@@ -159,7 +192,7 @@ __device__ __forceinline__ void qt_pack32(const uint32_t (&nu)[32], const QtLeve
       const uint32_t u0 = nu[q * HG + k], u1 = nu[q * HG + k + 1];
       float2 p4, p2, p1;
       lv.test(make_float2(fabsf(__uint_as_float(u0)), fabsf(__uint_as_float(u1))), p4, p2, p1);
-      if constexpr (COUNT) cnt.add(p4, p2, p1);
+      if constexpr (COUNT) cnt.add(q * HG + k, p4, p2, p1);
       float2 m5 = qm_add2(p1, qm_dup(0.5f));
       if constexpr (BITS >= 3) m5 = qm_fma2(p2, qm_dup(2.0f), m5);
       if constexpr (BITS == 4) m5 = qm_fma2(p4, qm_dup(4.0f), m5);
@@ -234,6 +267,112 @@ __device__ __forceinline__ void qt_st8(uint32_t addr, const uint32_t (&v)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
+// sixteen columns at v[at ..], no wait, and back; qt_wait64 orders every use of v behind the loads
+__device__ __forceinline__ void qt_ld16(uint32_t addr, float* v) {
+  uint32_t* u = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]),
+                 "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void qt_st16(uint32_t addr, const float* v) {
+  const uint32_t* u = reinterpret_cast<const uint32_t*>(v);
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(addr), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]), "r"(u[10]),
+               "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15]) : "memory");
+}
+__device__ __forceinline__ void qt_wait64(float (&v)[64]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 64; i += 8)
+    asm volatile("" : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[i + 2]), "+f"(v[i + 3]), "+f"(v[i + 4]), "+f"(v[i + 5]), "+f"(v[i + 6]), "+f"(v[i + 7]));
+}
+// the butterfly of distance H: a + b and a - b
+template <int H> __device__ __forceinline__ void qt_butterfly(float (&v)[64]) {
+#pragma unroll
+  for (int i = 0; i < 64; i += H == 1 ? 2 : 1)
+    if constexpr (H == 1) {
+      const float a = v[i], b = v[i + 1];
+      v[i] = a + b;
+      v[i + 1] = a - b;
+    } else if ((i & H) == 0 && (i & 1) == 0) {
+      const float2 a = make_float2(v[i], v[i + 1]), b = make_float2(v[i + H], v[i + H + 1]);
+      const float2 p = qm_add2(a, b), m = qm_sub2(a, b);
+      v[i] = p.x; v[i + 1] = p.y;
+      v[i + H] = m.x; v[i + H + 1] = m.y;
+    }
+}
+
+// Keys with a sketch: the residual -(u - c cs) of the values (minus u) at `tm`, its squares' sum, and the sketch words (the first column in
+// the most significant bit, before the last signs) -- two 128-point transforms with the signs `mid` between them, all in the order of the
+// warp-level kernel, whose bits these are: butterflies of distances 1 to 64, of which 64 registers hold six; the seventh, and the last two
+// of the second transform, take the columns from tensor memory again, 32 (or 16) of either half (quarter).
+template <int BITS>
+__device__ __forceinline__ float qt_sketch(uint32_t tm, const QtLevels<BITS>& lv, const float (&cent)[16], float cs, const float* mid, uint32_t (&words)[4]) {
+  constexpr int H = 1 << (BITS - 1);
+  float2 ee[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) ee[t] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    float v[64];
+#pragma unroll
+    for (int c = 0; c < 64; c += 16) qt_ld16(tm + 64 * half + c, v + c);
+    qt_wait64(v);
+#pragma unroll
+    for (int k = 0; k < 64; k += 2) {
+      const float2 nu = make_float2(v[k], v[k + 1]);
+      float2 p4, p2, p1, cm;
+      lv.test(make_float2(fabsf(nu.x), fabsf(nu.y)), p4, p2, p1);
+      if constexpr (BITS == 3) {   // level 2 p2 + p1
+        const float2 base = qm_fma2(p2, qm_dup(cent[6] - cent[4]), qm_dup(cent[4]));
+        const float2 slope = qm_fma2(p2, qm_dup((cent[7] - cent[6]) - (cent[5] - cent[4])), qm_dup(cent[5] - cent[4]));
+        cm = qm_fma2(p1, slope, base);
+      } else {
+        cm = qm_fma2(p1, qm_dup(cent[H + 1] - cent[H]), qm_dup(cent[H]));
+      }
+      cm.x = __int_as_float(__float_as_int(cm.x) | (~__float_as_int(nu.x) & 0x80000000));
+      cm.y = __int_as_float(__float_as_int(cm.y) | (~__float_as_int(nu.y) & 0x80000000));
+      const float2 r = qm_fma2(cm, qm_dup(cs), nu);
+      ee[(k & 15) >> 2] = qm_fma2(r, r, ee[(k & 15) >> 2]);
+      v[k] = r.x; v[k + 1] = r.y;
+    }
+    qt_butterfly<1>(v); qt_butterfly<2>(v); qt_butterfly<4>(v); qt_butterfly<8>(v); qt_butterfly<16>(v); qt_butterfly<32>(v);
+#pragma unroll
+    for (int c = 0; c < 64; c += 16) qt_st16(tm + 64 * half + c, v + c);
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll 1
+  for (int part = 0; part < 2; ++part) {   // columns 32 part .. + 31 of both halves
+    float v[64];
+#pragma unroll
+    for (int c = 0; c < 32; c += 16) qt_ld16(tm + 32 * part + c, v + c), qt_ld16(tm + 64 + 32 * part + c, v + 32 + c);
+    qt_wait64(v);
+    qt_butterfly<32>(v);
+#pragma unroll
+    for (int k = 0; k < 64; k += 4) {
+      const float4 m = *reinterpret_cast<const float4*>(mid + 32 * part + (k & 31) + 2 * (k & 32));
+      const float2 a = qm_mul2(make_float2(v[k], v[k + 1]), make_float2(m.x, m.y)), b = qm_mul2(make_float2(v[k + 2], v[k + 3]), make_float2(m.z, m.w));
+      v[k] = a.x; v[k + 1] = a.y; v[k + 2] = b.x; v[k + 3] = b.y;
+    }
+    qt_butterfly<1>(v); qt_butterfly<2>(v); qt_butterfly<4>(v); qt_butterfly<8>(v); qt_butterfly<16>(v);
+#pragma unroll
+    for (int c = 0; c < 32; c += 16) qt_st16(tm + 32 * part + c, v + c), qt_st16(tm + 64 + 32 * part + c, v + 32 + c);
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll 1
+  for (int part = 0; part < 2; ++part) {   // columns 16 part .. + 15 of the four quarters
+    float v[64];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) qt_ld16(tm + 32 * c + 16 * part, v + 16 * c);
+    qt_wait64(v);
+    qt_butterfly<16>(v); qt_butterfly<32>(v);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int k = 0; k < 16; ++k) words[c] = __funnelshift_l(__float_as_uint(v[16 * c + k]), words[c], 1);
+  }
+  return ((ee[0].x + ee[0].y) + (ee[1].x + ee[1].y)) + ((ee[2].x + ee[2].y) + (ee[3].x + ee[3].y));
+}
 __device__ __forceinline__ void qt_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sptr(bar)) : "memory");
 }
@@ -249,12 +388,13 @@ __device__ __noinline__ void qt_give_up(const TqQuantDst& dst, int i, int mine, 
     const int64_t rec = tq_dst_record(dst, v, within, good);
     if (good && dst.scale) *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.scale) + rec + within * 4) = nan;
     if (dst.norm) dst.norm[v] = nan;
+    if (good && dst.rnorm) *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.rnorm) + rec + within * 4) = nan;
   }
   if (status) *status = 1;
 }
 
 // SELFTEST: the first CTA's second tile is never reported as multiplied, and waits are short
-template <typename Tin, int BITS, bool NORMC, bool SELFTEST = false>
+template <typename Tin, int BITS, bool NORMC, bool SELFTEST = false, bool QJLS = false>
 __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_constant__ QtJob j0, const __grid_constant__ QtJob j1,
                                                                          int64_t n, int32_t* status) {
   constexpr long long LIMIT = SELFTEST ? TC_SELFTEST_CYCLES : TC_WAIT_CYCLES;
@@ -264,6 +404,8 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_failed;   // a wait gave up: nobody waits any more
   __shared__ __align__(16) uint32_t s_flip[4 * BITS];
+  __shared__ __align__(16) float s_mid[QJLS ? TQ_D : 4];   // signs between the transforms of the sketch
+  __shared__ __align__(16) uint32_t s_last[4];             // ... and behind them, as bits in the order of the sketch words
   const QtJob& job = blockIdx.y == 0 ? j0 : j1;
   const TqFast& f = job.f;
   const TqQuantDst& dst = job.dst;
@@ -297,6 +439,11 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
 #pragma unroll
       for (int k = 0; k < 32; ++k) w |= qm_bit(f.s2, (32 * (tid - 256) + k) / BITS) << (8 * (k >> 3) + 7 - (k & 7));
       s_flip[tid - 256] = w;
+    } else if (QJLS && tid >= 288 && tid < 288 + TQ_D) {
+      const int e = tid - 288;
+      s_mid[e] = qm_bit(f.s1, e) ^ qm_bit(f.j1, e) ? -1.f : 1.f;
+    } else if (QJLS && tid >= 416 && tid < 420) {
+      s_last[tid - 416] = __brev(f.j2[tid - 416]);
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -412,7 +559,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
     const float ts = safe * TQ_SQRT_D;                  // the sums are y * ||x|| * sqrt(d), y the rotated unit vector
     QtLevels<BITS> lv;
     lv.init(f.bnd, ts);
-    QtCounts<BITS> cnt;
+    std::conditional_t<QJLS, QtLaneCounts<BITS>, QtCounts<BITS>> cnt;
     cnt.zero();
     // ---- indices: 64 coordinates a turn, 8 BITS bytes ----
     // a zero vector takes the index of the value 0 in every coordinate
@@ -434,10 +581,13 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
         else if (k % 4 == 0) reinterpret_cast<uint4*>(p)[k / 4] = make_uint4(w[k], w[k + 1], w[k + 2], w[k + 3]);
       }
     });
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");   // the accumulator is free
-    __syncwarp();
-    if (lane == 0) qt_arrive(&d_free[sl]);
     float invn = 1.0f;
+    auto free_slot = [&]() {
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) qt_arrive(&d_free[sl]);
+    };
+    if constexpr (!QJLS) free_slot();
     if constexpr (NORMC) {
       float cn = sqrtf(fmaf((float)TQ_D, f.cent[HALF] * f.cent[HALF], cnt.squares(f.cent)));
       cn = cn > 1e-10f ? cn : 1.0f;                      // turboquant/polar_quant.py:110-111
@@ -445,6 +595,21 @@ __global__ void __launch_bounds__(QT_THREADS, 1) k_quantize_tc(const __grid_cons
     }
     if (good && dst.scale) {
       *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.scale) + rec + within * 4) = nrm * invn;
+    }
+    if constexpr (QJLS) {
+      uint32_t words[4] = {};
+      const float ee = qt_sketch<BITS>(tm, lv, f.cent, invn * ts, s_mid, words);
+      free_slot();
+      const float rn = nrm > 0.f ? sqrtf(ee) * TQ_RSQRT_D : 0.f;   // ||r|| = ||x|| * ||y - yhat'||
+      // (the values were minus the projections: a sign bit is a sketch bit; a zero input has no residual: all +1)
+      uint4 z;
+      z.x = nrm > 0.f ? __byte_perm(words[0] ^ s_last[0], 0, 0x0123) : 0xffffffffu;
+      z.y = nrm > 0.f ? __byte_perm(words[1] ^ s_last[1], 0, 0x0123) : 0xffffffffu;
+      z.z = nrm > 0.f ? __byte_perm(words[2] ^ s_last[2], 0, 0x0123) : 0xffffffffu;
+      z.w = nrm > 0.f ? __byte_perm(words[3] ^ s_last[3], 0, 0x0123) : 0xffffffffu;
+      if (good && dst.qjl) *reinterpret_cast<uint4*>(dst.qjl + rec + within * 16) = z;
+      if (good && dst.rnorm)   // sqrt(pi/2)/sqrt(d): turboquant/qjl.py:32,131
+        *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(dst.rnorm) + rec + within * 4) = dst.rscale_const ? rn * (1.2533141373155001f * TQ_RSQRT_D) : rn;
     }
     if (v < n && dst.norm) dst.norm[v] = nrm;
   }
@@ -462,9 +627,9 @@ bool qt_map(CUtensorMap* map, const void* x, int32_t dtype, int64_t ld, int64_t 
   return tc_map(map, dtype == TQ_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, TQ_D, n, ld * 2, 64, TQ_D);
 }
 
-template <typename Tin, int BITS, bool NORMC, bool SELFTEST = false>
+template <typename Tin, int BITS, bool NORMC, bool SELFTEST = false, bool QJLS = false>
 int launch_tc(const QtJob& j0, const QtJob& j1, int jobs, int64_t n, cudaStream_t st) {
-  auto kernel = k_quantize_tc<Tin, BITS, NORMC, SELFTEST>;
+  auto kernel = k_quantize_tc<Tin, BITS, NORMC, SELFTEST, QJLS>;
   static thread_local int configured_dev = -1;   // one per kernel
   int dev = 0;
   TQ_CUDA(cudaGetDevice(&dev));
@@ -479,7 +644,14 @@ int launch_tc(const QtJob& j0, const QtJob& j1, int jobs, int64_t n, cudaStream_
 }
 
 template <typename Tin>
-int launch_tc_bits(const QtJob& j0, const QtJob& j1, int jobs, bool normc, int64_t n, cudaStream_t st) {
+int launch_tc_bits(const QtJob& j0, const QtJob& j1, int jobs, bool normc, bool want_qjl, int64_t n, cudaStream_t st) {
+  if (want_qjl) {   // (the residual needs the norm correction whether or not the factor is stored)
+#define TQ_TC(B) \
+  if (j0.f.bits == B) return j0.f.norm_correction ? launch_tc<Tin, B, true, false, true>(j0, j1, 1, n, st) : launch_tc<Tin, B, false, false, true>(j0, j1, 1, n, st);
+    TQ_TC(2) TQ_TC(3)
+#undef TQ_TC
+    return TQ_ERR_UNSUPPORTED;
+  }
 #define TQ_TC(B) \
   if (j0.f.bits == B) return normc ? launch_tc<Tin, B, true>(j0, j1, jobs, n, st) : launch_tc<Tin, B, false>(j0, j1, jobs, n, st);
   TQ_TC(2) TQ_TC(3) TQ_TC(4)
@@ -492,12 +664,12 @@ int launch_tc_bits(const QtJob& j0, const QtJob& j1, int jobs, bool normc, int64
 // One tensor, or two of the same shape and format (x1 != nullptr), whose requests the warp-level kernel serves: false where that
 // kernel is to take them.
 bool tq_quantize_tc_try(const TqFast& f0, const void* x0, const TqQuantDst& d0, const TqFast* f1, const void* x1, const TqQuantDst* d1,
-                        int32_t dtype, int64_t ld, int64_t n, bool normc, cudaStream_t st, int* rc) {
+                        int32_t dtype, int64_t ld, int64_t n, bool normc, bool want_qjl, cudaStream_t st, int* rc) {
   if (dtype != TQ_F16 && dtype != TQ_BF16) return false;
-  if (n < qt_min_vectors(x1 != nullptr)) return false;
+  if (n < qt_min_vectors(x1 != nullptr, want_qjl) || (want_qjl && f0.bits == 4)) return false;
   // a thread stores its vector's indices up to 16 bytes at a time
   auto aligned = [](const TqQuantDst& d) {
-    return tq_aligned(d.idx, 16) && d.page_stride % 16 == 0 && d.head_stride % 16 == 0;
+    return tq_aligned(d.idx, 16) && tq_aligned(d.qjl, 16) && d.page_stride % 16 == 0 && d.head_stride % 16 == 0;
   };
   if (!tq_aligned(x0, 16) || !aligned(d0) || (x1 && (!tq_aligned(x1, 16) || !aligned(*d1)))) return false;
   QtJob j0, j1;
@@ -510,8 +682,8 @@ bool tq_quantize_tc_try(const TqFast& f0, const void* x0, const TqQuantDst& d0, 
     j1 = j0;
   }
   const int jobs = x1 ? 2 : 1;
-  *rc = dtype == TQ_F16 ? launch_tc_bits<__half>(j0, j1, jobs, normc, n, st)
-                        : launch_tc_bits<__nv_bfloat16>(j0, j1, jobs, normc, n, st);
+  *rc = dtype == TQ_F16 ? launch_tc_bits<__half>(j0, j1, jobs, normc, want_qjl, n, st)
+                        : launch_tc_bits<__nv_bfloat16>(j0, j1, jobs, normc, want_qjl, n, st);
   return true;
 }
 
