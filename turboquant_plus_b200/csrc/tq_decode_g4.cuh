@@ -944,7 +944,9 @@ bool layout_matches(const tq_cache_layout& L) {
 // streams pages (turbo4 / turbo4, 16 sequences of 8,192 tokens, per call of a chain: 62 us with four warps and one copy of the
 // tables, 37 with eight), but they are filled anew by every CTA: a chain of calls with one or two pages per CTA is ahead with
 // four warps (32/8 heads, 32 sequences of 100 tokens 7.5 -> 5.5 us, 16 of 256 6.9 -> 5.6, 8 of 1,024 7.4 -> 7.1; 16 of 1,024,
-// four pages: 9.9 against 11.0), unless many splits leave a long fold to the four (32 splits of a page: 5.8 against 6.1).
+// four pages: 9.9 against 11.0), unless many splits leave a long fold to the four (32 splits of a page: 5.8 against 6.1).  So are
+// single calls of more than one round (turbo4 / turbo4, 32/8 heads, 128 sequences of 100 tokens 27.2 -> 19.5 us, 214 of 147 46.1 -> 33.7,
+// ragged ones up to 147 42.2 -> 27.0; 64/8 heads 51.4 -> 41.7; with four pages, 256 of 512, 75.2 against 77.6).
 // Five to eight heads: four warps rotate and fold two heads each, 0.6 us and, with several splits, 0.8 us and 0.045 us per
 // split of a chained call, against 0.55 us saved per page of a CTA (64/8 heads of turbo3, eight warps / four: one sequence
 // of 4,096 tokens, 32 x 1 pages 6.7 / 9.8 us, of 65,536, 37 x 14, 23.7 / 21.2; 4 of 4,096, 8 x 4, 9.6 / 9.1; 16/2 heads, one
@@ -955,7 +957,7 @@ inline bool four_warps(const AttnParams& P, const SplitPlan& plan) {
     if (P.group > 4) return !wide && 12 * plan.chunk_pages > (plan.num_splits > 1 ? 31 : 13) + plan.num_splits;
     return !wide || (plan.chunk_pages <= 2 && plan.num_splits <= 16);
   }
-  return !wide && (int64_t)plan.num_splits * P.hkv * P.batch > 2 * (int64_t)tq_num_sms();
+  return (!wide || plan.chunk_pages <= 2) && (int64_t)plan.num_splits * P.hkv * P.batch > 2 * (int64_t)tq_num_sms();
 }
 
 }  // namespace
