@@ -304,6 +304,43 @@ __device__ __forceinline__ void fold_splits(const AttnParams& P, float v_alpha, 
     reinterpret_cast<float4*>(qbuf + head * TQ_D)[col4] = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
 }
 
+// Finished rows in V's rotated space (qbuf) -> rotated back, to the output
+template <int NT, int HEADS>
+__device__ __forceinline__ void store_rows(const AttnParams& P, const uint32_t (&vs1)[4], const uint32_t (&vs2)[4], const float* qbuf, size_t row0, int tid) {
+  const int lane = tid & 31, warp = tid >> 5;
+  if (P.v_rot) {  // dense rotation: x = R^T y
+    for (int e = tid; e < P.group * TQ_D; e += NT) {
+      const int head = e >> 7, j = e & 127;
+      float x = 0.f;
+#pragma unroll 8
+      for (int k = 0; k < TQ_D; ++k) x = fmaf(__ldg(P.v_rot + k * TQ_D + j), qbuf[head * TQ_D + k], x);
+      store_out(P.out, P.out_dtype, (row0 + head) * TQ_D + j, x);
+    }
+  } else {
+    for (int head = warp; head < P.group; head += NT / 32) {
+      float x[4];
+      const float4 v = *reinterpret_cast<const float4*>(qbuf + head * TQ_D + 4 * lane);
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+      if (!P.v_ident) warp_wht128(x, vs2, vs1, lane);  // R^T = D1 (H/sqrt d) D2
+      const size_t at = (row0 + head) * TQ_D + 4 * lane;
+      if (P.out_dtype != TQ_F32 && (reinterpret_cast<uintptr_t>(P.out) & 7) == 0) {   // a lane's four 16-bit results at once
+        uint2 u;
+        if (P.out_dtype == TQ_F16) {
+          u = make_uint2(pack_h2(x[0], x[1]), pack_h2(x[2], x[3]));
+        } else {
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]), hi = __floats2bfloat162_rn(x[2], x[3]);
+          u = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        }
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(P.out) + at) = u;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) store_out(P.out, P.out_dtype, at + k, x[k]);
+      }
+      if constexpr (HEADS <= NT / 32) break;
+    }
+  }
+}
+
 // Tail shared by the decode kernels, entered by the whole CTA after its split partial has been written:
 // take a ticket; the last CTA of a (sequence, kv head) folds all splits in a fixed order, un-rotates and stores.
 // One thread publishes the CTA's writes (the block barrier orders the other threads' stores before its
@@ -335,25 +372,7 @@ __device__ __forceinline__ void finish_splits(const AttnParams& P, const uint32_
   else
     for (int w = warp; w < P.group; w += NT / 32) fold_splits<1, V_Q8>(P, v_alpha, qbuf, row0, ns, w);
   group_sync<NT>(bar_id);
-  if (P.v_rot) {  // dense rotation: x = R^T y
-    for (int e = tid; e < P.group * TQ_D; e += NT) {
-      const int head = e >> 7, j = e & 127;
-      float x = 0.f;
-#pragma unroll 8
-      for (int k = 0; k < TQ_D; ++k) x = fmaf(__ldg(P.v_rot + k * TQ_D + j), qbuf[head * TQ_D + k], x);
-      store_out(P.out, P.out_dtype, (row0 + head) * TQ_D + j, x);
-    }
-  } else {
-    for (int head = warp; head < P.group; head += NT / 32) {
-      float x[4];
-      const float4 v = *reinterpret_cast<const float4*>(qbuf + head * TQ_D + 4 * lane);
-      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-      if (!P.v_ident) warp_wht128(x, vs2, vs1, lane);  // R^T = D1 (H/sqrt d) D2
-#pragma unroll
-      for (int k = 0; k < 4; ++k) store_out(P.out, P.out_dtype, (row0 + head) * TQ_D + 4 * lane + k, x[k]);
-      if constexpr (HEADS <= NT / 32) break;
-    }
-  }
+  store_rows<NT, HEADS>(P, vs1, vs2, qbuf, row0, tid);
 }
 __device__ __forceinline__ void load_q4(const void* q, int dtype, size_t i, float (&x)[4]) {
   if (dtype == TQ_F16) {

@@ -893,12 +893,27 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
         for (int k = 0; k < DPT; ++k) a[k] = fmaf(v[k], f, a[k]);
         Lsum = fmaf(sml[(w * NH + head) * 2 + 1], f, Lsum);
       }
-      const size_t slot = (row0 + head) * P.num_splits + split;
+      if (ns == 1) {
+        // The only split: finished here, as the fold of one would (its partial, a ticket and the way back were 2 us of each CTA;
+        // turbo3, 32/8 heads, 128 sequences of 100 tokens 15.4 -> 11.1, one of 128 5.8 -> 3.8)
+        const float inv = 1.0f / (Lsum * (VT::Q8 ? 1.0f : fv.alpha));
 #pragma unroll
-      for (int k = 0; k < DPT; k += 2)
-        *reinterpret_cast<float2*>(P.part_o + slot * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
-      if (dim == 0) *reinterpret_cast<float2*>(P.part_ml + slot * 2) = make_float2(M, Lsum);
+        for (int k = 0; k < DPT; ++k) qbuf[head * TQ_D + dim + k] = a[k] * inv;
+        if (P.lse && dim == 0) P.lse[row0 + head] = (M + log2f(Lsum)) * 0.6931471805599453f;
+      } else {
+        const size_t slot = (row0 + head) * P.num_splits + split;
+#pragma unroll
+        for (int k = 0; k < DPT; k += 2)
+          *reinterpret_cast<float2*>(P.part_o + slot * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
+        if (dim == 0) *reinterpret_cast<float2*>(P.part_ml + slot * 2) = make_float2(M, Lsum);
+      }
     }
+  }
+  if (ns == 1) {
+    if (tid == 0 && s_flags[0]) atomicExch(P.status, 1);
+    group_sync<NT>(bar_id);
+    store_rows<NT, NH>(P, fv.s1, fv.s2, qbuf, row0, tid);
+    return;
   }
   finish_splits<VT::Q8, NT, NH>(P, fv.s1, fv.s2, fv.alpha, qbuf, stage0, s_flags, row0, ns, b, kvh, tid, bar_id);
 }
