@@ -196,6 +196,47 @@ template <int VB, int OFF> __device__ __forceinline__ void load_v_words(uint32_t
   }
 }
 
+// Splits that a cluster holds at most, its barrier, and eight bytes out of the shared memory of its CTA `rank`, at the same place as `addr` here
+constexpr int CLUSTER_MOST = 8;
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float2 lds_remote2(uint32_t addr, int rank) {
+  float2 v;
+  asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %2, %3;\n ld.shared::cluster.v2.f32 {%0,%1}, [a];\n}\n"
+               : "=f"(v.x), "=f"(v.y) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+
+// DPT elements of a head's row out of the `ns` CTAs of the cluster: (maximum, sum) at `ml`, the elements at `row` in each.
+template <int DPT> __device__ __forceinline__ void cluster_fold(uint32_t ml, uint32_t row, int ns, float alpha, float* out, float* lse) {
+  float2 mls[CLUSTER_MOST], part[CLUSTER_MOST][DPT / 2];
+#pragma unroll
+  for (int r = 0; r < CLUSTER_MOST; ++r) mls[r] = r < ns ? lds_remote2(ml, r) : make_float2(-INFINITY, 0.f);
+#pragma unroll
+  for (int r = 0; r < CLUSTER_MOST; ++r)
+#pragma unroll
+    for (int k = 0; k < DPT / 2; ++k) part[r][k] = r < ns ? lds_remote2(row + 8 * k, r) : make_float2(0.f, 0.f);
+  float M = -INFINITY, sum = 0.f, a[DPT];
+#pragma unroll
+  for (int r = 0; r < CLUSTER_MOST; ++r) M = fmaxf(M, mls[r].x);
+#pragma unroll
+  for (int k = 0; k < DPT; ++k) a[k] = 0.f;
+#pragma unroll
+  for (int r = 0; r < CLUSTER_MOST; ++r) {
+    const float f = fast_exp2(mls[r].x - M);
+    sum = fmaf(mls[r].y, f, sum);
+#pragma unroll
+    for (int k = 0; k < DPT / 2; ++k) {
+      a[2 * k] = fmaf(part[r][k].x, f, a[2 * k]);
+      a[2 * k + 1] = fmaf(part[r][k].y, f, a[2 * k + 1]);
+    }
+  }
+  const float inv = 1.0f / (sum * alpha);
+#pragma unroll
+  for (int k = 0; k < DPT; ++k) out[k] = a[k] * inv;
+  if (lse) *lse = (M + log2f(sum)) * 0.6931471805599453f;
+}
+
 // Per-thread state of the page loop: o[set][blk] = head 4 set + t, dims 16 g + 4 blk .. + 3; maxima and sums of heads
 // 2 (t & 1), + 1 (NH 4) or 2 t, + 1 (NH 8).
 template <int NH> struct G4State {
@@ -573,7 +614,9 @@ __device__ __forceinline__ void g4_page(G4State<NH>& S, uint32_t st, const G4Thr
 // and the SM's warps are in a page loop 80 % of the time instead of 67 %.
 // TAIL: the call follows the append of the step's token (TQ_DECODE_OVERLAP_APPEND).  A template parameter, so that the
 // page loop of every other instantiation carries nothing for it.
-template <int KK, int VK, bool SPARSE, bool NODEQ, int NW, bool TAIL, int NH>
+// CL: the splits of a (sequence, KV head) are a cluster.  A template parameter: with the cluster's instructions in it, every other launch
+// of the kernel was 0.1 to 0.4 us longer.
+template <int KK, int VK, bool SPARSE, bool NODEQ, int NW, bool TAIL, int NH, bool CL>
 __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __grid_constant__ AttnParams P, const __grid_constant__ AttnQuant fk,
                                                                       const __grid_constant__ AttnQuant fv) {
   using C = G4<KK, VK, NW, NH>;
@@ -875,14 +918,14 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     // warp order
     constexpr int DPT = NH * TQ_D / NT;     // 2, 4 or 8
     const int head = tid / (TQ_D / DPT), dim = DPT * (tid % (TQ_D / DPT));
+    float a[DPT], M = -INFINITY, Lsum = 0.f;
     if (head < P.group) {
-      float mw[NW], M = -INFINITY;
+      float mw[NW];
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
         mw[w] = sml[(w * NH + head) * 2];
         M = fmaxf(M, mw[w]);
       }
-      float a[DPT], Lsum = 0.f;
 #pragma unroll
       for (int k = 0; k < DPT; ++k) a[k] = 0.f;
 #pragma unroll
@@ -893,41 +936,68 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
         for (int k = 0; k < DPT; ++k) a[k] = fmaf(v[k], f, a[k]);
         Lsum = fmaf(sml[(w * NH + head) * 2 + 1], f, Lsum);
       }
-      if (ns == 1) {
-        // The only split: finished here, as the fold of one would (its partial, a ticket and the way back were 2 us of each CTA;
-        // turbo3, 32/8 heads, 128 sequences of 100 tokens 15.4 -> 11.1, one of 128 5.8 -> 3.8)
+    }
+    if (ns == 1 || CL) {
+      // The only split: finished here, as the fold of one would (its partial, a ticket and the way back were 2 us of each CTA;
+      // turbo3, 32/8 heads, 128 sequences of 100 tokens 15.4 -> 11.1, one of 128 5.8 -> 3.8).  Splits in a cluster: the first CTA takes the others' rows out of
+      // their shared memory.
+      if (tid == 0 && s_flags[0]) atomicExch(P.status, 1);
+      if (CL && ns > 1) {
+        float2* ml = reinterpret_cast<float2*>(stage0);   // (the warps' rows there have been read)
+        group_sync<NT>(bar_id);
+        if (head < P.group) {
+#pragma unroll
+          for (int k = 0; k < DPT; k += 2) *reinterpret_cast<float2*>(qbuf + head * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
+          if (dim == 0) ml[head] = make_float2(M, Lsum);
+        }
+        cluster_arrive();
+        cluster_wait();
+        if (split != 0) {   // this CTA's memory stays until it has been read
+          cluster_arrive();
+          cluster_wait();
+          return;
+        }
+        float* rows = reinterpret_cast<float*>(stage0 + 1024);
+        if (head < P.group)
+          cluster_fold<DPT>(smem_u32(ml + head), smem_u32(qbuf + head * TQ_D + dim), ns, VT::Q8 ? 1.0f : fv.alpha, rows + head * TQ_D + dim,
+                            P.lse && dim == 0 ? P.lse + row0 + head : nullptr);
+        cluster_arrive();
+        group_sync<NT>(bar_id);
+        store_rows<NT, NH>(P, fv.s1, fv.s2, rows, row0, tid);
+        cluster_wait();
+        return;
+      }
+      if (head < P.group) {
         const float inv = 1.0f / (Lsum * (VT::Q8 ? 1.0f : fv.alpha));
 #pragma unroll
         for (int k = 0; k < DPT; ++k) qbuf[head * TQ_D + dim + k] = a[k] * inv;
         if (P.lse && dim == 0) P.lse[row0 + head] = (M + log2f(Lsum)) * 0.6931471805599453f;
-      } else {
-        const size_t slot = (row0 + head) * P.num_splits + split;
-#pragma unroll
-        for (int k = 0; k < DPT; k += 2)
-          *reinterpret_cast<float2*>(P.part_o + slot * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
-        if (dim == 0) *reinterpret_cast<float2*>(P.part_ml + slot * 2) = make_float2(M, Lsum);
       }
+      group_sync<NT>(bar_id);
+      store_rows<NT, NH>(P, fv.s1, fv.s2, qbuf, row0, tid);
+      return;
     }
-  }
-  if (ns == 1) {
-    if (tid == 0 && s_flags[0]) atomicExch(P.status, 1);
-    group_sync<NT>(bar_id);
-    store_rows<NT, NH>(P, fv.s1, fv.s2, qbuf, row0, tid);
-    return;
+    if (head < P.group) {
+      const size_t slot = (row0 + head) * P.num_splits + split;
+#pragma unroll
+      for (int k = 0; k < DPT; k += 2)
+        *reinterpret_cast<float2*>(P.part_o + slot * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
+      if (dim == 0) *reinterpret_cast<float2*>(P.part_ml + slot * 2) = make_float2(M, Lsum);
+    }
   }
   finish_splits<VT::Q8, NT, NH>(P, fv.s1, fv.s2, fv.alpha, qbuf, stage0, s_flags, row0, ns, b, kvh, tid, bar_id);
 }
 
-template <int KK, int VK, bool SPARSE, bool NODEQ, int NW = ATT_WARPS, bool TAIL = false, int NH = 4>
-int launch_attn_g4(const AttnParams& P_in, const SplitPlan& plan, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
-  const AttnParams P = with_splits(P_in, plan, NW == 4);
+template <int KK, int VK, bool SPARSE, bool NODEQ, int NW, bool TAIL, int NH, bool CL>
+int launch_attn_form(const AttnParams& P, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
   using C = G4<KK, VK, NW, NH>;
   static_assert((16 / NW) * (C::SMEM + 1024) <= 228 * 1024, "CTAs of the specialised decode kernel per SM");
+  constexpr auto kernel = k_decode_attn_g4<KK, VK, SPARSE, NODEQ, NW, TAIL, NH, CL>;
   static thread_local int configured_dev = -1;  // per instantiation
   int dev = 0;
   TQ_CUDA(cudaGetDevice(&dev));
   if (configured_dev != dev) {
-    TQ_CUDA(cudaFuncSetAttribute(k_decode_attn_g4<KK, VK, SPARSE, NODEQ, NW, TAIL, NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     configured_dev = dev;
   }
   AttnQuant ak, av;
@@ -936,9 +1006,24 @@ int launch_attn_g4(const AttnParams& P_in, const SplitPlan& plan, const TqFast& 
   memcpy(ak.s1, fk.s1, 16); memcpy(ak.s2, fk.s2, 16); memcpy(ak.j1, fk.j1, 16); memcpy(ak.j2, fk.j2, 16);
   memcpy(ak.cent16, fk.cent16, 32); ak.alpha = fk.lut_alpha;
   memcpy(av.s1, fv.s1, 16); memcpy(av.s2, fv.s2, 16); memcpy(av.cent16, fv.cent16, 32); av.alpha = fv.lut_alpha;
-  TQ_CUDA(tq_launch_early(k_decode_attn_g4<KK, VK, SPARSE, NODEQ, NW, TAIL, NH>, split_grid(P), 32 * NW,
-                          C::SMEM, st, P, ak, av));
+  TQ_CUDA(tq_launch_cluster(kernel, split_grid(P), 32 * NW, C::SMEM, st, CL ? P.num_splits : 1, P, ak, av));
   return tq_launch_check("k_decode_attn_g4");
+}
+
+template <int KK, int VK, bool SPARSE, bool NODEQ, int NW = ATT_WARPS, bool TAIL = false, int NH = 4>
+int launch_attn_g4(const AttnParams& P_in, const SplitPlan& plan, const TqFast& fk, const TqFast& fv, cudaStream_t st) {
+  const AttnParams P = with_splits(P_in, plan, NW == 4);
+  // Splits that are a cluster, in calls of few CTAs that no chain overlaps: the merge's way through memory, a ticket and two fences, made
+  // them 1 us longer (turbo3, 32/8 heads, behind the append of the step's token: one sequence of 517 tokens 9.3 -> 8.2 us, four 10.4 -> 9.3,
+  // eight of 500 10.8 -> 9.6; 16/2 heads, four of 1,000 10.0 -> 9.7).  Clusters of eight do not find their places where CTAs share SMs (four
+  // of 1,000, without appends between: 7.4 -> 8.9), clusters of sixteen not at all (16 of 2,000, 4/1 heads: 7.6 -> 10.8).
+  if constexpr (!SPARSE && !NODEQ && NW == ATT_WARPS) {
+    const int64_t ctas = (int64_t)P.num_splits * P.hkv * P.batch, sms = tq_num_sms();
+    if (P.num_splits > 1 && P.num_splits <= CLUSTER_MOST && !P.chunk_spread && (TAIL || (!P.q_early && !P.chain_head)) &&
+        ctas <= (P.num_splits <= 6 ? 2 * sms : sms))
+      return launch_attn_form<KK, VK, SPARSE, NODEQ, NW, TAIL, NH, true>(P, fk, fv, st);
+  }
+  return launch_attn_form<KK, VK, SPARSE, NODEQ, NW, TAIL, NH, false>(P, fk, fv, st);
 }
 
 template <int KK, int VK>

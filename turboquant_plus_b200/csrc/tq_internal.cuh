@@ -102,20 +102,28 @@ int tq_num_sms();
 // a dependency on this statement keeps them behind it.
 #define TQ_PDL_POINTER(p) asm volatile("" : "+l"(p)::"memory")
 
+// cluster: CTAs of a cluster along x
 template <typename... P, typename... A>
-inline cudaError_t tq_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline cudaError_t tq_launch_cluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t tq_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  return tq_launch_cluster(kernel, grid, block, smem, st, 1, args...);
 }
 
 // ---- device helpers ---------------------------------------------------------------------
