@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   uint8_t* ktile = sm + SP::OFF_KT;
   uint8_t* vtile = sm + SP::OFF_VT;
   uint8_t* stage0 = sm + SP::OFF_ST;
-  if (warp == 0) tmem_alloc_all<CG>(tbase);          // all 512 columns of the SM (one CTA per SM)
+  if (warp == SP::K_AT / 32) tmem_alloc_all<CG>(tbase);   // all 512 columns of the SM (one CTA per SM)
 
   auto issue = [&](int i) {
     const int64_t page = P.block_table[(size_t)b * P.max_pages + page_lo + i];
@@ -510,20 +510,27 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   // bytes apart (one line per lane and instruction); staged, a warp moves whole rows.  16-byte chunk w of row r sits at
   // chunk w ^ (r & 7) of its row, so that the accesses of consecutive rows fall into different banks.
   auto chunk_at = [&](int r, int w, int esz) { return stg + r * (TQ_D * esz) + ((w ^ (r & 7)) << 4); };
-  auto stage_rows = [&]() {
-    const int cpr = TQ_D * q_esz / 16;   // chunks per row
-#pragma unroll 8
-    for (int it = 0; it < cpr / 2; ++it) {
-      const int c = it * 256 + tid, r = c / cpr, w = c - r * cpr;
-      const int grow = rb * PF_ROWS + r;
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (grow < nrows) {
-        const int gq = grow / P.group, gh = grow - gq * P.group;
-        const size_t off = ((((size_t)b * P.tq + gq) * P.hq + (size_t)kvh * P.group + gh) * TQ_D) * q_esz + w * 16;
-        val = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(P.q) + off);
-      }
-      *reinterpret_cast<uint4*>(chunk_at(r, w, q_esz)) = val;
+  // Row threads, between q or out and the staged rows: move(chunk in shared memory, whether the chunk of rows has this row, byte offset in
+  // q or out) for each 16-byte chunk that this thread moves.  A row's number is divided by the group with a shift where that is a power of
+  // two, and the queries come by asynchronous copies: divided out for every chunk and loaded through registers, they took 8,000 clocks of a
+  // CTA's 28,000 beside its pages (8 chunks of 512 tokens against turbo3, 32 / 8 heads: 306 -> 273 us; two of 64 against 4,096: 90 -> 82).
+  const int group_log = (P.group & (P.group - 1)) == 0 ? 31 - __clz(P.group) : -1;
+  auto move_rows = [&](int esz, auto&& move) {
+    const int per_log = esz == 4 ? 5 : 4, w = tid & ((1 << per_log) - 1);
+    const size_t first = (size_t)b * P.tq * P.hq + (size_t)kvh * P.group;
+#pragma unroll 4
+    for (int it = 0; it < (1 << (per_log - 1)); ++it) {
+      const int r = (it * 256 + tid) >> per_log, grow = rb * PF_ROWS + r;
+      const int gq = group_log >= 0 ? grow >> group_log : grow / P.group, gh = grow - gq * P.group;
+      move(chunk_at(r, w, esz), grow < nrows, (first + (size_t)gq * P.hq + gh) * (TQ_D * esz) + w * 16);
     }
+  };
+  auto stage_rows = [&]() {
+    move_rows(q_esz, [&](uint8_t* to, bool there, size_t off) {   // (rows past the chunk come as zeros)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sptr(to)), "l"(reinterpret_cast<const uint8_t*>(P.q) + (there ? off : 0)),
+                   "r"(there ? 16 : 0) : "memory");
+    });
+    asm volatile("cp.async.wait_all;" ::: "memory");
   };
   auto read_row = [&]() {
     if (P.q_dtype == TQ_F32) {
@@ -752,7 +759,6 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     pf_sync_all<CG>();  // every role, of both CTAs, is done with tensor memory and the operand tiles
-    if (warp == 0) tmem_free_all<CG>(tb);
     if (CG == 2 && rb >= P.row_blocks) return;   // the pair's second block of an odd number
     l_run = scales[8 * PF_ROWS + rtid] + scales[9 * PF_ROWS + rtid];
     // A CTA that gave up a wait reports it, writes no partial and merges nothing, but still takes its ticket below:
@@ -833,7 +839,6 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       rows_sync();   // the exchange area of the rotation is read: the staging below is the same memory
       {
         const int esz = P.out_dtype == TQ_F32 ? 4 : 2;
-        const int cpr = TQ_D * esz / 16;
         if (P.out_dtype == TQ_F32) {
 #pragma unroll
           for (int j = 0; j < PF_HALF; j += 4)
@@ -856,17 +861,9 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
           }
         }
         rows_sync();
-#pragma unroll 8
-        for (int it = 0; it < cpr / 2; ++it) {
-          const int c = it * 256 + tid, r = c / cpr, w = c - r * cpr;
-          const int grow = rb * PF_ROWS + r;
-          if (grow < nrows) {
-            const int gq = grow / P.group, gh = grow - gq * P.group;
-            const size_t off = ((((size_t)b * P.tq + gq) * P.hq + (size_t)kvh * P.group + gh) * TQ_D) * esz + w * 16;
-            *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(P.out) + off) =
-                *reinterpret_cast<const uint4*>(chunk_at(r, w, esz));
-          }
-        }
+        move_rows(esz, [&](uint8_t* from, bool there, size_t off) {
+          if (there) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(P.out) + off) = *reinterpret_cast<const uint4*>(from);
+        });
       }
     }
     return;
@@ -1035,7 +1032,8 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  pf_sync_all<CG>();  // matches the row warps' barrier before the tensor memory is released
+  pf_sync_all<CG>();  // matches the row warps' barrier
+  if (warp == SP::K_AT / 32) tmem_free_all<CG>(tb);
 }
 
 }  // namespace
