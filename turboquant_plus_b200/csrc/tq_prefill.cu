@@ -513,7 +513,8 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   // Row threads, between q or out and the staged rows: move(chunk in shared memory, whether the chunk of rows has this row, byte offset in
   // q or out) for each 16-byte chunk that this thread moves.  A row's number is divided by the group with a shift where that is a power of
   // two, and the queries come by asynchronous copies: divided out for every chunk and loaded through registers, they took 8,000 clocks of a
-  // CTA's 28,000 beside its pages (8 chunks of 512 tokens against turbo3, 32 / 8 heads: 306 -> 273 us; two of 64 against 4,096: 90 -> 82).
+  // CTA's 28,000 beside its pages (with the append, 32 / 8 heads: a prompt of 3,999 tokens, turbo4 / turbo3, 306 -> 273 us; the last 128 of
+  // 8,192 positions of two sequences, q8_0 / turbo2, 90 -> 82).
   const int group_log = (P.group & (P.group - 1)) == 0 ? 31 - __clz(P.group) : -1;
   auto move_rows = [&](int esz, auto&& move) {
     const int per_log = esz == 4 ? 5 : 4, w = tid & ((1 << per_log) - 1);
