@@ -43,3 +43,30 @@ def test_prefill_pairs(kf, vf, group, chunk, lens):
             ref = o.attend_gqa(q[b, i][None].astype(np.float64), kh[:, :, :m], vh[:, :, :m], [m])[0]
             errs.append(max_rel(got[i], ref))
     assert max(errs) < TOL, f"{kf}/{vf}: {max(errs)}"
+
+
+@pytest.mark.parametrize("kf,vf", [("turbo3", "turbo3"), ("turbo4", "turbo2"), ("prod3", "turbo3")])
+@pytest.mark.parametrize("hkv,group,chunk,lens", [(8, 2, 128, [128, 1]), (8, 4, 64, [64, 200]), (8, 4, 90, [700, 90])])
+def test_first_page_beside_the_rows(kf, vf, hkv, group, chunk, lens):
+    """Dense rotations, whose rows need more of the memory that the first page's keys are dequantized into meanwhile, rows of both widths,
+    sequences of one page and of several: every query against a decode call of its own."""
+    import torch
+    import turboquant_plus_b200 as tq
+    gen = torch.Generator(device="cuda").manual_seed(chunk)
+    pages = -(-max(lens) // 128)
+    n = len(lens) * pages * 128
+    cache = tq.PagedKVCache(D, hkv, len(lens) * pages, 128, kf, vf, seed=42, rotation="dense")
+    k, v = (torch.randn((n, hkv, D), device="cuda", generator=gen) for _ in range(2))
+    cache.append(k, v, torch.arange(n, device="cuda"))
+    bt = torch.randperm(len(lens) * pages, device="cuda", generator=gen).to(torch.int32).view(len(lens), pages)
+    sl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q = torch.randn((len(lens), chunk, hkv * group, D), device="cuda", generator=gen).half()
+    got = cache.prefill_attend(q, bt, sl)
+    assert cache.kernel_status() == 0 and torch.equal(got, cache.prefill_attend(q.float(), bt, sl).half())
+    for i in range(0, chunk, 7):
+        seen = (sl - chunk + 1 + i).clamp(min=0)
+        live = (seen > 0).cpu()
+        assert not got[:, i][~live].any()
+        if live.any():
+            want = cache.attend(q[:, i].contiguous(), bt, seen)
+            assert max_rel(got[:, i][live].float().cpu().numpy(), want[live].float().cpu().numpy()) < 2e-3

@@ -93,15 +93,20 @@ __device__ __forceinline__ uint32_t pf_lds(uint32_t addr) {
   return v;
 }
 
-// 128-point sign * Walsh-Hadamard of a row, y = post (H/sqrt d) pre x, held by two threads, 64 elements each (thread `half` has elements 64 half ... 64 half + 63):
-// a 64-point transform in registers, then the last butterfly through `xs` ([element][row] floats, 64 KB of shared
-// memory that nothing else uses meanwhile).  Called by all 256 row threads (named barrier 2).
+// 128-point sign * Walsh-Hadamard of a row, y = post (H/sqrt d) pre x, held by two threads, 64 elements each: thread `half` comes with
+// elements 64 half ... 64 half + 63 and leaves with 32 half ... + 31 (x[0..31]) and 64 + 32 half ... + 31 (x[32..63]).  A 64-point transform
+// in registers, then the last butterfly: each thread forms both results of half of the pairs and passes the other's 32 elements through `xs`
+// ([element][row] floats, 32 KB of shared memory that nothing else uses meanwhile).  Called by all 256 row threads (named barrier 2).
 constexpr int PF_HALF = TQ_D / 2;
 __device__ __forceinline__ void rows_sync() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
+// element that x[j] of such a thread is, before (or without) a transform and after it
+template <bool ROTATED> __device__ __forceinline__ int pf_dim(int half, int j) {
+  return ROTATED ? 64 * (j >> 5) + 32 * half + (j & 31) : PF_HALF * half + j;
+}
 __device__ __forceinline__ void row_wht128_pair(float (&x)[PF_HALF], const uint32_t (&pre)[4], const uint32_t (&post)[4],
                                                 int half, float* xs, int r) {
   const uint32_t pre0 = half ? pre[2] : pre[0], pre1 = half ? pre[3] : pre[1];
-  const uint32_t post0 = half ? post[2] : post[0], post1 = half ? post[3] : post[1];
+  const uint32_t post0 = half ? post[1] : post[0], post1 = half ? post[3] : post[2];
 #pragma unroll
   for (int e = 0; e < PF_HALF; ++e) x[e] = (((e < 32 ? pre0 : pre1) >> (e & 31)) & 1u) ? -x[e] : x[e];
 #pragma unroll
@@ -116,13 +121,17 @@ __device__ __forceinline__ void row_wht128_pair(float (&x)[PF_HALF], const uint3
     }
   }
 #pragma unroll
-  for (int e = 0; e < PF_HALF; ++e) xs[(PF_HALF * half + e) * PF_ROWS + r] = x[e];
+  for (int e = 0; e < 32; ++e) {
+    xs[(32 * half + e) * PF_ROWS + r] = half ? x[e] : x[32 + e];
+    x[e] = half ? x[32 + e] : x[e];
+  }
   rows_sync();
 #pragma unroll
-  for (int e = 0; e < PF_HALF; ++e) {
-    const float y = xs[(PF_HALF * (half ^ 1) + e) * PF_ROWS + r];
-    const float z = half ? y - x[e] : x[e] + y;
-    x[e] = ((((e < 32 ? post0 : post1) >> (e & 31)) & 1u) ? -z : z) * TQ_RSQRT_D;
+  for (int e = 0; e < 32; ++e) {
+    const float y = xs[(32 * (half ^ 1) + e) * PF_ROWS + r];   // thread 0 has the pair's first element, thread 1 its second
+    const float s = x[e] + y, d = half ? y - x[e] : x[e] - y;
+    x[e] = (((post0 >> e) & 1u) ? -s : s) * TQ_RSQRT_D;
+    x[32 + e] = (((post1 >> e) & 1u) ? -d : d) * TQ_RSQRT_D;
   }
 }
 
@@ -373,7 +382,7 @@ template <int KK, int VK, int CG> struct PfSmem2 {
   static constexpr int OFF_SC = OFF_BAR + 256;          // float K scales[4 slots][128 tokens], then the row halves'
                                                         // exchange area float[2 buffers][2 halves][128 rows], then
                                                         // their parts of the row sum float[2 halves][128 rows]
-  static constexpr int OFF_KT = OFF_SC + 5120;          // K operand tiles (the first 64 KB from here also stage the rows)
+  static constexpr int OFF_KT = OFF_SC + 5120;          // K operand tiles (the first 64 KB from here also stage the output rows)
   static constexpr int OFF_VT = OFF_KT + KBUF * KT::TILES * TILE;   // V operand tiles, two
   static constexpr int OFF_ST = OFF_VT + 2 * TILE;      // page records in flight: as many as fit, at most four
   static constexpr int LIMIT = 227 * 1024;
@@ -447,8 +456,6 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
     for (int i = 0; i < 4; ++i) q8_big[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  SP::KLut::fill(sm + SP::OFF_K, fk.cent16, tid, SP::THREADS);
-  SP::VLut::fill(sm + SP::OFF_V, fv.cent16, tid, SP::THREADS);
   TQ_PDL_ENTER();   // so far only the parameters have been read
 
   // Row blocks from the last to the first: the later ones of a causal chunk see more pages, and what is left when the SMs
@@ -492,11 +499,6 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   if (tid == SP::COPIER)
     for (int i = 0; i < NST && i < np; ++i) issue(i);
 
-  if constexpr (KT::PROD) {   // both transforms of a row share registers and staging: the first goes to tensor memory first
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  }
   // ---- prologue (row warps): this row's query, rotated by the K rotation (q8_0 keys: as it is), scaled, fp16 hi + lo
   // into tensor memory; PROD keys: its projection by the sketch's transform as well.  Each of the row's two threads holds
   // one half of its elements ----
@@ -504,46 +506,55 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   const uint32_t TQc = 0, TQLc = 64, TPc = 128, TPLc = 192, TOc = 384;
   // score buffer of page i; P overlays its first 64 columns
   auto s_col = [](int bf) { return KT::SBUF == 2 ? 128u + 128u * bf : 256u; };
-  uint8_t* stg = ktile;                                            // the operand tiles are not in use yet
   const int q_esz = P.q_dtype == TQ_F32 ? 4 : 2;
+  // The rows' staging and exchange area ends where the records begin: 64 KB, or 32 in a pair whose 16-bit queries are rotated by
+  // transforms.  So the first page's K tile is another memory, and its producers fill their tables and dequantize it while the rows are
+  // rotated (7,000 clocks); one before and one behind them, the two were another 4,000.  With the append, 32 / 8 heads: a prompt of 3,999
+  // tokens, turbo4 / turbo3, 273 -> 268 us, the last 128 of 8,192 positions of two sequences, q8_0 / turbo2, 82 -> 78; 64 / 8 heads, the
+  // last 128 of 131,072, turbo3, 832 -> 817.  A pair's `wide` rows need that tile too.
+  const bool wide = CG == 2 && !KT::Q8 && (q_esz == 4 || P.k_rot_t != nullptr);
+  uint8_t* const rows_at = sm + SP::OFF_ST - (CG == 2 && !KT::Q8 && !wide ? 32768 : 65536);
   // Rows pass through shared memory: accessed directly, a thread's own half row would put the lanes of a load 256 or 512
   // bytes apart (one line per lane and instruction); staged, a warp moves whole rows.  16-byte chunk w of row r sits at
   // chunk w ^ (r & 7) of its row, so that the accesses of consecutive rows fall into different banks.
-  auto chunk_at = [&](int r, int w, int esz) { return stg + r * (TQ_D * esz) + ((w ^ (r & 7)) << 4); };
+  auto chunk_at = [](uint8_t* area, int r, int w, int esz) { return area + r * (TQ_D * esz) + ((w ^ (r & 7)) << 4); };
   // Row threads, between q or out and the staged rows: move(chunk in shared memory, whether the chunk of rows has this row, byte offset in
   // q or out) for each 16-byte chunk that this thread moves.  A row's number is divided by the group with a shift where that is a power of
   // two, and the queries come by asynchronous copies: divided out for every chunk and loaded through registers, they took 8,000 clocks of a
   // CTA's 28,000 beside its pages (with the append, 32 / 8 heads: a prompt of 3,999 tokens, turbo4 / turbo3, 306 -> 273 us; the last 128 of
   // 8,192 positions of two sequences, q8_0 / turbo2, 90 -> 82).
   const int group_log = (P.group & (P.group - 1)) == 0 ? 31 - __clz(P.group) : -1;
-  auto move_rows = [&](int esz, auto&& move) {
+  auto move_rows = [&](uint8_t* area, int esz, auto&& move) {
     const int per_log = esz == 4 ? 5 : 4, w = tid & ((1 << per_log) - 1);
     const size_t first = (size_t)b * P.tq * P.hq + (size_t)kvh * P.group;
 #pragma unroll 4
     for (int it = 0; it < (1 << (per_log - 1)); ++it) {
       const int r = (it * 256 + tid) >> per_log, grow = rb * PF_ROWS + r;
       const int gq = group_log >= 0 ? grow >> group_log : grow / P.group, gh = grow - gq * P.group;
-      move(chunk_at(r, w, esz), grow < nrows, (first + (size_t)gq * P.hq + gh) * (TQ_D * esz) + w * 16);
+      move(chunk_at(area, r, w, esz), grow < nrows, (first + (size_t)gq * P.hq + gh) * (TQ_D * esz) + w * 16);
     }
   };
   auto stage_rows = [&]() {
-    move_rows(q_esz, [&](uint8_t* to, bool there, size_t off) {   // (rows past the chunk come as zeros)
+    move_rows(rows_at, q_esz, [&](uint8_t* to, bool there, size_t off) {   // (rows past the chunk come as zeros)
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sptr(to)), "l"(reinterpret_cast<const uint8_t*>(P.q) + (there ? off : 0)),
                    "r"(there ? 16 : 0) : "memory");
     });
+  };
+  auto rows_staged = [&]() {
     asm volatile("cp.async.wait_all;" ::: "memory");
+    rows_sync();
   };
   auto read_row = [&]() {
     if (P.q_dtype == TQ_F32) {
 #pragma unroll
       for (int e = 0; e < PF_HALF; e += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(chunk_at(rtid, (PF_HALF * hf + e) / 4, 4));
+        const float4 v = *reinterpret_cast<const float4*>(chunk_at(rows_at, rtid, (PF_HALF * hf + e) / 4, 4));
         o[e] = v.x; o[e + 1] = v.y; o[e + 2] = v.z; o[e + 3] = v.w;
       }
     } else {
 #pragma unroll
       for (int e = 0; e < PF_HALF; e += 8) {
-        const uint4 w4 = *reinterpret_cast<const uint4*>(chunk_at(rtid, (PF_HALF * hf + e) / 8, 2));
+        const uint4 w4 = *reinterpret_cast<const uint4*>(chunk_at(rows_at, rtid, (PF_HALF * hf + e) / 8, 2));
         const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -555,9 +566,9 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
     }
   };
   auto rotate = [&](const float* dense_t, const uint32_t (&pre)[4], const uint32_t (&post)[4]) {
-    float* xs = reinterpret_cast<float*>(ktile);  // [k][row], 64 KB
+    float* xs = reinterpret_cast<float*>(rows_at);
     if (dense_t) {
-      // dense rotation: the rows staged transposed, then this thread's 64 elements of y = R x
+      // dense rotation: the rows staged transposed ([k][row], 64 KB), then this thread's 64 elements of y = R x
 #pragma unroll
       for (int k = 0; k < PF_HALF; ++k) xs[(PF_HALF * hf + k) * PF_ROWS + rtid] = o[k];
       rows_sync();
@@ -565,10 +576,10 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       for (int j = 0; j < PF_HALF; ++j) o[j] = 0.f;
       for (int k = 0; k < TQ_D; ++k) {
         const float xv = xs[k * PF_ROWS + rtid];
-        const float4* rr = reinterpret_cast<const float4*>(dense_t + (size_t)k * TQ_D + PF_HALF * hf);
+        const float4* rr = reinterpret_cast<const float4*>(dense_t + (size_t)k * TQ_D + 32 * hf);
 #pragma unroll
         for (int j = 0; j < PF_HALF; j += 4) {
-          const float4 r4 = __ldg(rr + (j >> 2));
+          const float4 r4 = __ldg(rr + pf_dim<true>(0, j) / 4);
           o[j] = fmaf(r4.x, xv, o[j]); o[j + 1] = fmaf(r4.y, xv, o[j + 1]);
           o[j + 2] = fmaf(r4.z, xv, o[j + 2]); o[j + 3] = fmaf(r4.w, xv, o[j + 3]);
         }
@@ -589,40 +600,43 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
         u[j] = *reinterpret_cast<const uint32_t*>(&h);
         ul[j] = pf_pack(a - hv.x, bq - hv.y);
       }
-      tmem_st16(tmem + hi_col + 32 * hf + 16 * c, u);
-      tmem_st16(tmem + lo_col + 32 * hf + 16 * c, ul);
+      tmem_st16(tmem + hi_col + pf_dim<!KT::Q8>(hf, 32 * c) / 2, u);
+      tmem_st16(tmem + lo_col + pf_dim<!KT::Q8>(hf, 32 * c) / 2, ul);
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   };
-  if (is_row) {
-    stage_rows();
-    rows_sync();
-    read_row();
-    rows_sync();                            // the staged rows are read: the rotation's exchange area is the same memory
-    if constexpr (!KT::Q8) rotate(P.k_rot_t, fk.s1, fk.s2);
-    if constexpr (KT::PROD) {
-      const uint32_t tm0 = *tbase + ((uint32_t)((warp & 3) * 32) << 16);
-      to_tmem(tm0, P.qscale / fk.lut_alpha, TQc, TQLc);
-      rows_sync();                          // the exchange area has been read
-      stage_rows();
-      rows_sync();
-      read_row();
-      rows_sync();
-      rotate(P.k_s_t, fk.j1, fk.j2);
-      to_tmem(tm0, P.qscale, TPc, TPLc);
-    }
-  }
+  if (is_row) stage_rows();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  pf_sync_all<CG>();  // tensor-memory base, tables and barriers visible; the staging area is free again
+  pf_sync_all<CG>();  // tensor-memory base and barriers visible
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tb = *tbase;
+  // rows done with their area (named barriers 3 and 4, at which the V and a pair's K producers wait before they write there)
+  constexpr int FREE_V = 256 + 32 * SP::PW, FREE_K = 256 + 32 * SP::PW;
 
   if (is_row) {
     // =========================== row warps ===========================
     const uint32_t tm = tb + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 lanes
     float* xch = scales + 512;                                     // [buffer][half][row]
-    if constexpr (!KT::PROD) to_tmem(tm, P.qscale / fk.lut_alpha, TQc, TQLc);
+    rows_staged();
+    read_row();
+    if constexpr (!KT::Q8) {
+      rows_sync();                          // the staged rows are read: the rotation's exchange area is the same memory
+      rotate(P.k_rot_t, fk.s1, fk.s2);
+    }
+    if constexpr (KT::PROD) {   // both transforms of a row share registers and staging: the first goes to tensor memory first
+      to_tmem(tm, P.qscale / fk.lut_alpha, TQc, TQLc);
+      rows_sync();                          // the exchange area has been read
+      stage_rows();
+      rows_staged();
+      read_row();
+      rows_sync();
+      rotate(P.k_s_t, fk.j1, fk.j2);
+    }
+    asm volatile("bar.arrive 3, %0;" ::"n"(FREE_V) : "memory");
+    if constexpr (CG == 2) asm volatile("bar.arrive 4, %0;" ::"n"(FREE_K) : "memory");
+    if constexpr (KT::PROD) to_tmem(tm, P.qscale, TPc, TPLc);
+    else to_tmem(tm, P.qscale / fk.lut_alpha, TQc, TQLc);
     pf_arrive_leader<CG>(q_ready, lane);             // the queries are in tensor memory
 
     float m_run = -INFINITY, l_run = 0.f;   // l_run: this half's part of the row sum
@@ -816,7 +830,7 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       const float inv = l_run > 0.f ? 1.0f / (l_run * fv.lut_alpha) : 0.f;
 #pragma unroll
       for (int j = 0; j < PF_HALF; ++j) o[j] *= inv;
-      float* ys = reinterpret_cast<float*>(ktile);  // [k][row]; the operand tiles are idle by now
+      float* ys = reinterpret_cast<float*>(ktile);  // the operand tiles are idle by now
       if (P.v_rot) {
 #pragma unroll
         for (int k = 0; k < PF_HALF; ++k) ys[(PF_HALF * hf + k) * PF_ROWS + rtid] = o[k];
@@ -825,10 +839,10 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
         for (int j = 0; j < PF_HALF; ++j) o[j] = 0.f;
         for (int k = 0; k < TQ_D; ++k) {
           const float yv = ys[k * PF_ROWS + rtid];
-          const float4* rr = reinterpret_cast<const float4*>(P.v_rot + (size_t)k * TQ_D + PF_HALF * hf);
+          const float4* rr = reinterpret_cast<const float4*>(P.v_rot + (size_t)k * TQ_D + 32 * hf);
 #pragma unroll
           for (int j = 0; j < PF_HALF; j += 4) {
-            const float4 r4 = __ldg(rr + (j >> 2));
+            const float4 r4 = __ldg(rr + pf_dim<true>(0, j) / 4);
             o[j] = fmaf(r4.x, yv, o[j]); o[j + 1] = fmaf(r4.y, yv, o[j + 1]);
             o[j + 2] = fmaf(r4.z, yv, o[j + 2]); o[j + 3] = fmaf(r4.w, yv, o[j + 3]);
           }
@@ -843,11 +857,11 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
         if (P.out_dtype == TQ_F32) {
 #pragma unroll
           for (int j = 0; j < PF_HALF; j += 4)
-            *reinterpret_cast<float4*>(chunk_at(rtid, (PF_HALF * hf + j) / 4, 4)) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+            *reinterpret_cast<float4*>(chunk_at(ktile, rtid, pf_dim<!VT::Q8>(hf, j) / 4, 4)) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
         } else if (P.out_dtype == TQ_F16) {
 #pragma unroll
           for (int j = 0; j < PF_HALF; j += 8)
-            *reinterpret_cast<uint4*>(chunk_at(rtid, (PF_HALF * hf + j) / 8, 2)) = make_uint4(pf_pack(o[j], o[j + 1]), pf_pack(o[j + 2], o[j + 3]),
+            *reinterpret_cast<uint4*>(chunk_at(ktile, rtid, pf_dim<!VT::Q8>(hf, j) / 8, 2)) = make_uint4(pf_pack(o[j], o[j + 1]), pf_pack(o[j + 2], o[j + 3]),
                                                                  pf_pack(o[j + 4], o[j + 5]), pf_pack(o[j + 6], o[j + 7]));
         } else {
 #pragma unroll
@@ -858,11 +872,11 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
               const __nv_bfloat162 h = __floats2bfloat162_rn(o[j + 2 * k], o[j + 2 * k + 1]);
               w[k] = *reinterpret_cast<const uint32_t*>(&h);
             }
-            *reinterpret_cast<uint4*>(chunk_at(rtid, (PF_HALF * hf + j) / 8, 2)) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4*>(chunk_at(ktile, rtid, pf_dim<!VT::Q8>(hf, j) / 8, 2)) = make_uint4(w[0], w[1], w[2], w[3]);
           }
         }
         rows_sync();
-        move_rows(esz, [&](uint8_t* from, bool there, size_t off) {
+        move_rows(ktile, esz, [&](uint8_t* from, bool there, size_t off) {
           if (there) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(P.out) + off) = *reinterpret_cast<const uint4*>(from);
         });
       }
@@ -885,8 +899,20 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
       const int tl = tid - SP::K_AT, tok = 64 * crank + tl;
       uint8_t* drow = ktile + (tl >> 3) * 2048 + (tl & 7) * 16;
       uint32_t marked = 0;   // q8_0: slots whose q8_big byte of this warp is set
+      bool waited = CG == 1;   // for the rows
+      if constexpr (KB > 0) {
+        SP::KLut::fill(sm + SP::OFF_K, fk.cent16, tl, 32 * SP::PW);
+        asm volatile("bar.sync 5, %0;" ::"n"(32 * SP::PW) : "memory");
+      }
       for (int i = 0; i < np; ++i) {
         const int bf = i & 1, st_i = i % NST;
+        if constexpr (CG == 2) {
+          if (i == (wide ? 0 : 1)) {
+            __syncwarp();
+            asm volatile("bar.sync 4, %0;" ::"n"(FREE_K) : "memory");
+            waited = true;
+          }
+        }
         bool ok = !*fail;
         if constexpr (SP::KBUF == 2) {
           if (ok && i >= 2) ok = tc_wait(&s_full[bf], (uint32_t)(((i - 2) >> 1) & 1));
@@ -929,9 +955,13 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
         pf_arrive_leader<CG>(&k_ready[bf], lane);
         pf_arrive_warp(&rec_free[st_i], lane);
       }
+      __syncwarp();
+      if (!waited) asm volatile("bar.arrive 4, %0;" ::"n"(FREE_K) : "memory");
     } else {
       // V producers
       constexpr int DIMS = TQ_D / CG;
+      if constexpr (VB > 0) SP::VLut::fill(sm + SP::OFF_V, fv.cent16, tid - SP::V_AT, 32 * SP::PW);
+      asm volatile("bar.sync 3, %0;" ::"n"(FREE_V) : "memory");
       for (int i = 0; i < np; ++i) {
         const int bf = i & 1, st_i = i % NST;
         bool ok = !*fail;
@@ -1119,7 +1149,9 @@ static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_page
 // an odd last row block occupies a whole pair, and the plan rounds on 74 places instead of 148: three row blocks x 8 KV heads
 // x 256 pages of turbo3 are 144 CTAs of 43 pages alone and 64 of 64 as pairs, 99 us against 113; nine x 16 x 32 one wave alone
 // and three as pairs, 71 against 113; at 2, 5, 7 and 11 row blocks pairs are ahead (5 x 8 x 1,024: 495 against 540).  Page
-// times are what long chunks measure; a CTA costs 18 us beside its pages, a split its partial and its part of the merge.  PROD keys have no pairs: their
+// times are what long chunks measure; a CTA is taken to cost 18 us beside its pages (it was 15 and is 10 now; counted as 11, and as 8 pages
+// instead of 12 in the plan, none of 34 shapes of 16 to 4,096 queries over up to 65,000 positions took another time), a split its partial
+// and its part of the merge.  PROD keys have no pairs: their
 // one score buffer puts scores, softmax and product of a page one after the other, 4 us a page in either form.
 static long pf_time_ns(const PfPlan& p, int k_format, int v_format, int cg) {
   const int wide = (k_format == TQ_FMT_TURBO4) + (v_format == TQ_FMT_TURBO4);   // tables of 256 pairs
