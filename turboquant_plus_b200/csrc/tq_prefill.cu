@@ -1122,13 +1122,16 @@ static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_page
   p.row_blocks = (chunk_tokens * (hq / hkv) + PF_ROWS - 1) / PF_ROWS;
   const long base = (long)((p.row_blocks + cg - 1) / cg) * hkv * batch;
   const int slots = tq_num_sms() / cg;  // one CTA per SM
-  const int cap = max_pages / 8 > 1 ? max_pages / 8 : 1;  // at least eight pages per split
-  // splits per row block: the count that minimises (waves of CTAs) x (pages per split + fixed cost of a CTA)
+  // Splits per row block: the count that minimises (waves of CTAs) x (pages per split + fixed cost of a CTA) + the CTA's work that merges
+  // them, 0.8 of a page each (without that, and down to three pages a split, 22 queries over 16,000 tokens of one KV head went from 55 to
+  // 69 us).  At least three pages per split: where eight were the least, 26 queries over 2,300 tokens of turbo3, 32 / 8 heads, took 37 us
+  // and take 31; 32 over 1,500 of turbo4 43 and 29; 128 over 4,000 of prod3 / turbo3, 16 / 4 heads, 74 and 63.
+  const int cap = max_pages / 3 > 1 ? max_pages / 3 : 1;
   int s = 1;
   long best = -1;
   for (int c = 1; c <= cap && c <= 64; ++c) {
     const long waves = (base * c + slots - 1) / slots;
-    const long cost = waves * ((max_pages + c - 1) / c + PF_CTA_COST_PAGES);
+    const long cost = 10 * waves * ((max_pages + c - 1) / c + PF_CTA_COST_PAGES) + (c > 1 ? 8 * c : 0);
     if (best < 0 || cost < best) {
       best = cost;
       s = c;
@@ -1164,7 +1167,7 @@ static long pf_time_ns(const PfPlan& p, int k_format, int v_format, int cg) {
 
 // A short chunk over q8_0 or PROD tensors: every query as a row of the decode kernel, which reads a page per row and KV head
 // where the kernel here multiplies 128 rows whatever the chunk has, converts every key to two or three operand tiles, and
-// splits no finer than eight pages.  Rows x KV heads x pages, and 12 ns a row and KV head, bound the one; pages of a wave, the
+// splits no finer than three pages.  Rows x KV heads x pages, and 12 ns a row and KV head, bound the one; pages of a wave, the
 // splits' merge and a start the other (q8_0 / turbo2, 32/8 heads, rows | tiles: 1 query over 256 pages 17 | 77 us, 4 47 | 78,
 // 8 over 32 pages 18 | 35, over 256 some 90 | 78; 48 over 2 pages 12 | 16; prod3 / turbo3, 4 over 256 53 | 109).  (turbo2/3/4
 // K and V always take the kernel here.)
