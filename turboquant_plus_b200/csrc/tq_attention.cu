@@ -432,7 +432,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) k_decode_attn(const AttnParams
       P.part_ml[slot * 2 + 1] = Lsum;
     }
   }
-  finish_splits<VT::Q8>(P, fv.s1, fv.s2, fv.lut_alpha, qbuf, stage0, s_flags, row0, ns, b, kvh);
+  if (merge_splits<VT::Q8>(P, fv.lut_alpha, qbuf, s_flags, row0, ns, b, kvh))
+    store_rows<ATT_THREADS, MAX_G>(P, fv.s1, fv.s2, qbuf, row0, threadIdx.x);
 }
 
 // ------------------------------------------------------------------------------------------

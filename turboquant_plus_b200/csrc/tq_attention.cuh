@@ -234,7 +234,7 @@ __device__ __forceinline__ void warp_wht128(float (&x)[4], const uint32_t (&pre)
   for (int k = 0; k < 4; ++k) x[k] = (((qb >> k) & 1u) ? -x[k] : x[k]) * TQ_RSQRT_D;
 }
 
-// Fold of the split partials of one head by one warp (see finish_splits).  A round covers 64 splits: lane j
+// Fold of the split partials of one head by one warp (see merge_splits).  A round covers 64 splits: lane j
 // fetches (max, sum) of splits s0 + j and s0 + 32 + j, twenty 16-byte loads per lane go out before anything
 // waits, the warp agrees on the maximum, then the rows are accumulated in split order.
 template <int HALVES, bool V_Q8>
@@ -341,16 +341,15 @@ __device__ __forceinline__ void store_rows(const AttnParams& P, const uint32_t (
   }
 }
 
-// Tail shared by the decode kernels, entered by the whole CTA after its split partial has been written:
-// take a ticket; the last CTA of a (sequence, kv head) folds all splits in a fixed order, un-rotates and stores.
+// Merge shared by the decode kernels, entered by the whole CTA after its split partial has been written:
+// take a ticket; the last CTA of a (sequence, kv head) folds all splits in a fixed order, and has rows to store (true).
 // One thread publishes the CTA's writes (the block barrier orders the other threads' stores before its
 // release), so the rest of the CTA does not execute a device-wide fence.
 // HEADS: most query heads per KV head of the kernel.
 template <bool V_Q8, int NT = ATT_THREADS, int HEADS = MAX_G>
-__device__ __forceinline__ void finish_splits(const AttnParams& P, const uint32_t (&vs1)[4], const uint32_t (&vs2)[4],
-                                              float v_alpha, float* qbuf, uint8_t* stage0, volatile int* s_flags,
-                                              size_t row0, int ns, int b, int kvh, int tid = threadIdx.x, int bar_id = 0) {
-  const int lane = tid & 31, warp = tid >> 5;
+__device__ __forceinline__ bool merge_splits(const AttnParams& P, float v_alpha, float* qbuf, volatile int* s_flags, size_t row0,
+                                              int ns, int b, int kvh, int tid = threadIdx.x, int bar_id = 0) {
+  const int warp = tid >> 5;
   group_sync<NT>(bar_id);
   if (tid == 0) {
     if (s_flags[0]) atomicExch(P.status, 1);
@@ -363,7 +362,7 @@ __device__ __forceinline__ void finish_splits(const AttnParams& P, const uint32_
     }
   }
   group_sync<NT>(bar_id);
-  if (!s_flags[1]) return;
+  if (!s_flags[1]) return false;
   // Warp (half, head) folds the splits of one head.  With at most four heads there are two warps per head and each
   // takes 64 of the 128 dims: lanes 0..15 then read even splits, lanes 16..31 odd ones (16 bytes each), and one
   // lane exchange joins the two at the end; with more heads a warp takes the whole row and every split.
@@ -372,7 +371,7 @@ __device__ __forceinline__ void finish_splits(const AttnParams& P, const uint32_
   else
     for (int w = warp; w < P.group; w += NT / 32) fold_splits<1, V_Q8>(P, v_alpha, qbuf, row0, ns, w);
   group_sync<NT>(bar_id);
-  store_rows<NT, HEADS>(P, vs1, vs2, qbuf, row0, tid);
+  return true;
 }
 __device__ __forceinline__ void load_q4(const void* q, int dtype, size_t i, float (&x)[4]) {
   if (dtype == TQ_F16) {

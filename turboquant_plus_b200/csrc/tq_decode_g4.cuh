@@ -913,6 +913,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     *reinterpret_cast<float4*>(sml + (warp * NH + 2 * t) * 2) = make_float4(S.m0, S.l0, S.m1, S.l1);
   }
   group_sync<NT>(bar_id);
+  float* rows = qbuf;   // of the finished output, in V's rotated space
   {
     // thread (head, DPT consecutive dims): NH heads x 128 dims over the CTA's threads; the warps' rows are added in
     // warp order
@@ -937,10 +938,11 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
         Lsum = fmaf(sml[(w * NH + head) * 2 + 1], f, Lsum);
       }
     }
+    // The only split is finished here, as the fold of one would (its partial, a ticket and the way back were 2 us of each CTA; turbo3,
+    // 32/8 heads, 128 sequences of 100 tokens 15.4 -> 11.1 us, one of 128 5.8 -> 3.8).  Splits in a cluster: the first CTA takes the
+    // others' rows out of their shared memory.  One copy of the code that stores rows: with one per way here, long contexts took 0.06 us
+    // a call longer.
     if (ns == 1 || CL) {
-      // The only split: finished here, as the fold of one would (its partial, a ticket and the way back were 2 us of each CTA;
-      // turbo3, 32/8 heads, 128 sequences of 100 tokens 15.4 -> 11.1, one of 128 5.8 -> 3.8).  Splits in a cluster: the first CTA takes the others' rows out of
-      // their shared memory.
       if (tid == 0 && s_flags[0]) atomicExch(P.status, 1);
       if (CL && ns > 1) {
         float2* ml = reinterpret_cast<float2*>(stage0);   // (the warps' rows there have been read)
@@ -957,35 +959,31 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
           cluster_wait();
           return;
         }
-        float* rows = reinterpret_cast<float*>(stage0 + 1024);
+        rows = reinterpret_cast<float*>(stage0 + 1024);
         if (head < P.group)
           cluster_fold<DPT>(smem_u32(ml + head), smem_u32(qbuf + head * TQ_D + dim), ns, VT::Q8 ? 1.0f : fv.alpha, rows + head * TQ_D + dim,
                             P.lse && dim == 0 ? P.lse + row0 + head : nullptr);
         cluster_arrive();
-        group_sync<NT>(bar_id);
-        store_rows<NT, NH>(P, fv.s1, fv.s2, rows, row0, tid);
-        cluster_wait();
-        return;
-      }
-      if (head < P.group) {
+      } else if (head < P.group) {
         const float inv = 1.0f / (Lsum * (VT::Q8 ? 1.0f : fv.alpha));
 #pragma unroll
         for (int k = 0; k < DPT; ++k) qbuf[head * TQ_D + dim + k] = a[k] * inv;
         if (P.lse && dim == 0) P.lse[row0 + head] = (M + log2f(Lsum)) * 0.6931471805599453f;
       }
       group_sync<NT>(bar_id);
-      store_rows<NT, NH>(P, fv.s1, fv.s2, qbuf, row0, tid);
-      return;
-    }
-    if (head < P.group) {
-      const size_t slot = (row0 + head) * P.num_splits + split;
+    } else {
+      if (head < P.group) {
+        const size_t slot = (row0 + head) * P.num_splits + split;
 #pragma unroll
-      for (int k = 0; k < DPT; k += 2)
-        *reinterpret_cast<float2*>(P.part_o + slot * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
-      if (dim == 0) *reinterpret_cast<float2*>(P.part_ml + slot * 2) = make_float2(M, Lsum);
+        for (int k = 0; k < DPT; k += 2)
+          *reinterpret_cast<float2*>(P.part_o + slot * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
+        if (dim == 0) *reinterpret_cast<float2*>(P.part_ml + slot * 2) = make_float2(M, Lsum);
+      }
+      if (!merge_splits<VT::Q8, NT, NH>(P, fv.alpha, qbuf, s_flags, row0, ns, b, kvh, tid, bar_id)) return;
     }
   }
-  finish_splits<VT::Q8, NT, NH>(P, fv.s1, fv.s2, fv.alpha, qbuf, stage0, s_flags, row0, ns, b, kvh, tid, bar_id);
+  store_rows<NT, NH>(P, fv.s1, fv.s2, rows, row0, tid);
+  if (CL && ns > 1) cluster_wait();
 }
 
 template <int KK, int VK, bool SPARSE, bool NODEQ, int NW, bool TAIL, int NH, bool CL>
