@@ -501,7 +501,7 @@ def run_ours(args):
             "decode_loop_us_per_layer": {"stream_order": loop.get("stream_order"), "overlap_append": loop.get("overlap_append"),
                                          "note": "per layer: quantize-on-append of one token, then decode attention over "
                                                  "ctx + 1 tokens; 40 layers, one graph, no host copies"},
-            "roofline_quantize_prod": {"bound": "hbm", "kernel": "k_quantize_mma<half,2,QJL stage> for the K rows + k_quantize_tc<half,3> for the V rows, 2^21 vectors each",
+            "roofline_quantize_prod": {"bound": "hbm", "kernel": "k_quantize_tc<half,2,QJL stage> for the K rows + k_quantize_tc<half,3> for the V rows, 2^21 vectors each",
                                        "vectors_per_s": 2 * nq32 / (appendp_ms * 1e-3),
                                        "achieved": appendp_bytes / (appendp_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                                        "frac": appendp_bytes / (appendp_ms * 1e-3) / 1e9 / peak,
