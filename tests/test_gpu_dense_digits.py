@@ -218,7 +218,7 @@ def _next_to_boundaries(quantizer, n, seed):
 @pytest.mark.parametrize("bits", [1, 2, 3, 4])
 @pytest.mark.parametrize("n", [4737, 9601, 40000])
 def test_outputs_next_to_boundaries(n, bits):
-    """What the leading products cannot decide: by the checker, by whole rows once its list is full, and with the sketch."""
+    """What the leading products cannot decide: by the deciding warp, by whole rows once its list is full, and with the sketch."""
     import torch
     import turboquant_plus_b200 as tq
     m, q = tq.TurboQuantMSE(D, bits, seed=6), tq.TurboQuant(D, bits + 1, seed=6)

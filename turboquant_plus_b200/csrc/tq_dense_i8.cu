@@ -9,7 +9,7 @@
 // with outlier channels), fp64 sums of 128 terms by 4.9e-16.
 //
 // What only decides something -- an index, a sign of the sketch -- needs fewer: the leading ten (indices) to 21 products (the sketch) leave a known
-// bound out, and what lies within it of a boundary is decided in fp64 (di_index, di_checker, di_rows_plain).  A residual is taken from 21
+// bound out, and what lies within it of a boundary is decided in fp64 (di_index, di_decider, di_rows_plain).  A residual is taken from 21
 // products.  Reconstructions are results themselves and take all 34.
 //
 // One persistent CTA per SM, 128 vectors a tile:
@@ -561,7 +561,7 @@ __device__ __forceinline__ int di_check8(const TqDenseQuant& a, const DiCodes& c
   return di_search(c, a.bits, y);
 }
 template <typename Tin>
-__device__ __forceinline__ void di_checker(DiList& list, const TqDenseQuant& a, const DiCodes& c, const Tin* x, int64_t ld, int lane) {
+__device__ __forceinline__ void di_decider(DiList& list, const TqDenseQuant& a, const DiCodes& c, const Tin* x, int64_t ld, int lane) {
   int done = 0;
   long long since = clock64();
 #pragma unroll 1
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
     }
     if constexpr (!PROD) {
       __syncwarp();
-      di_checker<Tin>(s_list, a, s_codes, x, ld, lane);
+      di_decider<Tin>(s_list, a, s_codes, x, ld, lane);
     }
   } else if (warp == DI_MMA) {
     int item = 0, operands = 0;
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       uint8_t* s_plain = s_plains[t & 1];
       // ---- y = R w: indices, ||c[idx]||^2, the centroids as the next operand.  Without the sketch of the 34 products of all digits ten,
       // which leave less than 2^-21 of r_scale out: one output in 90,000 of a rotation's with eight centroids is too close to a boundary
-      // and is left to the checker.  With the sketch, where other outputs hang on it, 14 products: one in six million; its row is for
+      // and is left to the decider.  With the sketch, where other outputs hang on it, 14 products: one in six million; its row is for
       // di_rows_plain.  Rows of zeros are on no boundary.
       uint32_t packed[DI_COLS / 4];
       uint32_t unsure = 0;   // groups of eight columns
