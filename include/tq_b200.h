@@ -111,7 +111,8 @@ int tq_quantize_status_sync(int32_t* status_out);
 /* Self-tests of that: a quantize or dequantize call whose kernel never reports one product of its first CTA's second tile as
  * done, with waits of 2^20 SM clocks (half a millisecond) instead of 2^30.  The kernels end normally, the context stays
  * usable.  Quantize: fp16 rows of a 3-bit WHT-mode quantizer with norm correction, or fp32 rows of a dense-mode
- * one of d = 128, 2 bits and a sketch; outputs as tq_quantize's (codes packed, or one a byte).  Dequantize: the latter's. */
+ * one of d = 128 and 2 bits, with a sketch or without (then a product of the third tile); outputs as tq_quantize's (codes packed,
+ * or one a byte).  Dequantize: with a sketch. */
 int tq_selftest_quantize_gives_up(const tq_quantizer* q, const void* x_dev, int64_t ld, int64_t n, uint8_t* out_codes_dev,
                                   float* out_norm_dev, float* out_scale_dev, uint8_t* out_qjl_dev, float* out_rnorm_dev, void* stream);
 int tq_selftest_dequantize_gives_up(const tq_quantizer* q, const uint8_t* idx_dev, const float* norm_dev, const uint8_t* qjl_dev,

@@ -1,5 +1,5 @@
 """Bounded waits of the tensor-core quantize and dequantize kernels that run out: a call whose first CTA never reports one product of
-its second tile as done.  What it did compute is right, the rest is marked as not a number, the status word says so once, and
+its second tile, or third, as done.  What it did compute is right, the rest is marked as not a number, the status word says so once, and
 the same calls then run as before."""
 import ctypes
 
@@ -24,11 +24,13 @@ def _first_cta(n, sms):
     return torch.where(tile % sms == 0, tile // sms, -1)
 
 
-def _check(seen, right, at):
-    """Rows of the outputs in `seen`, the first of which marks what was given up: tile 0 and other CTAs are right, tile 1 is not there."""
+def _check(seen, right, at, tile=1):
+    """Rows of the outputs in `seen`, the first of which marks what was given up: other CTAs and tiles before `tile` are right, `tile`
+    is not there."""
     import torch
     lost = seen[0].reshape(len(at), -1).isnan().any(1)
-    assert bool(lost[at == 1].all()) and not bool(lost[at <= 0].any())
+    assert bool(lost[at == tile].all()) and not bool(lost[at < tile - 1].any())
+    assert tile > 1 or not bool(lost[at < tile].any())
     for a, b in zip(seen, right):
         a, b = a.reshape(len(at), -1), b.reshape(len(at), -1)
         assert torch.equal(a[~lost], b[~lost])
@@ -88,3 +90,27 @@ def test_dense_calls_give_up():
     assert bool(lost[at >= 1].isnan().all())
     again = q.quantize_device(x)
     assert torch.equal(again["idx"], right[2]) and torch.equal(again["qjl"], right[3]) and torch.equal(back(), y) and _status(nv) == 0
+
+
+@pytest.mark.parametrize("tiles", [3, 4, 5])
+def test_dense_call_without_a_sketch_gives_up(tiles):
+    """In the last tile of a CTA, in the last but one and earlier: the rows look at a tile's sums a tile later."""
+    import torch
+    import turboquant_plus_b200 as tq
+    from turboquant_plus_b200 import _native as nv
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = TILE * (tiles - 1) * sms + 37
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, D, device="cuda", generator=gen)
+    q = tq.TurboQuantMSE(D, 2, seed=1).polar_quant
+    out = q.quantize_device(x)
+    right = out["norm"], out["idx"]
+    seen = tuple(torch.zeros_like(t) for t in right)
+    nv.call("tq_selftest_quantize_gives_up", q._native(x.device).handle, nv.ptr(x), D, n, nv.ptr(seen[1]), nv.ptr(seen[0]), None, None,
+            None, nv.stream_ptr())
+    assert _status(nv) == 1 and _status(nv) == 0
+    at = _first_cta(n, sms)
+    _check(seen, right, at, 2)
+    assert bool(seen[0][at >= 2].isnan().all())
+    again = q.quantize_device(x)
+    assert torch.equal(again["idx"], right[1]) and _status(nv) == 0

@@ -145,7 +145,7 @@ struct DiShared {
   uint32_t tmem;
   volatile int failed;   // a wait gave up: nobody waits any more
 };
-// SELFTEST: 0, or the product sum of the first CTA that is never reported (di_issue), one of its second tile; waits are short then
+// SELFTEST: 0, or the product sum of the first CTA that is never reported (di_issue); waits are short then
 template <int SELFTEST> __device__ __forceinline__ void di_wait(DiShared& s, uint64_t* bar, uint32_t parity) {
   tc_wait(bar, parity, &s.failed, SELFTEST ? TC_SELFTEST_CYCLES : TC_WAIT_CYCLES);
 }
@@ -749,15 +749,16 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
     int item = 0, t = PROD ? 0 : -1;
     if (mine > 0) load_tile(blockIdx.x);
     for (; t < mine; ++t) {
-      if (const int ahead = PROD ? t : t + 1; ahead < mine) {
-        nrm = next_nrm;
-        plain = next_plain;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (di_rows_any(sh.failed)) break;   // (in a tile before)
+      const int ahead = PROD ? t : t + 1;
+      if (ahead < mine) asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (di_rows_any(sh.failed)) break;   // (in the tile before, in every turn: di_give_up starts there)
+      nrm = next_nrm;
+      plain = next_plain;
+      if (ahead < mine) {
         prepare(ahead);
         if (!PROD && t < 0) continue;
       }
-      if (PROD || t + 1 >= mine) {
+      if constexpr (PROD) {
         nrm = next_nrm;
         plain = next_plain;
       }
@@ -1431,13 +1432,15 @@ bool tq_dense_i8_dequantize_try(const tq_quantizer* q, const TqDenseDequant& a, 
   }
 }
 
-// The self-tests' forms: fp32 rows of 2 bits and a sketch; fp64 results with a sketch
+// The self-tests' forms: fp32 rows of 2 bits, with a sketch (sum 18 is one of a CTA's second tile) or without (sum 10, of its third); fp64
+// results with a sketch
 int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, cudaStream_t st) {
   DiQuant A;
-  TQ_REQUIRE(a.bits == 2 && a.out_qjl && di_quant_args(a, q->dig, x, TQ_F32, ld, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED,
-             "self-test of the dense quantizer: fp32 rows of 128 elements, 2 bits and a sketch");
-  return di_launch<k_dense_quantize_i8<float, 2, true, 18>>(di_quant_smem<float, true>(), n, st, "k_dense_quantize_i8", A,
-                                                              reinterpret_cast<const float*>(x), ld, n);
+  TQ_REQUIRE(a.bits == 2 && !a.out_qjl == !a.out_rnorm && di_quant_args(a, q->dig, x, TQ_F32, ld, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED,
+             "self-test of the dense quantizer: fp32 rows of 128 elements and 2 bits");
+  const float* xt = reinterpret_cast<const float*>(x);
+  if (a.out_qjl) return di_launch<k_dense_quantize_i8<float, 2, true, 18>>(di_quant_smem<float, true>(), n, st, "k_dense_quantize_i8", A, xt, ld, n);
+  return di_launch<k_dense_quantize_i8<float, 2, false, 10>>(di_quant_smem<float, false>(), n, st, "k_dense_quantize_i8", A, xt, ld, n);
 }
 int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st) {
   DiDequant A;
