@@ -1,6 +1,6 @@
 """Bounded waits of the tensor-core quantize and dequantize kernels that run out: a call whose first CTA never reports one product of
 its second tile, or third, as done.  What it did compute is right, the rest is marked as not a number, the status word says so once, and
-the same calls then run as before."""
+the same calls then run as before.  And a call one of whose roles is late, which gives up nothing."""
 import ctypes
 
 import pytest
@@ -114,3 +114,21 @@ def test_dense_call_without_a_sketch_gives_up(tiles):
     assert bool(seen[0][at >= 2].isnan().all())
     again = q.quantize_device(x)
     assert torch.equal(again["idx"], right[1]) and _status(nv) == 0
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 5])
+def test_products_that_come_late(tiles):
+    """The warp that issues the products comes late to every operand, when the rows have already written the next one."""
+    import torch
+    import turboquant_plus_b200 as tq
+    from turboquant_plus_b200 import _native as nv
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = TILE * (tiles - 1) * sms + 37
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, D, device="cuda", generator=gen)
+    q = tq.TurboQuantMSE(D, 2, seed=1).polar_quant
+    right = q.quantize_device(x)
+    idx, norm = torch.zeros_like(right["idx"]), torch.zeros_like(right["norm"])
+    nv.call("tq_selftest_quantize_role", q._native(x.device).handle, nv.ptr(x), D, n, nv.ptr(idx), nv.ptr(norm), 0, nv.stream_ptr())
+    assert _status(nv) == 0
+    assert torch.equal(idx, right["idx"]) and torch.equal(norm, right["norm"])

@@ -90,6 +90,7 @@ SIGNATURES = {
     "tq_selftest_wait_gives_up": (C.c_int, [_P, _I64, _P]),
     "tq_quantize_status_sync": (C.c_int, [C.POINTER(_I32)]),
     "tq_selftest_quantize_gives_up": (C.c_int, [_P, _P, _I64, _I64, _P, _P, _P, _P, _P, _P]),
+    "tq_selftest_quantize_role": (C.c_int, [_P, _P, _I64, _I64, _P, _P, _I32, _P]),
     "tq_selftest_dequantize_gives_up": (C.c_int, [_P, _P, _P, _P, _P, _I64, _P, _P]),
     "tq_decode_attn": (C.c_int, [_P, _P, C.POINTER(CacheLayout), _P, _P, _I32, _P, _P, _I32, _I32, _I32, _F,
                                  _P, _I64, _P, _I32, _P]),

@@ -141,11 +141,13 @@ __device__ __forceinline__ double di_double(uint32_t v) { return __hiloint2doubl
 
 // Barriers and the way of the roles through them; the row warps and the MMA warp count alike.
 struct DiShared {
-  uint64_t b_full[DI_DIGITS], b_free[DI_DIGITS], d_full[2], d_free[2], a_ready, drained;
+  uint64_t b_full[DI_DIGITS], b_free[DI_DIGITS], d_full[2], d_free[2], a_ready[2], drained;
   uint32_t tmem;
   volatile int failed;   // a wait gave up: nobody waits any more
 };
-// SELFTEST: 0, or the product sum of the first CTA that is never reported (di_issue); waits are short then
+// SELFTEST: 0, or the product sum of the first CTA that is never reported (di_issue), or DI_LATE, an MMA warp that comes late to every
+// operand; waits are short then
+constexpr int DI_LATE = -1;
 template <int SELFTEST> __device__ __forceinline__ void di_wait(DiShared& s, uint64_t* bar, uint32_t parity) {
   tc_wait(bar, parity, &s.failed, SELFTEST ? TC_SELFTEST_CYCLES : TC_WAIT_CYCLES);
 }
@@ -154,8 +156,7 @@ __device__ __forceinline__ void di_init(DiShared& s) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sptr(bar)), "r"(count) : "memory");
   };
   for (int i = 0; i < DI_DIGITS; ++i) init(&s.b_full[i], 1), init(&s.b_free[i], 1);
-  for (int i = 0; i < 2; ++i) init(&s.d_full[i], 1), init(&s.d_free[i], DI_ROW_THREADS / 32);
-  init(&s.a_ready, DI_ROW_THREADS / 32);
+  for (int i = 0; i < 2; ++i) init(&s.d_full[i], 1), init(&s.d_free[i], DI_ROW_THREADS / 32), init(&s.a_ready[i], DI_ROW_THREADS / 32);
   init(&s.drained, 1);
   s.failed = 0;
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -643,14 +644,17 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
   } else if (warp == DI_MMA) {
     int item = 0, operands = 0;
     for (int i = 0; i < mine && !__any_sync(0xffffffffu, sh.failed); ++i) {
-      di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
+      if (SELFTEST == DI_LATE)
+        for (const long long t0 = clock64(); clock64() - t0 < 1 << 16;) {}
       if constexpr (!PROD) {
+        di_wait<SELFTEST>(sh, &sh.a_ready[i & 1], (uint32_t)((i >> 1) & 1));
         di_issue<4, 4, 3, SELFTEST>(sh, item, tiles_b, [](int) { return 0; }, [](int) {}, tb + 128 * (i & 1), tb + DI_ACC);
       } else {
+        di_wait<SELFTEST>(sh, &sh.a_ready[0], (uint32_t)(operands++ & 1));
         di_issue<4, 5, 4, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i, q); }, [](int) {}, tb, tb + DI_ACC);
-        di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
+        di_wait<SELFTEST>(sh, &sh.a_ready[0], (uint32_t)(operands++ & 1));
         di_issue<6, 6, 5, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i + 1, q); }, [](int) {}, tb, tb + DI_ACC);
-        di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(operands++ & 1));
+        di_wait<SELFTEST>(sh, &sh.a_ready[0], (uint32_t)(operands++ & 1));
         di_issue<6, 6, 5, SELFTEST>(sh, item, tiles_b, [&](int q) { return di_uses(3 * i + 2, q); }, [](int) {}, tb, tb + DI_ACC);
       }
     }
@@ -659,11 +663,14 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
     const int row = 32 * (warp & 3) + lane, h = warp >> 2;       // this thread's vector, and its columns 32 h .. + 31
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t area = tb + lanes, myacc = tb + DI_ACC + lanes + DI_COLS * h;
-    auto operand_ready = [&]() {
+    // A barrier for each half of the operand: without the sketch the rows are a tile ahead, and on one barrier nothing but their arithmetic's
+    // time kept them from completing the phase behind the one that the MMA warp still waits for.  They come to a half again once they
+    // have taken its sums, which the MMA warp issued behind that wait.
+    auto operand_ready = [&](int half) {
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) di_arrive(&sh.a_ready);
+      if (lane == 0) di_arrive(&sh.a_ready[half]);
     };
     constexpr int CHUNKS = TQ_D * (int)sizeof(Tin) / 16;
     auto load_tile = [&](int64_t tile) {
@@ -740,7 +747,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       // of all ones
       next_plain = next_nrm > 0.f ? !(next_nrm > 0x1p-60f && next_nrm < 0x1p63f && most < DI_LARGEST * 0x1p30f) || (__float_as_uint(next_nrm) & 0x7fffffu) == 0x7fffffu
                                   : next_nrm != 0.f || most != 0.f;
-      operand_ready();
+      operand_ready(PROD ? 0 : t & 1);
       if constexpr (!PROD) {
         di_rows_sync();                                            // (the rows have been read)
         if (t + 1 < mine) load_tile(blockIdx.x + (t + 1) * step);
@@ -836,7 +843,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
             di_store8<6, 1>(area, 8 * h + 2 * c, u);
           }
         }
-        operand_ready();
+        operand_ready(0);
       }
       if constexpr (!PROD) {
         if (unsure && !plain && a.out_idx) {
@@ -893,7 +900,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
           di_store8<6, 0>(area, 8 * h + 2 * c, u);
         }
         plain |= over > 62000u;
-        operand_ready();
+        operand_ready(0);
         di_rows_sync();   // (the sums of the squared centroids have been read, and the rows)
         s_part[h][row] = (rr[0] + rr[1]) + (rr[2] + rr[3]);
         if (t + 1 < mine) load_tile(blockIdx.x + (t + 1) * step);
@@ -996,7 +1003,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
         if (sum == DI_SUMS - 2) di_wait<SELFTEST>(sh, &s_digit[0], (uint32_t)(i & 1));
       }, tb, tb + DI_ACC);
       if constexpr (PROD) {
-        di_wait<SELFTEST>(sh, &sh.a_ready, (uint32_t)(i & 1));
+        di_wait<SELFTEST>(sh, &sh.a_ready[0], (uint32_t)(i & 1));
         di_issue<1, DI_DIGITS, DI_DIGITS - 1, SELFTEST>(sh, item, tiles_b, [&](int) { return 2 * i + 1; }, [](int) {}, tb + DI_SIGNS, tb + DI_ACC);
       }
     }
@@ -1078,7 +1085,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_dequantize_i8(const __g
         const uint32_t z = (signs >> (24 - 8 * k)) & 255u;
         di_st2(area + DI_SIGNS + 8 * h + 2 * k, s_sign[z >> 4], s_sign[z & 15]);
       }
-      ready(&sh.a_ready);
+      ready(&sh.a_ready[0]);
     };
     int item = 0, t = 0;
     if (mine > 0) {
@@ -1441,6 +1448,14 @@ int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, 
   const float* xt = reinterpret_cast<const float*>(x);
   if (a.out_qjl) return di_launch<k_dense_quantize_i8<float, 2, true, 18>>(di_quant_smem<float, true>(), n, st, "k_dense_quantize_i8", A, xt, ld, n);
   return di_launch<k_dense_quantize_i8<float, 2, false, 10>>(di_quant_smem<float, false>(), n, st, "k_dense_quantize_i8", A, xt, ld, n);
+}
+// fp32 rows of 2 bits without a sketch, in a run with a role out of step
+int tq_dense_i8_quantize_role(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, int, cudaStream_t st) {
+  DiQuant A;
+  TQ_REQUIRE(a.bits == 2 && di_quant_args(a, q->dig, x, TQ_F32, ld, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED,
+             "self-test of the dense quantizer: fp32 rows of 128 elements and 2 bits");
+  return di_launch<k_dense_quantize_i8<float, 2, false, DI_LATE>>(di_quant_smem<float, false>(), n, st, "k_dense_quantize_i8", A,
+                                                                  reinterpret_cast<const float*>(x), ld, n);
 }
 int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st) {
   DiDequant A;

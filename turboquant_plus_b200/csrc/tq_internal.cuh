@@ -326,8 +326,9 @@ bool tq_dense_i8_dequantize_try(const tq_quantizer* q, const TqDenseDequant& a, 
 // takes its address as a parameter: a device variable in a kernel's own module costs every launch outside a graph 0.6 to
 // 0.9 us (append of 8,192 tokens of turbo3: 14.1 us, 14.8 with a variable that only a branch not taken writes).
 int32_t* tq_quantize_status_word();
-// Runs in which one wait runs out (tq_selftest_quantize_gives_up)
+// Runs in which one wait runs out, or a role is out of step (tq_selftest_quantize_gives_up, tq_selftest_quantize_role)
 int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, cudaStream_t st);
+int tq_dense_i8_quantize_role(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, int role, cudaStream_t st);
 int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st);
 int tq_quantize_tc_selftest(const TqFast& f, const void* x, const TqQuantDst& d, int64_t ld, int64_t n, cudaStream_t st);
 
