@@ -116,7 +116,8 @@ int tq_quantize_status_sync(int32_t* status_out);
 int tq_selftest_quantize_gives_up(const tq_quantizer* q, const void* x_dev, int64_t ld, int64_t n, uint8_t* out_codes_dev,
                                   float* out_norm_dev, float* out_scale_dev, uint8_t* out_qjl_dev, float* out_rnorm_dev, void* stream);
 /* ... and of one role out of step: the same dense-mode call without a sketch, whose MMA warp (role 0) comes to every operand 2^16 SM
- * clocks after the rows have gone on.  The results are tq_quantize's. */
+ * clocks after the rows have gone on (the results are tq_quantize's), or whose warp that decides outputs close to a boundary (role 1)
+ * has no patience: every CTA gives up. */
 int tq_selftest_quantize_role(const tq_quantizer* q, const void* x_dev, int64_t ld, int64_t n, uint8_t* out_idx_dev, float* out_norm_dev,
                               int32_t role, void* stream);
 int tq_selftest_dequantize_gives_up(const tq_quantizer* q, const uint8_t* idx_dev, const float* norm_dev, const uint8_t* qjl_dev,

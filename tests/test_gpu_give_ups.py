@@ -117,6 +117,25 @@ def test_dense_call_without_a_sketch_gives_up(tiles):
 
 
 @pytest.mark.parametrize("tiles", [1, 2, 5])
+def test_outputs_that_nobody_decides(tiles):
+    """The warp that decides outputs close to a boundary leaves at once: the call says so, and what it marks as computed is right."""
+    import torch
+    import turboquant_plus_b200 as tq
+    from tests.test_gpu_dense_digits import _next_to_boundaries
+    from turboquant_plus_b200 import _native as nv
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = TILE * (tiles - 1) * sms + 37
+    q = tq.TurboQuantMSE(D, 2, seed=1).polar_quant
+    x = _next_to_boundaries(q, n, n)
+    right = q.quantize_device(x)
+    idx, norm = torch.zeros_like(right["idx"]), torch.zeros_like(right["norm"])
+    nv.call("tq_selftest_quantize_role", q._native(x.device).handle, nv.ptr(x), D, n, nv.ptr(idx), nv.ptr(norm), 1, nv.stream_ptr())
+    assert _status(nv) == 1 and _status(nv) == 0
+    lost = norm.isnan()
+    assert bool(lost.any()) and torch.equal(idx[~lost], right["idx"][~lost]) and torch.equal(norm[~lost], right["norm"][~lost])
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 5])
 def test_products_that_come_late(tiles):
     """The warp that issues the products comes late to every operand, when the rows have already written the next one."""
     import torch

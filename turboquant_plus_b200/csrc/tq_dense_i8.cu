@@ -146,8 +146,8 @@ struct DiShared {
   volatile int failed;   // a wait gave up: nobody waits any more
 };
 // SELFTEST: 0, or the product sum of the first CTA that is never reported (di_issue), or DI_LATE, an MMA warp that comes late to every
-// operand; waits are short then
-constexpr int DI_LATE = -1;
+// operand, or DI_HASTY, a decider whose wait runs out at once; waits are short then
+constexpr int DI_LATE = -1, DI_HASTY = -2;
 template <int SELFTEST> __device__ __forceinline__ void di_wait(DiShared& s, uint64_t* bar, uint32_t parity) {
   tc_wait(bar, parity, &s.failed, SELFTEST ? TC_SELFTEST_CYCLES : TC_WAIT_CYCLES);
 }
@@ -561,8 +561,10 @@ __device__ __forceinline__ int di_check8(const TqDenseQuant& a, const DiCodes& c
   y += __shfl_xor_sync(0xffffffffu, y, 2);
   return di_search(c, a.bits, y);
 }
-template <typename Tin>
-__device__ __forceinline__ void di_decider(DiList& list, const TqDenseQuant& a, const DiCodes& c, const Tin* x, int64_t ld, int lane) {
+template <typename Tin, int SELFTEST>
+__device__ __forceinline__ void di_decider(DiShared& s, DiList& list, const TqDenseQuant& a, const DiCodes& c, const Tin* x, int64_t ld, int lane,
+                                           int32_t* status) {
+  constexpr long long LIMIT = SELFTEST == DI_HASTY ? 0 : TC_WAIT_CYCLES;
   int done = 0;
   long long since = clock64();
 #pragma unroll 1
@@ -570,7 +572,14 @@ __device__ __forceinline__ void di_decider(DiList& list, const TqDenseQuant& a, 
     const bool last = list.closed != 0;
     const uint32_t e = list.entry[done];
     if (__any_sync(0xffffffffu, e == DiList::NONE)) {
-      if (__any_sync(0xffffffffu, last || clock64() - since > TC_WAIT_CYCLES)) break;   // (the limit: rows that never come to an end)
+      if (__any_sync(0xffffffffu, last)) break;
+      if (__any_sync(0xffffffffu, clock64() - since > LIMIT)) {   // a wait as any other: what the rows still add is not decided
+        if (lane == 0) {
+          s.failed = 1;
+          if (status) *status = 1;   // (the rows may have agreed on the end already)
+        }
+        break;
+      }
       __nanosleep(100);
       continue;
     }
@@ -639,7 +648,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
     }
     if constexpr (!PROD) {
       __syncwarp();
-      di_decider<Tin>(s_list, a, s_codes, x, ld, lane);
+      di_decider<Tin, SELFTEST>(sh, s_list, a, s_codes, x, ld, lane, A.status);
     }
   } else if (warp == DI_MMA) {
     int item = 0, operands = 0;
@@ -1450,12 +1459,13 @@ int tq_dense_i8_quantize_selftest(const tq_quantizer* q, const TqDenseQuant& a, 
   return di_launch<k_dense_quantize_i8<float, 2, false, 10>>(di_quant_smem<float, false>(), n, st, "k_dense_quantize_i8", A, xt, ld, n);
 }
 // fp32 rows of 2 bits without a sketch, in a run with a role out of step
-int tq_dense_i8_quantize_role(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, int, cudaStream_t st) {
+int tq_dense_i8_quantize_role(const tq_quantizer* q, const TqDenseQuant& a, const void* x, int64_t ld, int64_t n, int role, cudaStream_t st) {
   DiQuant A;
   TQ_REQUIRE(a.bits == 2 && di_quant_args(a, q->dig, x, TQ_F32, ld, A) && di_digits_ready(q, st), TQ_ERR_UNSUPPORTED,
              "self-test of the dense quantizer: fp32 rows of 128 elements and 2 bits");
-  return di_launch<k_dense_quantize_i8<float, 2, false, DI_LATE>>(di_quant_smem<float, false>(), n, st, "k_dense_quantize_i8", A,
-                                                                  reinterpret_cast<const float*>(x), ld, n);
+  const float* xt = reinterpret_cast<const float*>(x);
+  if (role == 0) return di_launch<k_dense_quantize_i8<float, 2, false, DI_LATE>>(di_quant_smem<float, false>(), n, st, "k_dense_quantize_i8", A, xt, ld, n);
+  return di_launch<k_dense_quantize_i8<float, 2, false, DI_HASTY>>(di_quant_smem<float, false>(), n, st, "k_dense_quantize_i8", A, xt, ld, n);
 }
 int tq_dense_i8_dequantize_selftest(const tq_quantizer* q, const TqDenseDequant& a, int64_t n, double* out, cudaStream_t st) {
   DiDequant A;

@@ -638,7 +638,7 @@ extern "C" int tq_selftest_quantize_gives_up(const tq_quantizer* q, const void* 
 
 extern "C" int tq_selftest_quantize_role(const tq_quantizer* q, const void* x_dev, int64_t ld, int64_t n, uint8_t* out_idx_dev,
                                          float* out_norm_dev, int32_t role, void* stream) {
-  TQ_REQUIRE(q && q->rotation != TQ_ROT_WHT && x_dev && out_idx_dev && n > 0 && ld >= q->d && role == 0, TQ_ERR_INVALID, "tq_selftest_quantize_role: bad arguments");
+  TQ_REQUIRE(q && q->rotation != TQ_ROT_WHT && x_dev && out_idx_dev && n > 0 && ld >= q->d && (role == 0 || role == 1), TQ_ERR_INVALID, "tq_selftest_quantize_role: bad arguments");
   TqDenseQuant t = dense_tensor_args(q);
   t.out_idx = out_idx_dev;
   t.out_norm = out_norm_dev;
