@@ -765,16 +765,15 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
     int item = 0, t = PROD ? 0 : -1;
     if (mine > 0) load_tile(blockIdx.x);
     for (; t < mine; ++t) {
-      const int ahead = PROD ? t : t + 1;
-      if (ahead < mine) asm volatile("cp.async.wait_group 0;" ::: "memory");
-      if (di_rows_any(sh.failed)) break;   // (in the tile before, in every turn: di_give_up starts there)
-      nrm = next_nrm;
-      plain = next_plain;
-      if (ahead < mine) {
+      if (const int ahead = PROD ? t : t + 1; ahead < mine) {
+        nrm = next_nrm;
+        plain = next_plain;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (di_rows_any(sh.failed)) break;   // (in a tile before)
         prepare(ahead);
         if (!PROD && t < 0) continue;
       }
-      if constexpr (PROD) {
+      if (PROD || t + 1 >= mine) {
         nrm = next_nrm;
         plain = next_plain;
       }
@@ -946,8 +945,11 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
     const bool failed = di_rows_any(sh.failed);
     if constexpr (!PROD)
       if (tid == 0) s_list.closed = 1;
-    if (failed) {   // the last tile begun and those behind it
-      di_give_up(a, t > 0 ? t - 1 : 0, mine, h == 0 ? row : -1, n, A.status);
+    if (failed) {
+      // The last tile begun and those behind it; without the sketch the one before it as well: the last turn prepares nothing, and does not
+      // look at what the turn before it has seen (a barrier of 0.4 us)
+      constexpr int BACK = PROD ? 1 : 2;
+      di_give_up(a, t > BACK ? t - BACK : 0, mine, h == 0 ? row : -1, n, A.status);
     }
   }
   __syncwarp();
