@@ -218,7 +218,7 @@ def _next_to_boundaries(quantizer, n, seed):
 @pytest.mark.parametrize("bits", [1, 2, 3, 4])
 @pytest.mark.parametrize("n", [4737, 9601, 40000])
 def test_outputs_next_to_boundaries(n, bits):
-    """What the leading products cannot decide: by the deciding warp, by whole rows once its list is full, and with the sketch."""
+    """What the leading products cannot decide: by the deciding warp, by whole rows while its ring is full, and with the sketch."""
     import torch
     import turboquant_plus_b200 as tq
     m, q = tq.TurboQuantMSE(D, bits, seed=6), tq.TurboQuant(D, bits + 1, seed=6)
@@ -237,3 +237,39 @@ def test_outputs_next_to_boundaries(n, bits):
     whole, parts = quantize(x), _pieces(quantize, x)
     assert torch.equal(whole[0], parts[0]) and torch.equal(whole[1], parts[1]) and torch.equal(whole[2], parts[2])
     assert bool(((whole[3] - parts[3]).abs() <= 1.2e-7 * parts[3]).all())
+
+
+def _nearest(quantizer, n, seed):
+    """The random fp32 row of `n` with the output that is nearest to a boundary."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(n, D, device="cuda", generator=gen)
+    bnd = torch.from_numpy((quantizer.centroids[1:] + quantizer.centroids[:-1]) / 2).cuda()
+    y = (x / x.norm(dim=1, keepdim=True)).double() @ torch.from_numpy(quantizer.rotation).cuda().T
+    return x[int((y[:, :, None] - bnd).abs().amin((1, 2)).argmin())]
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+@pytest.mark.parametrize("n,share", [(4737, 1.0), (20011, 1.0), (20011, 0.1), (40000, 0.02)])
+def test_copies_of_a_close_vector(n, share, dtype):
+    """Rows that all ask for fp64: every one of a tile, a part of the sixteen that are computed at a time, and one now and then."""
+    import torch
+    import turboquant_plus_b200 as tq
+    m, q = tq.TurboQuantMSE(D, 3, seed=6), tq.TurboQuant(D, 4, seed=6)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, D, device="cuda", generator=gen)
+    x[torch.rand(n, device="cuda", generator=gen) < share] = _nearest(m.polar_quant, 200000, n)
+    x = x.to(getattr(torch, dtype))
+    if dtype == "float16":                          # (rounded, the row is no longer close; rows out of the norm's range ask for fp64 too)
+        x[torch.rand(n, device="cuda", generator=gen) < share, 77] = float("inf")
+    for of in (m, q):
+        def quantize(v):
+            out = of.quantize_device(v) if of is q else of.polar_quant.quantize_device(v, want_scale=True)
+            return [out[name] for name in sorted(out)]
+        whole, parts = quantize(x), _pieces(quantize, x)
+        for a, b in zip(whole, parts):
+            if a.is_floating_point():
+                assert bool((((a - b).abs() <= 1.2e-7 * b.abs()) | (a == b) | (a.isnan() & b.isnan())).all())
+            else:
+                assert torch.equal(a, b)
+    assert torch.equal(m.quantize(x)[0], torch.cat([m.quantize(x[lo:lo + PIECE])[0] for lo in range(0, n, PIECE)]))

@@ -27,7 +27,9 @@
 // What bounds quantize: its rows' arithmetic, 12,000 clocks a tile without the sketch (norms 1,300, digits 2,100, sums 4,000, indices 2,600, the rest
 // barriers and stores) and 40,000 with it (sums 20,000, of which the MMAs take 13,000; residuals 7,000).  65,536 fp32 vectors, fp64
 // tensor cores / all 34 products each / here: 134 / 78 / 33 us, with the sketch 302 / 163 / 90 (105 where a row on a CTA's way is for
-// di_rows_plain, 14 us; about every second call).
+// di_rows_plain; about every second call).  di_rows_plain takes 9 us for up to sixteen rows of a tile, with the sketch 16: where every row
+// is one for it (copies of a vector with an output that close to a boundary, 65,536 of 3 bits) 83 us with all 34 products / 816 with
+// its rows one after the other / 281 now, with the sketch (reconstructions that are quantized again) 168 / 3,600 / 540.
 // What bounds dequantize: its rows, 20,000 clocks a tile where the MMAs (88 clocks each under the rows' loads of sums) take 12,000: sums 900 clocks
 // each, half of it fp64 additions, the next operand 500 a digit, results 3,700, norms and factors 3,000.  65,536 vectors, fp64 tensor
 // cores / all of it behind the last sum / here: 90 / 62 / 56 us, with the sketch 164 / 93 / 85.
@@ -372,77 +374,116 @@ __device__ __forceinline__ int di_search(const DiCodes& c, int bits, double y) {
   for (int b = 0; b < (1 << bits) - 1; ++b) m += c.bnd[b] < y ? 1 : 0;
   return m;
 }
-// Whole rows in fp64, one after the other, by all row threads: a warp multiplies eight elements of a vector with their rows of a matrix, all
-// loads in flight, and thread j < 128 adds up output j.  (A warp per row waited for one load after the other: 75 us a row.)
+// Whole rows in fp64, sixteen at a time, by all row threads on the fp64 tensor cores: a warp has eight outputs of all sixteen.
 struct DiPlain {
-  double part[DI_ROW_THREADS / 32][TQ_D], v[TQ_D], sum[4];
+  static constexpr int PITCH = TQ_D + 8;   // (a load's rows 64 bytes apart modulo 128: no bank conflicts)
+  double v[16][PITCH], part[DI_ROW_THREADS / 32][16];
+  int row[16];
 };
-__device__ __forceinline__ double di_plain_product(DiPlain& s, const double* __restrict__ m, int tid) {   // of s.v; thread j < 128: output j
-  const int lane = tid & 31, warp = tid >> 5;
-  di_rows_sync();
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  double2 r[8][2];
+// c = rows g (c0, c1) and g + 8 (c2, c3) of s.v times m, rows of which are outputs: 8 warp + 2 t and the next
+__device__ __forceinline__ void di_plain_product(double (&c)[4], const DiPlain& s, const double* __restrict__ m, int tid) {
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const double2* row = reinterpret_cast<const double2*>(m + (size_t)(8 * warp + g) * TQ_D + 2 * t);
+  double2 b[8];   // (eight loads in flight; with sixteen the function's registers cost its callers theirs)
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const double2* at = reinterpret_cast<const double2*>(m + (size_t)(8 * warp + k) * TQ_D + 4 * lane);
-    r[k][0] = __ldg(at);
-    r[k][1] = __ldg(at + 1);
+  for (int k = 0; k < 8; ++k) b[k] = __ldg(row + 4 * k);
+  c[0] = c[1] = c[2] = c[3] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {   // slots t and t + 4 of a step carry elements 8 k + 2 t and the next
+    const double2 lo = *reinterpret_cast<const double2*>(&s.v[g][8 * k + 2 * t]), hi = *reinterpret_cast<const double2*>(&s.v[g + 8][8 * k + 2 * t]);
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3]) : "d"(lo.x), "d"(hi.x), "d"(lo.y), "d"(hi.y), "d"(b[k & 7].x), "d"(b[k & 7].y));
+    if (k < 8) b[k] = __ldg(row + 4 * (k + 8));
   }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const double vk = s.v[8 * warp + k];
-    acc[0] = fma(r[k][0].x, vk, acc[0]);
-    acc[1] = fma(r[k][0].y, vk, acc[1]);
-    acc[2] = fma(r[k][1].x, vk, acc[2]);
-    acc[3] = fma(r[k][1].y, vk, acc[3]);
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) s.part[warp][4 * lane + j] = acc[j];
-  di_rows_sync();
-  double y = 0.0;
-  if (tid < TQ_D)
-#pragma unroll 4
-    for (int w = 0; w < DI_ROW_THREADS / 32; ++w) y += s.part[w][tid];
-  return y;
 }
-__device__ __forceinline__ double di_plain_sum(DiPlain& s, double x, int tid) {   // over the first 128 threads
+// this warp's part of a sum over the outputs of rows g and g + 8, and the sums of all warps behind a barrier
+__device__ __forceinline__ void di_plain_part(DiPlain& s, double lo, double hi, int tid) {
+  const int lane = tid & 31, warp = tid >> 5;
+  lo += __shfl_xor_sync(0xffffffffu, lo, 1);
+  hi += __shfl_xor_sync(0xffffffffu, hi, 1);
+  lo += __shfl_xor_sync(0xffffffffu, lo, 2);
+  hi += __shfl_xor_sync(0xffffffffu, hi, 2);
+  if ((lane & 3) == 0) s.part[warp][lane >> 2] = lo, s.part[warp][8 + (lane >> 2)] = hi;
+}
+__device__ __forceinline__ double di_plain_sum(const DiPlain& s, int r) {
+  double sum = 0.0;
 #pragma unroll
-  for (int h = 16; h > 0; h >>= 1) x += __shfl_xor_sync(0xffffffffu, x, h);
-  if (tid < TQ_D && (tid & 31) == 0) s.sum[tid >> 5] = x;
-  di_rows_sync();
-  return (s.sum[0] + s.sum[1]) + (s.sum[2] + s.sum[3]);
+  for (int w = 0; w < DI_ROW_THREADS / 32; ++w) sum += s.part[w][r];
+  return sum;
 }
 template <typename Tin>
 __device__ __noinline__ void di_rows_plain(DiPlain& s, const TqDenseQuant& a, const DiCodes& c, const uint8_t* plain, const float* norms, const Tin* x,
                                            int64_t ld, int64_t v0, int64_t n, int tid) {
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, out = 8 * warp + 2 * t;
+  uint32_t in[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) in[j] = __ballot_sync(0xffffffffu, plain[32 * j + lane] && v0 + 32 * j + lane < n);
+  unsigned long long lo = in[0] | (unsigned long long)in[1] << 32, hi = in[2] | (unsigned long long)in[3] << 32;
 #pragma unroll 1
-  for (int row = 0; row < DI_ROWS; ++row) {
-    const int64_t v = v0 + row;
-    if (!plain[row] || v >= n) continue;
-    const float nrm = norms[row], safe = nrm > 0.f ? nrm : 1.0f;
-    const double f = tid < TQ_D ? (double)di_f<Tin>(x[v * ld + tid]) : 0.0;
-    if (tid < TQ_D) s.v[tid] = (double)((float)f / safe);
-    const double y = di_plain_product(s, a.rot_t, tid);
-    const int m = di_search(c, a.bits, y);
-    if (tid < TQ_D && a.out_idx) a.out_idx[v * TQ_D + tid] = (uint8_t)m;
-    double cn = sqrt(di_plain_sum(s, tid < TQ_D ? c.cent[m] * c.cent[m] : 0.0, tid));
-    cn = cn > 1e-10 ? cn : 1.0;
-    if (tid == 0) {
-      if (a.out_norm) a.out_norm[v] = nrm;
-      if (a.out_scale) a.out_scale[v] = (float)(a.norm_correction ? (double)nrm / cn : (double)nrm);
+  while (lo | hi) {
+    int mine = -1;   // this warp's row
+#pragma unroll 1
+    for (int k = 0; k < 16; ++k) {
+      const int r = lo ? __ffsll(lo) - 1 : hi ? 63 + __ffsll(hi) : -1;
+      if (lo) lo &= lo - 1;
+      else hi &= hi - 1;
+      if (k == warp) mine = r;
     }
-    if (a.out_qjl || a.out_rnorm) {
-      if (tid < TQ_D) s.v[tid] = a.norm_correction ? c.cent[m] * (1.0 / cn) : c.cent[m];
-      const double e = f - di_plain_product(s, a.rot, tid) * (double)nrm;
-      const double rr = di_plain_sum(s, tid < TQ_D ? e * e : 0.0, tid);
-      if (tid == 0 && a.out_rnorm) a.out_rnorm[v] = (float)sqrt(rr);
-      if (a.out_qjl) {
-        if (tid < TQ_D) s.v[tid] = e;
-        const uint32_t z = __brev(__ballot_sync(0xffffffffu, !(di_plain_product(s, a.s_t, tid) < 0.0)));   // (first output in the most significant bit)
-        if (tid < TQ_D && (tid & 7) == 0) a.out_qjl[v * 16 + (tid >> 3)] = (uint8_t)(z >> (24 - (tid & 24)));
-      }
-    }
+    di_rows_sync();   // (the rows before have been read)
+    if (lane == 0) s.row[warp] = mine;
+    const float norm = mine >= 0 ? norms[mine] : 0.f, safe = norm > 0.f ? norm : 1.0f;
+#pragma unroll
+    for (int k = lane; k < TQ_D; k += 32) s.v[warp][k] = mine >= 0 ? (double)((float)di_d<Tin>(x[(v0 + mine) * ld + k]) / safe) : 0.0;
     di_rows_sync();
+    const int row[2] = {s.row[g], s.row[g + 8]};
+    double y[4];
+    di_plain_product(y, s, a.rot, tid);
+    int m[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = di_search(c, a.bits, y[i]);
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (row[q] >= 0 && a.out_idx) *reinterpret_cast<uint16_t*>(a.out_idx + (v0 + row[q]) * TQ_D + out) = (uint16_t)(m[2 * q] | m[2 * q + 1] << 8);
+    di_plain_part(s, c.cent[m[0]] * c.cent[m[0]] + c.cent[m[1]] * c.cent[m[1]], c.cent[m[2]] * c.cent[m[2]] + c.cent[m[3]] * c.cent[m[3]], tid);
+    di_rows_sync();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      double cn = sqrt(di_plain_sum(s, g + 8 * q));
+      cn = cn > 1e-10 ? cn : 1.0;
+      if (tid < 32 && t == 0 && row[q] >= 0) {
+        const float nrm = norms[row[q]];
+        if (a.out_norm) a.out_norm[v0 + row[q]] = nrm;
+        if (a.out_scale) a.out_scale[v0 + row[q]] = (float)(a.norm_correction ? (double)nrm / cn : (double)nrm);
+      }
+      const double inv = a.norm_correction ? 1.0 / cn : 1.0;
+      *reinterpret_cast<double2*>(&s.v[g + 8 * q][out]) = make_double2(c.cent[m[2 * q]] * inv, c.cent[m[2 * q + 1]] * inv);
+    }
+    if (!a.out_qjl && !a.out_rnorm) continue;
+    di_rows_sync();
+    di_plain_product(y, s, a.rot_t, tid);
+    double e[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = row[i >> 1];
+      e[i] = r >= 0 ? (double)(float)di_d<Tin>(x[(v0 + r) * ld + out + (i & 1)]) - y[i] * (double)norms[r] : 0.0;
+    }
+    di_plain_part(s, e[0] * e[0] + e[1] * e[1], e[2] * e[2] + e[3] * e[3], tid);
+    di_rows_sync();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      *reinterpret_cast<double2*>(&s.v[g + 8 * q][out]) = make_double2(e[2 * q], e[2 * q + 1]);
+      if (tid < 32 && t == 0 && row[q] >= 0 && a.out_rnorm) a.out_rnorm[v0 + row[q]] = (float)sqrt(di_plain_sum(s, g + 8 * q));
+    }
+    if (!a.out_qjl) continue;
+    di_rows_sync();
+    di_plain_product(y, s, a.s, tid);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {   // (first output in the most significant bit)
+      uint32_t z = (y[2 * q] < 0.0 ? 0u : 2u) << (6 - 2 * t) | (y[2 * q + 1] < 0.0 ? 0u : 1u) << (6 - 2 * t);
+      z |= __shfl_xor_sync(0xffffffffu, z, 1);
+      z |= __shfl_xor_sync(0xffffffffu, z, 2);
+      if (t == 0 && row[q] >= 0) a.out_qjl[(v0 + row[q]) * 16 + warp] = (uint8_t)z;
+    }
   }
 }
 template <typename T> __device__ __forceinline__ T di_from(double v) { return (T)v; }
@@ -527,15 +568,33 @@ template <int BITS> __device__ __forceinline__ uint32_t di_index_float(const DiQ
 
 // Outputs that are too close to a boundary, eight neighbouring columns an entry: the row warps add them once the indices are stored, the
 // copier's warp, which has nothing else to do by then, decides them in fp64.  (By the row warps themselves, whose code for it is not in the
-// instruction caches, a check cost 3 to 4 us, and some CTA of a large call had several.)
+// instruction caches, a check cost 3 to 4 us, and some CTA of a large call had several.)  A random tile has less than one; where there are
+// more than the ring holds, whole rows sixteen at a time are faster than one warp.
 struct DiList {
-  static constexpr int ROOM = 256;
+  static constexpr int ROOM = 32;
   static constexpr uint32_t NONE = 0xffffffffu;
-  volatile uint32_t entry[ROOM];   // row, column / 8 from bit 7, tile of the CTA from bit 11 on; written last
+  volatile uint32_t entry[ROOM];   // in turn; row, column / 8 from bit 7, tile of the CTA from bit 11 on; written last
   float norm[ROOM];
-  int count;                       // entries, and those that found no room: their rows are for di_rows_plain
+  int count;                       // entries so far
+  volatile int taken;              // ... of which the decider has read this many
   volatile int closed;             // no more to come
 };
+// One more, unless there is no room: the row is then for di_rows_plain
+__device__ __forceinline__ bool di_add(DiList& list, uint32_t entry, float norm) {
+  int at = *reinterpret_cast<volatile int*>(&list.count);
+  while (at - list.taken < DiList::ROOM) {   // (another turn only where another thread has added one)
+    const int seen = atomicCAS(&list.count, at, at + 1);
+    if (seen == at) {
+      __threadfence_block();
+      list.norm[at % DiList::ROOM] = norm;
+      __threadfence_block();
+      list.entry[at % DiList::ROOM] = entry;
+      return true;
+    }
+    at = seen;
+  }
+  return false;
+}
 // Indices of eight outputs of a row in fp64, by one warp: four lanes a column, 32 elements each, every load in flight
 template <typename Tin>
 __device__ __forceinline__ int di_check8(const TqDenseQuant& a, const DiCodes& c, const Tin* x, float nrm, int column, int lane) {
@@ -568,9 +627,9 @@ __device__ __forceinline__ void di_decider(DiShared& s, DiList& list, const TqDe
   int done = 0;
   long long since = clock64();
 #pragma unroll 1
-  while (done < DiList::ROOM) {
+  while (true) {
     const bool last = list.closed != 0;
-    const uint32_t e = list.entry[done];
+    const uint32_t e = list.entry[done % DiList::ROOM];
     if (__any_sync(0xffffffffu, e == DiList::NONE)) {
       if (__any_sync(0xffffffffu, last)) break;
       if (__any_sync(0xffffffffu, clock64() - since > LIMIT)) {   // a wait as any other: what the rows still add is not decided
@@ -585,9 +644,16 @@ __device__ __forceinline__ void di_decider(DiShared& s, DiList& list, const TqDe
     }
     since = clock64();
     __threadfence_block();
+    const float nrm = list.norm[done % DiList::ROOM];
+    __syncwarp();
+    ++done;
+    if (lane == 0) {
+      list.entry[(done - 1) % DiList::ROOM] = DiList::NONE;
+      __threadfence_block();
+      list.taken = done;
+    }
     const int64_t v = (blockIdx.x + (int64_t)(e >> 11) * gridDim.x) * DI_ROWS + (e & 127);
     const int column = 8 * ((e >> 7) & 15) + (lane >> 2);
-    const float nrm = list.norm[done++];
     const int m = di_check8<Tin>(a, c, x + v * ld, nrm, 8 * ((e >> 7) & 15), lane);
     if ((lane & 3) == 0) a.out_idx[v * TQ_D + column] = (uint8_t)m;
   }
@@ -624,7 +690,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
   }
   if constexpr (!PROD) {
     if (tid < DiList::ROOM) s_list.entry[tid] = DiList::NONE;
-    if (tid == 0) s_list.count = 0, s_list.closed = 0;
+    if (tid == 0) s_list.count = 0, s_list.taken = 0, s_list.closed = 0;
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sptr(&sh.tmem)), "r"(512u) : "memory");
@@ -856,16 +922,8 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       if constexpr (!PROD) {
         if (unsure && !plain && a.out_idx) {
           __threadfence_block();   // (the indices have been stored)
-          for (; unsure; unsure &= unsure - 1) {
-            const int at = atomicAdd(&s_list.count, 1);
-            if (at >= DiList::ROOM) {
-              plain = true;
-              continue;
-            }
-            s_list.norm[at] = nrm;
-            __threadfence_block();
-            s_list.entry[at] = (uint32_t)row | (uint32_t)(4 * h + __ffs(unsure) - 1) << 7 | (uint32_t)t << 11;
-          }
+          for (; unsure && !plain; unsure &= unsure - 1)
+            plain = !di_add(s_list, (uint32_t)row | (uint32_t)(4 * h + __ffs(unsure) - 1) << 7 | (uint32_t)t << 11, nrm);
         }
       }
       double cn = 1.0;

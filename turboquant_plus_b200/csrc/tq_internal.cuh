@@ -295,7 +295,7 @@ __device__ __forceinline__ int64_t tq_dst_record(const TqQuantDst& dst, int64_t 
 
 // dense-mode work on the fp64 tensor cores (tq_dense.cu); matrices padded to dp x dp
 struct TqDenseQuant {
-  const double *rot, *rot_t, *s, *s_t;   // R, R^T, S, S^T, rows contiguous
+  const double *rot, *rot_t, *s;   // R, R^T, S, rows contiguous
   const double *cent, *bnd;
   int32_t d, dp, bits, norm_correction;
   uint8_t *out_packed, *out_idx;

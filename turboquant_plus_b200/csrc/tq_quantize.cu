@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(128) k_quantize_dense(const TqDenseArgs a, con
 static TqDenseQuant dense_tensor_args(const tq_quantizer* q) {
   TqDenseQuant t;
   memset(&t, 0, sizeof(t));
-  t.rot = q->rotp; t.rot_t = q->rotp_t; t.s = q->sp; t.s_t = q->sp_t;
+  t.rot = q->rotp; t.rot_t = q->rotp_t; t.s = q->sp;
   t.cent = q->cent64; t.bnd = q->bnd64;
   t.d = q->d; t.dp = (q->d + 7) / 8 * 8; t.bits = q->bits; t.norm_correction = q->norm_correction;
   return t;
