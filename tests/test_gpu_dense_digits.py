@@ -273,3 +273,28 @@ def test_copies_of_a_close_vector(n, share, dtype):
             else:
                 assert torch.equal(a, b)
     assert torch.equal(m.quantize(x)[0], torch.cat([m.quantize(x[lo:lo + PIECE])[0] for lo in range(0, n, PIECE)]))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+@pytest.mark.parametrize("scale", [1e-7, 1e-5, 1e-3, 1e-2])
+def test_small_residuals(scale, dtype):
+    """Reconstructions quantized again, with noise of `scale` of their length: residuals from the rows' own rounding on.  Against small calls,
+    whose fp64 sums are off by 4.9e-16 of the vector's length: of a residual, of which fp32 rows leave 2.6e-8 or more, 2e-8, and by an
+    fp32 rounding of 6e-8 on both sides."""
+    import torch
+    import turboquant_plus_b200 as tq
+    n = 20011
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    q = tq.TurboQuant(D, 3, seed=6)
+    x = torch.randn(n, D, device="cuda", generator=gen) * torch.exp(torch.randn(n, 1, device="cuda", generator=gen))
+    code = q.polar_quant.quantize_device(x)
+    y = q.polar_quant.dequantize_device(code["norm"], idx=code["idx"])
+    y = (y + scale * y.norm(dim=1, keepdim=True) * torch.randn(n, D, device="cuda", generator=gen) / D ** 0.5).to(getattr(torch, dtype))
+
+    def quantize(v):
+        out = q.quantize_device(v)
+        return out["idx"], out["norm"], out["qjl"], out["rnorm"]
+
+    whole, parts = quantize(y), _pieces(quantize, y)
+    assert torch.equal(whole[0], parts[0]) and torch.equal(whole[1], parts[1]) and torch.equal(whole[2], parts[2])
+    assert float(((whole[3] - parts[3]).abs() / parts[3]).max()) <= 1.6e-7

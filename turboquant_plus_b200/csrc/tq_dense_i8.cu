@@ -352,6 +352,7 @@ struct DiQuant {
   int32_t zero_idx;                   // index of the value 0
   int32_t shift;                      // sums of 2^-44 to numbers of the boundaries
   double slack;                       // of a projection, per unit of the reconstruction's factor (di_quant_args)
+  float least;                        // elements of a residual that is too short are not above this many 2^-14 of its scale, likewise
   int32_t* status;                    // raised when a wait gives up
   TqDenseQuant q;
 };
@@ -938,8 +939,11 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       }
       if constexpr (PROD) {
         // ---- x_hat = norm R^T c / ||c||, residual x - x_hat, with the norm that is returned and stored (fp32).  Six digits each:
-        // what the 13 products left out would add is below 2^-36.4 of r_scale cent_scale, in practice 2^-44 of the residual's length, whose
-        // fp32 rounding is 2^-25 (with five digits 2^-36, and one residual norm in 4,000 came out a neighbour) ----
+        // what the 13 products left out would add to an element is below 2^-36.4 of r_scale cent_scale, to all 128 together 2^-32.9, in
+        // practice 2^-44 of the vector's length (with five digits 2^-36, and one residual norm in 4,000 came out a neighbour).  Residuals
+        // longer than 2^-6 of that unit, for a random rotation 2^-9 of the vector's length, are therefore within 2^-26.9 of their own, and
+        // rounded to fp32.  Shorter ones, of vectors that are reconstructions, are for di_rows_plain (norms off by 2e-6 otherwise): rows none
+        // of whose elements, of the columns of one thread, is above that (`least`) ----
         const double inv = a.norm_correction ? 1.0 / cn : 1.0;
         const double back = -0x1p-32 * A.r_scale * A.cent_scale * inv * (double)nrm;
         const double unit = nrm > 0.f && nrm < 1e38f ? ldexp(1.0, -(ilogbf(nrm) + 2)) : 1.0;   // |residual| x unit < 1 for a rotation
@@ -958,17 +962,20 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
           for (int k = 0; k < 8; ++k) {
             const double e = fma(di_double(acc[8 * c + k]), back, (double)f[k]);
             rr[k & 3] = fma(e, e, rr[k & 3]);
-            // to a whole number of 2^-46, in balanced digits; the upper half tells what is too large
+            // to a whole number of 2^-46, in balanced digits; the upper half tells what is too large, or too small in all elements
             const unsigned long long w = (unsigned long long)__double_as_longlong(fma(e, unit46, 6755399441055744.0));
             over = max(over, (uint32_t)(w >> 32) - 0x43380000u + 31000u);
             u[k] = di_split((w + 0x8080808080ull) ^ 0x8080808080ull);
           }
           di_store8<6, 0>(area, 8 * h + 2 * c, u);
         }
-        plain |= over > 62000u;
+        // (too large, or too small in all elements; rows of zeros are neither)
+        const uint32_t least = nrm != 0.f ? __float2uint_ru(fminf(A.least * (float)inv, 31000.f)) : 0u;
+        plain |= over - 31000u - least > 31000u - least;
         operand_ready(0);
         di_rows_sync();   // (the sums of the squared centroids have been read, and the rows)
-        s_part[h][row] = (rr[0] + rr[1]) + (rr[2] + rr[3]);
+        const double part = (rr[0] + rr[1]) + (rr[2] + rr[3]);
+        s_part[h][row] = part;
         if (t + 1 < mine) load_tile(blockIdx.x + (t + 1) * step);
         di_rows_sync();
         if (h == 0 && live && a.out_rnorm)
@@ -1450,6 +1457,7 @@ static bool di_quant_args(const TqDenseQuant& a, const TqDenseDigits& g, const v
   A.r_scale = g.r_scale / 4096.0;
   A.cent_scale = g.cent_scale;
   A.slack = 32768.0 * g.r_scale * g.cent_scale;
+  A.least = (float)(128.0 * g.r_scale * g.cent_scale);
   A.status = tq_quantize_status_word();
   for (int p = 0; p < DI_DIGITS; ++p) A.words[p] = make_uint2(g.words[p][0], g.words[p][1]);
   // Boundaries as numbers of 2^-27 of r_scale (no y is beyond 16 of them: entries of R are below r_scale, rows of w shorter than 1 + 2^-20),
