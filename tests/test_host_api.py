@@ -92,6 +92,22 @@ def test_runs_of_rows(layers, heads, rows, width):
     assert torch.equal(host.join(pieces), t) and (len(pieces) < 2 or not rows or host.join(pieces).data_ptr() != odd.data_ptr())
 
 
+def test_runs_of_single_rows_and_single_runs():
+    """A run of one row is contiguous whatever the stride between rows says; one run alone comes as torch.cat gives it."""
+    from turboquant_plus_b200 import _native as nv
+    host = nv.host()
+    t = torch.arange(512, dtype=torch.float32).reshape(2, 256)
+    halves = [t[:1, :128], t[:1, 128:]]                                  # one after the other in memory, rows 256 apart
+    assert all(h.is_contiguous() and h.stride(0) == 256 for h in halves)
+    assert torch.equal(host.join(halves), torch.cat(halves)) and host.join(halves).is_contiguous()
+    one = [t[0, 3:4].as_strided((1,), (7,)), t[0, 4:5].as_strided((1,), (7,))]
+    assert torch.equal(host.join(one), torch.cat(one))
+    for piece in (t[:, ::2], t.t(), t[:, 0], t.reshape(-1)[1:257], t[:1, 1:129]):
+        whole = host.join([piece])
+        assert torch.equal(whole, piece) and whole.is_contiguous() and whole.data_ptr() % 16 == 0
+    assert host.join([t]).data_ptr() == t.data_ptr()
+
+
 def test_runs_of_rows_refuses():
     from turboquant_plus_b200 import _native as nv
     host, t = nv.host(), torch.zeros(6, 4)

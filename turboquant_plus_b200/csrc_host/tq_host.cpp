@@ -348,7 +348,6 @@ PyObject* join(PyObject*, PyObject* list) {
     if (!PyList_Check(list) || PyList_GET_SIZE(list) == 0) raise(PyExc_ValueError, "join needs a list of tensors");
     const Py_ssize_t n = PyList_GET_SIZE(list);
     const at::Tensor& first = tensor(PyList_GET_ITEM(list, 0), "piece");
-    if (n == 1) return Py_NewRef(PyList_GET_ITEM(list, 0));
     bool plain = first.layout() == at::kStrided && first.has_storage() && !first.requires_grad() && !first.is_conj() && !first.is_neg() &&
                  first.dim() >= 1 && reinterpret_cast<uintptr_t>(first.const_data_ptr()) % 16 == 0;
     int64_t rows = 0, at = plain ? first.storage_offset() : 0;
@@ -362,10 +361,12 @@ PyObject* join(PyObject*, PyObject* list) {
         at += t.numel();
       }
     }
+    if (plain && n == 1) return Py_NewRef(PyList_GET_ITEM(list, 0));
     if (plain) {
-      std::vector<int64_t> sizes(first.sizes().begin(), first.sizes().end());
+      std::vector<int64_t> sizes(first.sizes().begin(), first.sizes().end()), strides(sizes.size(), 1);
       sizes[0] = rows;
-      return THPVariable_Wrap(first.as_strided(sizes, first.strides(), first.storage_offset()));
+      for (size_t k = sizes.size() - 1; k > 0; --k) strides[k - 1] = strides[k] * std::max<int64_t>(sizes[k], 1);   // (a piece's own: any where it has one row)
+      return THPVariable_Wrap(first.as_strided(sizes, strides, first.storage_offset()));
     }
     std::vector<at::Tensor> all;
     for (Py_ssize_t i = 0; i < n; ++i) all.push_back(tensor(PyList_GET_ITEM(list, i), "piece"));
