@@ -323,7 +323,9 @@ __device__ __forceinline__ void store_rows(const AttnParams& P, const uint32_t (
       x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
       if (!P.v_ident) warp_wht128(x, vs2, vs1, lane);  // R^T = D1 (H/sqrt d) D2
       const size_t at = (row0 + head) * TQ_D + 4 * lane;
-      if (P.out_dtype != TQ_F32 && (reinterpret_cast<uintptr_t>(P.out) & 7) == 0) {   // a lane's four 16-bit results at once
+      if (P.out_dtype == TQ_F32) {   // a lane's four results at once (the entries take outputs on 16 bytes)
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(P.out) + at) = make_float4(x[0], x[1], x[2], x[3]);
+      } else {
         uint2 u;
         if (P.out_dtype == TQ_F16) {
           u = make_uint2(pack_h2(x[0], x[1]), pack_h2(x[2], x[3]));
@@ -332,9 +334,6 @@ __device__ __forceinline__ void store_rows(const AttnParams& P, const uint32_t (
           u = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
         }
         *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(P.out) + at) = u;
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) store_out(P.out, P.out_dtype, at + k, x[k]);
       }
       if constexpr (HEADS <= NT / 32) break;
     }
