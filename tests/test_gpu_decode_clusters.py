@@ -42,3 +42,42 @@ def test_splits_of_a_cluster(k, v, group, lengths):
         scores = np.einsum("hd,htd->ht", qb[0], np.repeat(rows[0][0], group, axis=0)) / np.sqrt(D)
         want = scores.max(1) + np.log(np.exp(scores - scores.max(1, keepdims=True)).sum(1))
         assert np.abs(lse[b].cpu().numpy() - want).max() < 2e-3
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("lengths", [[517], [100], [1000, 257, 40]])
+def test_captured_with_its_append(lengths, dtype):
+    """The new token's append and the attention behind it as a graph, in every type of result: bit for bit what the calls give one by one,
+    and within one rounding of the type of the fp32 results."""
+    import torch
+    import turboquant_plus_b200 as tq
+    hkv, group = 2, 4
+    rng = np.random.default_rng(sum(lengths))
+    cache = tq.PagedKVCache(D, hkv, 60, 128, "turbo3", "turbo3", seed=42)
+    kh, vh = ([rng.standard_normal((n, hkv, D)).astype(np.float16) for n in lengths] for _ in range(2))
+    table = fill_cache(cache, kh, vh, lengths, rng)
+    pages, lens = torch.as_tensor(table).to(device="cuda", dtype=torch.int32), torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    last = lens.long() - 1
+    slots = pages.long()[torch.arange(len(lengths), device="cuda"), last // 128] * 128 + last % 128
+    k, v = (torch.as_tensor(rng.standard_normal((len(lengths), hkv, D)).astype(np.float16)).cuda() for _ in range(2))
+    q = torch.as_tensor(rng.standard_normal((len(lengths), hkv * group, D)).astype(np.float16)).cuda().to(getattr(torch, dtype))
+    ws = cache.workspace(len(lengths), hkv * group, pages.shape[1])
+
+    def step(out):
+        cache.append(k, v, slots)
+        cache.attend(q, pages, lens, out=out, workspace=ws, overlap="append")
+
+    eager, captured, graph = torch.empty_like(q), torch.zeros_like(q), torch.cuda.CUDAGraph()
+    step(eager)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        step(captured)
+    for _ in range(3):
+        captured.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(captured, eager) and cache.kernel_status(ws) == 0
+    graph.reset()
+    exact = cache.attend(q.float(), pages, lens)
+    eps = {"float16": 2.0 ** -11, "bfloat16": 2.0 ** -8, "float32": 2.0 ** -20}[dtype]
+    assert bool(((eager.float() - exact.float()).abs() <= eps * exact.float().abs() + 1e-7).all())

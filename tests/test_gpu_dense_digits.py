@@ -298,3 +298,33 @@ def test_small_residuals(scale, dtype):
     whole, parts = quantize(y), _pieces(quantize, y)
     assert torch.equal(whole[0], parts[0]) and torch.equal(whole[1], parts[1]) and torch.equal(whole[2], parts[2])
     assert float(((whole[3] - parts[3]).abs() / parts[3]).max()) <= 1.6e-7
+
+
+@pytest.mark.parametrize("width,column", [(256, 0), (256, 128), (130, 2), (257, 1), (129, 0)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_results_into_columns_of_wider_rows(width, column, accumulate):
+    """fp64 results beside, or added to, what wider rows hold: by tiled copies where base and rows are on 16 bytes, else by stores; a last tile
+    whose rows end within a warp's 32."""
+    import torch
+    import turboquant_plus_b200 as tq
+    from turboquant_plus_b200 import _native as nv
+    n = 9473 + 128 * 148 + 39
+    gen = torch.Generator(device="cuda").manual_seed(n + width)
+    q = tq.TurboQuantMSE(D, 3, seed=6).polar_quant
+    code = q.quantize_device(torch.randn(n, D, device="cuda", generator=gen))
+    held = torch.randn(n + 1, width, device="cuda", generator=gen, dtype=torch.float64)
+    handle, got = q._native(held.device).handle, []
+    for piece in (n, PIECE):
+        out = held.clone()
+        for lo in range(0, n, piece):
+            m = min(piece, n - lo)
+            nv.call("tq_dequantize_strided", handle, nv.ptr(code["idx"][lo:lo + m]), nv.ptr(code["norm"][lo:lo + m]), m, nv.ptr(out[lo:, column:]),
+                    width, accumulate, nv.stream_ptr())
+        got.append(out)
+    whole, few = got
+    rest = torch.ones(n + 1, width, dtype=torch.bool, device="cuda")
+    rest[:n, column:column + D] = False
+    assert torch.equal(whole[rest], held[rest])
+    a, b = whole[:n, column:column + D], few[:n, column:column + D]
+    assert not torch.equal(a, held[:n, column:column + D])
+    assert bool(((a - b).abs() <= 256 * 2.0 ** -53 * b.abs().amax(dim=1, keepdim=True)).all())
