@@ -45,6 +45,46 @@ def test_prefill_pairs(kf, vf, group, chunk, lens):
     assert max(errs) < TOL, f"{kf}/{vf}: {max(errs)}"
 
 
+def _coarse_bytes(chunk, hq, hkv, pages, sms):
+    """The workspace of one sequence's chunk with at least eight pages a split, in the form that needs more."""
+    blocks, most = -(-chunk * (hq // hkv) // 128), 0
+    for cg in (1, 2):
+        base, slots = -(-blocks // cg) * hkv, sms // cg
+        s = min(range(1, min(max(pages // 8, 1), 64) + 1), key=lambda c: -(-base * c // slots) * (-(-pages // c) + 12))
+        splits = -(-pages // -(-pages // s))
+        total = blocks * hkv * splits * (128 * D * 4 + 128 * 2 * 4) + 65536 * 4 + 256
+        most = max(most, -(-total // 256) * 256)
+    return most
+
+
+@pytest.mark.parametrize("kf,vf", [("turbo3", "turbo3"), ("q8_0", "turbo2"), ("prod3", "turbo3")])
+@pytest.mark.parametrize("hq,hkv,pages", [(32, 8, 20), (16, 2, 40), (4, 1, 9)])
+def test_workspaces_that_the_finest_plan_does_not_fit(kf, vf, hq, hkv, pages):
+    """A workspace for fewer splits serves the call: sized for a prompt's largest chunk, it has to do for its last one."""
+    import torch
+    import turboquant_plus_b200 as tq
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    gen = torch.Generator(device="cuda").manual_seed(pages)
+    cache = tq.PagedKVCache(D, hkv, pages, 128, kf, vf, seed=42)
+    n = pages * 128 - 40
+    cache.append(*(torch.randn((n, hkv, D), device="cuda", generator=gen) for _ in range(2)), torch.arange(n, device="cuda"))
+    table, lens = torch.arange(pages, dtype=torch.int32)[None], torch.tensor([n])
+    smaller = 0
+    for chunk in (16, 26, 40, 64, 96, 130, 200, 320, 512):
+        q = torch.randn((1, chunk, hq, D), device="cuda", generator=gen)
+        size = _coarse_bytes(chunk, hq, hkv, pages, sms)
+        smaller += size < tq._native.load().tq_prefill_workspace_bytes(1, chunk, hq, hkv, pages)
+        ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
+        out, want = cache.prefill_attend(q, table, lens, workspace=ws), cache.prefill_attend(q, table, lens)
+        assert cache.kernel_status(ws) == 0 and cache.kernel_status() == 0
+        # (probabilities are fp16 numbers relative to the largest of their split: either side is within TOL of exact sums)
+        assert float((out - want).abs().max() / want.abs().max()) < 2 * TOL
+        if kf == "turbo3":
+            with pytest.raises(RuntimeError):
+                cache.prefill_attend(q, table, lens, workspace=torch.zeros(65536 * 4 + 256, dtype=torch.uint8, device="cuda"))
+    assert smaller >= 3
+
+
 @pytest.mark.parametrize("kf,vf", [("turbo3", "turbo3"), ("turbo4", "turbo2"), ("prod3", "turbo3")])
 @pytest.mark.parametrize("hkv,group,chunk,lens", [(8, 2, 128, [128, 1]), (8, 4, 64, [64, 200]), (8, 4, 90, [700, 90])])
 def test_first_page_beside_the_rows(kf, vf, hkv, group, chunk, lens):

@@ -1116,8 +1116,9 @@ struct PfPlan {
 static const size_t PF_TAIL = 65536 * 4 + 256;  // tickets + status word, at the end of the workspace
 static const long PF_CTA_COST_PAGES = 12;  // prologue, partial and merge of a CTA, in units of one page of the main loop
 
-// the plan of a form: cg CTAs per operand tile
-static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_pages, int cg) {
+// The plan of a form: cg CTAs per operand tile.  coarse: at least eight pages per split, for workspaces that the finer one does not fit
+// (sized for a prompt's largest chunk, of few splits, they have to do for its last one).
+static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_pages, int cg, bool coarse = false) {
   PfPlan p;
   p.row_blocks = (chunk_tokens * (hq / hkv) + PF_ROWS - 1) / PF_ROWS;
   const long base = (long)((p.row_blocks + cg - 1) / cg) * hkv * batch;
@@ -1126,12 +1127,12 @@ static PfPlan pf_plan(int batch, int chunk_tokens, int hq, int hkv, int max_page
   // them, 0.8 of a page each (without that, and down to three pages a split, 22 queries over 16,000 tokens of one KV head went from 55 to
   // 69 us).  At least three pages per split: where eight were the least, 26 queries over 2,300 tokens of turbo3, 32 / 8 heads, took 37 us
   // and take 31; 32 over 1,500 of turbo4 43 and 29; 128 over 4,000 of prod3 / turbo3, 16 / 4 heads, 74 and 63.
-  const int cap = max_pages / 3 > 1 ? max_pages / 3 : 1;
+  const int least = coarse ? 8 : 3, cap = max_pages / least > 1 ? max_pages / least : 1;
   int s = 1;
   long best = -1;
   for (int c = 1; c <= cap && c <= 64; ++c) {
     const long waves = (base * c + slots - 1) / slots;
-    const long cost = 10 * waves * ((max_pages + c - 1) / c + PF_CTA_COST_PAGES) + (c > 1 ? 8 * c : 0);
+    const long cost = 10 * waves * ((max_pages + c - 1) / c + PF_CTA_COST_PAGES) + (c > 1 && !coarse ? 8 * c : 0);
     if (best < 0 || cost < best) {
       best = cost;
       s = c;
@@ -1247,17 +1248,21 @@ extern "C" int tq_prefill_attn(const tq_quantizer* kq, const tq_quantizer* vq, c
   P.hq = num_q_heads;
   P.hkv = L->num_kv_heads;
   P.group = num_q_heads / L->num_kv_heads;
-  PfPlan plan = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, 1);
-  if ((k_q8 || k_prod || v_q8) &&
-      pf_takes_rows(plan, pf_row_pages(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq),
-                    (int64_t)batch * chunk_tokens * L->num_kv_heads, k_prod, P.group) &&
-      tq_decode_workspace_bytes(batch * chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq) <= workspace_bytes)
-    return tq_decode_chunk(kq, vq, L, pool_dev, block_table_dev, max_pages_per_seq, kv_lens_dev, q_dev, q_dtype, batch, chunk_tokens,
-                           num_q_heads, scale, workspace_dev, workspace_bytes, out_dev, out_dtype, stream);
+  PfPlan plan;
   int cg = 1;
-  if (plan.row_blocks > 1 && !k_prod) {
-    const PfPlan pair = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, 2);
-    if (pf_time_ns(pair, L->k_format, L->v_format, 2) < pf_time_ns(plan, L->k_format, L->v_format, 1)) plan = pair, cg = 2;
+  for (const bool coarse : {false, true}) {
+    plan = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, cg = 1, coarse);
+    if ((k_q8 || k_prod || v_q8) &&
+        pf_takes_rows(plan, pf_row_pages(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq),
+                      (int64_t)batch * chunk_tokens * L->num_kv_heads, k_prod, P.group) &&
+        tq_decode_workspace_bytes(batch * chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq) <= workspace_bytes)
+      return tq_decode_chunk(kq, vq, L, pool_dev, block_table_dev, max_pages_per_seq, kv_lens_dev, q_dev, q_dtype, batch, chunk_tokens,
+                             num_q_heads, scale, workspace_dev, workspace_bytes, out_dev, out_dtype, stream);
+    if (plan.row_blocks > 1 && !k_prod) {
+      const PfPlan pair = pf_plan(batch, chunk_tokens, num_q_heads, L->num_kv_heads, max_pages_per_seq, 2, coarse);
+      if (pf_time_ns(pair, L->k_format, L->v_format, 2) < pf_time_ns(plan, L->k_format, L->v_format, 1)) plan = pair, cg = 2;
+    }
+    if ((int64_t)plan.total <= workspace_bytes) break;
   }
   TQ_REQUIRE((int64_t)plan.total <= workspace_bytes, TQ_ERR_TOO_LARGE,
              "prefill workspace of %lld bytes is smaller than the %lld needed (tq_prefill_workspace_bytes)",
