@@ -919,8 +919,21 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
     // warp order
     constexpr int DPT = NH * TQ_D / NT;     // 2, 4 or 8
     const int head = tid / (TQ_D / DPT), dim = DPT * (tid % (TQ_D / DPT));
+    // Four warps (chains, many CTAs): the partial of several splits is stored where its values are added up, the single split's way behind
+    // it; eight warps the other way round.  The order alone is worth this much (us; 32/8 heads; single splits in front / behind): 40 chained
+    // layers over 32,768 tokens 416.0 / 413.3 a step, 256 ragged sequences of prod3 / turbo3 1,268 / 1,264; one sequence of 128 tokens of
+    // turbo3 4.09 / 4.23, of 1,500 of turbo4 6.83 / 6.96.
+    constexpr bool EARLY = NW == 4;
+    static_assert(!(EARLY && CL), "clusters are of eight-warp CTAs");
     float a[DPT], M = -INFINITY, Lsum = 0.f;
     const bool several = ns != 1;
+    auto store_partial = [&]() {
+      const size_t slot = (row0 + head) * P.num_splits + split;
+#pragma unroll
+      for (int k = 0; k < DPT; k += 2)
+        *reinterpret_cast<float2*>(P.part_o + slot * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
+      if (dim == 0) *reinterpret_cast<float2*>(P.part_ml + slot * 2) = make_float2(M, Lsum);
+    };
     if (head < P.group) {
       float mw[NW];
 #pragma unroll
@@ -938,25 +951,18 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
         for (int k = 0; k < DPT; ++k) a[k] = fmaf(v[k], f, a[k]);
         Lsum = fmaf(sml[(w * NH + head) * 2 + 1], f, Lsum);
       }
-      if (!CL && several) {
-        const size_t slot = (row0 + head) * P.num_splits + split;
-#pragma unroll
-        for (int k = 0; k < DPT; k += 2)
-          *reinterpret_cast<float2*>(P.part_o + slot * TQ_D + dim + k) = make_float2(a[k], a[k + 1]);
-        if (dim == 0) *reinterpret_cast<float2*>(P.part_ml + slot * 2) = make_float2(M, Lsum);
-      }
+      if (EARLY && several) store_partial();
     }
     // The only split is finished here, as the fold of one would (its partial, a ticket and the way back were 2 us of each CTA; turbo3,
     // 32/8 heads, 128 sequences of 100 tokens 15.4 -> 11.1 us, one of 128 5.8 -> 3.8).  Splits in a cluster: the first CTA takes the
-    // others' rows out of their shared memory.  One copy of the code that stores rows, and the partial of several splits stored where its
-    // values were added up: with one copy per way here long contexts took 0.06 us a call longer, with the partial behind the single split's
-    // code another 0.06 (40 layers over 32,768 tokens 413.0 without a way for single splits / 416.0 / 413.3 now, 256 ragged sequences of
-    // prod3 / turbo3 1,261 / 1,268 / 1,264, two of 131,072 tokens of turbo4 93.8 / 94.3 / 93.8).
-    if (!CL && several) {
-      if (!merge_splits<VT::Q8, NT, NH>(P, fv.alpha, qbuf, s_flags, row0, ns, b, kvh, tid, bar_id)) return;
-    } else {
+    // others' rows out of their shared memory.  One copy of the code that stores rows: with one per way here, long contexts took 0.06 us
+    // a call longer.
+    auto merge = [&]() { return merge_splits<VT::Q8, NT, NH>(P, fv.alpha, qbuf, s_flags, row0, ns, b, kvh, tid, bar_id); };
+    if (EARLY && several) {
+      if (!merge()) return;
+    } else if (EARLY || CL || !several) {
       if (tid == 0 && s_flags[0]) atomicExch(P.status, 1);
-      if (CL && ns > 1) {
+      if (CL && several) {
         float2* ml = reinterpret_cast<float2*>(stage0);   // (the warps' rows there have been read)
         group_sync<NT>(bar_id);
         if (head < P.group) {
@@ -983,10 +989,13 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_decode_attn_g4(const __gri
         if (P.lse && dim == 0) P.lse[row0 + head] = (M + log2f(Lsum)) * 0.6931471805599453f;
       }
       group_sync<NT>(bar_id);
+    } else {
+      if (head < P.group) store_partial();
+      if (!merge()) return;
     }
   }
   store_rows<NT, NH>(P, fv.s1, fv.s2, rows, row0, tid);
-  if (CL && ns > 1) cluster_wait();
+  if (CL && ns != 1) cluster_wait();
 }
 
 template <int KK, int VK, bool SPARSE, bool NODEQ, int NW, bool TAIL, int NH, bool CL>

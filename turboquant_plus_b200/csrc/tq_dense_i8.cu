@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(DI_THREADS, 1) k_dense_quantize_i8(const __gri
       const float* s_norm = s_norms[t & 1];
       uint8_t* s_plain = s_plains[t & 1];
       // ---- y = R w: indices, ||c[idx]||^2, the centroids as the next operand.  Without the sketch of the 34 products of all digits ten,
-      // which leave less than 2^-21 of r_scale out: one output in 90,000 of a rotation's with eight centroids is too close to a boundary
+      // which leave at most 1.004 x 2^-21 of r_scale out (di_quant_args): one output in 90,000 of a rotation's with eight centroids is too close to a boundary
       // and is left to the decider.  With the sketch, where other outputs hang on it, 14 products: one in six million; its row is for
       // di_rows_plain.  Rows of zeros are on no boundary.
       uint32_t packed[DI_COLS / 4];

@@ -510,8 +510,8 @@ __global__ void __launch_bounds__(PfSmem2<KK, VK, CG>::THREADS, 1) k_prefill_att
   // The rows' staging and exchange area ends where the records begin: 64 KB, or 32 in a pair whose 16-bit queries are rotated by
   // transforms.  So the first page's K tile is another memory, and its producers fill their tables and dequantize it while the rows are
   // rotated (7,000 clocks); one before and one behind them, the two were another 4,000.  With the append, 32 / 8 heads: a prompt of 3,999
-  // tokens, turbo4 / turbo3, 273 -> 268 us, the last 128 of 8,192 positions of two sequences, q8_0 / turbo2, 82 -> 78; 64 / 8 heads, the
-  // last 128 of 131,072, turbo3, 832 -> 817.  A pair's `wide` rows need that tile too.
+  // tokens, turbo4 / turbo3, 273 -> 268 us, the last 128 of 8,192 positions of two sequences, q8_0 / turbo2, 82 -> 78 (64 / 8 heads, the
+  // last 128 of 131,072: 1 to 2 % of some 830 with the copies below, no more than its runs differ by).  A pair's `wide` rows need that tile too.
   const bool wide = CG == 2 && !KT::Q8 && (q_esz == 4 || P.k_rot_t != nullptr);
   uint8_t* const rows_at = sm + SP::OFF_ST - (CG == 2 && !KT::Q8 && !wide ? 32768 : 65536);
   // Rows pass through shared memory: accessed directly, a thread's own half row would put the lanes of a load 256 or 512
