@@ -390,7 +390,8 @@ int tq_attn_merge(const void* out_a_dev, const float* lse_a_dev, const void* out
  *   Short chunks over q8_0 or PROD tensors run as rows of the decode kernel, one per query with its causal length.
  *   The page range of a row block is split over several CTAs when the grid would otherwise not fill
  *   the GPU; the last split to finish folds the partials (ticket, as in tq_decode_attn).
- *   workspace_dev: tq_prefill_workspace_bytes(...) bytes, 256-byte aligned, initialised once with
+ *   workspace_dev: tq_prefill_workspace_bytes(...) bytes (where fewer hold the partials of splits of at least eight pages, such
+ *   splits are taken), 256-byte aligned, initialised once with
  *   tq_decode_workspace_init (or zero-filled); same tail layout as the decode workspace, so one
  *   buffer of the larger size serves both; tq_decode_status_sync reads its status word. */
 int64_t tq_prefill_workspace_bytes(int32_t batch, int32_t chunk_tokens, int32_t num_q_heads,
